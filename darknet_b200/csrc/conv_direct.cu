@@ -1,11 +1,12 @@
-// Direct convolution on the CUDA cores (fp32 FMA, fp32 accumulate).
+// Direct convolution on the CUDA cores (fp32 FMA, fp32 accumulate): a general kernel (any filter size, narrow groups), a
+// tiled GEMM for 1x1 and 3x3 filters with more than 16 filters per group, and a first-layer specialisation.
 //
 // Used where the tensor-core kernel does not apply: very narrow inputs (the
 // 3-channel first layer, which it reads straight from Darknet's NCHW input),
 // grouped convolutions, and DNB_MODE_FP32 networks.
 //
-// A block owns 128 consecutive output pixels and a slab of FB = 32 filters; a
-// thread owns one pixel and all 32 filters of the slab.  The slab's weights are
+// General kernel: a block owns 128 consecutive output pixels and a slab of FB filters; a
+// thread owns one pixel and all filters of the slab.  The slab's weights are
 // staged through shared memory in K chunks together with a (c,kh,kw) table, so
 // the inner loop is one predicated, warp-coalesced load of x and 32 FMAs fed by
 // broadcast 16-byte shared loads.  Accumulation runs over
@@ -19,13 +20,15 @@
 
 namespace dnb {
 
-constexpr int FB = 32;         // filters per thread / per block slab
+constexpr int FB = 32;         // filters per thread / per block slab (the general kernel also has narrower slabs)
 constexpr int KCHUNK = 192;    // taps staged per pass: 192 * (32*4 + 4) B = 25 KB
 constexpr int DTHREADS = 128;  // pixels per block
 
-template <typename TX, typename TY>
+// FB: filters per slab, 4 to 32: a grouped layer with few filters per group would spend most of a wide slab's FMAs on
+// filters that do not exist.
+template <typename TX, typename TY, int FB>
 __global__ void __launch_bounds__(DTHREADS)
-conv_direct_kernel(DirectArgs a)
+conv_direct_kernel(const __grid_constant__ DirectArgs a)
 {
     __shared__ __align__(16) float w_s[KCHUNK][FB];
     __shared__ int tap_s[KCHUNK];
@@ -72,7 +75,8 @@ conv_direct_kernel(DirectArgs a)
         }
         __syncthreads();
         if (live) {
-            for (int kk = 0; kk < kn; ++kk) {
+#pragma unroll 4
+            for (int kk = 0; kk < kn; ++kk) {   // four taps' loads in flight
                 const int t = tap_s[kk];
                 const int c = t >> 8, ih = ih0 + ((t >> 4) & 15), iw = iw0 + (t & 15);
                 float xv = 0.f;
@@ -135,11 +139,315 @@ conv_direct_kernel(DirectArgs a)
                 base[(size_t)p * a.y_cpitch + j] = from_float<TY>(out_s[p][j]);
             }
         }
+        // padding channels that the last slab does not reach
+        if (last)
+            for (int ch = n0 + cols; ch < min(a.y_cpitch, (g.n + 7) & ~7); ++ch)
+                if (live) reinterpret_cast<TY *>(a.y_nhwc)[(size_t)pix * a.y_cpitch + ch] = from_float<TY>(0.f);
     }
     if (a.y_nchw && live) {
         const size_t plane = (size_t)g.out_h * g.out_w;
         float *dst = a.y_nchw + ((size_t)b * g.n + n0) * plane + (size_t)oh * g.out_w + ow;
         for (int j = 0; j < nvalid; ++j) dst[j * plane] = out_s[threadIdx.x][j];
+    }
+}
+
+// ------------------------------------------------------------------ tiled fp32 GEMM (1x1 and 3x3 filters)
+// What bounds it is FMA issue and the 128 bytes per clock that shared memory returns to registers.  The
+// one-pixel-per-thread kernel above issues a load, its bounds tests and eight shared loads for every 32 FMAs and shares no
+// input value between threads.  Here a block multiplies BM pixels by BN filters from shared memory and a thread keeps
+// TM pixels x TN filters, two pixels to a packed fma.rn.f32x2 (the halves are independent IEEE fp32 FMAs): with 16 x 8 a
+// thread reads 96 bytes for 128 FMAs, under the one byte per FMA at which the two limits meet (8 x 8 with the weights
+// stored twice, as an operand pair, read 96 bytes for 64 and ran at 0.6 of this rate: LSU wavefronts 69 % under ncu).
+// A chunk of K is CPC channels x the taps of one filter row (VEC) or of all rows: every load's tap is a compile-time
+// constant, its bounds test one bit of a mask built once per thread.
+//   VEC false (NCHW, or channels-last tensors whose groups start off a 4-channel boundary): values go from global to
+//     shared memory with 4-byte cp.async, coalesced along the pixels of an NCHW row, three chunks in rotation.
+//   VEC true (channels-last): 4 channels of a pixel per load, through registers (the tile is channel-major in shared
+//     memory), two chunks in rotation.
+__device__ __forceinline__ void ffma2(unsigned long long &d, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long twice(float v)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ void cp_async4(void *dst, const void *src, bool in)   // zero where !in: the source is then not read
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// KS: 1 or 3.  (BM / TM) * (BN / TN) threads.
+template <typename TX, typename TY, int KS, int BM, int BN, int TM, int TN, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM == 16 ? 4 : 7)
+conv_fp32_gemm_kernel(const __grid_constant__ DirectArgs a)
+{
+    constexpr int THREADS = (BM / TM) * (BN / TN);
+    static_assert(THREADS == 64 && (BM / TM == 8 || BM / TM == 16), "two warps, 8 x 4 threads each");
+    static_assert(VEC || sizeof(TX) == 4, "cp.async copies f32 values");
+    constexpr int NPX = BM > THREADS ? BM / THREADS : 1;        // pixels whose values a thread fetches
+    constexpr int TPP = THREADS > BM ? THREADS / BM : 1;        // threads that share a pixel's values, by channel
+    constexpr int ROWS = VEC ? KS : 1;                          // chunks per channel block: one per filter row, or one
+    constexpr int TAPS = VEC ? KS : KS * KS;                    // taps per chunk
+    constexpr int CPC = KS == 1 ? (VEC ? 8 : 16) : (VEC ? 4 * TPP : 2);   // channels per chunk
+    constexpr int CPT = CPC / TPP;                              // ... that one thread fetches per pixel
+    constexpr int KC = CPC * TAPS;
+    constexpr int NST = VEC ? 2 : 3;
+    constexpr int BV = (KC * BN / 4 + THREADS - 1) / THREADS;
+    __shared__ __align__(16) float a_s[NST][KC][BM];
+    __shared__ __align__(16) float b_s[NST][KC][BN];
+
+    const ConvGeom &g = a.g;
+    const int cpg = g.c / g.groups, npg = g.n / g.groups;
+    const int fblocks = (npg + BN - 1) / BN;
+    const int grp = blockIdx.y / fblocks, f0 = (blockIdx.y - grp * fblocks) * BN;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long npix = (long long)g.batch * g.out_h * g.out_w;
+    const long long pix0 = (long long)blockIdx.x * BM;
+    const int csub = TPP > 1 ? (tid / BM) * CPT : 0;            // this thread's first channel of a chunk
+
+    const TX *xp[NPX];
+    uint32_t in_mask[NPX];
+#pragma unroll
+    for (int u = 0; u < NPX; ++u) {
+        const long long pix = pix0 + tid % BM + u * THREADS;
+        int b = 0, oh = 0, ow = 0;
+        if (pix < npix) {
+            ow = (int)(pix % g.out_w);
+            const long long t = pix / g.out_w;
+            oh = (int)(t % g.out_h);
+            b = (int)(t / g.out_h);
+        }
+        const int ih0 = oh * g.stride - g.pad, iw0 = ow * g.stride - g.pad;
+        xp[u] = reinterpret_cast<const TX *>(a.x) + b * a.xs_b + (long long)(grp * cpg + csub) * a.xs_c + (long long)ih0 * a.xs_h + (long long)iw0 * a.xs_w;
+        uint32_t m = 0;
+#pragma unroll
+        for (int t = 0; t < KS * KS; ++t)
+            if (pix < npix && (unsigned)(ih0 + t / KS) < (unsigned)g.h && (unsigned)(iw0 + t % KS) < (unsigned)g.w) m |= 1u << t;
+        in_mask[u] = m;
+    }
+    int off[TAPS];
+#pragma unroll
+    for (int t = 0; t < TAPS; ++t) off[t] = (int)((t / KS) * a.xs_h + (t % KS) * a.xs_w);
+    const float *wp = a.wpk + (size_t)grp * cpg * (KS * KS) * a.npg_pad + f0;
+    const int n_chunks = (cpg + CPC - 1) / CPC * ROWS;
+
+    // weights of chunk ch: row kk of the chunk is (channel c0 + kk / TAPS, tap kk % TAPS of the chunk's taps)
+    auto fetch_b = [&](int ch, int st) {
+        const int c0 = ch / ROWS * CPC, kh = ROWS > 1 ? ch % ROWS : 0;
+#pragma unroll
+        for (int v = 0; v < BV; ++v) {
+            const int i = tid + v * THREADS, kk = i / (BN / 4), q = i - kk * (BN / 4), c = c0 + kk / TAPS;
+            if (KC * BN / 4 % THREADS == 0 || i < KC * BN / 4) {
+                // npg_pad is a multiple of 32: four filters lie inside the packed row or beyond it together
+                const bool in = c < cpg && f0 + 4 * q < a.npg_pad;
+                cp_async16(&b_s[st][kk][4 * q], in ? wp + ((size_t)c * (KS * KS) + kh * KS + kk % TAPS) * a.npg_pad + 4 * q : a.wpk, in);
+            }
+        }
+    };
+    auto fetch_a = [&](int ch, int st) {      // VEC false
+        const int c0 = ch * CPC;
+#pragma unroll
+        for (int u = 0; u < NPX; ++u)
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const TX *p = xp[u] + (long long)(c0 + c) * a.xs_c;
+                const uint32_t m = c0 + csub + c < cpg ? in_mask[u] : 0u;
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t) {
+                    const bool in = (m >> t) & 1u;
+                    cp_async4(&a_s[st][(csub + c) * TAPS + t][tid % BM + u * THREADS], in ? p + off[t] : reinterpret_cast<const TX *>(a.x), in);
+                }
+            }
+    };
+    uint4 av[VEC ? NPX : 1][VEC ? TAPS * CPT / 4 : 1];          // VEC true: 4 channels of a pixel each (bf16: in the first two words)
+    auto load_a = [&](int ch) {
+        const int c0 = ch / ROWS * CPC, kh = ROWS > 1 ? ch % ROWS : 0;
+#pragma unroll
+        for (int u = 0; u < NPX; ++u) {
+            const TX *p = xp[u] + c0 + (long long)kh * a.xs_h;
+            const uint32_t m = in_mask[u] >> (kh * KS);
+#pragma unroll
+            for (int v = 0; v < CPT / 4; ++v)
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t) {
+                    // channels beyond the group's meet zero weights; 4-channel pieces never leave the pixel's pitch (a multiple of 8)
+                    const bool in = ((m >> t) & 1u) && c0 + csub + 4 * v < cpg;
+                    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+                    if (in) {
+                        if (sizeof(TX) == 4) r = __ldg(reinterpret_cast<const uint4 *>(p + off[t] + 4 * v));
+                        else { const uint2 h = __ldg(reinterpret_cast<const uint2 *>(p + off[t] + 4 * v)); r.x = h.x; r.y = h.y; }
+                    }
+                    av[u][v * TAPS + t] = r;
+                }
+        }
+    };
+    auto put_a = [&](int st) {
+#pragma unroll
+        for (int u = 0; u < NPX; ++u)
+#pragma unroll
+            for (int v = 0; v < CPT / 4; ++v)
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t) {
+                    const uint4 r = av[u][v * TAPS + t];
+                    float f[4];
+                    if (sizeof(TX) == 4) { f[0] = __uint_as_float(r.x); f[1] = __uint_as_float(r.y); f[2] = __uint_as_float(r.z); f[3] = __uint_as_float(r.w); }
+                    else { f[0] = __uint_as_float(r.x << 16); f[1] = __uint_as_float(r.x & 0xffff0000u); f[2] = __uint_as_float(r.y << 16); f[3] = __uint_as_float(r.y & 0xffff0000u); }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a_s[st][(csub + 4 * v + e) * TAPS + t][tid % BM + u * THREADS] = f[e];
+                }
+    };
+
+    // what this thread multiplies: pixel quads q * PSTEP + 4*tx, filter quads h * FSTEP + 4*ty
+    constexpr int PQ = TM / 4, FQ = TN / 4, PSTEP = BM / PQ, FSTEP = BN / FQ;
+    const int tx = BM / TM == 8 ? (lane & 7) : warp * 8 + (lane & 7), ty = BM / TM == 8 ? warp * 4 + (lane >> 3) : lane >> 3;
+    unsigned long long acc[TN][TM / 2];
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i) acc[j][i] = 0ull;
+    auto multiply = [&](int st) {
+#pragma unroll
+        for (int k = 0; k < KC; ++k) {
+            unsigned long long aa[TM / 2];
+            float bb[TN];
+#pragma unroll
+            for (int q = 0; q < PQ; ++q) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&a_s[st][k][q * PSTEP + 4 * tx]);
+                aa[2 * q] = v.x; aa[2 * q + 1] = v.y;
+            }
+#pragma unroll
+            for (int h = 0; h < FQ; ++h) {
+                const float4 v = *reinterpret_cast<const float4 *>(&b_s[st][k][h * FSTEP + 4 * ty]);
+                bb[4 * h] = v.x; bb[4 * h + 1] = v.y; bb[4 * h + 2] = v.z; bb[4 * h + 3] = v.w;
+            }
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const unsigned long long b2 = twice(bb[j]);
+#pragma unroll
+                for (int i = 0; i < TM / 2; ++i) ffma2(acc[j][i], aa[i], b2);
+            }
+        }
+    };
+    if (VEC) {
+        load_a(0);
+        fetch_b(0, 0);
+        cp_async_commit();
+        put_a(0);
+        cp_async_wait<0>();
+        __syncthreads();
+        for (int ch = 0; ch < n_chunks; ++ch) {
+            const bool more = ch + 1 < n_chunks;
+            if (more) { load_a(ch + 1); fetch_b(ch + 1, (ch + 1) & 1); }
+            cp_async_commit();
+            multiply(ch & 1);
+            if (more) put_a((ch + 1) & 1);
+            cp_async_wait<0>();
+            __syncthreads();
+        }
+    } else {
+        fetch_a(0, 0); fetch_b(0, 0); cp_async_commit();
+        if (n_chunks > 1) { fetch_a(1, 1); fetch_b(1, 1); }
+        cp_async_commit();
+        int st = 0, st2 = 2;
+        for (int ch = 0; ch < n_chunks; ++ch) {
+            cp_async_wait<1>();
+            __syncthreads();              // chunk ch has landed for everybody, and everybody is done with the buffer of chunk ch - 1
+            if (ch + 2 < n_chunks) { fetch_a(ch + 2, st2); fetch_b(ch + 2, st2); }
+            cp_async_commit();
+            multiply(st);
+            st = st == 2 ? 0 : st + 1;
+            st2 = st2 == 2 ? 0 : st2 + 1;
+        }
+        cp_async_wait<0>();
+    }
+
+    // folded batchnorm / bias, activation, stores straight from the registers, one filter quad at a time
+    const int n0 = grp * npg + f0;
+    const int nvalid = npg - f0;                            // filters of this block that exist, at least one
+    const int pad_end = min(a.y_cpitch, (g.n + 7) & ~7);
+    const bool last = grp == g.groups - 1 && f0 + BN >= npg;
+    const int cols = last ? min(BN, a.y_cpitch - n0) : min(BN, nvalid);   // the last block of the last group also writes the zero padding channels
+    if (a.y_nhwc && last && n0 + cols < pad_end)            // those that its columns do not reach
+        for (int i = tid; i < BM; i += THREADS)
+            for (int ch = n0 + cols; ch < pad_end; ++ch)
+                if (pix0 + i < npix) reinterpret_cast<TY *>(a.y_nhwc)[(size_t)(pix0 + i) * a.y_cpitch + ch] = from_float<TY>(0.f);
+    const bool whole_c = n0 % 4 == 0;                       // 4-channel pieces start aligned (the pitch is a multiple of 8)
+    const int plane = g.out_h * g.out_w;
+    const bool whole_p = plane % 4 == 0;                    // a pixel quad then lies in one plane, 16-byte aligned
+#pragma unroll
+    for (int h = 0; h < FQ; ++h) {
+        const int f = h * FSTEP + 4 * ty;
+        float sc[4], sh[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool real = f + e < nvalid;
+            sc[e] = real ? __ldg(a.ep.scale + n0 + f + e) : 0.f;
+            sh[e] = real ? __ldg(a.ep.shift + n0 + f + e) : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < PQ; ++q) {
+            float v[4][4];   // [pixel][filter]
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    const unsigned long long pair = acc[4 * h + e][2 * q + p / 2];
+                    float t = __uint_as_float((uint32_t)(p & 1 ? pair >> 32 : pair));
+                    t = activate_fast(t * sc[e] + sh[e], a.ep.activation);
+                    if (a.ep.round_tf32) t = round_tf32(t);
+                    v[p][e] = f + e < nvalid ? t : 0.f;
+                }
+            const long long pix = pix0 + q * PSTEP + 4 * tx;
+            if (a.y_nhwc) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    if (pix + p >= npix) continue;
+                    TY *row = reinterpret_cast<TY *>(a.y_nhwc) + (size_t)(pix + p) * a.y_cpitch + n0;
+                    if (whole_c && f + 4 <= cols) {
+                        if (sizeof(TY) == 4) {
+                            *reinterpret_cast<float4 *>(row + f) = make_float4(v[p][0], v[p][1], v[p][2], v[p][3]);
+                        } else {
+                            __nv_bfloat162 lo = __floats2bfloat162_rn(v[p][0], v[p][1]), hi = __floats2bfloat162_rn(v[p][2], v[p][3]);
+                            *reinterpret_cast<uint2 *>(row + f) = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (f + e < cols) row[f + e] = from_float<TY>(v[p][e]);
+                    }
+                }
+            }
+            if (a.y_nchw) {
+                if (whole_p) {
+                    if (pix < npix) {
+                        const int b = (int)(pix / plane), r = (int)(pix - (long long)b * plane);
+                        float *dst = a.y_nchw + ((size_t)b * g.n + n0 + f) * plane + r;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (f + e < nvalid) *reinterpret_cast<float4 *>(dst + (size_t)e * plane) = make_float4(v[0][e], v[1][e], v[2][e], v[3][e]);
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        if (pix + p >= npix) continue;
+                        const int b = (int)((pix + p) / plane), r = (int)(pix + p - (long long)b * plane);
+                        float *dst = a.y_nchw + ((size_t)b * g.n + n0 + f) * plane + r;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (f + e < nvalid) dst[(size_t)e * plane] = v[p][e];
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -269,14 +577,38 @@ conv_stem3x3_kernel(DirectArgs a)
     }
 }
 
+// Tile of the fp32 GEMM: 16 x 8 per thread where the filters fill 64 columns, 8 x 8 below that, and 32 x 32 tiles of
+// 4 x 4 threads where the larger ones would leave SMs empty (fewer than two blocks each): more, shorter blocks then.
+template <typename TX, typename TY, int KS, bool VEC>
+static int launch_gemm_tile(const DirectArgs &a, cudaStream_t s)
+{
+    const ConvGeom &g = a.g;
+    const long long npix = (long long)g.batch * g.out_h * g.out_w;
+    const int npg = g.n / g.groups;
+    int bm = 128, bn = npg > 32 ? 64 : 32;
+    auto blocks = [&](int m, int n) { return (npix + m - 1) / m * g.groups * ((npg + n - 1) / n); };
+    if (blocks(bm, bn) < 2LL * sm_count()) { bm = 32; bn = 32; }
+    dim3 grid((unsigned)((npix + bm - 1) / bm), (unsigned)(g.groups * ((npg + bn - 1) / bn)));
+    if (grid.y > 65535) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: too many filter blocks (%u)", grid.y);
+    if (bm == 32) conv_fp32_gemm_kernel<TX, TY, KS, 32, 32, 4, 4, VEC><<<grid, 64, 0, s>>>(a);
+    else if (bn == 64) conv_fp32_gemm_kernel<TX, TY, KS, 128, 64, 16, 8, VEC><<<grid, 64, 0, s>>>(a);
+    else conv_fp32_gemm_kernel<TX, TY, KS, 128, 32, 8, 8, VEC><<<grid, 64, 0, s>>>(a);
+    DNB_LAUNCH_CHECK("conv_fp32_gemm");
+    return DNB_OK;
+}
+
+template <typename TX, typename TY, bool VEC>
+static int launch_gemm(const DirectArgs &a, cudaStream_t s)
+{
+    return a.g.size == 3 ? launch_gemm_tile<TX, TY, 3, VEC>(a, s) : launch_gemm_tile<TX, TY, 1, VEC>(a, s);
+}
+
 int launch_conv_direct(const DirectArgs &a, cudaStream_t s)
 {
     const ConvGeom &g = a.g;
     if (g.size > 15) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: kernel size %d > 15", g.size);
     const long long npix = (long long)g.batch * g.out_h * g.out_w;
     const int npg = g.n / g.groups;
-    dim3 grid((unsigned)((npix + DTHREADS - 1) / DTHREADS), (unsigned)(g.groups * ((npg + FB - 1) / FB)));
-    if (grid.y > 65535) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: too many filter blocks (%u)", grid.y);
     const bool xb = a.x_dtype == DNB_BF16, yb = a.y_dtype == DNB_BF16;
     if (g.c == 3 && g.size == 3 && g.stride == 1 && g.pad == 1 && g.groups == 1 && !xb &&
         (!a.y_nhwc || (a.y_cpitch % 8 == 0))) {
@@ -288,10 +620,34 @@ int launch_conv_direct(const DirectArgs &a, cudaStream_t s)
         DNB_LAUNCH_CHECK("conv_stem3x3");
         return DNB_OK;
     }
-    if (!xb && !yb) conv_direct_kernel<float, float><<<grid, DTHREADS, 0, s>>>(a);
-    else if (!xb && yb) conv_direct_kernel<float, __nv_bfloat16><<<grid, DTHREADS, 0, s>>>(a);
-    else if (xb && !yb) conv_direct_kernel<__nv_bfloat16, float><<<grid, DTHREADS, 0, s>>>(a);
-    else conv_direct_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, DTHREADS, 0, s>>>(a);
+    // One input and one output type per plan mode: bf16 tensors belong to BF16 plans, which may also read or write f32.
+#define DIRECT_TYPES(GO)                                        \
+    do {                                                        \
+        if (!xb && !yb) GO(float, float);                       \
+        else if (!xb && yb) GO(float, __nv_bfloat16);           \
+        else if (xb && !yb) GO(__nv_bfloat16, float);           \
+        else GO(__nv_bfloat16, __nv_bfloat16);                  \
+    } while (0)
+    // The tiled kernel wants filters to fill its tile: below 17 per group a slab of the general kernel does less padded work.
+    if (npg > 16 && (g.size == 1 || g.size == 3) && a.xs_h < (1LL << 28) && a.xs_w < (1LL << 28)) {
+        const bool vec = a.xs_c == 1 && a.xs_w % 4 == 0 && (g.groups == 1 || (g.c / g.groups) % 4 == 0);
+        if (xb && vec) return yb ? launch_gemm<__nv_bfloat16, __nv_bfloat16, true>(a, s) : launch_gemm<__nv_bfloat16, float, true>(a, s);
+        if (!xb && vec) return yb ? launch_gemm<float, __nv_bfloat16, true>(a, s) : launch_gemm<float, float, true>(a, s);
+        if (!xb) return yb ? launch_gemm<float, __nv_bfloat16, false>(a, s) : launch_gemm<float, float, false>(a, s);
+    }
+    const int fb = npg <= 4 ? 4 : npg <= 8 ? 8 : npg <= 16 ? 16 : 32;
+    dim3 grid((unsigned)((npix + DTHREADS - 1) / DTHREADS), (unsigned)(g.groups * ((npg + fb - 1) / fb)));
+    if (grid.y > 65535) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: too many filter blocks (%u)", grid.y);
+#define SLAB_GO(TX, TY)                                                                       \
+    do {                                                                                      \
+        if (fb == 4) conv_direct_kernel<TX, TY, 4><<<grid, DTHREADS, 0, s>>>(a);              \
+        else if (fb == 8) conv_direct_kernel<TX, TY, 8><<<grid, DTHREADS, 0, s>>>(a);         \
+        else if (fb == 16) conv_direct_kernel<TX, TY, 16><<<grid, DTHREADS, 0, s>>>(a);       \
+        else conv_direct_kernel<TX, TY, 32><<<grid, DTHREADS, 0, s>>>(a);                     \
+    } while (0)
+    DIRECT_TYPES(SLAB_GO);
+#undef SLAB_GO
+#undef DIRECT_TYPES
     DNB_LAUNCH_CHECK("conv_direct");
     return DNB_OK;
 }
