@@ -129,7 +129,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
     TcShared *sh = reinterpret_cast<TcShared *>(s_shift + a.bn + 64);
     volatile int *abort_flag = &sh->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // uniform in the compiler's eyes
     const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;   // 0: the CTA that issues the pair's MMAs
     const bool leader = cta_rank == 0;
 
@@ -230,7 +230,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 }
             }
         } else
-        for (int tile = first_tile; lane == 0 && tile < total_tiles && ok; tile += grid_stride) {
+        for (int tile = first_tile; tile < total_tiles && ok; tile += grid_stride) {
             const int base = SPLIT ? tile / splits : tile, split = SPLIT ? tile - base * splits : 0;
             const int nt = base % n_tiles, pt = pixel_tile(base);
             const int ow0 = (pt % tiles_w) * wt;
@@ -238,36 +238,41 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             const int b0 = (pt / ptiles_wh) * bt;
             const int n0 = nt * bn + (PAIR ? (int)cta_rank * (bn >> 1) : 0);   // a pair's CTAs load one half of the filter tile each
             const int k0 = k_begin(split), k1 = SPLIT ? k_begin(split + 1) : k_iters;
-            int tap = k0 / c_blocks, cb = k0 - tap * c_blocks;
+            int ki = k0, tap = k0 / c_blocks, cb = k0 - tap * c_blocks;
             int kh = tap / ksize, kw = tap - kh * ksize;
-            for (int ki = k0; ki < k1; ++ki) {
+            // a tap at a time: what changes inside it is the channel block
+            while (ki < k1 && ok) {
                 // input row = oh*stride + kh - pad = stride*(oh + q) + parity
                 const int dh = kh - cpad, dw = kw - cpad;
                 int ph = 0, qh = dh, pw = 0, qw = dw;
                 if (cstride == 2) { ph = dh & 1; qh = (dh - ph) >> 1; pw = dw & 1; qw = (dw - pw) >> 1; }
                 const CUtensorMap *mx = maps + (ph * cstride + pw);
-                ok = mbar_wait_thread(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
-                if (!ok) break;
-                // wait-expiry test (debug bit 32): the last operand load of this CTA's first tile is never
-                // requested, so the MMA role's wait for it runs out and the CTA takes the abort path
-                if (withhold && tile == first_tile && ki == k1 - 1) { ok = false; break; }
-                const uint32_t bar = full0 + 8 * stage;
-                const uint32_t sa = ring + stage * stage_bytes;
-                if (PAIR) {
-                    // one barrier, in the even CTA, counts the bytes of both CTAs' loads of this slot
-                    if (leader) mbar_expect_tx(bar, 2u * tx_bytes);
-                    tma_load_4d_pair(sa, mx, bar, cb * bk, ow0 + qw, oh0 + qh, b0);
-                    tma_load_3d_pair(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
-                } else {
-                    mbar_expect_tx(bar, tx_bytes);
-                    tma_load_4d(sa, mx, bar, cb * bk, ow0 + qw, oh0 + qh, b0);
-                    tma_load_3d(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
+                const int iw0 = ow0 + qw, ih0 = oh0 + qh;
+                const int kend = min(k1, ki + c_blocks - cb);
+                for (; ki < kend; ++ki, ++cb) {
+                    ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
+                    if (!ok) break;
+                    // wait-expiry test (debug bit 32): the last operand load of this CTA's first tile is never
+                    // requested, so the MMA role's wait for it runs out and the CTA takes the abort path
+                    if (withhold && tile == first_tile && ki == k1 - 1) { ok = false; break; }
+                    const uint32_t bar = full0 + 8 * stage;
+                    const uint32_t sa = ring + stage * stage_bytes;
+                    if (elect_one()) {
+                        if (PAIR) {
+                            // one barrier, in the even CTA, counts the bytes of both CTAs' loads of this slot
+                            if (leader) mbar_expect_tx(bar, 2u * tx_bytes);
+                            tma_load_4d_pair(sa, mx, bar, cb * bk, iw0, ih0, b0);
+                            tma_load_3d_pair(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
+                        } else {
+                            mbar_expect_tx(bar, tx_bytes);
+                            tma_load_4d(sa, mx, bar, cb * bk, iw0, ih0, b0);
+                            tma_load_3d(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
+                        }
+                    }
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
-                if (++stage == stages) { stage = 0; phase ^= 1; }
-                if (++cb == c_blocks) {
-                    cb = 0; ++tap;
-                    if (++kw == ksize) { kw = 0; ++kh; }
-                }
+                cb = 0; ++tap;
+                if (++kw == ksize) { kw = 0; ++kh; }
             }
         }
         __syncwarp();
@@ -335,39 +340,42 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 if (ok) umma_commit(smem_u32(&sh->acc_full[acc]));
             }
         } else
-        for (int tile = first_tile; lane == 0 && leader && tile < total_tiles && ok; tile += grid_stride, ++it) {
+        if (leader)
+        for (int tile = first_tile; tile < total_tiles && ok; tile += grid_stride, ++it) {
             const int acc = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
-            ok = mbar_wait_thread(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1, abort_flag, status, WAIT_ACC_EMPTY, wait_limit);
+            ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1, abort_flag, status, WAIT_ACC_EMPTY, wait_limit);
             if (!ok) break;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + acc * acc_stride;
             const int split = SPLIT ? tile % splits : 0;
             const int kn = SPLIT ? k_begin(split + 1) - k_begin(split) : k_iters;   // this tile's share of the K loop
             for (int ki = 0; ki < kn; ++ki) {
-                ok = mbar_wait_thread(full0 + 8 * stage, phase, abort_flag, status, WAIT_FULL, wait_limit);
+                ok = mbar_wait_warp(full0 + 8 * stage, phase, abort_flag, status, WAIT_FULL, wait_limit);
                 if (!ok) break;
                 tc_fence_after();
-                if (dbg_mma & 16) {
-                } else if (PAIR) {   // the same descriptors address both CTAs' shared memory; row_bytes is 128 in pair mode
-                    umma_pair<is_bf16>(d_tmem, da, db, idesc, ki != 0);
-                    umma_pair<is_bf16>(d_tmem, da + 2, db + 2, idesc, 1u);
-                    umma_pair<is_bf16>(d_tmem, da + 4, db + 4, idesc, 1u);
-                    umma_pair<is_bf16>(d_tmem, da + 6, db + 6, idesc, 1u);
-                } else if (k_steps == 4) {
-                    umma<is_bf16>(d_tmem, da, db, idesc, ki != 0);
-                    umma<is_bf16>(d_tmem, da + 2, db + 2, idesc, 1u);
-                    umma<is_bf16>(d_tmem, da + 4, db + 4, idesc, 1u);
-                    umma<is_bf16>(d_tmem, da + 6, db + 6, idesc, 1u);
-                } else {
-                    for (int k = 0; k < k_steps; ++k) umma<is_bf16>(d_tmem, da + 2 * k, db + 2 * k, idesc, (ki | k) != 0);
+                if (elect_one()) {
+                    if (dbg_mma & 16) {
+                    } else if (PAIR) {   // the same descriptors address both CTAs' shared memory; row_bytes is 128 in pair mode
+                        umma_pair<is_bf16>(d_tmem, da, db, idesc, ki != 0);
+                        umma_pair<is_bf16>(d_tmem, da + 2, db + 2, idesc, 1u);
+                        umma_pair<is_bf16>(d_tmem, da + 4, db + 4, idesc, 1u);
+                        umma_pair<is_bf16>(d_tmem, da + 6, db + 6, idesc, 1u);
+                    } else if (k_steps == 4) {
+                        umma<is_bf16>(d_tmem, da, db, idesc, ki != 0);
+                        umma<is_bf16>(d_tmem, da + 2, db + 2, idesc, 1u);
+                        umma<is_bf16>(d_tmem, da + 4, db + 4, idesc, 1u);
+                        umma<is_bf16>(d_tmem, da + 6, db + 6, idesc, 1u);
+                    } else {
+                        for (int k = 0; k < k_steps; ++k) umma<is_bf16>(d_tmem, da + 2 * k, db + 2 * k, idesc, (ki | k) != 0);
+                    }
+                    // frees the slot (in both CTAs of a pair) when these MMAs retire
+                    if (PAIR) umma_commit_pair(empty0 + 8 * stage); else umma_commit(empty0 + 8 * stage);
                 }
-                // frees the slot (in both CTAs of a pair) when these MMAs retire
-                if (PAIR) umma_commit_pair(empty0 + 8 * stage); else umma_commit(empty0 + 8 * stage);
                 da += slot_step; db += slot_step;
                 if (++stage == stages) { stage = 0; phase ^= 1; da = da0; db = db0; }
             }
-            if (ok) {   // accumulator complete (in both CTAs of a pair) when all MMAs above retire
+            if (ok && elect_one()) {   // accumulator complete (in both CTAs of a pair) when all MMAs above retire
                 if (PAIR) umma_commit_pair(smem_u32(&sh->acc_full[acc])); else umma_commit(smem_u32(&sh->acc_full[acc]));
             }
         }

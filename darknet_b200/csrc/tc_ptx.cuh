@@ -71,6 +71,39 @@ __device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, 
     return true;
 }
 
+// Bounded wait for a loop that a whole warp runs in step (the TMA and MMA roles): every lane polls, the vote makes the
+// outcome, and with it the loop's control flow and all its counters, uniform in the compiler's eyes.  Such a loop keeps
+// its addresses, coordinates and descriptors in uniform registers, where the TMA and MMA instructions want them; with one
+// lane running the loop alone each of them was moved there operand by operand (an iteration of the MMA role then took
+// 680-860 clocks, of the TMA role 460-520, whatever the tensor pipe and the memory could do).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
+                                               long long limit = WAIT_LIMIT_CYCLES)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    int spins = 0;
+    while (!__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, 1000u))) {
+        if ((++spins & 0x3f) == 0) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            if (__any_sync(0xffffffffu, clock64() - t0 > limit)) {
+                if ((threadIdx.x & 31) == 0) {
+                    *abort_flag = 1;
+                    atomicCAS(status, 0, code);
+                }
+                return false;
+            }
+        }
+    }
+    return true;
+}
+// One lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
                                           unsigned backoff_ns = 0, long long limit = WAIT_LIMIT_CYCLES)
 {
