@@ -60,6 +60,8 @@ inline size_t tensor_elems(const dnb_tensor *t)
                                  : (size_t)t->n * t->c * t->h * t->w;
 }
 
+bool pdl_enabled();     // conv_tc.cu; DNB_PDL=0: plain launches
+
 // ---- kernels_mem.cu
 // signs: optional int8 channels-last tensor of pitch spitch that receives the output's signs (f32 channels-last tensors)
 int launch_maxpool(const dnb_tensor *x, const dnb_tensor *y, int size, int stride, int padding, cudaStream_t s, int8_t *signs = nullptr, int spitch = 0);

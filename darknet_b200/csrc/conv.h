@@ -85,13 +85,9 @@ struct alignas(64) TcArgs {
     int y_dtype, y_cpitch;
     float *y_nchw;
     int *status;          // device word: 0, or the code of the wait that expired
-    // split-K (layers with fewer tiles than SMs and a long K loop): total_tiles counts (output tile, K range) pairs
     int warp_stores;      // 1: every epilogue warp stores its own 32 rows (tmy_warp); 0: one store per chunk by one thread (tmy)
     void *sign_out;       // int8 kind: also write the output's signs here ([b][h][w][sign_cpitch] bytes), or null
     int sign_cpitch;
-    int splits;           // K ranges per output tile; 1 = off
-    void *split_scratch;  // [output tile][range][128 rows][bn] raw accumulators (f32, or int32 of the int8 kind)
-    int *split_counters;  // [output tile] ranges delivered so far; zero between launches
     ConvGeom g;
     ConvEpilogue ep;
 };
@@ -99,6 +95,36 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s);
 size_t conv_tc_smem_bytes(const TcArgs &a);
 size_t conv_tc_fixed_smem(int store_row_bytes, int bn, int stage_bufs);
 int conv_tc_max_smem();
+
+// ---- conv_tc_split.cu : the same convolution for launches that do not fill the GPU, one tile per cluster, K cut across it
+struct alignas(64) SplitArgs {
+    CUtensorMap tmx[4];   // as in TcArgs; boxes of wt x ht x bt pixels
+    CUtensorMap tmw;
+    int kind;             // 0 tf32, 1 bf16, 2 int8 signs
+    int pair;             // clusters of 2 * splits CTAs working in pairs; tiles then counts PAIRS of pixel tiles
+    int splits;           // K ranges = CTAs (pairs) per tile, 2..8
+    int tiles;            // output tiles = clusters
+    int row_bytes, bk, c_blocks, taps, bn, n_tiles;
+    int wt, ht, bt, rows; // a tile's pixels, rows = wt*ht*bt <= 128
+    int tiles_w, tiles_h;
+    int stages, a_bytes, b_bytes;
+    int work_bytes;       // ring or accumulator dump, whichever is larger
+    int tmem_cols;        // power of two >= bn
+    int n_write;          // channels written: n rounded to 8 for channels-last output, n for Darknet's layout alone
+    void *y_nhwc;
+    int y_cpitch;
+    float *y_nchw;
+    void *sign_out;
+    int sign_cpitch;
+    int *status;
+    int debug;
+    long long wait_limit;
+    ConvGeom g;
+    ConvEpilogue ep;
+};
+int launch_conv_tc_split(const SplitArgs &a, cudaStream_t s);
+size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes);
+int conv_tc_split_resident(int pair, int cluster);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
 int encode_tensor_map(CUtensorMap *map, int elem_kind /* 0 f32, 1 bf16, 2 bytes */, int rank, void *base, const uint64_t *dims,
@@ -170,18 +196,14 @@ struct dnb_conv_plan {
     bool signs_given;               // this plan's x_i8 is filled by the layer before it: no sign pass of its own
     const void *signs_of;           // ... as long as the input it is given is this tensor
     void *tc_sign_out;              // the sign output the cached launch block was built for
-    void *split_scratch;     // split-K partial sums and counters of the cached launch block (owned by the plan)
-    size_t split_scratch_bytes;
-    int *split_counters;
-    int split_counters_n;
+    bool keep_k_order;       // sum K in one order whatever the batch: no split (dense layers of a network with xnor layers)
+    bool tc_split;           // launches use the one-tile-per-cluster kernel and its block below
+    dnb::SplitArgs sp;
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout
     int device;
     long long wait_limit;    // bound of the kernels' waits in cycles (0: the default, about one second)
     int debug_bits;          // OR-ed into the launch block's debug field (dnb_conv_plan_set_diagnostics)
 };
-
-// zero the split-K counters a timed-out launch may have left part-way (on `s`; a null plan or one without counters: nothing)
-void conv_plan_reset_after_abort(dnb_conv_plan *p, cudaStream_t s = nullptr);
 
 // producers of a tensor-core xnor layer's int8 operand (see conv_plan.cu)
 int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int batch, int c, int h, int w);

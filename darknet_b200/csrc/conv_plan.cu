@@ -72,7 +72,6 @@ extern "C" void dnb_conv_plan_destroy(dnb_conv_plan *p)
     if (!p) return;
     cudaFree(p->scale); cudaFree(p->shift); cudaFree(p->w_tc); cudaFree(p->w_direct); cudaFree(p->w_bits);
     cudaFree(p->w_mean); cudaFree(p->x_nhwc_scratch); cudaFree(p->x_bits); cudaFree(p->w_i8); cudaFree(p->scale_i8); cudaFree(p->x_i8);
-    cudaFree(p->split_scratch); cudaFree(p->split_counters);
     if (!p->status_shared) cudaFree(p->status);
     delete p;
 }
@@ -88,9 +87,13 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
 {
     if (!p || !buf || len < 1) DNB_FAIL(DNB_EINVAL, "conv describe: bad argument");
     const TcArgs &a = p->tc;
-    if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
-        snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d splits=%d signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
-                 a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.splits, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
+    const bool tc = p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc);
+    if (tc && p->tc_x_ptr && p->tc_split)
+        snprintf(buf, len, "%s pair=%d halo=0 bn=%d tile=%dx%dx%d tiles=%d stages=%d splits=%d signs_in=%d signs_out=%d one_tile_per_cluster", kKernelNames[p->kernel], p->sp.pair,
+                 p->sp.bn, p->sp.wt, p->sp.ht, p->sp.bt, p->sp.tiles, p->sp.stages, p->sp.splits, p->signs_given ? 1 : 0, p->sp.sign_out ? 1 : 0);
+    else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
+        snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
+                 a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
     else
         snprintf(buf, len, "%s", dnb_conv_plan_kernel(p));
     return DNB_OK;
@@ -320,31 +323,173 @@ static void pick_pixel_tile(const ConvGeom &g, bool nchw_out, int *wt, int *ht, 
         }
 }
 
-static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
-                         const void *residual, int res_cpitch, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0)
+// ------------------------------------------------------------------ the kernel for launches that do not fill the GPU
+namespace {
+
+struct SplitPlan {
+    int pair = 0, bn = 0, splits = 0, stages = 0, wt = 0, ht = 0, bt = 0, ptiles = 0;
+    double cost = 1e300;   // microseconds, estimated
+};
+
+// The box of at most 128 pixels that covers the output with the fewest tiles; widest rows among equals.
+void split_pixel_tile(const ConvGeom &g, int *wt, int *ht, int *bt, int *ptiles)
 {
-    TcArgs &a = p->tc;
-    // A 1x1 convolution (stride 1, no padding) does not care which pixels are neighbours: with Darknet's layout among
-    // the outputs, the h x w plane is treated as one row of h*w pixels, so that a tile is a run of up to 128 contiguous
-    // pixels of every filter plane (and of the channels-last input) instead of a wt x ht patch.  DNB_TC_FLAT=0: never.
-    ConvGeom g = p->g;
-    {
-        const char *e = getenv("DNB_TC_FLAT");
-        if (nchw_out && g.size == 1 && g.stride == 1 && g.pad == 0 && !(e && atoi(e) == 0)) {
-            g.w = g.out_w = g.w * g.h;
-            g.h = g.out_h = 1;
+    long long best = 0;
+    for (int w = 1; w <= 128 && w <= g.out_w; ++w)
+        for (int h = 1; w * h <= 128 && h <= g.out_h; ++h) {
+            int b = 128 / (w * h);
+            if (b > g.batch) b = g.batch;
+            const long long n = (long long)((g.out_w + w - 1) / w) * ((g.out_h + h - 1) / h) * ((g.batch + b - 1) / b);
+            if (!best || n < best || (n == best && w > *wt)) { best = n; *wt = w; *ht = h; *bt = b; }
+        }
+    *ptiles = (int)best;
+}
+
+// Microseconds that one K iteration (128 pixels x bn filters x 128 bytes of channels) takes a CTA that has its SM to itself,
+// measured on B200: the larger of four MMAs (77 clocks each up to 128 filters, 128 for 256) and of the slot's trip from L2.
+double iter_us(int pair, int bn) { return pair ? 0.26 : bn <= 64 ? 0.15 : bn <= 128 ? 0.207 : 0.30; }
+
+struct SplitQuery {
+    int row_bytes, k_iters, n_pad, max_smem;
+    bool pair_ok, residual, long_sum;   // long_sum: 8192 products per output or more
+};
+
+// Cheapest tile of one launch at S ranges, in microseconds of a launch inside a chain of dependent ones (the sums were fitted
+// to a sweep over the 3x3 and 1x1 layers of YOLOv3 and ResNet-50 at 1 to 8 images; most choices come out within 15 % of what
+// they take): launch and first loads; K iterations; dump of the accumulator (4 ns a column); partial sums through distributed
+// shared memory (20 ns per KB); stores and residual, by the number of 16-byte pieces a thread finishes.
+SplitPlan split_of(const SplitQuery &q, const ConvGeom &g, int pair, int S)
+{
+    SplitPlan best;
+    int wt = 1, ht = 1, bt = 1, pt = 1;
+    split_pixel_tile(g, &wt, &ht, &bt, &pt);
+    const int sms = sm_count(), a_bytes = 128 * q.row_bytes, cluster = pair ? 2 * S : S;
+    const int resident = conv_tc_split_resident(pair, cluster);   // clusters live inside one GPC: SMs may be left over
+    for (int opt = 0; opt < 3 && resident > 0; ++opt) {
+        int bn = 64 << opt;
+        if (pair && bn != 256) continue;
+        if (!pair && bn > q.n_pad) {
+            if (opt > 0 && bn / 2 >= q.n_pad) continue;    // the narrower tile already holds every filter
+            bn = q.n_pad;
+        }
+        const int n_tiles = (q.n_pad + bn - 1) / bn;
+        const long long tiles = (long long)(pair ? (pt + 1) / 2 : pt) * n_tiles;
+        if (tiles > 4LL * sms) continue;
+        const int b_bytes = round_up((pair ? bn / 2 : bn) * q.row_bytes, 1024), per = (q.k_iters + S - 1) / S;
+        // the whole K range of a CTA in the ring if it fits: the deepest ring is what hides the loads' latency
+        int stages = (q.max_smem - 4096) / (a_bytes + b_bytes);
+        if (stages > 12) stages = 12;
+        if (stages > per) stages = per < 2 ? 2 : per;
+        if (stages < 2 || conv_tc_split_smem(stages, a_bytes + b_bytes, bn, nullptr) > (size_t)q.max_smem) continue;
+        const long long rounds = (tiles + resident - 1) / resident;
+        const double pieces = (128.0 / S) * (bn / 4) / 320.0, remote_kb = (double)(S - 1) / S * bn * 0.5;
+        const double finish = 0.004 * bn + 0.02 * remote_kb + pieces * (q.residual ? 0.32 : 0.22) + (pair ? 1.3 : 0.0);
+        const double cost = 4.5 + rounds * (per * iter_us(pair, bn) + finish) + (rounds - 1) * 4.0;
+        if (cost < best.cost) {
+            best.pair = pair; best.bn = bn; best.splits = S; best.stages = stages; best.wt = wt; best.ht = ht; best.bt = bt; best.ptiles = pt; best.cost = cost;
         }
     }
+    return best;
+}
+
+// The cheapest of all splits (only_s: of those into so many ranges).  One or two images get the same number of ranges, the
+// one that is best for one with an eye on two, so that an image's sums do not depend on whether another came with it.
+SplitPlan choose_split(const SplitQuery &q, const ConvGeom &g, int only_s, bool prefer_pair, int images)
+{
+    SplitPlan best[2];
+    double score[2] = {1e300, 1e300};
+    for (int S = only_s > 1 ? only_s : 2; S <= (only_s > 1 ? only_s : 8); ++S) {
+        if (S > q.k_iters || (only_s <= 1 && q.k_iters / S < 3)) break;
+        for (int pair = 0; pair < (q.pair_ok ? 2 : 1); ++pair) {
+            const SplitPlan sp = split_of(q, g, pair, S);
+            if (!sp.splits) continue;
+            double sc = sp.cost;
+            if (images == 1 && only_s <= 1) {
+                ConvGeom two = g;
+                if (two.batch == 1 && two.h == 1 && q.k_iters && g.size == 1) two.w = two.out_w = 2 * g.out_w;   // flattened pixels
+                else two.batch = 2;
+                const SplitPlan t = split_of(q, two, pair, S);
+                sc += t.splits ? 0.5 * t.cost : 1e6;
+            }
+            if (sc < score[pair]) { score[pair] = sc; best[pair] = sp; }
+        }
+    }
+    // near-ties go to pairs, and long sums sooner than short ones: fewer bytes through L2 for the same MMAs
+    const double tie = prefer_pair ? 1e9 : q.k_iters >= 144 && q.long_sum ? 1.5 : 1.05;
+    return best[1].splits && score[1] < tie * score[0] ? best[1] : best[0];
+}
+
+}  // namespace
+
+static int ensure_status(dnb_conv_plan *p)
+{
+    if (p->status) return DNB_OK;
+    DNB_CUDA(cudaMalloc((void **)&p->status, sizeof(int)));
+    DNB_CUDA(cudaMemset(p->status, 0, sizeof(int)));
+    return DNB_OK;
+}
+
+// Input maps of a convolution: lattice (ph, pw) of the input holds rows ph, ph+stride, ... and columns pw, pw+stride, ...
+static int encode_input_maps(CUtensorMap *maps, const ConvGeom &g, const dnb_tensor *x, int kind, int es, int c_pad, const uint32_t *box, int row_bytes)
+{
+    const size_t pix_bytes = (size_t)x->cpitch * es;
+    const int s = g.stride;
+    if (s > 2) DNB_FAIL(DNB_EUNSUPPORTED, "conv: stride %d on the tensor-core path (1 and 2 are covered)", s);
+    for (int ph = 0; ph < s; ++ph)
+        for (int pw = 0; pw < s; ++pw) {
+            const int hl = (g.h - ph + s - 1) / s, wl = (g.w - pw + s - 1) / s;
+            uint64_t dims[4] = {(uint64_t)c_pad, (uint64_t)(wl > 0 ? wl : 1), (uint64_t)(hl > 0 ? hl : 1), (uint64_t)g.batch};
+            uint64_t strides[3] = {pix_bytes * s, pix_bytes * g.w * s, pix_bytes * g.w * g.h};
+            char *base = (char *)x->data + ((size_t)ph * g.w + pw) * pix_bytes;
+            if (hl <= 0 || wl <= 0) base = (char *)x->data;  // lattice empty: never addressed in-bounds
+            DNB_TRY(encode_tensor_map(&maps[ph * s + pw], kind, 4, base, dims, strides, box, row_bytes));
+        }
+    return DNB_OK;
+}
+
+static int encode_weight_map(CUtensorMap *map, const dnb_conv_plan *p, int kind, int es, int c_pad, int taps, int bk, int rows, int row_bytes)
+{
+    uint64_t dims[3] = {(uint64_t)c_pad, (uint64_t)p->n_pad, (uint64_t)taps};
+    uint64_t strides[2] = {(uint64_t)c_pad * es, (uint64_t)c_pad * es * p->n_pad};
+    uint32_t box[3] = {(uint32_t)bk, (uint32_t)rows, 1u};
+    return encode_tensor_map(map, kind, 3, kind == 2 ? (void *)p->w_i8 : p->w_tc, dims, strides, box, row_bytes);
+}
+
+static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeom &g, const SplitPlan &sp, int kind, int es,
+                            void *y_nhwc, int y_cpitch, void *sign_out, int sign_cpitch)
+{
+    const TcArgs &t = p->tc;
+    SplitArgs &a = p->sp;
+    const int c_pad = kind == 2 ? p->c_pad_i8 : p->c_pad;
+    a.kind = kind; a.pair = sp.pair; a.splits = sp.splits; a.bn = sp.bn; a.stages = sp.stages;
+    a.row_bytes = t.row_bytes; a.bk = t.bk; a.c_blocks = t.c_blocks; a.taps = t.taps;
+    a.wt = sp.wt; a.ht = sp.ht; a.bt = sp.bt; a.rows = sp.wt * sp.ht * sp.bt;
+    a.tiles_w = (g.out_w + a.wt - 1) / a.wt;
+    a.tiles_h = (g.out_h + a.ht - 1) / a.ht;
+    a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
+    a.tiles = (a.pair ? (sp.ptiles + 1) / 2 : sp.ptiles) * a.n_tiles;
+    a.a_bytes = 128 * a.row_bytes;
+    a.b_bytes = round_up((a.pair ? a.bn / 2 : a.bn) * a.row_bytes, 1024);
+    conv_tc_split_smem(a.stages, a.a_bytes + a.b_bytes, a.bn, &a.work_bytes);
+    a.tmem_cols = 32;
+    while (a.tmem_cols < a.bn) a.tmem_cols *= 2;
+    const int n8 = round_up(g.n, 8);
+    a.n_write = y_nhwc ? (n8 < y_cpitch ? n8 : y_cpitch) : g.n;
+    a.sign_out = sign_out; a.sign_cpitch = sign_cpitch;
+    a.debug = t.debug; a.wait_limit = t.wait_limit;
+    a.g = g;
+    DNB_TRY(ensure_status(p));
+    const uint32_t box[4] = {(uint32_t)a.bk, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
+    DNB_TRY(encode_input_maps(a.tmx, g, x, kind, es, c_pad, box, a.row_bytes));
+    DNB_TRY(encode_weight_map(&a.tmw, p, kind, es, c_pad, a.taps, a.bk, a.pair ? a.bn / 2 : a.bn, a.row_bytes));
+    p->tc_split = true;
+    return DNB_OK;
+}
+
+// Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
+static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch)
+{
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
-    const int es = i8 ? 1 : (bf16 ? 2 : 4);
-    const int kind = i8 ? 2 : (bf16 ? 1 : 0);              // element kind of the operands (and of their tensor maps)
-    const int c_pad = i8 ? p->c_pad_i8 : p->c_pad;         // channel pitch of the operand tensors
-    a.is_bf16 = kind;
-    const int cbytes = c_pad * es;
-    a.row_bytes = cbytes >= 128 ? 128 : (cbytes >= 64 ? 64 : 32);
-    a.bk = a.row_bytes / es;
-    a.c_blocks = (c_pad + a.bk - 1) / a.bk;
-    a.taps = g.size * g.size;
     pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt);
     // Halo mode (experimental, off unless DNB_TC_HALO is 1 or 2): one activation box per channel block serves all
     // nine taps of a 3x3 stride-1 layer, which cuts the bytes that cross L2 -> shared memory by 2.3x on the
@@ -411,10 +556,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         // single CTAs per SM with two or three slots each starve on load latency, which outweighs the idle SMs.
         const int pair_tiles = (ptiles + 1) / 2 * (g.n / 256), clusters = sm_count() / 2;
         const int k_iters_p = g.size * g.size * a.c_blocks;
-        // (with split-K, below, a sixteenth of them is enough: every pair tile becomes up to eight)
-        const bool split_ok = !(getenv("DNB_TC_SPLITK") && atoi(getenv("DNB_TC_SPLITK")) == 0) && !i8;
-        const bool enough = pair_tiles >= clusters || (k_iters_p >= 64 && (2 * pair_tiles >= clusters || (split_ok && 16 * pair_tiles >= clusters)));
-        const bool legal = !a.halo && a.row_bytes == 128 && g.n % 256 == 0 && enough && y_nhwc && y_cpitch * (bf16 ? 2 : 4) >= 128;
+        const bool enough = pair_tiles >= clusters || (k_iters_p >= 64 && 2 * pair_tiles >= clusters);
+        const bool legal = !a.halo && a.row_bytes == 128 && g.n % 256 == 0 && enough && channels_last && y_cpitch * (bf16 ? 2 : 4) >= 128;
         if (legal && (knob == 2 || (knob == 1 && (g.size >= 3 || k_iters_p >= 16)))) {
             a.pair = 1;
             a.bn = 256;
@@ -422,6 +565,45 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         }
     }
     a.total_tiles = a.pair ? (ptiles + 1) / 2 * a.n_tiles : ptiles * a.n_tiles;
+}
+
+// Microseconds of the persistent kernel by the measure of split_of: an epilogue hides behind the next tile's K loop, or the
+// other way round, and the last one is exposed; 64-filter tiles alone on an SM wait for their MMAs' results longer.
+static double persistent_us(const TcArgs &a, int k_iters, bool residual)
+{
+    const long long slots = a.pair ? sm_count() / 2 : sm_count();
+    const double share = (double)((a.total_tiles + slots - 1) / slots);
+    const double loop = k_iters * (!a.pair && a.bn <= 64 && share < 2.0 ? 0.18 : a.pair ? 0.31 : iter_us(a.pair, a.bn));
+    const double epilogue = a.bn * (residual ? 0.02 : 0.015);
+    return 3.6 + share * (loop > epilogue ? loop : epilogue) + epilogue;
+}
+
+static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
+                         const void *residual, int res_cpitch, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0)
+{
+    TcArgs &a = p->tc;
+    // A 1x1 convolution (stride 1, no padding) does not care which pixels are neighbours: with Darknet's layout among
+    // the outputs, the h x w plane is treated as one row of h*w pixels, so that a tile is a run of up to 128 contiguous
+    // pixels of every filter plane (and of the channels-last input) instead of a wt x ht patch.  DNB_TC_FLAT=0: never.
+    ConvGeom g = p->g;
+    {
+        const char *e = getenv("DNB_TC_FLAT");
+        if (nchw_out && g.size == 1 && g.stride == 1 && g.pad == 0 && !(e && atoi(e) == 0)) {
+            g.w = g.out_w = g.w * g.h;
+            g.h = g.out_h = 1;
+        }
+    }
+    const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
+    const int es = i8 ? 1 : (bf16 ? 2 : 4);
+    const int kind = i8 ? 2 : (bf16 ? 1 : 0);              // element kind of the operands (and of their tensor maps)
+    const int c_pad = i8 ? p->c_pad_i8 : p->c_pad;         // channel pitch of the operand tensors
+    a.is_bf16 = kind;
+    const int cbytes = c_pad * es;
+    a.row_bytes = cbytes >= 128 ? 128 : (cbytes >= 64 ? 64 : 32);
+    a.bk = a.row_bytes / es;
+    a.c_blocks = (c_pad + a.bk - 1) / a.bk;
+    a.taps = g.size * g.size;
+    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch);
     a.n_pad = p->n_pad;
     a.n_tot = a.n_tiles * a.bn;
     a.a_bytes = 128 * a.row_bytes;
@@ -481,7 +663,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         stages = 2;
     }
     if (!a.halo) {
-        if (allow2 && a.tmem_cols <= 256 && !a.pair) {
+        // (not when every tile has an SM of its own: one deep ring then)
+        if (allow2 && a.tmem_cols <= 256 && !a.pair && a.total_tiles > sm_count()) {
             const int max2 = getenv("DNB_TC_MAX2") ? atoi(getenv("DNB_TC_MAX2")) : 4;   // ring slots per CTA when two share the SM
             const long budget = (228L * 1024) / 2 - 2048;   // per CTA when two share the SM (1 KB each is reserved by the system)
             for (int srb2 = srb; srb2 >= min_srb; srb2 /= 2) {   // narrower staged rows if that is what makes two CTAs fit
@@ -511,92 +694,66 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     if (stages < 2) DNB_FAIL(DNB_ECUDA, "conv: %d bytes of shared memory are too few for the operand ring", max_smem);
     a.stages = stages;
     a.store_row_bytes = srb;
-    // Split-K: a layer with fewer tiles than the GPU has room for and a long K loop (the 19x19 and 38x38 layers at
-    // small batches) cuts every tile's K loop into `splits` ranges that run as separate tiles; see the kernel.
-    // The cost model counts waves of tiles, in units of one K-loop iteration (about 0.3 us): a tile cut into S ranges
-    // costs K/S iterations plus the partial sums' trip through L2: one dump (about 10 units) and, in the CTA that
-    // finishes the tile, S dependent rounds of loads per staged chunk (about 16 units per range; measured on the 19x19
-    // layers of YOLOv3 at one image: 61 us unsplit, 46 us with eight ranges).  Only long K loops on a mostly empty GPU
-    // qualify: batches of one or two images.
-    // DNB_TC_SPLITK: 0 never, N > 1 forces N ranges wherever the variant exists (tests).
     {   // DNB_TC_WARP_STORES=1 (experiment, off): every epilogue warp stores its own 32 rows and the four warps meet once
         // per tile instead of twice per chunk.  Measured on YOLOv3-608 b64: the layers' event times drop by 0.5 %, the
         // step replayed as one CUDA graph takes 2 % longer (18.5 -> 18.9 ms), batch 8 and ResNet-50 do not move.
         const char *e = getenv("DNB_TC_WARP_STORES");
         a.warp_stores = e ? (atoi(e) != 0) : 0;
     }
-    a.splits = 1;
-    a.split_scratch = nullptr;
-    a.split_counters = nullptr;
+    // A launch that leaves SMs idle, or whose few tiles have a long K loop: one tile per cluster, K cut across it
+    // (conv_tc_split.cu).  Chosen where its estimate is below the persistent kernel's, which overlaps a tile's epilogue with the
+    // next one's MMAs and therefore wins once every SM has a few tiles.  DNB_TC_SPLITK: 0 never, N forces N ranges (tests).
+    p->tc_split = false;
     {
-        const char *e = getenv("DNB_TC_SPLITK");
-        const int knob = e ? atoi(e) : -1;
-        const int k_iters = g.size * g.size * a.c_blocks, cpc = srb / out_es;
-        const bool legal = knob != 0 && !a.halo && !i8 && srb == 128 && a.bn % cpc == 0 && (!residual || a.pair) && k_iters >= 4;
-        if (legal) {
-            const int slots = a.pair ? sm_count() / 2 : sm_count() * a.ctas_per_sm;
-            const int T = a.total_tiles;
-            int best_s = 1;
-            double best = (double)((T + slots - 1) / slots);
-            best *= k_iters;
-            const double alone_units = best;
-            for (int S = 2; S <= 8 && k_iters / S >= 8; ++S) {
-                const double cost = (double)(((long long)T * S + slots - 1) / slots) * ((double)k_iters / S + 10.0 + 16.0 * S);
-                if (cost < best) { best = cost; best_s = S; }
+        const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
+        const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1;
+        const int k_iters = g.size * g.size * a.c_blocks;
+        if (knob != 0 && !a.halo && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2)) {
+            // pixels of a 1x1 layer in one row: of the whole batch where nothing is stored per image
+            auto flat = [&](ConvGeom sg) {
+                if (sg.size == 1 && sg.stride == 1 && sg.pad == 0) {
+                    sg.w = sg.out_w = sg.w * sg.h * (nchw_out ? 1 : sg.batch);
+                    sg.h = sg.out_h = 1;
+                    if (!nchw_out) sg.batch = 1;
+                }
+                return sg;
+            };
+            SplitQuery q;
+            q.row_bytes = a.row_bytes; q.k_iters = k_iters; q.n_pad = p->n_pad; q.max_smem = max_smem;
+            q.pair_ok = pair_knob > 0 && a.row_bytes == 128 && g.n % 256 == 0 && k_iters >= 16;
+            q.residual = residual != nullptr;
+            q.long_sum = g.c * g.size * g.size >= 8192;
+            SplitPlan sp;
+            if (knob > 1) {
+                sp = choose_split(q, flat(g), knob < 8 ? knob : 8, true, g.batch);
+            } else {
+                // decided at one image for two images also (see choose_split)
+                ConvGeom dg = g;
+                TcArgs da = a;
+                if (g.batch == 2) {
+                    dg.batch = 1;
+                    pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch);
+                }
+                sp = choose_split(q, flat(dg), 0, false, dg.batch);
+                if (!(sp.cost < persistent_us(da, k_iters, q.residual))) sp = SplitPlan();
+                else if (g.batch == 2) sp = choose_split(q, flat(g), sp.splits, false, 2);
             }
-            if (best > 0.85 * alone_units) best_s = 1;   // not worth the extra traffic
-            if (knob > 1) best_s = knob < k_iters / 2 ? knob : k_iters / 2;
-            if (best_s > 8) best_s = 8;
-            a.splits = best_s > 1 ? best_s : 1;
+            if (sp.splits) DNB_TRY(build_split_args(p, x, flat(g), sp, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));
         }
-        if (a.splits > 1) {
-            const int out_tiles = (a.pair ? (ptiles + 1) / 2 * 2 : ptiles) * a.n_tiles;
-            const size_t need = (size_t)out_tiles * a.splits * 128 * a.bn * sizeof(float);
-            if (need > p->split_scratch_bytes) {
-                cudaFree(p->split_scratch);
-                p->split_scratch = nullptr; p->split_scratch_bytes = 0;
-                DNB_CUDA(cudaMalloc(&p->split_scratch, need));
-                p->split_scratch_bytes = need;
-            }
-            if (out_tiles > p->split_counters_n) {
-                cudaFree(p->split_counters);
-                p->split_counters = nullptr; p->split_counters_n = 0;
-                DNB_CUDA(cudaMalloc((void **)&p->split_counters, (size_t)out_tiles * sizeof(int)));
-                DNB_CUDA(cudaMemset(p->split_counters, 0, (size_t)out_tiles * sizeof(int)));
-                p->split_counters_n = out_tiles;
-            }
-            a.split_scratch = p->split_scratch;
-            a.split_counters = p->split_counters;
-            a.total_tiles *= a.splits;
-        }
+    }
+    if (p->tc_split) {
+        p->tc_sign_out = sign_out;
+        p->tc_x_ptr = x->data; p->tc_x_cpitch = x->cpitch; p->tc_y_ptr = y_nhwc; p->tc_y_cpitch = y_cpitch; p->tc_y_dtype = y_dtype;
+        p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_nchw_out = nchw_out ? 1 : 0;
+        return DNB_OK;
     }
     a.g = g;
-    if (!p->status) {
-        DNB_CUDA(cudaMalloc((void **)&p->status, sizeof(int)));
-        DNB_CUDA(cudaMemset(p->status, 0, sizeof(int)));
-    }
+    DNB_TRY(ensure_status(p));
     a.status = p->status;
-
-    // activation maps: lattice (ph, pw) of the input holds rows ph, ph+stride, ... and columns pw, pw+stride, ...
-    const size_t pix_bytes = (size_t)x->cpitch * es;
-    const int s = g.stride;
-    if (s > 2) DNB_FAIL(DNB_EUNSUPPORTED, "conv: stride %d on the tensor-core path (1 and 2 are covered)", s);
-    for (int ph = 0; ph < s; ++ph)
-        for (int pw = 0; pw < s; ++pw) {
-            const int hl = (g.h - ph + s - 1) / s, wl = (g.w - pw + s - 1) / s;
-            uint64_t dims[4] = {(uint64_t)c_pad, (uint64_t)(wl > 0 ? wl : 1), (uint64_t)(hl > 0 ? hl : 1), (uint64_t)g.batch};
-            uint64_t strides[3] = {pix_bytes * s, pix_bytes * g.w * s, pix_bytes * g.w * g.h};
-            uint32_t box[4] = {(uint32_t)a.bk, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
-            if (a.halo) { box[1] = (uint32_t)(a.wt + 2); box[2] = (uint32_t)(a.ht + 2); }
-            char *base = (char *)x->data + ((size_t)ph * g.w + pw) * pix_bytes;
-            if (hl <= 0 || wl <= 0) base = (char *)x->data;  // lattice empty: never addressed in-bounds
-            DNB_TRY(encode_tensor_map(&a.tmx[ph * s + pw], kind, 4, base, dims, strides, box, a.row_bytes));
-        }
     {
-        uint64_t dims[3] = {(uint64_t)c_pad, (uint64_t)p->n_pad, (uint64_t)a.taps};
-        uint64_t strides[2] = {(uint64_t)c_pad * es, (uint64_t)c_pad * es * p->n_pad};
-        uint32_t box[3] = {(uint32_t)a.bk, (uint32_t)(a.pair ? a.bn / 2 : a.bn), 1u};
-        DNB_TRY(encode_tensor_map(&a.tmw, kind, 3, i8 ? (void *)p->w_i8 : p->w_tc, dims, strides, box, a.row_bytes));
+        const uint32_t box[4] = {(uint32_t)a.bk, (uint32_t)(a.halo ? a.wt + 2 : a.wt), (uint32_t)(a.halo ? a.ht + 2 : a.ht), (uint32_t)a.bt};
+        DNB_TRY(encode_input_maps(a.tmx, g, x, kind, es, c_pad, box, a.row_bytes));
+        DNB_TRY(encode_weight_map(&a.tmw, p, kind, es, c_pad, a.taps, a.bk, a.pair ? a.bn / 2 : a.bn, a.row_bytes));
     }
     if (y_nhwc) {
         const size_t opix = (size_t)y_cpitch * out_es;
@@ -740,10 +897,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         else { a.xs_w = 1; a.xs_h = g.w; a.xs_c = (long long)g.h * g.w; a.xs_b = (long long)g.c * a.xs_c; }
         a.w = p->w_direct; a.npg_pad = p->npg_pad;
         a.y = y_nhwc; a.y_dtype = y_dtype; a.y_cpitch = y_cpitch;
-        if (!p->status) {
-            DNB_CUDA(cudaMalloc((void **)&p->status, sizeof(int)));
-            DNB_CUDA(cudaMemset(p->status, 0, sizeof(int)));
-        }
+        DNB_TRY(ensure_status(p));
         a.status = p->status;
         a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
         a.g = g; a.ep = ep;
@@ -784,6 +938,15 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         if (p->tc_x_ptr != xin.data || p->tc_y_ptr != nhwc || p->tc_y_cpitch != (nhwc ? y_cpitch : 0) || !p->status || p->tc_nchw_out != (nchw ? 1 : 0) ||
             p->tc_sign_out != sign_out)
             DNB_TRY(build_tc_args(p, &xin, nhwc, DNB_F32, nhwc ? y_cpitch : 0, nullptr, 0, nchw != nullptr, sign_out, sign_out ? next->c_pad_i8 : 0));
+        if (p->tc_split) {
+            SplitArgs &a = p->sp;
+            a.y_nhwc = nhwc; a.y_cpitch = nhwc ? y_cpitch : 0; a.y_nchw = nchw;
+            a.ep = ep;
+            a.ep.scale = p->scale_i8; a.ep.round_tf32 = 0; a.ep.raw_acc = acc_out ? 1 : 0;
+            if (acc_out) a.ep.activation = DNB_LINEAR;
+            a.status = p->status;
+            return launch_conv_tc_split(a, s);
+        }
         TcArgs &a = p->tc;
         a.y_nhwc = nhwc; a.y_dtype = DNB_F32; a.y_cpitch = nhwc ? y_cpitch : 0; a.y_nchw = nchw;
         ep.scale = p->scale_i8;
@@ -832,6 +995,13 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         p->tc_y_dtype != y_dtype || !p->status || p->tc_res_ptr != ep.residual || p->tc_res_cpitch != ep.res_cpitch ||
         p->tc_nchw_out != (y_nchw ? 1 : 0))
         DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, ep.residual, ep.res_cpitch, y_nchw != nullptr));
+    if (p->tc_split) {
+        SplitArgs &a = p->sp;
+        a.y_nhwc = y_nhwc; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
+        a.ep = ep;
+        a.status = p->status;
+        return launch_conv_tc_split(a, s);
+    }
     TcArgs &a = p->tc;
     a.y_nhwc = y_nhwc; a.y_dtype = y_dtype; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
     a.ep = ep;
@@ -892,12 +1062,6 @@ extern "C" int dnb_conv_xnor_accumulate(dnb_conv_plan *p, const dnb_tensor *x, i
     return conv_forward_impl(p, x, nullptr, nullptr, acc, (cudaStream_t)stream);
 }
 
-// A launch that gave up on a wait may have left split-K counters part-way: zero them before the plan runs again.
-void conv_plan_reset_after_abort(dnb_conv_plan *p, cudaStream_t s)
-{
-    if (p && p->split_counters) cudaMemsetAsync(p->split_counters, 0, (size_t)p->split_counters_n * sizeof(int), s);
-}
-
 // Device status word of the tensor-core kernel: 0, or the code of the bounded
 // wait that expired (DNB_ETIMEOUT is returned to the caller in that case).
 extern "C" int dnb_conv_plan_check_status(dnb_conv_plan *p)
@@ -907,7 +1071,6 @@ extern "C" int dnb_conv_plan_check_status(dnb_conv_plan *p)
     DNB_CUDA(cudaMemcpy(&v, p->status, sizeof(int), cudaMemcpyDeviceToHost));
     if (v) {
         cudaMemset(p->status, 0, sizeof(int));
-        conv_plan_reset_after_abort(p);
         DNB_FAIL(DNB_ETIMEOUT, "conv: a device-side wait expired (code %d: 101 ring slot free, 102 operands landed, 103 accumulator free, 104 accumulator ready, 105 residual tile, 106 shared memory window not 1024-byte aligned)", v);
     }
     return DNB_OK;

@@ -417,6 +417,11 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
             if (A.sign_out) { A.sign_pitch = A.out_c; B.launches = 1; }
         }
     }
+    // A sign hangs on a sum's last bit.  Where layers are binarised, the dense ones add in the same order at every batch
+    // size (integer sums do not care), so that an image's results do not depend on how many came with it.
+    bool any_xnor = false;
+    for (const Layer &L : net->layers) any_xnor = any_xnor || (L.kind == L_CONV && L.cd.xnor);
+    for (Layer &L : net->layers) if (L.plan) L.plan->keep_k_order = any_xnor;
     const Layer &last = net->layers.back();
     net->outputs = last.out_c * last.out_h * last.out_w;
     DNB_CUDA(cudaMalloc((void **)&net->input_dev, (size_t)net->batch * net->inputs * sizeof(float)));
@@ -866,7 +871,6 @@ extern "C" int dnb_network_collect(dnb_network *net, float **output)
         const int code = net->status_host[slot];
         net->status_host[slot] = 0;
         cudaMemsetAsync(net->status_dev + slot, 0, sizeof(int), net->stream);   // before the slot's next step, which follows on this stream
-        for (Layer &L : net->layers) conv_plan_reset_after_abort(L.plan, net->stream);
         char text[512];
         snprintf(text, sizeof(text), kTimeoutText, code);
         DNB_FAIL(DNB_ETIMEOUT, "network_predict: %s", text);
@@ -976,7 +980,6 @@ extern "C" int dnb_network_check_status(dnb_network *net)
     DNB_CUDA(cudaMemcpy(v, net->status_dev, sizeof(v), cudaMemcpyDeviceToHost));
     if (v[0] || v[1]) {
         DNB_CUDA(cudaMemset(net->status_dev, 0, sizeof(v)));
-        for (Layer &L : net->layers) conv_plan_reset_after_abort(L.plan);
         char text[512];
         snprintf(text, sizeof(text), kTimeoutText, v[0] ? v[0] : v[1]);
         DNB_FAIL(DNB_ETIMEOUT, "network_forward: %s", text);

@@ -42,3 +42,46 @@ def test_grouped_layers_with_bf16_storage(name):
     case["x"] = bf16_round(case["x"])
     _, got, _ = run_conv(case, dn.MODE_BF16, "nhwc", "nhwc")
     parity(got, oracle_conv(case), 2 ** -8)
+
+
+SPLIT_TILES = {   # (case, K ranges): one tile per cluster, the K loop cut across it
+    "ranges_longer_than_the_ring": (dict(b=1, c=512, h=9, w=13, n=40, size=3), "2"),
+    "uneven_ranges": (dict(b=1, c=48, h=11, w=7, n=33, size=3), "5"),
+    "fewer_rows_than_ranges": (dict(b=1, c=1024, h=1, w=5, n=100, size=1), "8"),
+    "one_filter_over_a_tile": (dict(b=2, c=64, h=10, w=12, n=257, size=3, act="linear"), "3"),
+    "flat_batch_ragged": (dict(b=3, c=256, h=7, w=11, n=72, size=1, act="logistic"), "4"),
+    "stride2_odd_map": (dict(b=2, c=40, h=21, w=17, n=24, size=3, stride=2), "6"),
+    "narrow_rows": (dict(b=2, c=16, h=12, w=10, n=20, size=3), "2"),
+    "pairs_odd_pixel_tiles": (dict(b=1, c=128, h=17, w=19, n=512, size=3), "7"),
+}
+
+
+@pytest.mark.parametrize("name", list(SPLIT_TILES))
+@pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
+def test_one_tile_per_cluster(name, mode, tol, monkeypatch):
+    """Tolerances are the tensor-core kernel's (the products' 10 or 7 mantissa bits); the two layouts of one launch are bit-equal."""
+    shape, ranges = SPLIT_TILES[name]
+    monkeypatch.setenv("DNB_TC_SPLITK", ranges)
+    case = conv_case(710, **shape)
+    want = oracle_conv(case)
+    plan, got, _ = run_conv(case, mode, "nhwc", "nhwc")
+    assert f"splits={ranges}" in plan.describe() and "one_tile_per_cluster" in plan.describe(), plan.describe()
+    parity(got, want, tol)
+    _, nchw, nhwc = run_conv(case, mode, "nchw", "nchw", both=True)
+    assert (nchw == nhwc).all()
+    parity(nchw, want, tol)
+    _, alone, _ = run_conv(case, mode, "nchw", "nchw")
+    parity(alone, want, tol)
+
+
+@pytest.mark.parametrize("shape", [dict(b=1, c=96, h=9, w=7, n=64, size=3), dict(b=2, c=256, h=7, w=7, n=40, size=1)])
+@pytest.mark.parametrize("ranges", ["2", "6"])
+def test_one_tile_per_cluster_integer_sums(shape, ranges, monkeypatch):
+    """The int8 kind: the ranges' integer sums are exact, so they equal the uncut kernel's whatever the cut."""
+    import numpy as np
+    case = conv_case(711, **shape)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    _, whole, _ = run_conv(case, dn.MODE_TF32, "nhwc", "nhwc", xnor=True)
+    monkeypatch.setenv("DNB_TC_SPLITK", ranges)
+    _, got, _ = run_conv(case, dn.MODE_TF32, "nhwc", "nhwc", xnor=True)
+    assert np.array_equal(got, whole)
