@@ -62,6 +62,25 @@ inline size_t tensor_elems(const dnb_tensor *t)
 
 bool pdl_enabled();     // conv_tc.cu; DNB_PDL=0: plain launches
 
+// A launch whose set-up may overlap the tail of the kernel before it in the stream (programmatic dependent launch).  The
+// kernel calls grid_dependency_wait() before it touches anything that an earlier kernel reads or writes, and lets the
+// kernel after it do the same with launch_dependents() (tc_ptx.cuh).
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, (P)args...);
+}
+
 // ---- kernels_mem.cu
 // signs: optional int8 channels-last tensor of pitch spitch that receives the output's signs (f32 channels-last tensors)
 int launch_maxpool(const dnb_tensor *x, const dnb_tensor *y, int size, int stride, int padding, cudaStream_t s, int8_t *signs = nullptr, int spitch = 0);

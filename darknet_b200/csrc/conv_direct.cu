@@ -17,6 +17,7 @@
 #include "common.h"
 #include "conv.h"
 #include "device_utils.cuh"
+#include "tc_ptx.cuh"
 
 namespace dnb {
 
@@ -30,6 +31,8 @@ template <typename TX, typename TY, int FB>
 __global__ void __launch_bounds__(DTHREADS)
 conv_direct_kernel(const __grid_constant__ DirectArgs a)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ __align__(16) float w_s[KCHUNK][FB];
     __shared__ int tap_s[KCHUNK];
     __shared__ __align__(16) float out_s[DTHREADS][FB + 4];   // +4 floats: rows stay 16-byte aligned, banks spread
@@ -190,6 +193,8 @@ template <typename TX, typename TY, int KS, int BM, int BN, int TM, int TN, bool
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM == 16 ? 4 : 7)
 conv_fp32_gemm_kernel(const __grid_constant__ DirectArgs a)
 {
+    grid_dependency_wait();
+    launch_dependents();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     static_assert(THREADS == 64 && (BM / TM == 8 || BM / TM == 16), "two warps, 8 x 4 threads each");
     static_assert(VEC || sizeof(TX) == 4, "cp.async copies f32 values");
@@ -463,6 +468,8 @@ template <typename TX, typename TY>
 __global__ void __launch_bounds__(STHREADS)
 conv_stem3x3_kernel(DirectArgs a)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ __align__(16) float w_s[27][FB];
 
     const ConvGeom g = a.g;
@@ -590,9 +597,9 @@ static int launch_gemm_tile(const DirectArgs &a, cudaStream_t s)
     if (blocks(bm, bn) < 2LL * sm_count()) { bm = 32; bn = 32; }
     dim3 grid((unsigned)((npix + bm - 1) / bm), (unsigned)(g.groups * ((npg + bn - 1) / bn)));
     if (grid.y > 65535) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: too many filter blocks (%u)", grid.y);
-    if (bm == 32) conv_fp32_gemm_kernel<TX, TY, KS, 32, 32, 4, 4, VEC><<<grid, 64, 0, s>>>(a);
-    else if (bn == 64) conv_fp32_gemm_kernel<TX, TY, KS, 128, 64, 16, 8, VEC><<<grid, 64, 0, s>>>(a);
-    else conv_fp32_gemm_kernel<TX, TY, KS, 128, 32, 8, 8, VEC><<<grid, 64, 0, s>>>(a);
+    if (bm == 32) DNB_CUDA((launch_overlapped(conv_fp32_gemm_kernel<TX, TY, KS, 32, 32, 4, 4, VEC>, grid, 64, 0, s, a)));
+    else if (bn == 64) DNB_CUDA((launch_overlapped(conv_fp32_gemm_kernel<TX, TY, KS, 128, 64, 16, 8, VEC>, grid, 64, 0, s, a)));
+    else DNB_CUDA((launch_overlapped(conv_fp32_gemm_kernel<TX, TY, KS, 128, 32, 8, 8, VEC>, grid, 64, 0, s, a)));
     DNB_LAUNCH_CHECK("conv_fp32_gemm");
     return DNB_OK;
 }
@@ -615,8 +622,8 @@ int launch_conv_direct(const DirectArgs &a, cudaStream_t s)
         const long long npairs = (long long)g.batch * g.out_h * ((g.out_w + 1) / 2);
         if (npairs >= (1LL << 31)) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: %lld pixel pairs", npairs);
         dim3 sgrid((unsigned)((npairs + STHREADS - 1) / STHREADS), (unsigned)((g.n + FB - 1) / FB));
-        if (yb) conv_stem3x3_kernel<float, __nv_bfloat16><<<sgrid, STHREADS, 0, s>>>(a);
-        else conv_stem3x3_kernel<float, float><<<sgrid, STHREADS, 0, s>>>(a);
+        if (yb) DNB_CUDA((launch_overlapped(conv_stem3x3_kernel<float, __nv_bfloat16>, sgrid, STHREADS, 0, s, a)));
+        else DNB_CUDA((launch_overlapped(conv_stem3x3_kernel<float, float>, sgrid, STHREADS, 0, s, a)));
         DNB_LAUNCH_CHECK("conv_stem3x3");
         return DNB_OK;
     }
@@ -640,10 +647,10 @@ int launch_conv_direct(const DirectArgs &a, cudaStream_t s)
     if (grid.y > 65535) DNB_FAIL(DNB_EUNSUPPORTED, "direct conv: too many filter blocks (%u)", grid.y);
 #define SLAB_GO(TX, TY)                                                                       \
     do {                                                                                      \
-        if (fb == 4) conv_direct_kernel<TX, TY, 4><<<grid, DTHREADS, 0, s>>>(a);              \
-        else if (fb == 8) conv_direct_kernel<TX, TY, 8><<<grid, DTHREADS, 0, s>>>(a);         \
-        else if (fb == 16) conv_direct_kernel<TX, TY, 16><<<grid, DTHREADS, 0, s>>>(a);       \
-        else conv_direct_kernel<TX, TY, 32><<<grid, DTHREADS, 0, s>>>(a);                     \
+        if (fb == 4) DNB_CUDA((launch_overlapped(conv_direct_kernel<TX, TY, 4>, grid, DTHREADS, 0, s, a)));              \
+        else if (fb == 8) DNB_CUDA((launch_overlapped(conv_direct_kernel<TX, TY, 8>, grid, DTHREADS, 0, s, a)));         \
+        else if (fb == 16) DNB_CUDA((launch_overlapped(conv_direct_kernel<TX, TY, 16>, grid, DTHREADS, 0, s, a)));       \
+        else DNB_CUDA((launch_overlapped(conv_direct_kernel<TX, TY, 32>, grid, DTHREADS, 0, s, a)));                     \
     } while (0)
     DIRECT_TYPES(SLAB_GO);
 #undef SLAB_GO

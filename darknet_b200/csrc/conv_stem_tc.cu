@@ -100,6 +100,8 @@ conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = sh->tmem_base;
+    grid_dependency_wait();   // up to here only the layer's own parameters were read
+    launch_dependents();
 
     // register copies: every asm statement below is a compiler memory barrier
     const float *const x = a.x;
@@ -335,6 +337,8 @@ conv_stem_tc_wide_kernel(const __grid_constant__ StemTcArgs a)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = sh->tmem_base;
+    grid_dependency_wait();   // up to here only the layer's own parameters were read
+    launch_dependents();
 
     const float *const x = a.x;
     const long long xs_b = a.xs_b;
@@ -510,7 +514,7 @@ static int launch_wide_one(const StemTcArgs &a, cudaStream_t s)
     if (per_sm < 1) DNB_FAIL(DNB_ECUDA, "first-layer kernel: %zu bytes of shared memory do not fit", smem);
     long long grid = (long long)sm_count() * per_sm;
     if (grid > a.tiles) grid = a.tiles;
-    kern<<<(unsigned)grid, ST_THREADS, smem, s>>>(a);
+    DNB_CUDA(launch_overlapped(kern, dim3((unsigned)grid), dim3(ST_THREADS), smem, s, a));
     DNB_LAUNCH_CHECK("conv_stem_tc_wide");
     return DNB_OK;
 }
@@ -537,7 +541,7 @@ static int launch_one(const StemTcArgs &a, size_t smem, int grid_limit_per_sm, c
     if (per_sm > grid_limit_per_sm) per_sm = grid_limit_per_sm;
     long long grid = (long long)sm_count() * per_sm;
     if (grid > a.tiles) grid = a.tiles;
-    kern<<<(unsigned)grid, ST_THREADS, smem, s>>>(a);
+    DNB_CUDA(launch_overlapped(kern, dim3((unsigned)grid), dim3(ST_THREADS), smem, s, a));
     DNB_LAUNCH_CHECK("conv_stem_tc");
     return DNB_OK;
 }

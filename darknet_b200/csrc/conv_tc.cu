@@ -159,8 +159,8 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
     if (PAIR) cluster_sync_all();   // the other CTA's barriers are initialised before anything is signalled across the pair
     tc_fence_after();
     // Everything above touched only this CTA's shared memory and TMEM: it may run while the previous layer's kernel is
-    // still draining.  From here on the previous layer's output is read and buffers it may still read are written.
-    grid_dependency_wait();
+    // still draining.  Each role calls grid_dependency_wait() before it reads that layer's output or writes a buffer that it
+    // may still read; the load role first requests the weights of its ring's first round, which no earlier kernel writes.
     launch_dependents();   // this grid is persistent and fully resident: the next layer's CTAs take SMs only as ours leave
     const uint32_t tmem_base = sh->tmem_base;
 
@@ -192,6 +192,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         uint32_t phase = 0;
         bool ok = true;
         if (a.halo) {
+            grid_dependency_wait();
             // one activation box per channel block, then the nine weight tiles that multiply it
             const int a_stages = a.a_stages, b_stages = a.b_stages;
             const uint32_t a_slot = a.a_slot, a_tx = a.a_box_bytes, b_slot = a.b_bytes, b_tx = (uint32_t)bn * row_bytes;
@@ -218,7 +219,26 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 }
             }
-        } else
+        } else {
+        int ahead = first_tile < total_tiles ? min(stages, k_iters) : 0;   // slots whose weights are requested before the wait
+        {
+            const int n0 = (first_tile % n_tiles) * bn + (PAIR ? (int)cta_rank * (bn >> 1) : 0);
+            int tap = 0, cb = 0;
+            for (int s = 0; s < ahead; ++s) {
+                const uint32_t bar = full0 + 8 * s, dst = ring + s * stage_bytes + a_bytes;
+                if (elect_one()) {
+                    if (PAIR) {
+                        if (leader) mbar_expect_tx(bar, 2u * tx_bytes);
+                        tma_load_3d_pair(dst, wmap, bar, cb * bk, n0, tap);
+                    } else {
+                        mbar_expect_tx(bar, tx_bytes);
+                        tma_load_3d(dst, wmap, bar, cb * bk, n0, tap);
+                    }
+                }
+                if (++cb == c_blocks) { cb = 0; ++tap; }
+            }
+        }
+        grid_dependency_wait();
         for (int tile = first_tile; tile < total_tiles && ok; tile += grid_stride) {
             const int nt = tile % n_tiles, pt = pixel_tile(tile);
             const int ow0 = (pt % tiles_w) * wt;
@@ -234,8 +254,11 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 const CUtensorMap *mx = maps + (ph * cstride + pw);
                 const int iw0 = ow0 + qw, ih0 = oh0 + qh;
                 for (int cb = 0; cb < c_blocks; ++cb) {
-                    ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
-                    if (!ok) break;
+                    const bool first = ahead > 0;   // its weights are on their way already
+                    if (!first) {
+                        ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
+                        if (!ok) break;
+                    }
                     // wait-expiry test (debug bit 32): the last operand load of this CTA's first tile is never
                     // requested, so the MMA role's wait for it runs out and the CTA takes the abort path
                     if (withhold && tile == first_tile && tap == taps - 1 && cb == c_blocks - 1) { ok = false; break; }
@@ -244,19 +267,21 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     if (elect_one()) {
                         if (PAIR) {
                             // one barrier, in the even CTA, counts the bytes of both CTAs' loads of this slot
-                            if (leader) mbar_expect_tx(bar, 2u * tx_bytes);
+                            if (leader && !first) mbar_expect_tx(bar, 2u * tx_bytes);
                             tma_load_4d_pair(sa, mx, bar, cb * bk, iw0, ih0, b0);
-                            tma_load_3d_pair(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
+                            if (!first) tma_load_3d_pair(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
                         } else {
-                            mbar_expect_tx(bar, tx_bytes);
+                            if (!first) mbar_expect_tx(bar, tx_bytes);
                             tma_load_4d(sa, mx, bar, cb * bk, iw0, ih0, b0);
-                            tma_load_3d(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
+                            if (!first) tma_load_3d(sa + a_bytes, wmap, bar, cb * bk, n0, tap);
                         }
                     }
+                    ahead -= first ? 1 : 0;
                     if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
                 if (++kw == ksize) { kw = 0; ++kh; }
             }
+        }
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -272,6 +297,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]);
         int *status = a.status;
         const int dbg_mma = a.debug;
+        grid_dependency_wait();   // only so that the bounds of the waits below count this launch's own time
         int stage = 0;
         uint32_t phase = 0;
         uint64_t da = da0, db = db0;
@@ -363,6 +389,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         __syncwarp();
     } else {
         // ---------------- epilogue: warps 2..5 own TMEM lanes 32*(warp%4) .. +31
+        grid_dependency_wait();
         const int quarter = warp & 3;
         const int m = quarter * 32 + lane;  // pixel index inside the tile = TMEM lane = staging row
         const int wl = m % wt, hl = (m / wt) % ht, bl = m / (wt * ht);

@@ -205,6 +205,7 @@ conv_tc_split_kernel(const __grid_constant__ SplitArgs a)
         uint32_t phase = 0;
         uint64_t da = da0, db = db0;
         bool ok = leader;
+        grid_dependency_wait();   // only so that the bounds of the waits below count this launch's own time
         for (int ki = 0; ki < kn && ok; ++ki) {
             ok = mbar_wait_warp(full0 + 8 * stage, phase, abort_flag, status, SP_WAIT_FULL, wait_limit);
             if (!ok) break;
@@ -257,6 +258,7 @@ conv_tc_split_kernel(const __grid_constant__ SplitArgs a)
             sh->pixel[m] = in ? (b * g.out_h + oh) * g.out_w + ow : -1;
             sh->nchw[m] = in ? (long long)b * g.n * g.out_h * g.out_w + oh * g.out_w + ow : 0;
         }
+        grid_dependency_wait();
         mbar_wait(smem_u32(&sh->acc_full), 0, abort_flag, status, SP_WAIT_ACC_FULL, 0, wait_limit);
         tc_fence_after();
         if (!*abort_flag) {   // (an aborted CTA's loads may still be landing where the dump goes; its tile is incomplete anyway)

@@ -17,6 +17,7 @@
 #include "common.h"
 #include "conv.h"
 #include "device_utils.cuh"
+#include "tc_ptx.cuh"
 
 namespace dnb {
 
@@ -239,6 +240,8 @@ template <typename T, bool NCHW>
 __global__ void __launch_bounds__(256)
 pack_sign_i8_kernel(const T *__restrict__ x, int8_t *__restrict__ out, size_t npix, size_t HW, int C, int Cp_in, int cpad)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const int groups = cpad / 16;
     const size_t total = npix * groups;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -276,9 +279,9 @@ int launch_pack_sign_i8(const dnb_tensor *x, int8_t *out, int cpad, cudaStream_t
     const size_t total = npix * (cpad / 16);
     const size_t blocks = (total + 255) / 256, cap = (size_t)sm_count() * 16;
     const int grid = (int)(blocks < cap ? (blocks ? blocks : 1) : cap);
-    if (x->layout == DNB_NCHW) pack_sign_i8_kernel<float, true><<<grid, 256, 0, s>>>((const float *)x->data, out, npix, HW, x->c, 0, cpad);
-    else if (x->dtype == DNB_F32) pack_sign_i8_kernel<float, false><<<grid, 256, 0, s>>>((const float *)x->data, out, npix, HW, x->c, x->cpitch, cpad);
-    else pack_sign_i8_kernel<__nv_bfloat16, false><<<grid, 256, 0, s>>>((const __nv_bfloat16 *)x->data, out, npix, HW, x->c, x->cpitch, cpad);
+    if (x->layout == DNB_NCHW) DNB_CUDA((launch_overlapped(pack_sign_i8_kernel<float, true>, grid, 256, 0, s, (const float *)x->data, out, npix, HW, x->c, 0, cpad)));
+    else if (x->dtype == DNB_F32) DNB_CUDA((launch_overlapped(pack_sign_i8_kernel<float, false>, grid, 256, 0, s, (const float *)x->data, out, npix, HW, x->c, x->cpitch, cpad)));
+    else DNB_CUDA((launch_overlapped(pack_sign_i8_kernel<__nv_bfloat16, false>, grid, 256, 0, s, (const __nv_bfloat16 *)x->data, out, npix, HW, x->c, x->cpitch, cpad)));
     DNB_LAUNCH_CHECK("pack_sign_i8");
     return DNB_OK;
 }

@@ -11,6 +11,7 @@
 // grid that is a multiple of the SM count.  None of them is GEMM-shaped.
 #include "common.h"
 #include "device_utils.cuh"
+#include "tc_ptx.cuh"
 
 namespace dnb {
 
@@ -51,6 +52,8 @@ __global__ void __launch_bounds__(256)
 maxpool_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, int W, int cvecs,
                     int OH, int OW, int size_rt, int stride, int off, int8_t *__restrict__ signs, int spitch)
 {
+    grid_dependency_wait();
+    launch_dependents();
     // signs (f32 tensors only): also write the signs of the output (+1 where > 0, else -1) as an int8 channels-last
     // tensor of pitch spitch, the operand of the tensor-core xnor layer that follows; every channel is a real one there
     using V = Vec16<T>;
@@ -117,6 +120,8 @@ maxpool_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, in
 __global__ void maxpool_nchw_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int H, int W,
                                     int OH, int OW, int size, int stride, int off)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const size_t total = (size_t)planes * OH * OW;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         int ow = (int)(i % OW);
@@ -150,9 +155,9 @@ int launch_maxpool(const dnb_tensor *x, const dnb_tensor *y, int size, int strid
     const int off = -(padding / 2);
 #define MAXPOOL_LAUNCH(T, ...)                                                                          \
     do {                                                                                                \
-        if (size == 2) maxpool_nhwc_kernel<T, 2><<<row_grid(y->n, oh), 256, 0, s>>>(__VA_ARGS__);       \
-        else if (size == 3) maxpool_nhwc_kernel<T, 3><<<row_grid(y->n, oh), 256, 0, s>>>(__VA_ARGS__);  \
-        else maxpool_nhwc_kernel<T, 0><<<row_grid(y->n, oh), 256, 0, s>>>(__VA_ARGS__);                 \
+        if (size == 2) DNB_CUDA((launch_overlapped(maxpool_nhwc_kernel<T, 2>, row_grid(y->n, oh), 256, 0, s, __VA_ARGS__)));       \
+        else if (size == 3) DNB_CUDA((launch_overlapped(maxpool_nhwc_kernel<T, 3>, row_grid(y->n, oh), 256, 0, s, __VA_ARGS__)));  \
+        else DNB_CUDA((launch_overlapped(maxpool_nhwc_kernel<T, 0>, row_grid(y->n, oh), 256, 0, s, __VA_ARGS__)));                 \
     } while (0)
     if (x->layout == DNB_NHWC) {
         if (x->cpitch != y->cpitch) DNB_FAIL(DNB_EINVAL, "maxpool: cpitch differs (%d vs %d)", x->cpitch, y->cpitch);
@@ -169,7 +174,7 @@ int launch_maxpool(const dnb_tensor *x, const dnb_tensor *y, int size, int strid
         if (x->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "maxpool: NCHW tensors must be f32");
         if (signs) DNB_FAIL(DNB_EINVAL, "maxpool: the sign output is built for channels-last tensors");
         size_t total = (size_t)y->n * y->c * oh * ow;
-        maxpool_nchw_kernel<<<grid_for(total, 128), 128, 0, s>>>((const float *)x->data, (float *)y->data, x->n * x->c, x->h, x->w, oh, ow, size, stride, off);
+        DNB_CUDA((launch_overlapped(maxpool_nchw_kernel, grid_for(total, 128), 128, 0, s, (const float *)x->data, (float *)y->data, x->n * x->c, x->h, x->w, oh, ow, size, stride, off)));
     }
 #undef MAXPOOL_LAUNCH
     DNB_LAUNCH_CHECK("maxpool");
@@ -183,6 +188,8 @@ __global__ void __launch_bounds__(256)
 upsample_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, int W, int cvecs, int xpitch_vecs, int ypitch_vecs,
                      int stride, float scale)
 {
+    grid_dependency_wait();
+    launch_dependents();
     // cvecs 16-byte vectors of channels per pixel are copied; input and output pixels may be further apart than that
     // (a tensor that is a channel range of a wider one, e.g. the slice of a [route] output it was placed in)
     using V = Vec16<T>;
@@ -209,6 +216,8 @@ upsample_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, i
 __global__ void upsample_nchw_kernel(const float *__restrict__ x, float *__restrict__ y, int planes, int H, int W,
                                      int stride, float scale)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const int OH = H * stride, OW = W * stride;
     const size_t total = (size_t)planes * OH * OW;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -234,16 +243,16 @@ int launch_upsample(const dnb_tensor *x, const dnb_tensor *y, int stride, float 
         const int cv = (x->cpitch < y->cpitch ? x->cpitch : y->cpitch) / per;
         if (cv * per < x->c || x->cpitch % per || y->cpitch % per) DNB_FAIL(DNB_EINVAL, "upsample: channel pitches %d and %d for %d channels", x->cpitch, y->cpitch, x->c);
         if (x->dtype == DNB_F32) {
-            upsample_nhwc_kernel<float><<<row_grid(y->n, y->h), 256, 0, s>>>((const float *)x->data, (float *)y->data, x->n, x->h, x->w, cv, x->cpitch / per,
-                                                                            y->cpitch / per, stride, scale);
+            DNB_CUDA((launch_overlapped(upsample_nhwc_kernel<float>, row_grid(y->n, y->h), 256, 0, s, (const float *)x->data, (float *)y->data, x->n, x->h, x->w, cv, x->cpitch / per,
+                                                                            y->cpitch / per, stride, scale)));
         } else {
-            upsample_nhwc_kernel<__nv_bfloat16><<<row_grid(y->n, y->h), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->n, x->h, x->w,
-                                                                                    cv, x->cpitch / per, y->cpitch / per, stride, scale);
+            DNB_CUDA((launch_overlapped(upsample_nhwc_kernel<__nv_bfloat16>, row_grid(y->n, y->h), 256, 0, s, (const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->n, x->h, x->w,
+                                                                                    cv, x->cpitch / per, y->cpitch / per, stride, scale)));
         }
     } else {
         if (x->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "upsample: NCHW tensors must be f32");
         size_t total = (size_t)y->n * y->c * y->h * y->w;
-        upsample_nchw_kernel<<<grid_for(total, 128), 128, 0, s>>>((const float *)x->data, (float *)y->data, x->n * x->c, x->h, x->w, stride, scale);
+        DNB_CUDA((launch_overlapped(upsample_nchw_kernel, grid_for(total, 128), 128, 0, s, (const float *)x->data, (float *)y->data, x->n * x->c, x->h, x->w, stride, scale)));
     }
     DNB_LAUNCH_CHECK("upsample");
     return DNB_OK;
@@ -255,6 +264,8 @@ template <typename T>
 __global__ void shortcut_flat_kernel(const T *__restrict__ x, const T *__restrict__ add, T *__restrict__ y,
                                      size_t nvec, float alpha, float beta, int act)
 {
+    grid_dependency_wait();
+    launch_dependents();
     using V = Vec16<T>;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
         V a, b, o;
@@ -282,6 +293,8 @@ template <typename T>
 __global__ void shortcut_general_kernel(const T *__restrict__ x, const T *__restrict__ add, T *__restrict__ y,
                                         ShortcutGeom g, float alpha, float beta, int act)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const size_t total = (size_t)g.B * g.C2 * g.H2 * g.W2;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         int b, c, h, w;
@@ -310,6 +323,8 @@ __global__ void __launch_bounds__(256)
 shortcut_rows_nhwc_kernel(const T *__restrict__ x, const T *__restrict__ add, T *__restrict__ y, ShortcutGeom g,
                           int cpitch, int add_cpitch, int add_h, int add_w, float alpha, float beta, int act)
 {
+    grid_dependency_wait();
+    launch_dependents();
     using V = Vec16<T>;
     const int cvecs = cpitch / V::N, rows = g.B * g.H2, row_vecs = g.W2 * cvecs;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -369,9 +384,9 @@ int launch_shortcut(const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor
         if (bytes % 16 == 0) {
             size_t nvec = bytes / 16;
             if (x->dtype == DNB_F32)
-                shortcut_flat_kernel<float><<<grid_for(nvec, 256), 256, 0, s>>>((const float *)x->data, (const float *)add->data, (float *)y->data, nvec, alpha, beta, activation);
+                DNB_CUDA((launch_overlapped(shortcut_flat_kernel<float>, grid_for(nvec, 256), 256, 0, s, (const float *)x->data, (const float *)add->data, (float *)y->data, nvec, alpha, beta, activation)));
             else
-                shortcut_flat_kernel<__nv_bfloat16><<<grid_for(nvec, 256), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data, (__nv_bfloat16 *)y->data, nvec, alpha, beta, activation);
+                DNB_CUDA((launch_overlapped(shortcut_flat_kernel<__nv_bfloat16>, grid_for(nvec, 256), 256, 0, s, (const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data, (__nv_bfloat16 *)y->data, nvec, alpha, beta, activation)));
             DNB_LAUNCH_CHECK("shortcut");
             return DNB_OK;
         }
@@ -398,20 +413,20 @@ int launch_shortcut(const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor
     }
     if (x->layout == DNB_NHWC && (long long)g.B * g.H2 < (1LL << 31) && (long long)g.W2 * x->cpitch < (1LL << 31)) {
         if (x->dtype == DNB_F32)
-            shortcut_rows_nhwc_kernel<float><<<row_grid(g.B, g.H2), 256, 0, s>>>((const float *)x->data, (const float *)add->data, (float *)y->data, g,
-                                                                              x->cpitch, add->cpitch, add->h, add->w, alpha, beta, activation);
+            DNB_CUDA((launch_overlapped(shortcut_rows_nhwc_kernel<float>, row_grid(g.B, g.H2), 256, 0, s, (const float *)x->data, (const float *)add->data, (float *)y->data, g,
+                                                                              x->cpitch, add->cpitch, add->h, add->w, alpha, beta, activation)));
         else
-            shortcut_rows_nhwc_kernel<__nv_bfloat16><<<row_grid(g.B, g.H2), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data,
+            DNB_CUDA((launch_overlapped(shortcut_rows_nhwc_kernel<__nv_bfloat16>, row_grid(g.B, g.H2), 256, 0, s, (const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data,
                                                                                       (__nv_bfloat16 *)y->data, g, x->cpitch, add->cpitch, add->h, add->w,
-                                                                                      alpha, beta, activation);
+                                                                                      alpha, beta, activation)));
         DNB_LAUNCH_CHECK("shortcut");
         return DNB_OK;
     }
     size_t total = (size_t)g.B * g.C2 * g.H2 * g.W2;
     if (x->dtype == DNB_F32)
-        shortcut_general_kernel<float><<<grid_for(total, 256), 256, 0, s>>>((const float *)x->data, (const float *)add->data, (float *)y->data, g, alpha, beta, activation);
+        DNB_CUDA((launch_overlapped(shortcut_general_kernel<float>, grid_for(total, 256), 256, 0, s, (const float *)x->data, (const float *)add->data, (float *)y->data, g, alpha, beta, activation)));
     else
-        shortcut_general_kernel<__nv_bfloat16><<<grid_for(total, 256), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data, (__nv_bfloat16 *)y->data, g, alpha, beta, activation);
+        DNB_CUDA((launch_overlapped(shortcut_general_kernel<__nv_bfloat16>, grid_for(total, 256), 256, 0, s, (const __nv_bfloat16 *)x->data, (const __nv_bfloat16 *)add->data, (__nv_bfloat16 *)y->data, g, alpha, beta, activation)));
     DNB_LAUNCH_CHECK("shortcut");
     return DNB_OK;
 }
@@ -421,6 +436,8 @@ template <typename V>
 __global__ void copy2d_kernel(const V *__restrict__ src, V *__restrict__ dst, size_t rows, size_t row_len,
                               size_t src_pitch, size_t dst_pitch)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const size_t total = rows * row_len;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         size_t r = i / row_len, k = i - r * row_len;
@@ -434,16 +451,16 @@ static int copy2d(const void *src, void *dst, size_t rows, size_t row_bytes, siz
     const size_t all = row_bytes | src_pitch_bytes | dst_pitch_bytes | (size_t)(uintptr_t)src | (size_t)(uintptr_t)dst;
     if (all % 16 == 0) {
         size_t n = rows * (row_bytes / 16);
-        copy2d_kernel<uint4><<<grid_for(n, 256), 256, 0, s>>>((const uint4 *)src, (uint4 *)dst, rows, row_bytes / 16, src_pitch_bytes / 16, dst_pitch_bytes / 16);
+        DNB_CUDA((launch_overlapped(copy2d_kernel<uint4>, grid_for(n, 256), 256, 0, s, (const uint4 *)src, (uint4 *)dst, rows, row_bytes / 16, src_pitch_bytes / 16, dst_pitch_bytes / 16)));
     } else if (all % 8 == 0) {
         size_t n = rows * (row_bytes / 8);
-        copy2d_kernel<uint2><<<grid_for(n, 256), 256, 0, s>>>((const uint2 *)src, (uint2 *)dst, rows, row_bytes / 8, src_pitch_bytes / 8, dst_pitch_bytes / 8);
+        DNB_CUDA((launch_overlapped(copy2d_kernel<uint2>, grid_for(n, 256), 256, 0, s, (const uint2 *)src, (uint2 *)dst, rows, row_bytes / 8, src_pitch_bytes / 8, dst_pitch_bytes / 8)));
     } else if (all % 4 == 0) {
         size_t n = rows * (row_bytes / 4);
-        copy2d_kernel<uint32_t><<<grid_for(n, 256), 256, 0, s>>>((const uint32_t *)src, (uint32_t *)dst, rows, row_bytes / 4, src_pitch_bytes / 4, dst_pitch_bytes / 4);
+        DNB_CUDA((launch_overlapped(copy2d_kernel<uint32_t>, grid_for(n, 256), 256, 0, s, (const uint32_t *)src, (uint32_t *)dst, rows, row_bytes / 4, src_pitch_bytes / 4, dst_pitch_bytes / 4)));
     } else {
         size_t n = rows * (row_bytes / 2);
-        copy2d_kernel<uint16_t><<<grid_for(n, 256), 256, 0, s>>>((const uint16_t *)src, (uint16_t *)dst, rows, row_bytes / 2, src_pitch_bytes / 2, dst_pitch_bytes / 2);
+        DNB_CUDA((launch_overlapped(copy2d_kernel<uint16_t>, grid_for(n, 256), 256, 0, s, (const uint16_t *)src, (uint16_t *)dst, rows, row_bytes / 2, src_pitch_bytes / 2, dst_pitch_bytes / 2)));
     }
     DNB_LAUNCH_CHECK("route copy");
     return DNB_OK;
@@ -492,6 +509,8 @@ int launch_route(const dnb_tensor *const *inputs, int count, const dnb_tensor *y
 template <typename T>
 __global__ void nchw_to_nhwc_kernel(const float *__restrict__ x, T *__restrict__ y, int C, int HW, int Cp, int rnd)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ float tile[32][33];
     const int b = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -519,6 +538,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 nhwc_to_nchw_kernel(const T *__restrict__ x, float *__restrict__ y, int C, int HW, int Cp, int yolo_entries)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ float tile[32][129];
     const int b = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 128;
@@ -573,6 +594,8 @@ template <typename TI, typename TO>
 __global__ void elementwise_convert_kernel(const TI *__restrict__ x, TO *__restrict__ y, size_t total, int rnd,
                                            int yolo_entries, int HW, int C)
 {
+    grid_dependency_wait();
+    launch_dependents();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float v = to_float<TI>(x[i]);
         if (yolo_entries > 0) {  // NCHW only
@@ -597,24 +620,24 @@ int launch_convert(const dnb_tensor *x, const dnb_tensor *y, int rnd, int yolo_a
     if (x->layout == DNB_NCHW && y->layout == DNB_NHWC) {
         if (x->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "convert: NCHW tensors must be f32");
         dim3 grid((HW + 31) / 32, (y->cpitch + 31) / 32, x->n);
-        if (y->dtype == DNB_F32) nchw_to_nhwc_kernel<float><<<grid, block, 0, s>>>((const float *)x->data, (float *)y->data, x->c, HW, y->cpitch, rnd);
-        else nchw_to_nhwc_kernel<__nv_bfloat16><<<grid, block, 0, s>>>((const float *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, y->cpitch, 0);
+        if (y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(nchw_to_nhwc_kernel<float>, grid, block, 0, s, (const float *)x->data, (float *)y->data, x->c, HW, y->cpitch, rnd)));
+        else DNB_CUDA((launch_overlapped(nchw_to_nhwc_kernel<__nv_bfloat16>, grid, block, 0, s, (const float *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, y->cpitch, 0)));
     } else if (x->layout == DNB_NHWC && y->layout == DNB_NCHW) {
         if (y->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "convert: NCHW tensors must be f32");
         dim3 grid((HW + 127) / 128, (x->c + 31) / 32, x->n);
-        if (x->dtype == DNB_F32) nhwc_to_nchw_kernel<float><<<grid, 256, 0, s>>>((const float *)x->data, (float *)y->data, x->c, HW, x->cpitch, entries);
-        else nhwc_to_nchw_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16 *)x->data, (float *)y->data, x->c, HW, x->cpitch, entries);
+        if (x->dtype == DNB_F32) DNB_CUDA((launch_overlapped(nhwc_to_nchw_kernel<float>, grid, 256, 0, s, (const float *)x->data, (float *)y->data, x->c, HW, x->cpitch, entries)));
+        else DNB_CUDA((launch_overlapped(nhwc_to_nchw_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16 *)x->data, (float *)y->data, x->c, HW, x->cpitch, entries)));
     } else if (x->layout == DNB_NCHW) {
         if (x->dtype != DNB_F32 || y->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "convert: NCHW tensors must be f32");
         size_t total = tensor_elems(x);
-        elementwise_convert_kernel<float, float><<<grid_for(total, 256), 256, 0, s>>>((const float *)x->data, (float *)y->data, total, rnd, entries, HW, x->c);
+        DNB_CUDA((launch_overlapped(elementwise_convert_kernel<float, float>, grid_for(total, 256), 256, 0, s, (const float *)x->data, (float *)y->data, total, rnd, entries, HW, x->c)));
     } else {
         if (x->cpitch != y->cpitch) DNB_FAIL(DNB_EINVAL, "convert: NHWC to NHWC needs equal cpitch");
         size_t total = tensor_elems(x);
-        if (x->dtype == DNB_F32 && y->dtype == DNB_F32) elementwise_convert_kernel<float, float><<<grid_for(total, 256), 256, 0, s>>>((const float *)x->data, (float *)y->data, total, rnd, 0, 1, 1);
-        else if (x->dtype == DNB_F32) elementwise_convert_kernel<float, __nv_bfloat16><<<grid_for(total, 256), 256, 0, s>>>((const float *)x->data, (__nv_bfloat16 *)y->data, total, 0, 0, 1, 1);
-        else if (y->dtype == DNB_F32) elementwise_convert_kernel<__nv_bfloat16, float><<<grid_for(total, 256), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (float *)y->data, total, 0, 0, 1, 1);
-        else elementwise_convert_kernel<__nv_bfloat16, __nv_bfloat16><<<grid_for(total, 256), 256, 0, s>>>((const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, total, 0, 0, 1, 1);
+        if (x->dtype == DNB_F32 && y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(elementwise_convert_kernel<float, float>, grid_for(total, 256), 256, 0, s, (const float *)x->data, (float *)y->data, total, rnd, 0, 1, 1)));
+        else if (x->dtype == DNB_F32) DNB_CUDA((launch_overlapped(elementwise_convert_kernel<float, __nv_bfloat16>, grid_for(total, 256), 256, 0, s, (const float *)x->data, (__nv_bfloat16 *)y->data, total, 0, 0, 1, 1)));
+        else if (y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(elementwise_convert_kernel<__nv_bfloat16, float>, grid_for(total, 256), 256, 0, s, (const __nv_bfloat16 *)x->data, (float *)y->data, total, 0, 0, 1, 1)));
+        else DNB_CUDA((launch_overlapped(elementwise_convert_kernel<__nv_bfloat16, __nv_bfloat16>, grid_for(total, 256), 256, 0, s, (const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, total, 0, 0, 1, 1)));
     }
     DNB_LAUNCH_CHECK("convert");
     return DNB_OK;
@@ -627,6 +650,8 @@ template <typename T>
 __global__ void avgpool_kernel(const T *__restrict__ x, T *__restrict__ y, int C, int HW, long long sb, long long sc,
                                long long sp, long long ysb)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ float part[8][33];
     const int b = blockIdx.y, c = blockIdx.x * 32 + threadIdx.x;
     float acc = 0.f;
@@ -653,8 +678,8 @@ int launch_avgpool(const dnb_tensor *x, const dnb_tensor *y, cudaStream_t s)
     if (x->layout == DNB_NHWC) { sc = 1; sp = x->cpitch; sb = (long long)HW * x->cpitch; ysb = y->cpitch; }
     else { sp = 1; sc = HW; sb = (long long)x->c * HW; ysb = y->c; }
     dim3 grid((x->c + 31) / 32, x->n), block(32, 8);
-    if (x->dtype == DNB_F32) avgpool_kernel<float><<<grid, block, 0, s>>>((const float *)x->data, (float *)y->data, x->c, HW, sb, sc, sp, ysb);
-    else avgpool_kernel<__nv_bfloat16><<<grid, block, 0, s>>>((const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, sb, sc, sp, ysb);
+    if (x->dtype == DNB_F32) DNB_CUDA((launch_overlapped(avgpool_kernel<float>, grid, block, 0, s, (const float *)x->data, (float *)y->data, x->c, HW, sb, sc, sp, ysb)));
+    else DNB_CUDA((launch_overlapped(avgpool_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, sb, sc, sp, ysb)));
     DNB_LAUNCH_CHECK("avgpool");
     return DNB_OK;
 }
@@ -665,6 +690,8 @@ template <typename T>
 __global__ void softmax_kernel(const T *__restrict__ x, T *__restrict__ y, int n, long long batch_stride,
                                int group_stride, float temp)
 {
+    grid_dependency_wait();
+    launch_dependents();
     __shared__ float red[32];
     const T *in = x + blockIdx.y * batch_stride + (long long)blockIdx.x * group_stride;
     T *out = y + blockIdx.y * batch_stride + (long long)blockIdx.x * group_stride;
@@ -699,8 +726,8 @@ int launch_softmax(const dnb_tensor *x, const dnb_tensor *y, int groups, float t
     if (x->layout == DNB_NHWC && x->cpitch != y->cpitch) DNB_FAIL(DNB_EINVAL, "softmax: cpitch differs");
     const long long bs = x->layout == DNB_NHWC ? x->cpitch : x->c;
     dim3 grid(groups, x->n);
-    if (x->dtype == DNB_F32) softmax_kernel<float><<<grid, 256, 0, s>>>((const float *)x->data, (float *)y->data, x->c / groups, bs, x->c / groups, temperature);
-    else softmax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->c / groups, bs, x->c / groups, temperature);
+    if (x->dtype == DNB_F32) DNB_CUDA((launch_overlapped(softmax_kernel<float>, grid, 256, 0, s, (const float *)x->data, (float *)y->data, x->c / groups, bs, x->c / groups, temperature)));
+    else DNB_CUDA((launch_overlapped(softmax_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16 *)x->data, (__nv_bfloat16 *)y->data, x->c / groups, bs, x->c / groups, temperature)));
     DNB_LAUNCH_CHECK("softmax");
     return DNB_OK;
 }
