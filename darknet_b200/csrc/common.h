@@ -64,13 +64,16 @@ bool pdl_enabled();     // conv_tc.cu; DNB_PDL=0: plain launches
 
 // A launch whose set-up may overlap the tail of the kernel before it in the stream (programmatic dependent launch).  The
 // kernel calls grid_dependency_wait() before it touches anything that an earlier kernel reads or writes, and lets the
-// kernel after it do the same with launch_dependents() (tc_ptx.cuh).
+// kernel after it do the same with launch_dependents_if_small() (tc_ptx.cuh).  Only grids of at most two blocks per SM start
+// early: larger ones would fill whatever room the running kernel leaves here and there, and their even share of blocks per
+// SM would be lost (Darknet-19 at batch 128 with every pooling layer started early: 1.30 -> 1.42 ms).
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    const long long blocks = (long long)grid.x * grid.y * grid.z;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() && blocks <= 2LL * sm_count() ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;

@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(DTHREADS)
 conv_direct_kernel(const __grid_constant__ DirectArgs a)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ __align__(16) float w_s[KCHUNK][FB];
     __shared__ int tap_s[KCHUNK];
     __shared__ __align__(16) float out_s[DTHREADS][FB + 4];   // +4 floats: rows stay 16-byte aligned, banks spread
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM == 16 ? 4 : 7)
 conv_fp32_gemm_kernel(const __grid_constant__ DirectArgs a)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     static_assert(THREADS == 64 && (BM / TM == 8 || BM / TM == 16), "two warps, 8 x 4 threads each");
     static_assert(VEC || sizeof(TX) == 4, "cp.async copies f32 values");
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(STHREADS)
 conv_stem3x3_kernel(DirectArgs a)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ __align__(16) float w_s[27][FB];
 
     const ConvGeom g = a.g;

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256)
 pack_sign_i8_kernel(const T *__restrict__ x, int8_t *__restrict__ out, size_t npix, size_t HW, int C, int Cp_in, int cpad)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     const int groups = cpad / 16;
     const size_t total = npix * groups;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {

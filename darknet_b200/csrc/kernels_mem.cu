@@ -53,7 +53,7 @@ maxpool_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, in
                     int OH, int OW, int size_rt, int stride, int off, int8_t *__restrict__ signs, int spitch)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     // signs (f32 tensors only): also write the signs of the output (+1 where > 0, else -1) as an int8 channels-last
     // tensor of pitch spitch, the operand of the tensor-core xnor layer that follows; every channel is a real one there
     using V = Vec16<T>;
@@ -121,7 +121,7 @@ __global__ void maxpool_nchw_kernel(const float *__restrict__ x, float *__restri
                                     int OH, int OW, int size, int stride, int off)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     const size_t total = (size_t)planes * OH * OW;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         int ow = (int)(i % OW);
@@ -189,7 +189,7 @@ upsample_nhwc_kernel(const T *__restrict__ x, T *__restrict__ y, int B, int H, i
                      int stride, float scale)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     // cvecs 16-byte vectors of channels per pixel are copied; input and output pixels may be further apart than that
     // (a tensor that is a channel range of a wider one, e.g. the slice of a [route] output it was placed in)
     using V = Vec16<T>;
@@ -217,7 +217,7 @@ __global__ void upsample_nchw_kernel(const float *__restrict__ x, float *__restr
                                      int stride, float scale)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     const int OH = H * stride, OW = W * stride;
     const size_t total = (size_t)planes * OH * OW;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -265,7 +265,6 @@ __global__ void shortcut_flat_kernel(const T *__restrict__ x, const T *__restric
                                      size_t nvec, float alpha, float beta, int act)
 {
     grid_dependency_wait();
-    launch_dependents();
     using V = Vec16<T>;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
         V a, b, o;
@@ -294,7 +293,6 @@ __global__ void shortcut_general_kernel(const T *__restrict__ x, const T *__rest
                                         ShortcutGeom g, float alpha, float beta, int act)
 {
     grid_dependency_wait();
-    launch_dependents();
     const size_t total = (size_t)g.B * g.C2 * g.H2 * g.W2;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         int b, c, h, w;
@@ -318,13 +316,13 @@ __global__ void shortcut_general_kernel(const T *__restrict__ x, const T *__rest
 // General shapes, channels-last: one output row (b, h) per block iteration, threads along the row's (w, 16-byte
 // channel vector) pairs.  The add tensor contributes where the reference's loops reach (src/blas.c:68-92): channels
 // below minc, and pixels (h, w) that are multiples of `sample`, read from (h/sample*stride, w/sample*stride).
+// (No early launch of the successor: with that test in front of it the loop was compiled to run 1.5 times as long.)
 template <typename T>
 __global__ void __launch_bounds__(256)
 shortcut_rows_nhwc_kernel(const T *__restrict__ x, const T *__restrict__ add, T *__restrict__ y, ShortcutGeom g,
                           int cpitch, int add_cpitch, int add_h, int add_w, float alpha, float beta, int act)
 {
     grid_dependency_wait();
-    launch_dependents();
     using V = Vec16<T>;
     const int cvecs = cpitch / V::N, rows = g.B * g.H2, row_vecs = g.W2 * cvecs;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -437,7 +435,7 @@ __global__ void copy2d_kernel(const V *__restrict__ src, V *__restrict__ dst, si
                               size_t src_pitch, size_t dst_pitch)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     const size_t total = rows * row_len;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         size_t r = i / row_len, k = i - r * row_len;
@@ -510,7 +508,7 @@ template <typename T>
 __global__ void nchw_to_nhwc_kernel(const float *__restrict__ x, T *__restrict__ y, int C, int HW, int Cp, int rnd)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ float tile[32][33];
     const int b = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 32;
@@ -539,7 +537,7 @@ __global__ void __launch_bounds__(256)
 nhwc_to_nchw_kernel(const T *__restrict__ x, float *__restrict__ y, int C, int HW, int Cp, int yolo_entries)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ float tile[32][129];
     const int b = blockIdx.z;
     const int c0 = blockIdx.y * 32, p0 = blockIdx.x * 128;
@@ -595,7 +593,7 @@ __global__ void elementwise_convert_kernel(const TI *__restrict__ x, TO *__restr
                                            int yolo_entries, int HW, int C)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float v = to_float<TI>(x[i]);
         if (yolo_entries > 0) {  // NCHW only
@@ -651,7 +649,7 @@ __global__ void avgpool_kernel(const T *__restrict__ x, T *__restrict__ y, int C
                                long long sp, long long ysb)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ float part[8][33];
     const int b = blockIdx.y, c = blockIdx.x * 32 + threadIdx.x;
     float acc = 0.f;
@@ -691,7 +689,7 @@ __global__ void softmax_kernel(const T *__restrict__ x, T *__restrict__ y, int n
                                int group_stride, float temp)
 {
     grid_dependency_wait();
-    launch_dependents();
+    launch_dependents_if_small();
     __shared__ float red[32];
     const T *in = x + blockIdx.y * batch_stride + (long long)blockIdx.x * group_stride;
     T *out = y + blockIdx.y * batch_stride + (long long)blockIdx.x * group_stride;

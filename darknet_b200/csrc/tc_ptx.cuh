@@ -200,6 +200,11 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 // launch_dependents() lets the kernel after this one be scheduled the same way.  Both are no-ops in a plain launch.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// ... from a kernel of many short blocks: where it fills the GPU, early successors would only take room from its own blocks.
+__device__ __forceinline__ void launch_dependents_if_small()
+{
+    if ((unsigned long long)gridDim.x * gridDim.y * gridDim.z <= 296ull) launch_dependents();
+}
 
 // ------------------------------------------------------------------ CTA pairs (cta_group::2)
 // Two CTAs of a cluster of two run one MMA of 256 rows: each holds 128 rows of A and half of B's columns in its own
