@@ -1,0 +1,20 @@
+// Parallel copy of ordinary host memory into a page-locked staging ring, chunk by chunk, so that the chunks' transfers to
+// the device overlap the copying of the later ones.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include <memory>
+
+namespace dnb {
+
+class CopyPool;
+
+// The process's pool of copying threads.  It is made by the first holder and joined when the last one lets go.
+std::shared_ptr<CopyPool> copy_pool();
+
+// Uploads `bytes` from pageable `src` to memory `dst` of the current device on `s`.  Returns once src has been read; the
+// transfers are then enqueued.  Safe to call from several threads (callers take turns).
+int upload_staged(CopyPool *pool, void *dst, const void *src, size_t bytes, cudaStream_t s);
+
+}  // namespace dnb

@@ -7,11 +7,13 @@
 #include <string.h>
 
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include "common.h"
 #include "conv.h"
+#include "host_copy.h"
 
 using namespace dnb;
 
@@ -156,6 +158,12 @@ struct dnb_network {
     cudaStream_t graph_stream = nullptr;
     int eager_runs = 0;
     std::vector<cudaEvent_t> events;
+    // the blocking call replays its step, layers and result copies, as one graph per slot (see dnb_network_predict)
+    cudaGraphExec_t step_exec[2] = {nullptr, nullptr};
+    int step_runs[2] = {0, 0};
+    bool step_graphs = true;              // off once something could not be captured
+    cudaEvent_t pulled = nullptr;         // copy stream: every result copy of a blocking step is enqueued
+    std::shared_ptr<CopyPool> copier;     // made with the first input in pageable memory
 };
 
 static void drop_graph(dnb_network *net);
@@ -448,6 +456,7 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
             DNB_CUDA(cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming));
             DNB_CUDA(cudaEventCreateWithFlags(&L.copied, cudaEventDisableTiming));
         }
+    DNB_CUDA(cudaEventCreateWithFlags(&net->pulled, cudaEventDisableTiming));
     DNB_CUDA(cudaMalloc((void **)&net->status_dev, 2 * sizeof(int)));
     DNB_CUDA(cudaMemset(net->status_dev, 0, 2 * sizeof(int)));
     DNB_CUDA(cudaMallocHost((void **)&net->status_host, 2 * sizeof(int)));
@@ -490,6 +499,8 @@ extern "C" void dnb_free_network(dnb_network *net)
     if (net->out_host) cudaFreeHost(net->out_host);
     if (net->status_host) cudaFreeHost(net->status_host);
     if (net->graph_exec) cudaGraphExecDestroy(net->graph_exec);
+    for (cudaGraphExec_t e : net->step_exec) if (e) cudaGraphExecDestroy(e);
+    if (net->pulled) cudaEventDestroy(net->pulled);
     cudaFree(net->status_dev);
     for (cudaEvent_t e : net->events) cudaEventDestroy(e);
     for (Layer &L : net->layers) if (L.done) cudaEventDestroy(L.done);
@@ -739,6 +750,11 @@ static void drop_graph(dnb_network *net)
     net->graph_input = nullptr;
     net->graph_stream = nullptr;
     net->eager_runs = 0;
+    for (int k = 0; k < 2; ++k) {
+        if (net->step_exec[k]) cudaGraphExecDestroy(net->step_exec[k]);
+        net->step_exec[k] = nullptr;
+        net->step_runs[k] = 0;
+    }
 }
 
 extern "C" int dnb_network_enable_graph(dnb_network *net, int on)
@@ -808,35 +824,40 @@ static int ensure_second_slot(dnb_network *net)
     return DNB_OK;
 }
 
-// Enqueues one step: images to the device on the upload stream, forward_network_gpu's loop
-// (src/network.c:772-785) on the compute stream, and each [yolo] layer's pull to the host
-// (src/yolo_layer.c:360) on the copy stream while the following layers compute.  Up to two steps may be
-// in flight, so the copies of one step overlap the layers of the next.
-extern "C" int dnb_network_submit(dnb_network *net, const float *input)
+// The batch's images to the device.  Page-locked memory goes straight to the copy engine; ordinary memory, where Darknet's
+// own loaders keep images, is carried over by a few threads (host_copy.cu) and has been read when this returns.
+static int upload(dnb_network *net, const float *input, float *in_dev, cudaStream_t s)
 {
-    if (!net || !input) DNB_FAIL(DNB_EINVAL, "network_submit: null argument");
-    if (!net->weights_loaded) DNB_FAIL(DNB_EINVAL, "network_submit: load_weights has not been called");
-    if (net->submitted - net->collected >= 2) DNB_FAIL(DNB_EINVAL, "network_submit: two steps are already in flight; collect one first");
-    DNB_TRY(check_current_device(net->device, "network_submit"));
-    const int slot = (int)(net->submitted & 1);
-    if (slot == 1) DNB_TRY(ensure_second_slot(net));
-    point_status(net, slot);
-    cudaStream_t s = net->stream, cs = net->copy_stream, hs = net->h2d_stream;
+    const size_t bytes = (size_t)net->batch * net->inputs * sizeof(float);
+    cudaPointerAttributes at;
+    const bool known = cudaPointerGetAttributes(&at, input) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    if (known && at.type != cudaMemoryTypeUnregistered) {
+        DNB_CUDA(cudaMemcpyAsync(in_dev, input, bytes, cudaMemcpyHostToDevice, s));
+        return DNB_OK;
+    }
+    if (!net->copier) net->copier = copy_pool();
+    return upload_staged(net->copier.get(), in_dev, input, bytes, s);
+}
+
+// One step's layers (forward_network_gpu's loop, src/network.c:772-785) on the compute stream, and on the copy stream each
+// [yolo] layer's pull to the host (src/yolo_layer.c:360) while the following layers compute, then the output layer's.
+// alone: no other step is in flight, so there is nobody to wait for and nobody who waits; the streams are joined at the end.
+static int enqueue_step(dnb_network *net, int slot, bool alone)
+{
+    cudaStream_t s = net->stream, cs = net->copy_stream;
     float *in_dev = net->input_slot[slot];
-    // the slot's buffers are free: the step that used them last has been collected
-    DNB_CUDA(cudaMemcpyAsync(in_dev, input, (size_t)net->batch * net->inputs * sizeof(float), cudaMemcpyHostToDevice, hs));
-    DNB_CUDA(cudaEventRecord(net->in_ready[slot], hs));
-    DNB_CUDA(cudaStreamWaitEvent(s, net->in_ready[slot], 0));
+    point_status(net, slot);
     DNB_TRY(prepare_input(net, in_dev, s));
     for (int i = 0; i < (int)net->layers.size(); ++i) {
         Layer &L = net->layers[i];
-        if (L.kind == L_YOLO && net->submitted > 0) DNB_CUDA(cudaStreamWaitEvent(s, L.copied, 0));   // the previous step's pull has read L.out
+        if (L.kind == L_YOLO && !alone && net->submitted > 0) DNB_CUDA(cudaStreamWaitEvent(s, L.copied, 0));   // the previous step's pull has read L.out
         DNB_TRY(forward_layer(net, i, in_dev, s));
         if (L.kind == L_YOLO) {
             DNB_CUDA(cudaEventRecord(L.done, s));
             DNB_CUDA(cudaStreamWaitEvent(cs, L.done, 0));
             DNB_CUDA(cudaMemcpyAsync(L.host_slot[slot], L.out.data, tensor_elems(&L.out) * sizeof(float), cudaMemcpyDeviceToHost, cs));
-            DNB_CUDA(cudaEventRecord(L.copied, cs));
+            if (!alone) DNB_CUDA(cudaEventRecord(L.copied, cs));
         }
     }
     // Every device-to-host copy goes through the copy stream: a copy enqueued on the compute stream would
@@ -844,7 +865,7 @@ extern "C" int dnb_network_submit(dnb_network *net, const float *input)
     Layer &last = net->layers.back();
     if (last.kind != L_YOLO) {   // the output layer is pulled last (src/network.c:786)
         dnb_tensor o{net->out_dev_nchw, DNB_NCHW, DNB_F32, net->batch, last.out_c, last.out_h, last.out_w, 0};
-        if (net->submitted > 0) DNB_CUDA(cudaStreamWaitEvent(s, net->copy_done[slot ^ 1], 0));   // the previous step's pull has read out_dev_nchw
+        if (!alone && net->submitted > 0) DNB_CUDA(cudaStreamWaitEvent(s, net->copy_done[slot ^ 1], 0));   // the previous step's pull has read out_dev_nchw
         DNB_TRY(launch_convert(&last.out, &o, 0, 0, 0, s));
     }
     DNB_CUDA(cudaEventRecord(net->fwd_done[slot], s));
@@ -852,7 +873,33 @@ extern "C" int dnb_network_submit(dnb_network *net, const float *input)
     if (last.kind != L_YOLO)
         DNB_CUDA(cudaMemcpyAsync(net->out_host_slot[slot], net->out_dev_nchw, (size_t)net->batch * net->outputs * sizeof(float), cudaMemcpyDeviceToHost, cs));
     DNB_CUDA(cudaMemcpyAsync(net->status_host + slot, net->status_dev + slot, sizeof(int), cudaMemcpyDeviceToHost, cs));
-    DNB_CUDA(cudaEventRecord(net->copy_done[slot], cs));
+    if (alone) {
+        DNB_CUDA(cudaEventRecord(net->pulled, cs));
+        DNB_CUDA(cudaStreamWaitEvent(s, net->pulled, 0));
+    }
+    return DNB_OK;
+}
+
+static int check_step(dnb_network *net, const float *input, const char *what)
+{
+    if (!net || !input) DNB_FAIL(DNB_EINVAL, "%s: null argument", what);
+    if (!net->weights_loaded) DNB_FAIL(DNB_EINVAL, "%s: load_weights has not been called", what);
+    return check_current_device(net->device, what);
+}
+
+// Enqueues one step.  Up to two steps may be in flight, so the copies of one step overlap the layers of the next.
+extern "C" int dnb_network_submit(dnb_network *net, const float *input)
+{
+    if (net && net->submitted - net->collected >= 2) DNB_FAIL(DNB_EINVAL, "network_submit: two steps are already in flight; collect one first");
+    DNB_TRY(check_step(net, input, "network_submit"));
+    const int slot = (int)(net->submitted & 1);
+    if (slot == 1) DNB_TRY(ensure_second_slot(net));
+    // the slot's buffers are free: the step that used them last has been collected
+    DNB_TRY(upload(net, input, net->input_slot[slot], net->h2d_stream));
+    DNB_CUDA(cudaEventRecord(net->in_ready[slot], net->h2d_stream));
+    DNB_CUDA(cudaStreamWaitEvent(net->stream, net->in_ready[slot], 0));
+    DNB_TRY(enqueue_step(net, slot, false));
+    DNB_CUDA(cudaEventRecord(net->copy_done[slot], net->copy_stream));
     ++net->submitted;
     return DNB_OK;
 }
@@ -880,12 +927,42 @@ extern "C" int dnb_network_collect(dnb_network *net, float **output)
     return DNB_OK;
 }
 
-// network_predict (src/network.c:497-508): one step, start to finish.
+// network_predict (src/network.c:497-508): one step, start to finish.  At small batches the hundred-odd launches of a step
+// cost the host more than the device needs for it, and nothing overlaps them in a blocking call.  So the first step of a
+// slot runs eagerly (plans build their tensor maps and scratch then), the second is captured, copies included, and every
+// later one is the upload and one graph launch.  (YOLOv3-tiny-416, one image: the host spent 100 us on a step's launches.)
 extern "C" int dnb_network_predict(dnb_network *net, const float *input, float **output)
 {
     if (!net || !input || !output) DNB_FAIL(DNB_EINVAL, "network_predict: null argument");
     if (net->submitted != net->collected) DNB_FAIL(DNB_EINVAL, "network_predict: a submitted step has not been collected");
-    DNB_TRY(dnb_network_submit(net, input));
+    DNB_TRY(check_step(net, input, "network_predict"));
+    const int slot = (int)(net->submitted & 1);
+    if (slot == 1) DNB_TRY(ensure_second_slot(net));
+    cudaStream_t s = net->stream;
+    DNB_TRY(upload(net, input, net->input_slot[slot], s));
+    if (net->step_exec[slot]) {
+        DNB_CUDA(cudaGraphLaunch(net->step_exec[slot], s));
+    } else if (!net->step_graphs || net->step_runs[slot]++ == 0) {
+        DNB_TRY(enqueue_step(net, slot, true));
+    } else {
+        cudaGraph_t graph = nullptr;
+        DNB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        const int rc = enqueue_step(net, slot, true);
+        const cudaError_t ce = cudaStreamEndCapture(s, &graph);
+        cudaError_t ie = cudaErrorUnknown;
+        if (rc == DNB_OK && ce == cudaSuccess && graph) ie = cudaGraphInstantiate(&net->step_exec[slot], graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        if (ie == cudaSuccess) {
+            DNB_CUDA(cudaGraphLaunch(net->step_exec[slot], s));
+        } else {                             // something on the path cannot be captured: eager from here on
+            cudaGetLastError();
+            net->step_exec[slot] = nullptr;
+            net->step_graphs = false;
+            DNB_TRY(enqueue_step(net, slot, true));
+        }
+    }
+    DNB_CUDA(cudaEventRecord(net->copy_done[slot], s));
+    ++net->submitted;
     return dnb_network_collect(net, output);
 }
 

@@ -85,3 +85,28 @@ def test_one_tile_per_cluster_integer_sums(shape, ranges, monkeypatch):
     monkeypatch.setenv("DNB_TC_SPLITK", ranges)
     _, got, _ = run_conv(case, dn.MODE_TF32, "nhwc", "nhwc", xnor=True)
     assert np.array_equal(got, whole)
+
+
+def test_predict_from_ordinary_and_page_locked_memory(tmp_path):
+    """The same images from ordinary host memory (carried over chunk by chunk), at an odd address, and from page-locked memory:
+    sizes below one chunk, a few chunks, and more chunks than the staging ring has slots; first, captured and replayed steps."""
+    import numpy as np
+    import torch
+    from darknet_b200 import synth
+    for batch, size in ((1, 32), (1, 450), (24, 512)):
+        cfg = (synth._net(batch, size, size) + synth._conv(16, 3, stride=2) + "\n[avgpool]\n" + synth._conv(10, 1, bn=False, act="linear"))
+        path = str(tmp_path / "n.weights")
+        synth.write_weights(path, synth.seeded_params(cfg, 1))
+        net = dn.Network(cfg, path, dn.MODE_TF32, text=True)
+        x = [synth.seeded_input(cfg, k) for k in range(2)]
+        want = [net.predict(torch.from_numpy(a).pin_memory()).copy() for a in x]
+        assert not np.array_equal(want[0], want[1])
+        odd = np.empty(x[0].size + 1, np.float32)[1:]
+        for k in (0, 1, 1, 0, 0):
+            odd[:] = x[k].reshape(-1)
+            assert np.array_equal(net.predict(x[k]), want[k])
+            assert np.array_equal(net.predict(odd), want[k])
+        net.submit(x[1])
+        net.submit(x[0])
+        assert np.array_equal(net.collect(), want[1]) and np.array_equal(net.collect(), want[0])
+        net.close()
