@@ -103,7 +103,9 @@ struct ConvEpilogue {
     int activation;       // dnb_activation
     int round_tf32;       // round f32 NHWC results to TF32-nearest
     // optional fused residual (the [shortcut] layer that follows the convolution):
-    // out = act2(alpha * act(conv) + beta * residual), residual channels-last, same extents as the output
+    // out = act2(alpha * act(conv) + beta * residual), residual channels-last.  It has the output's extents, or fewer channels
+    // (res_c, a multiple of 64; alpha is 1 then and the others get no addend) and res_stride times the width and height, of
+    // which every res_stride-th pixel is added (shortcut_cpu, src/blas.c:68-92)
     const void *residual;
     int res_cpitch;
     int activation2;
@@ -112,6 +114,8 @@ struct ConvEpilogue {
     // fused [yolo] head (tensor-core kernel only): > 0 = entries per anchor (5 + classes); the logistic is applied to
     // every output channel but the w and h entries of each anchor (ch % entries == 2 or 3), after the activation
     int yolo_entries;
+    int res_c, res_stride, res_h, res_w;   // extents of the residual; res_stride 1 or more
+    int res_out_h, res_out_w;              // the output map the residual belongs to (g may hold a 1x1 layer's pixels in one row)
 };
 
 struct ConvGeom {

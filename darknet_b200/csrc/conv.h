@@ -50,7 +50,7 @@ struct alignas(64) TcArgs {
     CUtensorMap tmx[4];   // activation maps: one per (row parity, column parity) lattice of a strided conv
     CUtensorMap tmw;      // weights [taps][n_pad][c_pad], channels innermost
     CUtensorMap tmy;      // NHWC output, written by TMA stores from the staging rows
-    CUtensorMap tmr;      // fused residual (same extents and box as tmy), loaded tile by tile in the epilogue
+    CUtensorMap tmr;      // fused residual (tmy's box over the pixels that are added), loaded tile by tile in the epilogue
     CUtensorMap tmy_warp; // the same output as 32-pixel boxes: the rows one epilogue warp stages (per-warp stores)
     CUtensorMap tms;      // sign output (int8 channels-last, the next xnor layer's operand): 32-channel boxes of the same pixels as tmy
     int is_bf16;          // operand kind: 0 kind::tf32 on f32 operands, 1 kind::f16 on bf16 operands, 2 kind::i8 on int8 sign tensors (xnor)
@@ -189,7 +189,7 @@ struct dnb_conv_plan {
     int tc_x_cpitch;
     const void *tc_y_ptr;    // NHWC output the store map was built for
     const void *tc_res_ptr;  // fused residual the load map was built for (NULL: none)
-    int tc_res_cpitch;
+    int tc_res_cpitch, tc_res_c, tc_res_stride;
     int tc_y_cpitch, tc_y_dtype;
     // xnor layers in a row (tensor-core kind): the producer's epilogue writes the consumer's int8 operand
     dnb_conv_plan *sign_consumer;   // this plan also fills that plan's x_i8 (set by the network object), or null
@@ -204,6 +204,10 @@ struct dnb_conv_plan {
     long long wait_limit;    // bound of the kernels' waits in cycles (0: the default, about one second)
     int debug_bits;          // OR-ed into the launch block's debug field (dnb_conv_plan_set_diagnostics)
 };
+
+// dnb_conv_shortcut_forward with an addend that may have fewer channels and a map that is a whole multiple of the output's
+bool conv_shortcut_fusable(const dnb_conv_plan *p, const dnb_tensor *add, const dnb_tensor *y, float alpha);
+int conv_shortcut_general(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor *y, float alpha, float beta, int activation2, cudaStream_t s);
 
 // producers of a tensor-core xnor layer's int8 operand (see conv_plan.cu)
 int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int batch, int c, int h, int w);

@@ -579,8 +579,10 @@ static double persistent_us(const TcArgs &a, int k_iters, bool residual)
 }
 
 static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
-                         const void *residual, int res_cpitch, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0)
+                         const ConvEpilogue *res, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0)
 {
+    const void *residual = res ? res->residual : nullptr;   // fused residual, if any
+    const int res_cpitch = res ? res->res_cpitch : 0, res_stride = residual ? res->res_stride : 1, res_c = residual ? res->res_c : 0;
     TcArgs &a = p->tc;
     // A 1x1 convolution (stride 1, no padding) does not care which pixels are neighbours: with Darknet's layout among
     // the outputs, the h x w plane is treated as one row of h*w pixels, so that a tile is a run of up to 128 contiguous
@@ -744,7 +746,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     if (p->tc_split) {
         p->tc_sign_out = sign_out;
         p->tc_x_ptr = x->data; p->tc_x_cpitch = x->cpitch; p->tc_y_ptr = y_nhwc; p->tc_y_cpitch = y_cpitch; p->tc_y_dtype = y_dtype;
-        p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_nchw_out = nchw_out ? 1 : 0;
+        p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_res_c = res_c; p->tc_res_stride = res_stride; p->tc_nchw_out = nchw_out ? 1 : 0;
         return DNB_OK;
     }
     a.g = g;
@@ -770,10 +772,12 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             DNB_TRY(encode_tensor_map(&a.tmy_warp, bf16, 4, y_nhwc, dims, strides, wbox, srb));
         }
         if (residual) {
+            // every res_stride-th pixel of the residual; channels it does not have are the TMA unit's zero fill
             const size_t rpix = (size_t)res_cpitch * out_es;
-            const int r_chan = round_up(g.n, 8) < res_cpitch ? round_up(g.n, 8) : res_cpitch;
+            const int r_chan = round_up(res_c, 8) < res_cpitch ? round_up(res_c, 8) : res_cpitch;
+            const uint64_t rw = res_stride > 1 ? (uint64_t)res->res_w : (uint64_t)g.out_w, rh = res_stride > 1 ? (uint64_t)res->res_h : (uint64_t)g.out_h;
             uint64_t rdims[4] = {(uint64_t)r_chan, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
-            uint64_t rstrides[3] = {rpix, rpix * g.out_w, rpix * g.out_w * g.out_h};
+            uint64_t rstrides[3] = {rpix * res_stride, rpix * rw * res_stride, rpix * rw * rh};
             DNB_TRY(encode_tensor_map(&a.tmr, bf16, 4, const_cast<void *>(residual), rdims, rstrides, box, srb));
         }
     }
@@ -791,6 +795,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     p->tc_y_dtype = y_dtype;
     p->tc_res_ptr = residual;
     p->tc_res_cpitch = res_cpitch;
+    p->tc_res_c = res_c;
+    p->tc_res_stride = res_stride;
     p->tc_nchw_out = nchw_out ? 1 : 0;
     return DNB_OK;
 }
@@ -883,6 +889,8 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         if (p->kernel != K_TC_TF32 && p->kernel != K_TC_BF16)
             DNB_FAIL(DNB_EUNSUPPORTED, "conv + shortcut: only tensor-core plans fuse the residual (this plan is %s)", kKernelNames[p->kernel]);
         ep.residual = res->add->data; ep.res_cpitch = res->add->cpitch; ep.activation2 = res->activation;
+        ep.res_c = res->add->c; ep.res_h = res->add->h; ep.res_w = res->add->w; ep.res_stride = res->add->w / g.out_w;
+        ep.res_out_h = g.out_h; ep.res_out_w = g.out_w;
         ep.alpha = res->alpha; ep.beta = res->beta;
     }
     // f32 channels-last results of a TF32 network feed the next tensor-core layer: round them once here (the tensor
@@ -937,7 +945,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         void *sign_out = (next && nhwc && nhwc == next->signs_of && next->x_i8) ? next->x_i8 : nullptr;
         if (p->tc_x_ptr != xin.data || p->tc_y_ptr != nhwc || p->tc_y_cpitch != (nhwc ? y_cpitch : 0) || !p->status || p->tc_nchw_out != (nchw ? 1 : 0) ||
             p->tc_sign_out != sign_out)
-            DNB_TRY(build_tc_args(p, &xin, nhwc, DNB_F32, nhwc ? y_cpitch : 0, nullptr, 0, nchw != nullptr, sign_out, sign_out ? next->c_pad_i8 : 0));
+            DNB_TRY(build_tc_args(p, &xin, nhwc, DNB_F32, nhwc ? y_cpitch : 0, nullptr, nchw != nullptr, sign_out, sign_out ? next->c_pad_i8 : 0));
         if (p->tc_split) {
             SplitArgs &a = p->sp;
             a.y_nhwc = nhwc; a.y_cpitch = nhwc ? y_cpitch : 0; a.y_nchw = nchw;
@@ -993,8 +1001,9 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         DNB_FAIL(DNB_EINVAL, "conv: a %s plan writes channels-last output as %s", kKernelNames[p->kernel], want == DNB_BF16 ? "bf16" : "f32");
     if (p->tc_x_ptr != xin.data || p->tc_x_cpitch != xin.cpitch || p->tc_y_ptr != y_nhwc || p->tc_y_cpitch != y_cpitch ||
         p->tc_y_dtype != y_dtype || !p->status || p->tc_res_ptr != ep.residual || p->tc_res_cpitch != ep.res_cpitch ||
+        (ep.residual && (p->tc_res_c != ep.res_c || p->tc_res_stride != ep.res_stride)) ||
         p->tc_nchw_out != (y_nchw ? 1 : 0))
-        DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, ep.residual, ep.res_cpitch, y_nchw != nullptr));
+        DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, &ep, y_nchw != nullptr));
     if (p->tc_split) {
         SplitArgs &a = p->sp;
         a.y_nhwc = y_nhwc; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
@@ -1030,9 +1039,29 @@ extern "C" int dnb_conv_shortcut_forward(dnb_conv_plan *p, const dnb_tensor *x, 
         DNB_FAIL(DNB_EINVAL, "conv + shortcut: residual and output must be channels-last in the plan's storage type");
     if (add->n != y->n || add->c != y->c || add->h != y->h || add->w != y->w)
         DNB_FAIL(DNB_EUNSUPPORTED, "conv + shortcut: the residual must have the output's extents (other shapes: dnb_shortcut_forward)");
+    return conv_shortcut_general(p, x, add, y, alpha, beta, activation2, (cudaStream_t)stream);
+}
+
+// What the epilogue covers: a map that is a whole multiple of the output's, and where channels are fewer, whole staged chunks
+// of them.  An addend smaller than the output (scattered with shortcut_cpu's `sample`) has its own pass.
+bool conv_shortcut_fusable(const dnb_conv_plan *p, const dnb_tensor *add, const dnb_tensor *y, float alpha)
+{
+    if (!p || (p->kernel != K_TC_TF32 && p->kernel != K_TC_BF16)) return false;
+    const int want = p->kernel == K_TC_BF16 ? DNB_BF16 : DNB_F32;
+    if (add->layout != DNB_NHWC || y->layout != DNB_NHWC || add->dtype != want || y->dtype != want || add->n != y->n) return false;
+    if (add->c == y->c && add->h == y->h && add->w == y->w) return true;
+    const int stride = add->w / y->w;
+    if (stride < 1 || add->w != stride * y->w || add->h != stride * y->h) return false;
+    return add->c == y->c || (add->c < y->c && add->c % 64 == 0 && alpha == 1.f);
+}
+
+int conv_shortcut_general(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor *y, float alpha, float beta, int activation2, cudaStream_t s)
+{
+    DNB_TRY(check_conv_io(p, x, y, nullptr));
+    DNB_TRY(check_tensor(add, "conv + shortcut residual"));
     Residual r;
     r.add = add; r.alpha = alpha; r.beta = beta; r.activation = activation2;
-    return conv_forward_impl(p, x, y, nullptr, nullptr, (cudaStream_t)stream, &r);
+    return conv_forward_impl(p, x, y, nullptr, nullptr, s, &r);
 }
 
 // Convolution followed by the [yolo] layer that reads it, one launch: forward_yolo_layer_gpu at inference copies

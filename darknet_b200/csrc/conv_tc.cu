@@ -449,6 +449,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             for (int d = 0; d < res_ahead; ++d) request_residual();
         const uint8_t *const res_base = reinterpret_cast<const uint8_t *>(a.ep.residual);
         const size_t res_pix_bytes = (size_t)a.ep.res_cpitch * (OUT_BF16 ? 2 : 4);
+        const int res_c = a.ep.res_c, res_stride = a.ep.res_stride, res_h = a.ep.res_h, res_w = a.ep.res_w;
         const float *const ep_scale = a.ep.scale, *const ep_shift = a.ep.shift;
         const int n_pad = a.n_pad;
         for (int tile = first_tile; tile < total_tiles; tile += grid_stride, ++it) {
@@ -484,9 +485,9 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             const uint4 *res_row = nullptr;
             uint4 res_next[res_direct ? RES_V : 1];
             if (res_direct) {
-                if (pix_ok && !no_res) res_row = reinterpret_cast<const uint4 *>(res_base + (((size_t)b * g.out_h + oh) * g.out_w + ow) * res_pix_bytes + (size_t)nt * bn * (OUT_BF16 ? 2 : 4));
+                if (pix_ok && !no_res) res_row = reinterpret_cast<const uint4 *>(res_base + (((size_t)b * res_h + oh * res_stride) * res_w + ow * res_stride) * res_pix_bytes + (size_t)nt * bn * (OUT_BF16 ? 2 : 4));
 #pragma unroll
-                for (int q = 0; q < RES_V; ++q) res_next[q] = res_row ? __ldg(res_row + q) : make_uint4(0u, 0u, 0u, 0u);
+                for (int q = 0; q < RES_V; ++q) res_next[q] = res_row && nt * bn < res_c ? __ldg(res_row + q) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll 1
             for (int c0 = (dbg & 8) ? bn : 0; c0 < bn; c0 += CPC) {
@@ -507,10 +508,11 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 if (res_direct) {
 #pragma unroll
                     for (int q = 0; q < RES_V; ++q) res[q] = res_next[q];
-                    if (c0 + CPC < bn && res_row) {
+                    if (c0 + CPC < bn && res_row) {   // channels beyond the residual's, whole chunks of them, get no addend
                         const uint4 *nx = res_row + (size_t)(c0 + CPC) * (OUT_BF16 ? 2 : 4) / 16;
+                        const bool has = nt * bn + c0 + CPC < res_c;
 #pragma unroll
-                        for (int q = 0; q < RES_V; ++q) res_next[q] = __ldg(nx + q);
+                        for (int q = 0; q < RES_V; ++q) res_next[q] = has ? __ldg(nx + q) : make_uint4(0u, 0u, 0u, 0u);
                     }
                 }
                 if (res_tiles) {

@@ -40,6 +40,7 @@ struct SplitShared {
     uint32_t tmem_base;
     int abort_flag;
     int pixel[128];            // output pixel ((b * out_h) + oh) * out_w + ow of a tile row, -1 outside the output
+    int res_pixel[128];        // pixel of the fused residual that is added there
     long long nchw[128];       // offset of that pixel in Darknet's layout, filter 0
 };
 
@@ -256,6 +257,10 @@ conv_tc_split_kernel(const __grid_constant__ SplitArgs a)
             const int ow = ow0 + wl, oh = oh0 + hl, b = b0 + bl;
             const bool in = m < a.rows && ow < g.out_w && oh < g.out_h && b < g.batch;
             sh->pixel[m] = in ? (b * g.out_h + oh) * g.out_w + ow : -1;
+            if (a.ep.residual) {   // (g may hold a 1x1 layer's pixels in one row: back to the map's own rows)
+                const int px = in ? sh->pixel[m] : 0, rx = px % a.ep.res_out_w, t2 = px / a.ep.res_out_w, ry = t2 % a.ep.res_out_h, rb = t2 / a.ep.res_out_h;
+                sh->res_pixel[m] = (rb * a.ep.res_h + ry * a.ep.res_stride) * a.ep.res_w + rx * a.ep.res_stride;
+            }
             sh->nchw[m] = in ? (long long)b * g.n * g.out_h * g.out_w + oh * g.out_w + ow : 0;
         }
         grid_dependency_wait();
@@ -312,8 +317,9 @@ conv_tc_split_kernel(const __grid_constant__ SplitArgs a)
                         if (s == split) p[u][s] = *reinterpret_cast<const uint4 *>(part + (size_t)row * pitch + 4 * q);
                         else p[u][s] = ld_cluster16(peer[s] + off);
                     }
-                if (a.ep.residual) {
-                    const size_t at = (size_t)pixel[u] * a.ep.res_cpitch + n_base + 4 * q;
+                res[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (a.ep.residual && n_base + 4 * q < a.ep.res_c) {   // channels beyond the residual's get no addend
+                    const size_t at = (size_t)sh->res_pixel[row] * a.ep.res_cpitch + n_base + 4 * q;
                     if (!OUT_BF16) res[u] = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(a.ep.residual) + at));
                     else { const uint2 r = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const __nv_bfloat16 *>(a.ep.residual) + at)); res[u].x = r.x; res[u].y = r.y; }
                 }

@@ -327,15 +327,16 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
             for (int id : L.inputs)
                 if (net->layers[id].kind == L_YOLO) DNB_FAIL(DNB_EUNSUPPORTED, "cfg: route from a [yolo] layer");
     }
-    // Fuse "convolution, then [shortcut] of equal shape" into the convolution's epilogue when nothing else
-    // reads the convolution's own output: one pass over the activations instead of three.
+    // Fuse "convolution, then [shortcut]" (of equal shape, or as ResNet's stages begin: fewer channels, a larger map) into
+    // the convolution's epilogue when nothing else reads the convolution's own output: one pass over the activations
+    // instead of three.  (ResNet-50, batch 256: the four passes that had other shapes took 0.86 ms of 7.7.)
     // DNB_FUSE_SHORTCUT=0 keeps every layer separate (every layer's output stays readable).
     const bool fuse = getenv("DNB_FUSE_SHORTCUT") ? atoi(getenv("DNB_FUSE_SHORTCUT")) != 0 : true;
     for (int i = 0; fuse && i + 1 < (int)net->layers.size(); ++i) {
         Layer &C = net->layers[i], &S = net->layers[i + 1];
         if (C.kind != L_CONV || !C.plan || (C.plan->kernel != 0 && C.plan->kernel != 1) || S.kind != L_SHORTCUT || S.from == i) continue;
         const Layer &F = net->layers[S.from];
-        if (F.kind == L_YOLO || F.out_c != S.out_c || F.out_h != S.out_h || F.out_w != S.out_w) continue;
+        if (F.kind == L_YOLO || !conv_shortcut_fusable(C.plan, &F.out, &S.out, S.alpha)) continue;
         bool read_elsewhere = false;
         for (int j = i + 2; j < (int)net->layers.size(); ++j) {
             const Layer &L = net->layers[j];
@@ -702,7 +703,7 @@ static int forward_layer(dnb_network *net, int i, const float *device_input, cud
     case L_CONV:
         if (L.fuses_next_shortcut) {
             Layer &S = net->layers[i + 1];
-            return dnb_conv_shortcut_forward(L.plan, &in, &net->layers[S.from].out, &S.out, S.alpha, S.beta, S.activation, s);
+            return conv_shortcut_general(L.plan, &in, &net->layers[S.from].out, &S.out, S.alpha, S.beta, S.activation, s);
         }
         if (L.fuses_next_yolo) {
             Layer &Y = net->layers[i + 1];

@@ -110,3 +110,27 @@ def test_predict_from_ordinary_and_page_locked_memory(tmp_path):
         net.submit(x[0])
         assert np.array_equal(net.collect(), want[1]) and np.array_equal(net.collect(), want[0])
         net.close()
+
+
+@pytest.mark.parametrize("batch,size,what", [(1, 16, "one_tile_per_cluster"), (3, 18, ""), (40, 44, "pair=1")])
+@pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
+def test_shortcut_of_another_shape_in_the_epilogue(batch, size, what, mode, tol, tmp_path):
+    """ResNet's stage boundaries in one launch each: the addend has fewer channels, and twice the map (every second pixel counts).
+    Against the checker layer by layer (four convolutions deep: the kernel tests' tolerances still hold)."""
+    from darknet_b200 import synth
+    from oracle import network as orc
+    cfg = (synth._net(batch, size, size, 16) + synth._conv(64, 3) + synth._conv(512, 3, stride=2, act="linear") + synth._shortcut(-2, "leaky") +
+           synth._conv(64, 1) + synth._conv(192, 1, act="linear") + synth._shortcut(-2, "leaky"))
+    params = synth.seeded_params(cfg, 5)
+    path = str(tmp_path / "s.weights")
+    synth.write_weights(path, params)
+    x = synth.seeded_input(cfg, 6, "normal")
+    want = orc.forward_network(cfg, params, x)
+    net = dn.Network(cfg, path, mode, text=True)
+    net.predict(x)
+    assert what in net.layer_describe(1), net.layer_describe(1)
+    for i in (2, 5):
+        parity(net.layer_output(i), want[i], tol, f"layer {i}")
+    for i in (1, 4):
+        with pytest.raises(dn.DarknetB200Error):
+            net.layer_output(i)          # the convolution has no output of its own
