@@ -26,17 +26,17 @@ struct DirectArgs {
 };
 int launch_conv_direct(const DirectArgs &a, cudaStream_t s);
 
-// ---- conv_stem_tc.cu : first layer (3x3, at most 3 input channels) on tcgen05, im2col rows built by the threads
+// ---- conv_stem_tc.cu : first layer (3x3 over at most 3 channels, 5x5 and 7x7 over RGB) on tcgen05, rows read straight from the image's patch
 struct alignas(64) StemTcArgs {
-    CUtensorMap tmy;                     // channels-last output as [pixel][channel], 32-row boxes
-    int tma_store;                       // rows leave through tmy (else plain stores)
+    CUtensorMap tmy;                     // channels-last output, boxes of 8 x 4 pixels and one row segment
+    int seg_bytes, segs;                 // a pixel's output row in segments of 32, 64 or 128 bytes
     const float *x;                      // f32 input, any layout through element strides
     long long xs_b, xs_c, xs_h, xs_w;
     const float *w;                      // weights [K][npg_pad], K = c*9 (the direct kernel's packing)
     int npg_pad;
     void *y;                             // channels-last output, pitch == n
     int y_dtype, y_cpitch;
-    int n_pad, tmem_cols, tiles, npix;   // filled by the launcher
+    int n_pad, tmem_cols, tiles, tiles_w, tiles_h;   // filled by the launcher
     int *status;
     long long wait_limit;                // bound of every device-side wait, SM clock cycles
     ConvGeom g;

@@ -134,3 +134,19 @@ def test_shortcut_of_another_shape_in_the_epilogue(batch, size, what, mode, tol,
     for i in (1, 4):
         with pytest.raises(dn.DarknetB200Error):
             net.layer_output(i)          # the convolution has no output of its own
+
+
+@pytest.mark.parametrize("name,shape", [
+    ("5x5_s2_one_row_over", dict(b=2, c=3, h=34, w=35, n=48, size=5, stride=2)),
+    ("3x3_s2_gray_narrower_than_a_tile", dict(b=3, c=1, h=3, w=9, n=16, size=3, stride=2)),
+    ("7x7_one_pixel", dict(b=2, c=3, h=1, w=1, n=16, size=7, act="logistic")),
+    ("3x3_two_channels_one_column_over", dict(b=1, c=2, h=33, w=17, n=32, size=3)),
+])
+@pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
+def test_first_layer_patches(name, shape, mode, tol):
+    """8 x 16 pixel tiles whose rows are read from the image's patch.  Tolerance as for the other first-layer cases: operands rounded
+    to TF32 (2^-11), K <= 147 of them, and for BF16 networks an output rounded to 2^-9."""
+    case = conv_case(710, **shape)
+    plan, got, _ = run_conv(case, mode, "nchw", "nhwc")
+    assert plan.kernel == "stem_tc_tf32"
+    parity(got, oracle_conv(case), tol, name)
