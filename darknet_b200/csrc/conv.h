@@ -182,6 +182,7 @@ struct dnb_conv_plan {
     int8_t *x_i8;            // int8 signs of the input, scratch
     size_t x_i8_bytes;
     int *status;             // device status word of the tensor-core kernel
+    bool borrowed;           // the parameter tensors belong to another plan (conv_plan_for_batch)
     bool status_shared;      // the word belongs to a network object (one word for all its plans)
     // tensor-core launch block, rebuilt when the input pointer changes
     dnb::TcArgs tc;
@@ -208,6 +209,8 @@ struct dnb_conv_plan {
 // dnb_conv_shortcut_forward with an addend that may have fewer channels and a map that is a whole multiple of the output's
 bool conv_shortcut_fusable(const dnb_conv_plan *p, const dnb_tensor *add, const dnb_tensor *y, float alpha);
 int conv_shortcut_general(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor *y, float alpha, float beta, int activation2, cudaStream_t s);
+
+dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch);
 
 // producers of a tensor-core xnor layer's int8 operand (see conv_plan.cu)
 int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int batch, int c, int h, int w);

@@ -67,9 +67,28 @@ extern "C" int dnb_conv_plan_create(const dnb_conv_desc *d, int mode, dnb_conv_p
     return DNB_OK;
 }
 
+// The same layer over another batch, with launch blocks and scratch of its own; its parameters are p's, which outlives it and
+// is given no new ones meanwhile.
+dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch)
+{
+    dnb_conv_plan *q = new dnb_conv_plan(*p);
+    q->d.batch = q->g.batch = batch;
+    q->borrowed = true;
+    q->x_nhwc_scratch = nullptr; q->x_bits = nullptr; q->x_i8 = nullptr;
+    q->x_nhwc_bytes = q->x_bits_bytes = q->x_i8_bytes = 0;
+    q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = nullptr;
+    q->sign_consumer = nullptr; q->signs_given = false; q->signs_of = nullptr;
+    return q;
+}
+
 extern "C" void dnb_conv_plan_destroy(dnb_conv_plan *p)
 {
     if (!p) return;
+    if (p->borrowed) {
+        cudaFree(p->x_nhwc_scratch); cudaFree(p->x_bits); cudaFree(p->x_i8);
+        delete p;
+        return;
+    }
     cudaFree(p->scale); cudaFree(p->shift); cudaFree(p->w_tc); cudaFree(p->w_direct); cudaFree(p->w_bits);
     cudaFree(p->w_mean); cudaFree(p->x_nhwc_scratch); cudaFree(p->x_bits); cudaFree(p->w_i8); cudaFree(p->scale_i8); cudaFree(p->x_i8);
     if (!p->status_shared) cudaFree(p->status);

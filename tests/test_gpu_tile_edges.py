@@ -150,3 +150,41 @@ def test_first_layer_patches(name, shape, mode, tol):
     plan, got, _ = run_conv(case, mode, "nchw", "nhwc")
     assert plan.kernel == "stem_tc_tf32"
     parity(got, oracle_conv(case), tol, name)
+
+
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
+def test_steps_in_parts(mode, tmp_path):
+    """A step whose upload and last pull are worth cutting up: first layers by parts, last ones by halves, a [yolo] layer, a
+    [route] and a fused and an unfused [shortcut] inside them.  A pixel's sums run in one order whatever the batch, so the step's results are the
+    whole-batch pass's to the bit: first, captured and replayed steps, one alone and two in flight."""
+    import numpy as np
+    import torch
+    from darknet_b200 import synth
+    yolo = synth._yolo("0,1", "10,14, 23,27", 2, 40)
+    cfg = (synth._net(16, 256, 256) + synth._conv(32, 3) + synth._conv(64, 3, stride=2) + synth._conv(64, 1) + synth._conv(64, 3) +
+           synth._shortcut(-3) + synth._conv(512, 3, stride=2) + synth._conv(90, 1, bn=False, act="linear") + yolo + "\n[route]\nlayers=-4\n" +
+           synth._conv(512, 3) + synth._conv(512, 3) + synth._conv(64, 1) + synth._shortcut(-4) + synth._conv(512, 3) + synth._conv(90, 1, bn=False, act="linear") + yolo)
+    path = str(tmp_path / "p.weights")
+    synth.write_weights(path, synth.seeded_params(cfg, 3))
+    net = dn.Network(cfg, path, mode, text=True)
+    heads = [i for i in range(net.n) if net.layer_type(i) == "yolo"]
+    x = [synth.seeded_input(cfg, k) for k in range(2)]
+    want = []
+    for a in x:
+        net.forward(torch.from_numpy(a).cuda())
+        torch.cuda.synchronize()
+        want.append([net.layer_output(i) for i in [4] + heads])
+    assert len(heads) == 2 and not np.array_equal(want[0][2], want[1][2])
+    pinned = [torch.from_numpy(a).pin_memory() for a in x]
+    for k in (0, 1, 0, 1, 1):
+        for images in (x[k], pinned[k]):
+            assert np.array_equal(net.predict(images).reshape(-1), want[k][2].reshape(-1))
+            assert np.array_equal(net.yolo_output(heads[0]).reshape(-1), want[k][1].reshape(-1))
+            assert np.array_equal(net.layer_output(4), want[k][0])
+    for _ in range(2):
+        net.submit(pinned[1])
+        net.submit(x[0])
+        for k in (1, 0):
+            assert np.array_equal(net.collect().reshape(-1), want[k][2].reshape(-1))
+            assert np.array_equal(net.yolo_output(heads[0]).reshape(-1), want[k][1].reshape(-1))
+    net.close()
