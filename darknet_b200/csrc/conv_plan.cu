@@ -53,7 +53,7 @@ extern "C" int dnb_conv_plan_create(const dnb_conv_desc *d, int mode, dnb_conv_p
     // the tensor-core kernel reads strided inputs through stride*stride lattices and carries maps for strides 1
     // and 2 only; wider strides (none in the benchmark networks) run on the CUDA-core kernel
     if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16) && d->stride > 2) p->kernel = K_DIRECT;
-    // RGB first layers of the TF32 / BF16 modes: tensor cores with thread-built im2col rows (DNB_STEM_TC=0 keeps the FP32 kernel)
+    // RGB first layers of the TF32 / BF16 modes: tensor cores, rows read from the patch in shared memory (DNB_STEM_TC=0 keeps the FP32 kernel)
     const char *stem_env = getenv("DNB_STEM_TC");
     p->stem_tc = p->kernel == K_DIRECT && mode != DNB_MODE_FP32 && !d->xnor && conv_stem_tc_covers(p->g) && !(stem_env && atoi(stem_env) == 0);
     // xnor layers: int8 sign tensors through the tensor cores (kind::i8, exact int32 sums) unless DNB_XNOR_TC=0 asks
