@@ -529,6 +529,48 @@ __global__ void nchw_to_nhwc_kernel(const float *__restrict__ x, T *__restrict__
     }
 }
 
+// The same for outputs whose rows take 16-byte (8-byte for bf16) stores: a tile of 32 channels x 128 pixels per block.  A thread
+// has 16 loads in flight instead of 4, a store instruction writes 4 channels at each of 32 places instead of one: bound by HBM,
+// where the tile above is bound by its loads' latency and its instructions.  The 129-float row pitch keeps both shared-memory
+// phases conflict-free.
+template <typename T>
+__global__ void __launch_bounds__(256)
+nchw_to_nhwc_wide_kernel(const float *__restrict__ x, T *__restrict__ y, int C, int HW, int Cp, int rnd)
+{
+    grid_dependency_wait();
+    launch_dependents_if_small();
+    __shared__ float tile[32][129];
+    const int b = blockIdx.z, c0 = blockIdx.y * 32, p0 = blockIdx.x * 128, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float *src = x + (size_t)b * C * HW;
+    T *dst = y + (size_t)b * HW * Cp;
+    float v[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = c0 + 4 * warp + i, p = p0 + 32 * j + lane;
+            v[i][j] = (c < C && p < HW) ? __ldg(src + (size_t)c * HW + p) : 0.f;
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) tile[4 * warp + i][32 * j + lane] = rnd ? round_tf32(v[i][j]) : v[i][j];
+    __syncthreads();
+    const int q = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int pt = 32 * i + 4 * warp + (lane >> 3), p = p0 + pt, c = c0 + 4 * q;
+        if (p >= HW || c >= Cp) continue;
+        const float a0 = tile[4 * q][pt], a1 = tile[4 * q + 1][pt], a2 = tile[4 * q + 2][pt], a3 = tile[4 * q + 3][pt];
+        if (sizeof(T) == 4) {
+            *reinterpret_cast<float4 *>(dst + (size_t)p * Cp + c) = make_float4(a0, a1, a2, a3);
+        } else {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(a0, a1), hi = __floats2bfloat162_rn(a2, a3);
+            *reinterpret_cast<uint2 *>(dst + (size_t)p * Cp + c) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+        }
+    }
+}
+
 // Channels-last to Darknet's layout: a tile of 128 pixels x 32 channels per block.  Loads are 16-byte
 // (8-byte for bf16) pieces of a pixel's channels, four pixels per warp instruction; stores are 128-byte
 // runs of one channel plane.  The 129-float row pitch keeps both shared-memory phases conflict-free.
@@ -618,7 +660,13 @@ int launch_convert(const dnb_tensor *x, const dnb_tensor *y, int rnd, int yolo_a
     if (x->layout == DNB_NCHW && y->layout == DNB_NHWC) {
         if (x->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "convert: NCHW tensors must be f32");
         dim3 grid((HW + 31) / 32, (y->cpitch + 31) / 32, x->n);
-        if (y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(nchw_to_nhwc_kernel<float>, grid, block, 0, s, (const float *)x->data, (float *)y->data, x->c, HW, y->cpitch, rnd)));
+        // four channels a store where the rows allow it (always between the network's own tensors); an image of a few pixels has
+        // no use for 128-pixel tiles
+        const bool wide = y->cpitch % 4 == 0 && (uintptr_t)y->data % (4 * elem_size(y->dtype)) == 0 && HW > 32;
+        const dim3 wide_grid((HW + 127) / 128, (y->cpitch + 31) / 32, x->n);
+        if (wide && y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(nchw_to_nhwc_wide_kernel<float>, wide_grid, dim3(256), 0, s, (const float *)x->data, (float *)y->data, x->c, HW, y->cpitch, rnd)));
+        else if (wide) DNB_CUDA((launch_overlapped(nchw_to_nhwc_wide_kernel<__nv_bfloat16>, wide_grid, dim3(256), 0, s, (const float *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, y->cpitch, 0)));
+        else if (y->dtype == DNB_F32) DNB_CUDA((launch_overlapped(nchw_to_nhwc_kernel<float>, grid, block, 0, s, (const float *)x->data, (float *)y->data, x->c, HW, y->cpitch, rnd)));
         else DNB_CUDA((launch_overlapped(nchw_to_nhwc_kernel<__nv_bfloat16>, grid, block, 0, s, (const float *)x->data, (__nv_bfloat16 *)y->data, x->c, HW, y->cpitch, 0)));
     } else if (x->layout == DNB_NHWC && y->layout == DNB_NCHW) {
         if (y->dtype != DNB_F32) DNB_FAIL(DNB_EINVAL, "convert: NCHW tensors must be f32");

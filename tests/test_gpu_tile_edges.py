@@ -188,3 +188,16 @@ def test_steps_in_parts(mode, tmp_path):
             assert np.array_equal(net.collect().reshape(-1), want[k][2].reshape(-1))
             assert np.array_equal(net.yolo_output(heads[0]).reshape(-1), want[k][1].reshape(-1))
     net.close()
+
+
+@pytest.mark.parametrize("c,h,w,pitch", [(33, 3, 43, 40), (32, 8, 16, 32), (5, 11, 3, 8), (70, 1, 257, 72), (64, 4, 8, 64)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_to_channels_last_tiles(c, h, w, pitch, dtype):
+    """Darknet's layout to channels-last in tiles of 32 channels x 128 pixels: one pixel or channel over a tile, padding channels
+    (zeroed).  A copy: the values are the input's, rounded to bf16 where that is the storage type."""
+    import torch
+    x = torch.randn(2, c, h, w, generator=torch.Generator().manual_seed(1)).cuda()
+    y = torch.full((2, h, w, pitch), 7.0, dtype=getattr(torch, dtype), device="cuda")
+    dn.convert(dn.as_tensor(x, dn.NCHW), dn.as_tensor(y, dn.NHWC, c))
+    torch.cuda.synchronize()
+    assert torch.equal(y[..., :c], x.permute(0, 2, 3, 1).to(y.dtype)) and not y[..., c:].any()
