@@ -705,6 +705,7 @@ static Part whole(const dnb_network *net) { return Part{0, net->batch, -1}; }
 static dnb_tensor part_of(const dnb_tensor &t, const Part &p)
 {
     dnb_tensor r = t;
+    if (p.piece < 0 || !t.data) return r;
     r.data = (char *)t.data + tensor_elems(&t) / t.n * p.first * elem_size(t.dtype);
     r.n = p.count;
     return r;
@@ -1038,6 +1039,17 @@ static void plan_step(dnb_network *net)
         const double bytes = L.fused_into_prev ? 0 : ((double)L.c * L.h * L.w + (double)L.out_c * L.out_h * L.out_w) * batch * elem_size(net->dtype);
         us[i] = std::max(ops / op_rate, bytes / byte_rate);
     }
+    // every tensor that layer i reads or writes has its part where the kernels' alignment rules want it
+    auto aligned = [&](const dnb_tensor &t, int each) {
+        return !t.data || tensor_elems(&t) / t.n * each * elem_size(t.dtype) % (t.layout == DNB_NHWC ? 128 : 16) == 0;
+    };
+    auto divisible = [&](int i, int each) {
+        const Layer &L = net->layers[i];
+        bool ok = aligned(L.out, each) && (i > 0 ? aligned(net->layers[i - 1].out, each) : aligned(net->input_nhwc, each) && (size_t)each * net->inputs % 4 == 0);
+        if (L.kind == L_SHORTCUT) ok = ok && aligned(net->layers[L.from].out, each);
+        for (int id : L.inputs) ok = ok && aligned(net->layers[id].out, each);
+        return ok;
+    };
     auto cuttable = [&](int i) { return i > 0 && i < n && !net->layers[i - 1].fuses_next_shortcut && !net->layers[i - 1].fuses_next_yolo; };
 
     const double upload_us = (double)batch * net->inputs * sizeof(float) / copy_rate;
@@ -1045,12 +1057,11 @@ static void plan_step(dnb_network *net)
     double best = worth_us;
     for (int k = 2; k <= MAX_PIECES && batch % k == 0; k *= 2) {
         const int each = batch / k;
-        if ((size_t)each * net->inputs % 4) break;   // parts on 16-byte boundaries
         double t = 0;
         for (int i = 0; i < n && t < upload_us; ++i) {
             const Layer &L = net->layers[i];
             const double blocks = std::ceil((double)each * L.out_h * L.out_w / 128) * ((L.out_c + 127) / 128);
-            if (L.kind == L_YOLO || L.kind == L_CONNECTED || blocks < 2.0 * sm_count()) break;
+            if (L.kind == L_YOLO || L.kind == L_CONNECTED || blocks < 2.0 * sm_count() || !divisible(i, each)) break;
             t += us[i];
             const double saved = std::min(t, upload_us) * (1 - 1.0 / k) - part_us * (i + 1) * (k - 1);
             if (cuttable(i + 1) && saved > best) { best = saved; front = i + 1; parts = k; }
@@ -1058,11 +1069,11 @@ static void plan_step(dnb_network *net)
     }
 
     int tail = n;
-    if (net->layers[n - 1].kind == L_YOLO && batch % 8 == 0) {   // halves of whole 16-byte units, whatever the map
+    if (net->layers[n - 1].kind == L_YOLO && batch % 2 == 0) {
         const double pull_us = (double)tensor_elems(&net->layers[n - 1].out) * sizeof(float) / copy_rate;
         double t = 0;
         best = worth_us;
-        for (int i = n - 1; i > front; --i) {
+        for (int i = n - 1; i > front && divisible(i, batch / 2); --i) {
             t += us[i];
             const double saved = std::min(t, pull_us) / 2 - half_us * (n - i);
             if (cuttable(i) && saved > best) { best = saved; tail = i; }

@@ -152,8 +152,9 @@ def test_first_layer_patches(name, shape, mode, tol):
     parity(got, oracle_conv(case), tol, name)
 
 
+@pytest.mark.parametrize("size,filters", [(256, 32), (255, 8)])   # 255 x 255 x 8 in bf16: only whole eighths are 128-byte multiples
 @pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
-def test_steps_in_parts(mode, tmp_path):
+def test_steps_in_parts(size, filters, mode, tmp_path):
     """A step whose upload and last pull are worth cutting up: first layers by parts, last ones by halves, a [yolo] layer, a
     [route] and a fused and an unfused [shortcut] inside them.  A pixel's sums run in one order whatever the batch, so the step's results are the
     whole-batch pass's to the bit: first, captured and replayed steps, one alone and two in flight."""
@@ -161,7 +162,7 @@ def test_steps_in_parts(mode, tmp_path):
     import torch
     from darknet_b200 import synth
     yolo = synth._yolo("0,1", "10,14, 23,27", 2, 40)
-    cfg = (synth._net(16, 256, 256) + synth._conv(32, 3) + synth._conv(64, 3, stride=2) + synth._conv(64, 1) + synth._conv(64, 3) +
+    cfg = (synth._net(16, size, size) + synth._conv(filters, 3) + synth._conv(64, 3, stride=2) + synth._conv(64, 1) + synth._conv(64, 3) +
            synth._shortcut(-3) + synth._conv(512, 3, stride=2) + synth._conv(90, 1, bn=False, act="linear") + yolo + "\n[route]\nlayers=-4\n" +
            synth._conv(512, 3) + synth._conv(512, 3) + synth._conv(64, 1) + synth._shortcut(-4) + synth._conv(512, 3) + synth._conv(90, 1, bn=False, act="linear") + yolo)
     path = str(tmp_path / "p.weights")
