@@ -37,6 +37,7 @@ struct alignas(64) StemTcArgs {
     void *y;                             // channels-last output, pitch == n
     int y_dtype, y_cpitch;
     int n_pad, tmem_cols, tiles, tiles_w, tiles_h;   // filled by the launcher
+    int npix, tma_store;                 // ... of conv_stem_rows.cu: output pixels; rows leave through tmy (else plain stores)
     int *status;
     long long wait_limit;                // bound of every device-side wait, SM clock cycles
     ConvGeom g;
@@ -44,6 +45,10 @@ struct alignas(64) StemTcArgs {
 };
 bool conv_stem_tc_covers(const ConvGeom &g);
 int launch_conv_stem_tc(StemTcArgs a, cudaStream_t s);
+
+// ---- conv_stem_rows.cu : the same layers with their products added in the im2col order (networks with xnor layers)
+bool conv_stem_rows_covers(const ConvGeom &g, int y_dtype);
+int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s);
 
 // ---- conv_tc.cu : implicit GEMM on tcgen05 / TMEM, operands by TMA
 struct alignas(64) TcArgs {
@@ -197,7 +202,7 @@ struct dnb_conv_plan {
     bool signs_given;               // this plan's x_i8 is filled by the layer before it: no sign pass of its own
     const void *signs_of;           // ... as long as the input it is given is this tensor
     void *tc_sign_out;              // the sign output the cached launch block was built for
-    bool keep_k_order;       // sum K in one order whatever the batch: no split (dense layers of a network with xnor layers)
+    bool keep_k_order;       // sum K in one order whatever the batch (dense layers of a network with xnor layers): no split, first layers in the im2col order
     bool tc_split;           // launches use the one-tile-per-cluster kernel and its block below
     dnb::SplitArgs sp;
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout

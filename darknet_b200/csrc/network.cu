@@ -442,7 +442,8 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         }
     }
     // A sign hangs on a sum's last bit.  Where layers are binarised, the dense ones add in the same order at every batch
-    // size (integer sums do not care), so that an image's results do not depend on how many came with it.
+    // size (integer sums do not care), so that an image's results do not depend on how many came with it, and a first layer
+    // on the tensor cores adds in the reference's order of the products.
     bool any_xnor = false;
     for (const Layer &L : net->layers) any_xnor = any_xnor || (L.kind == L_CONV && L.cd.xnor);
     for (Layer &L : net->layers) if (L.plan) L.plan->keep_k_order = any_xnor;
