@@ -21,6 +21,7 @@ struct DirectArgs {
     void *y_nhwc;                        // optional NHWC output
     int y_dtype, y_cpitch;
     float *y_nchw;                       // optional NCHW f32 output
+    int in_order;                        // add the products in the order c, kh, kw whatever the layout (keep_k_order)
     ConvGeom g;
     ConvEpilogue ep;
 };

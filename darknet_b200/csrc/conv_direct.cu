@@ -636,8 +636,10 @@ int launch_conv_direct(const DirectArgs &a, cudaStream_t s)
         else GO(__nv_bfloat16, __nv_bfloat16);                  \
     } while (0)
     // The tiled kernel wants filters to fill its tile: below 17 per group a slab of the general kernel does less padded work.
+    // A 3x3 chunk of its channels-last form holds a few channels of one filter row, so it adds row by row, in steps that depend
+    // on the tile; every other form adds in the order c, kh, kw, which is what a layer with signs behind it has to do.
     if (npg > 16 && (g.size == 1 || g.size == 3) && a.xs_h < (1LL << 28) && a.xs_w < (1LL << 28)) {
-        const bool vec = a.xs_c == 1 && a.xs_w % 4 == 0 && (g.groups == 1 || (g.c / g.groups) % 4 == 0);
+        const bool vec = a.xs_c == 1 && a.xs_w % 4 == 0 && (g.groups == 1 || (g.c / g.groups) % 4 == 0) && !(a.in_order && g.size == 3);
         if (xb && vec) return yb ? launch_gemm<__nv_bfloat16, __nv_bfloat16, true>(a, s) : launch_gemm<__nv_bfloat16, float, true>(a, s);
         if (!xb && vec) return yb ? launch_gemm<float, __nv_bfloat16, true>(a, s) : launch_gemm<float, float, true>(a, s);
         if (!xb) return yb ? launch_gemm<float, __nv_bfloat16, false>(a, s) : launch_gemm<float, float, false>(a, s);

@@ -938,6 +938,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         else { a.xs_w = 1; a.xs_h = g.w; a.xs_c = (long long)g.h * g.w; a.xs_b = (long long)g.c * a.xs_c; }
         a.wpk = p->w_direct; a.npg_pad = p->npg_pad;
         a.y_nhwc = y_nhwc; a.y_dtype = y_dtype; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
+        a.in_order = p->keep_k_order ? 1 : 0;
         a.g = g; a.ep = ep;
         return launch_conv_direct(a, s);
     }

@@ -71,3 +71,24 @@ def test_binarised_darknet19_is_pinned(tmp_path):
         for at in (0, 122):
             assert np.array_equal(small.predict(x[at:at + batch]).reshape(batch, -1), want[at:at + batch])
         small.close()
+
+
+@pytest.mark.parametrize("mode,groups", [(dn.MODE_FP32, 1), (dn.MODE_FP32, 2), (dn.MODE_TF32, 2)])
+@pytest.mark.parametrize("batch", [1, 26])     # small and large tiles of the fp32 GEMM
+def test_dense_layers_on_cuda_cores_add_in_the_reference_order(mode, groups, batch, tmp_path):
+    """A 3x3 layer between others, channels-last: inputs are 1, +2^30 and -2^30 lie at the first and the last tap of a group's
+    first channel, 1 at every product after them.  In the order c, kh, kw the sum is the number of small ones, exactly."""
+    cpg, npg = 24 // groups, 40 // groups
+    cfg = (synth._net(batch, 40, 40) + synth._conv(24, 3, bn=False, act="linear") + synth._conv(40, 3, bn=False, act="linear", groups=groups) +
+           synth._conv(32, 3, xnor=True))
+    params = synth.seeded_params(cfg, 1)
+    params[0].weights[...], params[0].biases[...] = 0, 1
+    w = np.ones((40, cpg * 9), np.float32)
+    w[:, 0], w[:, 1:8], w[:, 8] = 2.0 ** 30, 0, -2.0 ** 30
+    params[1].weights[...], params[1].biases[...] = w.reshape(params[1].weights.shape), 0
+    net = network(cfg, params, tmp_path, mode)
+    assert net.layer_kernel(1) == "direct_fp32" and npg > 16
+    net.predict(np.zeros((batch, 3, 40, 40), np.float32))
+    inner = net.layer_output(1).reshape((batch,) + net.layer_shape(1))[:, :, 1:-1, 1:-1]
+    assert (inner == 9 * (cpg - 1)).all()
+    net.close()
