@@ -24,6 +24,8 @@ namespace dnb {
 // Small enough that the first transfer starts early, large enough that what a transfer costs beside its bytes (5-6 us) stays
 // a fraction of its time on the bus (9 us per 512 KB); larger ones where there are many.
 constexpr size_t COPY_CHUNK = 512 * 1024, COPY_CHUNK_MAX = 1024 * 1024, COPY_MANY = 8 * 1024 * 1024;
+// A slot is as long as the longest chunk, whatever the upload's own: its event then guards the same bytes for every upload, and one
+// of another chunk length cannot reach bytes whose transfer has not been waited for.
 constexpr size_t COPY_RING = 16;
 // Below this a second thread cannot be awake before the copy is over.
 constexpr size_t COPY_ALONE = 1024 * 1024;
@@ -97,7 +99,7 @@ public:
             }
             if (told < open && job->done[told].load(std::memory_order_acquire)) {
                 const size_t at = told * chunk, len = bytes - at < chunk ? bytes - at : chunk, slot = told % COPY_RING;
-                if (err == cudaSuccess) err = cudaMemcpyAsync(dst + at, ring_ + slot * chunk, len, cudaMemcpyHostToDevice, s);
+                if (err == cudaSuccess) err = cudaMemcpyAsync(dst + at, ring_ + slot * COPY_CHUNK_MAX, len, cudaMemcpyHostToDevice, s);
                 if (err == cudaSuccess) err = cudaEventRecord(sent_[slot], s);
                 ++told;
             } else if (!job->one()) {
@@ -127,7 +129,7 @@ private:
                 if (i >= chunks || i >= limit.load(std::memory_order_acquire)) return false;
             } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
             const size_t at = i * chunk, len = bytes - at < chunk ? bytes - at : chunk;
-            copy_streaming(ring + i % COPY_RING * chunk, src + at, len);
+            copy_streaming(ring + i % COPY_RING * COPY_CHUNK_MAX, src + at, len);
             done[i].store(true, std::memory_order_release);
             return true;
         }
