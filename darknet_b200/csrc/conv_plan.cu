@@ -256,6 +256,7 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
             b[n] = biases[n];
         }
     }
+    p->params_set = false;   // until all of the tensors are the new ones
     DNB_TRY(upload(&p->scale, s));
     DNB_TRY(upload(&p->shift, b));
 

@@ -555,6 +555,28 @@ static int set_connected_params(dnb_network *net, Layer &L, int index, const flo
     return dnb_conv_plan_set_params(L.plan, packed.data(), biases, scales, mean, var);
 }
 
+// Before the first parameter tensor is replaced: no step of the network is under way, and nothing that holds the tensors' pointers
+// (captured steps, the plans of parts of a batch) is left, however the replacing ends.
+static int release_params(dnb_network *net)
+{
+    DNB_TRY(check_current_device(net->device, "network parameters"));
+    DNB_CUDA(cudaStreamSynchronize(net->h2d_stream));
+    DNB_CUDA(cudaStreamSynchronize(net->stream));
+    DNB_CUDA(cudaStreamSynchronize(net->copy_stream));
+    drop_graph(net);
+    return DNB_OK;
+}
+
+// ... of all layers: the network predicts again once every one of them has new parameters.
+static int begin_params(dnb_network *net)
+{
+    DNB_TRY(release_params(net));
+    net->weights_loaded = false;
+    net->convs_with_params = 0;
+    for (Layer &L : net->layers) L.params_given = false;
+    return DNB_OK;
+}
+
 static int load_weights_impl(dnb_network *net, const char *path, bool packed)
 {
     if (!net || !path) DNB_FAIL(DNB_EINVAL, "load_weights: null argument");
@@ -574,6 +596,7 @@ static int load_weights_impl(dnb_network *net, const char *path, bool packed)
     // File versions above 1000 store connected-layer matrices as [inputs][outputs] (src/parser.c:1244, 1098-1104);
     // convolutional layers are not affected by the version.
     const bool transposed = hdr[0] > 1000 || hdr[1] > 1000;
+    DNB_TRY(begin_params(net));
     int index = 0;
     for (Layer &L : net->layers) {
         if (L.kind == L_CONV) {
@@ -640,7 +663,6 @@ static int load_weights_impl(dnb_network *net, const char *path, bool packed)
         ++index;
     }
     net->weights_loaded = true;
-    drop_graph(net);   // a captured forward holds the pointers of the parameter tensors just replaced
     return DNB_OK;
 }
 
@@ -658,13 +680,13 @@ extern "C" int dnb_network_set_conv_params(dnb_network *net, int layer, const fl
     Layer &L = net->layers[layer];
     if (L.kind != L_CONV && L.kind != L_CONNECTED) DNB_FAIL(DNB_EINVAL, "set_conv_params: layer %d has no parameters", layer);
     if (net->submitted != net->collected) DNB_FAIL(DNB_EINVAL, "set_conv_params: a submitted step is still in flight; collect it first");
+    DNB_TRY(release_params(net));
     if (L.kind == L_CONNECTED) {
         if (!weights || !biases) DNB_FAIL(DNB_EINVAL, "set_conv_params: null argument");
         DNB_TRY(set_connected_params(net, L, layer, weights, biases, scales, rolling_mean, rolling_variance));
     } else {
         DNB_TRY(dnb_conv_plan_set_params(L.plan, weights, biases, scales, rolling_mean, rolling_variance));
     }
-    drop_graph(net);   // a captured forward holds the pointers of the parameter tensors just replaced
     if (!L.params_given) { L.params_given = true; ++net->convs_with_params; }
     int convs = 0;
     for (const Layer &K : net->layers) convs += K.kind == L_CONV || K.kind == L_CONNECTED;

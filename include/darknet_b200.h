@@ -282,7 +282,9 @@ int dnb_parse_network_cfg_text(const char *cfg_text, int mode, int batch_overrid
  * header forms (32- and 64-bit `seen`, :1234-1241), files whose version marks
  * transposed connected-layer matrices (major or minor above 1000, :1244, :1098-1104) and
  * convolutions declared flipped=1 in the cfg (:1206-1208) are read as the reference
- * reads them. */
+ * reads them.  A step that is in flight is finished first, with the parameters it was submitted with.  If
+ * the file ends early (DNB_EIO) the network holds parameters of both files: it refuses to predict until
+ * a load succeeds. */
 int dnb_load_weights(dnb_network *net, const char *weights_path);
 
 /* load_weights for a file in which every convolution with xnor=1 is stored in the reference's packed-binary layer

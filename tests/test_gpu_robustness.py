@@ -240,3 +240,45 @@ def test_stride_three_runs_on_the_cuda_core_kernel(mode):
     plan.forward(xd, yd)
     torch.cuda.synchronize()
     parity(yt.cpu().numpy(), oracle(x, wt, p, 3, stride=3), 1e-5, "stride 3")
+
+
+@pytest.mark.parametrize("size,batch", [(64, 2), (256, 16)])    # steps in one piece; steps in parts, with plans of their own
+def test_truncated_weights_file_after_predicting(size, batch, tmp_path):
+    """Steps captured with the old parameters are gone before the first tensor is replaced: a load that ends early leaves a network
+    that refuses to run, a good one leaves the new parameters, and a step in flight ends with those it was submitted with."""
+    yolo = synth._yolo("0,1", "10,14, 23,27", 2, 40)
+    cfg = (synth._net(batch, size, size) + synth._conv(32, 3) + synth._conv(64, 3, stride=2) + synth._conv(64, 3) + synth._conv(512, 3, stride=2) +
+           synth._conv(512, 3) + synth._conv(90, 1, bn=False, act="linear") + yolo)
+    paths, want = [str(tmp_path / f"{k}.weights") for k in range(2)], []
+    x = synth.seeded_input(cfg, 1)
+    for k in range(2):
+        synth.write_weights(paths[k], synth.seeded_params(cfg, k))
+        fresh = dn.Network(cfg, paths[k], dn.MODE_TF32, text=True)
+        want.append(fresh.predict(x).copy())
+        fresh.close()
+    assert not np.array_equal(want[0], want[1])
+    whole = open(paths[1], "rb").read()
+    short = str(tmp_path / "short.weights")
+    net = dn.Network(cfg, paths[0], dn.MODE_TF32, text=True)
+    xd = torch.from_numpy(x).cuda()
+    for keep in (len(whole) // 2, len(whole) - 4):
+        for _ in range(5):
+            assert np.array_equal(net.predict(x), want[0])
+        open(short, "wb").write(whole[:keep])
+        with pytest.raises(dn.DarknetB200Error) as e:
+            net.load_weights(short)
+        assert e.value.status == dn.EIO
+        for run in (lambda: net.predict(x), lambda: net.submit(x), lambda: net.forward(xd)):
+            with pytest.raises(dn.DarknetB200Error) as e:
+                run()
+            assert e.value.status == dn.EINVAL
+        net.load_weights(paths[0])
+    with pytest.raises(dn.DarknetB200Error):
+        net.load_weights(str(tmp_path / "missing.weights"))
+    assert np.array_equal(net.predict(x), want[0])       # nothing was touched
+    net.submit(x)
+    net.load_weights(paths[1])
+    assert np.array_equal(net.collect(), want[0])
+    for _ in range(5):
+        assert np.array_equal(net.predict(x), want[1])
+    net.close()
