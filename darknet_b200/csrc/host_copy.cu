@@ -13,6 +13,7 @@
 
 #include <atomic>
 #include <condition_variable>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -56,7 +57,9 @@ public:
     {
         const unsigned cores = std::thread::hardware_concurrency();
         const unsigned n = cores > 4 ? 3 : cores > 1 ? 1 : 0;   // beside the caller
-        for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+        try {
+            for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+        } catch (const std::exception &) {}   // no more threads to be had: those that there are, or the caller alone
     }
     ~CopyPool()
     {
@@ -73,7 +76,7 @@ public:
     int upload(char *dst, const char *src, size_t bytes, cudaStream_t s)
     {
         std::lock_guard<std::mutex> turn(turn_);
-        DNB_TRY(ready());
+        if (!ready()) return NOT_STAGED;
         const size_t chunk = bytes > COPY_MANY ? COPY_CHUNK_MAX : COPY_CHUNK, n = (bytes + chunk - 1) / chunk;
         auto job = std::make_shared<Job>();   // a worker may still look at it after the last chunk is taken
         job->ring = ring_; job->src = src; job->bytes = bytes; job->chunk = chunk; job->chunks = n;
@@ -135,17 +138,22 @@ private:
         }
     };
 
-    // The ring, and its events on the current device.
-    int ready()
+    // The ring, and its events on the current device.  False: they are not to be had.
+    bool ready()
     {
-        if (!ring_) DNB_CUDA(cudaHostAlloc((void **)&ring_, COPY_RING * COPY_CHUNK_MAX, cudaHostAllocPortable));
         int dev = 0;
-        DNB_CUDA(cudaGetDevice(&dev));
-        if (device_ == dev) return DNB_OK;
+        if (!ring_ && cudaHostAlloc((void **)&ring_, COPY_RING * COPY_CHUNK_MAX, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            ring_ = nullptr;
+            return false;
+        }
+        if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (device_ == dev) return true;
         drop_events();
-        for (size_t i = 0; i < COPY_RING; ++i) DNB_CUDA(cudaEventCreateWithFlags(&sent_[i], cudaEventDisableTiming));
+        for (cudaEvent_t &e : sent_)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); return false; }
         device_ = dev;
-        return DNB_OK;
+        return true;
     }
     void drop_events()
     {
@@ -190,16 +198,21 @@ std::shared_ptr<CopyPool> copy_pool()
     static std::weak_ptr<CopyPool> pool;
     std::lock_guard<std::mutex> g(lock);
     std::shared_ptr<CopyPool> p = pool.lock();
-    if (!p) {
+    if (p) return p;
+    try {
         p = std::make_shared<CopyPool>();
-        pool = p;
-    }
+    } catch (const std::exception &) {}
+    pool = p;
     return p;
 }
 
 int upload_staged(CopyPool *pool, void *dst, const void *src, size_t bytes, cudaStream_t s)
 {
-    return pool->upload((char *)dst, (const char *)src, bytes, s);
+    try {
+        return pool ? pool->upload((char *)dst, (const char *)src, bytes, s) : NOT_STAGED;
+    } catch (const std::exception &) {   // of what an upload sets up, before it does anything
+        return NOT_STAGED;
+    }
 }
 
 }  // namespace dnb

@@ -10,11 +10,13 @@ namespace dnb {
 
 class CopyPool;
 
-// The process's pool of copying threads.  It is made by the first holder and joined when the last one lets go.
+// The process's pool of copying threads.  It is made by the first holder and joined when the last one lets go.  Null: no memory.
 std::shared_ptr<CopyPool> copy_pool();
 
 // Uploads `bytes` from pageable `src` to memory `dst` of the current device on `s`.  Returns once src has been read; the
-// transfers are then enqueued.  Safe to call from several threads (callers take turns).
+// transfers are then enqueued.  Safe to call from several threads (callers take turns).  NOT_STAGED: nothing was done, the
+// driver's own path is the one to take (no pool, or no page-locked memory or events to be had).  Throws nothing.
+constexpr int NOT_STAGED = -1;
 int upload_staged(CopyPool *pool, void *dst, const void *src, size_t bytes, cudaStream_t s);
 
 }  // namespace dnb

@@ -912,7 +912,10 @@ static int upload(dnb_network *net, const float *input, float *in_dev, int image
         return DNB_OK;
     }
     if (!net->copier) net->copier = copy_pool();
-    return upload_staged(net->copier.get(), in_dev, input, bytes, s);
+    const int rc = upload_staged(net->copier.get(), in_dev, input, bytes, s);
+    if (rc != NOT_STAGED) return rc;
+    DNB_CUDA(cudaMemcpyAsync(in_dev, input, bytes, cudaMemcpyHostToDevice, s));
+    return DNB_OK;
 }
 
 // The layers up to and including the next [yolo] layer, or the last layer, from layer `begin` on.

@@ -2,8 +2,13 @@
 // at a time, only when somebody asks whether an event has completed, so whatever may still be unread in the staging ring is.
 //   host_copy_check in_turn     small, large, small ... uploads from one thread, nothing waited for in between
 //   host_copy_check threads     the same from two threads, a stream each
+//   host_copy_check no_threads  the system refuses every thread: the caller copies alone
+//   host_copy_check no_memory   there is no page-locked memory: nothing is staged, and the caller is told so
 // Prints "ok" and returns 0, or says what is wrong.
 #include <cuda_runtime.h>
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -22,6 +27,7 @@ struct Event { int pending = 0; };
 struct Op { Event *event; char *dst; const char *src; size_t bytes; };
 std::mutex engine;
 std::deque<Op> queued;
+bool no_threads, no_memory;
 
 void step()   // with the engine's lock
 {
@@ -34,7 +40,18 @@ void step()   // with the engine's lock
 }  // namespace
 
 extern "C" {
-cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned) { *p = malloc(bytes); return cudaSuccess; }
+int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *x)
+{
+    typedef int (*Create)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
+    static const Create create = (Create)dlsym(RTLD_NEXT, "pthread_create");
+    return no_threads ? EAGAIN : create(t, a, f, x);
+}
+cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned)
+{
+    if (no_memory) return cudaErrorMemoryAllocation;
+    *p = malloc(bytes);
+    return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
@@ -135,6 +152,8 @@ int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     std::vector<std::unique_ptr<Upload>> a, b;
+    no_threads = what == "no_threads";
+    no_memory = what == "no_memory";
     {
         std::shared_ptr<dnb::CopyPool> pool = dnb::copy_pool();
         if (what == "in_turn") {
@@ -145,6 +164,13 @@ int main(int argc, char **argv)
             ok[1] = sequence(pool.get(), b, 2, 1000, (cudaStream_t)2);
             t.join();
             if (!ok[0] || !ok[1] || !right(a) || !right(b)) return 1;
+        } else if (what == "no_threads") {
+            if (!sequence(pool.get(), a, 1, 1, nullptr) || !right(a)) return 1;
+        } else if (what == "no_memory") {
+            for (size_t words : SIZES) {
+                Upload u(words, 1);
+                if (dnb::upload_staged(pool.get(), u.dst.data(), u.src.data(), words * 4, nullptr) != dnb::NOT_STAGED || !queued.empty()) return 1;
+            }
         } else {
             printf("what?\n");
             return 2;
