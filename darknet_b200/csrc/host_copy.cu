@@ -1,12 +1,14 @@
 // Uploads of images that live in ordinary (pageable) host memory, which is where Darknet's load_image and network_predict's
 // callers keep them (src/image.c, calloc).  The driver's own path for such memory copies through its staging buffers on one
 // thread, about 15-20 GB/s on this hardware, and the caller waits for it; here a few threads copy chunks into a page-locked
-// ring and each chunk's DMA (55 GB/s) starts as soon as it is there.  The ring belongs to the pool: 16 MB per process, whatever
-// the number and the batch of its networks.  Measured on this path, 2 / 16.6 / 71 MB: driver 211 / 1351 / 6386 us, this 86 /
-// 484 / 1911 us.
+// ring and each chunk's DMA (55 GB/s) starts as soon as it is there.  The ring belongs to the pool: at most 16 MB per process, whatever
+// the number and the batch of its networks, and as many slots of it as the largest batch so far had chunks.  Measured on this
+// path, 2 / 16.6 / 71 MB: driver 211 / 1351 / 6386 us, this 86 / 484 / 1911 us.
 #include "host_copy.h"
 
+#include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 #if defined(__SSE2__)
 #include <emmintrin.h>
 #endif
@@ -27,7 +29,7 @@ namespace dnb {
 constexpr size_t COPY_CHUNK = 512 * 1024, COPY_CHUNK_MAX = 1024 * 1024, COPY_MANY = 8 * 1024 * 1024;
 // A slot is as long as the longest chunk, whatever the upload's own: its event then guards the same bytes for every upload, and one
 // of another chunk length cannot reach bytes whose transfer has not been waited for.
-constexpr size_t COPY_RING = 16;
+constexpr size_t COPY_RING = 16, COPY_GROUP = 2 * COPY_CHUNK_MAX;   // slots; page-locked memory is taken two slots at a time
 // Below this a second thread cannot be awake before the copy is over.
 constexpr size_t COPY_ALONE = 1024 * 1024;
 
@@ -53,14 +55,6 @@ static void copy_streaming(char *dst, const char *src, size_t bytes)
 
 class CopyPool {
 public:
-    CopyPool()
-    {
-        const unsigned cores = std::thread::hardware_concurrency();
-        const unsigned n = cores > 4 ? 3 : cores > 1 ? 1 : 0;   // beside the caller
-        try {
-            for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
-        } catch (const std::exception &) {}   // no more threads to be had: those that there are, or the caller alone
-    }
     ~CopyPool()
     {
         {
@@ -70,19 +64,24 @@ public:
         wake_.notify_all();
         for (std::thread &t : threads_) t.join();
         drop_events();
-        if (ring_) cudaFreeHost(ring_);
+        for (char *g : groups_) {
+            cudaHostUnregister(g);
+            free(g);
+        }
     }
 
-    int upload(char *dst, const char *src, size_t bytes, cudaStream_t s)
+    int upload(char *dst, const char *src, size_t bytes, size_t of, cudaStream_t s)
     {
         std::lock_guard<std::mutex> turn(turn_);
-        if (!ready()) return NOT_STAGED;
         const size_t chunk = bytes > COPY_MANY ? COPY_CHUNK_MAX : COPY_CHUNK, n = (bytes + chunk - 1) / chunk;
+        const size_t step = (of + chunk - 1) / chunk, depth = grow(step < COPY_RING ? step : COPY_RING);
+        if (!depth || !ready()) return NOT_STAGED;
+        const bool helped = bytes > COPY_ALONE && start_threads();
         auto job = std::make_shared<Job>();   // a worker may still look at it after the last chunk is taken
-        job->ring = ring_; job->src = src; job->bytes = bytes; job->chunk = chunk; job->chunks = n;
+        for (size_t i = 0; i < depth; ++i) job->slot[i] = slot_[i];
+        job->depth = depth; job->src = src; job->bytes = bytes; job->chunk = chunk; job->chunks = n;
         job->done.reset(new std::atomic<bool>[n]);
         for (size_t i = 0; i < n; ++i) job->done[i].store(false, std::memory_order_relaxed);
-        const bool helped = bytes > COPY_ALONE && !threads_.empty();
         if (helped) {
             {
                 std::lock_guard<std::mutex> g(lock_);
@@ -94,15 +93,15 @@ public:
         size_t told = 0, open = 0;             // chunks enqueued; chunks that may be copied (their ring slots are free)
         cudaError_t err = cudaSuccess;
         while (told < n) {
-            while (open < n && open < told + COPY_RING) {   // a slot is free when its last transfer has left it
-                const cudaError_t q = cudaEventQuery(sent_[open % COPY_RING]);
+            while (open < n && open < told + depth) {   // a slot is free when its last transfer has left it
+                const cudaError_t q = cudaEventQuery(sent_[open % depth]);
                 if (q == cudaErrorNotReady) break;
                 if (q != cudaSuccess) err = q;
                 job->limit.store(++open, std::memory_order_release);
             }
             if (told < open && job->done[told].load(std::memory_order_acquire)) {
-                const size_t at = told * chunk, len = bytes - at < chunk ? bytes - at : chunk, slot = told % COPY_RING;
-                if (err == cudaSuccess) err = cudaMemcpyAsync(dst + at, ring_ + slot * COPY_CHUNK_MAX, len, cudaMemcpyHostToDevice, s);
+                const size_t at = told * chunk, len = bytes - at < chunk ? bytes - at : chunk, slot = told % depth;
+                if (err == cudaSuccess) err = cudaMemcpyAsync(dst + at, slot_[slot], len, cudaMemcpyHostToDevice, s);
                 if (err == cudaSuccess) err = cudaEventRecord(sent_[slot], s);
                 ++told;
             } else if (!job->one()) {
@@ -119,9 +118,9 @@ public:
 
 private:
     struct Job {
-        char *ring = nullptr;
+        char *slot[COPY_RING] = {};
         const char *src = nullptr;
-        size_t bytes = 0, chunk = 0, chunks = 0;
+        size_t depth = 0, bytes = 0, chunk = 0, chunks = 0;
         std::atomic<size_t> next{0}, limit{0};
         std::unique_ptr<std::atomic<bool>[]> done;
         bool taken() const { return next.load(std::memory_order_relaxed) >= chunks; }
@@ -132,21 +131,49 @@ private:
                 if (i >= chunks || i >= limit.load(std::memory_order_acquire)) return false;
             } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
             const size_t at = i * chunk, len = bytes - at < chunk ? bytes - at : chunk;
-            copy_streaming(ring + i % COPY_RING * COPY_CHUNK_MAX, src + at, len);
+            copy_streaming(slot[i % depth], src + at, len);
             done[i].store(true, std::memory_order_release);
             return true;
         }
     };
 
-    // The ring, and its events on the current device.  False: they are not to be had.
+    // Slots of the ring up to `want`, as many as there are to be had.  Pages of 2 MB where the system has them: taking and
+    // locking 16 MB takes 3.7 ms with them, 13 to 20 with 4 KB pages.
+    size_t grow(size_t want)
+    {
+        while (slots_ < want && !full_) {
+            groups_.reserve(COPY_RING * COPY_CHUNK_MAX / COPY_GROUP);
+            char *g = (char *)aligned_alloc(COPY_GROUP, COPY_GROUP);
+            if (g) madvise(g, COPY_GROUP, MADV_HUGEPAGE);
+            if (!g || cudaHostRegister(g, COPY_GROUP, cudaHostRegisterPortable) != cudaSuccess) {
+                cudaGetLastError();
+                free(g);
+                full_ = true;                  // no more page-locked memory: go on with what there is
+                break;
+            }
+            groups_.push_back(g);
+            for (size_t at = 0; at < COPY_GROUP; at += COPY_CHUNK_MAX) slot_[slots_++] = g + at;
+        }
+        return slots_ < want ? slots_ : want;
+    }
+
+    bool start_threads()
+    {
+        if (threads_.empty() && !alone_) {
+            const unsigned cores = std::thread::hardware_concurrency();
+            const unsigned n = cores > 4 ? 3 : cores > 1 ? 1 : 0;   // beside the caller
+            try {
+                for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { work(); });
+            } catch (const std::exception &) {}                     // no more threads to be had: those that there are, or the caller alone
+            alone_ = threads_.empty();
+        }
+        return !alone_;
+    }
+
+    // The ring's events, on the current device.
     bool ready()
     {
         int dev = 0;
-        if (!ring_ && cudaHostAlloc((void **)&ring_, COPY_RING * COPY_CHUNK_MAX, cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            ring_ = nullptr;
-            return false;
-        }
         if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return false; }
         if (device_ == dev) return true;
         drop_events();
@@ -181,7 +208,10 @@ private:
         }
     }
 
-    char *ring_ = nullptr;
+    std::vector<char *> groups_;   // the ring's memory
+    char *slot_[COPY_RING] = {};
+    size_t slots_ = 0;
+    bool full_ = false, alone_ = false;
     cudaEvent_t sent_[COPY_RING] = {};
     int device_ = -1;
     std::mutex turn_, lock_;
@@ -192,13 +222,13 @@ private:
     std::vector<std::thread> threads_;
 };
 
-std::shared_ptr<CopyPool> copy_pool()
+std::shared_ptr<CopyPool> copy_pool(bool make)
 {
     static std::mutex lock;
     static std::weak_ptr<CopyPool> pool;
     std::lock_guard<std::mutex> g(lock);
     std::shared_ptr<CopyPool> p = pool.lock();
-    if (p) return p;
+    if (p || !make) return p;
     try {
         p = std::make_shared<CopyPool>();
     } catch (const std::exception &) {}
@@ -206,10 +236,10 @@ std::shared_ptr<CopyPool> copy_pool()
     return p;
 }
 
-int upload_staged(CopyPool *pool, void *dst, const void *src, size_t bytes, cudaStream_t s)
+int upload_staged(CopyPool *pool, void *dst, const void *src, size_t bytes, size_t of, cudaStream_t s)
 {
     try {
-        return pool ? pool->upload((char *)dst, (const char *)src, bytes, s) : NOT_STAGED;
+        return pool ? pool->upload((char *)dst, (const char *)src, bytes, of, s) : NOT_STAGED;
     } catch (const std::exception &) {   // of what an upload sets up, before it does anything
         return NOT_STAGED;
     }

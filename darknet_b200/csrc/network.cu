@@ -24,6 +24,7 @@ namespace {
 enum LayerKind { L_CONV, L_MAXPOOL, L_UPSAMPLE, L_SHORTCUT, L_ROUTE, L_YOLO, L_AVGPOOL, L_SOFTMAX, L_CONNECTED };
 const char *const kKindNames[] = {"convolutional", "maxpool", "upsample", "shortcut", "route", "yolo", "avgpool", "softmax", "connected"};
 
+constexpr unsigned long long STAGED_FROM = 2;   // steps on the driver's path for ordinary host memory, see upload
 constexpr int MAX_PIECES = 8;   // parts the batch is cut into at most, see plan_step
 
 // `count` images of the batch from `first` on; piece < 0 is the whole batch.
@@ -177,7 +178,7 @@ struct dnb_network {
     cudaEvent_t piece_in[MAX_PIECES] = {};   // upload stream: a piece's images are on the device
     std::vector<cudaGraphExec_t> item_exec[2];   // the schedule's items as graphs, per slot
     cudaEvent_t pulled = nullptr;         // copy stream: every result copy of a blocking step is enqueued
-    std::shared_ptr<CopyPool> copier;     // made with the first input in pageable memory
+    std::shared_ptr<CopyPool> copier;     // held once an input in pageable memory asked for it
 };
 
 static void drop_graph(dnb_network *net);
@@ -900,7 +901,9 @@ static int ensure_second_slot(dnb_network *net)
 }
 
 // The batch's images to the device.  Page-locked memory goes straight to the copy engine; ordinary memory, where Darknet's
-// own loaders keep images, is carried over by a few threads (host_copy.cu) and has been read when this returns.
+// own loaders keep images, is carried over by a few threads (host_copy.cu) and has been read when this returns.  A network's first
+// steps make no ring of page-locked memory of their own, but use the process's if there is one: it takes as long as a first step
+// (ResNet-50, one image, alone: first call 14.2 ms with a ring made in it, 1.0 without), and only a program that goes on gains by it.
 static int upload(dnb_network *net, const float *input, float *in_dev, int images, cudaStream_t s)
 {
     const size_t bytes = (size_t)images * net->inputs * sizeof(float);
@@ -911,8 +914,8 @@ static int upload(dnb_network *net, const float *input, float *in_dev, int image
         DNB_CUDA(cudaMemcpyAsync(in_dev, input, bytes, cudaMemcpyHostToDevice, s));
         return DNB_OK;
     }
-    if (!net->copier) net->copier = copy_pool();
-    const int rc = upload_staged(net->copier.get(), in_dev, input, bytes, s);
+    if (!net->copier) net->copier = copy_pool(net->submitted >= STAGED_FROM);
+    const int rc = upload_staged(net->copier.get(), in_dev, input, bytes, (size_t)net->batch * net->inputs * sizeof(float), s);
     if (rc != NOT_STAGED) return rc;
     DNB_CUDA(cudaMemcpyAsync(in_dev, input, bytes, cudaMemcpyHostToDevice, s));
     return DNB_OK;

@@ -4,6 +4,8 @@
 //   host_copy_check threads     the same from two threads, a stream each
 //   host_copy_check no_threads  the system refuses every thread: the caller copies alone
 //   host_copy_check no_memory   there is no page-locked memory: nothing is staged, and the caller is told so
+//   host_copy_check little_memory   there are two slots of it
+//   host_copy_check small       a few small images: little page-locked memory is taken, and no thread started
 // Prints "ok" and returns 0, or says what is wrong.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -27,7 +29,9 @@ struct Event { int pending = 0; };
 struct Op { Event *event; char *dst; const char *src; size_t bytes; };
 std::mutex engine;
 std::deque<Op> queued;
-bool no_threads, no_memory;
+bool no_threads;
+int threads_asked;
+size_t locked, may_lock = 16 << 20;   // bytes of page-locked memory: taken, and to be had
 
 void step()   // with the engine's lock
 {
@@ -44,15 +48,11 @@ int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), vo
 {
     typedef int (*Create)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
     static const Create create = (Create)dlsym(RTLD_NEXT, "pthread_create");
+    ++threads_asked;
     return no_threads ? EAGAIN : create(t, a, f, x);
 }
-cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned)
-{
-    if (no_memory) return cudaErrorMemoryAllocation;
-    *p = malloc(bytes);
-    return cudaSuccess;
-}
-cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
+cudaError_t cudaHostRegister(void *, size_t bytes, unsigned) { return (locked += bytes) > may_lock ? cudaErrorMemoryAllocation : cudaSuccess; }
+cudaError_t cudaHostUnregister(void *) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "error"; }
@@ -112,7 +112,7 @@ struct Upload {
     }
     bool run(dnb::CopyPool *pool, cudaStream_t s)
     {
-        const int rc = dnb::upload_staged(pool, dst.data(), src.data(), src.size() * 4, s);
+        const int rc = dnb::upload_staged(pool, dst.data(), src.data(), src.size() * 4, src.size() * 4, s);
         std::fill(src.begin(), src.end(), 0u);   // the images have been read when the call returns
         if (rc) printf("upload failed with %d: %s\n", rc, dnb::get_error());
         return rc == 0;
@@ -153,9 +153,10 @@ int main(int argc, char **argv)
     const std::string what = argc > 1 ? argv[1] : "";
     std::vector<std::unique_ptr<Upload>> a, b;
     no_threads = what == "no_threads";
-    no_memory = what == "no_memory";
+    if (what == "no_memory") may_lock = 0;
+    if (what == "little_memory") may_lock = 3 << 20;
     {
-        std::shared_ptr<dnb::CopyPool> pool = dnb::copy_pool();
+        std::shared_ptr<dnb::CopyPool> pool = dnb::copy_pool(true);
         if (what == "in_turn") {
             if (!sequence(pool.get(), a, 2, 1, nullptr) || !right(a)) return 1;
         } else if (what == "threads") {
@@ -164,12 +165,19 @@ int main(int argc, char **argv)
             ok[1] = sequence(pool.get(), b, 2, 1000, (cudaStream_t)2);
             t.join();
             if (!ok[0] || !ok[1] || !right(a) || !right(b)) return 1;
-        } else if (what == "no_threads") {
+        } else if (what == "small") {
+            no_threads = true;   // refused, and counted
+            for (unsigned k = 0; k < 5; ++k) {
+                a.emplace_back(new Upload(196608, k));   // 256 x 256 pixels
+                if (!a.back()->run(pool.get(), nullptr)) return 1;
+            }
+            if (!right(a) || locked > 2 << 20 || threads_asked) return 1;
+        } else if (what == "no_threads" || what == "little_memory") {
             if (!sequence(pool.get(), a, 1, 1, nullptr) || !right(a)) return 1;
         } else if (what == "no_memory") {
             for (size_t words : SIZES) {
                 Upload u(words, 1);
-                if (dnb::upload_staged(pool.get(), u.dst.data(), u.src.data(), words * 4, nullptr) != dnb::NOT_STAGED || !queued.empty()) return 1;
+                if (dnb::upload_staged(pool.get(), u.dst.data(), u.src.data(), words * 4, words * 4, nullptr) != dnb::NOT_STAGED || !queued.empty()) return 1;
             }
         } else {
             printf("what?\n");

@@ -26,6 +26,10 @@ def test_ring_slots_are_rewritten_only_after_their_transfers(check, how):
     check(how)
 
 
-@pytest.mark.parametrize("how", ["no_threads", "no_memory"])
+@pytest.mark.parametrize("how", ["no_threads", "no_memory", "little_memory"])
 def test_what_cannot_be_had_is_done_without(check, how):
     check(how)
+
+
+def test_small_images_take_little(check):
+    check("small")
