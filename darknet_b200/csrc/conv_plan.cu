@@ -351,18 +351,22 @@ struct SplitPlan {
     double cost = 1e300;   // microseconds, estimated
 };
 
+struct PixelBox { int wt = 1, ht = 1, bt = 1, tiles = 1; };
+
 // The box of at most 128 pixels that covers the output with the fewest tiles; widest rows among equals.
-void split_pixel_tile(const ConvGeom &g, int *wt, int *ht, int *bt, int *ptiles)
+PixelBox split_pixel_tile(const ConvGeom &g)
 {
+    PixelBox box;
     long long best = 0;
     for (int w = 1; w <= 128 && w <= g.out_w; ++w)
         for (int h = 1; w * h <= 128 && h <= g.out_h; ++h) {
             int b = 128 / (w * h);
             if (b > g.batch) b = g.batch;
             const long long n = (long long)((g.out_w + w - 1) / w) * ((g.out_h + h - 1) / h) * ((g.batch + b - 1) / b);
-            if (!best || n < best || (n == best && w > *wt)) { best = n; *wt = w; *ht = h; *bt = b; }
+            if (!best || n < best || (n == best && w > box.wt)) { best = n; box.wt = w; box.ht = h; box.bt = b; }
         }
-    *ptiles = (int)best;
+    box.tiles = (int)best;
+    return box;
 }
 
 // Microseconds that one K iteration (128 pixels x bn filters x 128 bytes of channels) takes a CTA that has its SM to itself,
@@ -378,11 +382,9 @@ struct SplitQuery {
 // to a sweep over the 3x3 and 1x1 layers of YOLOv3 and ResNet-50 at 1 to 8 images; most choices come out within 15 % of what
 // they take): launch and first loads; K iterations; dump of the accumulator (4 ns a column); partial sums through distributed
 // shared memory (20 ns per KB); stores and residual, by the number of 16-byte pieces a thread finishes.
-SplitPlan split_of(const SplitQuery &q, const ConvGeom &g, int pair, int S)
+SplitPlan split_of(const SplitQuery &q, const PixelBox &box, int pair, int S)
 {
     SplitPlan best;
-    int wt = 1, ht = 1, bt = 1, pt = 1;
-    split_pixel_tile(g, &wt, &ht, &bt, &pt);
     const int sms = sm_count(), a_bytes = 128 * q.row_bytes, cluster = pair ? 2 * S : S;
     const int resident = conv_tc_split_resident(pair, cluster);   // clusters live inside one GPC: SMs may be left over
     for (int opt = 0; opt < 3 && resident > 0; ++opt) {
@@ -393,7 +395,7 @@ SplitPlan split_of(const SplitQuery &q, const ConvGeom &g, int pair, int S)
             bn = q.n_pad;
         }
         const int n_tiles = (q.n_pad + bn - 1) / bn;
-        const long long tiles = (long long)(pair ? (pt + 1) / 2 : pt) * n_tiles;
+        const long long tiles = (long long)(pair ? (box.tiles + 1) / 2 : box.tiles) * n_tiles;
         if (tiles > 4LL * sms) continue;
         const int b_bytes = round_up((pair ? bn / 2 : bn) * q.row_bytes, 1024), per = (q.k_iters + S - 1) / S;
         // the whole K range of a CTA in the ring if it fits: the deepest ring is what hides the loads' latency
@@ -406,7 +408,7 @@ SplitPlan split_of(const SplitQuery &q, const ConvGeom &g, int pair, int S)
         const double finish = 0.004 * bn + 0.02 * remote_kb + pieces * (q.residual ? 0.32 : 0.22) + (pair ? 1.3 : 0.0);
         const double cost = 4.5 + rounds * (per * iter_us(pair, bn) + finish) + (rounds - 1) * 4.0;
         if (cost < best.cost) {
-            best.pair = pair; best.bn = bn; best.splits = S; best.stages = stages; best.wt = wt; best.ht = ht; best.bt = bt; best.ptiles = pt; best.cost = cost;
+            best.pair = pair; best.bn = bn; best.splits = S; best.stages = stages; best.wt = box.wt; best.ht = box.ht; best.bt = box.bt; best.ptiles = box.tiles; best.cost = cost;
         }
     }
     return best;
@@ -418,17 +420,20 @@ SplitPlan choose_split(const SplitQuery &q, const ConvGeom &g, int only_s, bool 
 {
     SplitPlan best[2];
     double score[2] = {1e300, 1e300};
+    const PixelBox box = split_pixel_tile(g);   // once: it is the same for every split, and a network has a hundred layers to plan
+    const bool with_two = images == 1 && only_s <= 1;
+    ConvGeom two = g;
+    if (two.batch == 1 && two.h == 1 && q.k_iters && g.size == 1) two.w = two.out_w = 2 * g.out_w;   // flattened pixels
+    else two.batch = 2;
+    const PixelBox box_two = with_two ? split_pixel_tile(two) : box;
     for (int S = only_s > 1 ? only_s : 2; S <= (only_s > 1 ? only_s : 8); ++S) {
         if (S > q.k_iters || (only_s <= 1 && q.k_iters / S < 3)) break;
         for (int pair = 0; pair < (q.pair_ok ? 2 : 1); ++pair) {
-            const SplitPlan sp = split_of(q, g, pair, S);
+            const SplitPlan sp = split_of(q, box, pair, S);
             if (!sp.splits) continue;
             double sc = sp.cost;
-            if (images == 1 && only_s <= 1) {
-                ConvGeom two = g;
-                if (two.batch == 1 && two.h == 1 && q.k_iters && g.size == 1) two.w = two.out_w = 2 * g.out_w;   // flattened pixels
-                else two.batch = 2;
-                const SplitPlan t = split_of(q, two, pair, S);
+            if (with_two) {
+                const SplitPlan t = split_of(q, box_two, pair, S);
                 sc += t.splits ? 0.5 * t.cost : 1e6;
             }
             if (sc < score[pair]) { score[pair] = sc; best[pair] = sp; }
