@@ -51,6 +51,13 @@ int launch_conv_stem_tc(StemTcArgs a, cudaStream_t s);
 bool conv_stem_rows_covers(const ConvGeom &g, int y_dtype);
 int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s);
 
+// The shared memory that a CTA with `cols` columns of TMEM asks for: its `bytes`, or its columns' share of the SM's (228 KB, 1 KB of
+// it reserved per CTA, against 512 columns) if that is more.  Whatever CTAs then meet on an SM, of this kernel or another one,
+// of this stream or another one, their columns fit together and no tcgen05.alloc ever waits.  One that waits can wait
+// for good: a CTA of a cluster keeps its columns until its peers are done, so clusters of two networks on two streams, each holding
+// what a peer of the other waits for on another SM, would never end, and no bounded wait covers an allocation.
+size_t tmem_smem(size_t bytes, int cols);
+
 // ---- conv_tc.cu : implicit GEMM on tcgen05 / TMEM, operands by TMA
 struct alignas(64) TcArgs {
     CUtensorMap tmx[4];   // activation maps: one per (row parity, column parity) lattice of a strided conv

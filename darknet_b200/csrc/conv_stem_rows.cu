@@ -498,17 +498,13 @@ bool conv_stem_rows_covers(const ConvGeom &g, int y_dtype)
 template <typename K>
 static int launch_rows(K kern, size_t smem, int most, const StemTcArgs &a, cudaStream_t s)
 {
-    // TMEM holds 512 columns per SM: never more CTAs on an SM than can all hold their accumulators at once.  The request is
-    // padded so that one more would not fit.
-    const int lim = 512 / a.tmem_cols;
+    smem = tmem_smem(smem, a.tmem_cols);
     const size_t sm_bytes = 228 * 1024, reserved = 1024;   // per SM, and per resident CTA
-    if ((smem + reserved) * (lim + 1) <= sm_bytes) smem = sm_bytes / (lim + 1) - reserved + 16;
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // all of the SM's configurable memory as shared memory, so that several CTAs are resident
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     int per_sm = (int)(sm_bytes / (smem + reserved));
     if (per_sm > most) per_sm = most;   // the kernel's register budget (__launch_bounds__)
-    if (per_sm > lim) per_sm = lim;
     if (per_sm < 1) DNB_FAIL(DNB_ECUDA, "first-layer kernel: %zu bytes of shared memory do not fit", smem);
     long long grid = (long long)sm_count() * per_sm;
     if (grid > a.tiles) grid = a.tiles;

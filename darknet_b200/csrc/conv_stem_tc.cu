@@ -333,17 +333,13 @@ static int launch_stem(const StemTcArgs &a, cudaStream_t s)
     using P = StemPatch<KS, S>;
     auto kern = conv_stem_tc_kernel<KS, S, ACT, OBF>;
     size_t smem = (size_t)a.segs * 128 * a.seg_bytes + (size_t)P::PAIRS * a.n_pad * 32 + 2 * sizeof(float4) * P::CELLS + 2 * sizeof(float) * a.n_pad + sizeof(StemShared) + 16;
-    // TMEM holds 512 columns per SM: never more CTAs on an SM than can all hold their accumulators at once.  The request is
-    // padded so that one more would not fit.
-    const int lim = 512 / a.tmem_cols;
+    smem = tmem_smem(smem, a.tmem_cols);
     const size_t sm_bytes = 228 * 1024, reserved = 1024;   // per SM, and per resident CTA
-    if ((smem + reserved) * (lim + 1) <= sm_bytes) smem = sm_bytes / (lim + 1) - reserved + 16;
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // all of the SM's configurable memory as shared memory, so that several CTAs are resident
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     int per_sm = (int)(sm_bytes / (smem + reserved));
     if (per_sm > stem_ctas(KS)) per_sm = stem_ctas(KS);   // the kernel's register budget (__launch_bounds__)
-    if (per_sm > lim) per_sm = lim;
     if (per_sm < 1) DNB_FAIL(DNB_ECUDA, "first-layer kernel: %zu bytes of shared memory do not fit", smem);
     long long grid = (long long)sm_count() * per_sm;
     if (grid > a.tiles) grid = a.tiles;

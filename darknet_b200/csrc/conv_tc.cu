@@ -698,6 +698,12 @@ size_t conv_tc_smem_bytes(const TcArgs &a)
     return (size_t)a.stages * (a.a_bytes + a.b_bytes) + conv_tc_fixed_smem(a.store_row_bytes, a.bn, a.stage_bufs);
 }
 
+size_t tmem_smem(size_t bytes, int cols)
+{
+    const size_t share = (size_t)cols * (228 * 1024 / 512) - 1024;
+    return bytes > share ? bytes : share;
+}
+
 int conv_tc_max_smem()
 {
     int dev = 0, v = 0;
@@ -770,7 +776,7 @@ static int launch_one(K kern, const TcArgs &a, size_t smem, cudaStream_t s)
 
 int launch_conv_tc(const TcArgs &a, cudaStream_t s)
 {
-    const size_t smem = conv_tc_smem_bytes(a);
+    const size_t smem = tmem_smem(conv_tc_smem_bytes(a), a.tmem_cols);
     const bool obf = a.is_bf16 == 1, i8 = a.is_bf16 == 2;   // int8 operands write f32 output
     const int cpc = a.store_row_bytes / (obf ? 2 : 4);
     if (cpc != 16 && cpc != 32 && cpc != 64) DNB_FAIL(DNB_EINVAL, "conv_tc: staged row of %d bytes", a.store_row_bytes);

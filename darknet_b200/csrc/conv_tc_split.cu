@@ -411,15 +411,11 @@ size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes)
 {
     size_t work = (size_t)stages * stage_bytes, dump = (size_t)128 * (bn + 4) * 4;
     if (dump > work) work = dump;
-    // No more CTAs on an SM than can all hold their accumulators (512 TMEM columns): an allocation that waited for a
-    // cluster which itself waits for another's would never end.
     int cols = 32;
     while (cols < bn) cols *= 2;
-    const size_t least = 228 * 1024 / (512 / cols + 1) - 1024;
-    if (work < least) work = least;
     work = (work + 15) / 16 * 16;
     if (work_bytes) *work_bytes = (int)work;
-    return work + sizeof(SplitShared) + 16;
+    return tmem_smem(work + sizeof(SplitShared) + 16, cols);
 }
 
 typedef void (*SplitKernel)(SplitArgs);

@@ -192,3 +192,23 @@ def test_bench_workloads_are_well_formed():
     assert abs(total - 140_691_900_416.0) < 1.0
     peaks = bench.load_peaks()
     assert peaks["hbm_gbs"] > 1000 and peaks["bf16_tflops"] >= peaks["bf16_sustained"] > 100
+
+
+def test_ctas_that_share_an_sm_can_all_hold_their_accumulators():
+    """Tensor-core kernels ask for at least their columns' share of an SM's shared memory (228 KB, 1 KB reserved per CTA, for 512
+    columns), so that no mix of CTAs that fits an SM by shared memory asks for more TMEM than there is."""
+    L = C.CDLL(os.path.join(os.path.dirname(dn.__file__), "libdarknet_b200.so"))
+    share, split = L._ZN3dnb9tmem_smemEmi, L._ZN3dnb18conv_tc_split_smemEiiiPi
+    share.restype = split.restype = C.c_size_t
+    fits = lambda smem, cols: 512 * (smem + 1024) >= cols * 228 * 1024 and smem <= 227 * 1024   # noqa: E731
+    for cols in (32, 64, 128, 256, 512):
+        for asked in (0, 20_000, 115_711, 115_713, 227 * 1024):
+            assert share(C.c_size_t(asked), cols) >= asked and fits(share(C.c_size_t(asked), cols), cols)
+    for bn in range(16, 257, 16):
+        cols = max(32, 1 << (bn - 1).bit_length())
+        for row_bytes in (32, 64, 128):
+            stage, work = 128 * row_bytes + (bn * row_bytes + 1023) // 1024 * 1024, C.c_int()
+            for stages in range(2, 13):
+                if stages * stage <= 220_000:
+                    smem = split(stages, stage, bn, C.byref(work))
+                    assert fits(smem, cols) and smem >= work.value >= stages * stage
