@@ -815,13 +815,21 @@ static int forward_eager(dnb_network *net, const float *device_input, cudaStream
     return DNB_OK;
 }
 
-static void drop_graph(dnb_network *net)
+// The captured device-resident forward, which belongs to one input and stream.
+static void drop_forward_graph(dnb_network *net)
 {
     if (net->graph_exec) cudaGraphExecDestroy(net->graph_exec);
     net->graph_exec = nullptr;
     net->graph_input = nullptr;
     net->graph_stream = nullptr;
     net->eager_runs = 0;
+}
+
+// ... and everything else that holds the parameters' pointers or the plans' launch blocks: the captured steps, which read the
+// network's own input buffers whatever forward is given, and the plans of parts of a batch.
+static void drop_graph(dnb_network *net)
+{
+    drop_forward_graph(net);
     for (int k = 0; k < 2; ++k) {
         if (net->step_exec[k]) cudaGraphExecDestroy(net->step_exec[k]);
         net->step_exec[k] = nullptr;
@@ -829,7 +837,7 @@ static void drop_graph(dnb_network *net)
         for (cudaGraphExec_t e : net->item_exec[k]) if (e) cudaGraphExecDestroy(e);
         net->item_exec[k].clear();
     }
-    for (Layer &L : net->layers)   // they hold the parameters' pointers too
+    for (Layer &L : net->layers)
         for (dnb_conv_plan *&q : L.piece_plan) { dnb_conv_plan_destroy(q); q = nullptr; }
 }
 
@@ -837,7 +845,7 @@ extern "C" int dnb_network_enable_graph(dnb_network *net, int on)
 {
     if (!net) DNB_FAIL(DNB_EINVAL, "enable_graph: null network");
     net->graph_enabled = on != 0;
-    if (!on) drop_graph(net);
+    if (!on) drop_forward_graph(net);
     return DNB_OK;
 }
 
@@ -859,7 +867,7 @@ extern "C" int dnb_network_forward(dnb_network *net, const float *device_input, 
         return DNB_OK;
     }
     if (net->graph_input != device_input || net->graph_stream != s) {
-        drop_graph(net);
+        drop_forward_graph(net);
         net->graph_input = device_input;
         net->graph_stream = s;
     }
@@ -872,7 +880,7 @@ extern "C" int dnb_network_forward(dnb_network *net, const float *device_input, 
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
         net->graph_enabled = false;          // something on the path cannot be captured: stay eager from here on
-        drop_graph(net);
+        drop_forward_graph(net);
         return forward_eager(net, device_input, s);
     }
     const cudaError_t ie = cudaGraphInstantiate(&net->graph_exec, graph, 0);

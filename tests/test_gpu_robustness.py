@@ -282,3 +282,28 @@ def test_truncated_weights_file_after_predicting(size, batch, tmp_path):
     for _ in range(5):
         assert np.array_equal(net.predict(x), want[1])
     net.close()
+
+
+def test_forward_on_other_buffers_keeps_the_blocking_calls_steps(tmp_path, monkeypatch):
+    """The blocking call's captured steps read the network's own input: a device-resident forward with graphs on, on one buffer after
+    the other, leaves them as they are.  Plans made after the first calls store nothing here (a diagnostic bit), so a step
+    that had to be made anew would hand out old results."""
+    cfg = (synth._net(16, 256, 256) + synth._conv(32, 3) + synth._conv(64, 3, stride=2) + synth._conv(64, 3) + synth._conv(512, 3, stride=2) +
+           synth._conv(90, 1, bn=False, act="linear") + synth._yolo("0,1", "10,14, 23,27", 2, 40))
+    path = str(tmp_path / "w")
+    synth.write_weights(path, synth.seeded_params(cfg, 2))
+    net = dn.Network(cfg, path, dn.MODE_TF32, text=True)
+    x = [synth.seeded_input(cfg, k) for k in range(2)]
+    want = [net.predict(a).copy() for a in x]
+    for _ in range(4):
+        net.predict(x[0])
+    monkeypatch.setenv("DNB_TC_DEBUG", "2")
+    net.enable_graph(True)
+    stream = torch.cuda.Stream()
+    for a in x:
+        net.forward(torch.from_numpy(a).cuda(), stream=stream.cuda_stream)
+        stream.synchronize()
+    net.enable_graph(False)
+    for k in (1, 0, 1):
+        assert np.array_equal(net.predict(x[k]), want[k])
+    net.close()
