@@ -67,6 +67,7 @@ struct Layer {
     int launches = 1;
     // a convolution that also performs the [shortcut] layer right after it, and that shortcut layer
     bool fuses_next_shortcut = false, fused_into_prev = false;
+    dnb_tensor own_out{};          // ... where that layer's addend has another shape: the convolution's own output, filled for who asks for it
     // a convolution that also performs the [yolo] layer right after it (that layer is then fused_into_prev too)
     bool fuses_next_yolo = false;
     // a maxpool layer that also writes the signs of its output, the next (tensor-core xnor) layer's operand
@@ -364,7 +365,10 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         C.fuses_next_shortcut = true;
         S.fused_into_prev = true;
         S.launches = 0;
-        cudaFree(C.out.data);      // never written: the convolution stores straight into the shortcut's output
+        // Never written by a step: the convolution stores straight into the shortcut's output.  An output that was to be read while
+        // only equal shapes were fused still is (own_output).
+        if (F.out.c != S.out.c || F.out.h != S.out.h || F.out.w != S.out.w) C.own_out = C.out;
+        else cudaFree(C.out.data);
         C.out.data = nullptr;
     }
     // Fuse "convolution, then [yolo]" when nothing else reads the convolution's output: the epilogue applies the yolo
@@ -513,6 +517,7 @@ extern "C" void dnb_free_network(dnb_network *net)
     for (Layer &L : net->layers) {
         if (L.plan) dnb_conv_plan_destroy(L.plan);
         if (!L.out_is_view) cudaFree(L.out.data);
+        cudaFree(L.own_out.data);
         for (float *hp : L.host_slot) if (hp) cudaFreeHost(hp);
         for (cudaEvent_t e : L.copied) if (e) cudaEventDestroy(e);
     }
@@ -695,19 +700,34 @@ extern "C" int dnb_network_set_conv_params(dnb_network *net, int layer, const fl
     return DNB_OK;
 }
 
+// Layer i's output as a step leaves it, in *t; the own output of a convolution that was fused with a shortcut of another shape is
+// made from its input, which is still there, on s.
+static int own_output(dnb_network *net, int i, dnb_tensor *t, cudaStream_t s)
+{
+    Layer &L = net->layers[i];
+    *t = L.out;
+    if (L.out.data) return DNB_OK;
+    if (!L.own_out.data)
+        DNB_FAIL(DNB_EUNSUPPORTED, "layer %d is fused into layer %d and has no output of its own (DNB_FUSE_SHORTCUT=0 / DNB_FUSE_YOLO=0 keep it)", i, i + 1);
+    const dnb_tensor in = i > 0 ? net->layers[i - 1].out : net->input_nhwc;
+    *t = L.own_out;
+    return dnb_conv_forward(L.plan, &in, t, nullptr, s);
+}
+
 // Layer `layer`'s current output in Darknet's layout (NCHW f32) into device memory of the caller, on `stream`.
 extern "C" int dnb_network_export_layer(dnb_network *net, int layer, float *device_nchw, void *stream)
 {
     if (!net || !device_nchw || layer < 0 || layer >= (int)net->layers.size()) DNB_FAIL(DNB_EINVAL, "export_layer: bad argument");
     Layer &L = net->layers[layer];
-    if (!L.out.data) DNB_FAIL(DNB_EUNSUPPORTED, "layer %d is fused into layer %d and has no output of its own", layer, layer + 1);
     cudaStream_t s = (cudaStream_t)stream;
+    dnb_tensor out;
+    DNB_TRY(own_output(net, layer, &out, s));
     if (L.out.layout == DNB_NCHW) {
         DNB_CUDA(cudaMemcpyAsync(device_nchw, L.out.data, tensor_elems(&L.out) * sizeof(float), cudaMemcpyDeviceToDevice, s));
         return DNB_OK;
     }
     dnb_tensor o{device_nchw, DNB_NCHW, DNB_F32, net->batch, L.out_c, L.out_h, L.out_w, 0};
-    return launch_convert(&L.out, &o, 0, 0, 0, s);
+    return launch_convert(&out, &o, 0, 0, 0, s);
 }
 
 // Every convolution launched from here on reports an expired wait in the status word of step slot `slot`.
@@ -1247,7 +1267,7 @@ extern "C" int dnb_network_layer_output_images(dnb_network *net, int i, int firs
     if (first < 0 || count < 1 || first + count > net->batch) DNB_FAIL(DNB_EINVAL, "layer_output: images %d..%d of a batch of %d", first, first + count - 1, net->batch);
     Layer &L = net->layers[i];
     if (net->submitted != net->collected) DNB_FAIL(DNB_EINVAL, "layer_output: a submitted step is still in flight; collect it first");
-    if (!L.out.data)
+    if (!L.out.data && !L.own_out.data)
         DNB_FAIL(DNB_EUNSUPPORTED, "layer %d is fused into layer %d and has no output of its own (DNB_FUSE_SHORTCUT=0 / DNB_FUSE_YOLO=0 keep it)", i, i + 1);
     const size_t per_image = (size_t)L.out_c * L.out_h * L.out_w;
     const size_t elems = (size_t)count * per_image;
@@ -1268,9 +1288,10 @@ extern "C" int dnb_network_layer_output_images(dnb_network *net, int i, int firs
         DNB_CUDA(cudaMalloc((void **)&net->export_dev, conv_elems * sizeof(float)));
         net->export_elems = conv_elems;
     }
-    dnb_tensor in = L.out;
+    dnb_tensor in;
+    DNB_TRY(own_output(net, i, &in, net->stream));
     in.n = conv_count;
-    in.data = (char *)L.out.data + (size_t)conv_first * image_bytes;
+    in.data = (char *)in.data + (size_t)conv_first * image_bytes;
     dnb_tensor o{net->export_dev, DNB_NCHW, DNB_F32, conv_count, L.out_c, L.out_h, L.out_w, 0};
     DNB_TRY(launch_convert(&in, &o, 0, 0, 0, net->stream));
     DNB_CUDA(cudaStreamSynchronize(net->stream));
