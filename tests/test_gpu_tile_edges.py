@@ -131,9 +131,14 @@ def test_shortcut_of_another_shape_in_the_epilogue(batch, size, what, mode, tol,
     assert what in net.layer_describe(1), net.layer_describe(1)
     for i in (2, 5):
         parity(net.layer_output(i), want[i], tol, f"layer {i}")
-    for i in (1, 4):
-        with pytest.raises(dn.DarknetB200Error):
-            net.layer_output(i)          # the convolution has no output of its own
+    for i in (1, 4):                     # made from the convolution's input on request: a step does not write it
+        parity(net.layer_output(i), want[i], tol, f"layer {i}")
+        assert (net.layer_output_images(i, batch - 1) == net.layer_output(i)[batch - 1:]).all()
+    for i in (2, 5):                     # ... and what the step wrote is still there, as is what the next one writes
+        parity(net.layer_output(i), want[i], tol, f"layer {i}")
+    again = net.predict(x).copy()
+    assert (net.predict(x) == again).all()
+    parity(net.layer_output(5), want[5], tol, "layer 5")
 
 
 @pytest.mark.parametrize("name,shape", [
