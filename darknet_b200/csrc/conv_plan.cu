@@ -934,8 +934,10 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         a.status = p->status;
         a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
         a.g = g; a.ep = ep;
-        // in the im2col order where layers take the signs of what follows from it (see conv_stem_rows.cu), else from the patch
-        return p->keep_k_order && conv_stem_rows_covers(g, y_dtype) ? launch_conv_stem_rows(a, s) : launch_conv_stem_tc(a, s);
+        // in the im2col order where layers take the signs of what follows from it (see conv_stem_rows.cu), else from the patch, whose
+        // offsets inside an image take rows of less than 2^25 values
+        const bool rows = (p->keep_k_order || a.xs_h >= (1LL << 31) / 64) && conv_stem_rows_covers(g, y_dtype);
+        return rows ? launch_conv_stem_rows(a, s) : launch_conv_stem_tc(a, s);
     }
     if (p->kernel == K_DIRECT) {   // also a first-layer plan asked for Darknet's layout or given bf16 input
         DirectArgs a;

@@ -337,7 +337,8 @@ conv_stem_rows_wide_kernel(const __grid_constant__ StemTcArgs a)
 
     const float *const x = a.x;
     const long long xs_b = a.xs_b;
-    const int xs_c = (int)a.xs_c, xs_h = (int)a.xs_h, xs_w = (int)a.xs_w;
+    const long long xs_c = a.xs_c, xs_h = a.xs_h;
+    const int xs_w = (int)a.xs_w;
     const int npix = a.npix, tiles = a.tiles, plane = g.out_h * g.out_w;
     const int runtime_act = a.ep.activation, do_round = a.ep.round_tf32;
     int *const status = a.status;
@@ -542,7 +543,7 @@ int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s)
 {
     const ConvGeom &g = a.g;
     if (!conv_stem_rows_covers(g, a.y_dtype) || a.y_cpitch != g.n) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: geometry outside its coverage");
-    if (a.xs_c >= (1LL << 31) / 4 || a.xs_h >= (1LL << 31) / 64) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: image too large for 32-bit offsets");
+    if (a.xs_c >= (1LL << 31) / 4 || a.xs_h >= (1LL << 31) / 4) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: image too large for 32-bit offsets");
     const long long npix = (long long)g.batch * g.out_h * g.out_w;
     a.npix = (int)npix;
     a.tiles = (int)((npix + SR_THREADS - 1) / SR_THREADS);

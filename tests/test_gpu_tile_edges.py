@@ -207,3 +207,29 @@ def test_to_channels_last_tiles(c, h, w, pitch, dtype):
     dn.convert(dn.as_tensor(x, dn.NCHW), dn.as_tensor(y, dn.NHWC, c))
     torch.cuda.synchronize()
     assert torch.equal(y[..., :c], x.permute(0, 2, 3, 1).to(y.dtype)) and not y[..., c:].any()
+
+
+def test_first_layer_of_a_very_long_image():
+    """A row of 2^25 + 37 pixels: beyond the offsets of the patch kernel.  Windows of the row against the checker (whose image is the
+    window and a pixel on each side); operands rounded to TF32."""
+    import numpy as np
+    import torch
+    from conftest import rel_to_max
+    w = (1 << 25) + 37
+    plan = dn.ConvPlan(1, 3, 1, w, 16, 3, 1, 1, 1, False, "linear")
+    g = np.random.Generator(np.random.Philox(key=[9, 9]))
+    wt, bias = g.standard_normal((16, 3, 3, 3), dtype=np.float32), g.standard_normal(16, dtype=np.float32)
+    plan.set_params(wt, bias)
+    x = torch.randn(1, 3, 1, w, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    y = torch.full((1, 1, w, 16), float("nan"), device="cuda")
+    plan.forward(dn.as_tensor(x, dn.NCHW), dn.as_tensor(y, dn.NHWC, 16))
+    plan.check_status()
+    from oracle import network as orc
+    for at in (0, 1000, (1 << 24) - 8, (1 << 25) - 20, w - 300):
+        lo, hi = max(at - 1, 0), min(at + 301, w)
+        want = orc.conv_forward(x[..., lo:hi].cpu().numpy(), wt, bias, None, None, None, stride=1, pad=1, groups=1, activation="linear")
+        want = want[..., at - lo:at - lo + 300]
+        got = y[:, :, at:at + 300].permute(0, 3, 1, 2).cpu().numpy()
+        assert rel_to_max(got, want) < 1e-2
+    del x, y
+    torch.cuda.empty_cache()
