@@ -67,13 +67,14 @@ bool pdl_enabled();     // conv_tc.cu; DNB_PDL=0: plain launches
 // kernel after it do the same with launch_dependents_if_small() (tc_ptx.cuh).  Only grids of at most two blocks per SM start
 // early: larger ones would fill whatever room the running kernel leaves here and there, and their even share of blocks per
 // SM would be lost (Darknet-19 at batch 128 with every pooling layer started early: 1.30 -> 1.42 ms).
+constexpr int EARLY_BLOCKS = 2 * 148;   // two per SM of a B200; launch_dependents_if_small() goes by the same number
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     const long long blocks = (long long)grid.x * grid.y * grid.z;
-    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() && blocks <= 2LL * sm_count() ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() && blocks <= EARLY_BLOCKS ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;

@@ -21,6 +21,7 @@
 // Replaces forward_convolutional_layer_gpu (src/convolutional_kernels.cu:73-135 of the reference) at small batches.
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "common.h"
@@ -432,19 +433,19 @@ static SplitKernel kernel_of(int kind, int pair, int cls)
     return pair ? kernel_of_class<MMA_TF32, true>(cls) : kernel_of_class<MMA_TF32, false>(cls);
 }
 
-// The kernel's attributes, set once per kernel and device (setting them twice, from two threads, is harmless).
+// The kernel's attributes, set once per kernel and device (twice, where two threads come at once: harmless).
 static int prepare_kernel(int kind, int pair, int cls)
 {
-    static bool done[64][3][2][2];
+    static std::atomic<bool> done[64][3][2][2];
     int dev = 0;
     DNB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) DNB_FAIL(DNB_ECUDA, "conv_tc_split: device %d", dev);
-    bool &d = done[dev][kind][pair ? 1 : 0][cls];
-    if (d) return DNB_OK;
+    std::atomic<bool> &d = done[dev][kind][pair ? 1 : 0][cls];
+    if (d.load(std::memory_order_acquire)) return DNB_OK;
     const SplitKernel kern = kernel_of(kind, pair, cls);
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    d = true;
+    d.store(true, std::memory_order_release);
     return DNB_OK;
 }
 

@@ -4,6 +4,8 @@
 #include <cuda.h>
 #include <stdint.h>
 
+#include "common.h"
+
 namespace dnb {
 
 // Default bound of every device-side wait, in SM clock cycles (about one second).  The bound travels in the
@@ -203,7 +205,7 @@ __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontr
 // ... from a kernel of many short blocks: where it fills the GPU, early successors would only take room from its own blocks.
 __device__ __forceinline__ void launch_dependents_if_small()
 {
-    if ((unsigned long long)gridDim.x * gridDim.y * gridDim.z <= 296ull) launch_dependents();
+    if ((unsigned long long)gridDim.x * gridDim.y * gridDim.z <= (unsigned long long)EARLY_BLOCKS) launch_dependents();
 }
 
 // ------------------------------------------------------------------ CTA pairs (cta_group::2)
