@@ -29,7 +29,7 @@ namespace dnb {
 constexpr size_t COPY_CHUNK = 512 * 1024, COPY_CHUNK_MAX = 1024 * 1024, COPY_MANY = 8 * 1024 * 1024;
 // A slot is as long as the longest chunk, whatever the upload's own: its event then guards the same bytes for every upload, and one
 // of another chunk length cannot reach bytes whose transfer has not been waited for.
-constexpr size_t COPY_RING = 16, COPY_GROUP = 2 * COPY_CHUNK_MAX;   // slots; page-locked memory is taken two slots at a time
+constexpr size_t COPY_RING = 16, COPY_GROUP = 2 * COPY_CHUNK_MAX;   // slots; page-locked memory is taken in multiples of two
 // Below this a second thread cannot be awake before the copy is over.
 constexpr size_t COPY_ALONE = 1024 * 1024;
 
@@ -64,7 +64,7 @@ public:
         wake_.notify_all();
         for (std::thread &t : threads_) t.join();
         drop_events();
-        for (char *g : groups_) {
+        for (char *g : blocks_) {
             cudaHostUnregister(g);
             free(g);
         }
@@ -137,24 +137,31 @@ private:
         }
     };
 
-    // Slots of the ring up to `want`, as many as there are to be had.  Pages of 2 MB where the system has them: taking and
-    // locking 16 MB takes 3.7 ms with them, 13 to 20 with 4 KB pages.
+    // Slots of the ring up to `want`, as many as there are to be had: what is missing at once, else two slots at a time.  Pages of 2 MB
+    // where the system has them: taking and locking 16 MB takes 3.7 ms with them, 13 to 20 with 4 KB pages.
     size_t grow(size_t want)
     {
-        while (slots_ < want && !full_) {
-            groups_.reserve(COPY_RING * COPY_CHUNK_MAX / COPY_GROUP);
-            char *g = (char *)aligned_alloc(COPY_GROUP, COPY_GROUP);
-            if (g) madvise(g, COPY_GROUP, MADV_HUGEPAGE);
-            if (!g || cudaHostRegister(g, COPY_GROUP, cudaHostRegisterPortable) != cudaSuccess) {
-                cudaGetLastError();
-                free(g);
-                full_ = true;                  // no more page-locked memory: go on with what there is
-                break;
-            }
-            groups_.push_back(g);
-            for (size_t at = 0; at < COPY_GROUP; at += COPY_CHUNK_MAX) slot_[slots_++] = g + at;
+        for (size_t bytes; slots_ < want && !full_;) {
+            blocks_.reserve(COPY_RING);
+            bytes = (want - slots_ + 1) / 2 * COPY_GROUP;
+            char *g = lock_pages(bytes);
+            if (!g && bytes > COPY_GROUP) g = lock_pages(bytes = COPY_GROUP);
+            full_ = !g;                        // no more page-locked memory: go on with what there is
+            if (!g) break;
+            blocks_.push_back(g);
+            for (size_t at = 0; at < bytes; at += COPY_CHUNK_MAX) slot_[slots_++] = g + at;
         }
         return slots_ < want ? slots_ : want;
+    }
+
+    static char *lock_pages(size_t bytes)
+    {
+        char *g = (char *)aligned_alloc(COPY_GROUP, bytes);
+        if (g) madvise(g, bytes, MADV_HUGEPAGE);
+        if (g && cudaHostRegister(g, bytes, cudaHostRegisterPortable) == cudaSuccess) return g;
+        cudaGetLastError();
+        free(g);
+        return nullptr;
     }
 
     bool start_threads()
@@ -203,12 +210,14 @@ private:
                 seen = generation_;
                 job = job_;
             }
+            // (Sleeping where there is nothing to copy for a while frees little, the threads copy most of the time, and made 284 MB
+            // take 10.0 ms instead of 9.4.)
             while (job && !job->taken())
                 if (!job->one()) std::this_thread::yield();
         }
     }
 
-    std::vector<char *> groups_;   // the ring's memory
+    std::vector<char *> blocks_;   // the ring's memory
     char *slot_[COPY_RING] = {};
     size_t slots_ = 0;
     bool full_ = false, alone_ = false;

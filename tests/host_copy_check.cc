@@ -51,7 +51,12 @@ int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), vo
     ++threads_asked;
     return no_threads ? EAGAIN : create(t, a, f, x);
 }
-cudaError_t cudaHostRegister(void *, size_t bytes, unsigned) { return (locked += bytes) > may_lock ? cudaErrorMemoryAllocation : cudaSuccess; }
+cudaError_t cudaHostRegister(void *, size_t bytes, unsigned)
+{
+    if (locked + bytes > may_lock) return cudaErrorMemoryAllocation;
+    locked += bytes;
+    return cudaSuccess;
+}
 cudaError_t cudaHostUnregister(void *) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
