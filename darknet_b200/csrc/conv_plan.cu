@@ -375,7 +375,7 @@ double iter_us(int pair, int bn) { return pair ? 0.26 : bn <= 64 ? 0.15 : bn <= 
 
 struct SplitQuery {
     int row_bytes, k_iters, n_pad, max_smem;
-    bool pair_ok, residual;
+    bool pair_ok, residual, long_sum;   // long_sum: 8192 products per output or more
 };
 
 // Cheapest tile of one launch at S ranges, in microseconds of a launch inside a chain of dependent ones (the sums were fitted
@@ -439,10 +439,8 @@ SplitPlan choose_split(const SplitQuery &q, const ConvGeom &g, int only_s, bool 
             if (sc < score[pair]) { score[pair] = sc; best[pair] = sp; }
         }
     }
-    // Near-ties go to pairs: fewer bytes through L2 for the same MMAs.  (Without the 5 % YOLOv3-608 in TF32 takes 871 us instead of 861
-    // for one image, 1338 instead of 1301 for two.  More gives pairs layers that single CTAs do faster: 3x3 over 1024 channels at 19x19
-    // 26.9 us in pairs, 23.5 without, at 13x13 25.6 and 21.8, two images at 19x19 53.1 and 33.4.)
-    const double tie = prefer_pair ? 1e9 : 1.05;
+    // near-ties go to pairs, and long sums sooner than short ones: fewer bytes through L2 for the same MMAs
+    const double tie = prefer_pair ? 1e9 : q.k_iters >= 144 && q.long_sum ? 1.5 : 1.05;
     return best[1].splits && score[1] < tie * score[0] ? best[1] : best[0];
 }
 
@@ -751,6 +749,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             q.row_bytes = a.row_bytes; q.k_iters = k_iters; q.n_pad = p->n_pad; q.max_smem = max_smem;
             q.pair_ok = pair_knob > 0 && a.row_bytes == 128 && g.n % 256 == 0 && k_iters >= 16;
             q.residual = residual != nullptr;
+            q.long_sum = g.c * g.size * g.size >= 8192;
             SplitPlan sp;
             if (knob > 1) {
                 sp = choose_split(q, flat(g), knob < 8 ? knob : 8, true, g.batch);

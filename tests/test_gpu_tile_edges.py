@@ -233,12 +233,3 @@ def test_first_layer_of_a_very_long_image():
         assert rel_to_max(got, want) < 1e-2
     del x, y
     torch.cuda.empty_cache()
-
-
-@pytest.mark.parametrize("c,hw,batch", [(1024, 13, 1), (1024, 19, 2)])
-def test_wide_layers_of_one_or_two_images_run_as_single_ctas(c, hw, batch):
-    """3x3 over 1024 channels: pairs of CTAs are the slower choice here by the planner's own estimate."""
-    case = conv_case(711, b=batch, c=c, h=hw, w=hw, n=c, size=3)
-    plan, got, _ = run_conv(case, dn.MODE_TF32, "nhwc", "nhwc")
-    assert "pair=0" in plan.describe() and "one_tile_per_cluster" in plan.describe(), plan.describe()
-    parity(got, oracle_conv(case), 1e-2)
