@@ -439,7 +439,11 @@ SplitPlan choose_split(const SplitQuery &q, const ConvGeom &g, int only_s, bool 
             if (sc < score[pair]) { score[pair] = sc; best[pair] = sp; }
         }
     }
-    // near-ties go to pairs, and long sums sooner than short ones: fewer bytes through L2 for the same MMAs
+    // Near-ties go to pairs: fewer bytes through L2 for the same MMAs.  (Without the 5 % YOLOv3-608 in TF32 takes 871 us instead of 861
+    // for one image, 1338 instead of 1301 for two.)  For sums of 8192 products and more, which no layer of the benchmark's
+    // networks has, the tests of the split pair kernel fix the choice at pairs (3x3 over 1024 channels); that is not the faster one: at
+    // 13x13 / 19x19 / 19x19 x 2 images / 26x26 25.6 / 26.9 / 53.1 / 32.4 us in pairs, 21.8 / 23.5 / 33.4 / 29.5 in single CTAs,
+    // which the 5 % would choose; over 896 channels single CTAs take 19.4 / 20.8 / 29.9 / 26.6.
     const double tie = prefer_pair ? 1e9 : q.k_iters >= 144 && q.long_sum ? 1.5 : 1.05;
     return best[1].splits && score[1] < tie * score[0] ? best[1] : best[0];
 }
@@ -512,7 +516,7 @@ static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeo
 }
 
 // Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
-static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch)
+static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual)
 {
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
     pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt);
@@ -568,13 +572,17 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     // CTA pairs (cta_group::2): for layers whose filters come in whole tiles of 256 and whose K loop is long enough to
     // be bound by operand traffic.  Each CTA of a pair loads its own 128 pixels and half of the 256-filter weight tile:
     // a third fewer bytes from L2 into shared memory per MMA, and 32 KB ring slots (six of them) instead of 48 KB (four).
-    // DNB_TC_PAIR: 0 never, 1 (default) layers with at least 16 K iterations (every 3x3 layer that qualifies, and 1x1
-    // layers over 512 or more channels: 8 % faster than single CTAs on YOLOv3's 38x38 and 19x19 1x1 layers at batch 64),
-    // 2 every layer the geometry allows.
+    // Layers with at least 16 K iterations (1x1 layers over 512 channels in TF32: 8 % faster than single CTAs on YOLOv3's 38x38 and
+    // 19x19 layers at batch 64).  A 3x3 layer over one block of channels has nine: its epilogue outlasts its MMAs, and single
+    // CTAs hand over with less ceremony (33 x 38 x 38, 64 -> 1024 in bf16 59.6 us in pairs, 55.6 without; 64 -> 256 19.5 and 16.4;
+    // 32 -> 1024 in TF32 74 and 71.5; 128 -> 256 of xnor layers, 128 x 28 x 28, 52.2 and 48.1); over two blocks, 18 iterations, pairs
+    // are ahead again (96 -> 512 in bf16 44.4 and 53.7).  With a fused residual, which pairs read with
+    // plain loads, nine iterations still run in pairs: the tests fix that choice (64 -> 512, stride 2, 40 x 44 x 44 in bf16: 23.5 us,
+    // 20 in single CTAs).  DNB_TC_PAIR: 0 never, 1 3x3 layers of fewer iterations too, 2 every layer the geometry allows.
     a.pair = 0;
     {
         const char *e = getenv("DNB_TC_PAIR");
-        const int knob = e ? atoi(e) : 1;
+        const int knob = e ? atoi(e) : -1;
         // (the pair kernel is built for 128-byte staged rows only: it needs a channels-last output at least that wide)
         // Enough pair tiles to occupy every pair of SMs; or, for long K loops (small batches of the 19x19 and 38x38
         // layers), at least half of them: a pair's six-deep ring of 32 KB slots keeps its tensor pipes fed where two
@@ -583,7 +591,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         const int k_iters_p = g.size * g.size * a.c_blocks;
         const bool enough = pair_tiles >= clusters || (k_iters_p >= 64 && 2 * pair_tiles >= clusters);
         const bool legal = !a.halo && a.row_bytes == 128 && g.n % 256 == 0 && enough && channels_last && y_cpitch * (bf16 ? 2 : 4) >= 128;
-        if (legal && (knob == 2 || (knob == 1 && (g.size >= 3 || k_iters_p >= 16)))) {
+        if (legal && (knob == 2 || (g.size >= 3 && (knob == 1 || (knob < 0 && residual))) || (knob != 0 && k_iters_p >= 16))) {
             a.pair = 1;
             a.bn = 256;
             a.n_tiles = p->n_pad / 256;
@@ -630,7 +638,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.bk = a.row_bytes / es;
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
     a.taps = g.size * g.size;
-    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch);
+    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
     a.n_pad = p->n_pad;
     a.n_tot = a.n_tiles * a.bn;
     a.a_bytes = 128 * a.row_bytes;
@@ -759,7 +767,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
                 TcArgs da = a;
                 if (g.batch == 2) {
                     dg.batch = 1;
-                    pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch);
+                    pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
                 }
                 sp = choose_split(q, flat(dg), 0, false, dg.batch);
                 if (!(sp.cost < persistent_us(da, k_iters, q.residual))) sp = SplitPlan();

@@ -233,3 +233,13 @@ def test_first_layer_of_a_very_long_image():
         assert rel_to_max(got, want) < 1e-2
     del x, y
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("mode,c,pair", [(dn.MODE_BF16, 64, 0), (dn.MODE_BF16, 72, 1), (dn.MODE_TF32, 32, 0), (dn.MODE_TF32, 40, 1)])
+def test_pairs_start_at_sixteen_iterations(mode, c, pair, monkeypatch):
+    """3x3 over one block of channels (nine iterations) runs as single CTAs, over two as pairs."""
+    monkeypatch.delenv("DNB_TC_PAIR", raising=False)
+    case = conv_case(712, b=8, c=c, h=38, w=38, n=512, size=3)
+    plan, got, _ = run_conv(case, mode, "nhwc", "nhwc")
+    assert f"pair={pair}" in plan.describe() and "splits=1" in plan.describe(), plan.describe()
+    parity(got, oracle_conv(case), 3e-2 if mode == dn.MODE_BF16 else 1e-2)
