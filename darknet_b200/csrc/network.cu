@@ -344,6 +344,8 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
             for (int id : L.inputs)
                 if (net->layers[id].kind == L_YOLO) DNB_FAIL(DNB_EUNSUPPORTED, "cfg: route from a [yolo] layer");
     }
+    bool any_xnor = false;
+    for (const Layer &L : net->layers) any_xnor = any_xnor || (L.kind == L_CONV && L.cd.xnor);
     // Fuse "convolution, then [shortcut]" (of equal shape, or as ResNet's stages begin: fewer channels, a larger map) into
     // the convolution's epilogue when nothing else reads the convolution's own output: one pass over the activations
     // instead of three.  (ResNet-50, batch 256: the four passes that had other shapes took 0.86 ms of 7.7.)
@@ -354,6 +356,8 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         if (C.kind != L_CONV || !C.plan || (C.plan->kernel != 0 && C.plan->kernel != 1) || S.kind != L_SHORTCUT || S.from == i) continue;
         const Layer &F = net->layers[S.from];
         if (F.kind == L_YOLO || !conv_shortcut_fusable(C.plan, &F.out, &S.out, S.alpha)) continue;
+        const bool other_shape = F.out.c != S.out.c || F.out.h != S.out.h || F.out.w != S.out.w;
+        if (other_shape && any_xnor) continue;   // their sums, which layers take the signs of, are rounded where they always were
         bool read_elsewhere = false;
         for (int j = i + 2; j < (int)net->layers.size(); ++j) {
             const Layer &L = net->layers[j];
@@ -367,7 +371,7 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         S.launches = 0;
         // Never written by a step: the convolution stores straight into the shortcut's output.  An output that was to be read while
         // only equal shapes were fused still is (own_output).
-        if (F.out.c != S.out.c || F.out.h != S.out.h || F.out.w != S.out.w) C.own_out = C.out;
+        if (other_shape) C.own_out = C.out;
         else cudaFree(C.out.data);
         C.out.data = nullptr;
     }
@@ -449,8 +453,6 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
     // A sign hangs on a sum's last bit.  Where layers are binarised, the dense ones add in the same order at every batch
     // size (integer sums do not care), so that an image's results do not depend on how many came with it, and a first layer
     // on the tensor cores adds in the reference's order of the products.
-    bool any_xnor = false;
-    for (const Layer &L : net->layers) any_xnor = any_xnor || (L.kind == L_CONV && L.cd.xnor);
     for (Layer &L : net->layers) if (L.plan) L.plan->keep_k_order = any_xnor;
     const Layer &last = net->layers.back();
     net->outputs = last.out_c * last.out_h * last.out_w;

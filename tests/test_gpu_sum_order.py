@@ -92,3 +92,18 @@ def test_dense_layers_on_cuda_cores_add_in_the_reference_order(mode, groups, bat
     inner = net.layer_output(1).reshape((batch,) + net.layer_shape(1))[:, :, 1:-1, 1:-1]
     assert (inner == 9 * (cpg - 1)).all()
     net.close()
+
+
+def test_shortcuts_of_another_shape_keep_their_roundings(tmp_path):
+    """In front of an xnor layer: the convolution's output is rounded to TF32, the sum with an addend of fewer channels and twice the
+    map is not, as the two layers do it one by one.  Computed here from the two layers' own outputs, to the bit."""
+    cfg = (synth._net(3, 20, 20, 16) + synth._conv(64, 3) + synth._conv(96, 3, stride=2, act="linear") + synth._shortcut(-2, "leaky") +
+           synth._conv(32, 3, xnor=True))
+    net = network(cfg, synth.seeded_params(cfg, 4), tmp_path)
+    net.predict(synth.seeded_input(cfg, 5, "normal"))
+    out = [net.layer_output(i).reshape((3,) + net.layer_shape(i)) for i in range(3)]
+    want = out[1].copy()
+    want[:, :64] += out[0][:, :, ::2, ::2]
+    want = np.where(want > 0, want, np.float32(0.1) * want)
+    assert np.array_equal(out[2], want)
+    net.close()
