@@ -307,3 +307,42 @@ def test_forward_on_other_buffers_keeps_the_blocking_calls_steps(tmp_path, monke
     for k in (1, 0, 1):
         assert np.array_equal(net.predict(x[k]), want[k])
     net.close()
+
+
+@pytest.mark.parametrize("threads", [1, 2])
+def test_images_of_two_networks_share_the_staging_ring(threads, tmp_path):
+    """A small and a large network, both fed from ordinary memory without waiting in between, from one thread and from two: what they
+    answer is what they answer for page-locked images."""
+    import threading
+    nets, x, want = [], [], []
+    for k, (batch, size) in enumerate(((1, 416), (8, 416))):     # 2 MB and 16.6 MB: chunks of 512 KB and of 1 MB
+        cfg = synth._net(batch, size, size) + synth._conv(16, 3, stride=2) + "\n[avgpool]\n" + synth._conv(10, 1, bn=False, act="linear")
+        path = str(tmp_path / f"{k}.weights")
+        synth.write_weights(path, synth.seeded_params(cfg, k))
+        nets.append(dn.Network(cfg, path, dn.MODE_TF32, text=True))
+        x.append([synth.seeded_input(cfg, 10 * k + i) for i in range(2)])
+        want.append([nets[k].predict(torch.from_numpy(a).pin_memory()).copy() for a in x[k]])
+        assert not np.array_equal(*want[k])
+    bad = []
+
+    def run(which):
+        for r in range(12):
+            for i in ((0, 1), (1, 0))[r & 1]:
+                for k in which:
+                    nets[k].submit(x[k][i])
+            for i in ((0, 1), (1, 0))[r & 1]:
+                for k in which:
+                    if not np.array_equal(nets[k].collect(), want[k][i]):
+                        bad.append((r, k, i))
+
+    if threads == 1:
+        run((0, 1))
+    else:
+        both = [threading.Thread(target=run, args=((k,),)) for k in range(2)]
+        for t in both:
+            t.start()
+        for t in both:
+            t.join()
+    assert not bad, bad
+    for net in nets:
+        net.close()
