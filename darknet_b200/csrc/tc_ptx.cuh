@@ -53,7 +53,7 @@ __device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t pa
     return done;
 }
 
-// Bounded wait for a loop that a single thread runs (the TMA and MMA roles): no warp traffic at all.
+// Bounded wait for a loop that a single thread runs (the TMA and MMA roles of the halo mode): no warp traffic at all.
 __device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
                                                  long long limit = WAIT_LIMIT_CYCLES)
 {

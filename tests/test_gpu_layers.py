@@ -322,7 +322,7 @@ STEM_CASES = {
 @pytest.mark.parametrize("name", list(STEM_CASES))
 @pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
 def test_conv_stem_tensor_core(name, mode):
-    """First-layer kernel (im2col rows built by the threads, TF32 products): f32 input in Darknet's
+    """First-layer kernel (rows read from the image's patch, TF32 products): f32 input in Darknet's
     layout or channels-last, channels-last output in the mode's storage type.  Asked for Darknet's
     layout on the output side, the same plan falls back to the FP32 kernel."""
     case = conv_case(150, **STEM_CASES[name])
