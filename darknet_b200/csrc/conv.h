@@ -139,6 +139,29 @@ int launch_conv_tc_split(const SplitArgs &a, cudaStream_t s);
 size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes);
 int conv_tc_split_resident(int pair, int cluster);
 
+// ---- conv_fp32_tc.cu : fp32 convolution as three TF32 products on the tensor cores, sums in fp32 registers
+struct alignas(64) Fp32TcArgs {
+    CUtensorMap tmx[4];   // as in TcArgs; boxes of 32 channels x wt x ht x bt pixels
+    CUtensorMap tmy;      // channels-last output, boxes of 32 channels (16 where bn is 32) and the tile's pixels
+    CUtensorMap tmw;      // [2*taps][n_pad][c_pad]: the weights' high halves, then their low halves
+    int c_blocks, taps, last_slices;   // last_slices: MMAs of 8 channels in a tap's last block of 32
+    int bn, n_tiles;      // filters per tile: 32, 64 or 128
+    int wt, ht, bt, tiles_w, tiles_h, total_tiles;
+    int n_pad;
+    const float *x;       // the input and its element strides (planes, and sums that are added up again)
+    long long xs_b, xs_c, xs_h, xs_w;
+    int planes;           // 1: a 1x1 layer over a Darknet tensor, no tmx
+    const float *w;       // the CUDA-core kernel's weights
+    int npg_pad;
+    float *y_nhwc, *y_nchw;
+    int *status;
+    int debug;
+    long long wait_limit;
+    ConvGeom g;
+    ConvEpilogue ep;
+};
+int launch_conv_fp32_tc(const Fp32TcArgs &a, cudaStream_t s);
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
 int encode_tensor_map(CUtensorMap *map, int elem_kind /* 0 f32, 1 bf16, 2 bytes */, int rank, void *base, const uint64_t *dims,
                       const uint64_t *strides_bytes /* rank-1 */, const uint32_t *box, int swizzle_bytes);
@@ -179,6 +202,7 @@ struct dnb_conv_plan {
     float *scale, *shift;    // [n_pad] folded batchnorm / bias
     void *w_tc;              // [taps][n_pad][c_pad] f32 (TF32-rounded) or bf16
     float *w_direct;         // [groups][K][npg_pad]
+    float *w_halves;         // [2*taps][n_pad][c_pad]: high and low TF32 halves (full-precision plans on the tensor cores)
     uint32_t *w_bits;        // [n][taps][cwords]
     float *w_mean;           // [n]
     int npg_pad, cwords;
@@ -213,6 +237,11 @@ struct dnb_conv_plan {
     bool keep_k_order;       // sum K in one order whatever the batch (dense layers of a network with xnor layers): no split, first layers in the im2col order
     bool tc_split;           // launches use the one-tile-per-cluster kernel and its block below
     dnb::SplitArgs sp;
+    bool status_in_block;    // the status word lies behind the weights
+    bool fp32_tc;            // this full-precision plan's layer is one that conv_fp32_tc.cu is made for
+    dnb::Fp32TcArgs ft;      // its launch block, for input ft_x_ptr
+    const void *ft_x_ptr, *ft_y_ptr;   // ... and channels-last output ft_y_ptr (or null)
+    int ft_x_cpitch, ft_y_cpitch, ft_layouts;
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout
     int device;
     long long wait_limit;    // bound of the kernels' waits in cycles (0: the default, about one second)

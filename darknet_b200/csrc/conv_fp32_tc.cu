@@ -1,0 +1,455 @@
+// Full-precision convolution on the sm_100a tensor cores: implicit GEMM as in conv_tc.cu, every fp32 operand as the sum of
+// two TF32 numbers, sums in fp32 registers.
+//
+//   x = xh + xl, w = wh + wl        (xh: x rounded to TF32; xl: the exact rest, rounded to TF32)
+//   x*w = xl*wh + xh*wl + xh*wh     (xl*wl, below 2^-24 of the product, is left out)
+//
+// What bounds the fp32 GEMM of conv_direct.cu is operand pairing and FMA issue on the CUDA cores, 37 TFLOP/s.  Three TF32 products on
+// the tensor pipe have 280 in them.  What has to hold is the precision: a product keeps 2^-24 or so of its value, and
+// the tensor core, which cuts its running sums off instead of rounding them, never adds more than the 32 channels of one tap: then
+// the partial sum leaves TMEM and is added in a register, rounded to nearest.  Error against 64 bits, root mean square over
+// root mean square: see fp32_tc_covers in conv_plan.cu, where it is set beside the CUDA-core kernel's.
+//
+// * Tile: 128 output pixels (a wt x ht x bt box) by BN filters; a step of K is one tap and 32 channels.
+// * Warp 0 loads a step by TMA: BN x 32 of wh and of wl, and of a channels-last input 16 KB as it is.  The input goes through
+//   registers anyway to be split, so its two halves are written to TMEM, where the MMA takes its A operand from: no shared memory for
+//   them, and half of what the MMAs would read there.
+// * A 1x1 layer over a Darknet tensor needs no channels-last copy of it: its channels are planes, so the threads that split fetch their
+//   pixel's 32 values themselves, coalesced along the plane, the next step's while this one's are multiplied (26 x 326 x 56 x 56 -> 34:
+//   71 us, through a copy 78).  With the shifted, short runs of a 3x3 layer's tile the same takes longer than the copy (8 x 64 x 104 x
+//   104 -> 128: 125 us, through a copy 97): lines in flight are more than the first-level cache has beside the ring.
+// * Warps 4-11 split, one half of them the even steps, the other the odd ones: a thread takes its pixel's row, writes 32 columns of
+//   xh and 32 of xl.  (Four warps for all steps: 110 us where eight take 80, 8 x 64 x 104 x 104 -> 128, 3x3; a step's way through a
+//   warp is all latency.)
+// * Warp 1 issues twelve MMAs a step into one of two accumulators.
+// * Warps 12-19 add the finished accumulator to registers, half the filters each, and after the tile's last step scale, shift,
+//   activate and store.  They take the registers that the other warps give up.
+// * A ring of four slots: shared memory for what TMA brings, and 64 columns of TMEM for the split rows, freed together.
+// * A sum that is infinite, not a number, or smaller than the low halves can hold is added up again in fp32, product by product, so
+//   what infinities and NaN in the input become is what the CUDA-core kernel makes of them.
+// * Every wait is bounded as in conv_tc.cu.
+#include <cuda.h>
+
+#include "common.h"
+#include "conv.h"
+#include "device_utils.cuh"
+#include "tc_ptx.cuh"
+
+namespace dnb {
+
+namespace {
+
+constexpr int FT_THREADS = 640;
+// registers a thread: 96 at launch; 128 * (40 + 2 * 96 + 2 * 120) of the launch's 128 * 5 * 96 after the shift
+constexpr int FT_REGS_ISSUE = 40, FT_REGS_SPLIT = 96, FT_REGS_SUM = 120;
+static_assert(FT_REGS_ISSUE + 2 * FT_REGS_SPLIT + 2 * FT_REGS_SUM <= 5 * 96, "no more registers than the launch has");
+constexpr int FT_STAGES = 4;
+constexpr int FT_A_BYTES = 128 * 128;
+constexpr int FT_TMEM = 512;               // four slots of 64 columns, two accumulators of up to 128
+
+struct FtShared {
+    uint64_t full[FT_STAGES];      // a step's tiles are in shared memory
+    uint64_t split[FT_STAGES];     // its input rows are in TMEM
+    uint64_t empty[FT_STAGES];     // its MMAs have retired
+    uint64_t acc_full[2], acc_empty[2];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+enum { FT_WAIT_EMPTY = 101, FT_WAIT_FULL = 102, FT_WAIT_ACC_EMPTY = 103, FT_WAIT_ACC_FULL = 104, FT_WAIT_SPLIT = 105, FT_BAD_BASE = 106 };
+
+// A from TMEM: row i of the operand in lane i, one column per TF32 value.
+__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Nearest TF32; infinities and NaN stay what they are.
+__device__ __forceinline__ float nearest_tf32(float x)
+{
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return __uint_as_float(r & 0xffffe000u);
+}
+
+// One output the way the CUDA-core kernel adds it: fp32, in the order c, kh, kw.
+__device__ __forceinline__ float plain_sum(const Fp32TcArgs &a, int b, int oh, int ow, int f)
+{
+    const ConvGeom &g = a.g;
+    float acc = 0.f;
+    const float *w = a.w + f;
+    for (int c = 0; c < g.c; ++c)
+        for (int kh = 0; kh < g.size; ++kh)
+            for (int kw = 0; kw < g.size; ++kw, w += a.npg_pad) {
+                const int ih = oh * g.stride - g.pad + kh, iw = ow * g.stride - g.pad + kw;
+                const bool in = (unsigned)ih < (unsigned)g.h && (unsigned)iw < (unsigned)g.w;
+                const float x = in ? __ldg(a.x + b * a.xs_b + c * a.xs_c + ih * a.xs_h + iw * a.xs_w) : 0.f;
+                acc = fmaf(x, __ldg(w), acc);
+            }
+    return acc;
+}
+
+// Sums whose size says that the halves may not have carried them: infinite, NaN, or below 2^-90 and not zero (a low half is 2^-12
+// of its operand or less, and two operands of 2^-45 have low halves that are still normal numbers).
+__device__ __forceinline__ bool out_of_range(float v)
+{
+    const uint32_t m = __float_as_uint(v) & 0x7fffffffu;
+    return m - 0x12800000u >= 0x7f800000u - 0x12800000u && m != 0u;
+}
+
+// The 128 threads of one of the two halves that sum meet, and agree on whether to go on.
+__device__ __forceinline__ bool meet(int half, bool fine)
+{
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all) : "r"(1 + half), "r"((uint32_t)fine) : "memory");
+    return all != 0;
+}
+
+template <int ACT>
+__device__ __forceinline__ float apply(float x, int act)
+{
+    if (ACT == DNB_LEAKY) return fmaxf(x, 0.1f * x);
+    return ACT == DNB_LINEAR ? x : activate_fast(x, act);
+}
+
+// BN: filters per tile; PLANES: a 1x1 layer over a Darknet tensor.
+template <int BN, int ACT, bool PLANES>
+__global__ void __launch_bounds__(FT_THREADS, 1)
+conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    constexpr uint32_t B_BYTES = BN * 128, STAGE = FT_A_BYTES + 2 * B_BYTES;
+    constexpr int COLS = BN / 2, LD = COLS < 32 ? COLS : 32;   // filters of one half of the summing warps, columns of a TMEM read and of a staged row
+    constexpr int ROW = LD * 4;
+    const uint32_t ring = smem_u32(smem_raw);
+    if (ring & 1023u) {
+        if (threadIdx.x == 0) atomicCAS(a.status, 0, FT_BAD_BASE);
+        return;
+    }
+    FtShared *sh = reinterpret_cast<FtShared *>(smem_raw + FT_STAGES * STAGE + 2 * 128 * ROW);
+    volatile int *abort_flag = &sh->abort_flag;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < FT_STAGES; ++s) {
+            mbar_init(smem_u32(&sh->full[s]), 1);
+            mbar_init(smem_u32(&sh->split[s]), 4);
+            mbar_init(smem_u32(&sh->empty[s]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&sh->acc_full[i]), 1);
+            mbar_init(smem_u32(&sh->acc_empty[i]), 8);
+        }
+        sh->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)FT_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    launch_dependents();
+    grid_dependency_wait();
+    const uint32_t tmem_base = sh->tmem_base, acc0 = tmem_base + FT_STAGES * 64;
+
+    const int taps = a.taps, c_blocks = a.c_blocks, steps = taps * c_blocks, last_slices = a.last_slices;
+    const int n_tiles = a.n_tiles, total_tiles = a.total_tiles;
+    const int wt = a.wt, ht = a.ht, bt = a.bt, tiles_w = a.tiles_w, tiles_h = a.tiles_h;
+    const long long limit = a.wait_limit;
+    int *status = a.status;
+    const uint32_t full0 = smem_u32(&sh->full[0]), split0 = smem_u32(&sh->split[0]), empty0 = smem_u32(&sh->empty[0]);
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FT_REGS_ISSUE));
+    if (warp == 0) {
+        // ---------------- loads
+        const int ksize = a.g.size, stride = a.g.stride, pad = a.g.pad;
+        const bool withhold = (a.debug & 32) != 0;
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+            const int n0 = tile % n_tiles * BN, pt = tile / n_tiles;
+            const int ow0 = pt % tiles_w * wt, oh0 = pt / tiles_w % tiles_h * ht, b0 = pt / (tiles_w * tiles_h) * bt;
+            for (int tap = 0, kh = 0, kw = 0; tap < taps && ok; ++tap) {
+                const int dh = kh - pad, dw = kw - pad;
+                int ph = 0, qh = dh, pw = 0, qw = dw;
+                if (stride == 2) { ph = dh & 1; qh = (dh - ph) >> 1; pw = dw & 1; qw = (dw - pw) >> 1; }
+                const CUtensorMap *mx = a.tmx + (ph * stride + pw);
+                for (int cb = 0; cb < c_blocks; ++cb) {
+                    ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, FT_WAIT_EMPTY, limit);
+                    if (!ok) break;
+                    if (withhold && tile == (int)blockIdx.x && tap == taps - 1 && cb == c_blocks - 1) { ok = false; break; }
+                    if (elect_one()) {
+                        const uint32_t bar = full0 + 8 * stage, slot = ring + stage * STAGE;
+                        mbar_expect_tx(bar, PLANES ? 2 * B_BYTES : STAGE);
+                        if (!PLANES) tma_load_4d(slot, mx, bar, cb * 32, ow0 + qw, oh0 + qh, b0);
+                        tma_load_3d(slot + FT_A_BYTES, &a.tmw, bar, cb * 32, n0, tap);
+                        tma_load_3d(slot + FT_A_BYTES + B_BYTES, &a.tmw, bar, cb * 32, n0, taps + tap);
+                    }
+                    if (++stage == FT_STAGES) { stage = 0; phase ^= 1; }
+                }
+                if (++kw == ksize) { kw = 0; ++kh; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------- MMAs
+        const uint32_t idesc = mma_idesc<MMA_TF32>(128u, (uint32_t)BN);
+        const uint64_t bh0 = make_smem_desc(ring + FT_A_BYTES, 128), bl0 = make_smem_desc(ring + FT_A_BYTES + B_BYTES, 128);
+        int stage = 0, it = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x)
+            for (int step = 0, cb = 0; step < steps; ++step, ++it) {
+                const int acc = it & 1;
+                ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), ((it >> 1) & 1) ^ 1, abort_flag, status, FT_WAIT_ACC_EMPTY, limit) &&
+                     mbar_wait_warp(split0 + 8 * stage, phase, abort_flag, status, FT_WAIT_SPLIT, limit);
+                if (!ok) break;
+                tc_fence_after();
+                const int slices = cb == c_blocks - 1 ? last_slices : 4;
+                if (elect_one()) {
+                    const uint32_t d = acc0 + acc * BN, ah = tmem_base + stage * 64, al = ah + 32;
+                    const uint64_t off = (uint64_t)(stage * (STAGE >> 4));
+                    // the small products first: they then meet the large ones in a sum that still has room for them
+                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, al + 8 * k, bh0 + off + 2 * k, idesc, k != 0);
+                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, ah + 8 * k, bl0 + off + 2 * k, idesc, 1u);
+                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, ah + 8 * k, bh0 + off + 2 * k, idesc, 1u);
+                    umma_commit(empty0 + 8 * stage);
+                    umma_commit(smem_u32(&sh->acc_full[acc]));
+                }
+                if (++cb == c_blocks) cb = 0;
+                if (++stage == FT_STAGES) { stage = 0; phase ^= 1; }
+            }
+        __syncwarp();
+    }
+    } else if (warp < 12) {
+        // ---------------- split: thread m's row of the input tile (128-byte swizzle) to TMEM lane m
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FT_REGS_SPLIT));
+        const int m = (warp & 3) * 32 + lane, q_xor = m & 7;
+        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+        const int mine = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        const long long count = (long long)mine * steps;
+        const int channels = a.g.c;
+        const long long xs_c = a.xs_c;
+        float x[PLANES ? 32 : 1];
+        // PLANES: this thread's 32 values of a step, zero beyond the plane and the channels; steps are asked for in order
+        int tile = blockIdx.x, in_tile = warp < 8 ? 0 : 1;
+        auto fetch = [&]() {
+            while (in_tile >= steps) { in_tile -= steps; tile += gridDim.x; }
+            const int pt = tile / n_tiles, pix = pt % tiles_w * wt + m % wt, b = pt / (tiles_w * tiles_h) * bt + m / (wt * ht), c0 = 32 * in_tile;
+            const float *p = a.x + (long long)b * a.xs_b + c0 * xs_c + pix;
+            const int live = pix < a.g.w && m / wt % ht == 0 && b < a.g.batch ? channels - c0 : 0;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) x[PLANES ? j : 0] = j < live ? __ldg(p + j * xs_c) : 0.f;
+            in_tile += 2;
+        };
+        if (PLANES && (warp < 8 ? 0 : 1) < count) fetch();
+        for (long long it = warp < 8 ? 0 : 1; it < count; it += 2) {
+            const int stage = (int)it & (FT_STAGES - 1);
+            if (!mbar_wait(full0 + 8 * stage, (uint32_t)(it / FT_STAGES) & 1, abort_flag, status, FT_WAIT_FULL, 0, limit)) break;
+            tc_fence_after();   // the slot's columns were last read by MMAs whose retirement let this load be issued
+            const uint8_t *row = smem_raw + stage * STAGE + m * 128;
+            const uint32_t dst = tmem_base + lane_base + stage * 64;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float v[4];
+                    if (PLANES) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[e] = x[PLANES ? 16 * h + 4 * q + e : 0];
+                    } else {
+                        const float4 f = *reinterpret_cast<const float4 *>(row + (((4 * h + q) ^ q_xor) << 4));
+                        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float xh = nearest_tf32(v[e]);
+                        hi[4 * q + e] = __float_as_uint(xh);
+                        lo[4 * q + e] = __float_as_uint(round_tf32(v[e] - xh));
+                    }
+                }
+                tmem_st16(dst + 16 * h, hi);
+                tmem_st16(dst + 32 + 16 * h, lo);
+            }
+            if (PLANES && it + 2 < count) fetch();
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(split0 + 8 * stage);
+        }
+    } else {
+        // ---------------- sums and epilogue
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FT_REGS_SUM));
+        const int half = warp < 16 ? 0 : 1, col0 = half * COLS;
+        const int quarter = warp & 3, m = quarter * 32 + lane;
+        uint8_t *const staged = smem_raw + FT_STAGES * STAGE + half * 128 * ROW, *const my_row = staged + m * ROW;
+        const int q_xor = (m >> (ROW == 128 ? 0 : 1)) & (ROW / 16 - 1);   // the store map's swizzle
+        const bool stores = quarter == 0 && lane == 0;
+        const int wl = m % wt, hl = (m / wt) % ht, bl = m / (wt * ht);
+        const ConvGeom g = a.g;
+        const int act = a.ep.activation;
+        int it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+            float sum[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+            for (int step = 0; step < steps; ++step, ++it) {
+                const int acc = it & 1;
+                ok = mbar_wait(smem_u32(&sh->acc_full[acc]), (it >> 1) & 1, abort_flag, status, FT_WAIT_ACC_FULL, 0, limit);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t src = acc0 + acc * BN + col0 + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+                for (int c = 0; c < COLS; c += LD) {
+                    uint32_t r[LD];
+#pragma unroll
+                    for (int u = 0; u < LD; u += 16) tmem_ld16(src + c + u, *reinterpret_cast<uint32_t(*)[16]>(&r[u]));
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < LD; ++j) sum[c + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[acc]));
+            }
+            if (!meet(half, ok && !*abort_flag)) break;
+            const int n0 = tile % n_tiles * BN + col0, pt = tile / n_tiles;
+            const int ow0 = pt % tiles_w * wt, oh0 = pt / tiles_w % tiles_h * ht, b0 = pt / (tiles_w * tiles_h) * bt;
+            const int ow = ow0 + wl, oh = oh0 + hl, b = b0 + bl;
+            const bool inside = ow < g.out_w && oh < g.out_h && b < g.batch;
+            const size_t plane = (size_t)g.out_h * g.out_w, pix = (size_t)oh * g.out_w + ow;
+            float *nchw = a.y_nchw && inside ? a.y_nchw + ((size_t)b * g.n + n0) * plane + pix : nullptr;
+            const int real = g.n - n0;
+            uint32_t again[(COLS + 31) / 32] = {};              // sums that fp32 has to add up itself
+#pragma unroll
+            for (int c = 0; c < COLS; c += LD) {
+                if (a.y_nhwc && (c > 0 || it > steps)) {        // the row's last store has been read
+                    if (stores) tma_store_wait_read0();
+                    meet(half, true);
+                }
+#pragma unroll
+                for (int q = c / 4; q < (c + LD) / 4; ++q) {
+                    float v[4];
+                    const bool in = n0 + 4 * q < a.n_pad;       // whole quads: n_pad is a multiple of 16
+                    const float4 sc = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.scale + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 sf = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.shift + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float t = sum[4 * q + e];
+                        if (out_of_range(t)) again[q / 8] |= 1u << (4 * (q & 7) + e);
+                        v[e] = 4 * q + e < real ? apply<ACT>(t * scv[e] + sfv[e], act) : 0.f;
+                    }
+                    if (a.y_nhwc) *reinterpret_cast<float4 *>(my_row + (((q - c / 4) ^ q_xor) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+                    if (nchw) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (4 * q + e < real) nchw[(size_t)(4 * q + e) * plane] = v[e];
+                    }
+                }
+                if (again[c / 32] && inside) {                  // rarely: into the staged row and the plane instead
+                    uint32_t bits = again[c / 32];
+                    while (bits) {
+                        const int j = (c & ~31) + __ffs(bits) - 1;
+                        bits &= bits - 1;
+                        if (j >= real) break;
+                        const float t = apply<ACT>(plain_sum(a, b, oh, ow, n0 + j) * __ldg(a.ep.scale + n0 + j) + __ldg(a.ep.shift + n0 + j), act);
+                        if (a.y_nhwc) *reinterpret_cast<float *>(my_row + ((((j - c) / 4) ^ q_xor) << 4) + 4 * ((j - c) & 3)) = t;
+                        if (nchw) nchw[(size_t)j * plane] = t;
+                    }
+                }
+                if (a.y_nhwc) {
+                    fence_async_smem();
+                    meet(half, true);
+                    // the TMA unit clips the box at the tensor's extents: ragged tiles need no predicates
+                    if (stores && c < real) { tma_store_4d(&a.tmy, smem_u32(staged), n0 + c, ow0, oh0, b0); tma_store_commit(); }
+                }
+            }
+        }
+        if (stores) tma_store_wait_all();
+    }
+
+    // ---------------- teardown (also the abort path)
+    if (*abort_flag) {   // give loads that are still in flight time to land before shared memory is released
+        const long long t0 = clock64();
+        while (clock64() - t0 < 4000000LL) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FT_TMEM) : "memory");
+    }
+}
+
+template <int BN, int ACT, bool PLANES>
+int launch_one(const Fp32TcArgs &a, cudaStream_t s)
+{
+    const size_t smem = tmem_smem(FT_STAGES * (size_t)(FT_A_BYTES + 2 * BN * 128) + 2 * 128 * (BN < 64 ? 64 : 128) + sizeof(FtShared), FT_TMEM);
+    DNB_CUDA(cudaFuncSetAttribute(conv_fp32_tc_kernel<BN, ACT, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.total_tiles < sm_count() ? a.total_tiles : sm_count()));
+    cfg.blockDim = dim3(FT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    DNB_CUDA(cudaLaunchKernelEx(&cfg, conv_fp32_tc_kernel<BN, ACT, PLANES>, a));
+    DNB_LAUNCH_CHECK("conv_fp32_tc");
+    return DNB_OK;
+}
+
+template <int BN, bool PLANES>
+int launch_act(const Fp32TcArgs &a, cudaStream_t s)
+{
+    switch (a.ep.activation) {
+    case DNB_LINEAR: return launch_one<BN, DNB_LINEAR, PLANES>(a, s);
+    case DNB_LEAKY: return launch_one<BN, DNB_LEAKY, PLANES>(a, s);
+    default: return launch_one<BN, -1, PLANES>(a, s);
+    }
+}
+
+template <int BN>
+int launch_bn(const Fp32TcArgs &a, cudaStream_t s)
+{
+    return a.planes ? launch_act<BN, true>(a, s) : launch_act<BN, false>(a, s);
+}
+
+}  // namespace
+
+int launch_conv_fp32_tc(const Fp32TcArgs &a, cudaStream_t s)
+{
+    switch (a.bn) {
+    case 32: return launch_bn<32>(a, s);
+    case 64: return launch_bn<64>(a, s);
+    default: return launch_bn<128>(a, s);
+    }
+}
+
+}  // namespace dnb

@@ -18,6 +18,39 @@ enum { K_TC_TF32 = 0, K_TC_BF16 = 1, K_DIRECT = 2, K_XNOR = 3 };
 static const char *const kKernelNames[] = {"tc_tf32", "tc_bf16", "direct_fp32", "xnor_popc"};
 static const char kXnorTcName[] = "xnor_tc";
 
+// Layers of full-precision plans that may run as three TF32 products on the tensor cores (conv_fp32_tc.cu): sums of 128 products and
+// more, where they are clearly no further from 64-bit sums than the CUDA-core kernel's, which rounds at every product (at 64 they are level).
+// Measured as the root mean square of the error over that of the layer, CUDA cores / tensor cores, for K products, in units of 1e-7:
+//   K = 16  0.80 / 1.02     K = 32  1.06 / 1.29     K = 64  1.45 / 1.30     K = 144  2.1 / 1.2     K = 576  4.3 / 1.5     K = 4608  11.4 / 2.4
+// (summed in TMEM over 64 channels at a time instead of 32: 3.6 at any of these, over 128: 7.8).
+static bool fp32_tc_covers(const ConvGeom &g)
+{
+    return g.groups == 1 && g.stride <= 2 && g.c >= 8 && g.c * g.size * g.size >= 128 && (long long)g.batch * g.h * g.w < (1LL << 31);
+}
+
+// Whether they should.  Microseconds of either kernel, measured on B200: a step of 32 channels of a tap takes a tile 0.72 on the tensor
+// cores (copies: the copy of a Darknet tensor comes on top); a block of the CUDA-core kernel's large tiles 64 ns a product where four share
+// an SM, one of its small ones 17.5 and 11.5 more for every other block there, its slabs of up to 16 filters 6 a product and filter.
+// 8 x 64 x 104 x 104 -> 128, 3x3: 317 -> 85 us (352 -> 97 from Darknet's layout); 1 x 512 x 13 x 13 -> 1024 133 -> 96; 8 x 100 x 38 x 38
+// -> 70, stride 2, from Darknet's layout would be 27 -> 34.  DNB_FP32_TC: 0 never, 1 whenever it can.
+static bool fp32_tc_pays(const ConvGeom &g, bool copies)
+{
+    if (const char *e = getenv("DNB_FP32_TC")) return atoi(e) != 0;
+    const double npix = (double)g.batch * g.out_h * g.out_w, K = (double)g.c * g.size * g.size, sms = sm_count();
+    const int bn = g.n <= 32 ? 32 : g.n <= 64 ? 64 : 128;
+    const double tiles = ceil(npix / 128) * ceil((double)g.n / bn);
+    double tc = 6 + ceil(tiles / sms) * (0.72 * g.size * g.size * ((g.c + 31) / 32) + 0.012 * bn);
+    if (copies) tc += 3 + 8.0 * g.batch * g.c * g.h * g.w / 5e6;
+    double direct;
+    if (g.n <= 16 || (g.size != 1 && g.size != 3)) direct = 5 + K * 0.006 * (g.n < 4 ? 4 : g.n) * ceil(npix / 128 / sms);
+    else if (ceil(npix / 128) * ceil(g.n / (g.n > 32 ? 64.0 : 32.0)) >= 2 * sms) {
+        const double b = ceil(npix / 128) * ceil(g.n / (g.n > 32 ? 64.0 : 32.0)) / sms;
+        direct = 6 + K * (g.n <= 32 ? 0.052 * b : b < 4 ? 0.04 + 0.05 * ceil(b) : 0.064 * b);
+    }
+    else direct = 5 + K * (0.006 + 0.0115 * ceil(ceil(npix / 32) * ceil(g.n / 32.0) / sms));
+    return tc < direct;
+}
+
 extern "C" int dnb_conv_plan_create(const dnb_conv_desc *d, int mode, dnb_conv_plan **out)
 {
     if (!d || !out) DNB_FAIL(DNB_EINVAL, "conv plan: null argument");
@@ -56,6 +89,7 @@ extern "C" int dnb_conv_plan_create(const dnb_conv_desc *d, int mode, dnb_conv_p
     // RGB first layers of the TF32 / BF16 modes: tensor cores, rows read from the patch in shared memory (DNB_STEM_TC=0 keeps the FP32 kernel)
     const char *stem_env = getenv("DNB_STEM_TC");
     p->stem_tc = p->kernel == K_DIRECT && mode != DNB_MODE_FP32 && !d->xnor && conv_stem_tc_covers(p->g) && !(stem_env && atoi(stem_env) == 0);
+    p->fp32_tc = p->kernel == K_DIRECT && mode == DNB_MODE_FP32 && fp32_tc_covers(p->g) && fp32_tc_pays(p->g, false);
     // xnor layers: int8 sign tensors through the tensor cores (kind::i8, exact int32 sums) unless DNB_XNOR_TC=0 asks
     // for the bit-packed popcount kernel; strides above 2 have no lattice maps and stay with the popcount kernel
     {
@@ -76,7 +110,7 @@ dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch)
     q->borrowed = true;
     q->x_nhwc_scratch = nullptr; q->x_bits = nullptr; q->x_i8 = nullptr;
     q->x_nhwc_bytes = q->x_bits_bytes = q->x_i8_bytes = 0;
-    q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = nullptr;
+    q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = q->ft_x_ptr = nullptr;
     q->sign_consumer = nullptr; q->signs_given = false; q->signs_of = nullptr;
     return q;
 }
@@ -91,7 +125,7 @@ extern "C" void dnb_conv_plan_destroy(dnb_conv_plan *p)
     }
     cudaFree(p->scale); cudaFree(p->shift); cudaFree(p->w_tc); cudaFree(p->w_direct); cudaFree(p->w_bits);
     cudaFree(p->w_mean); cudaFree(p->x_nhwc_scratch); cudaFree(p->x_bits); cudaFree(p->w_i8); cudaFree(p->scale_i8); cudaFree(p->x_i8);
-    if (!p->status_shared) cudaFree(p->status);
+    if (!p->status_shared && !p->status_in_block) cudaFree(p->status);
     delete p;
 }
 
@@ -113,8 +147,18 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
+    else if (p->fp32_tc && p->ft_x_ptr)
+        snprintf(buf, len, "%s three_tf32_products bn=%d tile=%dx%dx%d tiles=%d", dnb_conv_plan_kernel(p), p->ft.bn, p->ft.wt, p->ft.ht, p->ft.bt, p->ft.total_tiles);
     else
         snprintf(buf, len, "%s", dnb_conv_plan_kernel(p));
+    return DNB_OK;
+}
+
+static int ensure_status(dnb_conv_plan *p)
+{
+    if (p->status) return DNB_OK;
+    DNB_CUDA(cudaMalloc((void **)&p->status, sizeof(int)));
+    DNB_CUDA(cudaMemset(p->status, 0, sizeof(int)));
     return DNB_OK;
 }
 
@@ -151,6 +195,30 @@ __global__ void repack_tc_kernel(const float *__restrict__ w, T *__restrict__ ou
         } else {
             reinterpret_cast<__nv_bfloat16 *>(out)[i] = __float2bfloat16_rn(v);
         }
+    }
+}
+
+// the same layout twice: the weights rounded to TF32, and what the rounding left, rounded to TF32.  A status word behind them starts at 0.
+__global__ void split_weights_kernel(const float *__restrict__ w, float *__restrict__ out, int n, int c, int taps, int n_pad, int c_pad, int *status)
+{
+    if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    const size_t half = (size_t)taps * n_pad * c_pad;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < half; i += (size_t)gridDim.x * blockDim.x) {
+        const int cc = (int)(i % c_pad);
+        const size_t r = i / c_pad;
+        const int f = (int)(r % n_pad), t = (int)(r / n_pad);
+        float hi = 0.f, lo = 0.f;
+        if (f < n && cc < c) {
+            const float v = __ldg(w + ((size_t)f * c + cc) * taps + t);
+            uint32_t u = __float_as_uint(v);
+            if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & ~0x1fffu;
+            hi = __uint_as_float(u);
+            u = __float_as_uint(v - hi);
+            if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & ~0x1fffu;
+            lo = __uint_as_float(u);
+        }
+        out[i] = hi;
+        out[half + i] = lo;
     }
 }
 
@@ -280,8 +348,17 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
         repack_tc_kernel<__nv_bfloat16><<<grid_of(total), 256>>>(raw, dev, d.n, d.c, taps, p->n_pad, p->c_pad);
     } else if (p->kernel == K_DIRECT) {
         const size_t total = (size_t)d.groups * K * p->npg_pad;
-        DNB_TRY(device_alloc(&p->w_direct, total));
+        // one allocation: the CUDA-core kernel's weights, and for the tensor cores their halves and the status word
+        const size_t first = (total + 63) / 64 * 64, half = p->fp32_tc && !p->keep_k_order ? (size_t)taps * p->n_pad * p->c_pad : 0;
+        if (p->status_in_block) { p->status = nullptr; p->status_in_block = false; }
+        DNB_TRY(device_alloc(&p->w_direct, half ? first + 2 * half + 1 : total));
         repack_direct_kernel<<<grid_of(total), 256>>>(raw, p->w_direct, d.groups, npg, K, p->npg_pad);
+        if (half) {
+            p->w_halves = p->w_direct + first;
+            int *word = nullptr;
+            if (!p->status) { word = p->status = reinterpret_cast<int *>(p->w_halves + 2 * half); p->status_in_block = true; }
+            split_weights_kernel<<<grid_of(half), 256>>>(raw, p->w_halves, d.n, d.c, taps, p->n_pad, p->c_pad, word);
+        }
     } else {
         DNB_TRY(device_alloc(&p->w_bits, (size_t)d.n * taps * p->cwords));
         DNB_TRY(device_alloc(&p->w_mean, (size_t)d.n));
@@ -299,7 +376,7 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
     DNB_CUDA(cudaDeviceSynchronize());   // the staging copy is released on return
     p->params_set = true;
     // The launch block caches a tensor map over the weights just replaced: have the next forward rebuild it.
-    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = nullptr;
+    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = p->ft_x_ptr = nullptr;
     return DNB_OK;
 }
 
@@ -311,7 +388,7 @@ extern "C" int dnb_conv_plan_set_diagnostics(dnb_conv_plan *p, long long wait_li
     if (!p || wait_limit_cycles < 0) DNB_FAIL(DNB_EINVAL, "conv diagnostics: bad argument");
     p->wait_limit = wait_limit_cycles;
     p->debug_bits = debug_bits;
-    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = nullptr;
+    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = p->ft_x_ptr = nullptr;
     return DNB_OK;
 }
 
@@ -450,14 +527,6 @@ SplitPlan choose_split(const SplitQuery &q, const ConvGeom &g, int only_s, bool 
 
 }  // namespace
 
-static int ensure_status(dnb_conv_plan *p)
-{
-    if (p->status) return DNB_OK;
-    DNB_CUDA(cudaMalloc((void **)&p->status, sizeof(int)));
-    DNB_CUDA(cudaMemset(p->status, 0, sizeof(int)));
-    return DNB_OK;
-}
-
 // Input maps of a convolution: lattice (ph, pw) of the input holds rows ph, ph+stride, ... and columns pw, pw+stride, ...
 static int encode_input_maps(CUtensorMap *maps, const ConvGeom &g, const dnb_tensor *x, int kind, int es, int c_pad, const uint32_t *box, int row_bytes)
 {
@@ -482,6 +551,68 @@ static int encode_weight_map(CUtensorMap *map, const dnb_conv_plan *p, int kind,
     uint64_t strides[2] = {(uint64_t)c_pad * es, (uint64_t)c_pad * es * p->n_pad};
     uint32_t box[3] = {(uint32_t)bk, (uint32_t)rows, 1u};
     return encode_tensor_map(map, kind, 3, kind == 2 ? (void *)p->w_i8 : p->w_tc, dims, strides, box, row_bytes);
+}
+
+// Room for the channels-last copy of a Darknet tensor.  False where there is no memory, or where the stream is being captured and
+// nothing can be allocated: the CUDA-core kernel needs none.
+static bool fp32_tc_room(dnb_conv_plan *p, cudaStream_t s)
+{
+    if (p->x_nhwc_bytes) return true;   // a plan's need is always the same
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const size_t need = (size_t)p->g.batch * p->g.h * p->g.w * p->c_pad * sizeof(float);
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone || cudaMalloc(&p->x_nhwc_scratch, need) != cudaSuccess) {
+        cudaGetLastError();
+        p->x_nhwc_scratch = nullptr;
+        return false;
+    }
+    p->x_nhwc_bytes = need;
+    return true;
+}
+
+static int build_fp32_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_cpitch, bool nchw_out)
+{
+    Fp32TcArgs &a = p->ft;
+    ConvGeom g = p->g;
+    a.taps = g.size * g.size;
+    a.c_blocks = (p->c_pad + 31) / 32;
+    a.last_slices = (p->c_pad - 32 * (a.c_blocks - 1)) / 8;
+    a.bn = p->n_pad <= 32 ? 32 : p->n_pad <= 64 ? 64 : 128;
+    a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
+    a.planes = x->layout == DNB_NCHW ? 1 : 0;
+    const bool by_image = nchw_out || a.planes;
+    if (g.size == 1 && g.stride == 1 && g.pad == 0) {   // pixels in one row; of the whole batch where no tensor has planes
+        g.w = g.out_w = g.w * g.h * (by_image ? 1 : g.batch);
+        g.h = g.out_h = 1;
+        if (!by_image) g.batch = 1;
+    }
+    a.x = (const float *)x->data;
+    if (a.planes) { a.xs_w = 1; a.xs_h = g.w; a.xs_c = (long long)g.h * g.w; a.xs_b = g.c * a.xs_c; }
+    else { a.xs_c = 1; a.xs_w = x->cpitch; a.xs_h = (long long)g.w * x->cpitch; a.xs_b = g.h * a.xs_h; }
+    a.w = p->w_direct; a.npg_pad = p->npg_pad;
+    pick_pixel_tile(g, by_image, &a.wt, &a.ht, &a.bt);
+    a.tiles_w = (g.out_w + a.wt - 1) / a.wt;
+    a.tiles_h = (g.out_h + a.ht - 1) / a.ht;
+    a.total_tiles = a.n_tiles * a.tiles_w * a.tiles_h * ((g.batch + a.bt - 1) / a.bt);
+    a.n_pad = p->n_pad;
+    a.g = g;
+    a.debug = p->debug_bits;
+    a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
+    const uint32_t box[4] = {32u, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
+    if (!a.planes) DNB_TRY(encode_input_maps(a.tmx, g, x, 0, 4, p->c_pad, box, 128));
+    uint64_t dims[3] = {(uint64_t)p->c_pad, (uint64_t)p->n_pad, (uint64_t)(2 * a.taps)};
+    uint64_t strides[2] = {(uint64_t)p->c_pad * 4, (uint64_t)p->c_pad * 4 * p->n_pad};
+    uint32_t wbox[3] = {32u, (uint32_t)a.bn, 1u};
+    DNB_TRY(encode_tensor_map(&a.tmw, 0, 3, p->w_halves, dims, strides, wbox, 128));
+    if (y_nhwc) {
+        const size_t opix = (size_t)y_cpitch * 4;
+        const int n8 = round_up(g.n, 8), cols = a.bn / 2 < 32 ? a.bn / 2 : 32;
+        uint64_t ydims[4] = {(uint64_t)(n8 < y_cpitch ? n8 : y_cpitch), (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
+        uint64_t ystrides[3] = {opix, opix * g.out_w, opix * g.out_w * g.out_h};
+        uint32_t ybox[4] = {(uint32_t)cols, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
+        DNB_TRY(encode_tensor_map(&a.tmy, 0, 4, y_nhwc, ydims, ystrides, ybox, cols * 4));
+    }
+    p->ft_x_ptr = x->data; p->ft_x_cpitch = x->cpitch; p->ft_y_ptr = y_nhwc; p->ft_y_cpitch = y_cpitch; p->ft_layouts = 2 * a.planes + (nchw_out ? 1 : 0);
+    return DNB_OK;
 }
 
 static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeom &g, const SplitPlan &sp, int kind, int es,
@@ -946,6 +1077,22 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         // offsets inside an image take rows of less than 2^25 values
         const bool rows = (p->keep_k_order || a.xs_h >= (1LL << 31) / 64) && conv_stem_rows_covers(g, y_dtype);
         return rows ? launch_conv_stem_rows(a, s) : launch_conv_stem_tc(a, s);
+    }
+    const bool copies = x->layout == DNB_NCHW && !(g.size == 1 && g.stride == 1 && g.pad == 0);
+    if (p->fp32_tc && !p->keep_k_order && x->dtype == DNB_F32 && (!y_nhwc || y_dtype == DNB_F32) && (!copies || (fp32_tc_pays(g, true) && fp32_tc_room(p, s)))) {
+        dnb_tensor xin = *x;
+        if (copies) {
+            xin.data = p->x_nhwc_scratch; xin.layout = DNB_NHWC; xin.cpitch = p->c_pad;
+            DNB_TRY(launch_convert(x, &xin, 0, 0, 0, s));
+        }
+        const int layouts = (xin.layout == DNB_NCHW ? 2 : 0) + (y_nchw ? 1 : 0);
+        if (p->ft_x_ptr != xin.data || p->ft_x_cpitch != xin.cpitch || p->ft_y_ptr != y_nhwc || p->ft_y_cpitch != y_cpitch || p->ft_layouts != layouts)
+            DNB_TRY(build_fp32_tc_args(p, &xin, y_nhwc, y_cpitch, y_nchw != nullptr));
+        Fp32TcArgs &a = p->ft;
+        a.y_nhwc = (float *)y_nhwc; a.y_nchw = y_nchw;
+        a.status = p->status;
+        a.ep = ep;
+        return launch_conv_fp32_tc(a, s);
     }
     if (p->kernel == K_DIRECT) {   // also a first-layer plan asked for Darknet's layout or given bf16 input
         DirectArgs a;

@@ -33,6 +33,89 @@ def test_fp32_gemm_tiles(name, layouts):
     parity(got, oracle_conv(case), 1e-5)
 
 
+FP32_SPLIT = {   # three TF32 products: tiles of 32, 64 and 128 filters, ragged maps, K of one step and of a part of one, odd filters
+    "32_filters_15_channels": dict(b=2, c=15, h=9, w=13, n=18, size=3),
+    "64_filters_stride2_odd_map": dict(b=3, c=40, h=21, w=17, n=50, size=3, stride=2, act="logistic"),
+    "128_filters_and_one": dict(b=1, c=33, h=11, w=19, n=129, size=3, act="linear"),
+    "1x1_two_tiles_and_a_bit": dict(b=3, c=136, h=9, w=11, n=255, size=1),
+    "1x1_one_pixel": dict(b=1, c=200, h=1, w=1, n=255, size=1),
+    "5x5_no_padding": dict(b=2, c=8, h=12, w=9, n=33, size=5, pad=0),
+    "several_tiles_an_sm": dict(b=4, c=16, h=150, w=141, n=40, size=3),
+}
+
+
+@pytest.mark.parametrize("name", list(FP32_SPLIT))
+@pytest.mark.parametrize("layouts", [("nchw", "nchw"), ("nchw", "nhwc"), ("nhwc", "nhwc"), ("both", "nchw")])
+def test_full_precision_on_the_tensor_cores(name, layouts, monkeypatch):
+    """Each product is exact to about 2^-24 of its value and the sums of 32 channels are rounded as fp32 sums are; tolerance as for the
+    CUDA-core kernel, and the root mean square of the error against 64-bit sums is no larger than that kernel's (a fifth is the
+    spread of layers of a few hundred values)."""
+    import numpy as np
+    import torch
+    case = conv_case(720, **dict(FP32_SPLIT[name], act="linear"))
+    act = FP32_SPLIT[name].get("act", "leaky")
+    t = {k: torch.from_numpy(np.asarray(case[k], np.float64)) for k in ("x", "w", "biases", "scales", "mean", "var")}
+    exact = torch.nn.functional.conv2d(t["x"], t["w"], stride=case["stride"], padding=case["pad"])
+    col = lambda v: v[:, None, None]  # noqa: E731
+    exact = ((exact - col(t["mean"])) / (col(t["var"]).sqrt() + 1e-6) * col(t["scales"]) + col(t["biases"])).numpy()
+    rms, layout = {}, "nchw" if layouts[0] == "both" else layouts[0]
+    for knob in ("0", "1"):
+        monkeypatch.setenv("DNB_FP32_TC", knob)
+        plan, got, second = run_conv(case, dn.MODE_FP32, layout, layouts[1], both=layouts[0] == "both")
+        assert plan.kernel == "direct_fp32" and ("three_tf32_products" in plan.describe()) == (knob == "1"), plan.describe()
+        assert second is None or np.array_equal(got, second)
+        parity(got, exact, 1e-5)
+        rms[knob] = np.sqrt(((got - exact) ** 2).mean())
+    assert rms["1"] <= 1.2 * rms["0"], rms
+    case["act"] = act
+    _, got, _ = run_conv(case, dn.MODE_FP32, layout, layouts[1])
+    parity(got, oracle_conv(case), 1e-5)
+
+
+def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
+    """Infinities, NaN, values whose high half or whose sum overflows, and sums too small for low halves: bit for bit what the
+    CUDA-core kernel makes of them where that is not finite or tiny, close to it elsewhere."""
+    import numpy as np
+    case = conv_case(721, b=2, c=16, h=14, w=15, n=40, size=3, act="linear", bn=False)
+    case["biases"][...] = 0
+    x = case["x"]
+    x[0, 3, 4, 5], x[0, 0, 10, 2], x[1, 7, 0, 0], x[1, 2, 8, 8] = np.inf, np.nan, -np.inf, np.float32(3.4028235e38)
+    case["w"][5, :, 1, 1] = 0                                     # infinity times zero
+    x[1, :, 10:14, 10:15] *= np.float32(1e-33)
+    out = {}
+    for layout in ("nchw", "nhwc"):
+        for knob in ("0", "1"):
+            monkeypatch.setenv("DNB_FP32_TC", knob)
+            plan, out[knob], _ = run_conv(case, dn.MODE_FP32, "nchw", layout)
+            assert ("three_tf32_products" in plan.describe()) == (knob == "1")
+        odd = ~np.isfinite(out["0"])
+        tiny = np.abs(out["0"]) < 2.0 ** -91
+        assert odd.any() and tiny.any() and np.array_equal(np.isfinite(out["1"]), ~odd)
+        assert np.array_equal(out["0"][odd], out["1"][odd], equal_nan=True) and np.array_equal(out["0"][tiny], out["1"][tiny])
+        plain = ~odd & ~tiny & (np.abs(out["0"]) < 1e30)
+        assert np.abs(out["0"][plain] - out["1"][plain]).max() <= 1e-5 * np.abs(out["0"][plain]).max()
+
+
+def test_full_precision_wait_expiry(monkeypatch):
+    """A withheld operand load: the bounded wait runs out, the call reports it, and the next launch is right."""
+    import torch
+    monkeypatch.setenv("DNB_FP32_TC", "1")
+    case = conv_case(722, b=2, c=48, h=20, w=20, n=100, size=3)
+    plan = dn.ConvPlan(2, 48, 20, 20, 100, 3, 1, 1, 1, True, "leaky", False, dn.MODE_FP32)
+    plan.set_params(case["w"], case["biases"], case["scales"], case["mean"], case["var"])
+    x = torch.from_numpy(case["x"]).cuda()
+    y = torch.empty(2, 100, 20, 20, device="cuda")
+    plan.set_diagnostics(4_000_000, 32)
+    plan.forward(dn.as_tensor(x, dn.NCHW), dn.as_tensor(y, dn.NCHW))
+    with pytest.raises(dn.DarknetB200Error) as e:
+        plan.check_status()
+    assert e.value.status == dn.ETIMEOUT
+    plan.set_diagnostics(0, 0)
+    plan.forward(dn.as_tensor(x, dn.NCHW), dn.as_tensor(y, dn.NCHW))
+    plan.check_status()
+    parity(y.cpu().numpy(), oracle_conv(case), 1e-5)
+
+
 @pytest.mark.parametrize("name", ["groups_of_four_channels", "groups_off_four_channel_boundary", "slab_4"])
 def test_grouped_layers_with_bf16_storage(name):
     """A grouped layer of a BF16 network: bf16 in, fp32 sums, bf16 out.  The input is rounded first, so what is left is the
