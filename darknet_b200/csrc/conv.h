@@ -86,10 +86,11 @@ struct alignas(64) TcArgs {
     int debug;            // timing experiments only (DNB_TC_DEBUG): 1 no residual loads, 2 no output stores, 4 no wait before a residual request, 8 empty epilogue, 16 no MMAs;
                           // 32 (dnb_conv_plan_set_diagnostics): each CTA withholds the last operand load of its first tile, so a bounded wait runs out
     long long wait_limit; // bound of every device-side wait, SM clock cycles
-    int stage_bufs;       // staging buffers of the epilogue: 2, or 4 with a fused residual (tiles land in them first)
+    int stage_bufs;       // staging buffers of the epilogue: 2, or 4 with a fused residual (it lands in them first), 3 with signs, 0 where two groups write Darknet's layout only
     int pair;             // 1: clusters of two CTAs share every MMA (cta_group::2); total_tiles then counts PAIRS of pixel tiles,
                           // b_bytes and the weight map's box cover half a filter tile, bn is 256
     int ctas_per_sm;      // 2 for narrow tiles (TMEM and shared memory are sized so that two CTAs share an SM), else 1
+    int epi_groups;       // groups of four epilogue warps: 2 where a CTA has its SM to itself and staged rows are 128 bytes, else 1
     int a_bytes, b_bytes; // shared-memory bytes of one stage's activation / weight tile (1024-multiples)
     int store_row_bytes;  // bytes of one staged output row (128, 64 or 32) = swizzle span of tmy
     int n_pad;            // length of the scale / shift vectors
@@ -98,7 +99,7 @@ struct alignas(64) TcArgs {
     int y_dtype, y_cpitch;
     float *y_nchw;
     int *status;          // device word: 0, or the code of the wait that expired
-    int warp_stores;      // 1: every epilogue warp stores its own 32 rows (tmy_warp); 0: one store per chunk by one thread (tmy)
+    int warp_stores;      // one group, 1: every epilogue warp stores its own 32 rows (tmy_warp); 0: one store per chunk by one thread (tmy)
     void *sign_out;       // int8 kind: also write the output's signs here ([b][h][w][sign_cpitch] bytes), or null
     int sign_cpitch;
     ConvGeom g;

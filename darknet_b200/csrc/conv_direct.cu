@@ -181,12 +181,6 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool in)  
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool in)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // KS: 1 or 3.  (BM / TM) * (BN / TN) threads.
 template <typename TX, typename TY, int KS, int BM, int BN, int TM, int TN, bool VEC>
@@ -254,7 +248,7 @@ conv_fp32_gemm_kernel(const __grid_constant__ DirectArgs a)
             if (KC * BN / 4 % THREADS == 0 || i < KC * BN / 4) {
                 // npg_pad is a multiple of 32: four filters lie inside the packed row or beyond it together
                 const bool in = c < cpg && f0 + 4 * q < a.npg_pad;
-                cp_async16(&b_s[st][kk][4 * q], in ? wp + ((size_t)c * (KS * KS) + kh * KS + kk % TAPS) * a.npg_pad + 4 * q : a.wpk, in);
+                cp_async16(smem_u32(&b_s[st][kk][4 * q]), in ? wp + ((size_t)c * (KS * KS) + kh * KS + kk % TAPS) * a.npg_pad + 4 * q : a.wpk, in);
             }
         }
     };

@@ -115,7 +115,7 @@ __device__ __forceinline__ bool meet(int half, bool fine)
     uint32_t all;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\t"
-        "barrier.cta.red.and.pred q, %1, 128, p;\n\t"
+        "bar.red.and.pred q, %1, 128, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(all) : "r"(1 + half), "r"((uint32_t)fine) : "memory");
     return all != 0;

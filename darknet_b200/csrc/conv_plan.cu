@@ -145,8 +145,8 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
         snprintf(buf, len, "%s pair=%d halo=0 bn=%d tile=%dx%dx%d tiles=%d stages=%d splits=%d signs_in=%d signs_out=%d one_tile_per_cluster", kKernelNames[p->kernel], p->sp.pair,
                  p->sp.bn, p->sp.wt, p->sp.ht, p->sp.bt, p->sp.tiles, p->sp.stages, p->sp.splits, p->signs_given ? 1 : 0, p->sp.sign_out ? 1 : 0);
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
-        snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
-                 a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
+        snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
+                 a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
     else if (p->fp32_tc && p->ft_x_ptr)
         snprintf(buf, len, "%s three_tf32_products bn=%d tile=%dx%dx%d tiles=%d", dnb_conv_plan_kernel(p), p->ft.bn, p->ft.wt, p->ft.ht, p->ft.bt, p->ft.total_tiles);
     else
@@ -795,7 +795,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // Narrow tiles (bn <= 128) leave TMEM and, with a short ring, shared memory for a second CTA on the SM:
     // twice the warps hide the per-tile hand-offs that dominate layers with few K iterations.
     a.ctas_per_sm = 1;
-    a.stage_bufs = (residual && !a.pair) ? 4 : 2;   // a pair reads the residual with plain loads: nothing lands in the staging buffers
+    a.stage_bufs = residual ? 4 : 2;
     if (sign_out) a.stage_bufs = 3;   // the third buffer holds the staged signs
     a.sign_out = sign_out;
     a.sign_cpitch = sign_cpitch;
@@ -804,6 +804,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     int stages = 0;
     const bool allow2 = getenv("DNB_TC_CTAS") ? atoi(getenv("DNB_TC_CTAS")) >= 2 : true;
     a.a_stages = a.b_stages = a.a_slot = a.a_box_bytes = a.a_pitch = 0;
+    a.epi_groups = 1;
     if (a.halo) {
         // two rings: activation boxes (one per channel block) and weight tiles (nine per box).  A weight tile is
         // consumed in a quarter of the time an ordinary ring slot is, so that ring wants to be deep: one CTA per
@@ -838,7 +839,23 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
                 if (s2 >= 2) { a.ctas_per_sm = 2; stages = s2 > max2 ? max2 : s2; srb = srb2; break; }
             }
         }
-        if (a.ctas_per_sm == 1) {
+        // A CTA alone on its SM may have two groups of epilogue warps, if three ring slots and their 128-byte staged rows fit:
+        //  * pairs with a residual, always: 3x3 128 -> 256 at 64 x 76 x 76 in TF32 329 -> 306 us, 360 -> 311 under the power cap; 512 -> 2048
+        //    at 256 x 7 x 7 87 -> 73
+        //  * pairs of less than 32 K iterations, whose epilogue is as long as their MMAs: 3x3 128 -> 256 at 8 x 52 x 52 in bf16 25.4 -> 24.0;
+        //    over 36 iterations and more the second group only disturbs (282 -> 284, 260 -> 264)
+        //  * Darknet's layout, a store instruction per value: 1024 -> 255 at 64 x 19 x 19 87 -> 56
+        //  * xnor layers: 256 -> 128 at 128 x 28 x 28 28.1 -> 26.6, 512 -> 256 at 14 x 14 21.0 -> 19.0
+        // Other single CTAs are bound by memory (512 -> 256 at 64 x 52 x 52 in bf16 52 and 52), with a residual they want its tiles by TMA, three
+        // chunks ahead (64 -> 256 at 256 x 56 x 56 342 us, 416 through this path).  DNB_TC_EPI=1: one group (pairs with a residual: two).
+        const int loop = g.size * g.size * a.c_blocks, epi_knob = getenv("DNB_TC_EPI") ? atoi(getenv("DNB_TC_EPI")) : 2;
+        const bool two = residual ? a.pair != 0 : epi_knob != 1 && (a.pair ? loop < 32 : nchw_out || i8);
+        if (a.ctas_per_sm == 1 && two && (a.pair || !getenv("DNB_TC_SRB")) && (!y_nhwc || srb == 128)) {
+            const int bufs = y_nhwc ? a.stage_bufs : 0;
+            const int fit = (int)((max_smem - (long)conv_tc_fixed_smem(128, a.bn, bufs)) / (a.a_bytes + a.b_bytes));
+            if (fit >= 3) { a.epi_groups = 2; a.stage_bufs = bufs; stages = fit; srb = 128; }
+        }
+        if (a.ctas_per_sm == 1 && a.epi_groups == 1) {
             // The depth of the ring is what hides the operand loads' latency: four slots before wide staged rows.
             // The exception is a fused residual behind a short K loop, where the epilogue (one round of barrier,
             // residual wait and store per staged chunk) would outlast the tile's MMAs: fewer, wider chunks then.

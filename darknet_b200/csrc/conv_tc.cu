@@ -47,7 +47,6 @@
 
 namespace dnb {
 
-constexpr int TC_THREADS = 192;
 constexpr int MAX_STAGES = 8;
 constexpr int MAX_B_STAGES = 12;   // weight-tile ring of the halo mode
 constexpr int MAX_RES_BUFS = 4;   // staging buffers with a fused residual; tiles are requested two chunks ahead
@@ -81,6 +80,47 @@ __device__ __forceinline__ float act_apply(float x, int runtime_act)
     return activate_call(x, runtime_act);
 }
 
+// One output value: scale and shift of the sum, activation, [yolo] logistic or residual, rounding.
+template <int ACT, int ACT2, bool OUT_BF16, bool I8>
+__device__ __forceinline__ float finish_value(uint32_t acc, float scale, float shift, float res, float alpha, float beta, int runtime_act, int act2, int do_round, int yolo_entry)
+{
+    const float accv = I8 ? (float)(int)acc : __uint_as_float(acc);   // int32 sums of an xnor layer are exact in f32 (below 2^24)
+    float t = act_apply<ACT>(fmaf(accv, scale, shift), runtime_act);
+    // forward_yolo_layer_gpu's activations (src/yolo_layer.c:351-357): logistic on x, y, objectness, classes.  The entry index is the same
+    // for the whole warp (it depends on the column only); fast exponential and division (2 ulp)
+    if (ACT == ACT_YOLO && (yolo_entry < 2 || yolo_entry >= 4)) t = __fdividef(1.f, 1.f + __expf(-t));
+    if (ACT2 != ACT2_NONE) t = act_apply<ACT2>(alpha * t + beta * res, act2);
+    return !OUT_BF16 && do_round ? round_tf32(t) : t;
+}
+
+template <int N>
+__device__ __forceinline__ uint4 pack_bf16x8(const uint32_t (&r)[N], int j)
+{
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * i]), __uint_as_float(r[j + 2 * i + 1]));
+        w[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The epilogue's threads (one or two groups of 128) meet, and agree on whether to go on.
+template <int THREADS>
+__device__ __forceinline__ bool epilogue_agree(bool fine)
+{
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all) : "r"((uint32_t)fine), "n"(THREADS) : "memory");
+    return all != 0;
+}
+
+// The four warps of one group.
+__device__ __forceinline__ void group_bar(int group) { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); }
+
 // ACT: activation folded at compile time (DNB_LINEAR, DNB_LEAKY) or ACT_GENERIC (runtime switch).
 // ACT2: ACT2_NONE, or the activation of the fused shortcut layer (same three choices).  The epilogue's chunk
 // body is unrolled over CPC columns and shares the instruction cache with the TMA and MMA loops: every
@@ -99,10 +139,16 @@ __device__ __forceinline__ float act_apply(float x, int runtime_act)
 // is > 0, else -1, 0 beyond the layer's filters) as the int8 channels-last tensor that the xnor layer after it reads as
 // its operand: that layer's sign pass over the f32 tensor disappears.  The signs of a chunk are staged in a third
 // staging buffer (two 4 KB halves in rotation) and leave with the chunk's output rows, in the same bulk group.
-template <int ACT, int CPC, bool OUT_BF16, int ACT2, bool PAIR, bool I8 = false, bool SIGNS = false>
-__global__ void __launch_bounds__(TC_THREADS)
+// EG: groups of four epilogue warps.  Two CTAs on an SM bring eight epilogue warps between them; one CTA with four has every SM
+// sub-partition wait for a single warp's chain of TMEM read, residual, arithmetic, staging and store.  The second group takes alternate
+// chunks, with staged rows, a barrier and a storing thread of its own; with a residual (pairs) every warp is on its own, fetches the
+// residual of its 32 pixels and stores them.  Which launches have two: build_tc_args in conv_plan.cu.
+template <int ACT, int CPC, bool OUT_BF16, int ACT2, bool PAIR, bool I8 = false, bool SIGNS = false, int EG = 1>
+__global__ void __launch_bounds__(64 + 128 * EG)
 conv_tc_kernel(const __grid_constant__ TcArgs a)
 {
+    static_assert(EG == 1 || CPC * (OUT_BF16 ? 2 : 4) == 128, "two epilogue groups: 128-byte staged rows");
+    static_assert(ACT2 == ACT2_NONE || EG == (PAIR ? 2 : 1), "a pair fetches its residual into the staged rows of two groups, a single CTA by TMA");
     static_assert(!SIGNS || (I8 && CPC == 32 && !OUT_BF16), "the sign output belongs to the int8 kind with 128-byte staged rows");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // operand ring, 1024-byte aligned (the 128-byte swizzle pattern repeats every 1024 bytes).  The kernel
@@ -139,7 +185,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&sh->acc_full[i]), 1);
-            mbar_init(smem_u32(&sh->acc_empty[i]), PAIR ? 8 : 4);   // the epilogue warps of both CTAs of a pair
+            mbar_init(smem_u32(&sh->acc_empty[i]), (PAIR ? 8 : 4) * EG);   // the epilogue warps of both CTAs of a pair
         }
         for (int i = 0; i < MAX_RES_BUFS; ++i) mbar_init(smem_u32(&sh->res_full[i]), 1);
         sh->abort_flag = 0;
@@ -390,6 +436,223 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             }
         }
         __syncwarp();
+    } else if constexpr (EG == 2) {
+        // ---------------- epilogue, two groups: warps 2..9, TMEM lanes 32*(warp%4) .. +31, chunks group, group + 2, ...
+        grid_dependency_wait();
+        constexpr bool residual = ACT2 != ACT2_NONE;
+        constexpr int ROW = 128, OES = OUT_BF16 ? 2 : 4, PIECES = ROW / 16;
+        constexpr int NBUF = residual ? 2 : 1;                 // staged rows of a warp: its residual lands in the second while the first is finished
+        const int group = (warp - 2) >> 2, quarter = warp & 3, m0 = quarter * 32, m = m0 + lane;
+        const int lw = 31 - __clz(wt), lh = 31 - __clz(ht);    // powers of two
+        const int wl = m & (wt - 1), hl = (m >> lw) & (ht - 1), bl = m >> (lw + lh);
+        const int wl0 = m0 & (wt - 1), hl0 = (m0 >> lw) & (ht - 1), bl0 = m0 >> (lw + lh);   // origin of this warp's rows inside the tile
+        const ConvGeom g = a.g;
+        float *const y_nchw = a.y_nchw;
+        const bool y_nhwc = a.y_nhwc != nullptr;
+        const int runtime_act = a.ep.activation, act2 = a.ep.activation2, do_round = a.ep.round_tf32;
+        const float res_alpha = a.ep.alpha, res_beta = a.ep.beta;
+        const bool raw_acc = I8 && a.ep.raw_acc != 0;
+        const int yolo_entries = ACT == ACT_YOLO ? a.ep.yolo_entries : 1;
+        const int dbg = a.debug;
+        int *status = a.status;
+        uint8_t *const staged0 = stage_out + (size_t)group * NBUF * 128 * ROW, *const staged_signs = stage_out + 2 * 128 * ROW + (size_t)group * 128 * 32;
+        uint8_t *const my_signs = staged_signs + m * 32;
+        const bool store_thread = quarter == 2 && lane == 0;   // of this group
+        const int q_xor = lane & 7;                            // 128-byte swizzle
+        const float *const ep_scale = a.ep.scale, *const ep_shift = a.ep.shift;
+        const int n_pad = a.n_pad;
+        const size_t plane = (size_t)g.out_h * g.out_w;
+
+        // Residual: 128 bytes of each of the warp's 32 pixels, four pixels an instruction (eight lanes each), straight into the staged
+        // rows.  Requested one chunk ahead, across tiles; the tile after it is asked into L2 meanwhile.
+        const int res_stride = a.ep.res_stride, res_h = a.ep.res_h, res_w = a.ep.res_w, res_chan = min((a.ep.res_c + 7) & ~7, a.ep.res_cpitch);
+        const uint8_t *const res_base = reinterpret_cast<const uint8_t *>(a.ep.residual);
+        const size_t res_pix = (size_t)a.ep.res_cpitch * OES;
+        const bool no_res = (dbg & 1) != 0;
+        int pf_tile = group * CPC < bn ? first_tile : total_tiles, pf_c0 = group * CPC, pf_at = -1;
+        long long pf_off[residual ? 8 : 1];                    // the rows this lane has a piece of (negative: outside the image)
+        uint32_t pf_count = 0;
+        auto res_offset = [&](int tile, int mm) {              // of pixel mm of a tile; negative outside the image
+            const int pt = pixel_tile(tile);
+            const int ow = (pt % tiles_w) * wt + (mm & (wt - 1)), oh = ((pt / tiles_w) % tiles_h) * ht + ((mm >> lw) & (ht - 1)), b = (pt / ptiles_wh) * bt + (mm >> (lw + lh));
+            return ow < g.out_w && oh < g.out_h && b < g.batch ? (long long)((((size_t)b * res_h + oh * res_stride) * res_w + ow * res_stride) * res_pix) : -1ll;
+        };
+        auto request_residual = [&]() {
+            if (pf_tile < total_tiles && !no_res) {
+                if (pf_at != pf_tile) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) pf_off[residual ? i : 0] = res_offset(pf_tile, m0 + 4 * i + (lane >> 3));
+                    pf_at = pf_tile;
+                }
+                const int ch = (pf_tile % n_tiles) * bn + pf_c0 + (lane & 7) * (16 / OES);
+                const bool has = ch < res_chan;
+                const uint32_t dst = smem_u32(staged0 + ((pf_count & 1) * 128 + m0) * ROW);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = 4 * i + (lane >> 3);
+                    const bool in = has && pf_off[residual ? i : 0] >= 0;
+                    cp_async16(dst + r * ROW + (((lane & 7) ^ (r & 7)) << 4), in ? res_base + pf_off[residual ? i : 0] + (size_t)ch * OES : res_base, in);
+                }
+                pf_c0 += 2 * CPC;
+                if (pf_c0 >= bn) { pf_c0 = group * CPC; pf_tile += grid_stride; }
+            }
+            ++pf_count;
+            cp_async_commit();
+        };
+        if (residual) request_residual();
+
+        uint32_t chunk_count = 0;
+        int it = 0, loaded_nt = -1;
+        for (int tile = first_tile; tile < total_tiles; tile += grid_stride, ++it) {
+            const int acc = it & 1;
+            const int nt = tile % n_tiles, pt = pixel_tile(tile);
+            const int ow0 = (pt % tiles_w) * wt, oh0 = ((pt / tiles_w) % tiles_h) * ht, b0 = (pt / ptiles_wh) * bt;
+            const int ow = ow0 + wl, oh = oh0 + hl, b = b0 + bl;
+            const bool pix_ok = ow < g.out_w && oh < g.out_h && b < g.batch;
+            if (nt != loaded_nt) {
+                // this filter tile's vectors (zero beyond the layer's filters), once every warp is done with the last one's
+                epilogue_agree<256>(true);
+                for (int i = threadIdx.x - 64; i < bn + 64; i += 256) {
+                    const int gi = nt * bn + i;
+                    const bool in = i < bn && gi < n_pad;
+                    s_scale[i] = in ? __ldg(ep_scale + gi) : 0.f;
+                    s_shift[i] = in ? __ldg(ep_shift + gi) : 0.f;
+                }
+                loaded_nt = nt;
+            }
+            if (residual && group == 0 && !no_res && tile + grid_stride < total_tiles) {
+                const long long off = res_offset(tile + grid_stride, m);
+                const int n0 = (tile + grid_stride) % n_tiles * bn, bytes = (min(bn, res_chan - n0)) * OES;
+                if (off >= 0 && bytes > 0) prefetch_l2(res_base + off + (size_t)n0 * OES, (uint32_t)bytes);
+            }
+            const bool fine = mbar_wait(smem_u32(&sh->acc_full[acc]), (it >> 1) & 1, abort_flag, status, WAIT_ACC_FULL, 0, wait_limit);
+            if (!epilogue_agree<256>(fine && !*abort_flag)) break;
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + ((uint32_t)m0 << 16) + acc * acc_stride;
+            // deliberately not unrolled: the body has to stay in the instruction cache next to the MMA warp's loop
+#pragma unroll 1
+            for (int c0 = (dbg & 8) ? bn : group * CPC; c0 < bn; c0 += 2 * CPC) {
+                uint32_t r[CPC];
+#pragma unroll
+                for (int u = 0; u < CPC / 16; ++u) {
+                    if (c0 + 16 * u < bn) {
+                        tmem_ld16(t_row + c0 + 16 * u, *reinterpret_cast<uint32_t(*)[16]>(&r[16 * u]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[16 * u + j] = 0u;
+                    }
+                }
+                tmem_ld_wait();
+                uint8_t *const staged = staged0 + (residual ? (chunk_count & 1) * 128 * ROW : 0), *const row = staged + m * ROW;
+                uint4 res[residual ? PIECES : 1];
+                if (residual) {
+                    cp_async_wait<0>();
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < PIECES; ++q) res[residual ? q : 0] = no_res ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4 *>(row + ((q ^ q_xor) << 4));
+                }
+                const int nl0 = nt * bn + c0;                 // first filter of this chunk
+                const int nvalid = min(bn - c0, g.n - nl0);   // columns of this chunk that are real filters
+                int yolo_entry = ACT == ACT_YOLO ? nl0 % yolo_entries : 0;
+                const float4 *sc4 = reinterpret_cast<const float4 *>(s_scale + c0);
+                const float4 *sf4 = reinterpret_cast<const float4 *>(s_shift + c0);
+#pragma unroll
+                for (int q = 0; q < CPC / 4; ++q) {
+                    const float4 sc = sc4[q], sf = sf4[q];
+                    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int j = 4 * q + e;
+                        float rv = 0.f;
+                        if (residual) {
+                            const uint4 v4 = res[residual ? j * OES / 16 : 0];
+                            if (!OUT_BF16) rv = __uint_as_float((j & 3) == 0 ? v4.x : (j & 3) == 1 ? v4.y : (j & 3) == 2 ? v4.z : v4.w);
+                            else {
+                                const uint32_t wd = ((j >> 1) & 3) == 0 ? v4.x : ((j >> 1) & 3) == 1 ? v4.y : ((j >> 1) & 3) == 2 ? v4.z : v4.w;
+                                rv = __uint_as_float((j & 1) ? (wd & 0xffff0000u) : (wd << 16));
+                            }
+                        }
+                        const float t = finish_value<ACT, ACT2, OUT_BF16, I8>(r[j], scv[e], sfv[e], rv, res_alpha, res_beta, runtime_act, act2, do_round, yolo_entry);
+                        if (ACT == ACT_YOLO && ++yolo_entry == yolo_entries) yolo_entry = 0;
+                        constexpr bool self_zero = (ACT == DNB_LINEAR || ACT == DNB_LEAKY) && (ACT2 == ACT2_NONE || ACT2 == DNB_LINEAR || ACT2 == DNB_LEAKY);
+                        if (!(I8 && raw_acc)) r[j] = __float_as_uint((self_zero || j < nvalid) ? t : 0.f);
+                    }
+                }
+                if (residual) {
+                    // this warp's last store has read the other rows: the next chunk's residual may land there
+                    if (lane == 0) tma_store_wait_read0();
+                    __syncwarp();
+                    request_residual();
+                } else if (y_nhwc) {
+                    if (store_thread) tma_store_wait_read0();   // the group's last store has read these rows
+                    group_bar(group);
+                }
+                if (y_nhwc) {
+                    if (!OUT_BF16) {
+#pragma unroll
+                        for (int q = 0; q < PIECES; ++q)
+                            *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < PIECES; ++q)
+                            *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = pack_bf16x8<CPC>(r, 8 * q);
+                    }
+                    if (SIGNS) {
+                        // 32 signs of this pixel = one 32-byte row of a 32-byte-swizzled box: its two 16-byte halves swap on rows 4..7 of every 8
+                        uint32_t sw[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            uint32_t wd = 0u;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int j = 4 * q + e;
+                                const uint32_t sgn = j < nvalid ? (__uint_as_float(r[j]) > 0.f ? 0x01u : 0xFFu) : 0u;
+                                wd |= sgn << (8 * e);
+                            }
+                            sw[q] = wd;
+                        }
+                        const int sx = (lane >> 2) & 1;
+                        *reinterpret_cast<uint4 *>(my_signs + ((0 ^ sx) << 4)) = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+                        *reinterpret_cast<uint4 *>(my_signs + ((1 ^ sx) << 4)) = make_uint4(sw[4], sw[5], sw[6], sw[7]);
+                    }
+                    fence_async_smem();
+                    if (residual) __syncwarp(); else group_bar(group);
+                    // the TMA unit clips the box at the tensor's extents; a box that begins beyond them is not stored at all
+                    if (residual) {
+                        if (lane == 0 && !(dbg & 2) && ow0 + wl0 < g.out_w && oh0 + hl0 < g.out_h && b0 + bl0 < g.batch && nvalid > 0) {
+                            tma_store_4d(&a.tmy_warp, smem_u32(staged + m0 * ROW), nl0, ow0 + wl0, oh0 + hl0, b0 + bl0);
+                            tma_store_commit();
+                        }
+                    } else if (store_thread && !(dbg & 2) && (!PAIR || b0 < g.batch)) {
+                        tma_store_4d(&a.tmy, smem_u32(staged), nl0, ow0, oh0, b0);
+                        if (SIGNS) tma_store_4d(&a.tms, smem_u32(staged_signs), nl0, ow0, oh0, b0);
+                        tma_store_commit();
+                    }
+                }
+                if (y_nchw && pix_ok) {
+                    // Darknet-layout copy: this thread's pixel, one filter plane per column, straight from the registers (a warp's 32 pixels
+                    // are wt-long runs of each plane).  BF16 plans write what the channels-last copy holds: the value rounded to bf16.
+                    float *dst = y_nchw + ((size_t)b * g.n + nl0) * plane + (size_t)oh * g.out_w + ow;
+                    const int cols = min(CPC, g.n - nl0);
+#pragma unroll
+                    for (int j = 0; j < CPC; ++j) {
+                        if (j < cols) {
+                            float v = __uint_as_float(r[j]);
+                            if (OUT_BF16) v = __bfloat162float(__float2bfloat16_rn(v));
+                            dst[(size_t)j * plane] = v;
+                        }
+                    }
+                }
+                ++chunk_count;
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {   // a pair's accumulator is free when the epilogues of both CTAs have drained their rows
+                if (PAIR) mbar_arrive_leader(smem_u32(&sh->acc_empty[acc])); else mbar_arrive(smem_u32(&sh->acc_empty[acc]));
+            }
+        }
+        if (residual) cp_async_wait<0>();
+        if (residual ? lane == 0 : store_thread) tma_store_wait_all();
     } else {
         // ---------------- epilogue: warps 2..5 own TMEM lanes 32*(warp%4) .. +31
         grid_dependency_wait();
@@ -403,11 +666,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         const bool raw_acc = I8 && a.ep.raw_acc != 0;
         const int yolo_entries = ACT == ACT_YOLO ? a.ep.yolo_entries : 1;   // fused [yolo] head: a kernel variant of its own
         constexpr bool residual = ACT2 != ACT2_NONE;
-        // A CTA pair reads the residual with plain 16-byte loads, one staged chunk ahead, instead of TMA tiles into the
-        // staging buffers: residual tile loads inside the pair kernel raised an illegal-instruction fault on B200 whose
-        // cause was not found, so that combination is not built.  Each thread reads its own pixel's 128 contiguous bytes.
-        constexpr bool res_direct = residual && PAIR;
-        constexpr bool res_tiles = residual && !PAIR;
+        constexpr bool res_tiles = residual;
         const CUtensorMap *rmap = &a.tmr;
         const uint32_t buf_mask = res_tiles ? 3u : 1u;   // staging buffers in rotation
         constexpr int res_ahead = 3;   // residual tiles requested ahead of the chunk being finished (of four buffers)
@@ -419,7 +678,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         // Per-warp stores (no residual tiles, no sign output): every warp stages its own 32 rows, which are a box of the
         // output like the whole tile is, and sends them off itself; the four warps then meet once per tile instead of
         // twice per chunk, so one warp's TMEM or store wait no longer stalls the other three.
-        constexpr bool can_warp_store = ACT2 == ACT2_NONE || PAIR;
+        constexpr bool can_warp_store = ACT2 == ACT2_NONE;
         const bool warp_stores = can_warp_store && !SIGNS && a.warp_stores != 0 && a.y_nhwc != nullptr;
         const int m0 = quarter * 32;
         const int wl0 = m0 % wt, hl0 = (m0 / wt) % ht, bl0 = m0 / (wt * ht);   // origin of this warp's rows inside the tile
@@ -450,9 +709,6 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         };
         if (res_tiles && store_thread)
             for (int d = 0; d < res_ahead; ++d) request_residual();
-        const uint8_t *const res_base = reinterpret_cast<const uint8_t *>(a.ep.residual);
-        const size_t res_pix_bytes = (size_t)a.ep.res_cpitch * (OUT_BF16 ? 2 : 4);
-        const int res_c = a.ep.res_c, res_stride = a.ep.res_stride, res_h = a.ep.res_h, res_w = a.ep.res_w;
         const float *const ep_scale = a.ep.scale, *const ep_shift = a.ep.shift;
         const int n_pad = a.n_pad;
         for (int tile = first_tile; tile < total_tiles; tile += grid_stride, ++it) {
@@ -475,8 +731,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 loaded_nt = nt;
             }
             mbar_wait(smem_u32(&sh->acc_full[acc]), acc_phase, abort_flag, status, WAIT_ACC_FULL, 32, wait_limit);
-            epilogue_bar();                 // all four warps agree on the abort flag from here
-            if (*abort_flag) break;
+            if (!epilogue_agree<128>(!*abort_flag)) break;   // all four warps, which go on meeting each other
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * acc_stride;
             // One staged chunk of CPC columns per iteration: CPC/16 TMEM loads in flight, one wait, the
@@ -484,14 +739,6 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             // stay resident in the instruction cache next to the MMA warp's loop.
             const size_t plane = (size_t)g.out_h * g.out_w;
             constexpr int RES_V = CPC * (OUT_BF16 ? 2 : 4) / 16;      // 16-byte pieces of a staged row
-            // direct residual: this pixel's row of the residual tensor, the next chunk's 128 bytes always in flight
-            const uint4 *res_row = nullptr;
-            uint4 res_next[res_direct ? RES_V : 1];
-            if (res_direct) {
-                if (pix_ok && !no_res) res_row = reinterpret_cast<const uint4 *>(res_base + (((size_t)b * res_h + oh * res_stride) * res_w + ow * res_stride) * res_pix_bytes + (size_t)nt * bn * (OUT_BF16 ? 2 : 4));
-#pragma unroll
-                for (int q = 0; q < RES_V; ++q) res_next[q] = res_row && nt * bn < res_c ? __ldg(res_row + q) : make_uint4(0u, 0u, 0u, 0u);
-            }
 #pragma unroll 1
             for (int c0 = (dbg & 8) ? bn : 0; c0 < bn; c0 += CPC) {
                 uint32_t r[CPC];
@@ -508,16 +755,6 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     tmem_ld_wait();
                 }
                 uint4 res[RES_V];
-                if (res_direct) {
-#pragma unroll
-                    for (int q = 0; q < RES_V; ++q) res[q] = res_next[q];
-                    if (c0 + CPC < bn && res_row) {   // channels beyond the residual's, whole chunks of them, get no addend
-                        const uint4 *nx = res_row + (size_t)(c0 + CPC) * (OUT_BF16 ? 2 : 4) / 16;
-                        const bool has = nt * bn + c0 + CPC < res_c;
-#pragma unroll
-                        for (int q = 0; q < RES_V; ++q) res_next[q] = has ? __ldg(nx + q) : make_uint4(0u, 0u, 0u, 0u);
-                    }
-                }
                 if (res_tiles) {
                     // this chunk's residual tile (TMA zero-fills pixels and channels outside the tensor)
                     const uint32_t rb = chunk_count & 3u;
@@ -540,30 +777,19 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int j = 4 * q + e;
-                        const float accv = I8 ? (float)(int)r[j] : __uint_as_float(r[j]);   // int32 sums of an xnor layer are exact in f32 (below 2^24)
-                        float t = act_apply<ACT>(fmaf(accv, scv[e], sfv[e]), runtime_act);
-                        if (ACT == ACT_YOLO) {
-                            // forward_yolo_layer_gpu's activations (src/yolo_layer.c:351-357): logistic on x, y, objectness, classes.
-                            // The entry index is the same for the whole warp (it depends on the column only); the epilogue has
-                            // four warps to hide its latencies with, so the fast exponential and division are used (2 ulp).
-                            if (yolo_entry < 2 || yolo_entry >= 4) t = __fdividef(1.f, 1.f + __expf(-t));
-                            if (++yolo_entry == yolo_entries) yolo_entry = 0;
-                        }
+                        float rv = 0.f;
                         if (residual) {
-                            float rv = 0.f;
-                            {
-                                if (!OUT_BF16) {
-                                    const uint4 v4 = res[j / 4];
-                                    rv = __uint_as_float((j & 3) == 0 ? v4.x : (j & 3) == 1 ? v4.y : (j & 3) == 2 ? v4.z : v4.w);
-                                } else {
-                                    const uint4 v4 = res[j / 8];
-                                    const uint32_t wd = ((j >> 1) & 3) == 0 ? v4.x : ((j >> 1) & 3) == 1 ? v4.y : ((j >> 1) & 3) == 2 ? v4.z : v4.w;
-                                    rv = __uint_as_float((j & 1) ? (wd & 0xffff0000u) : (wd << 16));
-                                }
+                            if (!OUT_BF16) {
+                                const uint4 v4 = res[j / 4];
+                                rv = __uint_as_float((j & 3) == 0 ? v4.x : (j & 3) == 1 ? v4.y : (j & 3) == 2 ? v4.z : v4.w);
+                            } else {
+                                const uint4 v4 = res[j / 8];
+                                const uint32_t wd = ((j >> 1) & 3) == 0 ? v4.x : ((j >> 1) & 3) == 1 ? v4.y : ((j >> 1) & 3) == 2 ? v4.z : v4.w;
+                                rv = __uint_as_float((j & 1) ? (wd & 0xffff0000u) : (wd << 16));
                             }
-                            t = act_apply<ACT2>(res_alpha * t + res_beta * rv, act2);
                         }
-                        if (!OUT_BF16 && do_round) t = round_tf32(t);
+                        const float t = finish_value<ACT, ACT2, OUT_BF16, I8>(r[j], scv[e], sfv[e], rv, res_alpha, res_beta, runtime_act, act2, do_round, yolo_entry);
+                        if (ACT == ACT_YOLO && ++yolo_entry == yolo_entries) yolo_entry = 0;
                         // columns beyond the layer's filters: scale, shift, weights and residual are all zero there, so
                         // linear and leaky epilogues produce the zero by themselves; others need the mask
                         constexpr bool self_zero = (ACT == DNB_LINEAR || ACT == DNB_LEAKY) &&
@@ -589,17 +815,8 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                         *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
                 } else {
 #pragma unroll
-                    for (int q = 0; q < srb / 16; ++q) {       // 16-byte pieces of 8 bf16
-                        const int j = 8 * q;
-                        uint4 pk;
-                        __nv_bfloat162 h0 = __floats2bfloat162_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-                        __nv_bfloat162 h1 = __floats2bfloat162_rn(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                        __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5]));
-                        __nv_bfloat162 h3 = __floats2bfloat162_rn(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7]));
-                        pk.x = *reinterpret_cast<uint32_t *>(&h0); pk.y = *reinterpret_cast<uint32_t *>(&h1);
-                        pk.z = *reinterpret_cast<uint32_t *>(&h2); pk.w = *reinterpret_cast<uint32_t *>(&h3);
-                        *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = pk;
-                    }
+                    for (int q = 0; q < srb / 16; ++q)         // 16-byte pieces of 8 bf16
+                        *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = pack_bf16x8<CPC>(r, 8 * q);
                 }
                 if (SIGNS) {
                     // 32 signs of this pixel = one 32-byte row of a 32-byte-swizzled box: its two 16-byte halves swap on rows 4..7 of every 8
@@ -662,7 +879,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {   // a pair's accumulator is free when the epilogues of both CTAs have drained their rows
+            if (lane == 0) {
                 if (PAIR) mbar_arrive_leader(smem_u32(&sh->acc_empty[acc])); else mbar_arrive(smem_u32(&sh->acc_empty[acc]));
             }
         }
@@ -715,14 +932,14 @@ int conv_tc_max_smem()
 
 // Resident clusters of two CTAs of a pair-mode kernel with `smem` bytes of dynamic shared memory (cached per kernel).
 template <typename K>
-static int max_pair_clusters(K kernel, size_t smem)
+static int max_pair_clusters(K kernel, size_t smem, int threads)
 {
     static int cached = 0;
     static size_t cached_smem = 0;
     if (cached && cached_smem == smem) return cached;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
-    cfg.blockDim = dim3(TC_THREADS);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -754,7 +971,7 @@ static int launch_one(K kern, const TcArgs &a, size_t smem, cudaStream_t s)
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
     unsigned grid;
     if (a.pair) {
-        const int clusters_max = max_pair_clusters(kern, smem);
+        const int clusters_max = max_pair_clusters(kern, smem, 64 + 128 * a.epi_groups);
         grid = 2u * (unsigned)(a.total_tiles < clusters_max ? a.total_tiles : clusters_max);
     } else {
         const int slots = sm_count() * a.ctas_per_sm;
@@ -767,7 +984,7 @@ static int launch_one(K kern, const TcArgs &a, size_t smem, cudaStream_t s)
     attrs[1].val.clusterDim.x = 2; attrs[1].val.clusterDim.y = 1; attrs[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(TC_THREADS);
+    cfg.blockDim = dim3((unsigned)(64 + 128 * a.epi_groups));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attrs;
@@ -782,14 +999,24 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
     const bool obf = a.is_bf16 == 1, i8 = a.is_bf16 == 2;   // int8 operands write f32 output
     const int cpc = a.store_row_bytes / (obf ? 2 : 4);
     if (cpc != 16 && cpc != 32 && cpc != 64) DNB_FAIL(DNB_EINVAL, "conv_tc: staged row of %d bytes", a.store_row_bytes);
+    if (a.ep.residual && a.epi_groups != (a.pair ? 2 : 1)) DNB_FAIL(DNB_EINVAL, "conv_tc: a residual with %d epilogue groups", a.epi_groups);
+    if (a.epi_groups == 2 && a.store_row_bytes != 128) DNB_FAIL(DNB_EINVAL, "conv_tc: two epilogue groups need 128-byte staged rows");
     if (a.pair && !((!obf && cpc == 32) || (obf && cpc == 64))) DNB_FAIL(DNB_EINVAL, "conv_tc: pair mode needs 128-byte staged rows");
     // one instantiation per (activation, columns per staged chunk, output type, fused shortcut, pair mode, operand kind)
 #define DNB_TC_GO(ACT, CPC, OBF, ACT2, I8)                                                          \
     do {                                                                                            \
-        if (a.pair) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, true, I8>, a, smem, s)); \
+        constexpr int pair_eg = ACT2 != ACT2_NONE ? 2 : 1, single_eg = ACT2 != ACT2_NONE ? 1 : 2;   /* with a residual: always */ \
+        if (a.pair && a.epi_groups == 2) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, true, I8, false, 2>, a, smem, s)); \
+        else if (a.pair) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, true, I8, false, pair_eg>, a, smem, s)); \
+        else if (a.epi_groups == 2) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, false, I8, false, single_eg>, a, smem, s)); \
         else DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, false, I8>, a, smem, s));       \
     } while (0)
     // pair-mode kernels exist for 128-byte staged rows only, so the narrower variants are instantiated without it
+#define DNB_TC_GO_WIDE(ACT, CPC, OBF, ACT2, I8)                                                     \
+    do {                                                                                            \
+        if (a.epi_groups == 2) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, false, I8, false, 2>, a, smem, s)); \
+        else DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, false, I8>, a, smem, s));       \
+    } while (0)
 #define DNB_TC_GO_SINGLE(ACT, CPC, OBF, ACT2, I8) DNB_TRY(launch_one(conv_tc_kernel<ACT, CPC, OBF, ACT2, false, I8>, a, smem, s))
 #define DNB_TC_LAUNCH_ACT(ACT, ACT2)                                            \
     do {                                                                        \
@@ -804,9 +1031,9 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
 #define DNB_TC_LAUNCH_ACT_SINGLE(ACT, ACT2)                                     \
     do {                                                                        \
         if (a.pair) DNB_FAIL(DNB_EINVAL, "conv_tc: no pair variant of this epilogue"); \
-        if (!obf && cpc == 32) DNB_TC_GO_SINGLE(ACT, 32, false, ACT2, false);   \
+        if (!obf && cpc == 32) DNB_TC_GO_WIDE(ACT, 32, false, ACT2, false);     \
         else if (!obf && cpc == 16) DNB_TC_GO_SINGLE(ACT, 16, false, ACT2, false); \
-        else if (obf && cpc == 64) DNB_TC_GO_SINGLE(ACT, 64, true, ACT2, false); \
+        else if (obf && cpc == 64) DNB_TC_GO_WIDE(ACT, 64, true, ACT2, false);  \
         else if (obf && cpc == 32) DNB_TC_GO_SINGLE(ACT, 32, true, ACT2, false); \
         else if (obf && cpc == 16) DNB_TC_GO_SINGLE(ACT, 16, true, ACT2, false); \
         else DNB_FAIL(DNB_EINVAL, "conv_tc: no kernel for %d columns per chunk", cpc); \
@@ -815,7 +1042,9 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
     do {                                                                        \
         if (a.sign_out) {                                                       \
             if (cpc != 32 || a.stage_bufs != 3 || a.ep.raw_acc) DNB_FAIL(DNB_EINVAL, "conv_tc: the sign output needs 128-byte staged rows and a third staging buffer"); \
-            if (a.pair) DNB_TRY(launch_one(conv_tc_kernel<ACT, 32, false, ACT2_NONE, true, true, true>, a, smem, s)); \
+            if (a.pair && a.epi_groups == 2) DNB_TRY(launch_one(conv_tc_kernel<ACT, 32, false, ACT2_NONE, true, true, true, 2>, a, smem, s)); \
+            else if (a.pair) DNB_TRY(launch_one(conv_tc_kernel<ACT, 32, false, ACT2_NONE, true, true, true>, a, smem, s)); \
+            else if (a.epi_groups == 2) DNB_TRY(launch_one(conv_tc_kernel<ACT, 32, false, ACT2_NONE, false, true, true, 2>, a, smem, s)); \
             else DNB_TRY(launch_one(conv_tc_kernel<ACT, 32, false, ACT2_NONE, false, true, true>, a, smem, s)); \
         } else                                                                  \
         if (cpc == 32) DNB_TC_GO(ACT, 32, false, ACT2_NONE, true);              \
@@ -841,7 +1070,7 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
         // fused shortcut: the two pairs the reference's cfgs use (yolov3: leaky conv, linear shortcut; resnet:
         // linear conv, leaky shortcut) are compile-time, every other pair takes the run-time switches
         if (a.ep.yolo_entries) DNB_FAIL(DNB_EUNSUPPORTED, "conv_tc: a residual and a yolo head in one launch");
-        if (a.stage_bufs != (a.pair ? 2 : 4)) DNB_FAIL(DNB_EINVAL, "conv_tc: a fused residual needs four staging buffers (two in pair mode)");
+        if (a.stage_bufs != 4) DNB_FAIL(DNB_EINVAL, "conv_tc: a fused residual needs four staging buffers");
         if (a.ep.activation == DNB_LEAKY && a.ep.activation2 == DNB_LINEAR) DNB_TC_LAUNCH_ACT(DNB_LEAKY, DNB_LINEAR);
         else if (a.ep.activation == DNB_LINEAR && a.ep.activation2 == DNB_LEAKY) DNB_TC_LAUNCH_ACT(DNB_LINEAR, DNB_LEAKY);
         else DNB_TC_LAUNCH_ACT(ACT_GENERIC, ACT_GENERIC);
@@ -850,6 +1079,7 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
 #undef DNB_TC_LAUNCH_ACT_SINGLE
 #undef DNB_TC_LAUNCH_ACT
 #undef DNB_TC_GO_SINGLE
+#undef DNB_TC_GO_WIDE
 #undef DNB_TC_GO
     DNB_LAUNCH_CHECK("conv_tc");
     return DNB_OK;

@@ -326,3 +326,50 @@ def test_pairs_start_at_sixteen_iterations(mode, c, pair, monkeypatch):
     plan, got, _ = run_conv(case, mode, "nhwc", "nhwc")
     assert f"pair={pair}" in plan.describe() and "splits=1" in plan.describe(), plan.describe()
     parity(got, oracle_conv(case), 3e-2 if mode == dn.MODE_BF16 else 1e-2)
+
+
+TWO_GROUPS = {   # (case, in / out layout, residual, xnor): launches whose CTAs have two groups of epilogue warps, at odd sizes
+    "pair_residual_odd_tiles": (dict(b=9, c=64, h=19, w=17, n=256, size=3), "nhwc", True, False),
+    "pair_residual_two_filter_tiles": (dict(b=40, c=512, h=11, w=13, n=512, size=1), "nhwc", True, False),
+    "pair_short_loop": (dict(b=33, c=512, h=13, w=21, n=256, size=1), "nhwc", False, False),
+    "darknet_layout_half_a_chunk_over": (dict(b=40, c=256, h=13, w=19, n=272, size=3), "nchw", False, False),
+    "darknet_layout_fewer_filters_than_a_chunk": (dict(b=3, c=64, h=33, w=21, n=24, size=3), "nchw", False, False),
+    "xnor_one_chunk": (dict(b=5, c=96, h=11, w=13, n=32, size=3), "nhwc", False, True),
+    "xnor_ragged": (dict(b=70, c=256, h=14, w=15, n=200, size=1), "nhwc", False, True),
+}
+
+
+@pytest.mark.parametrize("name", list(TWO_GROUPS))
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
+def test_two_epilogue_groups(name, mode, monkeypatch):
+    """The second group of epilogue warps changes who finishes a value, not how: equal to one group's output to the bit (pairs with a residual,
+    which always have two: to the convolution's own output plus the residual, rounded once more)."""
+    import ctypes as C
+    import numpy as np
+    import torch
+    from gpu_util import dev_nhwc, empty_nhwc, host_from_nhwc
+    shape, layout, residual, xnor = TWO_GROUPS[name]
+    if xnor and mode == dn.MODE_BF16:
+        pytest.skip("xnor layers have one kind")
+    case = conv_case(730, **shape)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    out = {}
+    for groups in ("1", "2"):
+        monkeypatch.setenv("DNB_TC_EPI", groups)
+        plan, out[groups], _ = run_conv(case, mode, "nhwc", layout, xnor=xnor)
+        if not residual:
+            assert f"epi={groups}" in plan.describe(), plan.describe()
+    assert np.array_equal(out["1"], out["2"])
+    if not residual:
+        return
+    store = torch.bfloat16 if mode == dn.MODE_BF16 else torch.float32
+    add = np.random.Generator(np.random.Philox(key=[7, 7])).standard_normal(out["1"].shape, dtype=np.float32)
+    xt, xd = dev_nhwc(case["x"], store)
+    at, ad = dev_nhwc(add, store)
+    yt, yd = empty_nhwc(*out["1"].shape, store)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    dn.check(dn.lib().dnb_conv_shortcut_forward(plan.handle, C.byref(xd), C.byref(ad), C.byref(yd), 1.0, 1.0, dn.ACTIVATIONS["linear"], stream))
+    torch.cuda.synchronize()
+    plan.check_status()
+    assert "pair=1" in plan.describe() and "epi=2" in plan.describe(), plan.describe()
+    parity(host_from_nhwc(yt, case["w"].shape[0]), out["1"] + host_from_nhwc(at, add.shape[1]), 2 ** -7 if mode == dn.MODE_BF16 else 2 ** -10)
