@@ -646,6 +646,17 @@ static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeo
     return DNB_OK;
 }
 
+// Microseconds of the persistent kernel by the measure of split_of: an epilogue hides behind the next tile's K loop, or the
+// other way round, and the last one is exposed; 64-filter tiles alone on an SM wait for their MMAs' results longer.
+static double persistent_us(const TcArgs &a, int k_iters, bool residual)
+{
+    const long long slots = a.pair ? sm_count() / 2 : sm_count();
+    const double share = (double)((a.total_tiles + slots - 1) / slots);
+    const double loop = k_iters * (!a.pair && a.bn <= 64 && share < 2.0 ? 0.18 : a.pair ? 0.31 : iter_us(a.pair, a.bn));
+    const double epilogue = a.bn * (residual ? 0.02 : 0.015);
+    return 3.6 + share * (loop > epilogue ? loop : epilogue) + epilogue;
+}
+
 // Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
 static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual)
 {
@@ -689,8 +700,22 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         if (v >= 64 && v <= 256 && v % 64 == 0 && p->n_pad > v) a.bn = v;
     }
     a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
-    while (ptiles * a.n_tiles < sm_count() && a.bn >= 128 && a.bn % 128 == 0) {  // too few tiles to fill the SMs
-        a.bn /= 2;
+    // Too few tiles to fill the SMs: narrower ones, as long as the launch is estimated to end sooner.  Up to 128 filters an MMA takes
+    // the same 77 clocks, so what counts is how many tiles the fullest SM gets: 50 pixel tiles of 256 filters are better cut into 100 tiles of 128
+    // than into 200 of 64 (3x3 128 -> 256 at 76 x 76 20.9 -> 18.9 us, 256 -> 512 at 4 x 26 x 26 32.7 -> 26.8; YOLOv3-608, one image, in a graph 898 -> 874,
+    // YOLOv3-416, four, 1282 -> 1203).
+    if (ptiles * a.n_tiles < sm_count()) {
+        auto estimate = [&](int bn) {
+            TcArgs t;
+            t.pair = 0; t.bn = bn; t.total_tiles = ptiles * ((p->n_pad + bn - 1) / bn);
+            return persistent_us(t, g.size * g.size * a.c_blocks, residual);
+        };
+        int best = a.bn;
+        for (int bn = a.bn; bn >= 128 && bn % 128 == 0 && ptiles * ((p->n_pad + bn - 1) / bn) < sm_count();) {
+            bn /= 2;
+            if (estimate(bn) <= estimate(best)) best = bn;
+        }
+        a.bn = best;
         a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
     }
     // A launch that writes Darknet's layout spends a store per output element in its epilogue; behind a short K loop
@@ -729,17 +754,6 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         }
     }
     a.total_tiles = a.pair ? (ptiles + 1) / 2 * a.n_tiles : ptiles * a.n_tiles;
-}
-
-// Microseconds of the persistent kernel by the measure of split_of: an epilogue hides behind the next tile's K loop, or the
-// other way round, and the last one is exposed; 64-filter tiles alone on an SM wait for their MMAs' results longer.
-static double persistent_us(const TcArgs &a, int k_iters, bool residual)
-{
-    const long long slots = a.pair ? sm_count() / 2 : sm_count();
-    const double share = (double)((a.total_tiles + slots - 1) / slots);
-    const double loop = k_iters * (!a.pair && a.bn <= 64 && share < 2.0 ? 0.18 : a.pair ? 0.31 : iter_us(a.pair, a.bn));
-    const double epilogue = a.bn * (residual ? 0.02 : 0.015);
-    return 3.6 + share * (loop > epilogue ? loop : epilogue) + epilogue;
 }
 
 static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,

@@ -329,9 +329,9 @@ def test_pairs_start_at_sixteen_iterations(mode, c, pair, monkeypatch):
 
 
 TWO_GROUPS = {   # (case, in / out layout, residual, xnor): launches whose CTAs have two groups of epilogue warps, at odd sizes
-    "pair_residual_odd_tiles": (dict(b=9, c=64, h=19, w=17, n=256, size=3), "nhwc", True, False),
-    "pair_residual_two_filter_tiles": (dict(b=40, c=512, h=11, w=13, n=512, size=1), "nhwc", True, False),
-    "pair_short_loop": (dict(b=33, c=512, h=13, w=21, n=256, size=1), "nhwc", False, False),
+    "pair_residual_odd_tiles": (dict(b=61, c=64, h=19, w=17, n=256, size=3), "nhwc", True, False),
+    "pair_residual_two_filter_tiles": (dict(b=73, c=1024, h=11, w=13, n=512, size=1), "nhwc", True, False),
+    "pair_short_loop": (dict(b=73, c=72, h=13, w=21, n=256, size=3), "nhwc", False, False),
     "darknet_layout_half_a_chunk_over": (dict(b=40, c=256, h=13, w=19, n=272, size=3), "nchw", False, False),
     "darknet_layout_fewer_filters_than_a_chunk": (dict(b=3, c=64, h=33, w=21, n=24, size=3), "nchw", False, False),
     "xnor_one_chunk": (dict(b=5, c=96, h=11, w=13, n=32, size=3), "nhwc", False, True),
