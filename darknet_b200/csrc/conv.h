@@ -90,6 +90,7 @@ struct alignas(64) TcArgs {
     int pair;             // 1: clusters of two CTAs share every MMA (cta_group::2); total_tiles then counts PAIRS of pixel tiles,
                           // b_bytes and the weight map's box cover half a filter tile, bn is 256
     int ctas_per_sm;      // 2 for narrow tiles (TMEM and shared memory are sized so that two CTAs share an SM), else 1
+    int pool;             // 1: tmy (and tms) are the 2x2 stride-2 maxpool's output; wt and ht are even
     int epi_groups;       // groups of four epilogue warps: 2 where a CTA has its SM to itself and staged rows are 128 bytes, else 1
     int a_bytes, b_bytes; // shared-memory bytes of one stage's activation / weight tile (1024-multiples)
     int store_row_bytes;  // bytes of one staged output row (128, 64 or 32) = swizzle span of tmy
@@ -243,6 +244,8 @@ struct dnb_conv_plan {
     dnb::Fp32TcArgs ft;      // its launch block, for input ft_x_ptr
     const void *ft_x_ptr, *ft_y_ptr;   // ... and channels-last output ft_y_ptr (or null)
     int ft_x_cpitch, ft_y_cpitch, ft_layouts;
+    int tc_pool;             // the cached launch block writes the pooled output
+    int pool_fits;           // conv_pool_fusable's answer: 0 not asked yet, 1 yes, -1 no
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout
     int device;
     long long wait_limit;    // bound of the kernels' waits in cycles (0: the default, about one second)
@@ -253,8 +256,13 @@ struct dnb_conv_plan {
 bool conv_shortcut_fusable(const dnb_conv_plan *p, const dnb_tensor *add, const dnb_tensor *y, float alpha);
 int conv_shortcut_general(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor *y, float alpha, float beta, int activation2, cudaStream_t s);
 
+// Convolution and the 2x2 maxpool with stride 2 after it in one launch (persistent tensor-core kernel, leaky activation, even maps): y is the
+// maxpool's output.  conv_pool_fusable: whether the layer is one of those, and its launch one that fills the GPU.
+bool conv_pool_fusable(dnb_conv_plan *p);
+int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, cudaStream_t s);
+
 dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch);
 
 // producers of a tensor-core xnor layer's int8 operand (see conv_plan.cu)
 int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int batch, int c, int h, int w);
-bool conv_plan_link_signs(dnb_conv_plan *producer, dnb_conv_plan *consumer, const void *tensor);
+bool conv_plan_link_signs(dnb_conv_plan *producer, dnb_conv_plan *consumer, const void *tensor, bool pooled = false);

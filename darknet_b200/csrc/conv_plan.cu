@@ -403,7 +403,7 @@ static double nchw_run_penalty(int run)
     return scale * base;
 }
 
-static void pick_pixel_tile(const ConvGeom &g, bool nchw_out, int *wt, int *ht, int *bt)
+static void pick_pixel_tile(const ConvGeom &g, bool nchw_out, int *wt, int *ht, int *bt, bool even = false)
 {
     // wt*ht*bt == 128, powers of two; least padded work, then widest rows.
     // A launch that writes Darknet's layout stores, per filter plane, one run of wt pixels per tile row: runs shorter
@@ -412,6 +412,7 @@ static void pick_pixel_tile(const ConvGeom &g, bool nchw_out, int *wt, int *ht, 
     double best = 1e300;
     for (int w = 1; w <= 128; w *= 2)
         for (int h = 1; w * h <= 128; h *= 2) {
+            if (even && (w < 2 || h < 2)) continue;
             const int b = 128 / (w * h);
             const double work = (double)round_up(g.out_w, w) * round_up(g.out_h, h) * round_up(g.batch, b);
             double score = work * (1.0 + 1e-6 * (128 - w) + 1e-7 * (128 - h));
@@ -658,10 +659,10 @@ static double persistent_us(const TcArgs &a, int k_iters, bool residual)
 }
 
 // Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
-static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual)
+static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual, bool pool = false)
 {
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
-    pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt);
+    pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt, pool);
     // Halo mode (experimental, off unless DNB_TC_HALO is 1 or 2): one activation box per channel block serves all
     // nine taps of a 3x3 stride-1 layer, which cuts the bytes that cross L2 -> shared memory by 2.3x on the
     // 32- and 64-channel layers of large maps.  Measured on YOLOv3-608 batch 64 it does not pay yet: the 8 x 16
@@ -672,7 +673,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     {
         const char *e = getenv("DNB_TC_HALO");
         const int knob = e ? atoi(e) : 0;
-        if (knob != 0 && !i8 && g.size == 3 && g.stride == 1 && g.pad == 1 && a.row_bytes == 128 && g.out_w >= 8 && g.out_h >= 16) {
+        if (knob != 0 && !i8 && !pool && g.size == 3 && g.stride == 1 && g.pad == 1 && a.row_bytes == 128 && g.out_w >= 8 && g.out_h >= 16) {
             const double work_h = (double)round_up(g.out_w, 8) * round_up(g.out_h, 16) * g.batch;
             const double work_0 = (double)round_up(g.out_w, a.wt) * round_up(g.out_h, a.ht) * round_up(g.batch, a.bt);
             if (knob == 2 || (a.c_blocks <= 2 && work_h <= 1.08 * work_0)) { a.halo = 1; a.wt = 8; a.ht = 16; a.bt = 1; }
@@ -747,7 +748,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         const int k_iters_p = g.size * g.size * a.c_blocks;
         const bool enough = pair_tiles >= clusters || (k_iters_p >= 64 && 2 * pair_tiles >= clusters);
         const bool legal = !a.halo && a.row_bytes == 128 && g.n % 256 == 0 && enough && channels_last && y_cpitch * (bf16 ? 2 : 4) >= 128;
-        if (legal && (knob == 2 || (g.size >= 3 && (knob == 1 || (knob < 0 && residual))) || (knob != 0 && k_iters_p >= 16))) {
+        if (legal && !pool && (knob == 2 || (g.size >= 3 && (knob == 1 || (knob < 0 && residual))) || (knob != 0 && k_iters_p >= 16))) {
             a.pair = 1;
             a.bn = 256;
             a.n_tiles = p->n_pad / 256;
@@ -757,7 +758,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
 }
 
 static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
-                         const ConvEpilogue *res, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0)
+                         const ConvEpilogue *res, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0, bool pool = false)
 {
     const void *residual = res ? res->residual : nullptr;   // fused residual, if any
     const int res_cpitch = res ? res->res_cpitch : 0, res_stride = residual ? res->res_stride : 1, res_c = residual ? res->res_c : 0;
@@ -783,7 +784,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.bk = a.row_bytes / es;
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
     a.taps = g.size * g.size;
-    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
+    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, pool);
+    a.pool = pool ? 1 : 0;
     a.n_pad = p->n_pad;
     a.n_tot = a.n_tiles * a.bn;
     a.a_bytes = 128 * a.row_bytes;
@@ -794,7 +796,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // at least four ring stages
     const int out_es = bf16 ? 2 : 4;   // channels-last output uses the plan's storage type
     const int pitch_bytes = y_nhwc ? y_cpitch * out_es : 32;
-    const int min_srb = sign_out ? 128 : 16 * out_es;  // a staged row holds at least one 16-column piece of the accumulator; the sign output is built for 32 columns per chunk
+    const int min_srb = sign_out || pool ? 128 : 16 * out_es;  // a staged row holds at least one 16-column piece of the accumulator; the sign output is built for 32 columns per chunk
     int srb = pitch_bytes >= 128 ? 128 : (pitch_bytes >= 64 ? 64 : 32);
     if (srb < min_srb) srb = min_srb;  // the box may be wider than a narrow tensor: the TMA unit clips it
     if (sign_out && (pitch_bytes < 128 || !i8)) DNB_FAIL(DNB_EINVAL, "conv: the sign output needs an int8-kind plan with at least 32 output channels");
@@ -810,7 +812,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // twice the warps hide the per-tile hand-offs that dominate layers with few K iterations.
     a.ctas_per_sm = 1;
     a.stage_bufs = residual ? 4 : 2;
-    if (sign_out) a.stage_bufs = 3;   // the third buffer holds the staged signs
+    if (sign_out && !pool) a.stage_bufs = 3;   // the third buffer holds the staged signs (pooled rows and theirs fit the second one)
     a.sign_out = sign_out;
     a.sign_cpitch = sign_cpitch;
     a.debug = (getenv("DNB_TC_DEBUG") ? atoi(getenv("DNB_TC_DEBUG")) : 0) | p->debug_bits;
@@ -863,7 +865,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         // Other single CTAs are bound by memory (512 -> 256 at 64 x 52 x 52 in bf16 52 and 52), with a residual they want its tiles by TMA, three
         // chunks ahead (64 -> 256 at 256 x 56 x 56 342 us, 416 through this path).  DNB_TC_EPI=1: one group (pairs with a residual: two).
         const int loop = g.size * g.size * a.c_blocks, epi_knob = getenv("DNB_TC_EPI") ? atoi(getenv("DNB_TC_EPI")) : 2;
-        const bool two = residual ? a.pair != 0 : epi_knob != 1 && (a.pair ? loop < 32 : nchw_out || i8);
+        const bool two = pool ? false : residual ? a.pair != 0 : epi_knob != 1 && (a.pair ? loop < 32 : nchw_out || i8);
         if (a.ctas_per_sm == 1 && two && (a.pair || !getenv("DNB_TC_SRB")) && (!y_nhwc || srb == 128)) {
             const int bufs = y_nhwc ? a.stage_bufs : 0;
             const int fit = (int)((max_smem - (long)conv_tc_fixed_smem(128, a.bn, bufs)) / (a.a_bytes + a.b_bytes));
@@ -905,7 +907,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
         const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1;
         const int k_iters = g.size * g.size * a.c_blocks;
-        if (knob != 0 && !a.halo && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2)) {
+        if (knob != 0 && !a.halo && !pool && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2)) {
             // pixels of a 1x1 layer in one row: of the whole batch where nothing is stored per image
             auto flat = [&](ConvGeom sg) {
                 if (sg.size == 1 && sg.stride == 1 && sg.pad == 0) {
@@ -941,7 +943,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     if (p->tc_split) {
         p->tc_sign_out = sign_out;
         p->tc_x_ptr = x->data; p->tc_x_cpitch = x->cpitch; p->tc_y_ptr = y_nhwc; p->tc_y_cpitch = y_cpitch; p->tc_y_dtype = y_dtype;
-        p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_res_c = res_c; p->tc_res_stride = res_stride; p->tc_nchw_out = nchw_out ? 1 : 0;
+        p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_res_c = res_c; p->tc_res_stride = res_stride; p->tc_nchw_out = nchw_out ? 1 : 0; p->tc_pool = 0;
         return DNB_OK;
     }
     a.g = g;
@@ -957,9 +959,10 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         // the channel extent is the layer's own (padded to 8), the pitch whatever the tensor has: the output may be a
         // channel range of a wider tensor (a [route] output), and the boxes must not spill into its neighbour
         const int y_chan = round_up(g.n, 8) < y_cpitch ? round_up(g.n, 8) : y_cpitch;
-        uint64_t dims[4] = {(uint64_t)y_chan, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
-        uint64_t strides[3] = {opix, opix * g.out_w, opix * g.out_w * g.out_h};
-        uint32_t box[4] = {(uint32_t)(srb / out_es), (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
+        const int half = pool ? 2 : 1, yw = g.out_w / half, yh = g.out_h / half;
+        uint64_t dims[4] = {(uint64_t)y_chan, (uint64_t)yw, (uint64_t)yh, (uint64_t)g.batch};
+        uint64_t strides[3] = {opix, opix * yw, opix * yw * yh};
+        uint32_t box[4] = {(uint32_t)(srb / out_es), (uint32_t)(a.wt / half), (uint32_t)(a.ht / half), (uint32_t)a.bt};
         DNB_TRY(encode_tensor_map(&a.tmy, bf16, 4, y_nhwc, dims, strides, box, srb));
         {   // the 32 consecutive rows of one epilogue warp: wt*ht*bt = 128 in powers of two, so they are a box too
             const int w2 = a.wt < 32 ? a.wt : 32, h2 = a.ht < 32 / w2 ? a.ht : 32 / w2, b2 = 32 / (w2 * h2);
@@ -977,9 +980,10 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         }
     }
     if (sign_out) {
-        uint64_t dims[4] = {(uint64_t)sign_cpitch, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
-        uint64_t strides[3] = {(uint64_t)sign_cpitch, (uint64_t)sign_cpitch * g.out_w, (uint64_t)sign_cpitch * g.out_w * g.out_h};
-        uint32_t box[4] = {32u, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
+        const int half = pool ? 2 : 1, yw = g.out_w / half, yh = g.out_h / half;
+        uint64_t dims[4] = {(uint64_t)sign_cpitch, (uint64_t)yw, (uint64_t)yh, (uint64_t)g.batch};
+        uint64_t strides[3] = {(uint64_t)sign_cpitch, (uint64_t)sign_cpitch * yw, (uint64_t)sign_cpitch * yw * yh};
+        uint32_t box[4] = {32u, (uint32_t)(a.wt / half), (uint32_t)(a.ht / half), (uint32_t)a.bt};
         DNB_TRY(encode_tensor_map(&a.tms, 2, 4, sign_out, dims, strides, box, 32));
     }
     p->tc_sign_out = sign_out;
@@ -993,6 +997,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     p->tc_res_c = res_c;
     p->tc_res_stride = res_stride;
     p->tc_nchw_out = nchw_out ? 1 : 0;
+    p->tc_pool = pool ? 1 : 0;
     return DNB_OK;
 }
 
@@ -1021,11 +1026,11 @@ int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int 
     return consumer->x_i8;
 }
 
-bool conv_plan_link_signs(dnb_conv_plan *producer, dnb_conv_plan *consumer, const void *tensor)
+bool conv_plan_link_signs(dnb_conv_plan *producer, dnb_conv_plan *consumer, const void *tensor, bool pooled)
 {
     if (!producer || producer->kernel != K_XNOR || !producer->xnor_tc) return false;
     const ConvGeom &a = producer->g;
-    if (!conv_plan_expect_signs(consumer, tensor, a.batch, a.n, a.out_h, a.out_w)) return false;
+    if (!conv_plan_expect_signs(consumer, tensor, a.batch, a.n, pooled ? a.out_h / 2 : a.out_h, pooled ? a.out_w / 2 : a.out_w)) return false;
     producer->sign_consumer = consumer;
     return true;
 }
@@ -1054,6 +1059,7 @@ struct Residual {
     const dnb_tensor *add = nullptr;
     float alpha = 1.f, beta = 1.f;
     int activation = DNB_LINEAR;
+    bool pool = false;      // y is the output of the 2x2 maxpool after the convolution
     int yolo_entries = 0;   // instead of a residual: the [yolo] layer's activations, entries per anchor
 };
 
@@ -1092,6 +1098,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
     // core would truncate them instead, a bias that adds up over a network's depth).  A copy in Darknet's layout
     // written by the same launch holds the same rounded values.
     ep.round_tf32 = (p->mode == DNB_MODE_TF32 && y_nhwc && y_dtype == DNB_F32) ? 1 : 0;
+    const bool pool = res && res->pool;
 
     if (p->kernel == K_DIRECT && p->stem_tc && x->dtype == DNB_F32 && y_nhwc && !y_nchw && y_cpitch == g.n) {
         StemTcArgs a;
@@ -1159,8 +1166,8 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         dnb_conv_plan *next = p->sign_consumer;
         void *sign_out = (next && nhwc && nhwc == next->signs_of && next->x_i8) ? next->x_i8 : nullptr;
         if (p->tc_x_ptr != xin.data || p->tc_y_ptr != nhwc || p->tc_y_cpitch != (nhwc ? y_cpitch : 0) || !p->status || p->tc_nchw_out != (nchw ? 1 : 0) ||
-            p->tc_sign_out != sign_out)
-            DNB_TRY(build_tc_args(p, &xin, nhwc, DNB_F32, nhwc ? y_cpitch : 0, nullptr, nchw != nullptr, sign_out, sign_out ? next->c_pad_i8 : 0));
+            p->tc_sign_out != sign_out || p->tc_pool != (pool ? 1 : 0))
+            DNB_TRY(build_tc_args(p, &xin, nhwc, DNB_F32, nhwc ? y_cpitch : 0, nullptr, nchw != nullptr, sign_out, sign_out ? next->c_pad_i8 : 0, pool));
         if (p->tc_split) {
             SplitArgs &a = p->sp;
             a.y_nhwc = nhwc; a.y_cpitch = nhwc ? y_cpitch : 0; a.y_nchw = nchw;
@@ -1217,8 +1224,8 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
     if (p->tc_x_ptr != xin.data || p->tc_x_cpitch != xin.cpitch || p->tc_y_ptr != y_nhwc || p->tc_y_cpitch != y_cpitch ||
         p->tc_y_dtype != y_dtype || !p->status || p->tc_res_ptr != ep.residual || p->tc_res_cpitch != ep.res_cpitch ||
         (ep.residual && (p->tc_res_c != ep.res_c || p->tc_res_stride != ep.res_stride)) ||
-        p->tc_nchw_out != (y_nchw ? 1 : 0))
-        DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, &ep, y_nchw != nullptr));
+        p->tc_nchw_out != (y_nchw ? 1 : 0) || p->tc_pool != (pool ? 1 : 0))
+        DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, &ep, y_nchw != nullptr, nullptr, 0, pool));
     if (p->tc_split) {
         SplitArgs &a = p->sp;
         a.y_nhwc = y_nhwc; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
@@ -1294,6 +1301,42 @@ extern "C" int dnb_conv_yolo_forward(dnb_conv_plan *p, const dnb_tensor *x, cons
     Residual r;
     r.yolo_entries = classes + 5;
     return conv_forward_impl(p, x, y, nullptr, nullptr, (cudaStream_t)stream, &r);
+}
+
+// The launch that the layer would have by itself must be the persistent kernel's, in single CTAs: where it is cut along K or
+// runs in pairs, small maps of deep layers, the pass that is saved is not worth another kernel (512 -> 1024 at 14 x 14, 128 images: 12 us
+// of 1300).  Where it fills the GPU: 3x3 32 -> 64 at 64 x 112 x 112 in TF32 103 + 49 -> 96 us
+// with the pass; three such passes of Darknet-19 with xnor layers, 128 x 224 x 224, 1352 -> 1176 us a step.
+bool conv_pool_fusable(dnb_conv_plan *p)
+{
+    if (p->pool_fits) return p->pool_fits > 0;
+    p->pool_fits = -1;
+    const ConvGeom &g = p->g;
+    const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR && p->xnor_tc;
+    if (p->kernel != K_TC_TF32 && !bf16 && !i8) return false;
+    if (p->d.activation != DNB_LEAKY || g.out_h % 2 || g.out_w % 2 || g.n * (bf16 ? 2 : 4) < 128 || g.n % 8) return false;
+    TcArgs a;
+    const int es = i8 ? 1 : bf16 ? 2 : 4, c_pad = i8 ? p->c_pad_i8 : p->c_pad;
+    a.row_bytes = c_pad * es >= 128 ? 128 : c_pad * es >= 64 ? 64 : 32;
+    a.bk = a.row_bytes / es;
+    a.c_blocks = (c_pad + a.bk - 1) / a.bk;
+    pick_persistent_tiles(p, g, a, false, true, g.n, false);
+    const int k_iters = g.size * g.size * a.c_blocks;
+    if (a.pair || a.halo || a.total_tiles < (k_iters <= 12 ? sm_count() / 2 : sm_count())) return false;
+    p->pool_fits = 1;
+    return true;
+}
+
+int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, cudaStream_t s)
+{
+    const ConvGeom &g = p->g;
+    DNB_TRY(check_tensor(x, "conv + maxpool input"));
+    DNB_TRY(check_tensor(y, "conv + maxpool output"));
+    if (x->n != g.batch || x->c != g.c || x->h != g.h || x->w != g.w || y->n != g.batch || y->c != g.n || y->h != g.out_h / 2 || y->w != g.out_w / 2 || y->layout != DNB_NHWC)
+        DNB_FAIL(DNB_EINVAL, "conv + maxpool: extents or layout");
+    Residual r;
+    r.pool = true;
+    return conv_forward_impl(p, x, y, nullptr, nullptr, s, &r);
 }
 
 extern "C" int dnb_conv_xnor_accumulate(dnb_conv_plan *p, const dnb_tensor *x, int32_t *acc, void *stream)

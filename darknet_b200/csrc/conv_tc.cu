@@ -139,14 +139,18 @@ __device__ __forceinline__ void group_bar(int group) { asm volatile("bar.sync %0
 // is > 0, else -1, 0 beyond the layer's filters) as the int8 channels-last tensor that the xnor layer after it reads as
 // its operand: that layer's sign pass over the f32 tensor disappears.  The signs of a chunk are staged in a third
 // staging buffer (two 4 KB halves in rotation) and leave with the chunk's output rows, in the same bulk group.
+// POOL: the output is that of the 2x2 maxpool with stride 2 after the layer (forward_maxpool_layer, src/maxpool_layer.c:79-117); the layer's own
+// is not written.  A chunk's finished rows are staged as ever, a thread takes the largest of four of them, for a quarter of a pooled pixel, and what leaves is
+// a box of a quarter of the pixels: of the two passes' bytes, 9 per output value of the layer, one is left, and one launch.
 // EG: groups of four epilogue warps.  Two CTAs on an SM bring eight epilogue warps between them; one CTA with four has every SM
 // sub-partition wait for a single warp's chain of TMEM read, residual, arithmetic, staging and store.  The second group takes alternate
 // chunks, with staged rows, a barrier and a storing thread of its own; with a residual (pairs) every warp is on its own, fetches the
 // residual of its 32 pixels and stores them.  Which launches have two: build_tc_args in conv_plan.cu.
-template <int ACT, int CPC, bool OUT_BF16, int ACT2, bool PAIR, bool I8 = false, bool SIGNS = false, int EG = 1>
+template <int ACT, int CPC, bool OUT_BF16, int ACT2, bool PAIR, bool I8 = false, bool SIGNS = false, int EG = 1, bool POOL = false>
 __global__ void __launch_bounds__(64 + 128 * EG)
 conv_tc_kernel(const __grid_constant__ TcArgs a)
 {
+    static_assert(!POOL || (CPC * (OUT_BF16 ? 2 : 4) == 128 && ACT2 == ACT2_NONE && !PAIR && EG == 1), "the pooled output's variant");
     static_assert(EG == 1 || CPC * (OUT_BF16 ? 2 : 4) == 128, "two epilogue groups: 128-byte staged rows");
     static_assert(ACT2 == ACT2_NONE || EG == (PAIR ? 2 : 1), "a pair fetches its residual into the staged rows of two groups, a single CTA by TMA");
     static_assert(!SIGNS || (I8 && CPC == 32 && !OUT_BF16), "the sign output belongs to the int8 kind with 128-byte staged rows");
@@ -679,7 +683,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         // output like the whole tile is, and sends them off itself; the four warps then meet once per tile instead of
         // twice per chunk, so one warp's TMEM or store wait no longer stalls the other three.
         constexpr bool can_warp_store = ACT2 == ACT2_NONE;
-        const bool warp_stores = can_warp_store && !SIGNS && a.warp_stores != 0 && a.y_nhwc != nullptr;
+        const bool warp_stores = can_warp_store && !SIGNS && !POOL && a.warp_stores != 0 && a.y_nhwc != nullptr;
         const int m0 = quarter * 32;
         const int wl0 = m0 % wt, hl0 = (m0 / wt) % ht, bl0 = m0 / (wt * ht);   // origin of this warp's rows inside the tile
         constexpr bool out_bf16 = OUT_BF16;
@@ -798,7 +802,11 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 }
                 const uint32_t buf = chunk_count & buf_mask;
-                if (!res_tiles) {
+                uint8_t *const pooled = stage_out + 128 * srb + (size_t)(chunk_count & 1u) * 5120;   // POOL: 32 rows of 128 bytes, and of 32 of signs
+                if (POOL) {
+                    if (store_thread && chunk_count >= 2) tma_store_wait_read1();   // the store that last read these pooled rows is done
+                    epilogue_bar();                                                 // ... and everybody with the last chunk's staged rows
+                } else if (!res_tiles) {
                     if (warp_stores) {
                         if (lane == 0 && chunk_count >= 2) tma_store_wait_read1();   // this warp's store that last read its rows of the buffer is done
                         __syncwarp();
@@ -808,7 +816,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 }   // with a residual the buffer is this thread's to overwrite: its tile landed after that store, and
                     // a thread reads and writes its own row only
-                uint8_t *row = stage_out + (size_t)buf * 128 * srb + (size_t)m * srb;
+                uint8_t *row = stage_out + (size_t)(POOL ? 0u : buf) * 128 * srb + (size_t)m * srb;
                 if (!out_bf16) {
 #pragma unroll
                     for (int q = 0; q < srb / 16; ++q)         // 16-byte pieces of 4 floats
@@ -818,6 +826,41 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     for (int q = 0; q < srb / 16; ++q)         // 16-byte pieces of 8 bf16
                         *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = pack_bf16x8<CPC>(r, 8 * q);
                 }
+                if (POOL) {
+                    epilogue_bar();
+                    // pooled pixel et / 4 (half the tile's extents), 16-byte pieces et % 4 and that + 4 of its row
+                    constexpr int VALUES = OUT_BF16 ? 8 : 4;
+                    const int et = threadIdx.x - 64, pp = et >> 2, pw = wt >> 1, ph = ht >> 1;
+                    const int top = ((pp / (pw * ph)) * ht + 2 * (pp / pw % ph)) * wt + 2 * (pp % pw);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int q = (et & 3) + 4 * h;
+                        uint32_t best[VALUES];
+#pragma unroll
+                        for (int e = 0; e < VALUES; ++e) best[e] = __float_as_uint(-FLT_MAX);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int rr = top + (i & 1) + (i >> 1) * wt;
+                            const uint4 v = *reinterpret_cast<const uint4 *>(stage_out + (size_t)rr * srb + ((q ^ (rr & 7)) << 4));
+                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int e = 0; e < VALUES; ++e) {
+                                const uint32_t bits = !OUT_BF16 ? w[e & 3] : (e & 1) ? (w[e / 2] & 0xffff0000u) : (w[e / 2] << 16);
+                                best[e] = __float_as_uint(fmaxf(__uint_as_float(best[e]), __uint_as_float(bits)));
+                            }
+                        }
+                        uint4 o;
+                        if constexpr (OUT_BF16) o = pack_bf16x8<VALUES>(best, 0);
+                        else o = make_uint4(best[0], best[1], best[2], best[3]);
+                        *reinterpret_cast<uint4 *>(pooled + pp * 128 + ((q ^ (pp & 7)) << 4)) = o;
+                        if (SIGNS) {   // of the pooled values, 4 channels a word
+                            uint32_t wd = 0u;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) wd |= (4 * q + e < nvalid ? (__uint_as_float(best[e]) > 0.f ? 0x01u : 0xFFu) : 0u) << (8 * e);
+                            *reinterpret_cast<uint32_t *>(pooled + 4096 + pp * 32 + (((q >> 2) ^ ((pp >> 2) & 1)) << 4) + 4 * (q & 3)) = wd;
+                        }
+                    }
+                } else
                 if (SIGNS) {
                     // 32 signs of this pixel = one 32-byte row of a 32-byte-swizzled box: its two 16-byte halves swap on rows 4..7 of every 8
                     uint32_t sw[8];
@@ -847,7 +890,13 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 } else
                 epilogue_bar();
-                if (!warp_stores && store_thread) {
+                if (POOL) {
+                    if (store_thread) {
+                        if (!(dbg & 2)) tma_store_4d(ymap, smem_u32(pooled), nl0, ow0 >> 1, oh0 >> 1, b0);
+                        if (SIGNS) tma_store_4d(&a.tms, smem_u32(pooled + 4096), nl0, ow0 >> 1, oh0 >> 1, b0);
+                        tma_store_commit();
+                    }
+                } else if (!warp_stores && store_thread) {
                     // the TMA unit clips the box at the tensor's extents: ragged tiles need no predicates
                     if (y_nhwc && !(dbg & 2) && (!PAIR || b0 < g.batch)) tma_store_4d(ymap, smem_u32(stage_out + (size_t)buf * 128 * srb), nl0, ow0, oh0, b0);
                     if (SIGNS && (!PAIR || b0 < g.batch))
@@ -860,7 +909,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                         request_residual();
                     }
                 }
-                if (y_nchw && pix_ok) {
+                if (!POOL && y_nchw && pix_ok) {
                     // Darknet-layout copy: this thread's pixel, one filter plane per column, straight from the registers
                     // (a warp's 32 pixels are wt-long runs of each plane).  BF16 plans write what the channels-last
                     // copy holds: the value rounded to bf16.
@@ -1002,6 +1051,16 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
     if (a.ep.residual && a.epi_groups != (a.pair ? 2 : 1)) DNB_FAIL(DNB_EINVAL, "conv_tc: a residual with %d epilogue groups", a.epi_groups);
     if (a.epi_groups == 2 && a.store_row_bytes != 128) DNB_FAIL(DNB_EINVAL, "conv_tc: two epilogue groups need 128-byte staged rows");
     if (a.pair && !((!obf && cpc == 32) || (obf && cpc == 64))) DNB_FAIL(DNB_EINVAL, "conv_tc: pair mode needs 128-byte staged rows");
+    if (a.pool) {
+        if (a.pair || a.epi_groups != 1 || a.store_row_bytes != 128 || a.ep.activation != DNB_LEAKY || a.ep.residual || a.ep.yolo_entries || a.y_nchw || (a.wt | a.ht) & 1)
+            DNB_FAIL(DNB_EINVAL, "conv_tc: no pooled variant of this launch");
+        if (i8 && a.sign_out) DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 32, false, ACT2_NONE, false, true, true, 1, true>, a, smem, s));
+        else if (i8) DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 32, false, ACT2_NONE, false, true, false, 1, true>, a, smem, s));
+        else if (obf) DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 64, true, ACT2_NONE, false, false, false, 1, true>, a, smem, s));
+        else DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 32, false, ACT2_NONE, false, false, false, 1, true>, a, smem, s));
+        DNB_LAUNCH_CHECK("conv_tc");
+        return DNB_OK;
+    }
     // one instantiation per (activation, columns per staged chunk, output type, fused shortcut, pair mode, operand kind)
 #define DNB_TC_GO(ACT, CPC, OBF, ACT2, I8)                                                          \
     do {                                                                                            \

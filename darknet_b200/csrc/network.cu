@@ -70,6 +70,8 @@ struct Layer {
     dnb_tensor own_out{};          // ... where that layer's addend has another shape: the convolution's own output, filled for who asks for it
     // a convolution that also performs the [yolo] layer right after it (that layer is then fused_into_prev too)
     bool fuses_next_yolo = false;
+    // a convolution that also performs the 2x2 maxpool with stride 2 right after it (own_out is there for who asks for its own output)
+    bool fuses_next_pool = false;
     // a maxpool layer that also writes the signs of its output, the next (tensor-core xnor) layer's operand
     int8_t *sign_out = nullptr;
     int sign_pitch = 0;
@@ -398,6 +400,30 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         cudaFree(C.out.data);      // never written: the convolution stores straight into the yolo layer's output
         C.out.data = nullptr;
     }
+    // Fuse "convolution, then 2x2 [maxpool] with stride 2" when nothing else reads the convolution's output: its epilogue writes the largest of
+    // each four pixels, and the pass that read the whole map back disappears.  The convolution's own output is made from its input for
+    // who asks for it (own_output).  DNB_FUSE_POOL=0 keeps the two layers separate.
+    const bool fuse_pool = getenv("DNB_FUSE_POOL") ? atoi(getenv("DNB_FUSE_POOL")) != 0 : true;
+    for (int i = 1; fuse_pool && i + 1 < (int)net->layers.size(); ++i) {
+        Layer &C = net->layers[i], &M = net->layers[i + 1];
+        if (C.kind != L_CONV || !C.plan || M.kind != L_MAXPOOL || M.size != 2 || M.stride != 2 || M.padding < 0 || M.padding > 1 || !C.out.data) continue;
+        if (M.out_h != C.out_h / 2 || M.out_w != C.out_w / 2) continue;
+        bool read_elsewhere = false, sign_pass = false;
+        for (int j = i + 2; j < (int)net->layers.size(); ++j) {
+            const Layer &L = net->layers[j];
+            if (L.kind == L_SHORTCUT && L.from == i) read_elsewhere = true;
+            if (L.kind == L_ROUTE)
+                for (int id : L.inputs) if (id == i) read_elsewhere = true;
+            // the maxpool kernel also writes the next xnor layer's operand; of the convolutions only an xnor layer does
+            if (j == i + 2 && L.kind == L_CONV && L.cd.xnor && !C.cd.xnor) sign_pass = true;
+        }
+        if (read_elsewhere || sign_pass || !conv_pool_fusable(C.plan)) continue;
+        C.fuses_next_pool = true;
+        M.fused_into_prev = true;
+        M.launches = 0;
+        C.own_out = C.out;
+        C.out.data = nullptr;
+    }
     // Zero-copy [route]: where a route input is produced by a layer whose kernel can write a channel range of a wider
     // channels-last tensor (tensor-core convolutions, with or without a fused shortcut, and upsample), and everything that
     // reads it can read such a range (convolutions, routes, the yolo head, upsample), the input's tensor BECOMES its
@@ -445,6 +471,8 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
         if (B.kind != L_CONV || !B.plan || !A.out.data || A.out.layout != DNB_NHWC) continue;
         if (A.kind == L_CONV && A.plan) {
             if (conv_plan_link_signs(A.plan, B.plan, A.out.data)) B.launches = 1;   // no sign pass of its own
+        } else if (A.kind == L_MAXPOOL && A.fused_into_prev) {
+            if (conv_plan_link_signs(net->layers[i - 1].plan, B.plan, A.out.data, true)) B.launches = 1;
         } else if (A.kind == L_MAXPOOL && A.out.dtype == DNB_F32 && A.out.cpitch == A.out_c) {
             A.sign_out = conv_plan_expect_signs(B.plan, A.out.data, net->batch, A.out_c, A.out_h, A.out_w);
             if (A.sign_out) { A.sign_pitch = A.out_c; B.launches = 1; }
@@ -702,7 +730,7 @@ extern "C" int dnb_network_set_conv_params(dnb_network *net, int layer, const fl
     return DNB_OK;
 }
 
-// Layer i's output as a step leaves it, in *t; the own output of a convolution that was fused with a shortcut of another shape is
+// Layer i's output as a step leaves it, in *t; the own output of a convolution that was fused with a shortcut of another shape or a maxpool is
 // made from its input, which is still there, on s.
 static int own_output(dnb_network *net, int i, dnb_tensor *t, cudaStream_t s)
 {
@@ -792,6 +820,10 @@ static int forward_layer(dnb_network *net, int i, const float *device_input, con
             const dnb_tensor add = part_of(net->layers[S.from].out, p), sum = part_of(S.out, p);
             return conv_shortcut_general(plan_of(L, p), &in, &add, &sum, S.alpha, S.beta, S.activation, s);
         }
+        if (L.fuses_next_pool) {
+            const dnb_tensor pooled = part_of(net->layers[i + 1].out, p);
+            return conv_pool_forward(plan_of(L, p), &in, &pooled, s);
+        }
         if (L.fuses_next_yolo) {
             Layer &Y = net->layers[i + 1];
             const dnb_tensor head = part_of(Y.out, p);
@@ -806,7 +838,9 @@ static int forward_layer(dnb_network *net, int i, const float *device_input, con
         flat.c = flat.cpitch = L.cd.c;
         return dnb_conv_forward(plan_of(L, p), &flat, &out, nullptr, s);
     }
-    case L_MAXPOOL: return launch_maxpool(&in, &out, L.size, L.stride, L.padding, s, L.sign_out, L.sign_pitch);
+    case L_MAXPOOL:
+        if (L.fused_into_prev) return DNB_OK;   // done by the convolution before it
+        return launch_maxpool(&in, &out, L.size, L.stride, L.padding, s, L.sign_out, L.sign_pitch);
     case L_UPSAMPLE: return launch_upsample(&in, &out, L.stride, L.scale, s);
     case L_SHORTCUT: {
         if (L.fused_into_prev) return DNB_OK;   // done by the convolution before it
@@ -1109,7 +1143,7 @@ static void plan_step(dnb_network *net)
         for (int id : L.inputs) ok = ok && aligned(net->layers[id].out, each);
         return ok;
     };
-    auto cuttable = [&](int i) { return i > 0 && i < n && !net->layers[i - 1].fuses_next_shortcut && !net->layers[i - 1].fuses_next_yolo; };
+    auto cuttable = [&](int i) { return i > 0 && i < n && !net->layers[i - 1].fuses_next_shortcut && !net->layers[i - 1].fuses_next_yolo && !net->layers[i - 1].fuses_next_pool; };
 
     const double upload_us = (double)batch * net->inputs * sizeof(float) / copy_rate;
     int front = 0, parts = 1;
