@@ -38,6 +38,9 @@ struct alignas(64) StemTcArgs {
     void *y;                             // channels-last output, pitch == n
     int y_dtype, y_cpitch;
     int n_pad, tmem_cols, tiles, tiles_w, tiles_h;   // filled by the launcher
+    int pool;                            // 1: y is the 2x2 stride-2 maxpool's output
+    float *keep;                         // pooled output: where a copy of the images (Darknet's layout) goes, or null
+    int8_t *signs;                       // pooled output of conv_stem_rows.cu: its signs, 32 bytes a pixel, or null
     int npix, tma_store;                 // ... of conv_stem_rows.cu: output pixels; rows leave through tmy (else plain stores)
     int *status;
     long long wait_limit;                // bound of every device-side wait, SM clock cycles
@@ -45,10 +48,12 @@ struct alignas(64) StemTcArgs {
     ConvEpilogue ep;
 };
 bool conv_stem_tc_covers(const ConvGeom &g);
+bool conv_stem_pool_covers(const ConvGeom &g, int y_dtype, int activation);
 int launch_conv_stem_tc(StemTcArgs a, cudaStream_t s);
 
 // ---- conv_stem_rows.cu : the same layers with their products added in the im2col order (networks with xnor layers)
 bool conv_stem_rows_covers(const ConvGeom &g, int y_dtype);
+bool conv_stem_rows_pool_covers(const ConvGeom &g, int y_dtype);
 int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s);
 
 // The shared memory that a CTA with `cols` columns of TMEM asks for: its `bytes`, or its columns' share of the SM's (228 KB, 1 KB of
@@ -256,10 +261,12 @@ struct dnb_conv_plan {
 bool conv_shortcut_fusable(const dnb_conv_plan *p, const dnb_tensor *add, const dnb_tensor *y, float alpha);
 int conv_shortcut_general(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *add, const dnb_tensor *y, float alpha, float beta, int activation2, cudaStream_t s);
 
-// Convolution and the 2x2 maxpool with stride 2 after it in one launch (persistent tensor-core kernel, leaky activation, even maps): y is the
+// Convolution and the 2x2 maxpool with stride 2 after it in one launch (first-layer or persistent tensor-core kernel, leaky activation, even maps): y is the
 // maxpool's output.  conv_pool_fusable: whether the layer is one of those, and its launch one that fills the GPU.
-bool conv_pool_fusable(dnb_conv_plan *p);
-int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, cudaStream_t s);
+// in_order: the layer will be one of a network with xnor layers.
+bool conv_pool_fusable(dnb_conv_plan *p, bool in_order);
+// keep: a first layer also copies its input, a Darknet tensor, there (null: it does not).
+int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, float *keep, cudaStream_t s);
 
 dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch);
 

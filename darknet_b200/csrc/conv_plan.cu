@@ -1028,7 +1028,7 @@ int8_t *conv_plan_expect_signs(dnb_conv_plan *consumer, const void *tensor, int 
 
 bool conv_plan_link_signs(dnb_conv_plan *producer, dnb_conv_plan *consumer, const void *tensor, bool pooled)
 {
-    if (!producer || producer->kernel != K_XNOR || !producer->xnor_tc) return false;
+    if (!producer || !((producer->kernel == K_XNOR && producer->xnor_tc) || (pooled && producer->stem_tc && producer->g.n == 32))) return false;   // a first layer with its maxpool writes them too
     const ConvGeom &a = producer->g;
     if (!conv_plan_expect_signs(consumer, tensor, a.batch, a.n, pooled ? a.out_h / 2 : a.out_h, pooled ? a.out_w / 2 : a.out_w)) return false;
     producer->sign_consumer = consumer;
@@ -1059,6 +1059,7 @@ struct Residual {
     const dnb_tensor *add = nullptr;
     float alpha = 1.f, beta = 1.f;
     int activation = DNB_LINEAR;
+    float *keep = nullptr;
     bool pool = false;      // y is the output of the 2x2 maxpool after the convolution
     int yolo_entries = 0;   // instead of a residual: the [yolo] layer's activations, entries per anchor
 };
@@ -1100,6 +1101,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
     ep.round_tf32 = (p->mode == DNB_MODE_TF32 && y_nhwc && y_dtype == DNB_F32) ? 1 : 0;
     const bool pool = res && res->pool;
 
+    if (pool && p->kernel == K_DIRECT && !(x->dtype == DNB_F32 && y_nhwc && y_cpitch == g.n)) DNB_FAIL(DNB_EINVAL, "conv + maxpool: the first layer's tensors");
     if (p->kernel == K_DIRECT && p->stem_tc && x->dtype == DNB_F32 && y_nhwc && !y_nchw && y_cpitch == g.n) {
         StemTcArgs a;
         a.x = (const float *)x->data;
@@ -1111,6 +1113,10 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         a.status = p->status;
         a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
         a.g = g; a.ep = ep;
+        a.pool = pool ? 1 : 0;
+        a.keep = pool && x->layout == DNB_NCHW ? res->keep : nullptr;
+        dnb_conv_plan *const next = p->sign_consumer;
+        a.signs = pool && next && y_nhwc == next->signs_of ? next->x_i8 : nullptr;
         // in the im2col order where layers take the signs of what follows from it (see conv_stem_rows.cu), else from the patch, whose
         // offsets inside an image take rows of less than 2^25 values
         const bool rows = (p->keep_k_order || a.xs_h >= (1LL << 31) / 64) && conv_stem_rows_covers(g, y_dtype);
@@ -1307,12 +1313,18 @@ extern "C" int dnb_conv_yolo_forward(dnb_conv_plan *p, const dnb_tensor *x, cons
 // runs in pairs, small maps of deep layers, the pass that is saved is not worth another kernel (512 -> 1024 at 14 x 14, 128 images: 12 us
 // of 1300).  Where it fills the GPU: 3x3 32 -> 64 at 64 x 112 x 112 in TF32 103 + 49 -> 96 us
 // with the pass; three such passes of Darknet-19 with xnor layers, 128 x 224 x 224, 1352 -> 1176 us a step.
-bool conv_pool_fusable(dnb_conv_plan *p)
+bool conv_pool_fusable(dnb_conv_plan *p, bool in_order)
 {
     if (p->pool_fits) return p->pool_fits > 0;
     p->pool_fits = -1;
     const ConvGeom &g = p->g;
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR && p->xnor_tc;
+    if (p->stem_tc) {
+        const int dtype = p->mode == DNB_MODE_BF16 ? DNB_BF16 : DNB_F32;
+        if (!conv_stem_pool_covers(g, dtype, p->d.activation) || g.w >= (1 << 25) || (in_order && !conv_stem_rows_pool_covers(g, dtype))) return false;
+        p->pool_fits = 1;
+        return true;
+    }
     if (p->kernel != K_TC_TF32 && !bf16 && !i8) return false;
     if (p->d.activation != DNB_LEAKY || g.out_h % 2 || g.out_w % 2 || g.n * (bf16 ? 2 : 4) < 128 || g.n % 8) return false;
     TcArgs a;
@@ -1327,7 +1339,7 @@ bool conv_pool_fusable(dnb_conv_plan *p)
     return true;
 }
 
-int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, cudaStream_t s)
+int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y, float *keep, cudaStream_t s)
 {
     const ConvGeom &g = p->g;
     DNB_TRY(check_tensor(x, "conv + maxpool input"));
@@ -1336,6 +1348,7 @@ int conv_pool_forward(dnb_conv_plan *p, const dnb_tensor *x, const dnb_tensor *y
         DNB_FAIL(DNB_EINVAL, "conv + maxpool: extents or layout");
     Residual r;
     r.pool = true;
+    r.keep = keep;
     return conv_forward_impl(p, x, y, nullptr, nullptr, s, &r);
 }
 

@@ -45,7 +45,9 @@ __device__ __forceinline__ float rows_act(float x, int runtime_act)
 
 // C: input channels (1..3); ACT: activation folded at compile time or SR_ACT_GENERIC; OUT_BF16: storage
 // type of the channels-last output.
-template <int C, int ACT, bool OUT_BF16>
+// POOL (f32, 32 filters): the output is that of the 2x2 maxpool with stride 2 after the layer, and optionally its signs, the next xnor layer's operand.
+// Four neighbouring threads own the pixels of a window: a warp takes the largest of each four staged rows and stores eight.
+template <int C, int ACT, bool OUT_BF16, bool POOL = false>
 __global__ void __launch_bounds__(SR_THREADS, 5)
 conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
 {
@@ -102,7 +104,7 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
     const float *const x = a.x;
     const long long xs_b = a.xs_b;
     const int xs_c = (int)a.xs_c, xs_h = (int)a.xs_h, xs_w = (int)a.xs_w;
-    const int npix = a.npix, tiles = a.tiles, plane = g.out_h * g.out_w;
+    const int npix = a.npix, tiles = a.tiles, plane = POOL ? (g.out_h >> 1) * (g.out_w >> 1) : g.out_h * g.out_w;   // POOL: windows
     const int runtime_act = a.ep.activation, do_round = a.ep.round_tf32;
     uint8_t *const y = reinterpret_cast<uint8_t *>(a.y);
     const size_t y_row_bytes = (size_t)a.y_cpitch * (OUT_BF16 ? 2 : 4);
@@ -127,14 +129,17 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
     for (int tile = blockIdx.x;; tile += gridDim.x, ++it) {
         const bool have = tile < tiles;   // uniform over the CTA
         const int buf = it & 1;
+        long long keep_at = -1;           // POOL: where this thread's pixel lies in the copy of the images
         // ---- this thread's 27 input values of the next tile: requested first, used after the epilogue below
         float v[K];
         if (have) {
-            const int p = tile * SR_THREADS + tid;
+            const int p = POOL ? tile * (SR_THREADS / 4) + (tid >> 2) : tile * SR_THREADS + tid;   // POOL: in windows
             const bool valid = p < npix;
-            const int b = p / plane, rem = p - b * plane;
-            const int oy = rem / g.out_w, ox = rem - oy * g.out_w;
+            const int b = p / plane, rem = p - b * plane, row_w = POOL ? g.out_w >> 1 : g.out_w;
+            const int py = rem / row_w, px = rem - py * row_w;
+            const int oy = POOL ? 2 * py + ((tid >> 1) & 1) : py, ox = POOL ? 2 * px + (tid & 1) : px;
             const int iy0 = oy * g.stride - g.pad, ix0 = ox * g.stride - g.pad;
+            if (POOL && a.keep && valid) keep_at = b * xs_b + (long long)oy * xs_h + ox;
             // three row and three column validity flags and one base pointer: a tap costs one predicated load
             const bool rv0 = valid && (unsigned)iy0 < (unsigned)g.h, rv1 = valid && (unsigned)(iy0 + 1) < (unsigned)g.h,
                        rv2 = valid && (unsigned)(iy0 + 2) < (unsigned)g.h;
@@ -207,7 +212,33 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
                         }
                     }
                 }
-                if (tma) {
+                if (POOL) {
+                    __syncwarp();
+                    uint8_t *const mine = sA + pb * SR_A_BYTES + warp * 32 * 128;
+                    const int k = lane >> 2, first = prev_tile * (SR_THREADS / 4) + warp * 8;   // the warp's first window
+                    uint4 best[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int q = (lane & 3) + 4 * h;
+                        uint4 v4[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v4[i] = *reinterpret_cast<const uint4 *>(mine + (4 * k + i) * 128 + ((q ^ ((4 * k + i) & 7)) << 4));
+                        best[h] = largest_of_four<false>(v4);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int q = (lane & 3) + 4 * h;
+                        *reinterpret_cast<uint4 *>(mine + k * 128 + ((q ^ k) << 4)) = best[h];
+                        if (a.signs && first + k < npix) *reinterpret_cast<uint32_t *>(a.signs + (size_t)(first + k) * 32 + 4 * q) = four_signs(best[h]);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && first < npix) {
+                        tma_store_2d(ymap, smem_u32(mine), 0, first);
+                        tma_store_commit();
+                    }
+                } else if (tma) {
                     // each warp stores its own 32 rows: no CTA-wide barrier between the rows and the store
                     fence_async_smem();
                     __syncwarp();
@@ -227,6 +258,10 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
                 // Staged rows narrower than an im2col row (fewer than 128 bytes of output per pixel) put this thread's
                 // im2col row over rows that OTHER warps staged two tiles ago: every warp's stores must have read them.
                 if (out_row_bytes < 128) __syncthreads();
+            }
+            if (POOL && keep_at >= 0) {   // the window's middle is the pixel itself
+#pragma unroll
+                for (int c = 0; c < C; ++c) a.keep[keep_at + c * xs_c] = v[c * 9 + 4];
             }
             uint8_t *row = sA + buf * SR_A_BYTES + row_off;
 #pragma unroll
@@ -496,6 +531,8 @@ bool conv_stem_rows_covers(const ConvGeom &g, int y_dtype)
            (long long)g.batch * g.out_h * g.out_w + SR_THREADS < (1LL << 31);
 }
 
+bool conv_stem_rows_pool_covers(const ConvGeom &g, int y_dtype) { return conv_stem_rows_covers(g, y_dtype) && y_dtype == DNB_F32 && g.n == 32; }
+
 template <typename K>
 static int launch_rows(K kern, size_t smem, int most, const StemTcArgs &a, cudaStream_t s)
 {
@@ -518,6 +555,8 @@ template <int C, bool OBF>
 static int launch_narrow(const StemTcArgs &a, cudaStream_t s)
 {
     const size_t smem = 2 * SR_A_BYTES + (size_t)a.n_pad * 128 + 2 * sizeof(float) * a.n_pad + sizeof(StemRowsShared) + 16;
+    if constexpr (!OBF)
+        if (a.pool) return launch_rows(conv_stem_rows_kernel<C, DNB_LEAKY, false, true>, smem, 5, a, s);
     if (a.ep.activation == DNB_LEAKY) return launch_rows(conv_stem_rows_kernel<C, DNB_LEAKY, OBF>, smem, 5, a, s);
     return launch_rows(conv_stem_rows_kernel<C, SR_ACT_GENERIC, OBF>, smem, 5, a, s);
 }
@@ -544,9 +583,11 @@ int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s)
     const ConvGeom &g = a.g;
     if (!conv_stem_rows_covers(g, a.y_dtype) || a.y_cpitch != g.n) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: geometry outside its coverage");
     if (a.xs_c >= (1LL << 31) / 4 || a.xs_h >= (1LL << 31) / 4) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: image too large for 32-bit offsets");
-    const long long npix = (long long)g.batch * g.out_h * g.out_w;
+    if (a.pool && !(conv_stem_pool_covers(g, a.y_dtype, a.ep.activation) && conv_stem_rows_pool_covers(g, a.y_dtype))) DNB_FAIL(DNB_EINVAL, "first-layer kernel: no pooled variant of this layer");
+    const long long npix = (long long)g.batch * g.out_h * g.out_w / (a.pool ? 4 : 1);   // output pixels
+    const int per_tile = a.pool ? SR_THREADS / 4 : SR_THREADS;
     a.npix = (int)npix;
-    a.tiles = (int)((npix + SR_THREADS - 1) / SR_THREADS);
+    a.tiles = (int)((npix + per_tile - 1) / per_tile);
     a.n_pad = round_up(g.n, 16);
     a.tmem_cols = 32;
     while (a.tmem_cols < a.n_pad) a.tmem_cols *= 2;
@@ -557,7 +598,7 @@ int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s)
     if (a.tma_store) {
         const uint64_t dims[2] = {(uint64_t)g.n, (uint64_t)npix};
         const uint64_t strides[1] = {(uint64_t)rb};
-        const uint32_t box[2] = {(uint32_t)(half / es), 32u};
+        const uint32_t box[2] = {(uint32_t)(half / es), a.pool ? 8u : 32u};
         DNB_TRY(encode_tensor_map(&a.tmy, es == 2 ? 1 : 0, 2, a.y, dims, strides, box, half));
     }
     return es == 2 ? launch_geometry<true>(a, s) : launch_geometry<false>(a, s);

@@ -105,7 +105,9 @@ __device__ __forceinline__ uint64_t plain_smem_desc(uint32_t addr, uint32_t lead
 
 // KS: filter size; S: stride; ACT: activation folded at compile time or ST_ACT_GENERIC; OUT_BF16: storage type of the
 // channels-last output.
-template <int KS, int S, int ACT, bool OUT_BF16>
+// POOL: the output is that of the 2x2 maxpool with stride 2 after the layer.  A warp's 32 pixels are four rows of eight, two rows of four
+// windows: it stages them as ever, takes the largest of each four staged pieces and stores eight pixels.
+template <int KS, int S, int ACT, bool OUT_BF16, bool POOL>
 __global__ void __launch_bounds__(stem_threads(KS, S), stem_ctas(KS))
 conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
 {
@@ -189,6 +191,7 @@ conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
             yx[i] = e < P::W * P::H ? (py << 8) | px | ((py * P::PITCH + P::column(px)) << 16) : -1;
         }
         StemTile at(blockIdx.x, tiles_w, tiles_h);        // the tile whose patch is fetched next
+        StemTile got = at;                                // ... and the one whose patch was
         auto fetch = [&]() {
             const int ix0 = at.tx * ST_TW * S - pad, iy0 = at.ty * ST_TH * S - pad;
             const float *xp = x + (size_t)at.b * xs_b + (long long)iy0 * xs_h + (long long)ix0 * xs_w;   // dereferenced only inside the image
@@ -201,8 +204,10 @@ conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
                 v[i][1] = in && two ? __ldg(p + xs_c) : 0.f;
                 v[i][2] = in && three ? __ldg(p + 2 * xs_c) : 0.f;
             }
+            got = at;
             at.advance(step, tiles_w, tiles_h);
         };
+        float *const keep = POOL ? a.keep : nullptr;
         const uint32_t idesc = mma_idesc<MMA_TF32>(128u, (uint32_t)n_pad);
         const uint64_t da0 = plain_smem_desc(smem_u32(patch0), 0, S * P::PITCH * 16), db0 = plain_smem_desc(smem_u32(sB), 128, 256);
         const uint64_t b_step = (uint64_t)(n_pad * 2);
@@ -217,6 +222,17 @@ conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
             for (int i = 0; i < P::PER_THREAD; ++i)
                 if (yx[i] >= 0) patch[yx[i] >> 16] = make_float4(round_tf32(v[i][0]), round_tf32(v[i][1]), round_tf32(v[i][2]), 0.f);
             fence_async_smem();   // cells visible to the tensor cores
+            if (POOL && keep) {   // a copy of the images: the patch's inner pixels (stride 1, padding 1)
+#pragma unroll
+                for (int i = 0; i < P::PER_THREAD; ++i) {
+                    const int py = (yx[i] >> 8) & 255, px = yx[i] & 255, iy = got.ty * ST_TH - pad + py, ix = got.tx * ST_TW - pad + px;
+                    if (yx[i] < 0 || px < pad || px >= pad + ST_TW || py < pad || py >= pad + ST_TH || iy >= img_h || ix >= img_w) continue;
+                    float *p = keep + (size_t)got.b * xs_b + (long long)iy * xs_h + ix;
+                    p[0] = v[i][0];
+                    if (two) p[xs_c] = v[i][1];
+                    if (three) p[2 * xs_c] = v[i][2];
+                }
+            }
             if (tile + (int)gridDim.x < tiles) fetch();   // a whole tile's time to arrive
             stop = builders_meet<BUILD>(!ok);
             if (warp == 4 && !stop) {
@@ -294,9 +310,37 @@ conv_stem_tc_kernel(const __grid_constant__ StemTcArgs a)
                 }
             }
             tc_fence_before();
+            if (POOL) {
+                // one segment; lane's piece of pooled pixel (rows of 32, 64 or 128 bytes: 16, 32 or 64 pieces)
+                __syncwarp();
+                uint8_t *const mine = sO + (uint32_t)(warp * 32) * seg_bytes;
+                const uint32_t pieces = seg_bytes >> 4;
+                auto swizzled = [&](uint32_t row, uint32_t q) { return row * seg_bytes + ((q ^ ((seg_bytes == 128 ? row : seg_bytes == 64 ? row >> 1 : row >> 2) & q_mask)) << 4); };
+                uint4 best[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t e = lane + 32 * h, pp = e / pieces, q = e - pp * pieces;
+                    if (e >= 8 * pieces) continue;
+                    const uint32_t top = (pp >> 2) * 16 + (pp & 3) * 2;
+                    uint4 v[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const uint4 *>(mine + swizzled(top + (i & 1) + (i >> 1) * 8, q));
+                    best[h] = largest_of_four<OUT_BF16>(v);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t e = lane + 32 * h, pp = e / pieces, q = e - pp * pieces;
+                    if (e < 8 * pieces) *reinterpret_cast<uint4 *>(mine + swizzled(pp, q)) = best[h];
+                }
+            }
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) {
+            if (POOL && lane == 0) {
+                mbar_arrive(empty0 + 8 * acc);
+                if (at.ty * ST_TH + 4 * warp < g.out_h) tma_store_4d(ymap, smem_u32(sO) + (uint32_t)(warp * 32) * seg_bytes, 0, at.tx * (ST_TW / 2), at.ty * (ST_TH / 2) + 2 * warp, at.b);
+                tma_store_commit();
+            } else if (lane == 0) {
                 mbar_arrive(empty0 + 8 * acc);
                 for (uint32_t sg = 0; sg < segs && at.ty * ST_TH + 4 * warp < g.out_h; ++sg)   // (rows below the map: nothing to store)
                     tma_store_4d(ymap, smem_u32(sO) + sg * 128u * seg_bytes + (uint32_t)(warp * 32) * seg_bytes, (int)sg * seg_chan, at.tx * ST_TW, at.ty * ST_TH + 4 * warp, at.b);
@@ -327,11 +371,17 @@ bool conv_stem_tc_covers(const ConvGeom &g)
     return (narrow || wide) && g.groups == 1 && g.n % 16 == 0 && g.n <= 64 && g.stride >= 1 && g.stride <= 2;
 }
 
-template <int KS, int S, int ACT, bool OBF>
+// The maxpool after it in the same launch: 3x3 layers with stride 1 and padding 1, whole windows, pixels of at most 128 bytes, the leaky activation.
+bool conv_stem_pool_covers(const ConvGeom &g, int y_dtype, int activation)
+{
+    return conv_stem_tc_covers(g) && g.size == 3 && g.stride == 1 && g.pad == 1 && g.out_h % 2 == 0 && g.out_w % 2 == 0 && g.n * (y_dtype == DNB_BF16 ? 2 : 4) <= 128 && activation == DNB_LEAKY;
+}
+
+template <int KS, int S, int ACT, bool OBF, bool POOL = false>
 static int launch_stem(const StemTcArgs &a, cudaStream_t s)
 {
     using P = StemPatch<KS, S>;
-    auto kern = conv_stem_tc_kernel<KS, S, ACT, OBF>;
+    auto kern = conv_stem_tc_kernel<KS, S, ACT, OBF, POOL>;
     size_t smem = (size_t)a.segs * 128 * a.seg_bytes + (size_t)P::PAIRS * a.n_pad * 32 + 2 * sizeof(float4) * P::CELLS + 2 * sizeof(float) * a.n_pad + sizeof(StemShared) + 16;
     smem = tmem_smem(smem, a.tmem_cols);
     const size_t sm_bytes = 228 * 1024, reserved = 1024;   // per SM, and per resident CTA
@@ -351,6 +401,8 @@ static int launch_stem(const StemTcArgs &a, cudaStream_t s)
 template <int KS, int S, bool OBF>
 static int launch_act(const StemTcArgs &a, cudaStream_t s)
 {
+    if constexpr (KS == 3 && S == 1)
+        if (a.pool) return launch_stem<KS, S, DNB_LEAKY, OBF, true>(a, s);
     if (a.ep.activation == DNB_LEAKY) return launch_stem<KS, S, DNB_LEAKY, OBF>(a, s);
     if (a.ep.activation == DNB_LINEAR) return launch_stem<KS, S, DNB_LINEAR, OBF>(a, s);
     return launch_stem<KS, S, ST_ACT_GENERIC, OBF>(a, s);
@@ -381,9 +433,11 @@ int launch_conv_stem_tc(StemTcArgs a, cudaStream_t s)
     const int es = a.y_dtype == DNB_BF16 ? 2 : 4, rb = g.n * es;
     a.seg_bytes = rb > 64 ? 128 : (rb > 32 ? 64 : 32);
     a.segs = (rb + a.seg_bytes - 1) / a.seg_bytes;
-    const uint64_t dims[4] = {(uint64_t)g.n, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
-    const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)rb * g.out_w, (uint64_t)rb * g.out_w * g.out_h};
-    const uint32_t box[4] = {(uint32_t)(a.seg_bytes / es), (uint32_t)ST_TW, 4u, 1u};   // a warp's four pixel rows
+    if (a.pool && (!conv_stem_pool_covers(g, a.y_dtype, a.ep.activation) || a.segs != 1)) DNB_FAIL(DNB_EINVAL, "first-layer kernel: no pooled variant of this layer");
+    const int half = a.pool ? 2 : 1, yw = g.out_w / half, yh = g.out_h / half;
+    const uint64_t dims[4] = {(uint64_t)g.n, (uint64_t)yw, (uint64_t)yh, (uint64_t)g.batch};
+    const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)rb * yw, (uint64_t)rb * yw * yh};
+    const uint32_t box[4] = {(uint32_t)(a.seg_bytes / es), (uint32_t)ST_TW / half, 4u / half, 1u};   // a warp's four pixel rows
     DNB_TRY(encode_tensor_map(&a.tmy, es == 2 ? 1 : 0, 4, a.y, dims, strides, box, a.seg_bytes));
     if (g.size == 7) return launch_size<7>(a, s);
     if (g.size == 5) return launch_size<5>(a, s);

@@ -829,34 +829,22 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                 if (POOL) {
                     epilogue_bar();
                     // pooled pixel et / 4 (half the tile's extents), 16-byte pieces et % 4 and that + 4 of its row
-                    constexpr int VALUES = OUT_BF16 ? 8 : 4;
                     const int et = threadIdx.x - 64, pp = et >> 2, pw = wt >> 1, ph = ht >> 1;
                     const int top = ((pp / (pw * ph)) * ht + 2 * (pp / pw % ph)) * wt + 2 * (pp % pw);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int q = (et & 3) + 4 * h;
-                        uint32_t best[VALUES];
-#pragma unroll
-                        for (int e = 0; e < VALUES; ++e) best[e] = __float_as_uint(-FLT_MAX);
+                        uint4 v[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int rr = top + (i & 1) + (i >> 1) * wt;
-                            const uint4 v = *reinterpret_cast<const uint4 *>(stage_out + (size_t)rr * srb + ((q ^ (rr & 7)) << 4));
-                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                            for (int e = 0; e < VALUES; ++e) {
-                                const uint32_t bits = !OUT_BF16 ? w[e & 3] : (e & 1) ? (w[e / 2] & 0xffff0000u) : (w[e / 2] << 16);
-                                best[e] = __float_as_uint(fmaxf(__uint_as_float(best[e]), __uint_as_float(bits)));
-                            }
+                            v[i] = *reinterpret_cast<const uint4 *>(stage_out + (size_t)rr * srb + ((q ^ (rr & 7)) << 4));
                         }
-                        uint4 o;
-                        if constexpr (OUT_BF16) o = pack_bf16x8<VALUES>(best, 0);
-                        else o = make_uint4(best[0], best[1], best[2], best[3]);
+                        const uint4 o = largest_of_four<OUT_BF16>(v);
                         *reinterpret_cast<uint4 *>(pooled + pp * 128 + ((q ^ (pp & 7)) << 4)) = o;
                         if (SIGNS) {   // of the pooled values, 4 channels a word
-                            uint32_t wd = 0u;
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) wd |= (4 * q + e < nvalid ? (__uint_as_float(best[e]) > 0.f ? 0x01u : 0xFFu) : 0u) << (8 * e);
+                            const int left = nvalid - 4 * q;   // real filters among the four
+                            const uint32_t wd = four_signs(o) & (left >= 4 ? ~0u : left > 0 ? (1u << (8 * left)) - 1u : 0u);
                             *reinterpret_cast<uint32_t *>(pooled + 4096 + pp * 32 + (((q >> 2) ^ ((pp >> 2) & 1)) << 4) + 4 * (q & 3)) = wd;
                         }
                     }

@@ -70,4 +70,32 @@ template <typename T> __device__ __forceinline__ T from_float(float v);
 template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
+// Four 16-byte pieces (floats, or bf16 values) of a 2x2 maxpool's window: its largest values, as forward_maxpool_layer finds them, from the
+// lowest float up (src/maxpool_layer.c:88-107), so that a NaN never wins.
+template <bool BF16>
+__device__ __forceinline__ uint4 largest_of_four(const uint4 (&v)[4])
+{
+    uint32_t out[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        float a = -FLT_MAX, b = -FLT_MAX;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t w = e == 0 ? v[i].x : e == 1 ? v[i].y : e == 2 ? v[i].z : v[i].w;
+            if (!BF16) a = fmaxf(a, __uint_as_float(w));
+            else { a = fmaxf(a, __uint_as_float(w << 16)); b = fmaxf(b, __uint_as_float(w & 0xffff0000u)); }
+        }
+        if (!BF16) out[e] = __float_as_uint(a);
+        else { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); out[e] = *reinterpret_cast<const uint32_t *>(&h); }
+    }
+    return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+// Signs of four floats as bytes: +1 where > 0, else -1.
+__device__ __forceinline__ uint32_t four_signs(uint4 v)
+{
+    return (__uint_as_float(v.x) > 0.f ? 0x01u : 0xFFu) | (__uint_as_float(v.y) > 0.f ? 0x01u : 0xFFu) << 8 | (__uint_as_float(v.z) > 0.f ? 0x01u : 0xFFu) << 16 |
+           (__uint_as_float(v.w) > 0.f ? 0x01u : 0xFFu) << 24;
+}
+
 }  // namespace dnb

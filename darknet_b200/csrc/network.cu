@@ -177,6 +177,7 @@ struct dnb_network {
     cudaGraphExec_t step_exec[2] = {nullptr, nullptr};
     int step_runs[2] = {0, 0};
     bool step_graphs = true;              // off once something could not be captured
+    const float *images = nullptr;        // the network's own buffer with the images of the last pass, where a first layer's own output is made on request
     std::vector<Item> schedule;           // a step, where its batch is enqueued in parts (see plan_step); else empty
     cudaEvent_t piece_in[MAX_PIECES] = {};   // upload stream: a piece's images are on the device
     std::vector<cudaGraphExec_t> item_exec[2];   // the schedule's items as graphs, per slot
@@ -404,7 +405,7 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
     // each four pixels, and the pass that read the whole map back disappears.  The convolution's own output is made from its input for
     // who asks for it (own_output).  DNB_FUSE_POOL=0 keeps the two layers separate.
     const bool fuse_pool = getenv("DNB_FUSE_POOL") ? atoi(getenv("DNB_FUSE_POOL")) != 0 : true;
-    for (int i = 1; fuse_pool && i + 1 < (int)net->layers.size(); ++i) {
+    for (int i = 0; fuse_pool && i + 1 < (int)net->layers.size(); ++i) {
         Layer &C = net->layers[i], &M = net->layers[i + 1];
         if (C.kind != L_CONV || !C.plan || M.kind != L_MAXPOOL || M.size != 2 || M.stride != 2 || M.padding < 0 || M.padding > 1 || !C.out.data) continue;
         if (M.out_h != C.out_h / 2 || M.out_w != C.out_w / 2) continue;
@@ -414,10 +415,11 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
             if (L.kind == L_SHORTCUT && L.from == i) read_elsewhere = true;
             if (L.kind == L_ROUTE)
                 for (int id : L.inputs) if (id == i) read_elsewhere = true;
-            // the maxpool kernel also writes the next xnor layer's operand; of the convolutions only an xnor layer does
-            if (j == i + 2 && L.kind == L_CONV && L.cd.xnor && !C.cd.xnor) sign_pass = true;
+            // the maxpool kernel also writes the next xnor layer's operand; of the convolutions only an xnor layer or a first one does
+            if (j == i + 2 && L.kind == L_CONV && L.cd.xnor && !C.cd.xnor && !C.plan->stem_tc) sign_pass = true;
         }
-        if (read_elsewhere || sign_pass || !conv_pool_fusable(C.plan)) continue;
+        if (read_elsewhere || sign_pass || !conv_pool_fusable(C.plan, any_xnor)) continue;
+        if (i == 0 && net->mode == DNB_MODE_BF16 && C.out.dtype != DNB_BF16) continue;
         C.fuses_next_pool = true;
         M.fused_into_prev = true;
         M.launches = 0;
@@ -739,7 +741,9 @@ static int own_output(dnb_network *net, int i, dnb_tensor *t, cudaStream_t s)
     if (L.out.data) return DNB_OK;
     if (!L.own_out.data)
         DNB_FAIL(DNB_EUNSUPPORTED, "layer %d is fused into layer %d and has no output of its own (DNB_FUSE_SHORTCUT=0 / DNB_FUSE_YOLO=0 keep it)", i, i + 1);
-    const dnb_tensor in = i > 0 ? net->layers[i - 1].out : net->input_nhwc;
+    if (i == 0 && !net->input_nhwc.data && !net->images) DNB_FAIL(DNB_EINVAL, "layer 0: no step has run");
+    const dnb_tensor in = i > 0 ? net->layers[i - 1].out : net->input_nhwc.data ? net->input_nhwc
+                          : dnb_tensor{(void *)net->images, DNB_NCHW, DNB_F32, net->batch, net->c, net->h, net->w, 0};
     *t = L.own_out;
     return dnb_conv_forward(L.plan, &in, t, nullptr, s);
 }
@@ -821,8 +825,17 @@ static int forward_layer(dnb_network *net, int i, const float *device_input, con
             return conv_shortcut_general(plan_of(L, p), &in, &add, &sum, S.alpha, S.beta, S.activation, s);
         }
         if (L.fuses_next_pool) {
+            // The first layer's own output is made from the images, if it is asked for: those of a caller may be gone by then, so they are copied.
+            // conv_stem_rows.cu does it on the way (Darknet-19-xnor, 128 images: 1057 us a step, 1073 with a copy before it), the other kernel for
+            // few images, for which a copy is mostly a launch (YOLOv3-tiny, one: 131 and 134; 16: 439 and 432).
+            float *keep = nullptr;
+            if (i == 0 && device_input != net->input_slot[0] && device_input != net->input_slot[1]) {
+                const size_t bytes = (size_t)net->batch * net->inputs * sizeof(float);
+                if (L.plan->keep_k_order || bytes <= (size_t)8 << 20) keep = net->input_dev;
+                else DNB_CUDA(cudaMemcpyAsync(net->input_dev, device_input, bytes, cudaMemcpyDeviceToDevice, s));
+            }
             const dnb_tensor pooled = part_of(net->layers[i + 1].out, p);
-            return conv_pool_forward(plan_of(L, p), &in, &pooled, s);
+            return conv_pool_forward(plan_of(L, p), &in, &pooled, keep, s);
         }
         if (L.fuses_next_yolo) {
             Layer &Y = net->layers[i + 1];
@@ -912,6 +925,7 @@ extern "C" int dnb_network_forward(dnb_network *net, const float *device_input, 
     if (net->submitted != net->collected) DNB_FAIL(DNB_EINVAL, "network_forward: a submitted step is still in flight (the layers' outputs are shared); collect it first");
     DNB_TRY(check_current_device(net->device, "network_forward"));
     point_status(net, 0);
+    net->images = net->input_dev;
     cudaStream_t s = (cudaStream_t)stream;  // NULL is the legacy default stream, as everywhere in CUDA
     if (!net->graph_enabled || !s) return forward_eager(net, device_input, s);   // the legacy stream cannot be captured
 
@@ -1220,6 +1234,7 @@ extern "C" int dnb_network_collect(dnb_network *net, float **output)
     if (net->submitted == net->collected) DNB_FAIL(DNB_EINVAL, "network_collect: nothing has been submitted");
     const int slot = (int)(net->collected & 1);
     ++net->collected;
+    net->images = net->input_slot[slot];
     DNB_CUDA(cudaEventSynchronize(net->copy_done[slot]));   // follows fwd_done[slot] and every copy of the step
     for (Layer &L : net->layers) if (L.kind == L_YOLO) L.host_out = L.host_slot[slot];
     if (net->status_host[slot]) {
@@ -1412,6 +1427,7 @@ extern "C" int dnb_network_forward_timed(dnb_network *net, const float *device_i
     if (net->submitted != net->collected) DNB_FAIL(DNB_EINVAL, "network_forward_timed: a submitted step is still in flight; collect it first");
     DNB_TRY(check_current_device(net->device, "network_forward_timed"));
     point_status(net, 0);
+    net->images = net->input_dev;
     const int n = (int)net->layers.size();
     while ((int)net->events.size() < (slot + 1) * (n + 1)) {
         cudaEvent_t e;

@@ -377,29 +377,44 @@ def test_two_epilogue_groups(name, mode, monkeypatch):
 
 @pytest.mark.parametrize("mode,xnor,batch,size", [
     (dn.MODE_TF32, False, 3, 60), (dn.MODE_TF32, False, 64, 22), (dn.MODE_BF16, False, 5, 68), (dn.MODE_TF32, True, 4, 60), (dn.MODE_TF32, True, 40, 28)])
-def test_maxpool_in_the_convolutions_epilogue(mode, xnor, batch, size, tmp_path, monkeypatch):
+@pytest.mark.parametrize("first_filters", [16, 32])
+def test_maxpool_in_the_convolutions_epilogue(mode, xnor, batch, size, first_filters, tmp_path, monkeypatch):
     """Convolutions with the 2x2 maxpool after them in one launch against two launches, to the bit: maps that end inside a tile, filters
     beyond a staged chunk, signs for an xnor layer, filters whose every value is an infinity or NaN, the convolutions' own outputs."""
     import numpy as np
     from darknet_b200 import synth
     pool = "\n[maxpool]\nsize=2\nstride=2\n"
-    cfg = (synth._net(batch, 4 * size, 4 * size) + synth._conv(32, 3, stride=2) + synth._conv(72, 3, xnor=xnor) + pool + synth._conv(96, 3, xnor=xnor) + pool +
+    cfg = (synth._net(batch, 4 * size, 4 * size) + synth._conv(first_filters, 3) + pool + synth._conv(72, 3, xnor=xnor) + pool + synth._conv(96, 3, xnor=xnor) + pool +
            synth._conv(128, 1, xnor=xnor) + synth._conv(160, 3, xnor=xnor) + "\n[avgpool]\n")
     params = synth.seeded_params(cfg, 8)
+    params[0].biases[3] = -np.inf
     for f, v in ((0, np.inf), (1, -np.inf), (2, np.nan)):
         params[1].biases[f] = v
-    if xnor:      # keep what follows finite: an infinity's sign is a sign, NaN's is -1
-        params[1].biases[2] = 0
     path = str(tmp_path / "m.weights")
     synth.write_weights(path, params)
-    x = synth.seeded_input(cfg, 9, "normal")
+    import torch
+    x, y = synth.seeded_input(cfg, 9, "normal"), synth.seeded_input(cfg, 10, "normal")
+    stream, dev = torch.cuda.Stream(), None
     out = []
     for fuse in ("0", "1"):
         monkeypatch.setenv("DNB_FUSE_POOL", fuse)
         net = dn.Network(cfg, path, mode, text=True)
         launches = net.launches
         net.predict(x)
-        out.append([net.layer_output(i) for i in (2, 4, 1, 3, 5, 6)] + [net.predict(x).copy(), net.layer_output_images(1, batch - 1), launches])
+        got = [net.layer_output(i) for i in (1, 3, 5, 0, 2, 4, 6, 7)] + [net.predict(x).copy(), net.layer_output_images(2, batch - 1)]
+        for graph in (False, True, True, True):      # the device's images are overwritten before the first layer's own output is asked for
+            net.enable_graph(graph)
+            dev = torch.from_numpy(x).cuda() if not graph else dev
+            dev.copy_(torch.from_numpy(x))
+            stream.wait_stream(torch.cuda.current_stream())
+            net.forward(dev, stream=stream.cuda_stream)
+            stream.synchronize()
+            dev.zero_()
+            got += [net.layer_output(i) for i in (0, 2, 7)]
+        net.submit(x), net.submit(y)
+        net.collect(), net.collect()
+        got += [net.layer_output(i) for i in (0, 1, 7)]
+        out.append(got + [launches])
         net.close()
     assert out[1][-1] < out[0][-1]
     for a, b in zip(*[o[:-1] for o in out]):
