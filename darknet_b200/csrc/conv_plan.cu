@@ -663,22 +663,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
 {
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
     pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt, pool);
-    // Halo mode (experimental, off unless DNB_TC_HALO is 1 or 2): one activation box per channel block serves all
-    // nine taps of a 3x3 stride-1 layer, which cuts the bytes that cross L2 -> shared memory by 2.3x on the
-    // 32- and 64-channel layers of large maps.  Measured on YOLOv3-608 batch 64 it does not pay yet: the 8 x 16
-    // tile, the two rings it needs and the smaller share of shared memory left for each slow the 304x304 and
-    // 152x152 layers by 25-35 % (an isolated 32 -> 64 layer without a residual gains 11 %).  1: where the
-    // heuristic below allows; 2: wherever the geometry allows (the tests use this).
     a.halo = 0;
-    {
-        const char *e = getenv("DNB_TC_HALO");
-        const int knob = e ? atoi(e) : 0;
-        if (knob != 0 && !i8 && !pool && g.size == 3 && g.stride == 1 && g.pad == 1 && a.row_bytes == 128 && g.out_w >= 8 && g.out_h >= 16) {
-            const double work_h = (double)round_up(g.out_w, 8) * round_up(g.out_h, 16) * g.batch;
-            const double work_0 = (double)round_up(g.out_w, a.wt) * round_up(g.out_h, a.ht) * round_up(g.batch, a.bt);
-            if (knob == 2 || (a.c_blocks <= 2 && work_h <= 1.08 * work_0)) { a.halo = 1; a.wt = 8; a.ht = 16; a.bt = 1; }
-        }
-    }
     a.tiles_w = (g.out_w + a.wt - 1) / a.wt;
     a.tiles_h = (g.out_h + a.ht - 1) / a.ht;
     a.tiles_b = (g.batch + a.bt - 1) / a.bt;
@@ -819,31 +804,45 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
     int stages = 0;
     const bool allow2 = getenv("DNB_TC_CTAS") ? atoi(getenv("DNB_TC_CTAS")) >= 2 : true;
-    a.a_stages = a.b_stages = a.a_slot = a.a_box_bytes = a.a_pitch = 0;
+    a.a_slot = a.a_box_slot = a.a_box_bytes = a.a_pitch = 0;
     a.epi_groups = 1;
-    if (a.halo) {
-        // two rings: activation boxes (one per channel block) and weight tiles (nine per box).  A weight tile is
-        // consumed in a quarter of the time an ordinary ring slot is, so that ring wants to be deep: one CTA per
-        // SM unless two still leave six weight slots each.
-        a.a_pitch = a.wt + 2;
-        a.a_box_bytes = (a.wt + 2) * (a.ht + 2) * a.row_bytes;
-        a.a_slot = round_up(a.a_box_bytes, 1024);
-        auto fit = [&](long budget, int srb_try, int a_want, int b_min) {
-            const long left = budget - (long)conv_tc_fixed_smem(srb_try, a.bn, a.stage_bufs) - (long)a_want * a.a_slot;
-            const int b = left > 0 ? (int)(left / a.b_bytes) : 0;
-            if (b < b_min) return false;
-            a.a_stages = a_want; a.b_stages = b > 12 ? 12 : b; srb = srb_try;
+    a.halo = 0;
+    // Halo mode, where two CTAs with the layer's weights fit an SM: what a layer over few channels waits for is the rows its copies are made of,
+    // 128 pixels and the filters for every tap, and with the weights in place and one box for all taps they are a tenth.  3x3 32 -> 64 at
+    // 64 x 304 x 304 in bf16 with a residual 926 -> 487 us, of xnor layers with the maxpool at 128 x 112 x 112 226 -> 138, 16 -> 32 in TF32 at
+    // 16 x 208 x 208 72 -> 49.  One CTA alone with its weights is slower than two without (32 -> 64 in TF32 854 -> 900, 64 -> 128 in bf16 at 152 x
+    // 152 280 -> 390, of xnor layers at 56 x 56 79 -> 95, 32 -> 64 with stride 2 in bf16 685 -> 790).  Same order of the sums.
+    // DNB_TC_HALO: 0 never, 2 wherever the geometry and shared memory allow.
+    const int halo_knob = getenv("DNB_TC_HALO") ? atoi(getenv("DNB_TC_HALO")) : 1;
+    if (halo_knob != 0 && g.size == 3 && g.pad == 1 && a.n_tiles == 1 && !a.pair && g.out_w >= 8 && g.out_h >= 16) {
+        const int lattices = g.stride * g.stride, htiles = ((g.out_w + 7) / 8) * ((g.out_h + 15) / 16) * g.batch;
+        a.a_pitch = g.stride == 1 ? 10 : 9;
+        a.a_box_bytes = a.a_pitch * (g.stride == 1 ? 18 : 17) * a.row_bytes;
+        a.a_box_slot = round_up(a.a_box_bytes, 1024);
+        a.a_slot = lattices * a.c_blocks * a.a_box_slot;
+        const long weights = (long)a.taps * a.c_blocks * a.b_bytes;
+        auto fit = [&](long budget, int srb_try, int most) {
+            const long left = budget - weights - (long)conv_tc_fixed_smem(srb_try, a.bn, a.stage_bufs);
+            const int n = left > 0 ? (int)(left / a.a_slot) : 0;
+            if (n < 2) return false;
+            stages = n > most ? most : n; srb = srb_try;
             return true;
         };
         bool done = false;
-        if (allow2 && a.tmem_cols <= 256) {
-            const long budget = (228L * 1024) / 2 - 2048;
-            for (int srb2 = srb; srb2 >= min_srb && !done; srb2 /= 2) done = fit(budget, srb2, 2, 6);
-            if (done) a.ctas_per_sm = 2;
+        if (halo_knob == 2 || (htiles >= 2 * sm_count() && htiles <= 1.2 * a.total_tiles)) {
+            const int widest = srb;
+            if (allow2 && a.tmem_cols <= 256 && htiles > sm_count())
+                for (int t = widest; t >= min_srb && !done; t /= 2) { done = fit((228L * 1024) / 2 - 2048, t, 4); if (done) a.ctas_per_sm = 2; }
+            for (int t = widest; halo_knob == 2 && t >= min_srb && !done; t /= 2) done = fit(max_smem, t, 4);
+            if (!done) srb = widest;
         }
-        for (int srb2 = srb; srb2 >= min_srb && !done; srb2 /= 2) done = fit(max_smem, srb2, 3, 6) || fit(max_smem, srb2, 2, 4);
-        if (!done) a.halo = 0;   // the tile shape stays 8 x 16: still a valid tiling for the ordinary rings below
-        stages = 2;
+        if (done) {
+            a.halo = 1;
+            a.wt = 8; a.ht = 16; a.bt = 1;
+            a.tiles_w = (g.out_w + 7) / 8; a.tiles_h = (g.out_h + 15) / 16; a.tiles_b = g.batch;
+            a.total_tiles = htiles;
+            if (a.ctas_per_sm == 1 && srb == 128 && !residual && !pool && (y_nhwc || sign_out) && !nchw_out) a.epi_groups = 2;
+        }
     }
     if (!a.halo) {
         // (not when every tile has an SM of its own: one deep ring then)
@@ -950,7 +949,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     DNB_TRY(ensure_status(p));
     a.status = p->status;
     {
-        const uint32_t box[4] = {(uint32_t)a.bk, (uint32_t)(a.halo ? a.wt + 2 : a.wt), (uint32_t)(a.halo ? a.ht + 2 : a.ht), (uint32_t)a.bt};
+        const uint32_t box[4] = {(uint32_t)a.bk, (uint32_t)(a.halo ? a.a_pitch : a.wt), (uint32_t)(a.halo ? a.a_box_bytes / (a.a_pitch * a.row_bytes) : a.ht), (uint32_t)a.bt};
         DNB_TRY(encode_input_maps(a.tmx, g, x, kind, es, c_pad, box, a.row_bytes));
         DNB_TRY(encode_weight_map(&a.tmw, p, kind, es, c_pad, a.taps, a.bk, a.pair ? a.bn / 2 : a.bn, a.row_bytes));
     }
@@ -1334,7 +1333,7 @@ bool conv_pool_fusable(dnb_conv_plan *p, bool in_order)
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
     pick_persistent_tiles(p, g, a, false, true, g.n, false);
     const int k_iters = g.size * g.size * a.c_blocks;
-    if (a.pair || a.halo || a.total_tiles < (k_iters <= 12 ? sm_count() / 2 : sm_count())) return false;
+    if (a.pair || a.total_tiles < (k_iters <= 12 ? sm_count() / 2 : sm_count())) return false;
     p->pool_fits = 1;
     return true;
 }

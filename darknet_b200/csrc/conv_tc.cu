@@ -48,15 +48,13 @@
 namespace dnb {
 
 constexpr int MAX_STAGES = 8;
-constexpr int MAX_B_STAGES = 12;   // weight-tile ring of the halo mode
 constexpr int MAX_RES_BUFS = 4;   // staging buffers with a fused residual; tiles are requested two chunks ahead
 
 // ------------------------------------------------------------------ kernel
 struct TcShared {
-    uint64_t full[MAX_STAGES];     // operand ring (halo mode: the ring of activation boxes)
+    uint64_t full[MAX_STAGES];     // operand ring (halo mode: the ring of tiles' activation boxes)
     uint64_t empty[MAX_STAGES];
-    uint64_t full_b[MAX_B_STAGES]; // halo mode: the ring of weight tiles
-    uint64_t empty_b[MAX_B_STAGES];
+    uint64_t weights;              // halo mode: the layer's weights have landed
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
     uint64_t res_full[MAX_RES_BUFS];   // residual tile landed in its staging buffer
@@ -164,7 +162,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         return;
     }
     const uint32_t stage_bytes = a.a_bytes + a.b_bytes;
-    const size_t ring_bytes = a.halo ? (size_t)a.a_stages * a.a_slot + (size_t)a.b_stages * a.b_bytes : (size_t)a.stages * stage_bytes;
+    const size_t ring_bytes = a.halo ? (size_t)a.stages * a.a_slot + (size_t)a.taps * a.c_blocks * a.b_bytes : (size_t)a.stages * stage_bytes;
     uint8_t *after_ring = smem_raw + (ring - smem_u32(smem_raw)) + ring_bytes;
     // staging buffers of 128 rows x store_row_bytes: two for plain stores; four when a residual is fused, each
     // then receiving a residual tile first and the finished output rows, in place, afterwards
@@ -183,10 +181,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             mbar_init(smem_u32(&sh->full[s]), 1);
             mbar_init(smem_u32(&sh->empty[s]), 1);
         }
-        for (int s = 0; s < MAX_B_STAGES; ++s) {
-            mbar_init(smem_u32(&sh->full_b[s]), 1);
-            mbar_init(smem_u32(&sh->empty_b[s]), 1);
-        }
+        mbar_init(smem_u32(&sh->weights), 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&sh->acc_full[i]), 1);
             mbar_init(smem_u32(&sh->acc_empty[i]), (PAIR ? 8 : 4) * EG);   // the epilogue warps of both CTAs of a pair
@@ -232,8 +227,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
     const long long wait_limit = a.wait_limit;
 
     if (warp == 0) {
-        // ---------------- TMA producer: the whole warp runs the loop and an elected lane issues the loads (halo mode: one
-        // lane runs it, the others wait at the __syncwarp)
+        // ---------------- TMA producer: the whole warp runs the loop and an elected lane issues the loads 
         const int ksize = a.g.size, cstride = a.g.stride, cpad = a.g.pad;
         const uint32_t tx_bytes = 128u * row_bytes + (uint32_t)(PAIR ? bn >> 1 : bn) * row_bytes;
         const CUtensorMap *maps = a.tmx;
@@ -245,32 +239,33 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         uint32_t phase = 0;
         bool ok = true;
         if (a.halo) {
-            grid_dependency_wait();
-            // one activation box per channel block, then the nine weight tiles that multiply it
-            const int a_stages = a.a_stages, b_stages = a.b_stages;
-            const uint32_t a_slot = a.a_slot, a_tx = a.a_box_bytes, b_slot = a.b_bytes, b_tx = (uint32_t)bn * row_bytes;
-            const uint32_t ring_b = ring + a_stages * a_slot;
-            const uint32_t fullb0 = smem_u32(&sh->full_b[0]), emptyb0 = smem_u32(&sh->empty_b[0]);
-            int sb = 0;
-            uint32_t phase_b = 0;
-            for (int tile = blockIdx.x; lane == 0 && tile < total_tiles && ok; tile += grid_stride) {
-                const int nt = tile % n_tiles, pt = tile / n_tiles;
-                const int ow0 = (pt % tiles_w) * wt, oh0 = ((pt / tiles_w) % tiles_h) * ht, b0 = (pt / ptiles_wh) * bt;
-                const int n0 = nt * bn;
-                for (int cb = 0; cb < c_blocks && ok; ++cb) {
-                    ok = mbar_wait_thread(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
-                    if (!ok) break;
-                    mbar_expect_tx(full0 + 8 * stage, a_tx);
-                    tma_load_4d(ring + stage * a_slot, maps, full0 + 8 * stage, cb * bk, ow0 - cpad, oh0 - cpad, b0);
-                    if (++stage == a_stages) { stage = 0; phase ^= 1; }
-                    for (int tap = 0; tap < taps; ++tap) {
-                        ok = mbar_wait_thread(emptyb0 + 8 * sb, phase_b ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
-                        if (!ok) break;
-                        mbar_expect_tx(fullb0 + 8 * sb, b_tx);
-                        tma_load_3d(ring_b + sb * b_slot, wmap, fullb0 + 8 * sb, cb * bk, n0, tap);
-                        if (++sb == b_stages) { sb = 0; phase_b ^= 1; }
-                    }
+            // the layer's weights once, then per tile one box of each lattice and channel block
+            const uint32_t weights = ring + stages * a.a_slot, wbar = smem_u32(&sh->weights), b_bytes = a.b_bytes;
+            if (first_tile < total_tiles && elect_one()) {
+                mbar_expect_tx(wbar, (uint32_t)(k_iters * bn * row_bytes));
+                for (int i = 0, tap = 0, cb = 0; i < k_iters; ++i) {
+                    tma_load_3d(weights + i * b_bytes, wmap, wbar, cb * bk, 0, tap);
+                    if (++cb == c_blocks) { cb = 0; ++tap; }
                 }
+            }
+            __syncwarp();
+            grid_dependency_wait();
+            const uint32_t a_slot = a.a_slot, box_slot = a.a_box_slot, tx = (uint32_t)(cstride * cstride * c_blocks) * (uint32_t)a.a_box_bytes;
+            for (int tile = first_tile; tile < total_tiles && ok; tile += grid_stride) {
+                const int ow0 = (tile % tiles_w) * wt, oh0 = ((tile / tiles_w) % tiles_h) * ht, b0 = (tile / ptiles_wh) * bt;
+                ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, WAIT_EMPTY, wait_limit);
+                if (!ok) break;
+                if (withhold && tile == first_tile) { ok = false; break; }
+                if (elect_one()) {
+                    const uint32_t bar = full0 + 8 * stage;
+                    uint32_t dst = ring + stage * a_slot;
+                    mbar_expect_tx(bar, tx);
+                    // both strides: the lattice's row of the first tap is one above the tile's first
+                    for (int l = 0; l < cstride * cstride; ++l)
+                        for (int cb = 0; cb < c_blocks; ++cb, dst += box_slot) tma_load_4d(dst, maps + l, bar, cb * bk, ow0 - 1, oh0 - 1, b0);
+                }
+                __syncwarp();
+                if (++stage == stages) { stage = 0; phase ^= 1; }
             }
         } else {
         int ahead = first_tile < total_tiles ? min(stages, k_iters) : 0;   // slots whose weights are requested before the wait
@@ -338,8 +333,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ---------------- MMA issuer: the whole warp runs the loop and an elected lane issues (halo mode: one lane runs
-        // it).  Its instruction stream per ring slot has to stay well below the 4 x 128 cycles the tensor pipe needs for the slot's MMAs, so everything is in registers:
+        // ---------------- MMA issuer: the whole warp runs the loop and an elected lane issues.  Its instruction stream per ring slot has to stay well below the 4 x 128 cycles the tensor pipe needs for the slot's MMAs, so everything is in registers:
         // barrier addresses and operand descriptors advance by constants, the accumulator-ready commit
         // sits after the k loop.
         constexpr int is_bf16 = I8 ? MMA_I8 : (OUT_BF16 ? MMA_BF16 : MMA_TF32);   // operand kind of the MMAs
@@ -357,49 +351,42 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         int it = 0;
         bool ok = true;
         if (a.halo) {
-            const int a_stages = a.a_stages, b_stages = a.b_stages, pitch = a.a_pitch, ksize = a.g.size;
-            const uint32_t fullb0 = smem_u32(&sh->full_b[0]), emptyb0 = smem_u32(&sh->empty_b[0]);
-            // A descriptor of a box: rows of 128 bytes, 8-row groups one box row (pitch pixels) apart
-            uint64_t dbox0 = make_smem_desc(ring, 128);
-            dbox0 = (dbox0 & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(pitch * 8) << 32);
-            const uint64_t dw0 = make_smem_desc(ring + a_stages * a.a_slot, 128);
-            const uint64_t a_step = (uint64_t)(a.a_slot >> 4), b_step = (uint64_t)(a.b_bytes >> 4);
-            int sb = 0;
-            uint32_t phase_b = 0;
-            for (int tile = blockIdx.x; lane == 0 && tile < total_tiles && ok; tile += grid_stride, ++it) {
+            // A descriptor of a tap: rows of row_bytes from the box's row of the tap on, 8-row groups one box row (pitch pixels) apart
+            const int pitch = a.a_pitch, ksize = a.g.size, cstride = a.g.stride;
+            const uint64_t row16 = (uint64_t)(row_bytes >> 4), box16 = (uint64_t)(a.a_box_slot >> 4), slot16 = (uint64_t)(a.a_slot >> 4), b16 = (uint64_t)(a.b_bytes >> 4);
+            uint64_t dbox0 = make_smem_desc(ring, row_bytes);
+            dbox0 = (dbox0 & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(pitch * row16) << 32);
+            const uint64_t dw0 = make_smem_desc(ring + stages * a.a_slot, row_bytes);
+            if (first_tile < total_tiles) ok = mbar_wait_warp(smem_u32(&sh->weights), 0, abort_flag, status, WAIT_FULL, wait_limit);
+            for (int tile = first_tile; tile < total_tiles && ok; tile += grid_stride, ++it) {
                 const int acc = it & 1;
-                const uint32_t acc_phase = (it >> 1) & 1;
-                ok = mbar_wait_thread(smem_u32(&sh->acc_empty[acc]), acc_phase ^ 1, abort_flag, status, WAIT_ACC_EMPTY, wait_limit);
+                ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), ((it >> 1) & 1) ^ 1, abort_flag, status, WAIT_ACC_EMPTY, wait_limit) &&
+                     mbar_wait_warp(full0 + 8 * stage, phase, abort_flag, status, WAIT_FULL, wait_limit);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * acc_stride;
+                const uint64_t dslot = dbox0 + stage * slot16;
+                uint64_t dw = dw0;
                 uint32_t accumulate = 0u;
-                for (int cb = 0; cb < c_blocks && ok; ++cb) {
-                    ok = mbar_wait_thread(full0 + 8 * stage, phase, abort_flag, status, WAIT_FULL, wait_limit);
-                    if (!ok) break;
-                    const uint64_t dbox = dbox0 + stage * a_step;
-                    int kh = 0, kw = 0;
-                    for (int tap = 0; tap < taps; ++tap) {
-                        ok = mbar_wait_thread(fullb0 + 8 * sb, phase_b, abort_flag, status, WAIT_FULL, wait_limit);
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint64_t da = dbox + (uint64_t)((kh * pitch + kw) * 8);   // 128-byte rows in 16-byte units
-                        const uint64_t db = dw0 + sb * b_step;
-                        if (!(dbg_mma & 16)) {
-                            umma<is_bf16>(d_tmem, da, db, idesc, accumulate);
-                            umma<is_bf16>(d_tmem, da + 2, db + 2, idesc, 1u);
-                            umma<is_bf16>(d_tmem, da + 4, db + 4, idesc, 1u);
-                            umma<is_bf16>(d_tmem, da + 6, db + 6, idesc, 1u);
+                for (int kh = 0; kh < ksize; ++kh)
+                    for (int kw = 0; kw < ksize; ++kw) {
+                        // stride 2: taps 0 and 2 read the odd lattice, a row (column) apart, tap 1 the even one
+                        int l = 0, dy = kh, dx = kw;
+                        if (cstride == 2) { l = (kh != 1 ? 2 : 0) + (kw != 1 ? 1 : 0); dy = kh == 0 ? 0 : 1; dx = kw == 0 ? 0 : 1; }
+                        uint64_t da = dslot + (uint64_t)(l * c_blocks) * box16 + (uint64_t)(dy * pitch + dx) * row16;
+                        for (int cb = 0; cb < c_blocks; ++cb, da += box16, dw += b16) {
+                            if (elect_one() && !(dbg_mma & 16)) {
+                                umma<is_bf16>(d_tmem, da, dw, idesc, accumulate);
+                                for (int k = 1; k < k_steps; ++k) umma<is_bf16>(d_tmem, da + 2 * k, dw + 2 * k, idesc, 1u);
+                            }
+                            accumulate = 1u;
                         }
-                        accumulate = 1u;
-                        umma_commit(emptyb0 + 8 * sb);   // the weight tile is free when these MMAs retire
-                        if (++sb == b_stages) { sb = 0; phase_b ^= 1; }
-                        if (++kw == ksize) { kw = 0; ++kh; }
                     }
-                    if (ok) umma_commit(empty0 + 8 * stage);   // and the box when all nine taps have read it
-                    if (++stage == a_stages) { stage = 0; phase ^= 1; }
+                if (elect_one()) {
+                    umma_commit(empty0 + 8 * stage);
+                    umma_commit(smem_u32(&sh->acc_full[acc]));
                 }
-                if (ok) umma_commit(smem_u32(&sh->acc_full[acc]));
+                if (++stage == stages) { stage = 0; phase ^= 1; }
             }
         } else
         if (leader)
@@ -949,7 +936,7 @@ size_t conv_tc_fixed_smem(int store_row_bytes, int bn, int stage_bufs)
 
 size_t conv_tc_smem_bytes(const TcArgs &a)
 {
-    if (a.halo) return (size_t)a.a_stages * a.a_slot + (size_t)a.b_stages * a.b_bytes + conv_tc_fixed_smem(a.store_row_bytes, a.bn, a.stage_bufs);
+    if (a.halo) return (size_t)a.stages * a.a_slot + (size_t)a.taps * a.c_blocks * a.b_bytes + conv_tc_fixed_smem(a.store_row_bytes, a.bn, a.stage_bufs);
     return (size_t)a.stages * (a.a_bytes + a.b_bytes) + conv_tc_fixed_smem(a.store_row_bytes, a.bn, a.stage_bufs);
 }
 

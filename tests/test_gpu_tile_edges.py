@@ -419,3 +419,32 @@ def test_maxpool_in_the_convolutions_epilogue(mode, xnor, batch, size, first_fil
     assert out[1][-1] < out[0][-1]
     for a, b in zip(*[o[:-1] for o in out]):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+HALO = {   # one box for the nine taps, weights in shared memory: row widths, strides, channel blocks, ragged maps
+    "tf32_64_byte_rows": (dict(b=3, c=16, h=37, w=27, n=32, size=3), dn.MODE_TF32, False),
+    "tf32_two_blocks": (dict(b=2, c=40, h=33, w=18, n=48, size=3, act="linear"), dn.MODE_TF32, False),
+    "tf32_stride2": (dict(b=2, c=24, h=63, w=37, n=32, size=3, stride=2), dn.MODE_TF32, False),
+    "bf16_64_byte_rows": (dict(b=3, c=32, h=35, w=29, n=64, size=3), dn.MODE_BF16, False),
+    "bf16_stride2_even_map": (dict(b=2, c=32, h=64, w=48, n=64, size=3, stride=2), dn.MODE_BF16, False),
+    "int8_32_byte_rows": (dict(b=3, c=32, h=36, w=28, n=64, size=3), dn.MODE_TF32, True),
+    "int8_64_byte_rows_stride2": (dict(b=2, c=64, h=41, w=33, n=80, size=3, stride=2), dn.MODE_TF32, True),
+}
+
+
+@pytest.mark.parametrize("name", list(HALO))
+def test_one_box_for_nine_taps(name, monkeypatch):
+    """Equal to the ordinary rings to the bit: the same products in the same order, in either layout."""
+    import numpy as np
+    shape, mode, xnor = HALO[name]
+    case = conv_case(740, **shape)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    out = {}
+    for knob in ("0", "2"):
+        monkeypatch.setenv("DNB_TC_HALO", knob)
+        plan, a, b = run_conv(case, mode, "nhwc", "nchw", xnor=xnor, both=True)
+        assert ("halo=1" in plan.describe()) == (knob == "2"), plan.describe()
+        _, c, _ = run_conv(case, mode, "nhwc", "nhwc", xnor=xnor)
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+        out[knob] = a
+    assert np.array_equal(out["0"], out["2"])
