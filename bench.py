@@ -355,13 +355,15 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
     # HBM: algorithmic bytes = input + output of the layer in its storage type, the weights once, and the residual
     # a fused [shortcut] reads, over the same event durations
     es = 2.0 if mode == "bf16" else 4.0
+    # a convolution that also does the 2x2 maxpool after it writes a quarter of its map
+    written = [0.25 if i + 1 < net.n and kinds[i + 1] == "maxpool" and mean_ms[i + 1] < 0.005 else 1.0 for i in range(net.n)]
     small = np.array([bool(tc[i]) and not big3[i] for i in range(net.n)])
     mem_bytes = 0.0
     for i in np.nonzero(small)[0]:
         c, h, w = net.layer_shape(int(i))
         stride = int(sections[i][1].get("stride", 1))
         sh = shapes[int(i)]
-        mem_bytes += es * per_gpu * (sh.c * (h * stride) * (w * stride) + sh.n * h * w) + es * sh.n * sh.c * sh.size * sh.size
+        mem_bytes += es * per_gpu * (sh.c * (h * stride) * (w * stride) + written[i] * sh.n * h * w) + es * sh.n * sh.c * sh.size * sh.size
         if i + 1 < net.n and kinds[i + 1] == "shortcut" and mean_ms[i + 1] < 0.01:   # fused: its add is read by this launch
             mem_bytes += es * per_gpu * sh.n * h * w
     small_ms = float(mean_ms[small].sum())
@@ -427,7 +429,7 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
                 sh = shapes[int(i)]
                 stride = int(sections[int(i)][1].get("stride", 1))
                 in_e = float(per_gpu) * sh.c * (h * stride) * (w * stride)
-                out_e = float(per_gpu) * sh.n * h * w
+                out_e = written[i] * float(per_gpu) * sh.n * h * w
                 desc = net.layer_describe(int(i))
                 given, gives = "signs_in=1" in desc, "signs_out=1" in desc
                 passes += 0 if given else 1

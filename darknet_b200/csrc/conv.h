@@ -88,12 +88,12 @@ struct alignas(64) TcArgs {
     // and with its weights.  `stages` tiles' boxes are a ring of a_slot bytes each.
     int halo, a_slot, a_box_slot, a_box_bytes, a_pitch;
     int tmem_cols;        // TMEM columns the CTA allocates: a power of two >= 2*bn (two accumulators)
-    int debug;            // timing experiments only (DNB_TC_DEBUG): 1 no residual loads, 2 no output stores, 4 no wait before a residual request, 8 empty epilogue, 16 no MMAs;
+    int debug;            // timing experiments only (DNB_TC_DEBUG): 1 no residual loads, 2 no output stores, 4 no wait before a residual request (one group), 8 empty epilogue, 16 no MMAs;
                           // 32 (dnb_conv_plan_set_diagnostics): each CTA withholds the last operand load of its first tile, so a bounded wait runs out
     long long wait_limit; // bound of every device-side wait, SM clock cycles
     int stage_bufs;       // staging buffers of the epilogue: 2, or 4 with a fused residual (it lands in them first), 3 with signs, 0 where two groups write Darknet's layout only
     int pair;             // 1: clusters of two CTAs share every MMA (cta_group::2); total_tiles then counts PAIRS of pixel tiles,
-                          // b_bytes and the weight map's box cover half a filter tile, bn is 256
+                          // b_bytes and the weight map's box cover half a filter tile, bn is 128 or 256
     int ctas_per_sm;      // 2 for narrow tiles (TMEM and shared memory are sized so that two CTAs share an SM), else 1
     int pool;             // 1: tmy (and tms) are the 2x2 stride-2 maxpool's output; wt and ht are even
     int epi_groups;       // groups of four epilogue warps: 2 where a CTA has its SM to itself and staged rows are 128 bytes, else 1

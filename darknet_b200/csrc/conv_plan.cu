@@ -647,9 +647,24 @@ static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeo
     return DNB_OK;
 }
 
-// Microseconds of the persistent kernel by the measure of split_of: an epilogue hides behind the next tile's K loop, or the
-// other way round, and the last one is exposed; 64-filter tiles alone on an SM wait for their MMAs' results longer.
-static double persistent_us(const TcArgs &a, int k_iters, bool residual)
+// Microseconds of the persistent kernel, in a chain of dependent launches as split_of has it.  A K iteration measured on B200 with 3x3 layers
+// of 256 to 1024 channels at 1 to 16 images: pairs 0.168 (128 filters) and 0.287 (256), single CTAs 0.317 (256), 0.187 (128) and 0.18 (64)
+// with an SM to themselves, 0.26 and 0.135 where two share one and its room for ring slots.  An epilogue hides behind the next tile's loop, or
+// the other way round, and the last one is exposed.
+static double persistent_us(int pair, int bn, long long tiles, int k_iters, bool residual)
+{
+    const long long slots = pair ? sm_count() / 2 : sm_count();
+    const bool shared = !pair && bn <= 128 && tiles > sm_count();
+    const double rounds = (double)((tiles + slots - 1) / slots);
+    const double iteration = pair ? (bn <= 128 ? 0.168 : 0.287) : bn <= 64 ? (shared ? 0.135 : 0.18) : bn <= 128 ? (shared ? 0.26 : 0.187) : 0.317;
+    const double loop = k_iters * iteration, epilogue = bn * (residual ? 0.02 : 0.015);
+    return 4.2 + (pair ? 1.0 : 0.0) + rounds * (loop > epilogue ? loop : epilogue) + 0.8 * epilogue;
+}
+
+// Whether K is cut, and how often, is part of a layer's result: its sums are added in another order.  So that choice stands by itself, on tiles
+// halved until they fill the SMs (pick_persistent_tiles, plain) and the measure that it was fitted with, and better tiles for the
+// persistent kernel, which change no sum, leave every output as it was.
+static double uncut_us(const TcArgs &a, int k_iters, bool residual)
 {
     const long long slots = a.pair ? sm_count() / 2 : sm_count();
     const double share = (double)((a.total_tiles + slots - 1) / slots);
@@ -659,7 +674,8 @@ static double persistent_us(const TcArgs &a, int k_iters, bool residual)
 }
 
 // Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
-static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual, bool pool = false)
+// plain: by the number of tiles alone (see uncut_us).
+static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual, bool pool = false, bool plain = false)
 {
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
     pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt, pool);
@@ -690,16 +706,15 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     // the same 77 clocks, so what counts is how many tiles the fullest SM gets: 50 pixel tiles of 256 filters are better cut into 100 tiles of 128
     // than into 200 of 64 (3x3 128 -> 256 at 76 x 76 20.9 -> 18.9 us, 256 -> 512 at 4 x 26 x 26 32.7 -> 26.8; YOLOv3-608, one image, in a graph 898 -> 874,
     // YOLOv3-416, four, 1282 -> 1203).
+    const int k_iters = g.size * g.size * a.c_blocks;
+    auto estimate = [&](int pair, int bn) {
+        return persistent_us(pair, bn, (long long)(pair ? (ptiles + 1) / 2 : ptiles) * ((p->n_pad + bn - 1) / bn), k_iters, residual);
+    };
     if (ptiles * a.n_tiles < sm_count()) {
-        auto estimate = [&](int bn) {
-            TcArgs t;
-            t.pair = 0; t.bn = bn; t.total_tiles = ptiles * ((p->n_pad + bn - 1) / bn);
-            return persistent_us(t, g.size * g.size * a.c_blocks, residual);
-        };
         int best = a.bn;
         for (int bn = a.bn; bn >= 128 && bn % 128 == 0 && ptiles * ((p->n_pad + bn - 1) / bn) < sm_count();) {
             bn /= 2;
-            if (estimate(bn) <= estimate(best)) best = bn;
+            if (plain || estimate(0, bn) <= estimate(0, best)) best = bn;
         }
         a.bn = best;
         a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
@@ -718,8 +733,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     // 19x19 layers at batch 64).  A 3x3 layer over one block of channels has nine: its epilogue outlasts its MMAs, and single
     // CTAs hand over with less ceremony (33 x 38 x 38, 64 -> 1024 in bf16 59.6 us in pairs, 55.6 without; 64 -> 256 19.5 and 16.4;
     // 32 -> 1024 in TF32 74 and 71.5; 128 -> 256 of xnor layers, 128 x 28 x 28, 52.2 and 48.1); over two blocks, 18 iterations, pairs
-    // are ahead again (96 -> 512 in bf16 44.4 and 53.7).  With a fused residual, which pairs read with
-    // plain loads, nine iterations still run in pairs: the tests fix that choice (64 -> 512, stride 2, 40 x 44 x 44 in bf16: 23.5 us,
+    // are ahead again (96 -> 512 in bf16 44.4 and 53.7).  With a fused residual nine iterations still run in pairs: the tests fix that choice (64 -> 512, stride 2, 40 x 44 x 44 in bf16: 23.5 us,
     // 20 in single CTAs).  DNB_TC_PAIR: 0 never, 1 3x3 layers of fewer iterations too, 2 every layer the geometry allows.
     a.pair = 0;
     {
@@ -730,13 +744,26 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         // layers), at least half of them: a pair's six-deep ring of 32 KB slots keeps its tensor pipes fed where two
         // single CTAs per SM with two or three slots each starve on load latency, which outweighs the idle SMs.
         const int pair_tiles = (ptiles + 1) / 2 * (g.n / 256), clusters = sm_count() / 2;
-        const int k_iters_p = g.size * g.size * a.c_blocks;
-        const bool enough = pair_tiles >= clusters || (k_iters_p >= 64 && 2 * pair_tiles >= clusters);
-        const bool legal = !a.halo && a.row_bytes == 128 && g.n % 256 == 0 && enough && channels_last && y_cpitch * (bf16 ? 2 : 4) >= 128;
-        if (legal && !pool && (knob == 2 || (g.size >= 3 && (knob == 1 || (knob < 0 && residual))) || (knob != 0 && k_iters_p >= 16))) {
+        const bool enough = pair_tiles >= clusters || (k_iters >= 64 && 2 * pair_tiles >= clusters);
+        const bool legal = a.row_bytes == 128 && channels_last && y_cpitch * (bf16 ? 2 : 4) >= 128 && !pool;
+        const bool wanted = legal && (knob == 2 || (g.size >= 3 && (knob == 1 || (knob < 0 && residual))) || (knob != 0 && k_iters >= 16));
+        if (wanted && g.n % 256 == 0 && enough) {
             a.pair = 1;
             a.bn = 256;
             a.n_tiles = p->n_pad / 256;
+        }
+        // A launch of a few rounds: the whole rounds it takes decide between tiles.  A pair over 128 filters loads as little per MMA as it can
+        // (24 KB an iteration and CTA, 0.168 us) and comes in halves of a pair over 256, which is the better one in full rounds: 3x3 512 -> 512 at 16 x
+        // 26 x 26 in TF32 99.6 -> 80.9 us (pairs over 256: 90.0), 256 -> 256 at 8 x 52 x 52 49.2 -> 45.0, 1024 -> 1024 at 16 x 19 x 19 196 -> 162, and in
+        // bf16 8 x 52 x 52 27.7 -> 25.9; 2 x 76 x 76 stays with 256 (30.0 and 31.4).
+        if (knob < 0 && !plain && !i8 && g.n % 128 == 0 && (ptiles + 1) / 2 * ((g.n + 255) / 256) < 6 * clusters) {
+            double best = estimate(a.pair, a.bn);
+            for (int pair = a.pair; pair < 2; ++pair)
+                for (int bn = 128; bn <= 256; bn *= 2) {
+                    if (g.n % bn || (pair && !(wanted && k_iters >= 16)) || (!pair && nchw_out)) continue;
+                    const double us = estimate(pair, bn);
+                    if (us < 0.97 * best) { best = us; a.pair = pair; a.bn = bn; a.n_tiles = p->n_pad / bn; }
+                }
         }
     }
     a.total_tiles = a.pair ? (ptiles + 1) / 2 * a.n_tiles : ptiles * a.n_tiles;
@@ -927,13 +954,11 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             } else {
                 // decided at one image for two images also (see choose_split)
                 ConvGeom dg = g;
+                if (g.batch == 2) dg.batch = 1;
                 TcArgs da = a;
-                if (g.batch == 2) {
-                    dg.batch = 1;
-                    pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
-                }
+                pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, false, true);
                 sp = choose_split(q, flat(dg), 0, false, dg.batch);
-                if (!(sp.cost < persistent_us(da, k_iters, q.residual))) sp = SplitPlan();
+                if (!(sp.cost < uncut_us(da, k_iters, q.residual))) sp = SplitPlan();
                 else if (g.batch == 2) sp = choose_split(q, flat(g), sp.splits, false, 2);
             }
             if (sp.splits) DNB_TRY(build_split_args(p, x, flat(g), sp, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));

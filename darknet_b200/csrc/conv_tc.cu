@@ -15,13 +15,13 @@
 //   per row/column parity), so every load is still a dense box.
 // * Accumulators live in TMEM (fp32); two accumulator buffers of bn columns let the
 //   epilogue of tile i overlap the MMAs of tile i+1.
-// * Warp roles in a 192-thread CTA: warp 0 issues TMA, warp 1 issues tcgen05.mma and
+// * Warp roles in a 192- or 320-thread CTA: warp 0 issues TMA, warp 1 issues tcgen05.mma and
 //   owns the TMEM allocation (both loop as whole warps and elect a lane for the
 //   instruction itself: inside one lane's branch an iteration took 284 cycles; 33 x 38 x 38,
-//   128 -> 1024 3x3 in bf16 95 -> 85 us, 16 x 304 x 304, 32 -> 64 in TF32 207 -> 192), warps 2-5 drain TMEM
+//   128 -> 1024 3x3 in bf16 95 -> 85 us, 16 x 304 x 304, 32 -> 64 in TF32 207 -> 192), warps 2-5 (or 2-9) drain TMEM
 //   and apply the fused epilogue: folded batchnorm or bias, activation, optionally
 //   the residual add of a following shortcut layer (its tile arrives by TMA in the
-//   staging buffer the finished rows then overwrite), TF32 rounding, TMA store of
+//   staging buffer the finished rows then overwrite; pairs copy it there), or the maxpool after the layer, TF32 rounding, TMA store of
 //   the channels-last rows and/or plain stores of Darknet's NCHW layout.
 // * Persistent: one CTA per SM (two when the filter tile is at most 128 wide) walks
 //   tiles blockIdx.x, +gridDim.x, ...; tiles that share a pixel box are adjacent so
@@ -137,7 +137,7 @@ __device__ __forceinline__ void group_bar(int group) { asm volatile("bar.sync %0
 // is > 0, else -1, 0 beyond the layer's filters) as the int8 channels-last tensor that the xnor layer after it reads as
 // its operand: that layer's sign pass over the f32 tensor disappears.  The signs of a chunk are staged in a third
 // staging buffer (two 4 KB halves in rotation) and leave with the chunk's output rows, in the same bulk group.
-// POOL: the output is that of the 2x2 maxpool with stride 2 after the layer (forward_maxpool_layer, src/maxpool_layer.c:79-117); the layer's own
+// POOL: the output is that of the 2x2 maxpool with stride 2 after the layer (forward_maxpool_layer, src/maxpool_layer.c:79-114); the layer's own
 // is not written.  A chunk's finished rows are staged as ever, a thread takes the largest of four of them, for a quarter of a pooled pixel, and what leaves is
 // a box of a quarter of the pixels: of the two passes' bytes, 9 per output value of the layer, one is left, and one launch.
 // EG: groups of four epilogue warps.  Two CTAs on an SM bring eight epilogue warps between them; one CTA with four has every SM

@@ -71,7 +71,7 @@ template <> __device__ __forceinline__ float from_float<float>(float v) { return
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
 // Four 16-byte pieces (floats, or bf16 values) of a 2x2 maxpool's window: its largest values, as forward_maxpool_layer finds them, from the
-// lowest float up (src/maxpool_layer.c:88-107), so that a NaN never wins.
+// lowest float up (src/maxpool_layer.c:103-105), so that a NaN never wins.
 template <bool BF16>
 __device__ __forceinline__ uint4 largest_of_four(const uint4 (&v)[4])
 {
