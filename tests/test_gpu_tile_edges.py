@@ -448,3 +448,18 @@ def test_one_box_for_nine_taps(name, monkeypatch):
         assert np.array_equal(a, b) and np.array_equal(a, c)
         out[knob] = a
     assert np.array_equal(out["0"], out["2"])
+
+
+@pytest.mark.parametrize("mode,c", [(dn.MODE_TF32, 512), (dn.MODE_BF16, 1024)])
+def test_pairs_over_128_filters(mode, c, monkeypatch):
+    """A launch of three rounds of such pairs where pairs over 256 filters or single CTAs take two of twice the length, on a ragged map: equal to single CTAs to the bit."""
+    import numpy as np
+    case = conv_case(750, b=15, c=c, h=25, w=27, n=512, size=1)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    monkeypatch.delenv("DNB_TC_PAIR", raising=False)
+    plan, got, _ = run_conv(case, mode, "nhwc", "nhwc")
+    assert "pair=1" in plan.describe() and "bn=128" in plan.describe(), plan.describe()
+    monkeypatch.setenv("DNB_TC_PAIR", "0")
+    plan, single, _ = run_conv(case, mode, "nhwc", "nhwc")
+    assert "pair=0" in plan.describe() and np.array_equal(got, single)
+    parity(got, oracle_conv(case), 3e-2 if mode == dn.MODE_BF16 else 1e-2)
