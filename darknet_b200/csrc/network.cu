@@ -831,7 +831,8 @@ static int forward_layer(dnb_network *net, int i, const float *device_input, con
             float *keep = nullptr;
             if (i == 0 && device_input != net->input_slot[0] && device_input != net->input_slot[1]) {
                 const size_t bytes = (size_t)net->batch * net->inputs * sizeof(float);
-                if (L.plan->keep_k_order || bytes <= (size_t)8 << 20) keep = net->input_dev;
+                // (an xnor layer that comes first has no kernel that writes the copy)
+                if (L.plan->stem_tc && (L.plan->keep_k_order || bytes <= (size_t)8 << 20)) keep = net->input_dev;
                 else DNB_CUDA(cudaMemcpyAsync(net->input_dev, device_input, bytes, cudaMemcpyDeviceToDevice, s));
             }
             const dnb_tensor pooled = part_of(net->layers[i + 1].out, p);
