@@ -421,6 +421,34 @@ def test_maxpool_in_the_convolutions_epilogue(mode, xnor, batch, size, first_fil
         assert np.array_equal(a, b, equal_nan=True)
 
 
+@pytest.mark.parametrize("batch,size", [(2, 160), (40, 48)])
+def test_own_output_of_a_first_xnor_layer_with_its_maxpool(batch, size, tmp_path):
+    """The first layer's own output after a forward over a caller's buffer that is overwritten since: made from those images, not from a
+    predict's before it or from nothing.  Equal to that of a predict over the same images, to the bit."""
+    import numpy as np
+    import torch
+    from darknet_b200 import synth
+    pool = "\n[maxpool]\nsize=2\nstride=2\n"
+    cfg = synth._net(batch, size, size) + synth._conv(64, 3, xnor=True) + pool + synth._conv(32, 3, xnor=True) + "\n[avgpool]\n"
+    params = synth.seeded_params(cfg, 11)
+    path = str(tmp_path / "x.weights")
+    synth.write_weights(path, params)
+    x, y = synth.seeded_input(cfg, 12, "normal"), synth.seeded_input(cfg, 13, "normal")
+    net = dn.Network(cfg, path, dn.MODE_TF32, text=True)
+    net.predict(x)
+    want = [net.layer_output(i) for i in range(net.n)]
+    net.predict(y), net.predict(y)      # both of the network's own image buffers
+    dev = torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    net.forward(dev)
+    torch.cuda.synchronize()
+    dev.zero_()
+    torch.cuda.synchronize()
+    for i in range(net.n):
+        assert np.array_equal(net.layer_output(i), want[i]), i
+    net.close()
+
+
 HALO = {   # one box for the nine taps, weights in shared memory: row widths, strides, channel blocks, ragged maps
     "tf32_64_byte_rows": (dict(b=3, c=16, h=37, w=27, n=32, size=3), dn.MODE_TF32, False),
     "tf32_two_blocks": (dict(b=2, c=40, h=33, w=18, n=48, size=3, act="linear"), dn.MODE_TF32, False),
