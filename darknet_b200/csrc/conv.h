@@ -1,6 +1,7 @@
 // Internal argument blocks of the convolution kernels and the plan object.
 #pragma once
 #include <cuda.h>
+#include <cuda_bf16.h>
 
 #include <vector>
 
@@ -146,12 +147,12 @@ int launch_conv_tc_split(const SplitArgs &a, cudaStream_t s);
 size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes);
 int conv_tc_split_resident(int pair, int cluster);
 
-// ---- conv_fp32_tc.cu : fp32 convolution as three TF32 products on the tensor cores, sums in fp32 registers
+// ---- conv_fp32_tc.cu : fp32 convolution by three bf16 parts of every operand on the tensor cores, sums in fp32 registers
 struct alignas(64) Fp32TcArgs {
     CUtensorMap tmx[4];   // as in TcArgs; boxes of 32 channels x wt x ht x bt pixels
     CUtensorMap tmy;      // channels-last output, boxes of 32 channels (16 where bn is 32) and the tile's pixels
-    CUtensorMap tmw;      // [2*taps][n_pad][c_pad]: the weights' high halves, then their low halves
-    int c_blocks, taps, last_slices;   // last_slices: MMAs of 8 channels in a tap's last block of 32
+    CUtensorMap tmw;      // [c_blocks*taps][3][n_pad][32]: the weights' three parts
+    int c_blocks, taps, last_slices;   // last_slices: MMAs of 16 channels in the last block of 32
     int bn, n_tiles;      // filters per tile: 32, 64 or 128
     int wt, ht, bt, tiles_w, tiles_h, total_tiles;
     int n_pad;
@@ -209,7 +210,7 @@ struct dnb_conv_plan {
     float *scale, *shift;    // [n_pad] folded batchnorm / bias
     void *w_tc;              // [taps][n_pad][c_pad] f32 (TF32-rounded) or bf16
     float *w_direct;         // [groups][K][npg_pad]
-    float *w_halves;         // [2*taps][n_pad][c_pad]: high and low TF32 halves (full-precision plans on the tensor cores)
+    __nv_bfloat16 *w_parts;  // [c_blocks][taps][3][n_pad][32]: the weights' three bf16 parts (full-precision plans on the tensor cores)
     uint32_t *w_bits;        // [n][taps][cwords]
     float *w_mean;           // [n]
     int npg_pad, cwords;

@@ -1,31 +1,33 @@
 // Full-precision convolution on the sm_100a tensor cores: implicit GEMM as in conv_tc.cu, every fp32 operand as the sum of
-// two TF32 numbers, sums in fp32 registers.
+// three bf16 numbers (the splitting of Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For
+// Higher-Precision Computations", 2019), sums in fp32 registers.
 //
-//   x = xh + xl, w = wh + wl        (xh: x rounded to TF32; xl: the exact rest, rounded to TF32)
-//   x*w = xl*wh + xh*wl + xh*wh     (xl*wl, below 2^-24 of the product, is left out)
+//   x = x0 + x1 + x2, w = w0 + w1 + w2    (x0: x rounded to bf16; x1: the rest, rounded to bf16; x2: what is left, exactly: 8 + 8 + 8 bits)
+//   x*w = x0*w0 + (x1*w2 + x2*w1 + x1*w1 + x2*w0 + x0*w2 + x1*w0 + x0*w1)       (x2*w2, at most 2^-34 of the product, is left out)
 //
-// What bounds the fp32 GEMM of conv_direct.cu is operand pairing and FMA issue on the CUDA cores, 37 TFLOP/s.  Three TF32 products on
-// the tensor pipe have 280 in them.  What has to hold is the precision: a product keeps 2^-24 or so of its value, and
-// the tensor core, which cuts its running sums off instead of rounding them, never adds more than the 32 channels of one tap: then
-// the partial sum leaves TMEM and is added in a register, rounded to nearest.  Error against 64 bits, root mean square over
-// root mean square: see fp32_tc_covers in conv_plan.cu, where it is set beside the CUDA-core kernel's.
+// What bounds the fp32 GEMM of conv_direct.cu is operand pairing and FMA issue on the CUDA cores, 37 TFLOP/s.  What has to hold is its
+// precision.  The products of bf16 numbers are exact in the tensor core; its running sums, which it cuts off instead of rounding them, are not.  So
+// there are two: the large products' (x0*w0, 16 bits each) leaves TMEM after the 32 channels of a tap and is added to a register, rounded to
+// nearest; the small ones', whose cut-off digits count 2^-8 of that, goes on for up to 64 such steps, and is added at the end.  A sum of one product is
+// that product rounded, 2^-24 as in fp32, of a few mostly just as well, and a factor of 1 is exact.  (Two TF32 halves with one sum for all, 22 bits
+// and cut off, were 2.4 times as far from 64 bits as fp32 for sums of one to a few products; the small sums added step by step, a rounding
+// more for each, 1.2 times.)  Error of dense sums: see fp32_tc_covers in conv_plan.cu, where it is set beside the CUDA-core kernel's.
 //
-// * Tile: 128 output pixels (a wt x ht x bt box) by BN filters; a step of K is one tap and 32 channels.
-// * Warp 0 loads a step by TMA: BN x 32 of wh and of wl, and of a channels-last input 16 KB as it is.  The input goes through
-//   registers anyway to be split, so its two halves are written to TMEM, where the MMA takes its A operand from: no shared memory for
+// * Tile: 128 output pixels (a wt x ht x bt box) by BN filters; a step of K is one tap and 32 channels, sixteen MMAs.
+// * Warp 0 loads a step by TMA: BN x 32 of each part of w, and of a channels-last input 16 KB as it is.  The input goes through
+//   registers anyway to be split, so its parts are written to TMEM, where the MMA takes its A operand from: no shared memory for
 //   them, and half of what the MMAs would read there.
 // * A 1x1 layer over a Darknet tensor needs no channels-last copy of it: its channels are planes, so the threads that split fetch their
-//   pixel's 32 values themselves, coalesced along the plane, the next step's while this one's are multiplied (26 x 326 x 56 x 56 -> 34:
-//   71 us, through a copy 78).  With the shifted, short runs of a 3x3 layer's tile the same takes longer than the copy (8 x 64 x 104 x
-//   104 -> 128: 125 us, through a copy 97): lines in flight are more than the first-level cache has beside the ring.
-// * Warps 4-11 split, one half of them the even steps, the other the odd ones: a thread takes its pixel's row, writes 32 columns of
-//   xh and 32 of xl.  (Four warps for all steps: 110 us where eight take 80, 8 x 64 x 104 x 104 -> 128, 3x3; a step's way through a
+//   pixel's 32 values themselves, coalesced along the plane, the next step's while this one's are multiplied.
+// * Warps 4-11 split, one half of them the even steps, the other the odd ones: a thread takes its pixel's row, writes 16 columns of
+//   each part.  (Four warps for all steps: 110 us where eight took 80, 8 x 64 x 104 x 104 -> 128, 3x3; a step's way through a
 //   warp is all latency.)
-// * Warp 1 issues twelve MMAs a step into one of two accumulators.
-// * Warps 12-19 add the finished accumulator to registers, half the filters each, and after the tile's last step scale, shift,
+// * Warp 1 issues a step's MMAs, the large products' first, into one of two accumulators that is added up while the small ones' MMAs run, then those.
+// * Warps 12-19 add the finished accumulators to registers, half the filters each, and after the tile's last step scale, shift,
 //   activate and store.  They take the registers that the other warps give up.
-// * A ring of four slots: shared memory for what TMA brings, and 64 columns of TMEM for the split rows, freed together.
-// * A sum that is infinite, not a number, or smaller than the low halves can hold is added up again in fp32, product by product, so
+// * A ring of four slots of shared memory for what TMA brings, and one of 48 columns of TMEM each for the split rows: two beside three
+//   accumulators of 128 columns, four beside narrower ones.
+// * A sum that is infinite, not a number, or smaller than the parts can hold is added up again in fp32, product by product, so
 //   what infinities and NaN in the input become is what the CUDA-core kernel makes of them.
 // * Every wait is bounded as in conv_tc.cu.
 #include <cuda.h>
@@ -45,26 +47,42 @@ constexpr int FT_REGS_ISSUE = 40, FT_REGS_SPLIT = 96, FT_REGS_SUM = 120;
 static_assert(FT_REGS_ISSUE + 2 * FT_REGS_SPLIT + 2 * FT_REGS_SUM <= 5 * 96, "no more registers than the launch has");
 constexpr int FT_STAGES = 4;
 constexpr int FT_A_BYTES = 128 * 128;
-constexpr int FT_TMEM = 512;               // four slots of 64 columns, two accumulators of up to 128
+constexpr int FT_TMEM = 512;
+constexpr int FT_SLOT = 48;                // columns of a split row: 16 of each part
+constexpr int FT_RUN = 64;                 // steps after which the small products' sum is added up
+template <int BN> constexpr int FT_SLOTS = BN == 128 ? 2 : 4;
+static_assert(FT_SLOTS<128> * FT_SLOT + 3 * 128 <= FT_TMEM && FT_SLOTS<64> * FT_SLOT + 3 * 64 <= FT_TMEM, "columns");
 
 struct FtShared {
     uint64_t full[FT_STAGES];      // a step's tiles are in shared memory
-    uint64_t split[FT_STAGES];     // its input rows are in TMEM
     uint64_t empty[FT_STAGES];     // its MMAs have retired
-    uint64_t acc_full[2], acc_empty[2];
+    uint64_t split[4];             // a step's input rows are in TMEM
+    uint64_t split_empty[4];       // ... and the MMAs that read them have retired
+    uint64_t acc_full[3], acc_empty[3];   // the large products' two, the small ones'
     uint32_t tmem_base;
     int abort_flag;
 };
 
 enum { FT_WAIT_EMPTY = 101, FT_WAIT_FULL = 102, FT_WAIT_ACC_EMPTY = 103, FT_WAIT_ACC_FULL = 104, FT_WAIT_SPLIT = 105, FT_BAD_BASE = 106 };
 
-// A from TMEM: row i of the operand in lane i, one column per TF32 value.
-__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+// A from TMEM: row i of the operand in lane i, a column per two bf16 values.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// x1*w2 + x2*w1 + x1*w1 + x2*w0 + x0*w2 + x1*w0 + x0*w1 over K slices of 16 channels; the parts of w lie PART bytes apart
+template <uint32_t PART, int K>
+__device__ __forceinline__ void small_products(uint32_t d, uint32_t x, uint64_t w, uint32_t idesc, uint32_t accumulate)
+{
+    constexpr int xi[7] = {1, 2, 1, 2, 0, 1, 0}, wi[7] = {2, 1, 1, 0, 2, 0, 1};
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+#pragma unroll
+        for (int k = 0; k < K; ++k) umma_bf16_ts(d, x + 16 * xi[i] + 8 * k, w + wi[i] * (PART >> 4) + 2 * k, idesc, i + k ? 1u : accumulate);
 }
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
@@ -76,12 +94,14 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Nearest TF32; infinities and NaN stay what they are.
-__device__ __forceinline__ float nearest_tf32(float x)
+// Two values' nearest bf16 as one word (first in the low half), and what is left of them.  An infinity leaves a NaN.
+__device__ __forceinline__ uint32_t take_bf16(float &a, float &b)
 {
     uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return __uint_as_float(r & 0xffffe000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    a -= __uint_as_float(r << 16);
+    b -= __uint_as_float(r & 0xffff0000u);
+    return r;
 }
 
 // One output the way the CUDA-core kernel adds it: fp32, in the order c, kh, kw.
@@ -101,8 +121,7 @@ __device__ __forceinline__ float plain_sum(const Fp32TcArgs &a, int b, int oh, i
     return acc;
 }
 
-// Sums whose size says that the halves may not have carried them: infinite, NaN, or below 2^-90 and not zero (a low half is 2^-12
-// of its operand or less, and two operands of 2^-45 have low halves that are still normal numbers).
+// Sums whose size says that the parts may not have carried them: infinite, NaN, or below 2^-90 and not zero.
 __device__ __forceinline__ bool out_of_range(float v)
 {
     const uint32_t m = __float_as_uint(v) & 0x7fffffffu;
@@ -134,7 +153,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1)
 conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr uint32_t B_BYTES = BN * 128, STAGE = FT_A_BYTES + 2 * B_BYTES;
+    constexpr uint32_t B_BYTES = BN * 64, STAGE = FT_A_BYTES + 3 * B_BYTES;   // 32 channels of one part of w; a stage
+    constexpr int SLOTS = FT_SLOTS<BN>;
     constexpr int COLS = BN / 2, LD = COLS < 32 ? COLS : 32;   // filters of one half of the summing warps, columns of a TMEM read and of a staged row
     constexpr int ROW = LD * 4;
     const uint32_t ring = smem_u32(smem_raw);
@@ -149,10 +169,13 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
     if (threadIdx.x == 0) {
         for (int s = 0; s < FT_STAGES; ++s) {
             mbar_init(smem_u32(&sh->full[s]), 1);
-            mbar_init(smem_u32(&sh->split[s]), 4);
             mbar_init(smem_u32(&sh->empty[s]), 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int s = 0; s < SLOTS; ++s) {
+            mbar_init(smem_u32(&sh->split[s]), 4);
+            mbar_init(smem_u32(&sh->split_empty[s]), 1);
+        }
+        for (int i = 0; i < 3; ++i) {
             mbar_init(smem_u32(&sh->acc_full[i]), 1);
             mbar_init(smem_u32(&sh->acc_empty[i]), 8);
         }
@@ -169,14 +192,15 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
     tc_fence_after();
     launch_dependents();
     grid_dependency_wait();
-    const uint32_t tmem_base = sh->tmem_base, acc0 = tmem_base + FT_STAGES * 64;
+    const uint32_t tmem_base = sh->tmem_base, acc0 = tmem_base + SLOTS * FT_SLOT;
 
     const int taps = a.taps, c_blocks = a.c_blocks, steps = taps * c_blocks, last_slices = a.last_slices;
     const int n_tiles = a.n_tiles, total_tiles = a.total_tiles;
     const int wt = a.wt, ht = a.ht, bt = a.bt, tiles_w = a.tiles_w, tiles_h = a.tiles_h;
     const long long limit = a.wait_limit;
     int *status = a.status;
-    const uint32_t full0 = smem_u32(&sh->full[0]), split0 = smem_u32(&sh->split[0]), empty0 = smem_u32(&sh->empty[0]);
+    const uint32_t full0 = smem_u32(&sh->full[0]), empty0 = smem_u32(&sh->empty[0]), split0 = smem_u32(&sh->split[0]), split_empty0 = smem_u32(&sh->split_empty[0]);
+    const uint32_t acc_full0 = smem_u32(&sh->acc_full[0]), acc_empty0 = smem_u32(&sh->acc_empty[0]);
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FT_REGS_ISSUE));
@@ -190,55 +214,70 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             const int n0 = tile % n_tiles * BN, pt = tile / n_tiles;
             const int ow0 = pt % tiles_w * wt, oh0 = pt / tiles_w % tiles_h * ht, b0 = pt / (tiles_w * tiles_h) * bt;
-            for (int tap = 0, kh = 0, kw = 0; tap < taps && ok; ++tap) {
-                const int dh = kh - pad, dw = kw - pad;
-                int ph = 0, qh = dh, pw = 0, qw = dw;
-                if (stride == 2) { ph = dh & 1; qh = (dh - ph) >> 1; pw = dw & 1; qw = (dw - pw) >> 1; }
-                const CUtensorMap *mx = a.tmx + (ph * stride + pw);
-                for (int cb = 0; cb < c_blocks; ++cb) {
+            for (int cb = 0; cb < c_blocks && ok; ++cb)          // the taps of a block of channels: their rows are neighbours
+                for (int tap = 0, kh = 0, kw = 0; tap < taps; ++tap) {
+                    const int dh = kh - pad, dw = kw - pad;
+                    int ph = 0, qh = dh, pw = 0, qw = dw;
+                    if (stride == 2) { ph = dh & 1; qh = (dh - ph) >> 1; pw = dw & 1; qw = (dw - pw) >> 1; }
+                    const CUtensorMap *mx = a.tmx + (ph * stride + pw);
                     ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, FT_WAIT_EMPTY, limit);
                     if (!ok) break;
                     if (withhold && tile == (int)blockIdx.x && tap == taps - 1 && cb == c_blocks - 1) { ok = false; break; }
                     if (elect_one()) {
                         const uint32_t bar = full0 + 8 * stage, slot = ring + stage * STAGE;
-                        mbar_expect_tx(bar, PLANES ? 2 * B_BYTES : STAGE);
+                        mbar_expect_tx(bar, PLANES ? 3 * B_BYTES : STAGE);
                         if (!PLANES) tma_load_4d(slot, mx, bar, cb * 32, ow0 + qw, oh0 + qh, b0);
-                        tma_load_3d(slot + FT_A_BYTES, &a.tmw, bar, cb * 32, n0, tap);
-                        tma_load_3d(slot + FT_A_BYTES + B_BYTES, &a.tmw, bar, cb * 32, n0, taps + tap);
+                        tma_load_4d(slot + FT_A_BYTES, &a.tmw, bar, 0, n0, 0, cb * taps + tap);   // three tiles of BN rows, one of each part
                     }
                     if (++stage == FT_STAGES) { stage = 0; phase ^= 1; }
+                    if (++kw == ksize) { kw = 0; ++kh; }
                 }
-                if (++kw == ksize) { kw = 0; ++kh; }
-            }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMAs
-        const uint32_t idesc = mma_idesc<MMA_TF32>(128u, (uint32_t)BN);
-        const uint64_t bh0 = make_smem_desc(ring + FT_A_BYTES, 128), bl0 = make_smem_desc(ring + FT_A_BYTES + B_BYTES, 128);
-        int stage = 0, it = 0;
-        uint32_t phase = 0;
+        const uint32_t idesc = mma_idesc<MMA_BF16>(128u, (uint32_t)BN);
+        const uint64_t b_desc0 = make_smem_desc(ring + FT_A_BYTES, 64);
+        int stage = 0, slot = 0, acc = 0, run = 0;
+        uint32_t phase = 0, slot_phase = 0, acc_phase = 0, small_phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x)
-            for (int step = 0, cb = 0; step < steps; ++step, ++it) {
-                const int acc = it & 1;
-                ok = mbar_wait_warp(smem_u32(&sh->acc_empty[acc]), ((it >> 1) & 1) ^ 1, abort_flag, status, FT_WAIT_ACC_EMPTY, limit) &&
-                     mbar_wait_warp(split0 + 8 * stage, phase, abort_flag, status, FT_WAIT_SPLIT, limit);
+            for (int step = 0, tap = 0, cb = 0; step < steps; ++step) {
+                const bool whole = cb != c_blocks - 1 || last_slices == 2;   // all 32 channels; else the first 16
+                const uint32_t x0 = tmem_base + slot * FT_SLOT;
+                const uint64_t w0 = b_desc0 + (uint64_t)(stage * (STAGE >> 4));
+                ok = mbar_wait_warp(acc_empty0 + 8 * acc, acc_phase ^ 1, abort_flag, status, FT_WAIT_ACC_EMPTY, limit) &&
+                     mbar_wait_warp(full0 + 8 * stage, phase, abort_flag, status, FT_WAIT_FULL, limit) &&
+                     mbar_wait_warp(split0 + 8 * slot, slot_phase, abort_flag, status, FT_WAIT_SPLIT, limit);
                 if (!ok) break;
                 tc_fence_after();
-                const int slices = cb == c_blocks - 1 ? last_slices : 4;
                 if (elect_one()) {
-                    const uint32_t d = acc0 + acc * BN, ah = tmem_base + stage * 64, al = ah + 32;
-                    const uint64_t off = (uint64_t)(stage * (STAGE >> 4));
-                    // the small products first: they then meet the large ones in a sum that still has room for them
-                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, al + 8 * k, bh0 + off + 2 * k, idesc, k != 0);
-                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, ah + 8 * k, bl0 + off + 2 * k, idesc, 1u);
-                    for (int k = 0; k < slices; ++k) umma_tf32_ts(d, ah + 8 * k, bh0 + off + 2 * k, idesc, 1u);
-                    umma_commit(empty0 + 8 * stage);
-                    umma_commit(smem_u32(&sh->acc_full[acc]));
+                    const uint32_t d = acc0 + acc * BN;
+                    umma_bf16_ts(d, x0, w0, idesc, 0u);
+                    if (whole) umma_bf16_ts(d, x0 + 8, w0 + 2, idesc, 1u);
+                    umma_commit(acc_full0 + 8 * acc);
                 }
-                if (++cb == c_blocks) cb = 0;
+                acc ^= 1;
+                if (!acc) acc_phase ^= 1;
+                if (run == 0) {
+                    ok = mbar_wait_warp(acc_empty0 + 16, small_phase ^ 1, abort_flag, status, FT_WAIT_ACC_EMPTY, limit);
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                const bool last = run == FT_RUN - 1 || step == steps - 1;
+                if (elect_one()) {   // the smallest first: they then meet the larger ones in a sum that still has room for them
+                    const uint32_t d = acc0 + 2 * BN;
+                    if (whole) small_products<B_BYTES, 2>(d, x0, w0, idesc, run != 0);
+                    else small_products<B_BYTES, 1>(d, x0, w0, idesc, run != 0);
+                    umma_commit(empty0 + 8 * stage);
+                    umma_commit(split_empty0 + 8 * slot);
+                    if (last) umma_commit(acc_full0 + 16);
+                }
+                ++run;
+                if (last) { run = 0; small_phase ^= 1; }
+                if (++tap == taps) { tap = 0; ++cb; }
                 if (++stage == FT_STAGES) { stage = 0; phase ^= 1; }
+                if (++slot == SLOTS) { slot = 0; slot_phase ^= 1; }
             }
         __syncwarp();
     }
@@ -265,39 +304,36 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         };
         if (PLANES && (warp < 8 ? 0 : 1) < count) fetch();
         for (long long it = warp < 8 ? 0 : 1; it < count; it += 2) {
-            const int stage = (int)it & (FT_STAGES - 1);
+            const int stage = (int)it & (FT_STAGES - 1), slot = (int)it & (SLOTS - 1);
             if (!mbar_wait(full0 + 8 * stage, (uint32_t)(it / FT_STAGES) & 1, abort_flag, status, FT_WAIT_FULL, 0, limit)) break;
-            tc_fence_after();   // the slot's columns were last read by MMAs whose retirement let this load be issued
             const uint8_t *row = smem_raw + stage * STAGE + m * 128;
-            const uint32_t dst = tmem_base + lane_base + stage * 64;
+            const uint32_t dst = tmem_base + lane_base + slot * FT_SLOT;
+            uint32_t part[3][16];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t hi[16], lo[16];
+            for (int q = 0; q < 8; ++q) {
+                float v[4];
+                if (PLANES) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float v[4];
-                    if (PLANES) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = x[PLANES ? 16 * h + 4 * q + e : 0];
-                    } else {
-                        const float4 f = *reinterpret_cast<const float4 *>(row + (((4 * h + q) ^ q_xor) << 4));
-                        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float xh = nearest_tf32(v[e]);
-                        hi[4 * q + e] = __float_as_uint(xh);
-                        lo[4 * q + e] = __float_as_uint(round_tf32(v[e] - xh));
-                    }
+                    for (int e = 0; e < 4; ++e) v[e] = x[PLANES ? 4 * q + e : 0];
+                } else {
+                    const float4 f = *reinterpret_cast<const float4 *>(row + ((q ^ q_xor) << 4));
+                    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
                 }
-                tmem_st16(dst + 16 * h, hi);
-                tmem_st16(dst + 32 + 16 * h, lo);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    part[i][2 * q] = take_bf16(v[0], v[1]);
+                    part[i][2 * q + 1] = take_bf16(v[2], v[3]);
+                }
             }
+            if (!mbar_wait(split_empty0 + 8 * slot, ((uint32_t)(it / SLOTS) & 1) ^ 1, abort_flag, status, FT_WAIT_SPLIT, 0, limit)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int i = 0; i < 3; ++i) tmem_st16(dst + 16 * i, part[i]);
             if (PLANES && it + 2 < count) fetch();
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(split0 + 8 * stage);
+            if (lane == 0) mbar_arrive(split0 + 8 * slot);
         }
     } else {
         // ---------------- sums and epilogue
@@ -310,18 +346,17 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         const int wl = m % wt, hl = (m / wt) % ht, bl = m / (wt * ht);
         const ConvGeom g = a.g;
         const int act = a.ep.activation;
-        int it = 0;
-        bool ok = true;
+        int acc = 0;
+        uint32_t acc_phase = 0, small_phase = 0;
+        bool ok = true, stored = false;
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             float sum[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
-            for (int step = 0; step < steps; ++step, ++it) {
-                const int acc = it & 1;
-                ok = mbar_wait(smem_u32(&sh->acc_full[acc]), (it >> 1) & 1, abort_flag, status, FT_WAIT_ACC_FULL, 0, limit);
-                if (!ok) break;
+            auto add_up = [&](int which, uint32_t parity) {
+                if (!mbar_wait(acc_full0 + 8 * which, parity, abort_flag, status, FT_WAIT_ACC_FULL, 0, limit)) return false;
                 tc_fence_after();
-                const uint32_t src = acc0 + acc * BN + col0 + ((uint32_t)(quarter * 32) << 16);
+                const uint32_t src = acc0 + which * BN + col0 + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll
                 for (int c = 0; c < COLS; c += LD) {
                     uint32_t r[LD];
@@ -333,7 +368,18 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[acc]));
+                if (lane == 0) mbar_arrive(acc_empty0 + 8 * which);
+                return true;
+            };
+            for (int step = 0; step < steps && ok; ) {
+                const int end = min(steps, step + FT_RUN);
+                for (; step < end && ok; ++step) {
+                    ok = add_up(acc, acc_phase);
+                    acc ^= 1;
+                    if (!acc) acc_phase ^= 1;
+                }
+                if (ok) ok = add_up(2, small_phase);
+                small_phase ^= 1;
             }
             if (!meet(half, ok && !*abort_flag)) break;
             const int n0 = tile % n_tiles * BN + col0, pt = tile / n_tiles;
@@ -346,7 +392,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
             uint32_t again[(COLS + 31) / 32] = {};              // sums that fp32 has to add up itself
 #pragma unroll
             for (int c = 0; c < COLS; c += LD) {
-                if (a.y_nhwc && (c > 0 || it > steps)) {        // the row's last store has been read
+                if (a.y_nhwc && (c > 0 || stored)) {            // the row's last store has been read
                     if (stores) tma_store_wait_read0();
                     meet(half, true);
                 }
@@ -388,6 +434,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
                     if (stores && c < real) { tma_store_4d(&a.tmy, smem_u32(staged), n0 + c, ow0, oh0, b0); tma_store_commit(); }
                 }
             }
+            stored = true;
         }
         if (stores) tma_store_wait_all();
     }
@@ -408,7 +455,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
 template <int BN, int ACT, bool PLANES>
 int launch_one(const Fp32TcArgs &a, cudaStream_t s)
 {
-    const size_t smem = tmem_smem(FT_STAGES * (size_t)(FT_A_BYTES + 2 * BN * 128) + 2 * 128 * (BN < 64 ? 64 : 128) + sizeof(FtShared), FT_TMEM);
+    const size_t smem = tmem_smem(FT_STAGES * (size_t)(FT_A_BYTES + 3 * BN * 64) + 2 * 128 * (BN < 64 ? 64 : 128) + sizeof(FtShared), FT_TMEM);
     DNB_CUDA(cudaFuncSetAttribute(conv_fp32_tc_kernel<BN, ACT, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

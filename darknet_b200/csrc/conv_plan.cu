@@ -18,28 +18,27 @@ enum { K_TC_TF32 = 0, K_TC_BF16 = 1, K_DIRECT = 2, K_XNOR = 3 };
 static const char *const kKernelNames[] = {"tc_tf32", "tc_bf16", "direct_fp32", "xnor_popc"};
 static const char kXnorTcName[] = "xnor_tc";
 
-// Layers of full-precision plans that may run as three TF32 products on the tensor cores (conv_fp32_tc.cu): sums of 128 products and
-// more, where they are clearly no further from 64-bit sums than the CUDA-core kernel's, which rounds at every product (at 64 they are level).
+// Layers of full-precision plans that may run as products of three bf16 parts on the tensor cores (conv_fp32_tc.cu): sums of 128 products and
+// more, which are less far from 64-bit sums than the CUDA-core kernel's, which rounds at every product.
 // Measured as the root mean square of the error over that of the layer, CUDA cores / tensor cores, for K products, in units of 1e-7:
-//   K = 16  0.80 / 1.02     K = 32  1.06 / 1.29     K = 64  1.45 / 1.30     K = 144  2.1 / 1.2     K = 576  4.3 / 1.5     K = 4608  11.4 / 2.4
-// (summed in TMEM over 64 channels at a time instead of 32: 3.6 at any of these, over 128: 7.8).
+//   K = 128  2.0 / 0.70     K = 144  2.1 / 0.73     K = 576  4.3 / 0.99     K = 2304  8.5 / 1.7     K = 4608  11.4 / 2.2
 static bool fp32_tc_covers(const ConvGeom &g)
 {
     return g.groups == 1 && g.stride <= 2 && g.c >= 8 && g.c * g.size * g.size >= 128 && (long long)g.batch * g.h * g.w < (1LL << 31);
 }
 
-// Whether they should.  Microseconds of either kernel, measured on B200: a step of 32 channels of a tap takes a tile 0.72 on the tensor
-// cores (copies: the copy of a Darknet tensor comes on top); a block of the CUDA-core kernel's large tiles 64 ns a product where four share
+// Whether they should.  Microseconds of either kernel, measured on B200: a step of 32 channels of a tap takes a tile 1.04 on the tensor
+// cores, 0.75 where it has up to 64 filters (copies: the copy of a Darknet tensor comes on top); a block of the CUDA-core kernel's large tiles 64 ns a product where four share
 // an SM, one of its small ones 17.5 and 11.5 more for every other block there, its slabs of up to 16 filters 6 a product and filter.
-// 8 x 64 x 104 x 104 -> 128, 3x3: 317 -> 85 us (352 -> 97 from Darknet's layout); 1 x 512 x 13 x 13 -> 1024 133 -> 96; 8 x 100 x 38 x 38
-// -> 70, stride 2, from Darknet's layout would be 27 -> 34.  DNB_FP32_TC: 0 never, 1 whenever it can.
+// 8 x 64 x 104 x 104 -> 128, 3x3: 316 -> 107 us (352 -> 118 from Darknet's layout); 32 x 64 x 104 x 104 -> 64 602 -> 272; 8 x 100 x 38 x 38
+// -> 70, stride 2, from Darknet's layout would be 27 -> 42.  DNB_FP32_TC: 0 never, 1 whenever it can.
 static bool fp32_tc_pays(const ConvGeom &g, bool copies)
 {
     if (const char *e = getenv("DNB_FP32_TC")) return atoi(e) != 0;
     const double npix = (double)g.batch * g.out_h * g.out_w, K = (double)g.c * g.size * g.size, sms = sm_count();
     const int bn = g.n <= 32 ? 32 : g.n <= 64 ? 64 : 128;
     const double tiles = ceil(npix / 128) * ceil((double)g.n / bn);
-    double tc = 6 + ceil(tiles / sms) * (0.72 * g.size * g.size * ((g.c + 31) / 32) + 0.012 * bn);
+    double tc = 6 + ceil(tiles / sms) * ((bn <= 64 ? 0.75 : 1.04) * g.size * g.size * ((g.c + 31) / 32) + 0.012 * bn);
     if (copies) tc += 3 + 8.0 * g.batch * g.c * g.h * g.w / 5e6;
     double direct;
     if (g.n <= 16 || (g.size != 1 && g.size != 3)) direct = 5 + K * 0.006 * (g.n < 4 ? 4 : g.n) * ceil(npix / 128 / sms);
@@ -148,7 +147,7 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
     else if (p->fp32_tc && p->ft_x_ptr)
-        snprintf(buf, len, "%s three_tf32_products bn=%d tile=%dx%dx%d tiles=%d", dnb_conv_plan_kernel(p), p->ft.bn, p->ft.wt, p->ft.ht, p->ft.bt, p->ft.total_tiles);
+        snprintf(buf, len, "%s three_bf16_parts bn=%d tile=%dx%dx%d tiles=%d", dnb_conv_plan_kernel(p), p->ft.bn, p->ft.wt, p->ft.ht, p->ft.bt, p->ft.total_tiles);
     else
         snprintf(buf, len, "%s", dnb_conv_plan_kernel(p));
     return DNB_OK;
@@ -198,27 +197,21 @@ __global__ void repack_tc_kernel(const float *__restrict__ w, T *__restrict__ ou
     }
 }
 
-// the same layout twice: the weights rounded to TF32, and what the rounding left, rounded to TF32.  A status word behind them starts at 0.
-__global__ void split_weights_kernel(const float *__restrict__ w, float *__restrict__ out, int n, int c, int taps, int n_pad, int c_pad, int *status)
+// [c_blocks][taps][3][n_pad][32]: the weights as sums of three bf16 numbers, each the nearest to what the ones before it leave (the last
+// one exactly that).  A status word behind them starts at 0.
+__global__ void split_weights_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ out, int n, int c, int taps, int n_pad, int c_blocks, int *status)
 {
     if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
-    const size_t half = (size_t)taps * n_pad * c_pad;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < half; i += (size_t)gridDim.x * blockDim.x) {
-        const int cc = (int)(i % c_pad);
-        const size_t r = i / c_pad;
-        const int f = (int)(r % n_pad), t = (int)(r / n_pad);
-        float hi = 0.f, lo = 0.f;
-        if (f < n && cc < c) {
-            const float v = __ldg(w + ((size_t)f * c + cc) * taps + t);
-            uint32_t u = __float_as_uint(v);
-            if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & ~0x1fffu;
-            hi = __uint_as_float(u);
-            u = __float_as_uint(v - hi);
-            if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & ~0x1fffu;
-            lo = __uint_as_float(u);
+    const size_t part = (size_t)n_pad * 32, total = part * taps * c_blocks;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t step = i / part, r = i - step * part;
+        const int cc = (int)(step / taps) * 32 + (int)(r & 31), t = (int)(step % taps), f = (int)(r >> 5);
+        float v = f < n && cc < c ? __ldg(w + ((size_t)f * c + cc) * taps + t) : 0.f;
+        for (int k = 0; k < 3; ++k) {
+            const __nv_bfloat16 h = __float2bfloat16_rn(v);
+            out[(3 * step + k) * part + r] = h;
+            v -= __bfloat162float(h);
         }
-        out[i] = hi;
-        out[half + i] = lo;
     }
 }
 
@@ -348,16 +341,17 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
         repack_tc_kernel<__nv_bfloat16><<<grid_of(total), 256>>>(raw, dev, d.n, d.c, taps, p->n_pad, p->c_pad);
     } else if (p->kernel == K_DIRECT) {
         const size_t total = (size_t)d.groups * K * p->npg_pad;
-        // one allocation: the CUDA-core kernel's weights, and for the tensor cores their halves and the status word
-        const size_t first = (total + 63) / 64 * 64, half = p->fp32_tc && !p->keep_k_order ? (size_t)taps * p->n_pad * p->c_pad : 0;
+        // one allocation: the CUDA-core kernel's weights, and for the tensor cores their three parts and the status word
+        const int c_blocks = (d.c + 31) / 32;
+        const size_t first = (total + 63) / 64 * 64, parts = p->fp32_tc && !p->keep_k_order ? (size_t)c_blocks * taps * 3 * p->n_pad * 32 : 0;   // bf16 values
         if (p->status_in_block) { p->status = nullptr; p->status_in_block = false; }
-        DNB_TRY(device_alloc(&p->w_direct, half ? first + 2 * half + 1 : total));
+        DNB_TRY(device_alloc(&p->w_direct, parts ? first + parts / 2 + 1 : total));
         repack_direct_kernel<<<grid_of(total), 256>>>(raw, p->w_direct, d.groups, npg, K, p->npg_pad);
-        if (half) {
-            p->w_halves = p->w_direct + first;
+        if (parts) {
+            p->w_parts = reinterpret_cast<__nv_bfloat16 *>(p->w_direct + first);
             int *word = nullptr;
-            if (!p->status) { word = p->status = reinterpret_cast<int *>(p->w_halves + 2 * half); p->status_in_block = true; }
-            split_weights_kernel<<<grid_of(half), 256>>>(raw, p->w_halves, d.n, d.c, taps, p->n_pad, p->c_pad, word);
+            if (!p->status) { word = p->status = reinterpret_cast<int *>(p->w_parts + parts); p->status_in_block = true; }
+            split_weights_kernel<<<grid_of(parts / 3), 256>>>(raw, p->w_parts, d.n, d.c, taps, p->n_pad, c_blocks, word);
         }
     } else {
         DNB_TRY(device_alloc(&p->w_bits, (size_t)d.n * taps * p->cwords));
@@ -575,8 +569,8 @@ static int build_fp32_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhw
     Fp32TcArgs &a = p->ft;
     ConvGeom g = p->g;
     a.taps = g.size * g.size;
-    a.c_blocks = (p->c_pad + 31) / 32;
-    a.last_slices = (p->c_pad - 32 * (a.c_blocks - 1)) / 8;
+    a.c_blocks = (g.c + 31) / 32;
+    a.last_slices = (g.c - 32 * (a.c_blocks - 1) + 15) / 16;
     a.bn = p->n_pad <= 32 ? 32 : p->n_pad <= 64 ? 64 : 128;
     a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
     a.planes = x->layout == DNB_NCHW ? 1 : 0;
@@ -600,10 +594,11 @@ static int build_fp32_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhw
     a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
     const uint32_t box[4] = {32u, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
     if (!a.planes) DNB_TRY(encode_input_maps(a.tmx, g, x, 0, 4, p->c_pad, box, 128));
-    uint64_t dims[3] = {(uint64_t)p->c_pad, (uint64_t)p->n_pad, (uint64_t)(2 * a.taps)};
-    uint64_t strides[2] = {(uint64_t)p->c_pad * 4, (uint64_t)p->c_pad * 4 * p->n_pad};
-    uint32_t wbox[3] = {32u, (uint32_t)a.bn, 1u};
-    DNB_TRY(encode_tensor_map(&a.tmw, 0, 3, p->w_halves, dims, strides, wbox, 128));
+    const uint64_t row = 64;   // 32 channels of one part
+    uint64_t dims[4] = {32u, (uint64_t)p->n_pad, 3u, (uint64_t)a.taps * a.c_blocks};
+    uint64_t strides[3] = {row, row * p->n_pad, row * p->n_pad * 3};
+    uint32_t wbox[4] = {32u, (uint32_t)a.bn, 3u, 1u};
+    DNB_TRY(encode_tensor_map(&a.tmw, 1, 4, p->w_parts, dims, strides, wbox, 64));
     if (y_nhwc) {
         const size_t opix = (size_t)y_cpitch * 4;
         const int n8 = round_up(g.n, 8), cols = a.bn / 2 < 32 ? a.bn / 2 : 32;

@@ -62,8 +62,12 @@ typedef enum dnb_activation {
 typedef enum dnb_mode {
     DNB_MODE_TF32 = 0,  /* fp32 storage, TF32 tensor-core products, fp32 accumulate */
     DNB_MODE_BF16 = 1,  /* bf16 storage between layers, fp32 accumulate             */
-    DNB_MODE_FP32 = 2   /* fp32 FMA on the CUDA cores (no tensor cores): slow, for
-                           narrow layers and as an exact-arithmetic cross-check     */
+    DNB_MODE_FP32 = 2   /* fp32 storage, products and sums: fp32 FMA on the CUDA cores,
+                           or, for layers that gain by it, every operand as the exact
+                           sum of three bf16 numbers on the tensor cores, partial sums
+                           added in fp32 (no further from exact sums than the FMAs; the
+                           order of the additions is another).  DNB_FP32_TC=0 in the
+                           environment keeps all layers on the CUDA cores.            */
 } dnb_mode;
 
 typedef enum dnb_layout { DNB_NCHW = 0, DNB_NHWC = 1 } dnb_layout;
@@ -205,7 +209,8 @@ int dnb_conv_plan_check_status(dnb_conv_plan *plan);
 int dnb_conv_plan_set_diagnostics(dnb_conv_plan *plan, long long wait_limit_cycles, int debug_bits);
 
 /* Name of the kernel a plan dispatches to ("tc_tf32", "tc_bf16", "direct_fp32",
- * "xnor_popc"); static storage. */
+ * "xnor_tc", "xnor_popc"); static storage.  "direct_fp32" is every FP32-mode, grouped and
+ * first layer; dnb_conv_plan_describe tells which of those use the tensor cores. */
 const char *dnb_conv_plan_kernel(const dnb_conv_plan *plan);
 
 /* One line about the plan for logs and tests, written to buf (at most len bytes with the

@@ -33,7 +33,7 @@ def test_fp32_gemm_tiles(name, layouts):
     parity(got, oracle_conv(case), 1e-5)
 
 
-FP32_SPLIT = {   # three TF32 products: tiles of 32, 64 and 128 filters, ragged maps, K of one step and of a part of one, odd filters
+FP32_SPLIT = {   # three bf16 parts: tiles of 32, 64 and 128 filters, ragged maps, K of one step and of a part of one, odd filters
     "32_filters_15_channels": dict(b=2, c=15, h=9, w=13, n=18, size=3),
     "64_filters_stride2_odd_map": dict(b=3, c=40, h=21, w=17, n=50, size=3, stride=2, act="logistic"),
     "128_filters_and_one": dict(b=1, c=33, h=11, w=19, n=129, size=3, act="linear"),
@@ -47,7 +47,7 @@ FP32_SPLIT = {   # three TF32 products: tiles of 32, 64 and 128 filters, ragged 
 @pytest.mark.parametrize("name", list(FP32_SPLIT))
 @pytest.mark.parametrize("layouts", [("nchw", "nchw"), ("nchw", "nhwc"), ("nhwc", "nhwc"), ("both", "nchw")])
 def test_full_precision_on_the_tensor_cores(name, layouts, monkeypatch):
-    """Each product is exact to about 2^-24 of its value and the sums of 32 channels are rounded as fp32 sums are; tolerance as for the
+    """Each product is exact to about 2^-33 of its value and the sums of 32 channels are rounded as fp32 sums are; tolerance as for the
     CUDA-core kernel, and the root mean square of the error against 64-bit sums is no larger than that kernel's (a fifth is the
     spread of layers of a few hundred values)."""
     import numpy as np
@@ -62,7 +62,7 @@ def test_full_precision_on_the_tensor_cores(name, layouts, monkeypatch):
     for knob in ("0", "1"):
         monkeypatch.setenv("DNB_FP32_TC", knob)
         plan, got, second = run_conv(case, dn.MODE_FP32, layout, layouts[1], both=layouts[0] == "both")
-        assert plan.kernel == "direct_fp32" and ("three_tf32_products" in plan.describe()) == (knob == "1"), plan.describe()
+        assert plan.kernel == "direct_fp32" and ("three_bf16_parts" in plan.describe()) == (knob == "1"), plan.describe()
         assert second is None or np.array_equal(got, second)
         parity(got, exact, 1e-5)
         rms[knob] = np.sqrt(((got - exact) ** 2).mean())
@@ -70,6 +70,57 @@ def test_full_precision_on_the_tensor_cores(name, layouts, monkeypatch):
     case["act"] = act
     _, got, _ = run_conv(case, dn.MODE_FP32, layout, layouts[1])
     parity(got, oracle_conv(case), 1e-5)
+
+
+SPARSE = {   # what an output is made of: a product or a few of them among zeros, values of one sign
+    "identity_1x1": dict(b=1, c=128, h=33, w=37, n=128, size=1),
+    "few_inputs": dict(b=2, c=256, h=24, w=25, n=96, size=1),
+    "few_inputs_3x3": dict(b=2, c=40, h=24, w=25, n=64, size=3),
+    "few_weights_3x3": dict(b=2, c=64, h=24, w=25, n=130, size=3),
+    "positive": dict(b=2, c=64, h=24, w=25, n=64, size=3, dist="uniform"),
+    "wide_range": dict(b=2, c=128, h=24, w=25, n=64, size=1),
+}
+
+
+@pytest.mark.parametrize("name", list(SPARSE))
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+def test_full_precision_of_sparse_sums(name, layout, monkeypatch):
+    """Sums of one or a few products are no further from 64 bits than the CUDA cores' (2 % and a tenth: the spread of the root mean square and of the largest error over some
+    1e5 outputs), and a factor of 1 gives the input back to the bit."""
+    import numpy as np
+    import torch
+    case = conv_case(723, **dict(SPARSE[name], act="linear", bn=False))
+    case["biases"][...] = 0
+    g = np.random.default_rng(724)
+    x, w = case["x"], case["w"]
+    K = w.shape[1] * w.shape[2] * w.shape[3]
+    if name.startswith("identity"):
+        w[:, :, 0, 0] = np.eye(128, dtype=np.float32)
+        x *= np.exp2(g.integers(-30, 30, x.shape)).astype(np.float32)
+    elif name.startswith("few_inputs"):
+        x *= g.random(x.shape) < 2.5 / K
+    elif name.startswith("few_weights"):
+        w *= g.random(w.shape) < 2.5 / K
+    elif name == "positive":
+        w[...] = np.abs(w)
+    else:
+        x *= np.exp2(g.integers(-12, 12, x.shape)).astype(np.float32)
+    exact = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(w).double(), padding=case["pad"]).numpy()
+    err = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("DNB_FP32_TC", knob)
+        plan, got, _ = run_conv(case, dn.MODE_FP32, layout, layout)
+        assert (plan.describe() != "direct_fp32") == (knob == "1")
+        d = np.abs(got - exact)
+        some = exact != 0
+        assert not got[~some].any()
+        rel = d[some] / np.abs(exact[some])
+        err[knob] = (float(np.sqrt((d ** 2).mean() / (exact ** 2).mean())), float(d.max() / np.abs(exact).max())) + ((float(np.sqrt((rel ** 2).mean())), float(rel.max())) if "few" in name else ())
+        if name.startswith("identity"):
+            assert np.array_equal(got, x), knob
+    assert err["1"][0] <= 1.02 * err["0"][0] and err["1"][1] <= 1.1 * err["0"][1], err
+    if "few" in name:   # of each output by itself, but for those that cancel
+        assert err["1"][2] <= 1.5 * err["0"][2] or err["1"][3] <= 1.1 * err["0"][3], err
 
 
 def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
@@ -87,7 +138,7 @@ def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
         for knob in ("0", "1"):
             monkeypatch.setenv("DNB_FP32_TC", knob)
             plan, out[knob], _ = run_conv(case, dn.MODE_FP32, "nchw", layout)
-            assert ("three_tf32_products" in plan.describe()) == (knob == "1")
+            assert ("three_bf16_parts" in plan.describe()) == (knob == "1")
         odd = ~np.isfinite(out["0"])
         tiny = np.abs(out["0"]) < 2.0 ** -91
         assert odd.any() and tiny.any() and np.array_equal(np.isfinite(out["1"]), ~odd)
