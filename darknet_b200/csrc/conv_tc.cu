@@ -1141,9 +1141,16 @@ int encode_tensor_map(CUtensorMap *map, int elem_kind, int rank, void *base, con
     CUtensorMapSwizzle sw = swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                             : swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
     const CUtensorMapDataType dt = elem_kind == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : (elem_kind == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
-    CUresult r = fn(map, dt, (cuuint32_t)rank, base,
-                    d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&]() {
+        return fn(map, dt, (cuuint32_t)rank, base, d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread's first call: the runtime would make the device's context its own on demand, the driver does not
+        int device = 0;
+        DNB_CUDA(cudaGetDevice(&device));
+        DNB_CUDA(cudaSetDevice(device));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS)
         DNB_FAIL(DNB_ECUDA, "cuTensorMapEncodeTiled failed with %d (rank %d, dims %llu %llu %llu, box %u %u %u, swizzle %d)", (int)r, rank,
                  (unsigned long long)d[0], (unsigned long long)d[1], (unsigned long long)(rank > 2 ? d[2] : 0), bx[0], bx[1], rank > 2 ? bx[2] : 0, swizzle_bytes);

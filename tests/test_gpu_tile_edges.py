@@ -167,6 +167,40 @@ def test_full_precision_wait_expiry(monkeypatch):
     parity(y.cpu().numpy(), oracle_conv(case), 1e-5)
 
 
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_FP32])
+def test_first_call_from_a_new_host_thread(mode, monkeypatch):
+    """A thread that has not used the GPU yet runs a plan for tensors that it has not run for: equal to the same call from here."""
+    import threading
+
+    import torch
+    from gpu_util import dev_nhwc
+    monkeypatch.setenv("DNB_FP32_TC", "1")
+    case = conv_case(726, b=1, c=64, h=19, w=19, n=64, size=3)
+    plan = dn.ConvPlan(1, 64, 19, 19, 64, 3, 1, 1, 1, True, "leaky", False, mode)
+    plan.set_params(case["w"], case["biases"], case["scales"], case["mean"], case["var"])
+    xt, xd = dev_nhwc(case["x"])
+    ys = [torch.zeros(1, 64, 19, 19, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    stream = torch.cuda.current_stream().cuda_stream
+    yd = [dn.as_tensor(y, dn.NCHW) for y in ys]
+    failed = []
+
+    def other():
+        try:
+            plan.forward(xd, yd[0], stream=stream)
+        except dn.DarknetB200Error as e:
+            failed.append(e)
+
+    t = threading.Thread(target=other)
+    t.start()
+    t.join()
+    assert not failed, failed
+    plan.forward(xd, yd[1], stream=stream)
+    torch.cuda.synchronize()
+    assert torch.equal(*ys)
+    parity(ys[0].cpu().numpy(), oracle_conv(case), 1e-2 if mode == dn.MODE_TF32 else 1e-5)
+
+
 @pytest.mark.parametrize("name", ["groups_of_four_channels", "groups_off_four_channel_boundary", "slab_4"])
 def test_grouped_layers_with_bf16_storage(name):
     """A grouped layer of a BF16 network: bf16 in, fp32 sums, bf16 out.  The input is rounded first, so what is left is the
