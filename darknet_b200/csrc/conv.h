@@ -158,7 +158,7 @@ struct alignas(64) Fp32TcArgs {
     int n_pad;
     const float *x;       // the input and its element strides (planes, and sums that are added up again)
     long long xs_b, xs_c, xs_h, xs_w;
-    int planes;           // 1: a 1x1 layer over a Darknet tensor, no tmx
+    int planes;           // 1: the input is a Darknet tensor, no tmx
     const float *w;       // the CUDA-core kernel's weights
     int npg_pad;
     float *y_nhwc, *y_nchw;
@@ -247,9 +247,6 @@ struct dnb_conv_plan {
     dnb::SplitArgs sp;
     bool status_in_block;    // the status word lies behind the weights
     bool fp32_tc;            // this full-precision plan's layer is one that conv_fp32_tc.cu is made for
-    dnb::Fp32TcArgs ft;      // its launch block, for input ft_x_ptr
-    const void *ft_x_ptr, *ft_y_ptr;   // ... and channels-last output ft_y_ptr (or null)
-    int ft_x_cpitch, ft_y_cpitch, ft_layouts;
     int tc_pool;             // the cached launch block writes the pooled output
     int pool_fits;           // conv_pool_fusable's answer: 0 not asked yet, 1 yes, -1 no
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout

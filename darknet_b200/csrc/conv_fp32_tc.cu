@@ -17,8 +17,10 @@
 // * Warp 0 loads a step by TMA: BN x 32 of each part of w, and of a channels-last input 16 KB as it is.  The input goes through
 //   registers anyway to be split, so its parts are written to TMEM, where the MMA takes its A operand from: no shared memory for
 //   them, and half of what the MMAs would read there.
-// * A 1x1 layer over a Darknet tensor needs no channels-last copy of it: its channels are planes, so the threads that split fetch their
-//   pixel's 32 values themselves, coalesced along the plane, the next step's while this one's are multiplied.
+// * A Darknet tensor needs no channels-last copy: its channels are planes, so the threads that split fetch their pixel's 32 values
+//   themselves, along the plane's rows, the next step's while this one's are multiplied.  The ring then holds filters only, and what
+//   is left of an SM's 256 KB caches the rows, which the nine taps of a block of channels read one after the other.  No scratch, no
+//   allocation, no state but the plan's weights: a plan may run on several streams and threads at once, and under capture as without.
 // * Warps 4-11 split, one half of them the even steps, the other the odd ones: a thread takes its pixel's row, writes 16 columns of
 //   each part.  (Four warps for all steps: 110 us where eight took 80, 8 x 64 x 104 x 104 -> 128, 3x3; a step's way through a
 //   warp is all latency.)
@@ -94,6 +96,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+__device__ const float ft_zero = 0.f;   // what a tap outside the image reads: 32 predicates a step cost more than 32 loads of it (32 x 64 x 104 x 104 -> 64: 373 us, 289 without)
+
 // Two values' nearest bf16 as one word (first in the low half), and what is left of them.  An infinity leaves a NaN.
 __device__ __forceinline__ uint32_t take_bf16(float &a, float &b)
 {
@@ -147,13 +151,13 @@ __device__ __forceinline__ float apply(float x, int act)
     return ACT == DNB_LINEAR ? x : activate_fast(x, act);
 }
 
-// BN: filters per tile; PLANES: a 1x1 layer over a Darknet tensor.
+// BN: filters per tile; PLANES: the input is a Darknet tensor.
 template <int BN, int ACT, bool PLANES>
 __global__ void __launch_bounds__(FT_THREADS, 1)
 conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr uint32_t B_BYTES = BN * 64, STAGE = FT_A_BYTES + 3 * B_BYTES;   // 32 channels of one part of w; a stage
+    constexpr uint32_t B_BYTES = BN * 64, A_BYTES = PLANES ? 0 : FT_A_BYTES, STAGE = A_BYTES + 3 * B_BYTES;   // 32 channels of one part of w; a stage
     constexpr int SLOTS = FT_SLOTS<BN>;
     constexpr int COLS = BN / 2, LD = COLS < 32 ? COLS : 32;   // filters of one half of the summing warps, columns of a TMEM read and of a staged row
     constexpr int ROW = LD * 4;
@@ -227,7 +231,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
                         const uint32_t bar = full0 + 8 * stage, slot = ring + stage * STAGE;
                         mbar_expect_tx(bar, PLANES ? 3 * B_BYTES : STAGE);
                         if (!PLANES) tma_load_4d(slot, mx, bar, cb * 32, ow0 + qw, oh0 + qh, b0);
-                        tma_load_4d(slot + FT_A_BYTES, &a.tmw, bar, 0, n0, 0, cb * taps + tap);   // three tiles of BN rows, one of each part
+                        tma_load_4d(slot + A_BYTES, &a.tmw, bar, 0, n0, 0, cb * taps + tap);   // three tiles of BN rows, one of each part
                     }
                     if (++stage == FT_STAGES) { stage = 0; phase ^= 1; }
                     if (++kw == ksize) { kw = 0; ++kh; }
@@ -237,7 +241,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
     } else if (warp == 1) {
         // ---------------- MMAs
         const uint32_t idesc = mma_idesc<MMA_BF16>(128u, (uint32_t)BN);
-        const uint64_t b_desc0 = make_smem_desc(ring + FT_A_BYTES, 64);
+        const uint64_t b_desc0 = make_smem_desc(ring + A_BYTES, 64);
         int stage = 0, slot = 0, acc = 0, run = 0;
         uint32_t phase = 0, slot_phase = 0, acc_phase = 0, small_phase = 0;
         bool ok = true;
@@ -288,20 +292,46 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         const int mine = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
         const long long count = (long long)mine * steps;
-        const int channels = a.g.c;
+        // PLANES: this thread's 32 values of a step, zero beyond the image and the channels; steps are asked for in order
+        const int channels = a.g.c, ksize = a.g.size, img_h = a.g.h, img_w = a.g.w;
         const long long xs_c = a.xs_c;
         float x[PLANES ? 32 : 1];
-        // PLANES: this thread's 32 values of a step, zero beyond the plane and the channels; steps are asked for in order
-        int tile = blockIdx.x, in_tile = warp < 8 ? 0 : 1;
-        auto fetch = [&]() {
-            while (in_tile >= steps) { in_tile -= steps; tile += gridDim.x; }
-            const int pt = tile / n_tiles, pix = pt % tiles_w * wt + m % wt, b = pt / (tiles_w * tiles_h) * bt + m / (wt * ht), c0 = 32 * in_tile;
-            const float *p = a.x + (long long)b * a.xs_b + c0 * xs_c + pix;
-            const int live = pix < a.g.w && m / wt % ht == 0 && b < a.g.batch ? channels - c0 : 0;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) x[PLANES ? j : 0] = j < live ? __ldg(p + j * xs_c) : 0.f;
-            in_tile += 2;
+        int tile = blockIdx.x, cb = 0, kh = 0, kw = 0, ih0 = 0, iw0 = 0;
+        const float *image = nullptr;     // null outside the output
+        auto at_tile = [&]() {
+            const int pt = tile / n_tiles;
+            const int ow = pt % tiles_w * wt + m % wt, oh = pt / tiles_w % tiles_h * ht + m / wt % ht, b = pt / (tiles_w * tiles_h) * bt + m / (wt * ht);
+            ih0 = oh * a.g.stride - a.g.pad; iw0 = ow * a.g.stride - a.g.pad;
+            image = ow < a.g.out_w && oh < a.g.out_h && b < a.g.batch ? a.x + (long long)b * a.xs_b : nullptr;
         };
+        auto advance = [&]() {            // one step
+            if (++kw < ksize) return;
+            kw = 0;
+            if (++kh < ksize) return;
+            kh = 0;
+            if (++cb < c_blocks) return;
+            cb = 0;
+            tile += gridDim.x;
+            at_tile();
+        };
+        auto fetch = [&]() {
+            const int ih = ih0 + kh, iw = iw0 + kw;
+            const bool in = image != nullptr && (unsigned)ih < (unsigned)img_h && (unsigned)iw < (unsigned)img_w;
+            const float *p = in ? image + (cb * 32 * xs_c + ih * a.xs_h + iw) : &ft_zero;
+            const long long next = in ? xs_c : 0;
+            if (cb * 32 + 32 <= channels) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j, p += next) x[PLANES ? j : 0] = __ldg(p);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j, p += next) x[PLANES ? j : 0] = cb * 32 + j < channels ? __ldg(p) : 0.f;
+            }
+            advance(); advance();
+        };
+        if (PLANES) {
+            at_tile();
+            if (warp >= 8) advance();
+        }
         if (PLANES && (warp < 8 ? 0 : 1) < count) fetch();
         for (long long it = warp < 8 ? 0 : 1; it < count; it += 2) {
             const int stage = (int)it & (FT_STAGES - 1), slot = (int)it & (SLOTS - 1);
@@ -329,11 +359,11 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
             tc_fence_after();
 #pragma unroll
             for (int i = 0; i < 3; ++i) tmem_st16(dst + 16 * i, part[i]);
-            if (PLANES && it + 2 < count) fetch();
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(split0 + 8 * slot);
+            if (PLANES && it + 2 < count) fetch();
         }
     } else {
         // ---------------- sums and epilogue
@@ -455,8 +485,12 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
 template <int BN, int ACT, bool PLANES>
 int launch_one(const Fp32TcArgs &a, cudaStream_t s)
 {
-    const size_t smem = tmem_smem(FT_STAGES * (size_t)(FT_A_BYTES + 3 * BN * 64) + 2 * 128 * (BN < 64 ? 64 : 128) + sizeof(FtShared), FT_TMEM);
-    DNB_CUDA(cudaFuncSetAttribute(conv_fp32_tc_kernel<BN, ACT, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
+    // The launch asks for no more shared memory than it uses, unlike the other kernels with TMEM (tmem_smem): its 61440 registers already
+    // keep every kernel that allocates columns off its SM.
+    static_assert(FT_THREADS * 96 + 128 * 40 > 65536, "no other CTA of four warps beside it");
+    const size_t smem = FT_STAGES * (size_t)((PLANES ? 0 : FT_A_BYTES) + 3 * BN * 64) + 2 * 128 * (BN < 64 ? 64 : 128) + sizeof(FtShared);
+    DNB_CUDA(cudaFuncSetAttribute(conv_fp32_tc_kernel<BN, ACT, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DNB_CUDA(cudaFuncSetAttribute(conv_fp32_tc_kernel<BN, ACT, PLANES>, cudaFuncAttributePreferredSharedMemoryCarveout, (int)((smem + 1024) * 100 / (228 * 1024) + 1)));
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;

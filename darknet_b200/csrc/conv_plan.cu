@@ -27,24 +27,28 @@ static bool fp32_tc_covers(const ConvGeom &g)
     return g.groups == 1 && g.stride <= 2 && g.c >= 8 && g.c * g.size * g.size >= 128 && (long long)g.batch * g.h * g.w < (1LL << 31);
 }
 
-// Whether they should.  Microseconds of either kernel, measured on B200: a step of 32 channels of a tap takes a tile 1.04 on the tensor
-// cores, 0.75 where it has up to 64 filters (copies: the copy of a Darknet tensor comes on top); a block of the CUDA-core kernel's large tiles 64 ns a product where four share
-// an SM, one of its small ones 17.5 and 11.5 more for every other block there, its slabs of up to 16 filters 6 a product and filter.
-// 8 x 64 x 104 x 104 -> 128, 3x3: 316 -> 107 us (352 -> 118 from Darknet's layout); 32 x 64 x 104 x 104 -> 64 602 -> 272; 8 x 100 x 38 x 38
-// -> 70, stride 2, from Darknet's layout would be 27 -> 42.  DNB_FP32_TC: 0 never, 1 whenever it can.
-static bool fp32_tc_pays(const ConvGeom &g, bool copies)
+static int fp32_tc_filters(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; }   // of a tile
+
+// Whether they should: for either layout, so that a plan's sums are the same in both.  Microseconds of either kernel, measured on B200: a step of
+// 32 channels of a tap takes a tile of 128 filters 1.04 on the tensor cores, of 64 0.75, of 32 0.59; a block of the CUDA-core kernel's large tiles of 64
+// filters 64 ns a product where four share an SM, of 32 filters 34 and 50 more, one of its small ones 17.5 and 11.5 more for every other block
+// there, its slabs of up to 16 filters 6 a product and filter.  Of 208 launches between 10 us and 1 ms 199 take the faster kernel, or one within 5 %
+// of it; the worst choice was 1.17 times the other's time.  8 x 64 x 104 x 104 -> 128, 3x3: 316 -> 108 us, from Darknet's layout 352 -> 113; 32 x 64 x 104 x 104
+// -> 64 676 -> 284; 8 x 100 x 38 x 38 -> 70, stride 2, would be 27 -> 42.  DNB_FP32_TC: 0 never, 1 whenever it can.
+static bool fp32_tc_pays(const ConvGeom &g)
 {
     if (const char *e = getenv("DNB_FP32_TC")) return atoi(e) != 0;
     const double npix = (double)g.batch * g.out_h * g.out_w, K = (double)g.c * g.size * g.size, sms = sm_count();
-    const int bn = g.n <= 32 ? 32 : g.n <= 64 ? 64 : 128;
+    const int bn = fp32_tc_filters(g.n);
     const double tiles = ceil(npix / 128) * ceil((double)g.n / bn);
-    double tc = 6 + ceil(tiles / sms) * ((bn <= 64 ? 0.75 : 1.04) * g.size * g.size * ((g.c + 31) / 32) + 0.012 * bn);
-    if (copies) tc += 3 + 8.0 * g.batch * g.c * g.h * g.w / 5e6;
+    const double tc = 6 + ceil(tiles / sms) * ((bn == 32 ? 0.59 : bn == 64 ? 0.75 : 1.04) * g.size * g.size * ((g.c + 31) / 32) + 0.012 * bn);
     double direct;
-    if (g.n <= 16 || (g.size != 1 && g.size != 3)) direct = 5 + K * 0.006 * (g.n < 4 ? 4 : g.n) * ceil(npix / 128 / sms);
-    else if (ceil(npix / 128) * ceil(g.n / (g.n > 32 ? 64.0 : 32.0)) >= 2 * sms) {
+    if (g.n <= 16 || (g.size != 1 && g.size != 3)) {
+        const int slab = g.n < 4 ? 4 : g.n > 16 ? 16 : g.n;
+        direct = 5 + K * 0.006 * slab * ceil(ceil(npix / 128) * ((g.n + 15) / 16) / sms);
+    } else if (ceil(npix / 128) * ceil(g.n / (g.n > 32 ? 64.0 : 32.0)) >= 2 * sms) {
         const double b = ceil(npix / 128) * ceil(g.n / (g.n > 32 ? 64.0 : 32.0)) / sms;
-        direct = 6 + K * (g.n <= 32 ? 0.052 * b : b < 4 ? 0.04 + 0.05 * ceil(b) : 0.064 * b);
+        direct = 6 + K * (g.n <= 32 ? 0.05 + 0.034 * b : b < 4 ? 0.04 + 0.05 * ceil(b) : 0.064 * b);
     }
     else direct = 5 + K * (0.006 + 0.0115 * ceil(ceil(npix / 32) * ceil(g.n / 32.0) / sms));
     return tc < direct;
@@ -88,7 +92,7 @@ extern "C" int dnb_conv_plan_create(const dnb_conv_desc *d, int mode, dnb_conv_p
     // RGB first layers of the TF32 / BF16 modes: tensor cores, rows read from the patch in shared memory (DNB_STEM_TC=0 keeps the FP32 kernel)
     const char *stem_env = getenv("DNB_STEM_TC");
     p->stem_tc = p->kernel == K_DIRECT && mode != DNB_MODE_FP32 && !d->xnor && conv_stem_tc_covers(p->g) && !(stem_env && atoi(stem_env) == 0);
-    p->fp32_tc = p->kernel == K_DIRECT && mode == DNB_MODE_FP32 && fp32_tc_covers(p->g) && fp32_tc_pays(p->g, false);
+    p->fp32_tc = p->kernel == K_DIRECT && mode == DNB_MODE_FP32 && fp32_tc_covers(p->g) && fp32_tc_pays(p->g);
     // xnor layers: int8 sign tensors through the tensor cores (kind::i8, exact int32 sums) unless DNB_XNOR_TC=0 asks
     // for the bit-packed popcount kernel; strides above 2 have no lattice maps and stay with the popcount kernel
     {
@@ -109,7 +113,7 @@ dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch)
     q->borrowed = true;
     q->x_nhwc_scratch = nullptr; q->x_bits = nullptr; q->x_i8 = nullptr;
     q->x_nhwc_bytes = q->x_bits_bytes = q->x_i8_bytes = 0;
-    q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = q->ft_x_ptr = nullptr;
+    q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = nullptr;
     q->sign_consumer = nullptr; q->signs_given = false; q->signs_of = nullptr;
     return q;
 }
@@ -146,8 +150,8 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
-    else if (p->fp32_tc && p->ft_x_ptr)
-        snprintf(buf, len, "%s three_bf16_parts bn=%d tile=%dx%dx%d tiles=%d", dnb_conv_plan_kernel(p), p->ft.bn, p->ft.wt, p->ft.ht, p->ft.bt, p->ft.total_tiles);
+    else if (p->fp32_tc && !p->keep_k_order)
+        snprintf(buf, len, "%s three_bf16_parts bn=%d", dnb_conv_plan_kernel(p), fp32_tc_filters(p->d.n));
     else
         snprintf(buf, len, "%s", dnb_conv_plan_kernel(p));
     return DNB_OK;
@@ -370,7 +374,7 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
     DNB_CUDA(cudaDeviceSynchronize());   // the staging copy is released on return
     p->params_set = true;
     // The launch block caches a tensor map over the weights just replaced: have the next forward rebuild it.
-    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = p->ft_x_ptr = nullptr;
+    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = nullptr;
     return DNB_OK;
 }
 
@@ -382,7 +386,7 @@ extern "C" int dnb_conv_plan_set_diagnostics(dnb_conv_plan *p, long long wait_li
     if (!p || wait_limit_cycles < 0) DNB_FAIL(DNB_EINVAL, "conv diagnostics: bad argument");
     p->wait_limit = wait_limit_cycles;
     p->debug_bits = debug_bits;
-    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = p->ft_x_ptr = nullptr;
+    p->tc_x_ptr = p->tc_y_ptr = p->tc_res_ptr = nullptr;
     return DNB_OK;
 }
 
@@ -548,33 +552,17 @@ static int encode_weight_map(CUtensorMap *map, const dnb_conv_plan *p, int kind,
     return encode_tensor_map(map, kind, 3, kind == 2 ? (void *)p->w_i8 : p->w_tc, dims, strides, box, row_bytes);
 }
 
-// Room for the channels-last copy of a Darknet tensor.  False where there is no memory, or where the stream is being captured and
-// nothing can be allocated: the CUDA-core kernel needs none.
-static bool fp32_tc_room(dnb_conv_plan *p, cudaStream_t s)
+// The launch block is made for each call, not kept: two streams or threads may have the same plan in use.
+static int build_fp32_tc_args(const dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_cpitch, float *y_nchw, const ConvEpilogue &ep, Fp32TcArgs &a)
 {
-    if (p->x_nhwc_bytes) return true;   // a plan's need is always the same
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    const size_t need = (size_t)p->g.batch * p->g.h * p->g.w * p->c_pad * sizeof(float);
-    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone || cudaMalloc(&p->x_nhwc_scratch, need) != cudaSuccess) {
-        cudaGetLastError();
-        p->x_nhwc_scratch = nullptr;
-        return false;
-    }
-    p->x_nhwc_bytes = need;
-    return true;
-}
-
-static int build_fp32_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_cpitch, bool nchw_out)
-{
-    Fp32TcArgs &a = p->ft;
     ConvGeom g = p->g;
     a.taps = g.size * g.size;
     a.c_blocks = (g.c + 31) / 32;
     a.last_slices = (g.c - 32 * (a.c_blocks - 1) + 15) / 16;
-    a.bn = p->n_pad <= 32 ? 32 : p->n_pad <= 64 ? 64 : 128;
+    a.bn = fp32_tc_filters(p->d.n);
     a.n_tiles = (p->n_pad + a.bn - 1) / a.bn;
     a.planes = x->layout == DNB_NCHW ? 1 : 0;
-    const bool by_image = nchw_out || a.planes;
+    const bool by_image = y_nchw || a.planes;
     if (g.size == 1 && g.stride == 1 && g.pad == 0) {   // pixels in one row; of the whole batch where no tensor has planes
         g.w = g.out_w = g.w * g.h * (by_image ? 1 : g.batch);
         g.h = g.out_h = 1;
@@ -607,7 +595,9 @@ static int build_fp32_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhw
         uint32_t ybox[4] = {(uint32_t)cols, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
         DNB_TRY(encode_tensor_map(&a.tmy, 0, 4, y_nhwc, ydims, ystrides, ybox, cols * 4));
     }
-    p->ft_x_ptr = x->data; p->ft_x_cpitch = x->cpitch; p->ft_y_ptr = y_nhwc; p->ft_y_cpitch = y_cpitch; p->ft_layouts = 2 * a.planes + (nchw_out ? 1 : 0);
+    a.y_nhwc = (float *)y_nhwc; a.y_nchw = y_nchw;
+    a.status = p->status;
+    a.ep = ep;
     return DNB_OK;
 }
 
@@ -1141,20 +1131,9 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         const bool rows = (p->keep_k_order || a.xs_h >= (1LL << 31) / 64) && conv_stem_rows_covers(g, y_dtype);
         return rows ? launch_conv_stem_rows(a, s) : launch_conv_stem_tc(a, s);
     }
-    const bool copies = x->layout == DNB_NCHW && !(g.size == 1 && g.stride == 1 && g.pad == 0);
-    if (p->fp32_tc && !p->keep_k_order && x->dtype == DNB_F32 && (!y_nhwc || y_dtype == DNB_F32) && (!copies || (fp32_tc_pays(g, true) && fp32_tc_room(p, s)))) {
-        dnb_tensor xin = *x;
-        if (copies) {
-            xin.data = p->x_nhwc_scratch; xin.layout = DNB_NHWC; xin.cpitch = p->c_pad;
-            DNB_TRY(launch_convert(x, &xin, 0, 0, 0, s));
-        }
-        const int layouts = (xin.layout == DNB_NCHW ? 2 : 0) + (y_nchw ? 1 : 0);
-        if (p->ft_x_ptr != xin.data || p->ft_x_cpitch != xin.cpitch || p->ft_y_ptr != y_nhwc || p->ft_y_cpitch != y_cpitch || p->ft_layouts != layouts)
-            DNB_TRY(build_fp32_tc_args(p, &xin, y_nhwc, y_cpitch, y_nchw != nullptr));
-        Fp32TcArgs &a = p->ft;
-        a.y_nhwc = (float *)y_nhwc; a.y_nchw = y_nchw;
-        a.status = p->status;
-        a.ep = ep;
+    if (p->fp32_tc && !p->keep_k_order && x->dtype == DNB_F32 && (!y_nhwc || y_dtype == DNB_F32)) {
+        Fp32TcArgs a;
+        DNB_TRY(build_fp32_tc_args(p, x, y_nhwc, y_cpitch, y_nchw, ep, a));
         return launch_conv_fp32_tc(a, s);
     }
     if (p->kernel == K_DIRECT) {   // also a first-layer plan asked for Darknet's layout or given bf16 input

@@ -147,6 +147,68 @@ def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
         assert np.abs(out["0"][plain] - out["1"][plain]).max() <= 1e-5 * np.abs(out["0"][plain]).max()
 
 
+@pytest.mark.parametrize("shape", [dict(b=4, c=64, h=52, w=51, n=128, size=3), dict(b=2, c=40, h=61, w=64, n=60, size=3, stride=2), dict(b=4, c=128, h=52, w=52, n=64, size=1)])
+def test_full_precision_plan_in_several_hands(shape, monkeypatch):
+    """One FP32 plan over different Darknet tensors on two streams at once, from two threads at once, and captured before its first plain
+    call: every output is the one of a call by itself, to the bit, and no call takes device memory."""
+    import threading
+
+    import numpy as np
+    import torch
+    monkeypatch.setenv("DNB_FP32_TC", "1")
+    case = conv_case(725, **shape)
+    b, c, h, w = case["x"].shape
+    n, size = case["w"].shape[0], case["w"].shape[2]
+    plan = dn.ConvPlan(b, c, h, w, n, size, case["stride"], case["pad"], 1, True, "leaky", False, dn.MODE_FP32)
+    plan.set_params(case["w"], case["biases"], case["scales"], case["mean"], case["var"])
+    xs = [torch.from_numpy(case["x"] * np.float32(f)).cuda() for f in (1, -2, 3, 0.5)]
+    ys = [torch.empty(b, n, plan.out_h, plan.out_w, device="cuda") for _ in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    forward = lambda i, out: plan.forward(dn.as_tensor(xs[i], dn.NCHW), dn.as_tensor(out, dn.NCHW), stream=streams[i].cuda_stream)  # noqa: E731
+    torch.cuda.synchronize()
+    warm = dn.ConvPlan(b, c, h, w, n, size, case["stride"], case["pad"], 1, True, "leaky", False, dn.MODE_FP32)   # loads the kernel
+    warm.set_params(case["w"], case["biases"], case["scales"], case["mean"], case["var"])
+    warm.forward(dn.as_tensor(xs[0], dn.NCHW), dn.as_tensor(ys[0], dn.NCHW))
+    torch.cuda.synchronize()
+    taken = lambda: -torch.cuda.mem_get_info()[0] - torch.cuda.memory_reserved()  # noqa: E731
+    before = taken()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        forward(0, ys[0])
+    graph.replay()
+    torch.cuda.synchronize()
+    captured = ys[0].clone()
+    want = []
+    for i in range(len(xs)):
+        forward(i, ys[i])
+        torch.cuda.synchronize()
+        want.append(ys[i].clone())
+    assert torch.equal(captured, want[0])
+    parity(want[0].cpu().numpy(), oracle_conv(case), 1e-5)
+    for _ in range(3):
+        for y in ys:
+            y.zero_()
+        torch.cuda.synchronize()
+        for _ in range(8):                                     # calls of two and more streams in flight together
+            for i in range(len(xs)):
+                forward(i, ys[i])
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, v) for y, v in zip(ys, want))
+    for y in ys:
+        y.zero_()
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=lambda i=i: [forward(i, ys[i]) for _ in range(50)]) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    plan.check_status()
+    assert all(torch.equal(y, v) for y, v in zip(ys, want))
+    assert taken() - before < 8 << 20                          # the graph's own; a copy of one input would be 2.6 MB for each stream and call
+    graph.reset()
+
+
 def test_full_precision_wait_expiry(monkeypatch):
     """A withheld operand load: the bounded wait runs out, the call reports it, and the next launch is right."""
     import torch
