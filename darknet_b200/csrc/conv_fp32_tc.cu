@@ -29,8 +29,8 @@
 //   activate and store.  They take the registers that the other warps give up.
 // * A ring of four slots of shared memory for what TMA brings, and one of 48 columns of TMEM each for the split rows: two beside three
 //   accumulators of 128 columns, four beside narrower ones.
-// * A sum that is infinite, not a number, or smaller than the parts can hold is added up again in fp32, product by product, so
-//   what infinities and NaN in the input become is what the CUDA-core kernel makes of them.
+// * A pixel with a sum that is infinite, not a number, or smaller than the parts can hold is added up again in fp32, product by product in
+//   the CUDA-core kernel's order, so what infinities and NaN in the input become is what that kernel makes of them.
 // * Every wait is bounded as in conv_tc.cu.
 #include <cuda.h>
 
@@ -108,23 +108,6 @@ __device__ __forceinline__ uint32_t take_bf16(float &a, float &b)
     return r;
 }
 
-// One output the way the CUDA-core kernel adds it: fp32, in the order c, kh, kw.
-__device__ __forceinline__ float plain_sum(const Fp32TcArgs &a, int b, int oh, int ow, int f)
-{
-    const ConvGeom &g = a.g;
-    float acc = 0.f;
-    const float *w = a.w + f;
-    for (int c = 0; c < g.c; ++c)
-        for (int kh = 0; kh < g.size; ++kh)
-            for (int kw = 0; kw < g.size; ++kw, w += a.npg_pad) {
-                const int ih = oh * g.stride - g.pad + kh, iw = ow * g.stride - g.pad + kw;
-                const bool in = (unsigned)ih < (unsigned)g.h && (unsigned)iw < (unsigned)g.w;
-                const float x = in ? __ldg(a.x + b * a.xs_b + c * a.xs_c + ih * a.xs_h + iw * a.xs_w) : 0.f;
-                acc = fmaf(x, __ldg(w), acc);
-            }
-    return acc;
-}
-
 // Sums whose size says that the parts may not have carried them: infinite, NaN, or below 2^-90 and not zero.
 __device__ __forceinline__ bool out_of_range(float v)
 {
@@ -149,6 +132,134 @@ __device__ __forceinline__ float apply(float x, int act)
 {
     if (ACT == DNB_LEAKY) return fmaxf(x, 0.1f * x);
     return ACT == DNB_LINEAR ? x : activate_fast(x, act);
+}
+
+// Where the sums of pixel m (of 128) and of one half's filters of a tile belong.
+struct FtTile {
+    int n0, ow0, oh0, b0, ow, oh, b;
+    bool inside;
+    __device__ __forceinline__ FtTile(const Fp32TcArgs &a, int tile, int bn, int col0, int m)
+    {
+        const int pt = tile / a.n_tiles;
+        n0 = tile % a.n_tiles * bn + col0;
+        ow0 = pt % a.tiles_w * a.wt; oh0 = pt / a.tiles_w % a.tiles_h * a.ht; b0 = pt / (a.tiles_w * a.tiles_h) * a.bt;
+        ow = ow0 + m % a.wt; oh = oh0 + m / a.wt % a.ht; b = b0 + m / (a.wt * a.ht);
+        inside = ow < a.g.out_w && oh < a.g.out_h && b < a.g.batch;
+    }
+};
+
+// Scale, shift, activation and stores of a finished tile's half.
+template <int BN, int ACT>
+__device__ __forceinline__ void finish_tile(const Fp32TcArgs &a, const FtTile &at, const float (&sum)[BN / 2], uint8_t *staged, int half, int m, bool stored)
+{
+    constexpr int COLS = BN / 2, LD = COLS < 32 ? COLS : 32, ROW = LD * 4;
+    const ConvGeom &g = a.g;
+    const int act = a.ep.activation, n0 = at.n0, real = g.n - n0;
+    const bool stores = m == 0;
+    uint8_t *const my_row = staged + m * ROW;
+    const int q_xor = (m >> (ROW == 128 ? 0 : 1)) & (ROW / 16 - 1);   // the store map's swizzle
+    const size_t plane = (size_t)g.out_h * g.out_w, pix = (size_t)at.oh * g.out_w + at.ow;
+    float *const nchw = a.y_nchw && at.inside ? a.y_nchw + ((size_t)at.b * g.n + n0) * plane + pix : nullptr;
+#pragma unroll
+    for (int c = 0; c < COLS; c += LD) {
+        if (a.y_nhwc && (c > 0 || stored)) {            // the row's last store has been read
+            if (stores) tma_store_wait_read0();
+            meet(half, true);
+        }
+#pragma unroll
+        for (int q = c / 4; q < (c + LD) / 4; ++q) {
+            float v[4];
+            const bool in = n0 + 4 * q < a.n_pad;       // whole quads: n_pad is a multiple of 16
+            const float4 sc = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.scale + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 sf = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.shift + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = 4 * q + e < real ? apply<ACT>(sum[4 * q + e] * scv[e] + sfv[e], act) : 0.f;
+            if (a.y_nhwc) *reinterpret_cast<float4 *>(my_row + (((q - c / 4) ^ q_xor) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+            if (nchw) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (4 * q + e < real) nchw[(size_t)(4 * q + e) * plane] = v[e];
+            }
+        }
+        if (a.y_nhwc) {
+            fence_async_smem();
+            meet(half, true);
+            // the TMA unit clips the box at the tensor's extents: ragged tiles need no predicates
+            if (stores && c < real) { tma_store_4d(&a.tmy, smem_u32(staged), n0 + c, at.ow0, at.oh0, at.b0); tma_store_commit(); }
+        }
+    }
+}
+
+// Rarely: the sums of an odd pixel in the order c, kh, kw, the CUDA-core kernel's over a Darknet tensor, each weight from shared memory, where the half's
+// threads put 32 products' at a time; the other pixels' threads add 0 * w.  (A sum at a time in its own thread, 8 x 64 x 104 x 104 -> 128 full of
+// NaN took 53 ms.  So it takes five times as long as the CUDA-core kernel, which reads a weight for eight pixels.)
+template <int COLS>   // at most 32
+__device__ __noinline__ void add_again(const Fp32TcArgs &a, float *sums, uint8_t *staged, bool odd, int half, int n0, int b, int oh, int ow)
+{
+    const ConvGeom &g = a.g;
+    float sum[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sum[j] = sums[j];
+    float4 *const wk = reinterpret_cast<float4 *>(staged);
+    const int products = g.c * g.size * g.size, ih0 = oh * g.stride - g.pad, iw0 = ow * g.stride - g.pad;
+    const float *const image = a.x + (long long)b * a.xs_b;
+    int k = 0, c = 0, kh = 0, kw = 0;               // of the next input value
+    auto next_x = [&]() {
+        const int ih = ih0 + kh, iw = iw0 + kw;
+        const bool in = odd && k < products && (unsigned)ih < (unsigned)g.h && (unsigned)iw < (unsigned)g.w;
+        const float v = in ? __ldg(image + c * a.xs_c + ih * a.xs_h + iw * a.xs_w) : 0.f;
+        ++k;
+        if (++kw == g.size) { kw = 0; if (++kh == g.size) { kh = 0; ++c; } }
+        return v;
+    };
+    float x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = next_x();
+    for (int k0 = 0; k0 < products; k0 += 32) {
+        meet(half, true);
+        for (int i = threadIdx.x & 127; i < 32 * COLS / 4; i += 128) {
+            const int kk = k0 + i / (COLS / 4), f = n0 + 4 * (i % (COLS / 4));
+            wk[i] = kk < products && f < a.npg_pad ? __ldg(reinterpret_cast<const float4 *>(a.w + (size_t)kk * a.npg_pad + f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        meet(half, true);
+#pragma unroll 1
+        for (int kk = 0; kk < 32; kk += 4) {
+            float later[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) later[u] = next_x();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+#pragma unroll
+                for (int q = 0; q < COLS / 4; ++q) {
+                    const float4 w = wk[(kk + u) * (COLS / 4) + q];
+                    sum[4 * q] = fmaf(x[u], w.x, sum[4 * q]);
+                    sum[4 * q + 1] = fmaf(x[u], w.y, sum[4 * q + 1]);
+                    sum[4 * q + 2] = fmaf(x[u], w.z, sum[4 * q + 2]);
+                    sum[4 * q + 3] = fmaf(x[u], w.w, sum[4 * q + 3]);
+                }
+                x[u] = later[u];
+            }
+        }
+    }
+    meet(half, true);
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sums[j] = sum[j];
+}
+
+// ... and a tile that has such pixels.  A function of its own: its registers are not the kernel's loop's.
+template <int BN, int ACT>
+__device__ __noinline__ void odd_tile(const Fp32TcArgs &a, float *sums, uint8_t *staged, bool odd, int half, int tile, int m, bool stored)
+{
+    constexpr int COLS = BN / 2, LD = COLS < 32 ? COLS : 32;
+    const FtTile at(a, tile, BN, half * COLS, m);
+    if (a.y_nhwc && stored && m == 0) tma_store_wait_read0();
+#pragma unroll 1
+    for (int c = 0; c < COLS; c += LD) add_again<LD>(a, sums + c, staged, odd, half, at.n0 + c, at.b, at.oh, at.ow);
+    float sum[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sum[j] = sums[j];
+    finish_tile<BN, ACT>(a, at, sum, staged, half, m, stored);
 }
 
 // BN: filters per tile; PLANES: the input is a Darknet tensor.
@@ -295,7 +406,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         // PLANES: this thread's 32 values of a step, zero beyond the image and the channels; steps are asked for in order
         const int channels = a.g.c, ksize = a.g.size, img_h = a.g.h, img_w = a.g.w;
         const long long xs_c = a.xs_c;
-        float x[PLANES ? 32 : 1];
+        float x[32];
         int tile = blockIdx.x, cb = 0, kh = 0, kw = 0, ih0 = 0, iw0 = 0;
         const float *image = nullptr;     // null outside the output
         auto at_tile = [&]() {
@@ -321,10 +432,10 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
             const long long next = in ? xs_c : 0;
             if (cb * 32 + 32 <= channels) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j, p += next) x[PLANES ? j : 0] = __ldg(p);
+                for (int j = 0; j < 32; ++j, p += next) x[j] = __ldg(p);
             } else {
 #pragma unroll
-                for (int j = 0; j < 32; ++j, p += next) x[PLANES ? j : 0] = cb * 32 + j < channels ? __ldg(p) : 0.f;
+                for (int j = 0; j < 32; ++j, p += next) x[j] = cb * 32 + j < channels ? __ldg(p) : 0.f;
             }
             advance(); advance();
         };
@@ -338,27 +449,26 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
             if (!mbar_wait(full0 + 8 * stage, (uint32_t)(it / FT_STAGES) & 1, abort_flag, status, FT_WAIT_FULL, 0, limit)) break;
             const uint8_t *row = smem_raw + stage * STAGE + m * 128;
             const uint32_t dst = tmem_base + lane_base + slot * FT_SLOT;
+            if (!PLANES) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float4 f = *reinterpret_cast<const float4 *>(row + ((q ^ q_xor) << 4));
+                    x[4 * q] = f.x; x[4 * q + 1] = f.y; x[4 * q + 2] = f.z; x[4 * q + 3] = f.w;
+                }
+            }
             uint32_t part[3][16];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float v[4];
-                if (PLANES) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) v[e] = x[PLANES ? 4 * q + e : 0];
-                } else {
-                    const float4 f = *reinterpret_cast<const float4 *>(row + ((q ^ q_xor) << 4));
-                    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-                }
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    part[i][2 * q] = take_bf16(v[0], v[1]);
-                    part[i][2 * q + 1] = take_bf16(v[2], v[3]);
-                }
+            for (int j = 0; j < 16; ++j) {
+                part[0][j] = take_bf16(x[2 * j], x[2 * j + 1]);
+                part[1][j] = take_bf16(x[2 * j], x[2 * j + 1]);
             }
             if (!mbar_wait(split_empty0 + 8 * slot, ((uint32_t)(it / SLOTS) & 1) ^ 1, abort_flag, status, FT_WAIT_SPLIT, 0, limit)) break;
             tc_fence_after();
+            tmem_st16(dst, part[0]);
+            tmem_st16(dst + 16, part[1]);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) tmem_st16(dst + 16 * i, part[i]);
+            for (int j = 0; j < 16; ++j) part[2][j] = take_bf16(x[2 * j], x[2 * j + 1]);   // here for the registers
+            tmem_st16(dst + 32, part[2]);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -370,12 +480,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FT_REGS_SUM));
         const int half = warp < 16 ? 0 : 1, col0 = half * COLS;
         const int quarter = warp & 3, m = quarter * 32 + lane;
-        uint8_t *const staged = smem_raw + FT_STAGES * STAGE + half * 128 * ROW, *const my_row = staged + m * ROW;
-        const int q_xor = (m >> (ROW == 128 ? 0 : 1)) & (ROW / 16 - 1);   // the store map's swizzle
-        const bool stores = quarter == 0 && lane == 0;
-        const int wl = m % wt, hl = (m / wt) % ht, bl = m / (wt * ht);
-        const ConvGeom g = a.g;
-        const int act = a.ep.activation;
+        uint8_t *const staged = smem_raw + FT_STAGES * STAGE + half * 128 * ROW;
         int acc = 0;
         uint32_t acc_phase = 0, small_phase = 0;
         bool ok = true, stored = false;
@@ -412,61 +517,21 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
                 small_phase ^= 1;
             }
             if (!meet(half, ok && !*abort_flag)) break;
-            const int n0 = tile % n_tiles * BN + col0, pt = tile / n_tiles;
-            const int ow0 = pt % tiles_w * wt, oh0 = pt / tiles_w % tiles_h * ht, b0 = pt / (tiles_w * tiles_h) * bt;
-            const int ow = ow0 + wl, oh = oh0 + hl, b = b0 + bl;
-            const bool inside = ow < g.out_w && oh < g.out_h && b < g.batch;
-            const size_t plane = (size_t)g.out_h * g.out_w, pix = (size_t)oh * g.out_w + ow;
-            float *nchw = a.y_nchw && inside ? a.y_nchw + ((size_t)b * g.n + n0) * plane + pix : nullptr;
-            const int real = g.n - n0;
-            uint32_t again[(COLS + 31) / 32] = {};              // sums that fp32 has to add up itself
+            const FtTile at(a, tile, BN, col0, m);
+            bool odd = false;
 #pragma unroll
-            for (int c = 0; c < COLS; c += LD) {
-                if (a.y_nhwc && (c > 0 || stored)) {            // the row's last store has been read
-                    if (stores) tma_store_wait_read0();
-                    meet(half, true);
-                }
+            for (int j = 0; j < COLS; ++j) odd = odd || out_of_range(sum[j]);
+            odd = odd && at.inside;
+            if (meet(half, !odd)) finish_tile<BN, ACT>(a, at, sum, staged, half, m, stored);
+            else {
+                float again[COLS];
 #pragma unroll
-                for (int q = c / 4; q < (c + LD) / 4; ++q) {
-                    float v[4];
-                    const bool in = n0 + 4 * q < a.n_pad;       // whole quads: n_pad is a multiple of 16
-                    const float4 sc = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.scale + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float4 sf = in ? __ldg(reinterpret_cast<const float4 *>(a.ep.shift + n0) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float t = sum[4 * q + e];
-                        if (out_of_range(t)) again[q / 8] |= 1u << (4 * (q & 7) + e);
-                        v[e] = 4 * q + e < real ? apply<ACT>(t * scv[e] + sfv[e], act) : 0.f;
-                    }
-                    if (a.y_nhwc) *reinterpret_cast<float4 *>(my_row + (((q - c / 4) ^ q_xor) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
-                    if (nchw) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (4 * q + e < real) nchw[(size_t)(4 * q + e) * plane] = v[e];
-                    }
-                }
-                if (again[c / 32] && inside) {                  // rarely: into the staged row and the plane instead
-                    uint32_t bits = again[c / 32];
-                    while (bits) {
-                        const int j = (c & ~31) + __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        if (j >= real) break;
-                        const float t = apply<ACT>(plain_sum(a, b, oh, ow, n0 + j) * __ldg(a.ep.scale + n0 + j) + __ldg(a.ep.shift + n0 + j), act);
-                        if (a.y_nhwc) *reinterpret_cast<float *>(my_row + ((((j - c) / 4) ^ q_xor) << 4) + 4 * ((j - c) & 3)) = t;
-                        if (nchw) nchw[(size_t)j * plane] = t;
-                    }
-                }
-                if (a.y_nhwc) {
-                    fence_async_smem();
-                    meet(half, true);
-                    // the TMA unit clips the box at the tensor's extents: ragged tiles need no predicates
-                    if (stores && c < real) { tma_store_4d(&a.tmy, smem_u32(staged), n0 + c, ow0, oh0, b0); tma_store_commit(); }
-                }
+                for (int j = 0; j < COLS; ++j) again[j] = odd ? 0.f : sum[j];
+                odd_tile<BN, ACT>(a, again, staged, odd, half, tile, m, stored);
             }
             stored = true;
         }
-        if (stores) tma_store_wait_all();
+        if (quarter == 0 && lane == 0) tma_store_wait_all();
     }
 
     // ---------------- teardown (also the abort path)

@@ -147,6 +147,47 @@ def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
         assert np.abs(out["0"][plain] - out["1"][plain]).max() <= 1e-5 * np.abs(out["0"][plain]).max()
 
 
+@pytest.mark.parametrize("shape", [dict(b=4, c=64, h=52, w=51, n=200, size=3), dict(b=2, c=15, h=33, w=40, n=30, size=3, stride=2), dict(b=3, c=131, h=26, w=27, n=64, size=1)])
+@pytest.mark.parametrize("layouts", [("nchw", "nchw"), ("nchw", "nhwc"), ("nhwc", "nhwc")])
+def test_full_precision_without_finite_sums(shape, layouts, monkeypatch):
+    """Every sum infinite or NaN, and one pixel in a hundred: what the CUDA cores make of it, in a few times their time (not in 60 and more)."""
+    import numpy as np
+    import torch
+    from gpu_util import dev_nchw, dev_nhwc, empty_nchw, empty_nhwc
+    case = conv_case(727, **dict(shape, act="linear", bn=False))
+    g = np.random.default_rng(728)
+    b, c, h, w = case["x"].shape
+    n, size = case["w"].shape[0], case["w"].shape[2]
+    few = case["x"].copy()
+    few[g.random(few.shape) < 0.01 / c] = np.inf
+    every = np.full_like(few, np.nan)
+    every[:, :, ::2] = -np.inf
+    for x in (few, every):
+        out, us = {}, {}
+        for knob in ("0", "1"):
+            monkeypatch.setenv("DNB_FP32_TC", knob)
+            plan = dn.ConvPlan(b, c, h, w, n, size, case["stride"], case["pad"], 1, False, "linear", False, dn.MODE_FP32)
+            plan.set_params(case["w"], case["biases"])
+            xt, xd = dev_nchw(x) if layouts[0] == "nchw" else dev_nhwc(x)
+            yt, yd = (empty_nchw if layouts[1] == "nchw" else empty_nhwc)(b, n, plan.out_h, plan.out_w)
+            times = []
+            for _ in range(3):
+                e0, e1 = torch.cuda.Event(True), torch.cuda.Event(True)
+                e0.record()
+                plan.forward(xd, yd)
+                e1.record()
+                torch.cuda.synchronize()
+                times.append(e0.elapsed_time(e1) * 1e3)
+            plan.check_status()
+            us[knob] = min(times)
+            out[knob] = yt.cpu().numpy()
+        odd = ~np.isfinite(out["0"])
+        assert odd.any() and np.array_equal(np.isfinite(out["1"]), ~odd) and np.array_equal(out["0"][odd], out["1"][odd], equal_nan=True)
+        if not odd.all():
+            parity(out["1"][~odd], out["0"][~odd], 1e-5)
+        assert us["1"] < 8 * us["0"] + 50, us
+
+
 @pytest.mark.parametrize("shape", [dict(b=4, c=64, h=52, w=51, n=128, size=3), dict(b=2, c=40, h=61, w=64, n=60, size=3, stride=2), dict(b=4, c=128, h=52, w=52, n=64, size=1)])
 def test_full_precision_plan_in_several_hands(shape, monkeypatch):
     """One FP32 plan over different Darknet tensors on two streams at once, from two threads at once, and captured before its first plain
