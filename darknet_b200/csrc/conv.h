@@ -159,6 +159,7 @@ struct alignas(64) Fp32TcArgs {
     const float *x;       // the input and its element strides (planes, and sums that are added up again)
     long long xs_b, xs_c, xs_h, xs_w;
     int planes;           // 1: the input is a Darknet tensor, no tmx
+    uint32_t smallest;    // bits of the smallest input, but zero, that the parts stand for
     const float *w;       // the CUDA-core kernel's weights
     int npg_pad;
     float *y_nhwc, *y_nchw;
@@ -247,6 +248,7 @@ struct dnb_conv_plan {
     dnb::SplitArgs sp;
     bool status_in_block;    // the status word lies behind the weights
     bool fp32_tc;            // this full-precision plan's layer is one that conv_fp32_tc.cu is made for
+    uint32_t fp32_smallest;  // ... its smallest input (see there), or 0 where its weights keep it on the CUDA cores
     int tc_pool;             // the cached launch block writes the pooled output
     int pool_fits;           // conv_pool_fusable's answer: 0 not asked yet, 1 yes, -1 no
     int tc_nchw_out;         // the cached launch block was built for a launch that also writes Darknet's layout

@@ -29,8 +29,10 @@
 //   activate and store.  They take the registers that the other warps give up.
 // * A ring of four slots of shared memory for what TMA brings, and one of 48 columns of TMEM each for the split rows: two beside three
 //   accumulators of 128 columns, four beside narrower ones.
-// * A pixel with a sum that is infinite, not a number, or smaller than the parts can hold is added up again in fp32, product by product in
-//   the CUDA-core kernel's order, so what infinities and NaN in the input become is what that kernel makes of them.
+// * Parts and products must be numbers that bf16 and the tensor core's fp32 hold in full.  The threads that split look at what they split: a pixel that has
+//   read a value other than zero below a.smallest (2^-90 over the layer's smallest weight, at least 2^-100: every product is then 2^-90 or more, and
+//   what counts of it, 2^-26, a normal number) is added up again in fp32, product by product in the CUDA-core kernel's order, and so is one with a sum that
+//   is infinite or NaN, which operands beyond bf16's largest number make too.  Layers with weights below 2^-45 run on the CUDA cores.
 // * Every wait is bounded as in conv_tc.cu.
 #include <cuda.h>
 
@@ -61,6 +63,7 @@ struct FtShared {
     uint64_t split[4];             // a step's input rows are in TMEM
     uint64_t split_empty[4];       // ... and the MMAs that read them have retired
     uint64_t acc_full[3], acc_empty[3];   // the large products' two, the small ones'
+    uint32_t tiny[2][2][4];        // of a tile (even and odd ones in turn): pixels that have read a tiny value, by half of the splitting warps and quarter
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -106,13 +109,6 @@ __device__ __forceinline__ uint32_t take_bf16(float &a, float &b)
     a -= __uint_as_float(r << 16);
     b -= __uint_as_float(r & 0xffff0000u);
     return r;
-}
-
-// Sums whose size says that the parts may not have carried them: infinite, NaN, or below 2^-90 and not zero.
-__device__ __forceinline__ bool out_of_range(float v)
-{
-    const uint32_t m = __float_as_uint(v) & 0x7fffffffu;
-    return m - 0x12800000u >= 0x7f800000u - 0x12800000u && m != 0u;
 }
 
 // The 128 threads of one of the two halves that sum meet, and agree on whether to go on.
@@ -403,6 +399,12 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         const int mine = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
         const long long count = (long long)mine * steps;
+        // The smallest value but zero this thread's pixel has read of the tile, as twice its bits less one (zero is then the largest).  A tile has four steps or
+        // more, two of them this half's; its word is written before the last of them is handed on and read with the tile's last sums.  Before it is
+        // written again, two tiles on, a step of the tile between has been added up, by threads that had read the word.
+        const uint32_t bound = 2u * a.smallest - 1u;
+        uint32_t least = ~0u;
+        int left = warp < 8 ? steps : steps - 1, parity = 0;   // steps of the tile from this half's next one on
         // PLANES: this thread's 32 values of a step, zero beyond the image and the channels; steps are asked for in order
         const int channels = a.g.c, ksize = a.g.size, img_h = a.g.h, img_w = a.g.w;
         const long long xs_c = a.xs_c;
@@ -459,6 +461,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
             uint32_t part[3][16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
+                least = __vimin3_u32(least, 2u * __float_as_uint(x[2 * j]) - 1u, 2u * __float_as_uint(x[2 * j + 1]) - 1u);
                 part[0][j] = take_bf16(x[2 * j], x[2 * j + 1]);
                 part[1][j] = take_bf16(x[2 * j], x[2 * j + 1]);
             }
@@ -469,6 +472,13 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
 #pragma unroll
             for (int j = 0; j < 16; ++j) part[2][j] = take_bf16(x[2 * j], x[2 * j + 1]);   // here for the registers
             tmem_st16(dst + 32, part[2]);
+            if ((left -= 2) <= 0) {
+                const uint32_t rows = __ballot_sync(0xffffffffu, least < bound);
+                if (lane == 0) *(volatile uint32_t *)&sh->tiny[parity][warp < 8 ? 0 : 1][warp & 3] = rows;
+                least = ~0u;
+                left += steps;
+                parity ^= 1;
+            }
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -482,7 +492,7 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
         const int quarter = warp & 3, m = quarter * 32 + lane;
         uint8_t *const staged = smem_raw + FT_STAGES * STAGE + half * 128 * ROW;
         int acc = 0;
-        uint32_t acc_phase = 0, small_phase = 0;
+        uint32_t acc_phase = 0, small_phase = 0, parity = 0;
         bool ok = true, stored = false;
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             float sum[COLS];
@@ -517,11 +527,13 @@ conv_fp32_tc_kernel(const __grid_constant__ Fp32TcArgs a)
                 small_phase ^= 1;
             }
             if (!meet(half, ok && !*abort_flag)) break;
-            const FtTile at(a, tile, BN, col0, m);
-            bool odd = false;
+            float all = 0.f;                                    // NaN where a sum is infinite or NaN
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) odd = odd || out_of_range(sum[j]);
-            odd = odd && at.inside;
+            for (int j = 0; j < COLS; ++j) all = fmaf(sum[j], 0.f, all);
+            const uint32_t rows = *(volatile uint32_t *)&sh->tiny[parity][0][quarter] | *(volatile uint32_t *)&sh->tiny[parity][1][quarter];
+            parity ^= 1;
+            const FtTile at(a, tile, BN, col0, m);
+            const bool odd = at.inside && (all != 0.f || (rows >> lane & 1u));
             if (meet(half, !odd)) finish_tile<BN, ACT>(a, at, sum, staged, half, m, stored);
             else {
                 float again[COLS];

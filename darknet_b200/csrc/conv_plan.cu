@@ -27,6 +27,20 @@ static bool fp32_tc_covers(const ConvGeom &g)
     return g.groups == 1 && g.stride <= 2 && g.c >= 8 && g.c * g.size * g.size >= 128 && (long long)g.batch * g.h * g.w < (1LL << 31);
 }
 
+// Bits of the smallest input, but zero, whose products with weights of these sizes (bits) are 2^-90 or more, at least 2^-100; 0 where that would be
+// more than 2^-45, or where a weight is infinite, NaN or beyond bf16's largest number: such a layer stays on the CUDA cores.
+static uint32_t fp32_tc_smallest_input(uint32_t least, uint32_t most)
+{
+    if (most >= 0x7f7f8000u) return 0;
+    const int e = most ? (int)(least >> 23) - 127 : 0;   // the smallest weight is 2^e or more (no weight but zeros: any input does)
+    if (e < -45) return 0;
+    const int x = -90 - e < -100 ? -100 : -90 - e;
+    return (uint32_t)(x + 127) << 23;
+}
+
+// Whether a launch of this plan runs on the tensor cores (after set_params; before it, whether the layer is one for them).
+static bool on_fp32_tc(const dnb_conv_plan *p) { return p->fp32_tc && !p->keep_k_order && (!p->params_set || p->fp32_smallest); }
+
 static int fp32_tc_filters(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; }   // of a tile
 
 // Whether they should: for either layout, so that a plan's sums are the same in both.  Microseconds of either kernel, measured on B200: a step of
@@ -150,7 +164,7 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
-    else if (p->fp32_tc && !p->keep_k_order)
+    else if (on_fp32_tc(p))
         snprintf(buf, len, "%s three_bf16_parts bn=%d", dnb_conv_plan_kernel(p), fp32_tc_filters(p->d.n));
     else
         snprintf(buf, len, "%s", dnb_conv_plan_kernel(p));
@@ -202,21 +216,28 @@ __global__ void repack_tc_kernel(const float *__restrict__ w, T *__restrict__ ou
 }
 
 // [c_blocks][taps][3][n_pad][32]: the weights as sums of three bf16 numbers, each the nearest to what the ones before it leave (the last
-// one exactly that).  A status word behind them starts at 0.
-__global__ void split_weights_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ out, int n, int c, int taps, int n_pad, int c_blocks, int *status)
+// one exactly that).  range: the bits of the smallest |weight| but zero, of the largest.  A status word behind them starts at 0.
+__global__ void split_weights_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ out, int n, int c, int taps, int n_pad, int c_blocks, uint32_t *range, int *status)
 {
     if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+    uint32_t least = ~0u, most = 0u;
     const size_t part = (size_t)n_pad * 32, total = part * taps * c_blocks;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t step = i / part, r = i - step * part;
         const int cc = (int)(step / taps) * 32 + (int)(r & 31), t = (int)(step % taps), f = (int)(r >> 5);
         float v = f < n && cc < c ? __ldg(w + ((size_t)f * c + cc) * taps + t) : 0.f;
+        const uint32_t size = __float_as_uint(v) & 0x7fffffffu;
+        if (size && size < least) least = size;
+        if (size > most) most = size;
         for (int k = 0; k < 3; ++k) {
             const __nv_bfloat16 h = __float2bfloat16_rn(v);
             out[(3 * step + k) * part + r] = h;
             v -= __bfloat162float(h);
         }
     }
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) { atomicMin(range, least); atomicMax(range + 1, most); }
 }
 
 // CUDA-core layout [groups][K][npg_pad], K = c/groups * size * size, filters innermost
@@ -349,13 +370,20 @@ extern "C" int dnb_conv_plan_set_params(dnb_conv_plan *p, const float *weights, 
         const int c_blocks = (d.c + 31) / 32;
         const size_t first = (total + 63) / 64 * 64, parts = p->fp32_tc && !p->keep_k_order ? (size_t)c_blocks * taps * 3 * p->n_pad * 32 : 0;   // bf16 values
         if (p->status_in_block) { p->status = nullptr; p->status_in_block = false; }
-        DNB_TRY(device_alloc(&p->w_direct, parts ? first + parts / 2 + 1 : total));
+        p->fp32_smallest = 0;
+        DNB_TRY(device_alloc(&p->w_direct, parts ? first + parts / 2 + 3 : total));
         repack_direct_kernel<<<grid_of(total), 256>>>(raw, p->w_direct, d.groups, npg, K, p->npg_pad);
         if (parts) {
             p->w_parts = reinterpret_cast<__nv_bfloat16 *>(p->w_direct + first);
+            uint32_t *const range = reinterpret_cast<uint32_t *>(p->w_parts + parts);
             int *word = nullptr;
-            if (!p->status) { word = p->status = reinterpret_cast<int *>(p->w_parts + parts); p->status_in_block = true; }
-            split_weights_kernel<<<grid_of(parts / 3), 256>>>(raw, p->w_parts, d.n, d.c, taps, p->n_pad, c_blocks, word);
+            if (!p->status) { word = p->status = reinterpret_cast<int *>(range + 2); p->status_in_block = true; }
+            DNB_CUDA(cudaMemsetAsync(range, 0xff, sizeof(uint32_t)));
+            DNB_CUDA(cudaMemsetAsync(range + 1, 0, sizeof(uint32_t)));
+            split_weights_kernel<<<grid_of(parts / 3), 256>>>(raw, p->w_parts, d.n, d.c, taps, p->n_pad, c_blocks, range, word);
+            uint32_t bits[2];
+            DNB_CUDA(cudaMemcpy(bits, range, sizeof(bits), cudaMemcpyDeviceToHost));
+            p->fp32_smallest = fp32_tc_smallest_input(bits[0], bits[1]);
         }
     } else {
         DNB_TRY(device_alloc(&p->w_bits, (size_t)d.n * taps * p->cwords));
@@ -577,6 +605,7 @@ static int build_fp32_tc_args(const dnb_conv_plan *p, const dnb_tensor *x, void 
     a.tiles_h = (g.out_h + a.ht - 1) / a.ht;
     a.total_tiles = a.n_tiles * a.tiles_w * a.tiles_h * ((g.batch + a.bt - 1) / a.bt);
     a.n_pad = p->n_pad;
+    a.smallest = p->fp32_smallest;
     a.g = g;
     a.debug = p->debug_bits;
     a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
@@ -1131,7 +1160,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         const bool rows = (p->keep_k_order || a.xs_h >= (1LL << 31) / 64) && conv_stem_rows_covers(g, y_dtype);
         return rows ? launch_conv_stem_rows(a, s) : launch_conv_stem_tc(a, s);
     }
-    if (p->fp32_tc && !p->keep_k_order && x->dtype == DNB_F32 && (!y_nhwc || y_dtype == DNB_F32)) {
+    if (on_fp32_tc(p) && x->dtype == DNB_F32 && (!y_nhwc || y_dtype == DNB_F32)) {
         Fp32TcArgs a;
         DNB_TRY(build_fp32_tc_args(p, x, y_nhwc, y_cpitch, y_nchw, ep, a));
         return launch_conv_fp32_tc(a, s);

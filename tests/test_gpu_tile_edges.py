@@ -147,6 +147,31 @@ def test_full_precision_on_the_tensor_cores_out_of_range(monkeypatch):
         assert np.abs(out["0"][plain] - out["1"][plain]).max() <= 1e-5 * np.abs(out["0"][plain]).max()
 
 
+@pytest.mark.parametrize("name,x_exp,w_exp", [("tiny_inputs_huge_weights", -118, 40), ("products_below_normal_numbers", -70, -40), ("at_the_line", -52, -38), ("tiny_weights", 30, -60), ("subnormal_weights", 100, -140)])
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+def test_full_precision_of_tiny_operands(name, x_exp, w_exp, layout, monkeypatch):
+    """Rows of pixels whose operands' parts or products are not normal numbers beside rows of ordinary size: tiny ones as the CUDA-core kernel adds
+    them, to the bit; layers with tiny weights run there altogether."""
+    import numpy as np
+    case = conv_case(729, b=2, c=80, h=21, w=23, n=72, size=3, act="linear", bn=False)
+    case["biases"][...] = 0
+    x, w = case["x"], case["w"]
+    w[...] = np.sign(w) * np.exp2(w_exp + np.abs(w) * 4).astype(np.float32)
+    x[:, :, 6:13] = (x[:, :, 6:13].astype(np.float64) * 2.0 ** x_exp).astype(np.float32)
+    x[1, :, 16] = 0
+    out = {}
+    for knob in ("0", "1"):
+        monkeypatch.setenv("DNB_FP32_TC", knob)
+        plan, out[knob], _ = run_conv(case, dn.MODE_FP32, layout, layout)
+        assert ("three_bf16_parts" in plan.describe()) == (knob == "1" and w_exp >= -45)
+    assert np.isfinite(out["0"]).all() and out["0"][:, :, 8:11].any()
+    if layout == "nchw" and name != "at_the_line":     # over channels-last tensors the CUDA-core kernel's order is another
+        assert np.array_equal(out["0"][:, :, 7:12], out["1"][:, :, 7:12])
+    for rows in (slice(0, 5), slice(8, 11), slice(14, None)):
+        scale = np.abs(out["0"][:, :, rows]).max()
+        assert np.abs(out["1"][:, :, rows] - out["0"][:, :, rows].astype(np.float64)).max() <= 2e-6 * scale
+
+
 @pytest.mark.parametrize("shape", [dict(b=4, c=64, h=52, w=51, n=200, size=3), dict(b=2, c=15, h=33, w=40, n=30, size=3, stride=2), dict(b=3, c=131, h=26, w=27, n=64, size=1)])
 @pytest.mark.parametrize("layouts", [("nchw", "nchw"), ("nchw", "nhwc"), ("nhwc", "nhwc")])
 def test_full_precision_without_finite_sums(shape, layouts, monkeypatch):
