@@ -40,6 +40,10 @@
 // (forward_shortcut_layer_gpu, src/shortcut_layer.c:75-80; src/blas_kernels.cu:711-745) when the caller asks for the fusion.
 #include <cuda.h>
 
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include "common.h"
 #include "conv.h"
 #include "device_utils.cuh"
@@ -954,13 +958,19 @@ int conv_tc_max_smem()
     return v;
 }
 
-// Resident clusters of two CTAs of a pair-mode kernel with `smem` bytes of dynamic shared memory (cached per kernel).
+// Resident clusters of two CTAs of a pair-mode kernel with `smem` bytes of dynamic shared memory, kept for each kernel, size and
+// device (the kernels are many, their type is one).
 template <typename K>
 static int max_pair_clusters(K kernel, size_t smem, int threads)
 {
-    static int cached = 0;
-    static size_t cached_smem = 0;
-    if (cached && cached_smem == smem) return cached;
+    static std::mutex lock;
+    static std::map<std::tuple<const void *, size_t, int, int>, int> known;
+    int device = 0;
+    cudaGetDevice(&device);
+    const auto key = std::make_tuple((const void *)kernel, smem, threads, device);
+    std::lock_guard<std::mutex> guard(lock);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
     cfg.blockDim = dim3((unsigned)threads);
@@ -971,7 +981,7 @@ static int max_pair_clusters(K kernel, size_t smem, int threads)
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = sm_count() / 2; }
-    cached = n; cached_smem = smem;
+    known[key] = n;
     return n;
 }
 
