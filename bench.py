@@ -268,9 +268,10 @@ def run_reference(args):
             break
     ms = 1000.0 * float(np.mean(times))
     value = images / (ms / 1000.0)
+    code = "reference CPU path (stock -Ofast -fopenmp build)" if ref.kind == "reference" else "this repository's CPU restatement of the reference, which is not built here"
     line = {"impl": "reference", "metric": ref.metric, "value": value, "unit": UNIT, "n_gpus": args.gpus, "steps": len(times), "warmup": args.warmup,
             "ms_per_step": ms, "higher_is_better": True, "scaling": args.scaling, "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-            "config": {"workload": f"{ref.desc}, reference CPU path (stock -Ofast -fopenmp build), {images} image per step, "
+            "config": {"workload": f"{ref.desc}, {code}, {images} image per step, "
                                    f"{ref.cores} host threads"},
             "cpu_baseline": {"value": value, "unit": UNIT, "cores": ref.cores, "kind": ref.kind,
                              "sample": f"{images} image(s) of {ref.desc} per step, network_predict on the host cores"},
@@ -356,7 +357,7 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
     # a fused [shortcut] reads, over the same event durations
     es = 2.0 if mode == "bf16" else 4.0
     # a convolution that also does the 2x2 maxpool after it writes a quarter of its map
-    written = [0.25 if i + 1 < net.n and kinds[i + 1] == "maxpool" and mean_ms[i + 1] < 0.005 else 1.0 for i in range(net.n)]
+    written = [0.25 if i + 1 < net.n and net.layer_describe(i + 1) == "maxpool fused" else 1.0 for i in range(net.n)]
     small = np.array([bool(tc[i]) and not big3[i] for i in range(net.n)])
     mem_bytes = 0.0
     for i in np.nonzero(small)[0]:
@@ -364,7 +365,7 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
         stride = int(sections[i][1].get("stride", 1))
         sh = shapes[int(i)]
         mem_bytes += es * per_gpu * (sh.c * (h * stride) * (w * stride) + written[i] * sh.n * h * w) + es * sh.n * sh.c * sh.size * sh.size
-        if i + 1 < net.n and kinds[i + 1] == "shortcut" and mean_ms[i + 1] < 0.01:   # fused: its add is read by this launch
+        if i + 1 < net.n and net.layer_describe(i + 1) == "shortcut fused":   # its add is read by this launch
             mem_bytes += es * per_gpu * sh.n * h * w
     small_ms = float(mean_ms[small].sum())
     hbm_part = None

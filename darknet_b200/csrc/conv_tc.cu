@@ -52,7 +52,7 @@
 namespace dnb {
 
 constexpr int MAX_STAGES = 8;
-constexpr int MAX_RES_BUFS = 4;   // staging buffers with a fused residual; tiles are requested two chunks ahead
+constexpr int MAX_RES_BUFS = 4;   // staging buffers with a fused residual; tiles are requested three chunks ahead
 
 // ------------------------------------------------------------------ kernel
 struct TcShared {
@@ -689,7 +689,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         uint32_t pf_count = 0;                 // chunks requested so far (buffer = count & 3)
         int pf_tile = first_tile, pf_c0 = 0;   // the next chunk to request
         const int dbg = a.debug;
-        // diagnostics: bit 1 no residual loads at all, bit 64 none in the second CTA of a pair (wrong results, no waits)
+        // diagnostics: bit 1 no residual loads at all (wrong results, no waits)
         const bool no_res = (dbg & 1) != 0;
         auto request_residual = [&]() {
             if (pf_tile >= total_tiles || no_res) return;

@@ -1309,7 +1309,7 @@ extern "C" int dnb_network_layer_describe(const dnb_network *net, int i, char *b
     if (!net || !buf || len < 1 || i < 0 || i >= (int)net->layers.size()) DNB_FAIL(DNB_EINVAL, "layer_describe: bad argument");
     const Layer &L = net->layers[i];
     if (L.plan) return dnb_conv_plan_describe(L.piece_plan[0] && !L.plan->tc_x_ptr ? L.piece_plan[0] : L.plan, buf, len);   // a layer that only ran in parts
-    snprintf(buf, len, "%s", kKindNames[L.kind]);
+    snprintf(buf, len, "%s%s", kKindNames[L.kind], L.fused_into_prev ? " fused" : "");
     return DNB_OK;
 }
 

@@ -53,26 +53,6 @@ __device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t pa
     return done;
 }
 
-// Bounded wait for a loop that a single thread runs (the TMA and MMA roles of the halo mode): no warp traffic at all.
-__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
-                                                 long long limit = WAIT_LIMIT_CYCLES)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    int spins = 0;
-    while (!mbar_try_wait_hint(bar, parity, 1000u)) {
-        if ((++spins & 0x3f) == 0) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > limit) {
-                *abort_flag = 1;
-                atomicCAS(status, 0, code);
-                return false;
-            }
-        }
-    }
-    return true;
-}
-
 // Bounded wait for a loop that a whole warp runs in step (the TMA and MMA roles): every lane polls, the vote makes the
 // outcome, and with it the loop's control flow and all its counters, uniform in the compiler's eyes.  Such a loop keeps
 // its addresses, coordinates and descriptors in uniform registers, where the TMA and MMA instructions want them; with one
@@ -303,7 +283,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t sr
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read2() { asm volatile("cp.async.bulk.wait_group.read 2;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // 16 bytes from global to shared memory, or 16 zero bytes; completes in groups

@@ -362,7 +362,8 @@ int dnb_network_outputs(const dnb_network *net);
 int dnb_network_layer_shape(const dnb_network *net, int layer, int *out_c, int *out_h, int *out_w);
 const char *dnb_network_layer_type(const dnb_network *net, int layer);
 const char *dnb_network_layer_kernel(const dnb_network *net, int layer);
-/* dnb_conv_plan_describe for a convolutional layer, the section name for the others. */
+/* dnb_conv_plan_describe for a convolutional layer, the section name for the others, with " fused"
+ * after it where the launch of the layer before does the layer's work. */
 int dnb_network_layer_describe(const dnb_network *net, int layer, char *buf, int len);
 
 /* Copy layer `layer`'s current output to host memory as Darknet lays it out
