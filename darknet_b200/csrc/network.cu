@@ -1134,7 +1134,7 @@ static int enqueue_schedule(dnb_network *net, int slot, const float *input, bool
 static void plan_step(dnb_network *net)
 {
     const double copy_rate = 50e3, byte_rate = 4e6;   // bytes per us
-    const double op_rate = net->mode == DNB_MODE_BF16 ? 1.0e9 : (net->mode == DNB_MODE_TF32 ? 5.4e8 : 3e7);   // operations per us
+    const double tc_rate = net->mode == DNB_MODE_BF16 ? 1.0e9 : net->mode == DNB_MODE_TF32 ? 5.4e8 : 1.1e8, cuda_core_rate = 3e7;   // operations per us
     const double part_us = 4, half_us = 6, worth_us = 50;
     const int n = (int)net->layers.size(), batch = net->batch;
     net->schedule.clear();
@@ -1144,8 +1144,10 @@ static void plan_step(dnb_network *net)
         if (L.kind == L_CONV && L.cd.xnor) return;
         double ops = 0;
         if (L.kind == L_CONV) ops = 2.0 * L.cd.n * L.cd.size * L.cd.size * (L.cd.c / L.cd.groups) * L.out_h * L.out_w * batch;
-        const double bytes = L.fused_into_prev ? 0 : ((double)L.c * L.h * L.w + (double)L.out_c * L.out_h * L.out_w) * batch * elem_size(net->dtype);
-        us[i] = std::max(ops / op_rate, bytes / byte_rate);
+        const double written = (double)L.out_c * L.out_h * L.out_w / (L.fuses_next_pool ? 4 : 1);
+        const double bytes = L.fused_into_prev ? 0 : ((double)L.c * L.h * L.w + written) * batch * elem_size(net->dtype);
+        const bool cuda_cores = net->mode == DNB_MODE_FP32 && L.plan && !L.plan->fp32_tc;
+        us[i] = std::max(ops / (cuda_cores ? cuda_core_rate : tc_rate), bytes / byte_rate);
     }
     // every tensor that layer i reads or writes has its part where the kernels' alignment rules want it
     auto aligned = [&](const dnb_tensor &t, int each) {
