@@ -47,7 +47,7 @@ static int fp32_tc_filters(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; } 
 // 32 channels of a tap takes a tile of 128 filters 1.04 on the tensor cores, of 64 0.75, of 32 0.59; a block of the CUDA-core kernel's large tiles of 64
 // filters 64 ns a product where four share an SM, of 32 filters 34 and 50 more, one of its small ones 17.5 and 11.5 more for every other block
 // there, its slabs of up to 16 filters 6 a product and filter.  Of 208 launches between 10 us and 1 ms 199 take the faster kernel, or one within 5 %
-// of it; the worst choice was 1.17 times the other's time.  8 x 64 x 104 x 104 -> 128, 3x3: 316 -> 104 us, from Darknet's layout 352 -> 113; 32 x 64 x 104 x 104
+// of it; the worst choice was 1.2 times the other's time.  8 x 64 x 104 x 104 -> 128, 3x3: 316 -> 104 us, from Darknet's layout 352 -> 113; 32 x 64 x 104 x 104
 // -> 64 676 -> 298; 8 x 100 x 38 x 38 -> 70, stride 2, would be 27 -> 42.  DNB_FP32_TC: 0 never, 1 whenever it can.
 static bool fp32_tc_pays(const ConvGeom &g)
 {
