@@ -147,6 +147,37 @@ int launch_conv_tc_split(const SplitArgs &a, cudaStream_t s);
 size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes);
 int conv_tc_split_resident(int pair, int cluster);
 
+// ---- conv_tc_taps.cu : 3x3 layers with stride 1 in CTA pairs, one load of pixels for all nine taps
+constexpr int TAPS_MAX_X = 3, TAPS_MAX_W = 36;
+struct alignas(64) TapsArgs {
+    CUtensorMap tmx;      // im2col map: the input with a column of zeros before each row and a row of zeros before each image
+    CUtensorMap tmw;      // weights, half a filter tile of 128 bytes of channels
+    int bf16;             // operands and channels-last output bf16, else f32 (TF32 products)
+    int bk, c_blocks;     // channels of a block (128 bytes), blocks
+    int bn, n_tiles;      // filters per tile, a multiple of 16
+    int pitch, rows;      // positions of a row (w + 1); of a tile's load (128 + 2 * pitch + 2)
+    int ptiles;           // tiles of 128 positions
+    int total_tiles;      // pairs of them times n_tiles
+    int x_stages, x_slot; // ring of pixel boxes, bytes of one
+    int w_stages, w_bytes;// ring of filter tiles
+    int resident;         // 1: the ring holds all of the layer's filters, loaded once
+    int staged_bytes;     // rows of the eight epilogue warps: 4 KB each, 8 with a residual, none for Darknet's layout alone
+    int table;            // entries of the scale and shift tables in shared memory
+    int tmem_cols, n_pad;
+    int y_chan;           // channels written to y_nhwc
+    void *y_nhwc;
+    int y_cpitch;
+    float *y_nchw;
+    int *status;
+    int debug;
+    long long wait_limit;
+    ConvGeom g;
+    ConvEpilogue ep;
+};
+int launch_conv_tc_taps(const TapsArgs &a, cudaStream_t s);
+size_t conv_tc_taps_smem(const TapsArgs &a);
+size_t conv_tc_taps_fixed_smem(const TapsArgs &a);   // what its rings leave
+
 // ---- conv_fp32_tc.cu : fp32 convolution by three bf16 parts of every operand on the tensor cores, sums in fp32 registers
 struct alignas(64) Fp32TcArgs {
     CUtensorMap tmx[4];   // as in TcArgs; boxes of 32 channels x wt x ht x bt pixels
@@ -174,6 +205,10 @@ int launch_conv_fp32_tc(const Fp32TcArgs &a, cudaStream_t s);
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
 int encode_tensor_map(CUtensorMap *map, int elem_kind /* 0 f32, 1 bf16, 2 bytes */, int rank, void *base, const uint64_t *dims,
                       const uint64_t *strides_bytes /* rank-1 */, const uint32_t *box, int swizzle_bytes);
+
+// Map for loads in im2col mode of an NHWC tensor: `rows` pixels of `chan` channels (128 bytes, 128-byte swizzle) along the bounding box that has one column
+// before each row and one row before each image.
+int encode_im2col_map(CUtensorMap *map, int elem_kind, void *base, const uint64_t *dims, const uint64_t *strides_bytes, uint32_t chan, uint32_t rows);
 
 // ---- conv_xnor.cu : bit-packed popcount GEMM
 struct XnorArgs {
@@ -246,6 +281,10 @@ struct dnb_conv_plan {
     bool keep_k_order;       // sum K in one order whatever the batch (dense layers of a network with xnor layers): no split, first layers in the im2col order
     bool tc_split;           // launches use the one-tile-per-cluster kernel and its block below
     dnb::SplitArgs sp;
+    bool tc_taps;            // ... or conv_tc_taps.cu and its block
+    dnb::TapsArgs tp;
+    int whole_batch;         // of the plan that this one is a part of (see taps_pay), its own otherwise
+    bool tap_order;          // sums over taps, then blocks of channels, on whichever kernel: not conv_tc_taps.cu
     bool status_in_block;    // the status word lies behind the weights
     bool fp32_tc;            // this full-precision plan's layer is one that conv_fp32_tc.cu is made for
     uint32_t fp32_smallest;  // ... its smallest input (see there), or 0 where its weights keep it on the CUDA cores

@@ -125,6 +125,7 @@ dnb_conv_plan *conv_plan_for_batch(const dnb_conv_plan *p, int batch)
     dnb_conv_plan *q = new dnb_conv_plan(*p);
     q->d.batch = q->g.batch = batch;
     q->borrowed = true;
+    q->whole_batch = p->g.batch;
     q->x_nhwc_scratch = nullptr; q->x_bits = nullptr; q->x_i8 = nullptr;
     q->x_nhwc_bytes = q->x_bits_bytes = q->x_i8_bytes = 0;
     q->tc_x_ptr = q->tc_y_ptr = q->tc_res_ptr = nullptr;
@@ -161,6 +162,9 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
     if (tc && p->tc_x_ptr && p->tc_split)
         snprintf(buf, len, "%s pair=%d halo=0 bn=%d tile=%dx%dx%d tiles=%d stages=%d splits=%d signs_in=%d signs_out=%d one_tile_per_cluster", kKernelNames[p->kernel], p->sp.pair,
                  p->sp.bn, p->sp.wt, p->sp.ht, p->sp.bt, p->sp.tiles, p->sp.stages, p->sp.splits, p->signs_given ? 1 : 0, p->sp.sign_out ? 1 : 0);
+    else if (tc && p->tc_x_ptr && p->tc_taps)
+        snprintf(buf, len, "%s pair=1 halo=0 bn=%d tiles=%d stages=%d+%d epi=2 splits=1 one_load_for_nine_taps%s", kKernelNames[p->kernel], p->tp.bn, p->tp.total_tiles,
+                 p->tp.x_stages, p->tp.w_stages, p->tp.resident ? " resident" : "");
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
@@ -783,6 +787,130 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     a.total_tiles = a.pair ? (ptiles + 1) / 2 * a.n_tiles : ptiles * a.n_tiles;
 }
 
+// ------------------------------------------------------------------ 3x3 layers with one load for nine taps (conv_tc_taps.cu)
+// The launch's tiles and rings; p->tp holds them.  False where the kernel has no form of it.
+static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channels_last, bool residual)
+{
+    TapsArgs &a = p->tp;
+    const int es = p->kernel == K_TC_BF16 ? 2 : 4;
+    a.bf16 = es == 2 ? 1 : 0;
+    a.bk = 128 / es;
+    a.c_blocks = (p->c_pad + a.bk - 1) / a.bk;
+    a.pitch = g.w + 1;
+    a.rows = 128 + 2 * a.pitch + 2;
+    if (a.rows > 1024) return false;
+    const long long positions = (long long)g.batch * a.pitch * (g.h + 1) - a.pitch - 1;
+    if (positions > (1LL << 31) - 4096) return false;
+    a.ptiles = (int)((positions + 127) / 128);
+    a.bn = bn;
+    a.n_tiles = (p->n_pad + bn - 1) / bn;
+    const long long tiles = (long long)((a.ptiles + 1) / 2) * a.n_tiles;
+    if (tiles > 1 << 30) return false;
+    a.total_tiles = (int)tiles;
+    a.x_slot = round_up(a.rows * 128, 1024);
+    a.w_bytes = round_up(bn / 2 * 128, 1024);
+    a.staged_bytes = channels_last ? (residual ? 65536 : 32768) : 0;
+    a.table = round_up(a.n_tiles * bn, 64) + 64;
+    a.tmem_cols = 32;
+    while (a.tmem_cols < 2 * bn) a.tmem_cols *= 2;
+    a.x_stages = a.w_stages = 0;
+    a.resident = 0;
+    const long budget = conv_tc_max_smem() - (long)conv_tc_taps_fixed_smem(a);
+    const int all = 9 * a.c_blocks;
+    if (a.n_tiles == 1 && all <= TAPS_MAX_W && 2L * a.x_slot + (long)all * a.w_bytes <= budget) {
+        a.resident = 1;
+        a.w_stages = all;
+        a.x_stages = (int)((budget - (long)all * a.w_bytes) / a.x_slot);
+    } else {
+        a.x_stages = 2;
+        long left = budget - 2L * a.x_slot;
+        // a third box where the filters' ring keeps its depth
+        if (left - a.x_slot >= 8L * a.w_bytes) { a.x_stages = 3; left -= a.x_slot; }
+        a.w_stages = left > 0 ? (int)(left / a.w_bytes) : 0;
+        if (a.w_stages > 12) a.w_stages = 12;
+    }
+    if (a.x_stages > TAPS_MAX_X) a.x_stages = TAPS_MAX_X;
+    return a.x_stages >= 2 && a.w_stages >= 3;
+}
+
+// Whether the kernel has a variant for such a launch of the plan.
+static bool taps_covers(const dnb_conv_plan *p, const ConvEpilogue *res, bool nchw_out)
+{
+    const int es = p->kernel == K_TC_BF16 ? 2 : 4;
+    if ((p->kernel != K_TC_TF32 && p->kernel != K_TC_BF16) || p->g.size != 3 || p->g.stride != 1 || p->g.pad != 1 || p->keep_k_order) return false;
+    if (p->tap_order && p->c_pad * es > 128) return false;   // (one block of channels: there is one order)
+    if (p->c_pad * es < 128 || (p->d.activation != DNB_LEAKY && p->d.activation != DNB_LINEAR) || (res && res->yolo_entries)) return false;
+    return !(res && res->residual) ||
+           (res->res_stride == 1 && res->res_c == p->g.n && !nchw_out && res->activation2 == (p->d.activation == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY));
+}
+
+// Microseconds of such a launch.  Fitted to 600 measured ones (3x3 layers of 32 to 1024 filters over 32 to 640 channels, maps of 7 to 152, 1 to 128 images, either type and
+// layout; 7 % root mean square): an iteration is the four MMAs of a tap and 128 bytes of channels, 0.174 up to 128 filters and 0.31 at 256; the im2col load
+// takes 3.7 ns a position; a tile's epilogue 6 ns a filter, 19 in Darknet's layout, 27 with a residual.
+static double taps_us(const TapsArgs &a, bool nchw_out, bool residual)
+{
+    const double clusters = sm_count() / 2, rounds = ceil(a.total_tiles / clusters);
+    const double mma = 9.0 * a.c_blocks * (a.bn <= 128 ? 0.174 : 0.174 + 0.136 * (a.bn - 128) / 128);
+    const double load = a.c_blocks * a.rows * 0.0037, epilogue = a.bn * (nchw_out ? 0.019 : residual ? 0.027 : 0.006);
+    const double longest = mma > load ? (mma > epilogue ? mma : epilogue) : (load > epilogue ? load : epilogue);
+    return 5.3 + rounds * (longest + 0.65) + 0.55 * epilogue + load / a.c_blocks;
+}
+
+// The best tile of a launch of geometry g, in p->tp; its estimated time, or 1e300.
+static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last, bool nchw_out, bool residual)
+{
+    const char *e = getenv("DNB_TC_TAPS_BN");
+    const int only = e ? atoi(e) : 0;
+    int best_bn = 0;
+    double best = 1e300;
+    for (int bn = 64; bn <= 256; bn *= 2) {
+        const int width = bn < p->n_pad ? bn : p->n_pad;
+        if ((only && bn != only) || (bn > 64 && bn / 2 >= p->n_pad) || !taps_tiles(p, g, width, channels_last, residual)) continue;
+        const double us = taps_us(p->tp, nchw_out, residual);
+        if (us < best) { best = us; best_bn = width; }
+    }
+    return best_bn && taps_tiles(p, g, best_bn, channels_last, residual) ? best : 1e300;
+}
+
+// Whether a launch takes that kernel: where its estimate is a tenth below what the others take.  others_us: the estimate of the launch that it would
+// be, cut along K or not.  Those estimates are of launches in a chain; in the measure of taps_us, launches by themselves, cut ones take 1.3 times
+// theirs and whole ones 1.12, in Darknet's layout 1.55 and 1.3 (stores in the short rows of a tile), with a residual 1.25 and 1.05.  On 300 random
+// launches the rule takes 80 here, 4 of them to their loss (of 5 to 8 %), and all of the launches take 0.947 of what they did: 16 x 256 x 52 x 52
+// -> 512 in Darknet's layout 153 -> 126 us, 2 x 120 x 76 x 76 -> 128 26.8 -> 14.2, 256 x 128 x 28 x 28 -> 128 128 -> 106, 34 x 232 x 38 x 38 -> 255 in bf16 85 -> 42.
+// Launches of many rounds of pairs over 256 filters run into the power cap in either kernel (64 x 256 x 38 x 38 -> 512 265 -> 261 alone, 300 -> 307
+// inside YOLOv3-608) and stay where less padding is multiplied.
+// The kernel adds in another order, so g is that of the whole batch where the plan is for a part of it, and of one image where there are two: an
+// image's sums then hang neither on the parts nor on the other image.
+// DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
+static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
+{
+    const char *e = getenv("DNB_TC_TAPS"), *split = getenv("DNB_TC_SPLITK");
+    const int knob = e ? atoi(e) : 1;
+    if (knob == 0) return false;
+    if (!e && (getenv("DNB_TC_PAIR") || getenv("DNB_TC_EPI") || getenv("DNB_TC_HALO") || getenv("DNB_TC_WARP_STORES") || (split && atoi(split) > 1))) return false;
+    const bool residual = res && res->residual;
+    const double slack = nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 1.05) : cut ? 1.3 : 1.12;
+    const double us = best_taps(p, g, channels_last, nchw_out, residual);
+    return us < 1e300 && (knob == 2 || us < 0.9 * slack * others_us);
+}
+
+static int build_taps_args(dnb_conv_plan *p, const dnb_tensor *x, const void *y_nhwc, int y_cpitch)
+{
+    TapsArgs &a = p->tp;
+    const ConvGeom &g = p->g;
+    const int es = a.bf16 ? 2 : 4;
+    a.g = g;
+    a.n_pad = p->n_pad;
+    const int n8 = round_up(g.n, 8);
+    a.y_chan = y_nhwc ? (n8 < y_cpitch ? n8 : y_cpitch) : 0;
+    a.debug = p->tc.debug; a.wait_limit = p->tc.wait_limit;
+    DNB_TRY(ensure_status(p));
+    const uint64_t pix = (uint64_t)x->cpitch * es;
+    const uint64_t dims[4] = {(uint64_t)p->c_pad, (uint64_t)g.w, (uint64_t)g.h, (uint64_t)g.batch}, strides[3] = {pix, pix * g.w, pix * g.w * g.h};
+    DNB_TRY(encode_im2col_map(&a.tmx, a.bf16, x->data, dims, strides, (uint32_t)a.bk, (uint32_t)a.rows));
+    return encode_weight_map(&a.tmw, p, a.bf16, es, p->c_pad, 9, a.bk, a.bn / 2, 128);
+}
+
 static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
                          const ConvEpilogue *res, bool nchw_out, void *sign_out = nullptr, int sign_cpitch = 0, bool pool = false)
 {
@@ -810,6 +938,9 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.bk = a.row_bytes / es;
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
     a.taps = g.size * g.size;
+    a.debug = (getenv("DNB_TC_DEBUG") ? atoi(getenv("DNB_TC_DEBUG")) : 0) | p->debug_bits;
+    a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
+    p->tc_taps = p->tc_split = false;
     pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, pool);
     a.pool = pool ? 1 : 0;
     a.n_pad = p->n_pad;
@@ -841,8 +972,6 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     if (sign_out && !pool) a.stage_bufs = 3;   // the third buffer holds the staged signs (pooled rows and theirs fit the second one)
     a.sign_out = sign_out;
     a.sign_cpitch = sign_cpitch;
-    a.debug = (getenv("DNB_TC_DEBUG") ? atoi(getenv("DNB_TC_DEBUG")) : 0) | p->debug_bits;
-    a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
     int stages = 0;
     const bool allow2 = getenv("DNB_TC_CTAS") ? atoi(getenv("DNB_TC_CTAS")) >= 2 : true;
     a.a_slot = a.a_box_slot = a.a_box_bytes = a.a_pitch = 0;
@@ -942,43 +1071,57 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // A launch that leaves SMs idle, or whose few tiles have a long K loop: one tile per cluster, K cut across it
     // (conv_tc_split.cu).  Chosen where its estimate is below the persistent kernel's, which overlaps a tile's epilogue with the
     // next one's MMAs and therefore wins once every SM has a few tiles.  DNB_TC_SPLITK: 0 never, N forces N ranges (tests).
-    p->tc_split = false;
-    {
+    const bool may_cut = [&] {
         const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
         const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1;
-        const int k_iters = g.size * g.size * a.c_blocks;
-        if (knob != 0 && !a.halo && !pool && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2)) {
-            // pixels of a 1x1 layer in one row: of the whole batch where nothing is stored per image
-            auto flat = [&](ConvGeom sg) {
-                if (sg.size == 1 && sg.stride == 1 && sg.pad == 0) {
-                    sg.w = sg.out_w = sg.w * sg.h * (nchw_out ? 1 : sg.batch);
-                    sg.h = sg.out_h = 1;
-                    if (!nchw_out) sg.batch = 1;
-                }
-                return sg;
-            };
-            SplitQuery q;
-            q.row_bytes = a.row_bytes; q.k_iters = k_iters; q.n_pad = p->n_pad; q.max_smem = max_smem;
-            q.pair_ok = pair_knob > 0 && a.row_bytes == 128 && g.n % 256 == 0 && k_iters >= 16;
-            q.residual = residual != nullptr;
-            q.long_sum = g.c * g.size * g.size >= 8192;
-            SplitPlan sp;
-            if (knob > 1) {
-                sp = choose_split(q, flat(g), knob < 8 ? knob : 8, true, g.batch);
-            } else {
-                // decided at one image for two images also (see choose_split)
-                ConvGeom dg = g;
-                if (g.batch == 2) dg.batch = 1;
-                TcArgs da = a;
-                pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, false, true);
-                sp = choose_split(q, flat(dg), 0, false, dg.batch);
-                if (!(sp.cost < uncut_us(da, k_iters, q.residual))) sp = SplitPlan();
-                else if (g.batch == 2) sp = choose_split(q, flat(g), sp.splits, false, 2);
-            }
-            if (sp.splits) DNB_TRY(build_split_args(p, x, flat(g), sp, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));
+        return knob != 0 && !a.halo && !pool && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2);
+    }();
+    // pixels of a 1x1 layer in one row: of the whole batch where nothing is stored per image
+    auto flat = [&](ConvGeom sg) {
+        if (sg.size == 1 && sg.stride == 1 && sg.pad == 0) {
+            sg.w = sg.out_w = sg.w * sg.h * (nchw_out ? 1 : sg.batch);
+            sg.h = sg.out_h = 1;
+            if (!nchw_out) sg.batch = 1;
         }
+        return sg;
+    };
+    auto cut_at = [&](const ConvGeom &at) {   // the cut launch of that geometry, no ranges where it is not cut
+        const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
+        const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1, k_iters = at.size * at.size * a.c_blocks;
+        SplitQuery q;
+        q.row_bytes = a.row_bytes; q.k_iters = k_iters; q.n_pad = p->n_pad; q.max_smem = max_smem;
+        q.pair_ok = pair_knob > 0 && a.row_bytes == 128 && at.n % 256 == 0 && k_iters >= 16;
+        q.residual = residual != nullptr;
+        q.long_sum = at.c * at.size * at.size >= 8192;
+        if (knob > 1) return choose_split(q, flat(at), knob < 8 ? knob : 8, true, at.batch);
+        // decided at one image for two images also (see choose_split)
+        ConvGeom dg = at;
+        if (at.batch == 2) dg.batch = 1;
+        TcArgs da = a;
+        pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, false, true);
+        SplitPlan sp = choose_split(q, flat(dg), 0, false, dg.batch);
+        if (!(sp.cost < uncut_us(da, k_iters, q.residual))) sp = SplitPlan();
+        else if (at.batch == 2) sp = choose_split(q, flat(at), sp.splits, false, 2);
+        return sp;
+    };
+    const SplitPlan cut = may_cut ? cut_at(g) : SplitPlan();
+    if (!pool && !i8 && taps_covers(p, res, nchw_out)) {
+        const int whole = p->whole_batch > g.batch ? p->whole_batch : g.batch;
+        ConvGeom dg = p->g;
+        dg.batch = whole <= 2 ? 1 : whole;
+        SplitPlan dcut = cut;
+        TcArgs da = a;
+        if (dg.batch != g.batch) {
+            if (may_cut) dcut = cut_at(dg);
+            pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
+        }
+        const double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, 9 * a.c_blocks, residual != nullptr);
+        p->tc_taps = taps_pay(p, dg, dcut.splits != 0, others, res, y_nhwc != nullptr, nchw_out) &&
+                     best_taps(p, g, y_nhwc != nullptr, nchw_out, residual != nullptr) < 1e300;
     }
-    if (p->tc_split) {
+    if (p->tc_taps) DNB_TRY(build_taps_args(p, x, y_nhwc, y_cpitch));
+    else if (cut.splits) DNB_TRY(build_split_args(p, x, flat(g), cut, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));
+    if (p->tc_split || p->tc_taps) {
         p->tc_sign_out = sign_out;
         p->tc_x_ptr = x->data; p->tc_x_cpitch = x->cpitch; p->tc_y_ptr = y_nhwc; p->tc_y_cpitch = y_cpitch; p->tc_y_dtype = y_dtype;
         p->tc_res_ptr = residual; p->tc_res_cpitch = res_cpitch; p->tc_res_c = res_c; p->tc_res_stride = res_stride; p->tc_nchw_out = nchw_out ? 1 : 0; p->tc_pool = 0;
@@ -1265,6 +1408,13 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         a.ep = ep;
         a.status = p->status;
         return launch_conv_tc_split(a, s);
+    }
+    if (p->tc_taps) {
+        TapsArgs &a = p->tp;
+        a.y_nhwc = y_nhwc; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;
+        a.ep = ep;
+        a.status = p->status;
+        return launch_conv_tc_taps(a, s);
     }
     TcArgs &a = p->tc;
     a.y_nhwc = y_nhwc; a.y_dtype = y_dtype; a.y_cpitch = y_cpitch; a.y_nchw = y_nchw;

@@ -1129,9 +1129,21 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
     return DNB_OK;
 }
 
+typedef CUresult (*EncodeIm2colFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const int *, const int *,
+                                   cuuint32_t, cuuint32_t, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// A host thread's first call: the runtime would make the device's context its own on demand, the driver does not.
+template <typename F>
+static CUresult with_context(F encode)
+{
+    CUresult r = encode();
+    int device = 0;
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) r = encode();
+    return r;
+}
 
 int encode_tensor_map(CUtensorMap *map, int elem_kind, int rank, void *base, const uint64_t *dims,
                       const uint64_t *strides_bytes, const uint32_t *box, int swizzle_bytes)
@@ -1151,19 +1163,35 @@ int encode_tensor_map(CUtensorMap *map, int elem_kind, int rank, void *base, con
     CUtensorMapSwizzle sw = swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                             : swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
     const CUtensorMapDataType dt = elem_kind == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : (elem_kind == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
-    auto encode = [&]() {
+    const CUresult r = with_context([&]() {
         return fn(map, dt, (cuuint32_t)rank, base, d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    };
-    CUresult r = encode();
-    if (r == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread's first call: the runtime would make the device's context its own on demand, the driver does not
-        int device = 0;
-        DNB_CUDA(cudaGetDevice(&device));
-        DNB_CUDA(cudaSetDevice(device));
-        r = encode();
-    }
+    });
     if (r != CUDA_SUCCESS)
         DNB_FAIL(DNB_ECUDA, "cuTensorMapEncodeTiled failed with %d (rank %d, dims %llu %llu %llu, box %u %u %u, swizzle %d)", (int)r, rank,
                  (unsigned long long)d[0], (unsigned long long)d[1], (unsigned long long)(rank > 2 ? d[2] : 0), bx[0], bx[1], rank > 2 ? bx[2] : 0, swizzle_bytes);
+    return DNB_OK;
+}
+
+int encode_im2col_map(CUtensorMap *map, int elem_kind, void *base, const uint64_t *dims, const uint64_t *strides_bytes, uint32_t chan, uint32_t rows)
+{
+    static EncodeIm2colFn fn = nullptr;
+    if (!fn) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        DNB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &p, cudaEnableDefault, &q));
+        if (!p || q != cudaDriverEntryPointSuccess) DNB_FAIL(DNB_ECUDA, "cuTensorMapEncodeIm2col is not available from this driver");
+        fn = (EncodeIm2colFn)p;
+    }
+    const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]}, st[3] = {strides_bytes[0], strides_bytes[1], strides_bytes[2]};
+    const int lower[2] = {-1, -1}, upper[2] = {0, 0};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    const CUresult r = with_context([&]() {
+        return fn(map, elem_kind == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, d, st, lower, upper, chan, rows, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
+    if (r != CUDA_SUCCESS)
+        DNB_FAIL(DNB_ECUDA, "cuTensorMapEncodeIm2col failed with %d (dims %llu %llu %llu %llu, %u channels, %u pixels)", (int)r, (unsigned long long)d[0],
+                 (unsigned long long)d[1], (unsigned long long)d[2], (unsigned long long)d[3], chan, rows);
     return DNB_OK;
 }
 

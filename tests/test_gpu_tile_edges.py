@@ -704,3 +704,81 @@ def test_pairs_over_128_filters(mode, c, monkeypatch):
     plan, single, _ = run_conv(case, mode, "nhwc", "nhwc")
     assert "pair=0" in plan.describe() and np.array_equal(got, single)
     parity(got, oracle_conv(case), 3e-2 if mode == dn.MODE_BF16 else 1e-2)
+
+
+TAPS = {   # one load of pixels for the nine taps: tiles across rows and images, maps smaller than a tile, filters beyond a tile or a chunk, ragged blocks of channels
+    "one_tile": dict(b=1, c=64, h=13, w=13, n=64, size=3),
+    "rows_of_one_pixel": dict(b=33, c=64, h=3, w=1, n=48, size=3),
+    "odd_pixel_tiles_residual": dict(b=2, c=96, h=19, w=19, n=128, size=3, act="linear"),
+    "several_images_a_tile": dict(b=9, c=128, h=7, w=5, n=256, size=3),
+    "half_a_chunk_ragged_channels": dict(b=4, c=72, h=26, w=25, n=200, size=3),
+    "three_filter_tiles": dict(b=7, c=160, h=9, w=14, n=264, size=3, act="linear"),
+    "wide_rows": dict(b=1, c=64, h=21, w=150, n=40, size=3),
+    "rounds_of_tiles_residual": dict(b=9, c=64, h=38, w=38, n=512, size=3),
+}
+
+
+@pytest.mark.parametrize("name", list(TAPS))
+@pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
+def test_one_load_for_nine_taps(name, mode, tol, monkeypatch):
+    """Whole numbers, whose sums are exact in any order: equal to the kernel that loads tap by tap to the bit, in either layout.  Others: within the mode's
+    tolerance of the checker; with a residual to the kernel's output plus it, rounded once more."""
+    import ctypes as C
+    import numpy as np
+    import torch
+    from gpu_util import dev_nhwc, empty_nhwc, host_from_nhwc, padding_is_zero
+    case = conv_case(760, **TAPS[name])
+    whole = dict(case, x=np.rint(2 * case["x"]), w=np.rint(case["w"] / np.abs(case["w"]).max() * 6), biases=np.rint(9 * case["biases"]), scales=None, mean=None, var=None)
+    out = {}
+    for knob in ("0", "2"):
+        monkeypatch.setenv("DNB_TC_TAPS", knob)
+        plan, a, b = run_conv(whole, mode, "nhwc", "nchw", both=True)
+        assert ("one_load_for_nine_taps" in plan.describe()) == (knob == "2"), plan.describe()
+        plan, c, _ = run_conv(whole, mode, "nhwc", "nhwc")
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+        out[knob] = a
+    assert np.array_equal(out["0"], out["2"])
+    plan, out["2"], _ = run_conv(case, mode, "nhwc", "nhwc")
+    parity(out["2"], oracle_conv(case), tol)
+    if "residual" not in name:
+        return
+    store = torch.bfloat16 if mode == dn.MODE_BF16 else torch.float32
+    add = np.random.Generator(np.random.Philox(key=[8, 8])).standard_normal(out["2"].shape, dtype=np.float32)
+    act2 = "leaky" if case["act"] == "linear" else "linear"
+    xt, xd = dev_nhwc(case["x"], store)
+    at, ad = dev_nhwc(add, store)
+    yt, yd = empty_nhwc(*out["2"].shape, store)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    dn.check(dn.lib().dnb_conv_shortcut_forward(plan.handle, C.byref(xd), C.byref(ad), C.byref(yd), 1.0, 1.0, dn.ACTIVATIONS[act2], stream))
+    torch.cuda.synchronize()
+    plan.check_status()
+    assert "one_load_for_nine_taps" in plan.describe(), plan.describe()
+    want = out["2"] + host_from_nhwc(at, add.shape[1])
+    if act2 == "leaky":
+        want = np.where(want > 0, want, np.float32(0.1) * want)
+    # both terms are rounded to the storage type (half an ulp of 11 or 8 bits each, and once more the sum)
+    parity(host_from_nhwc(yt, add.shape[1]), want, 2 ** -7 if mode == dn.MODE_BF16 else 2 ** -10)
+    assert padding_is_zero(yt, add.shape[1])
+
+
+def test_one_load_for_nine_taps_wait_expiry(monkeypatch):
+    """A withheld load makes a wait run out: the launch ends early, says so, and the next one is sound."""
+    import numpy as np
+    monkeypatch.setenv("DNB_TC_TAPS", "2")
+    case = conv_case(761, b=3, c=64, h=30, w=30, n=64, size=3)
+    plan, good, _ = run_conv(case, dn.MODE_TF32, "nhwc", "nhwc")
+    from gpu_util import dev_nhwc, empty_nhwc, host_from_nhwc
+    import torch
+    xt, xd = dev_nhwc(case["x"])
+    yt, yd = empty_nhwc(*good.shape)
+    plan.set_diagnostics(4_000_000, 32)
+    plan.forward(xd, yd)
+    torch.cuda.synchronize()
+    with pytest.raises(dn.DarknetB200Error) as e:
+        plan.check_status()
+    assert e.value.status == dn.ETIMEOUT
+    plan.set_diagnostics(0, 0)
+    plan.forward(xd, yd)
+    torch.cuda.synchronize()
+    plan.check_status()
+    assert np.array_equal(host_from_nhwc(yt, good.shape[1]), good)
