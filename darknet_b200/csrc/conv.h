@@ -148,11 +148,12 @@ size_t conv_tc_split_smem(int stages, int stage_bytes, int bn, int *work_bytes);
 int conv_tc_split_resident(int pair, int cluster);
 
 // ---- conv_tc_taps.cu : 3x3 layers with stride 1 in CTA pairs, one load of pixels for all nine taps
-constexpr int TAPS_MAX_X = 3, TAPS_MAX_W = 36;
+constexpr int TAPS_MAX_X = 6, TAPS_MAX_W = 36;
 struct alignas(64) TapsArgs {
     CUtensorMap tmx;      // im2col map: the input with a column of zeros before each row and a row of zeros before each image
     CUtensorMap tmw;      // weights, half a filter tile of 128 bytes of channels
     int bf16;             // operands and channels-last output bf16, else f32 (TF32 products)
+    int taps, pixels;     // 9, or 1 (1x1 layers); of those the pixels of the whole batch
     int bk, c_blocks;     // channels of a block (128 bytes), blocks
     int bn, n_tiles;      // filters per tile, a multiple of 16
     int pitch, rows;      // positions of a row (w + 1); of a tile's load (128 + 2 * pitch + 2)

@@ -163,8 +163,8 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
         snprintf(buf, len, "%s pair=%d halo=0 bn=%d tile=%dx%dx%d tiles=%d stages=%d splits=%d signs_in=%d signs_out=%d one_tile_per_cluster", kKernelNames[p->kernel], p->sp.pair,
                  p->sp.bn, p->sp.wt, p->sp.ht, p->sp.bt, p->sp.tiles, p->sp.stages, p->sp.splits, p->signs_given ? 1 : 0, p->sp.sign_out ? 1 : 0);
     else if (tc && p->tc_x_ptr && p->tc_taps)
-        snprintf(buf, len, "%s pair=1 halo=0 bn=%d tiles=%d stages=%d+%d epi=2 splits=1 one_load_for_nine_taps%s", kKernelNames[p->kernel], p->tp.bn, p->tp.total_tiles,
-                 p->tp.x_stages, p->tp.w_stages, p->tp.resident ? " resident" : "");
+        snprintf(buf, len, "%s pair=1 halo=0 bn=%d tiles=%d stages=%d+%d epi=2 splits=1 one_load_for_%s%s", kKernelNames[p->kernel], p->tp.bn, p->tp.total_tiles,
+                 p->tp.x_stages, p->tp.w_stages, p->tp.taps == 9 ? "nine_taps" : "a_block", p->tp.resident ? " resident" : "");
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
@@ -669,13 +669,13 @@ static int build_split_args(dnb_conv_plan *p, const dnb_tensor *x, const ConvGeo
 // of 256 to 1024 channels at 1 to 16 images: pairs 0.168 (128 filters) and 0.287 (256), single CTAs 0.317 (256), 0.187 (128) and 0.18 (64)
 // with an SM to themselves, 0.26 and 0.135 where two share one and its room for ring slots.  An epilogue hides behind the next tile's loop, or
 // the other way round, and the last one is exposed.
-static double persistent_us(int pair, int bn, long long tiles, int k_iters, bool residual)
+static double persistent_us(int pair, int bn, long long tiles, int k_iters, bool residual, bool yolo = false)
 {
     const long long slots = pair ? sm_count() / 2 : sm_count();
     const bool shared = !pair && bn <= 128 && tiles > sm_count();
     const double rounds = (double)((tiles + slots - 1) / slots);
     const double iteration = pair ? (bn <= 128 ? 0.168 : 0.287) : bn <= 64 ? (shared ? 0.135 : 0.18) : bn <= 128 ? (shared ? 0.26 : 0.187) : 0.317;
-    const double loop = k_iters * iteration, epilogue = bn * (residual ? 0.02 : 0.015);
+    const double loop = k_iters * iteration, epilogue = bn * (yolo ? 0.06 : residual ? 0.02 : 0.015);   // (a [yolo] layer's logistic: two special functions and a store a value)
     return 4.2 + (pair ? 1.0 : 0.0) + rounds * (loop > epilogue ? loop : epilogue) + 0.8 * epilogue;
 }
 
@@ -787,7 +787,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     a.total_tiles = a.pair ? (ptiles + 1) / 2 * a.n_tiles : ptiles * a.n_tiles;
 }
 
-// ------------------------------------------------------------------ 3x3 layers with one load for nine taps (conv_tc_taps.cu)
+// ------------------------------------------------------------------ 3x3 layers with one load for nine taps, 1x1 layers with their filters in place (conv_tc_taps.cu)
 // The launch's tiles and rings; p->tp holds them.  False where the kernel has no form of it.
 static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channels_last, bool residual)
 {
@@ -796,11 +796,14 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
     a.bf16 = es == 2 ? 1 : 0;
     a.bk = 128 / es;
     a.c_blocks = (p->c_pad + a.bk - 1) / a.bk;
+    a.g = p->g;
+    a.taps = g.size * g.size;
     a.pitch = g.w + 1;
-    a.rows = 128 + 2 * a.pitch + 2;
+    a.rows = a.taps == 1 ? 128 : 128 + 2 * a.pitch + 2;
     if (a.rows > 1024) return false;
-    const long long positions = (long long)g.batch * a.pitch * (g.h + 1) - a.pitch - 1;
+    const long long pixels = (long long)g.batch * g.h * g.w, positions = a.taps == 1 ? pixels : (long long)g.batch * a.pitch * (g.h + 1) - a.pitch - 1;
     if (positions > (1LL << 31) - 4096) return false;
+    a.pixels = (int)pixels;
     a.ptiles = (int)((positions + 127) / 128);
     a.bn = bn;
     a.n_tiles = (p->n_pad + bn - 1) / bn;
@@ -810,17 +813,19 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
     a.x_slot = round_up(a.rows * 128, 1024);
     a.w_bytes = round_up(bn / 2 * 128, 1024);
     a.staged_bytes = channels_last ? (residual ? 65536 : 32768) : 0;
-    a.table = round_up(a.n_tiles * bn, 64) + 64;
+    a.table = round_up(a.n_tiles * bn, 64);
     a.tmem_cols = 32;
     while (a.tmem_cols < 2 * bn) a.tmem_cols *= 2;
     a.x_stages = a.w_stages = 0;
     a.resident = 0;
     const long budget = conv_tc_max_smem() - (long)conv_tc_taps_fixed_smem(a);
-    const int all = 9 * a.c_blocks;
-    if (a.n_tiles == 1 && all <= TAPS_MAX_W && 2L * a.x_slot + (long)all * a.w_bytes <= budget) {
+    const int all = a.taps * a.c_blocks * a.n_tiles, least = a.taps == 1 ? 3 : 2;   // boxes in flight, where they are all that is loaded
+    if ((a.taps == 1 || a.n_tiles == 1) && all <= TAPS_MAX_W && (long)least * a.x_slot + (long)all * a.w_bytes <= budget) {
         a.resident = 1;
         a.w_stages = all;
         a.x_stages = (int)((budget - (long)all * a.w_bytes) / a.x_slot);
+    } else if (a.taps == 1) {
+        a.x_stages = a.w_stages = (int)(budget / (a.x_slot + a.w_bytes));
     } else {
         a.x_stages = 2;
         long left = budget - 2L * a.x_slot;
@@ -830,34 +835,43 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
         if (a.w_stages > 12) a.w_stages = 12;
     }
     if (a.x_stages > TAPS_MAX_X) a.x_stages = TAPS_MAX_X;
-    return a.x_stages >= 2 && a.w_stages >= 3;
+    return a.x_stages >= 2 && (a.resident || a.w_stages >= 3);
 }
 
-// Whether the kernel has a variant for such a launch of the plan.
+// Whether the kernel has a variant for such a launch of the plan.  A 1x1 layer with a residual has not: its addend arrives by TMA, three chunks
+// ahead, in conv_tc.cu (64 -> 256 at 256 x 56 x 56 335 us, 363 here).
 static bool taps_covers(const dnb_conv_plan *p, const ConvEpilogue *res, bool nchw_out)
 {
+    const ConvGeom &g = p->g;
     const int es = p->kernel == K_TC_BF16 ? 2 : 4;
-    if ((p->kernel != K_TC_TF32 && p->kernel != K_TC_BF16) || p->g.size != 3 || p->g.stride != 1 || p->g.pad != 1 || p->keep_k_order) return false;
+    if ((p->kernel != K_TC_TF32 && p->kernel != K_TC_BF16) || g.stride != 1 || p->c_pad * es < 128 || (p->d.activation != DNB_LEAKY && p->d.activation != DNB_LINEAR)) return false;
+    if (g.size == 1) return g.pad == 0 && !(res && res->residual);
+    if (g.size != 3 || g.pad != 1 || p->keep_k_order || (res && res->yolo_entries)) return false;
     if (p->tap_order && p->c_pad * es > 128) return false;   // (one block of channels: there is one order)
-    if (p->c_pad * es < 128 || (p->d.activation != DNB_LEAKY && p->d.activation != DNB_LINEAR) || (res && res->yolo_entries)) return false;
     return !(res && res->residual) ||
-           (res->res_stride == 1 && res->res_c == p->g.n && !nchw_out && res->activation2 == (p->d.activation == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY));
+           (res->res_stride == 1 && res->res_c == g.n && !nchw_out && res->activation2 == (p->d.activation == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY));
 }
 
-// Microseconds of such a launch.  Fitted to 600 measured ones (3x3 layers of 32 to 1024 filters over 32 to 640 channels, maps of 7 to 152, 1 to 128 images, either type and
-// layout; 7 % root mean square): an iteration is the four MMAs of a tap and 128 bytes of channels, 0.174 up to 128 filters and 0.31 at 256; the im2col load
-// takes 3.7 ns a position; a tile's epilogue 6 ns a filter, 19 in Darknet's layout, 27 with a residual.
-static double taps_us(const TapsArgs &a, bool nchw_out, bool residual)
+// Microseconds of such a launch, fitted to 600 measured launches of 3x3 and 1100 of 1x1 layers (32 to 1024 filters over 32 to 2048 channels, maps of 7 to 152, 1 to
+// 128 images, either type and layout; 7 and 12 % root mean square): an iteration is the four MMAs of a tap and 128 bytes of channels, 0.174 up to 128
+// filters and 0.31 at 256, a box for a single tap more; the im2col load takes 3.7 ns a position; a tile's epilogue 6 ns a filter, 19 in Darknet's
+// layout, 27 with a residual.  A 1x1 layer moves its tensors at 6.1 TB/s at most.
+static double taps_us(const TapsArgs &a, bool nchw_out, bool residual, bool yolo)
 {
-    const double clusters = sm_count() / 2, rounds = ceil(a.total_tiles / clusters);
-    const double mma = 9.0 * a.c_blocks * (a.bn <= 128 ? 0.174 : 0.174 + 0.136 * (a.bn - 128) / 128);
-    const double load = a.c_blocks * a.rows * 0.0037, epilogue = a.bn * (nchw_out ? 0.019 : residual ? 0.027 : 0.006);
+    const double clusters = sm_count() / 2, rounds = ceil(a.total_tiles / clusters), wide = a.bn <= 128 ? 0.0 : (a.bn - 128) / 128.0;
+    const double epilogue = a.bn * (yolo ? 0.03 : nchw_out ? 0.019 : residual ? 0.027 : 0.006);
+    if (a.taps == 1) {
+        const double mma = a.c_blocks * (0.26 + 0.103 * wide), bytes = (double)a.pixels * (a.c_blocks * 128.0 + a.g.n * (nchw_out || !a.bf16 ? 4.0 : 2.0));
+        const double tiles = rounds * ((mma > epilogue ? mma : epilogue) + 0.6);
+        return 7.2 + (tiles > bytes / 6.1e6 ? tiles : bytes / 6.1e6);
+    }
+    const double mma = 9.0 * a.c_blocks * (0.174 + 0.136 * wide), load = a.c_blocks * a.rows * 0.0037;
     const double longest = mma > load ? (mma > epilogue ? mma : epilogue) : (load > epilogue ? load : epilogue);
     return 5.3 + rounds * (longest + 0.65) + 0.55 * epilogue + load / a.c_blocks;
 }
 
 // The best tile of a launch of geometry g, in p->tp; its estimated time, or 1e300.
-static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last, bool nchw_out, bool residual)
+static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last, bool nchw_out, bool residual, bool yolo)
 {
     const char *e = getenv("DNB_TC_TAPS_BN");
     const int only = e ? atoi(e) : 0;
@@ -866,21 +880,26 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
     for (int bn = 64; bn <= 256; bn *= 2) {
         const int width = bn < p->n_pad ? bn : p->n_pad;
         if ((only && bn != only) || (bn > 64 && bn / 2 >= p->n_pad) || !taps_tiles(p, g, width, channels_last, residual)) continue;
-        const double us = taps_us(p->tp, nchw_out, residual);
+        const double us = taps_us(p->tp, nchw_out, residual, yolo);
         if (us < best) { best = us; best_bn = width; }
     }
     return best_bn && taps_tiles(p, g, best_bn, channels_last, residual) ? best : 1e300;
 }
 
-// Whether a launch takes that kernel: where its estimate is a tenth below what the others take.  others_us: the estimate of the launch that it would
+// Whether a launch takes that kernel: where its estimate is well below what the others take.  others_us: the estimate of the launch that it would
 // be, cut along K or not.  Those estimates are of launches in a chain; in the measure of taps_us, launches by themselves, cut ones take 1.3 times
-// theirs and whole ones 1.12, in Darknet's layout 1.55 and 1.3 (stores in the short rows of a tile), with a residual 1.25 and 1.05.  On 300 random
+// theirs and whole ones 1.12, in Darknet's layout 1.55 and 1.3 (stores in the short rows of a tile), with a residual 1.25 and 0.95 (1.05 alone, but 64 x 64 x 152 x 152 -> 128
+// is 516 -> 485 us alone and 548 -> 568 inside YOLOv3-608).  On 300 random 3x3
 // launches the rule takes 80 here, 4 of them to their loss (of 5 to 8 %), and all of the launches take 0.947 of what they did: 16 x 256 x 52 x 52
 // -> 512 in Darknet's layout 153 -> 126 us, 2 x 120 x 76 x 76 -> 128 26.8 -> 14.2, 256 x 128 x 28 x 28 -> 128 128 -> 106, 34 x 232 x 38 x 38 -> 255 in bf16 85 -> 42.
 // Launches of many rounds of pairs over 256 filters run into the power cap in either kernel (64 x 256 x 38 x 38 -> 512 265 -> 261 alone, 300 -> 307
 // inside YOLOv3-608) and stay where less padding is multiplied.
-// The kernel adds in another order, so g is that of the whole batch where the plan is for a part of it, and of one image where there are two: an
-// image's sums then hang neither on the parts nor on the other image.
+// The kernel adds the products of a 3x3 layer in another order, so g is that of the whole batch where the plan is for a part of it, and of one image where
+// there are two: an image's sums then hang neither on the parts nor on the other image.
+// 1x1 layers add in the same order and are never cut here: what they gain is that their filters are loaded once (wide tiles, which are at least even alone, take a
+// tenth less power: 64 x 512 x 52 x 52 -> 256 in bf16 53.2 -> 51.9 us alone, 62.9 -> 59.5 back to back) and the stores in
+// Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138, with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch that does not fill the
+// pairs of SMs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
 static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
@@ -889,9 +908,12 @@ static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double other
     if (knob == 0) return false;
     if (!e && (getenv("DNB_TC_PAIR") || getenv("DNB_TC_EPI") || getenv("DNB_TC_HALO") || getenv("DNB_TC_WARP_STORES") || (split && atoi(split) > 1))) return false;
     const bool residual = res && res->residual;
-    const double slack = nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 1.05) : cut ? 1.3 : 1.12;
-    const double us = best_taps(p, g, channels_last, nchw_out, residual);
-    return us < 1e300 && (knob == 2 || us < 0.9 * slack * others_us);
+    const bool yolo = res && res->yolo_entries > 0;
+    const double slack = yolo ? 1.0 : nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 0.95) : cut ? 1.3 : 1.12;
+    const double us = best_taps(p, g, channels_last, nchw_out, residual, yolo);
+    if (us >= 1e300 || knob == 2) return us < 1e300;
+    if (g.size == 1) return !cut && p->tp.total_tiles >= sm_count() / 2 && us < (yolo ? 0.9 : p->tp.resident && p->tp.bn >= 192 ? 1.05 : 0.8) * slack * others_us;
+    return us < 0.9 * slack * others_us;
 }
 
 static int build_taps_args(dnb_conv_plan *p, const dnb_tensor *x, const void *y_nhwc, int y_cpitch)
@@ -899,7 +921,6 @@ static int build_taps_args(dnb_conv_plan *p, const dnb_tensor *x, const void *y_
     TapsArgs &a = p->tp;
     const ConvGeom &g = p->g;
     const int es = a.bf16 ? 2 : 4;
-    a.g = g;
     a.n_pad = p->n_pad;
     const int n8 = round_up(g.n, 8);
     a.y_chan = y_nhwc ? (n8 < y_cpitch ? n8 : y_cpitch) : 0;
@@ -907,8 +928,14 @@ static int build_taps_args(dnb_conv_plan *p, const dnb_tensor *x, const void *y_
     DNB_TRY(ensure_status(p));
     const uint64_t pix = (uint64_t)x->cpitch * es;
     const uint64_t dims[4] = {(uint64_t)p->c_pad, (uint64_t)g.w, (uint64_t)g.h, (uint64_t)g.batch}, strides[3] = {pix, pix * g.w, pix * g.w * g.h};
-    DNB_TRY(encode_im2col_map(&a.tmx, a.bf16, x->data, dims, strides, (uint32_t)a.bk, (uint32_t)a.rows));
-    return encode_weight_map(&a.tmw, p, a.bf16, es, p->c_pad, 9, a.bk, a.bn / 2, 128);
+    if (a.taps == 9) {
+        DNB_TRY(encode_im2col_map(&a.tmx, a.bf16, x->data, dims, strides, (uint32_t)a.bk, (uint32_t)a.rows));
+    } else {
+        const uint64_t flat_dims[3] = {(uint64_t)p->c_pad, (uint64_t)a.pixels, 1}, flat_strides[2] = {pix, pix * a.pixels};
+        const uint32_t box[3] = {(uint32_t)a.bk, 128u, 1u};
+        DNB_TRY(encode_tensor_map(&a.tmx, a.bf16, 3, x->data, flat_dims, flat_strides, box, 128));
+    }
+    return encode_weight_map(&a.tmw, p, a.bf16, es, p->c_pad, a.taps, a.bk, a.bn / 2, 128);
 }
 
 static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, int y_dtype, int y_cpitch,
@@ -1107,7 +1134,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     const SplitPlan cut = may_cut ? cut_at(g) : SplitPlan();
     if (!pool && !i8 && taps_covers(p, res, nchw_out)) {
         const int whole = p->whole_batch > g.batch ? p->whole_batch : g.batch;
-        ConvGeom dg = p->g;
+        ConvGeom dg = g;
         dg.batch = whole <= 2 ? 1 : whole;
         SplitPlan dcut = cut;
         TcArgs da = a;
@@ -1115,9 +1142,9 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             if (may_cut) dcut = cut_at(dg);
             pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
         }
-        const double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, 9 * a.c_blocks, residual != nullptr);
+        const double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, a.taps * a.c_blocks, residual != nullptr, res && res->yolo_entries);
         p->tc_taps = taps_pay(p, dg, dcut.splits != 0, others, res, y_nhwc != nullptr, nchw_out) &&
-                     best_taps(p, g, y_nhwc != nullptr, nchw_out, residual != nullptr) < 1e300;
+                     best_taps(p, g, y_nhwc != nullptr, nchw_out, residual != nullptr, res && res->yolo_entries) < 1e300;
     }
     if (p->tc_taps) DNB_TRY(build_taps_args(p, x, y_nhwc, y_cpitch));
     else if (cut.splits) DNB_TRY(build_split_args(p, x, flat(g), cut, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));

@@ -13,6 +13,8 @@
 // Roles (352 threads, CTA pairs with cta_group::2 MMAs): warp 0 loads filters, warp 10 pixels, warp 1 of the even CTA issues the MMAs, warps 2..9 drain the
 // accumulator: each a chunk of 128 bytes of every pixel of its 32, staged in rows of its own, stored eight lanes a pixel.  No two epilogue warps meet.
 // Where the layer's filters fit shared memory beside two boxes they are loaded once (64 -> 64 in TF32).
+// 1x1 layers run here too (ONE): a position is a pixel of the batch, a plain load of 128 of them serves a block of channels; what is gained there is that the
+// filters stay in shared memory (512 -> 256 in bf16: 128 KB of each CTA of a pair) and the stores in Darknet's layout.
 // K runs over blocks of channels, then taps (conv_tc.cu and conv_tc_split.cu: taps, then blocks).
 //
 // Replaces forward_convolutional_layer_gpu (src/convolutional_kernels.cu:73-135 of the reference), and the shortcut layer after it
@@ -42,6 +44,8 @@ struct TapsShared {
 
 enum { TAPS_WAIT_EMPTY = 101, TAPS_WAIT_FULL = 102, TAPS_WAIT_ACC_EMPTY = 103, TAPS_WAIT_ACC_FULL = 104, TAPS_BAD_SMEM_BASE = 106 };
 
+constexpr int TAPS_YOLO = -3;   // linear, then the logistic of a [yolo] layer on every entry but w and h of each anchor (1x1 layers, Darknet's layout)
+
 template <int ACT>
 __device__ __forceinline__ float taps_act(float x)
 {
@@ -49,12 +53,13 @@ __device__ __forceinline__ float taps_act(float x)
 }
 
 // RES: a residual of the output's shape is added, then ACT2 (the other of the two activations).
-template <int ACT, bool BF16, bool RES>
+// ONE: a 1x1 layer: positions are the pixels of the whole batch, a block of channels has one tap.
+template <int ACT, bool BF16, bool RES, bool ONE>
 __global__ void __launch_bounds__(TAPS_THREADS, 1)
 conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
 {
     constexpr int KIND = BF16 ? MMA_BF16 : MMA_TF32, OES = BF16 ? 2 : 4, CPC = 128 / OES;   // CPC: columns of a chunk
-    constexpr int ACT2 = ACT == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY;
+    constexpr int ACT2 = ACT == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY, TAPS = ONE ? 1 : 9;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t ring = smem_u32(smem_raw);
     if (ring & 1023u) {   // uniform over the pair: both CTAs' windows start at the same offset
@@ -112,13 +117,15 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+        // resident: every filter tile once, in the order of the ring's slots
+        const int begin = resident ? 0 : first_tile, end = resident ? n_tiles : total_tiles, step = resident ? 1 : tile_step;
+        for (int tile = begin; tile < end && ok; tile += step) {
             const int n0 = (tile % n_tiles) * bn + (int)cta_rank * half;
             for (int cb = 0; cb < c_blocks && ok; ++cb)
-                for (int tap = 0; tap < 9; ++tap) {
+                for (int tap = 0; tap < TAPS; ++tap) {
                     ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, TAPS_WAIT_EMPTY, wait_limit);
                     if (!ok) break;
-                    if (withhold && tile == first_tile && cb == c_blocks - 1 && tap == 8) { ok = false; break; }   // wait-expiry test
+                    if (withhold && tile == begin && cb == c_blocks - 1 && tap == TAPS - 1) { ok = false; break; }   // wait-expiry test
                     if (elect_one()) {
                         const uint32_t bar = full0 + 8 * stage;
                         if (leader) mbar_expect_tx(bar, 2u * bytes);
@@ -127,7 +134,6 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                     __syncwarp();
                     if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
-            if (resident) break;
         }
         __syncwarp();
     } else if (warp == 10) {
@@ -142,7 +148,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         grid_dependency_wait();
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int pt = min(pixel_tile(tile), last);   // the second CTA of the last of an odd number of pixel tiles does the first's again, and stores nothing
-            const int at = pt * 128, row = at / pitch, img = row / h1;
+            const int at = pt * 128, row = ONE ? 0 : at / pitch, img = ONE ? 0 : row / h1;
             const int x0 = at - row * pitch - 1, y0 = row - img * h1 - 1;
             for (int cb = 0; cb < c_blocks; ++cb) {
                 ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, TAPS_WAIT_EMPTY, wait_limit);
@@ -150,7 +156,8 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 if (elect_one()) {
                     const uint32_t bar = full0 + 8 * stage;
                     if (leader) mbar_expect_tx(bar, 2u * bytes);
-                    tma_load_im2col_4d_pair(ring + stage * slot_bytes, map, bar, cb * bk, x0, y0, img);
+                    if (ONE) tma_load_3d_pair(ring + stage * slot_bytes, map, bar, cb * bk, at, 0);
+                    else tma_load_im2col_4d_pair(ring + stage * slot_bytes, map, bar, cb * bk, x0, y0, img);
                 }
                 __syncwarp();
                 if (++stage == stages) { stage = 0; phase ^= 1; }
@@ -177,12 +184,13 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * acc_stride;
+                if (resident && n_tiles > 1) { ws = (tile % n_tiles) * c_blocks * TAPS; dw = dw0 + (uint64_t)ws * w_step; }
                 for (int cb = 0; cb < c_blocks && ok; ++cb) {
                     ok = mbar_wait_warp(xf + 8 * xs, xp, abort_flag, status, TAPS_WAIT_FULL, wait_limit);
                     if (!ok) break;
                     uint64_t da = dx;
-                    for (int kh = 0; kh < 3 && ok; ++kh, da += row_step)
-                        for (int kw = 0; kw < 3; ++kw) {
+                    for (int kh = 0; kh < (ONE ? 1 : 3) && ok; ++kh, da += row_step)
+                        for (int kw = 0; kw < (ONE ? 1 : 3); ++kw) {
                             ok = mbar_wait_warp(wf + 8 * ws, wp, abort_flag, status, TAPS_WAIT_FULL, wait_limit);
                             if (!ok) break;
                             tc_fence_after();
@@ -195,7 +203,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                                 }
                                 if (!resident) umma_commit_pair(we + 8 * ws);
                             }
-                            if (kw < 2) da += 8;
+                            if (!ONE && kw < 2) da += 8;
                             dw += w_step;
                             if (++ws == w_stages) { ws = 0; wp ^= resident ? 0u : 1u; dw = dw0; }
                         }
@@ -213,17 +221,24 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         grid_dependency_wait();
         const int group = (warp - 2) >> 2, quarter = warp & 3, chunks = (bn + CPC - 1) / CPC;
         const ConvGeom g = a.g;
-        const int h1 = g.h + 1, ptiles = a.ptiles, y_chan = a.y_chan, do_round = a.ep.round_tf32;
+        const int h1 = g.h + 1, plane = g.h * g.w, ptiles = a.ptiles, y_chan = a.y_chan, do_round = a.ep.round_tf32;
         uint8_t *const y_nhwc = reinterpret_cast<uint8_t *>(a.y_nhwc);
         float *const y_nchw = a.y_nchw;
         const size_t y_pix = (size_t)a.y_cpitch * OES, res_pix = RES ? (size_t)a.ep.res_cpitch * OES : 0;
         const uint8_t *const res_base = reinterpret_cast<const uint8_t *>(a.ep.residual);
         const float alpha = a.ep.alpha, beta = a.ep.beta;
-        const int dbg = a.debug;
+        const int dbg = a.debug, yolo_entries = ACT == TAPS_YOLO ? a.ep.yolo_entries : 1;
         uint8_t *const staged0 = stage_out + (size_t)(warp - 2) * (RES ? 8192 : 4096);
         // the pixel of this lane's position of a tile, -1 for one of the extra column or row, or past the batch
         auto pixel_of = [&](int tile, int &b, int &y, int &x) {
             const int pt = pixel_tile(tile);
+            if (ONE) {   // (b and x: the image and the pixel of its plane, for Darknet's layout only)
+                const int f = pt * 128 + quarter * 32 + lane;
+                b = y = 0;
+                x = f;
+                if (y_nchw) { b = f / plane; x = f - b * plane; }
+                return pt < ptiles && f < a.pixels ? f : -1;
+            }
             const int f = pt * 128 + pitch + 1 + quarter * 32 + lane, row = f / pitch;
             x = f - row * pitch - 1;
             b = row / h1;
@@ -294,6 +309,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 }
                 tmem_ld_wait();
                 const int nl0 = nt * bn + c0;
+                int entry = ACT == TAPS_YOLO ? nl0 % yolo_entries : 0;   // of the chunk's first column: the same for the whole warp
                 const float4 *const sc4 = reinterpret_cast<const float4 *>(s_scale + nl0), *const sf4 = reinterpret_cast<const float4 *>(s_shift + nl0);
 #pragma unroll
                 for (int q = 0; q < CPC / 4; ++q) {
@@ -311,6 +327,10 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         float t = taps_act<ACT>(fmaf(__uint_as_float(r[4 * q + e]), scv[e], sfv[e]));
+                        if (ACT == TAPS_YOLO) {   // forward_yolo_layer_gpu (src/yolo_layer.c:351-357)
+                            if (entry < 2 || entry >= 4) t = __fdividef(1.f, 1.f + __expf(-t));
+                            if (++entry == yolo_entries) entry = 0;
+                        }
                         if (RES) t = taps_act<ACT2>(alpha * t + beta * __uint_as_float(rw[e]));
                         r[4 * q + e] = __float_as_uint(!BF16 && do_round ? round_tf32(t) : t);
                     }
@@ -345,7 +365,6 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 }
                 if (y_nchw && pixel >= 0) {
                     // Darknet's layout: this lane's pixel, a store per filter plane; a warp's positions are runs of rows of the plane
-                    const size_t plane = (size_t)g.h * g.w;
                     float *dst = y_nchw + ((size_t)b * g.n + nl0) * plane + (size_t)y * g.w + x;
                     const int cols = min(min(CPC, bn - c0), g.n - nl0);
 #pragma unroll
@@ -390,12 +409,12 @@ size_t conv_tc_taps_smem(const TapsArgs &a)
 }
 
 typedef void (*TapsKernel)(TapsArgs);
-static TapsKernel taps_kernel(int act, bool bf16, bool res)
+template <int ACT>
+static TapsKernel taps_kernel_of(bool bf16, bool res, bool one)
 {
-    if (act == DNB_LEAKY) return bf16 ? (res ? conv_tc_taps_kernel<DNB_LEAKY, true, true> : conv_tc_taps_kernel<DNB_LEAKY, true, false>)
-                                      : (res ? conv_tc_taps_kernel<DNB_LEAKY, false, true> : conv_tc_taps_kernel<DNB_LEAKY, false, false>);
-    return bf16 ? (res ? conv_tc_taps_kernel<DNB_LINEAR, true, true> : conv_tc_taps_kernel<DNB_LINEAR, true, false>)
-                : (res ? conv_tc_taps_kernel<DNB_LINEAR, false, true> : conv_tc_taps_kernel<DNB_LINEAR, false, false>);
+    if (one) return bf16 ? conv_tc_taps_kernel<ACT, true, false, true> : conv_tc_taps_kernel<ACT, false, false, true>;
+    return bf16 ? (res ? conv_tc_taps_kernel<ACT, true, true, false> : conv_tc_taps_kernel<ACT, true, false, false>)
+                : (res ? conv_tc_taps_kernel<ACT, false, true, false> : conv_tc_taps_kernel<ACT, false, false, false>);
 }
 
 // Resident pairs of a kernel with `smem` bytes, kept for each kernel, size and device.
@@ -426,11 +445,15 @@ static int taps_resident(TapsKernel kern, size_t smem)
 int launch_conv_tc_taps(const TapsArgs &a, cudaStream_t s)
 {
     const int act2 = a.ep.activation == DNB_LEAKY ? DNB_LINEAR : DNB_LEAKY;
-    if ((a.ep.activation != DNB_LEAKY && a.ep.activation != DNB_LINEAR) || (a.ep.residual && (a.ep.activation2 != act2 || !a.y_nhwc)) || a.ep.yolo_entries)
+    const bool yolo = a.ep.yolo_entries > 0;
+    if ((a.ep.activation != DNB_LEAKY && a.ep.activation != DNB_LINEAR) || (a.ep.residual && (a.ep.activation2 != act2 || !a.y_nhwc || a.taps == 1)) ||
+        (yolo && (a.ep.activation != DNB_LINEAR || a.ep.residual || a.y_nhwc || a.taps != 1)))
         DNB_FAIL(DNB_EINVAL, "conv_tc_taps: no variant of this epilogue");
-    if (a.bn < 16 || a.bn > 256 || a.bn % 16 || a.x_stages < 2 || a.x_stages > TAPS_MAX_X || a.w_stages < 2 || a.w_stages > TAPS_MAX_W || a.rows > 1024)
+    if (a.bn < 16 || a.bn > 256 || a.bn % 16 || a.x_stages < 2 || a.x_stages > TAPS_MAX_X || a.w_stages < 1 || a.w_stages > TAPS_MAX_W || a.rows > 1024)
         DNB_FAIL(DNB_EINVAL, "conv_tc_taps: plan out of range (bn %d, stages %d and %d, rows %d)", a.bn, a.x_stages, a.w_stages, a.rows);
-    const TapsKernel kern = taps_kernel(a.ep.activation, a.bf16 != 0, a.ep.residual != nullptr);
+    const TapsKernel kern = yolo ? (a.bf16 ? conv_tc_taps_kernel<TAPS_YOLO, true, false, true> : conv_tc_taps_kernel<TAPS_YOLO, false, false, true>)
+                                 : a.ep.activation == DNB_LEAKY ? taps_kernel_of<DNB_LEAKY>(a.bf16 != 0, a.ep.residual != nullptr, a.taps == 1)
+                                                                : taps_kernel_of<DNB_LINEAR>(a.bf16 != 0, a.ep.residual != nullptr, a.taps == 1);
     const size_t smem = conv_tc_taps_smem(a);
     DNB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tc_max_smem()));
     const int most = taps_resident(kern, smem);

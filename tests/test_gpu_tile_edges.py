@@ -782,3 +782,45 @@ def test_one_load_for_nine_taps_wait_expiry(monkeypatch):
     torch.cuda.synchronize()
     plan.check_status()
     assert np.array_equal(host_from_nhwc(yt, good.shape[1]), good)
+
+
+ONES = {   # 1x1 layers on the same kernel: pixels beyond the last tile, ragged channels, filters in place and in a ring, half a chunk of filters
+    "in_place": dict(b=3, c=64, h=19, w=17, n=64, size=1),
+    "one_pixel": dict(b=1, c=72, h=1, w=1, n=24, size=1, act="linear"),
+    "in_place_two_filter_tiles": dict(b=5, c=96, h=13, w=14, n=320, size=1),
+    "a_ring": dict(b=2, c=1032, h=13, w=13, n=250, size=1),
+    "rounds_of_tiles": dict(b=9, c=128, h=52, w=51, n=255, size=1, act="linear", bn=False),
+}
+
+
+@pytest.mark.parametrize("name", list(ONES))
+@pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
+def test_1x1_layers_with_their_filters_in_place(name, mode, tol, monkeypatch):
+    """The same products in the same order as in the kernel with a ring: equal to the bit, in either layout; with a [yolo] layer's logistic too."""
+    import ctypes as C
+    import numpy as np
+    import torch
+    from gpu_util import dev_nhwc, empty_nchw
+    case = conv_case(770, **ONES[name])
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    out = {}
+    for knob in ("0", "2"):
+        monkeypatch.setenv("DNB_TC_TAPS", knob)
+        plan, a, b = run_conv(case, mode, "nhwc", "nchw", both=True)
+        assert ("one_load_for_a_block" in plan.describe()) == (knob == "2"), plan.describe()
+        _, c, _ = run_conv(case, mode, "nhwc", "nhwc")
+        _, d, _ = run_conv(case, mode, "nchw", "nchw")
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+        out[knob] = [a, d]
+        if case["act"] == "linear":
+            n = a.shape[1]
+            xt, xd = dev_nhwc(case["x"], torch.bfloat16 if mode == dn.MODE_BF16 else torch.float32)
+            yt, yd = empty_nchw(*a.shape)
+            stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+            dn.check(dn.lib().dnb_conv_yolo_forward(plan.handle, C.byref(xd), C.byref(yd), 3, n // 3 - 5, stream))
+            torch.cuda.synchronize()
+            plan.check_status()
+            out[knob].append(yt.cpu().numpy())
+    for a, b in zip(out["0"], out["2"]):
+        assert np.array_equal(a, b)
+    parity(out["2"][0], oracle_conv(case), tol)
