@@ -95,8 +95,8 @@ struct alignas(64) TcArgs {
     int stage_bufs;       // staging buffers of the epilogue: 2, or 4 with a fused residual (it lands in them first), 3 with signs, 0 where two groups write Darknet's layout only
     int pair;             // 1: clusters of two CTAs share every MMA (cta_group::2); total_tiles then counts PAIRS of pixel tiles,
                           // b_bytes and the weight map's box cover half a filter tile, bn is 128 or 256
-    int ctas_per_sm;      // 2 for narrow tiles (TMEM and shared memory are sized so that two CTAs share an SM), else 1
-    int pool;             // 1: tmy (and tms) are the 2x2 stride-2 maxpool's output; wt and ht are even
+    int ctas_per_sm;      // 2 for narrow tiles (TMEM and shared memory are sized so that two CTAs share an SM), up to 4 for pooled ones, else 1
+    int pool;             // 1: y_nhwc (and sign_out) are the 2x2 stride-2 maxpool's output, plain stores; wt and ht are even, wt at most 16
     int epi_groups;       // groups of four epilogue warps: 2 where a CTA has its SM to itself and staged rows are 128 bytes, else 1
     int a_bytes, b_bytes; // shared-memory bytes of one stage's activation / weight tile (1024-multiples)
     int store_row_bytes;  // bytes of one staged output row (128, 64 or 32) = swizzle span of tmy

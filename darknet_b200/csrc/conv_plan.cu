@@ -442,7 +442,7 @@ static void pick_pixel_tile(const ConvGeom &g, bool nchw_out, int *wt, int *ht, 
     double best = 1e300;
     for (int w = 1; w <= 128; w *= 2)
         for (int h = 1; w * h <= 128; h *= 2) {
-            if (even && (w < 2 || h < 2)) continue;
+            if (even && (w < 2 || h < 2 || w > 16)) continue;   // a warp's lanes hold whole windows
             const int b = 128 / (w * h);
             const double work = (double)round_up(g.out_w, w) * round_up(g.out_h, h) * round_up(g.batch, b);
             double score = work * (1.0 + 1e-6 * (128 - w) + 1e-7 * (128 - h));
@@ -996,7 +996,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // twice the warps hide the per-tile hand-offs that dominate layers with few K iterations.
     a.ctas_per_sm = 1;
     a.stage_bufs = residual ? 4 : 2;
-    if (sign_out && !pool) a.stage_bufs = 3;   // the third buffer holds the staged signs (pooled rows and theirs fit the second one)
+    if (sign_out) a.stage_bufs = 3;   // the third buffer holds the staged signs
+    if (pool) a.stage_bufs = 0;       // pooled rows leave from registers
     a.sign_out = sign_out;
     a.sign_cpitch = sign_cpitch;
     int stages = 0;
@@ -1010,6 +1011,9 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // 16 x 208 x 208 72 -> 49.  One CTA alone with its weights is slower than two without (32 -> 64 in TF32 854 -> 900, 64 -> 128 in bf16 at 152 x
     // 152 280 -> 390, of xnor layers at 56 x 56 79 -> 95, 32 -> 64 with stride 2 in bf16 685 -> 790).  Same order of the sums.
     // DNB_TC_HALO: 0 never, 2 wherever the geometry and shared memory allow.
+    // Pooled launches stage nothing and their epilogue is the longer part: as many CTAs as TMEM takes (xnor 32 -> 64 at 128 x 112 x 112 103 us with two, 93 with
+    // three, 90 with four; 16 -> 32 in TF32 at 16 x 208 x 208 49, 42, 37)
+    const int most_ctas = pool && a.tmem_cols <= 128 ? 4 : 2;
     const int halo_knob = getenv("DNB_TC_HALO") ? atoi(getenv("DNB_TC_HALO")) : 1;
     if (halo_knob != 0 && g.size == 3 && g.pad == 1 && a.n_tiles == 1 && !a.pair && g.out_w >= 8 && g.out_h >= 16) {
         const int lattices = g.stride * g.stride, htiles = ((g.out_w + 7) / 8) * ((g.out_h + 15) / 16) * g.batch;
@@ -1029,7 +1033,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         if (halo_knob == 2 || (htiles >= 2 * sm_count() && htiles <= 1.2 * a.total_tiles)) {
             const int widest = srb;
             if (allow2 && a.tmem_cols <= 256 && htiles > sm_count())
-                for (int t = widest; t >= min_srb && !done; t /= 2) { done = fit((228L * 1024) / 2 - 2048, t, 4); if (done) a.ctas_per_sm = 2; }
+                for (int n = most_ctas; n >= 2 && !done; --n)
+                    for (int t = widest; t >= min_srb && !done; t /= 2) { done = fit((228L * 1024) / n - 2048, t, 4); if (done) a.ctas_per_sm = n; }
             for (int t = widest; halo_knob == 2 && t >= min_srb && !done; t /= 2) done = fit(max_smem, t, 4);
             if (!done) srb = widest;
         }
@@ -1162,15 +1167,14 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         DNB_TRY(encode_input_maps(a.tmx, g, x, kind, es, c_pad, box, a.row_bytes));
         DNB_TRY(encode_weight_map(&a.tmw, p, kind, es, c_pad, a.taps, a.bk, a.pair ? a.bn / 2 : a.bn, a.row_bytes));
     }
-    if (y_nhwc) {
+    if (y_nhwc && !pool) {
         const size_t opix = (size_t)y_cpitch * out_es;
         // the channel extent is the layer's own (padded to 8), the pitch whatever the tensor has: the output may be a
         // channel range of a wider tensor (a [route] output), and the boxes must not spill into its neighbour
         const int y_chan = round_up(g.n, 8) < y_cpitch ? round_up(g.n, 8) : y_cpitch;
-        const int half = pool ? 2 : 1, yw = g.out_w / half, yh = g.out_h / half;
-        uint64_t dims[4] = {(uint64_t)y_chan, (uint64_t)yw, (uint64_t)yh, (uint64_t)g.batch};
-        uint64_t strides[3] = {opix, opix * yw, opix * yw * yh};
-        uint32_t box[4] = {(uint32_t)(srb / out_es), (uint32_t)(a.wt / half), (uint32_t)(a.ht / half), (uint32_t)a.bt};
+        uint64_t dims[4] = {(uint64_t)y_chan, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
+        uint64_t strides[3] = {opix, opix * g.out_w, opix * g.out_w * g.out_h};
+        uint32_t box[4] = {(uint32_t)(srb / out_es), (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
         DNB_TRY(encode_tensor_map(&a.tmy, bf16, 4, y_nhwc, dims, strides, box, srb));
         {   // the 32 consecutive rows of one epilogue warp: wt*ht*bt = 128 in powers of two, so they are a box too
             const int w2 = a.wt < 32 ? a.wt : 32, h2 = a.ht < 32 / w2 ? a.ht : 32 / w2, b2 = 32 / (w2 * h2);
@@ -1187,11 +1191,10 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             DNB_TRY(encode_tensor_map(&a.tmr, bf16, 4, const_cast<void *>(residual), rdims, rstrides, box, srb));
         }
     }
-    if (sign_out) {
-        const int half = pool ? 2 : 1, yw = g.out_w / half, yh = g.out_h / half;
-        uint64_t dims[4] = {(uint64_t)sign_cpitch, (uint64_t)yw, (uint64_t)yh, (uint64_t)g.batch};
-        uint64_t strides[3] = {(uint64_t)sign_cpitch, (uint64_t)sign_cpitch * yw, (uint64_t)sign_cpitch * yw * yh};
-        uint32_t box[4] = {32u, (uint32_t)(a.wt / half), (uint32_t)(a.ht / half), (uint32_t)a.bt};
+    if (sign_out && !pool) {
+        uint64_t dims[4] = {(uint64_t)sign_cpitch, (uint64_t)g.out_w, (uint64_t)g.out_h, (uint64_t)g.batch};
+        uint64_t strides[3] = {(uint64_t)sign_cpitch, (uint64_t)sign_cpitch * g.out_w, (uint64_t)sign_cpitch * g.out_w * g.out_h};
+        uint32_t box[4] = {32u, (uint32_t)a.wt, (uint32_t)a.ht, (uint32_t)a.bt};
         DNB_TRY(encode_tensor_map(&a.tms, 2, 4, sign_out, dims, strides, box, 32));
     }
     p->tc_sign_out = sign_out;

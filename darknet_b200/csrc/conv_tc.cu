@@ -142,8 +142,10 @@ __device__ __forceinline__ void group_bar(int group) { asm volatile("bar.sync %0
 // its operand: that layer's sign pass over the f32 tensor disappears.  The signs of a chunk are staged in a third
 // staging buffer (two 4 KB halves in rotation) and leave with the chunk's output rows, in the same bulk group.
 // POOL: the output is that of the 2x2 maxpool with stride 2 after the layer (forward_maxpool_layer, src/maxpool_layer.c:79-114); the layer's own
-// is not written.  A chunk's finished rows are staged as ever, a thread takes the largest of four of them, for a quarter of a pooled pixel, and what leaves is
-// a box of a quarter of the pixels: of the two passes' bytes, 9 per output value of the layer, one is left, and one launch.
+// is not written.  Of the two passes' bytes, 9 per output value of the layer, one is left, and one launch.  The four pixels of a window are lanes of one warp
+// (tiles are at most 16 pixels wide), which exchange halves of their columns and keep the larger values, twice: a lane ends with 32 bytes of a pooled pixel, one
+// store.  No row is staged and no warp waits for another; through staged rows and three
+// barriers a chunk xnor 32 -> 64 at 128 x 112 x 112 took 138 us, 64 -> 128 at 56 x 56 88, 128 -> 256 at 28 x 28 61; this 78, 49 and 35.
 // EG: groups of four epilogue warps.  Two CTAs on an SM bring eight epilogue warps between them; one CTA with four has every SM
 // sub-partition wait for a single warp's chain of TMEM read, residual, arithmetic, staging and store.  The second group takes alternate
 // chunks, with staged rows, a barrier and a storing thread of its own; with a residual (pairs) every warp is on its own, fetches the
@@ -431,6 +433,100 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
             }
         }
         __syncwarp();
+    } else if constexpr (POOL) {
+        // ---------------- epilogue, pooled output: warps 2..5 own TMEM lanes 32*(warp%4) .. +31
+        grid_dependency_wait();
+        const int quarter = warp & 3, m = quarter * 32 + lane;
+        const int wl = m % wt, hl = (m / wt) % ht, bl = m / (wt * ht);
+        const ConvGeom g = a.g;
+        const int do_round = a.ep.round_tf32, n_pad = a.n_pad, y_cpitch = a.y_cpitch, sign_cpitch = a.sign_cpitch, dbg = a.debug;
+        uint8_t *const y_nhwc = reinterpret_cast<uint8_t *>(a.y_nhwc);
+        int8_t *const sign_out = SIGNS ? reinterpret_cast<int8_t *>(a.sign_out) : nullptr;
+        const float *const ep_scale = a.ep.scale, *const ep_shift = a.ep.shift;
+        int *status = a.status;
+        const bool right = (lane & 1) != 0, below = (lane & wt) != 0;   // of the window's pixels
+        constexpr int OES = OUT_BF16 ? 2 : 4, WORDS = 32;               // 128 bytes of every pixel a chunk
+        const bool sectors = (((uintptr_t)y_nhwc | (uintptr_t)y_cpitch * OES) & 31u) == 0;   // (bf16 tensors of an odd number of 8 channels: not)
+        int it = 0, loaded_nt = -1;
+        for (int tile = first_tile; tile < total_tiles; tile += grid_stride, ++it) {
+            const int acc = it & 1, nt = tile % n_tiles, pt = tile / n_tiles;
+            const int ow = (pt % tiles_w) * wt + wl, oh = ((pt / tiles_w) % tiles_h) * ht + hl, b = (pt / ptiles_wh) * bt + bl;
+            const bool pix_ok = ow < g.out_w && oh < g.out_h && b < g.batch;
+            const size_t pixel = ((size_t)b * (g.out_h >> 1) + (oh >> 1)) * (g.out_w >> 1) + (ow >> 1);
+            if (nt != loaded_nt) {
+                epilogue_bar();   // every warp is done with the last filter tile's vectors
+                for (int i = threadIdx.x - 64; i < bn + 64; i += 128) {
+                    const int gi = nt * bn + i;
+                    const bool in = i < bn && gi < n_pad;
+                    s_scale[i] = in ? __ldg(ep_scale + gi) : 0.f;
+                    s_shift[i] = in ? __ldg(ep_shift + gi) : 0.f;
+                }
+                loaded_nt = nt;
+            }
+            const bool fine = mbar_wait(smem_u32(&sh->acc_full[acc]), (it >> 1) & 1, abort_flag, status, WAIT_ACC_FULL, 0, wait_limit);
+            if (!epilogue_agree<128>(fine && !*abort_flag)) break;
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * acc_stride;
+#pragma unroll 1
+            for (int c0 = (dbg & 8) ? bn : 0; c0 < bn; c0 += CPC) {
+                uint32_t r[CPC];
+#pragma unroll
+                for (int u = 0; u < CPC / 16; ++u) {
+                    if (c0 + 16 * u < bn) {
+                        tmem_ld16(t_row + c0 + 16 * u, *reinterpret_cast<uint32_t(*)[16]>(&r[16 * u]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[16 * u + j] = 0u;
+                    }
+                }
+                tmem_ld_wait();
+                const float4 *const sc4 = reinterpret_cast<const float4 *>(s_scale + c0), *const sf4 = reinterpret_cast<const float4 *>(s_shift + c0);
+                uint32_t v[WORDS];   // the finished values, as they would be stored
+#pragma unroll
+                for (int q = 0; q < CPC / 4; ++q) {
+                    const float4 sc = sc4[q], sf = sf4[q];
+                    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
+                    float t[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)   // (an xnor layer's activation does not change which value is the largest: it follows, on a quarter of them)
+                        t[e] = I8 ? fmaf((float)(int)r[4 * q + e], scv[e], sfv[e]) : finish_value<ACT, ACT2_NONE, OUT_BF16, false>(r[4 * q + e], scv[e], sfv[e], 0.f, 1.f, 0.f, 0, 0, do_round, 0);
+                    if (!OUT_BF16) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[(4 * q + e) % WORDS] = __float_as_uint(t[e]);
+                    } else {
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(t[0], t[1]), hi = __floats2bfloat162_rn(t[2], t[3]);
+                        v[(2 * q) % WORDS] = *reinterpret_cast<const uint32_t *>(&lo);
+                        v[(2 * q + 1) % WORDS] = *reinterpret_cast<const uint32_t *>(&hi);
+                    }
+                }
+                // the window's other column, then its other row: a lane gives away the half that its neighbour keeps
+                uint32_t h[16], o[8];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) h[j] = larger<OUT_BF16>(right ? v[16 + j] : v[j], __shfl_xor_sync(0xffffffffu, right ? v[j] : v[16 + j], 1));
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = larger<OUT_BF16>(I8 ? 0xffffffffu : lowest<OUT_BF16>(), larger<OUT_BF16>(below ? h[8 + j] : h[j], __shfl_xor_sync(0xffffffffu, below ? h[j] : h[8 + j], wt)));
+                if (I8)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) o[j] = larger<false>(lowest<false>(), __float_as_uint(act_apply<ACT>(__uint_as_float(o[j]), 0)));
+                const int ch = nt * bn + c0 + ((right ? 16 : 0) + (below ? 8 : 0)) * (4 / OES);   // (a layer's filters are a multiple of 8, of 16 in bf16 but for a last half)
+                if (pix_ok && ch < g.n && !(dbg & 2)) {
+                    uint8_t *const dst = y_nhwc + (pixel * y_cpitch + ch) * OES;
+                    if (sectors && (!OUT_BF16 || ch + 8 < g.n)) {
+                        st_global_32(dst, o);
+                    } else {
+                        *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+                        if (!OUT_BF16 || ch + 8 < g.n) *reinterpret_cast<uint4 *>(dst + 16) = make_uint4(o[4], o[5], o[6], o[7]);
+                    }
+                    if (SIGNS) {
+                        const uint2 sg = make_uint2(four_signs(make_uint4(o[0], o[1], o[2], o[3])), four_signs(make_uint4(o[4], o[5], o[6], o[7])));
+                        *reinterpret_cast<uint2 *>(sign_out + pixel * sign_cpitch + ch) = sg;
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[acc]));
+        }
     } else if constexpr (EG == 2) {
         // ---------------- epilogue, two groups: warps 2..9, TMEM lanes 32*(warp%4) .. +31, chunks group, group + 2, ...
         grid_dependency_wait();
@@ -674,7 +770,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
         // output like the whole tile is, and sends them off itself; the four warps then meet once per tile instead of
         // twice per chunk, so one warp's TMEM or store wait no longer stalls the other three.
         constexpr bool can_warp_store = ACT2 == ACT2_NONE;
-        const bool warp_stores = can_warp_store && !SIGNS && !POOL && a.warp_stores != 0 && a.y_nhwc != nullptr;
+        const bool warp_stores = can_warp_store && !SIGNS && a.warp_stores != 0 && a.y_nhwc != nullptr;
         const int m0 = quarter * 32;
         const int wl0 = m0 % wt, hl0 = (m0 / wt) % ht, bl0 = m0 / (wt * ht);   // origin of this warp's rows inside the tile
         constexpr bool out_bf16 = OUT_BF16;
@@ -793,11 +889,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 }
                 const uint32_t buf = chunk_count & buf_mask;
-                uint8_t *const pooled = stage_out + 128 * srb + (size_t)(chunk_count & 1u) * 5120;   // POOL: 32 rows of 128 bytes, and of 32 of signs
-                if (POOL) {
-                    if (store_thread && chunk_count >= 2) tma_store_wait_read1();   // the store that last read these pooled rows is done
-                    epilogue_bar();                                                 // ... and everybody with the last chunk's staged rows
-                } else if (!res_tiles) {
+                if (!res_tiles) {
                     if (warp_stores) {
                         if (lane == 0 && chunk_count >= 2) tma_store_wait_read1();   // this warp's store that last read its rows of the buffer is done
                         __syncwarp();
@@ -807,7 +899,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 }   // with a residual the buffer is this thread's to overwrite: its tile landed after that store, and
                     // a thread reads and writes its own row only
-                uint8_t *row = stage_out + (size_t)(POOL ? 0u : buf) * 128 * srb + (size_t)m * srb;
+                uint8_t *row = stage_out + (size_t)buf * 128 * srb + (size_t)m * srb;
                 if (!out_bf16) {
 #pragma unroll
                     for (int q = 0; q < srb / 16; ++q)         // 16-byte pieces of 4 floats
@@ -817,29 +909,6 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     for (int q = 0; q < srb / 16; ++q)         // 16-byte pieces of 8 bf16
                         *reinterpret_cast<uint4 *>(row + ((q ^ q_xor) << 4)) = pack_bf16x8<CPC>(r, 8 * q);
                 }
-                if (POOL) {
-                    epilogue_bar();
-                    // pooled pixel et / 4 (half the tile's extents), 16-byte pieces et % 4 and that + 4 of its row
-                    const int et = threadIdx.x - 64, pp = et >> 2, pw = wt >> 1, ph = ht >> 1;
-                    const int top = ((pp / (pw * ph)) * ht + 2 * (pp / pw % ph)) * wt + 2 * (pp % pw);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int q = (et & 3) + 4 * h;
-                        uint4 v[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int rr = top + (i & 1) + (i >> 1) * wt;
-                            v[i] = *reinterpret_cast<const uint4 *>(stage_out + (size_t)rr * srb + ((q ^ (rr & 7)) << 4));
-                        }
-                        const uint4 o = largest_of_four<OUT_BF16>(v);
-                        *reinterpret_cast<uint4 *>(pooled + pp * 128 + ((q ^ (pp & 7)) << 4)) = o;
-                        if (SIGNS) {   // of the pooled values, 4 channels a word
-                            const int left = nvalid - 4 * q;   // real filters among the four
-                            const uint32_t wd = four_signs(o) & (left >= 4 ? ~0u : left > 0 ? (1u << (8 * left)) - 1u : 0u);
-                            *reinterpret_cast<uint32_t *>(pooled + 4096 + pp * 32 + (((q >> 2) ^ ((pp >> 2) & 1)) << 4) + 4 * (q & 3)) = wd;
-                        }
-                    }
-                } else
                 if (SIGNS) {
                     // 32 signs of this pixel = one 32-byte row of a 32-byte-swizzled box: its two 16-byte halves swap on rows 4..7 of every 8
                     uint32_t sw[8];
@@ -869,13 +938,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                     }
                 } else
                 epilogue_bar();
-                if (POOL) {
-                    if (store_thread) {
-                        if (!(dbg & 2)) tma_store_4d(ymap, smem_u32(pooled), nl0, ow0 >> 1, oh0 >> 1, b0);
-                        if (SIGNS) tma_store_4d(&a.tms, smem_u32(pooled + 4096), nl0, ow0 >> 1, oh0 >> 1, b0);
-                        tma_store_commit();
-                    }
-                } else if (!warp_stores && store_thread) {
+                if (!warp_stores && store_thread) {
                     // the TMA unit clips the box at the tensor's extents: ragged tiles need no predicates
                     if (y_nhwc && !(dbg & 2) && (!PAIR || b0 < g.batch)) tma_store_4d(ymap, smem_u32(stage_out + (size_t)buf * 128 * srb), nl0, ow0, oh0, b0);
                     if (SIGNS && (!PAIR || b0 < g.batch))
@@ -888,7 +951,7 @@ conv_tc_kernel(const __grid_constant__ TcArgs a)
                         request_residual();
                     }
                 }
-                if (!POOL && y_nchw && pix_ok) {
+                if (y_nchw && pix_ok) {
                     // Darknet-layout copy: this thread's pixel, one filter plane per column, straight from the registers
                     // (a warp's 32 pixels are wt-long runs of each plane).  BF16 plans write what the channels-last
                     // copy holds: the value rounded to bf16.
@@ -1037,7 +1100,7 @@ int launch_conv_tc(const TcArgs &a, cudaStream_t s)
     if (a.epi_groups == 2 && a.store_row_bytes != 128) DNB_FAIL(DNB_EINVAL, "conv_tc: two epilogue groups need 128-byte staged rows");
     if (a.pair && !((!obf && cpc == 32) || (obf && cpc == 64))) DNB_FAIL(DNB_EINVAL, "conv_tc: pair mode needs 128-byte staged rows");
     if (a.pool) {
-        if (a.pair || a.epi_groups != 1 || a.store_row_bytes != 128 || a.ep.activation != DNB_LEAKY || a.ep.residual || a.ep.yolo_entries || a.y_nchw || (a.wt | a.ht) & 1)
+        if (a.pair || a.epi_groups != 1 || a.store_row_bytes != 128 || a.ep.activation != DNB_LEAKY || a.ep.residual || a.ep.yolo_entries || a.y_nchw || (a.wt | a.ht) & 1 || a.wt > 16)
             DNB_FAIL(DNB_EINVAL, "conv_tc: no pooled variant of this launch");
         if (i8 && a.sign_out) DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 32, false, ACT2_NONE, false, true, true, 1, true>, a, smem, s));
         else if (i8) DNB_TRY(launch_one(conv_tc_kernel<DNB_LEAKY, 32, false, ACT2_NONE, false, true, false, 1, true>, a, smem, s));

@@ -91,6 +91,16 @@ __device__ __forceinline__ uint4 largest_of_four(const uint4 (&v)[4])
     return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
+// The larger of two floats, or of two pairs of bf16 values; a NaN never wins.  lowest: what a maxpool starts from (in bf16 it rounds to -infinity).
+template <bool BF16>
+__device__ __forceinline__ uint32_t larger(uint32_t a, uint32_t b)
+{
+    if (!BF16) return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+    const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162 *>(&a), *reinterpret_cast<const __nv_bfloat162 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&m);
+}
+template <bool BF16> __device__ __forceinline__ uint32_t lowest() { return BF16 ? 0xff80ff80u : 0xff7fffffu; }
+
 // Signs of four floats as bytes: +1 where > 0, else -1.
 __device__ __forceinline__ uint32_t four_signs(uint4 v)
 {

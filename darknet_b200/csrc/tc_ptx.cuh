@@ -299,6 +299,12 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool i
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// a whole 32-byte sector, 32-byte aligned
+__device__ __forceinline__ void st_global_32(void *dst, const uint32_t (&v)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
 // asks for `bytes` (a multiple of 16) at a 16-byte aligned address to be brought into L2
 __device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes)
 {
