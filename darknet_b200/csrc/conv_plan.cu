@@ -1528,7 +1528,7 @@ bool conv_pool_fusable(dnb_conv_plan *p, bool in_order)
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR && p->xnor_tc;
     if (p->stem_tc) {
         const int dtype = p->mode == DNB_MODE_BF16 ? DNB_BF16 : DNB_F32;
-        if (!conv_stem_pool_covers(g, dtype, p->d.activation) || g.w >= (1 << 25) || (in_order && !conv_stem_rows_pool_covers(g, dtype))) return false;
+        if (!conv_stem_pool_covers(g, dtype, p->d.activation) || g.w >= (1 << 25) || (in_order && (g.w >= (1 << 22) || !conv_stem_rows_pool_covers(g, dtype)))) return false;   // (32-bit offsets inside a tile's patch)
         p->pool_fits = 1;
         return true;
     }

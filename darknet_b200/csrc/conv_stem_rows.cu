@@ -45,9 +45,7 @@ __device__ __forceinline__ float rows_act(float x, int runtime_act)
 
 // C: input channels (1..3); ACT: activation folded at compile time or SR_ACT_GENERIC; OUT_BF16: storage
 // type of the channels-last output.
-// POOL (f32, 32 filters): the output is that of the 2x2 maxpool with stride 2 after the layer, and optionally its signs, the next xnor layer's operand.
-// Four neighbouring threads own the pixels of a window: a warp takes the largest of each four staged rows and stores eight.
-template <int C, int ACT, bool OUT_BF16, bool POOL = false>
+template <int C, int ACT, bool OUT_BF16>
 __global__ void __launch_bounds__(SR_THREADS, 5)
 conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
 {
@@ -104,7 +102,7 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
     const float *const x = a.x;
     const long long xs_b = a.xs_b;
     const int xs_c = (int)a.xs_c, xs_h = (int)a.xs_h, xs_w = (int)a.xs_w;
-    const int npix = a.npix, tiles = a.tiles, plane = POOL ? (g.out_h >> 1) * (g.out_w >> 1) : g.out_h * g.out_w;   // POOL: windows
+    const int npix = a.npix, tiles = a.tiles, plane = g.out_h * g.out_w;
     const int runtime_act = a.ep.activation, do_round = a.ep.round_tf32;
     uint8_t *const y = reinterpret_cast<uint8_t *>(a.y);
     const size_t y_row_bytes = (size_t)a.y_cpitch * (OUT_BF16 ? 2 : 4);
@@ -129,17 +127,14 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
     for (int tile = blockIdx.x;; tile += gridDim.x, ++it) {
         const bool have = tile < tiles;   // uniform over the CTA
         const int buf = it & 1;
-        long long keep_at = -1;           // POOL: where this thread's pixel lies in the copy of the images
         // ---- this thread's 27 input values of the next tile: requested first, used after the epilogue below
         float v[K];
         if (have) {
-            const int p = POOL ? tile * (SR_THREADS / 4) + (tid >> 2) : tile * SR_THREADS + tid;   // POOL: in windows
+            const int p = tile * SR_THREADS + tid;
             const bool valid = p < npix;
-            const int b = p / plane, rem = p - b * plane, row_w = POOL ? g.out_w >> 1 : g.out_w;
-            const int py = rem / row_w, px = rem - py * row_w;
-            const int oy = POOL ? 2 * py + ((tid >> 1) & 1) : py, ox = POOL ? 2 * px + (tid & 1) : px;
+            const int b = p / plane, rem = p - b * plane;
+            const int oy = rem / g.out_w, ox = rem - oy * g.out_w;
             const int iy0 = oy * g.stride - g.pad, ix0 = ox * g.stride - g.pad;
-            if (POOL && a.keep && valid) keep_at = b * xs_b + (long long)oy * xs_h + ox;
             // three row and three column validity flags and one base pointer: a tap costs one predicated load
             const bool rv0 = valid && (unsigned)iy0 < (unsigned)g.h, rv1 = valid && (unsigned)(iy0 + 1) < (unsigned)g.h,
                        rv2 = valid && (unsigned)(iy0 + 2) < (unsigned)g.h;
@@ -212,33 +207,7 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
                         }
                     }
                 }
-                if (POOL) {
-                    __syncwarp();
-                    uint8_t *const mine = sA + pb * SR_A_BYTES + warp * 32 * 128;
-                    const int k = lane >> 2, first = prev_tile * (SR_THREADS / 4) + warp * 8;   // the warp's first window
-                    uint4 best[2];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int q = (lane & 3) + 4 * h;
-                        uint4 v4[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) v4[i] = *reinterpret_cast<const uint4 *>(mine + (4 * k + i) * 128 + ((q ^ ((4 * k + i) & 7)) << 4));
-                        best[h] = largest_of_four<false>(v4);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int q = (lane & 3) + 4 * h;
-                        *reinterpret_cast<uint4 *>(mine + k * 128 + ((q ^ k) << 4)) = best[h];
-                        if (a.signs && first + k < npix) *reinterpret_cast<uint32_t *>(a.signs + (size_t)(first + k) * 32 + 4 * q) = four_signs(best[h]);
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && first < npix) {
-                        tma_store_2d(ymap, smem_u32(mine), 0, first);
-                        tma_store_commit();
-                    }
-                } else if (tma) {
+                if (tma) {
                     // each warp stores its own 32 rows: no CTA-wide barrier between the rows and the store
                     fence_async_smem();
                     __syncwarp();
@@ -258,10 +227,6 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
                 // Staged rows narrower than an im2col row (fewer than 128 bytes of output per pixel) put this thread's
                 // im2col row over rows that OTHER warps staged two tiles ago: every warp's stores must have read them.
                 if (out_row_bytes < 128) __syncthreads();
-            }
-            if (POOL && keep_at >= 0) {   // the window's middle is the pixel itself
-#pragma unroll
-                for (int c = 0; c < C; ++c) a.keep[keep_at + c * xs_c] = v[c * 9 + 4];
             }
             uint8_t *row = sA + buf * SR_A_BYTES + row_off;
 #pragma unroll
@@ -300,6 +265,287 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------ with the 2x2 maxpool after it (3x3, stride 1, 32 filters, f32)
+// The output is that of the maxpool with stride 2 after the layer, and optionally its signs, the next xnor layer's operand.  Same rows, same order of the
+// products.  What bounded the form before (27 predicated loads and roundings a pixel, every value finished, staged and read back; 62 % of the issue slots) was
+// instructions, so
+//  * a tile is 16 x 8 windows of an image.  Its patch is loaded and rounded once, 18 values a thread, into shared memory, one tile ahead; a thread builds the
+//    rows of its window's four pixels from pairs of values, two pixels at a time;
+//  * the pixels of the same place in their windows are one MMA's 128 rows: a thread finds the four sums of its window in four accumulators, and what it
+//    scales, activates and rounds is the largest, none of which changes which one that is.  Sums of filters with a negative scale change sign first.  A
+//    warp that meets an infinity or NaN finishes all four, as the layer alone would, and then compares.
+// 128 x 224 x 224: 250 -> 141 us.  Bytes: 51; the sixteen MMAs a tile, 77 clocks each: 55; shared memory (rows written and read by the MMAs, patch): some 80.
+constexpr int SRP_TW = 16, SRP_TH = 8, SRP_PITCH = 2 * SRP_TW + 2, SRP_ROWS = 2 * SRP_TH + 2;
+
+struct StemRowsPoolShared {
+    uint64_t done[2];       // the MMAs over the windows' upper, lower pixels have retired
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+// The largest of four sums, NaN if one is.
+__device__ __forceinline__ float largest_or_nan(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    float m;
+    asm("{\n\t.reg .f32 t;\n\tmax.NaN.f32 t, %1, %2, %3;\n\tmax.NaN.f32 %0, t, %4;\n\t}"
+        : "=f"(m) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d)));
+    return m;
+}
+
+template <int C>
+__global__ void __launch_bounds__(SR_THREADS, 4)
+conv_stem_rows_pool_kernel(const __grid_constant__ StemTcArgs a)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023u) {
+        if (threadIdx.x == 0) atomicCAS(a.status, 0, SR_BAD_SMEM_BASE);
+        return;
+    }
+    constexpr int K = C * 9, PLANE = SRP_PITCH * SRP_ROWS, N = 32, PIECES = (K + 3) / 4;
+    constexpr int LINES = SR_THREADS / SRP_PITCH, STEPS = SRP_ROWS / LINES;   // patch rows loaded at once, and how often, of a plane
+    static_assert(SRP_ROWS % LINES == 0, "whole planes");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t *const sA = smem;                            // 2 x 128 rows x 128 bytes: a window's left pixel, its right one
+    uint8_t *const sB = smem + 2 * SR_A_BYTES;           // 32 rows x 128 bytes
+    float *const s_scale = reinterpret_cast<float *>(sB + N * 128), *const s_shift = s_scale + N;
+    float *const patch = s_shift + N;                    // two patches of C planes of 18 x 34
+    StemRowsPoolShared *const sh = reinterpret_cast<StemRowsPoolShared *>(patch + 2 * C * PLANE);
+    volatile int *const abort_flag = &sh->abort_flag;
+    const ConvGeom g = a.g;
+
+    // filters as above; zeros where an im2col row has no value
+    for (int i = tid; i < N * 8; i += SR_THREADS) {
+        const int f = i >> 3, q = i & 7;
+        uint32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int k = 4 * q + e;
+            v[e] = k < K ? __float_as_uint(round_tf32(__ldg(a.w + (size_t)k * a.npg_pad + f))) : 0u;
+        }
+        *reinterpret_cast<uint4 *>(sB + f * 128 + ((q ^ (f & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    for (int i = tid; i < 2 * SR_A_BYTES / 16; i += SR_THREADS) reinterpret_cast<uint4 *>(sA)[i] = make_uint4(0u, 0u, 0u, 0u);
+    bool below_zero = false, odd_scale = false;
+    if (tid < N) {
+        const float sc = __ldg(a.ep.scale + tid);
+        s_scale[tid] = fabsf(sc);
+        s_shift[tid] = __ldg(a.ep.shift + tid);
+        below_zero = sc < 0.f;
+        odd_scale = !(fabsf(sc) > 0.f && fabsf(sc) < INFINITY);
+    }
+    if (tid == 0) {
+        mbar_init(smem_u32(&sh->done[0]), 1);
+        mbar_init(smem_u32(&sh->done[1]), 1);
+        sh->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, below_zero);
+        if (tid == 0) *reinterpret_cast<uint32_t *>(patch) = bits;   // for the other warps, until the first patch
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)), "r"((uint32_t)a.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_async_smem();
+    tc_fence_before();
+    const bool plain = !__syncthreads_or(odd_scale);
+    tc_fence_after();
+    const uint32_t tmem_base = sh->tmem_base, negative = *reinterpret_cast<uint32_t *>(patch);
+    __syncthreads();
+    grid_dependency_wait();   // up to here only the layer's own parameters were read
+    launch_dependents();
+
+    const float *const x = a.x;
+    float *const keep = a.keep;
+    const long long xs_b = a.xs_b;
+    const int xs_c = (int)a.xs_c, xs_h = (int)a.xs_h, xs_w = (int)a.xs_w;
+    const int tiles = a.tiles, tiles_w = a.tiles_w, tiles_wh = a.tiles_w * a.tiles_h, do_round = a.ep.round_tf32;
+    int8_t *const signs = a.signs;
+    int *const status = a.status;
+    const long long wait_limit = a.wait_limit;
+    const uint32_t idesc = mma_idesc<MMA_TF32>(128u, (uint32_t)N);
+    const uint64_t db = make_smem_desc(smem_u32(sB), 128), da0 = make_smem_desc(smem_u32(sA), 128);
+    const uint32_t done0 = smem_u32(&sh->done[0]);
+
+    const int wx = tid & (SRP_TW - 1), wy = tid / SRP_TW, sw = tid & 7;
+    const float *const from = patch + 2 * wy * SRP_PITCH + 2 * wx;
+    uint8_t *const row = sA + tid * 128;
+
+    // A thread loads one column of every third row of the patch: value (c, k) is row line + LINES * k of plane c.
+    const bool loads = tid < LINES * SRP_PITCH;
+    const int line = tid / SRP_PITCH, column = tid - line * SRP_PITCH;
+    const bool own_column = column >= 1 && column <= 2 * SRP_TW;
+    const long long step_h = (long long)LINES * xs_h;
+    float v[C][STEPS];
+    const float *base = x;             // of the tile whose values are in v: may lie before the image, dereferenced only inside
+    int next_b, next_y, next_x;        // its image and first window
+    bool in_column;
+    auto fetch = [&](int tile) {
+        const int b = tile / tiles_wh, r = tile - b * tiles_wh, ty = r / tiles_w;
+        next_b = b; next_y = ty * SRP_TH; next_x = (r - ty * tiles_w) * SRP_TW;
+        const int yy = 2 * next_y - 1 + line, xx = 2 * next_x - 1 + column;
+        base = x + b * xs_b + (long long)yy * xs_h + (long long)xx * xs_w;
+        in_column = loads && (unsigned)xx < (unsigned)g.w;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int k = 0; k < STEPS; ++k) v[c][k] = in_column && (unsigned)(yy + LINES * k) < (unsigned)g.h ? __ldg(base + c * xs_c + k * step_h) : 0.f;
+    };
+    // rows of the window's two pixels at `from`
+    auto build = [&](const float *src) {
+        float w[2][PIECES * 4];
+#pragma unroll
+        for (int k = K; k < PIECES * 4; ++k) w[0][k] = w[1][k] = 0.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int kh = 0; kh < 3; ++kh) {
+                const float2 p0 = *reinterpret_cast<const float2 *>(src + c * PLANE + kh * SRP_PITCH), p1 = *reinterpret_cast<const float2 *>(src + c * PLANE + kh * SRP_PITCH + 2);
+                const int k = c * 9 + kh * 3;
+                w[0][k] = p0.x; w[0][k + 1] = p0.y; w[0][k + 2] = p1.x;
+                w[1][k] = p0.y; w[1][k + 1] = p1.x; w[1][k + 2] = p1.y;
+            }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < PIECES; ++q)
+                *reinterpret_cast<float4 *>(row + h * SR_A_BYTES + ((q ^ sw) << 4)) = make_float4(w[h][4 * q], w[h][4 * q + 1], w[h][4 * q + 2], w[h][4 * q + 3]);
+        fence_async_smem();
+    };
+    auto multiply = [&](int lower) {   // one thread
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint64_t da = da0 + (uint64_t)(h * (SR_A_BYTES >> 4));
+            const uint32_t d = tmem_base + (uint32_t)(2 * lower + h) * N;
+            umma<MMA_TF32>(d, da, db, idesc, 0u);
+            umma<MMA_TF32>(d, da + 2, db + 2, idesc, 1u);
+            umma<MMA_TF32>(d, da + 4, db + 4, idesc, 1u);
+            umma<MMA_TF32>(d, da + 6, db + 6, idesc, 1u);
+        }
+        umma_commit(done0 + 8 * lower);
+    };
+    auto finish = [&](float sum, float sc, float sf) {
+        float t = fmaf(sum, sc, sf);
+        t = fmaxf(t, 0.1f * t);
+        return do_round ? round_tf32(t) : t;
+    };
+
+    // what was fetched, into the patch of its tile
+    auto put = [&](float *to_patch) {
+        if (loads) {
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int k = 0; k < STEPS; ++k) to_patch[c * PLANE + k * (LINES * SRP_PITCH) + tid] = round_tf32(v[c][k]);
+        }
+        if (keep && in_column && own_column) {   // a copy of the images: every value by the tile whose pixel it is
+            float *const to = keep + (base - x);
+            const int left = g.h - (2 * next_y - 1 + line);   // image rows from this thread's first on
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int k = 0; k < STEPS; ++k) {
+                    const bool own = (k > 0 || line > 0) && (k < STEPS - 1 || line < LINES - 1);   // not the rows above and below
+                    if (own && LINES * k < left) to[c * xs_c + k * step_h] = v[c][k];
+                }
+        }
+    };
+
+    bool failed = false;
+    if ((int)blockIdx.x < tiles) { fetch(blockIdx.x); put(patch); }
+    __syncthreads();
+    int it = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {   // uniform over the CTA
+        const int b = next_b, tile_y = next_y, tile_x = next_x, py = next_y + wy, px = next_x + wx;
+        const bool more = tile + (int)gridDim.x < tiles;
+        if (more) fetch(tile + gridDim.x);
+        if (lane == 0) tma_store_wait_read0();   // the last tile's store has read this warp's rows
+        __syncwarp();
+        build(from + (it & 1) * (C * PLANE));
+        __syncthreads();
+        if (tid == 0) multiply(0);
+        __syncwarp();
+        if (!mbar_wait(done0, (uint32_t)(it & 1), abort_flag, status, SR_WAIT_ACC, 0, wait_limit)) failed = true;
+        if (!failed) build(from + (it & 1) * (C * PLANE) + SRP_PITCH);
+        if (more) put(patch + ((it + 1) & 1) * (C * PLANE));
+        if (__syncthreads_or(failed)) break;
+        if (tid == 0) multiply(1);
+        __syncwarp();
+        if (!mbar_wait(done0 + 8, (uint32_t)(it & 1), abort_flag, status, SR_WAIT_ACC, 0, wait_limit)) { failed = true; continue; }   // all leave together, at the next tile's vote
+        // ---- the window's largest sums
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16);
+        const bool stores = 2 * py < g.out_h && 2 * px < g.out_w;
+        const size_t window = ((size_t)b * (g.out_h >> 1) + py) * (g.out_w >> 1) + px;
+        uint32_t sg[8];
+#pragma unroll
+        for (int c0 = 0; c0 < N; c0 += 16) {
+            uint32_t r[4][16], o[16];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) tmem_ld16(t_row + p * N + c0, r[p]);
+            tmem_ld_wait();
+            if (negative) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[p][j] ^= (negative << (31 - c0 - j)) & 0x80000000u;
+            }
+            bool odd_value = !plain;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float m = largest_or_nan(r[0][j], r[1][j], r[2][j], r[3][j]);
+                odd_value |= !(fabsf(m) < INFINITY);
+                o[j] = __float_as_uint(m);
+            }
+            if (__any_sync(0xffffffffu, odd_value)) {   // (a block by itself: as a condition at every value it cost its instructions every time)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float sc = s_scale[c0 + j], sf = s_shift[c0 + j];
+                    float t = finish(__uint_as_float(r[0][j]), sc, sf);
+#pragma unroll
+                    for (int p = 1; p < 4; ++p) t = fmaxf(t, finish(__uint_as_float(r[p][j]), sc, sf));
+                    o[j] = __float_as_uint(fmaxf(-FLT_MAX, t));
+                }
+            } else {
+                const float4 *const sc4 = reinterpret_cast<const float4 *>(s_scale + c0), *const sf4 = reinterpret_cast<const float4 *>(s_shift + c0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 sc = sc4[q], sf = sf4[q];
+                    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, sfv[4] = {sf.x, sf.y, sf.z, sf.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[4 * q + e] = __float_as_uint(fmaxf(-FLT_MAX, finish(__uint_as_float(o[4 * q + e]), scv[e], sfv[e])));
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sg[c0 / 4 + q] = four_signs_no_nan(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+            // staged where the tile's rows were, which its MMAs have read
+#pragma unroll
+            for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4 *>(row + (((c0 / 4 + q) ^ sw) << 4)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) {   // a warp's 16 x 2 windows; the TMA unit clips them
+            tma_store_4d(&a.tmy, smem_u32(sA + warp * 4096), 0, tile_x, tile_y + 2 * warp, b);
+            tma_store_commit();
+        }
+        if (signs && stores) st_global_32(signs + window * 32, sg);
+        tc_fence_before();        // this thread's TMEM loads precede the barriers before the next MMAs
+    }
+    if (lane == 0) tma_store_wait_all();
+
+    // ---- teardown (also the abort path)
+    if (*abort_flag) {   // give MMAs that may still read shared memory time to retire
+        const long long t0 = clock64();
+        while (clock64() - t0 < 4000000LL) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)a.tmem_cols) : "memory");
     }
 }
 
@@ -556,7 +802,10 @@ static int launch_narrow(const StemTcArgs &a, cudaStream_t s)
 {
     const size_t smem = 2 * SR_A_BYTES + (size_t)a.n_pad * 128 + 2 * sizeof(float) * a.n_pad + sizeof(StemRowsShared) + 16;
     if constexpr (!OBF)
-        if (a.pool) return launch_rows(conv_stem_rows_kernel<C, DNB_LEAKY, false, true>, smem, 5, a, s);
+        if (a.pool) {
+            const size_t pooled = 2 * SR_A_BYTES + 32 * 128 + 2 * sizeof(float) * 32 + 2 * sizeof(float) * C * SRP_PITCH * SRP_ROWS + sizeof(StemRowsPoolShared) + 16;
+            return launch_rows(conv_stem_rows_pool_kernel<C>, pooled, 4, a, s);
+        }
     if (a.ep.activation == DNB_LEAKY) return launch_rows(conv_stem_rows_kernel<C, DNB_LEAKY, OBF>, smem, 5, a, s);
     return launch_rows(conv_stem_rows_kernel<C, SR_ACT_GENERIC, OBF>, smem, 5, a, s);
 }
@@ -584,13 +833,23 @@ int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s)
     if (!conv_stem_rows_covers(g, a.y_dtype) || a.y_cpitch != g.n) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: geometry outside its coverage");
     if (a.xs_c >= (1LL << 31) / 4 || a.xs_h >= (1LL << 31) / 4) DNB_FAIL(DNB_EUNSUPPORTED, "first-layer kernel: image too large for 32-bit offsets");
     if (a.pool && !(conv_stem_pool_covers(g, a.y_dtype, a.ep.activation) && conv_stem_rows_pool_covers(g, a.y_dtype))) DNB_FAIL(DNB_EINVAL, "first-layer kernel: no pooled variant of this layer");
-    const long long npix = (long long)g.batch * g.out_h * g.out_w / (a.pool ? 4 : 1);   // output pixels
-    const int per_tile = a.pool ? SR_THREADS / 4 : SR_THREADS;
-    a.npix = (int)npix;
-    a.tiles = (int)((npix + per_tile - 1) / per_tile);
     a.n_pad = round_up(g.n, 16);
     a.tmem_cols = 32;
     while (a.tmem_cols < a.n_pad) a.tmem_cols *= 2;
+    if (a.pool) {
+        a.tiles_w = (g.out_w / 2 + SRP_TW - 1) / SRP_TW;
+        a.tiles_h = (g.out_h / 2 + SRP_TH - 1) / SRP_TH;
+        a.tiles = g.batch * a.tiles_w * a.tiles_h;
+        a.tmem_cols = 128;   // four accumulators of 32 columns
+        const uint64_t pw = (uint64_t)g.out_w / 2, ph = (uint64_t)g.out_h / 2;
+        const uint64_t dims[4] = {32u, pw, ph, (uint64_t)g.batch}, strides[3] = {128u, 128u * pw, 128u * pw * ph};
+        const uint32_t box[4] = {32u, (uint32_t)SRP_TW, 32u / SRP_TW, 1u};
+        DNB_TRY(encode_tensor_map(&a.tmy, 0, 4, a.y, dims, strides, box, 128));
+        return launch_geometry<false>(a, s);
+    }
+    const long long npix = (long long)g.batch * g.out_h * g.out_w;   // output pixels
+    a.npix = (int)npix;
+    a.tiles = (int)((npix + SR_THREADS - 1) / SR_THREADS);
     // rows of 32, 64 or 128 bytes leave through TMA stores from swizzled staging rows, the wide kernel's 256-byte rows in two halves;
     // other ones by plain stores
     const int es = a.y_dtype == DNB_BF16 ? 2 : 4, rb = g.n * es, half = rb > 128 ? 128 : rb;
@@ -598,7 +857,7 @@ int launch_conv_stem_rows(StemTcArgs a, cudaStream_t s)
     if (a.tma_store) {
         const uint64_t dims[2] = {(uint64_t)g.n, (uint64_t)npix};
         const uint64_t strides[1] = {(uint64_t)rb};
-        const uint32_t box[2] = {(uint32_t)(half / es), a.pool ? 8u : 32u};
+        const uint32_t box[2] = {(uint32_t)(half / es), 32u};
         DNB_TRY(encode_tensor_map(&a.tmy, es == 2 ? 1 : 0, 2, a.y, dims, strides, box, half));
     }
     return es == 2 ? launch_geometry<true>(a, s) : launch_geometry<false>(a, s);
