@@ -12,11 +12,20 @@ import numpy as np
 from . import (ACTIVATIONS, BF16, F32, MODE_TF32, NCHW, NHWC, ConvDesc, Tensor, check, lib)
 
 
+_current = None
+
+
 def _stream(stream=None) -> C.c_void_p:
+    """The stream a call goes to: the caller's, or torch's current one.  torch.cuda.current_stream() makes a Python object of it, 3.2 us of the 8.5
+    that the smallest call takes its host; torch's own handle of it is there in 0.2."""
+    global _current
     if stream is not None:
         return C.c_void_p(int(stream))
-    import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if _current is None:
+        import torch
+        raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.current_device
+        _current = (lambda: raw(device())) if raw else (lambda: torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_current())
 
 
 def as_tensor(t, layout: int = NCHW, c: int | None = None) -> Tensor:

@@ -824,3 +824,16 @@ def test_1x1_layers_with_their_filters_in_place(name, mode, tol, monkeypatch):
     for a, b in zip(out["0"], out["2"]):
         assert np.array_equal(a, b)
     parity(out["2"][0], oracle_conv(case), tol)
+
+
+def test_calls_go_to_the_current_stream():
+    """Inside torch's stream contexts, nested and left again, and to the stream that the caller names."""
+    import torch
+    from darknet_b200.api import _stream
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        assert _stream().value == a.cuda_stream
+        with torch.cuda.stream(b):
+            assert _stream().value == b.cuda_stream and _stream(a.cuda_stream).value == a.cuda_stream
+        assert _stream().value == a.cuda_stream
+    assert (_stream().value or 0) == torch.cuda.current_stream().cuda_stream
