@@ -156,13 +156,15 @@ struct alignas(64) TapsArgs {
     int taps, pixels;     // 9, or 1 (1x1 layers); of those the pixels of the whole batch
     int bk, c_blocks;     // channels of a block (128 bytes), blocks
     int bn, n_tiles;      // filters per tile, a multiple of 16
-    int pitch, rows;      // positions of a row (w + 1); of a tile's load (128 + 2 * pitch + 2)
-    int ptiles;           // tiles of 128 positions
+    int boxes;            // 1: tiles are boxes of 8 x 16 pixels, a load one of 10 x 18, by tiles_w and tiles_h of an image; 0: 128 positions in a row
+    int tiles_w, tiles_h;
+    int pitch, rows;      // positions of a row (w + 1, of a box 10); of a tile's load (128 + 2 * pitch + 2, of a box 180)
+    int ptiles;           // pixel tiles
     int total_tiles;      // pairs of them times n_tiles
     int x_stages, x_slot; // ring of pixel boxes, bytes of one
     int w_stages, w_bytes;// ring of filter tiles
     int resident;         // 1: the ring holds all of the layer's filters, loaded once
-    int staged_bytes;     // rows of the eight epilogue warps: 4 KB each, 8 with a residual, none for Darknet's layout alone
+    int staged_bytes;     // rows of the eight epilogue warps: 4 KB each, 12 with a residual, none for Darknet's layout alone
     int table;            // entries of the scale and shift tables in shared memory
     int tmem_cols, n_pad;
     int y_chan;           // channels written to y_nhwc

@@ -164,7 +164,7 @@ extern "C" int dnb_conv_plan_describe(const dnb_conv_plan *p, char *buf, int len
                  p->sp.bn, p->sp.wt, p->sp.ht, p->sp.bt, p->sp.tiles, p->sp.stages, p->sp.splits, p->signs_given ? 1 : 0, p->sp.sign_out ? 1 : 0);
     else if (tc && p->tc_x_ptr && p->tc_taps)
         snprintf(buf, len, "%s pair=1 halo=0 bn=%d tiles=%d stages=%d+%d epi=2 splits=1 one_load_for_%s%s", kKernelNames[p->kernel], p->tp.bn, p->tp.total_tiles,
-                 p->tp.x_stages, p->tp.w_stages, p->tp.taps == 9 ? "nine_taps" : "a_block", p->tp.resident ? " resident" : "");
+                 p->tp.x_stages, p->tp.w_stages, p->tp.taps == 9 ? "nine_taps" : "a_block", p->tp.boxes ? (p->tp.resident ? " boxes resident" : " boxes") : p->tp.resident ? " resident" : "");
     else if ((p->kernel == K_TC_TF32 || p->kernel == K_TC_BF16 || (p->kernel == K_XNOR && p->xnor_tc)) && p->tc_x_ptr)
         snprintf(buf, len, "%s pair=%d halo=%d bn=%d tile=%dx%dx%d tiles=%d stages=%d ctas_per_sm=%d srb=%d epi=%d splits=1 signs_in=%d signs_out=%d", kKernelNames[p->kernel], a.pair, a.halo,
                  a.bn, a.wt, a.ht, a.bt, a.total_tiles, a.stages, a.ctas_per_sm, a.store_row_bytes, a.epi_groups, p->signs_given ? 1 : 0, a.sign_out ? 1 : 0);
@@ -789,7 +789,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
 
 // ------------------------------------------------------------------ 3x3 layers with one load for nine taps, 1x1 layers with their filters in place (conv_tc_taps.cu)
 // The launch's tiles and rings; p->tp holds them.  False where the kernel has no form of it.
-static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channels_last, bool residual)
+static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool boxes, bool channels_last, bool residual)
 {
     TapsArgs &a = p->tp;
     const int es = p->kernel == K_TC_BF16 ? 2 : 4;
@@ -798,10 +798,13 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
     a.c_blocks = (p->c_pad + a.bk - 1) / a.bk;
     a.g = p->g;
     a.taps = g.size * g.size;
-    a.pitch = g.w + 1;
-    a.rows = a.taps == 1 ? 128 : 128 + 2 * a.pitch + 2;
-    if (a.rows > 1024) return false;
-    const long long pixels = (long long)g.batch * g.h * g.w, positions = a.taps == 1 ? pixels : (long long)g.batch * a.pitch * (g.h + 1) - a.pitch - 1;
+    a.boxes = boxes ? 1 : 0;
+    a.tiles_w = (g.w + 7) / 8; a.tiles_h = (g.h + 15) / 16;
+    a.pitch = boxes ? 10 : g.w + 1;
+    a.rows = a.taps == 1 ? 128 : boxes ? 180 : 128 + 2 * a.pitch + 2;
+    if (a.rows > 1024 || (boxes && a.taps == 1)) return false;
+    const long long pixels = (long long)g.batch * g.h * g.w;
+    const long long positions = a.taps == 1 ? pixels : boxes ? 128LL * a.tiles_w * a.tiles_h * g.batch : (long long)g.batch * a.pitch * (g.h + 1) - a.pitch - 1;
     if (positions > (1LL << 31) - 4096) return false;
     a.pixels = (int)pixels;
     a.ptiles = (int)((positions + 127) / 128);
@@ -812,7 +815,7 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
     a.total_tiles = (int)tiles;
     a.x_slot = round_up(a.rows * 128, 1024);
     a.w_bytes = round_up(bn / 2 * 128, 1024);
-    a.staged_bytes = channels_last ? (residual ? 65536 : 32768) : 0;
+    a.staged_bytes = channels_last ? (residual ? 98304 : 32768) : 0;
     a.table = round_up(a.n_tiles * bn, 64);
     a.tmem_cols = 32;
     while (a.tmem_cols < 2 * bn) a.tmem_cols *= 2;
@@ -835,7 +838,7 @@ static bool taps_tiles(dnb_conv_plan *p, const ConvGeom &g, int bn, bool channel
         if (a.w_stages > 12) a.w_stages = 12;
     }
     if (a.x_stages > TAPS_MAX_X) a.x_stages = TAPS_MAX_X;
-    return a.x_stages >= 2 && (a.resident || a.w_stages >= 3);
+    return a.x_stages >= 2 && (a.resident || a.w_stages >= 4);
 }
 
 // Whether the kernel has a variant for such a launch of the plan.  A 1x1 layer with a residual has not: its addend arrives by TMA, three chunks
@@ -865,7 +868,7 @@ static double taps_us(const TapsArgs &a, bool nchw_out, bool residual, bool yolo
         const double tiles = rounds * ((mma > epilogue ? mma : epilogue) + 0.6);
         return 7.2 + (tiles > bytes / 6.1e6 ? tiles : bytes / 6.1e6);
     }
-    const double mma = 9.0 * a.c_blocks * (0.174 + 0.136 * wide), load = a.c_blocks * a.rows * 0.0037;
+    const double mma = 9.0 * a.c_blocks * (0.174 + 0.136 * wide), load = a.c_blocks * a.rows * (a.boxes ? 0.0011 : 0.0037);
     const double longest = mma > load ? (mma > epilogue ? mma : epilogue) : (load > epilogue ? load : epilogue);
     return 5.3 + rounds * (longest + 0.65) + 0.55 * epilogue + load / a.c_blocks;
 }
@@ -875,31 +878,35 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
 {
     const char *e = getenv("DNB_TC_TAPS_BN");
     const int only = e ? atoi(e) : 0;
-    int best_bn = 0;
+    const char *be = getenv("DNB_TC_TAPS_BOX");
+    int best_bn = 0, best_boxes = 0;
     double best = 1e300;
-    for (int bn = 64; bn <= 256; bn *= 2) {
-        const int width = bn < p->n_pad ? bn : p->n_pad;
-        if ((only && bn != only) || (bn > 64 && bn / 2 >= p->n_pad) || !taps_tiles(p, g, width, channels_last, residual)) continue;
-        const double us = taps_us(p->tp, nchw_out, residual, yolo);
-        if (us < best) { best = us; best_bn = width; }
-    }
-    return best_bn && taps_tiles(p, g, best_bn, channels_last, residual) ? best : 1e300;
+    for (int bn = 64; bn <= 256; bn *= 2)
+        for (int boxes = 0; boxes < 2; ++boxes) {
+            if (be && atoi(be) != boxes) continue;
+            const int width = bn < p->n_pad ? bn : p->n_pad;
+            if ((only && bn != only) || (bn > 64 && bn / 2 >= p->n_pad) || !taps_tiles(p, g, width, boxes, channels_last, residual)) continue;
+            const double us = taps_us(p->tp, nchw_out, residual, yolo);
+            if (us < best) { best = us; best_bn = width; best_boxes = boxes; }
+        }
+    return best_bn && taps_tiles(p, g, best_bn, best_boxes, channels_last, residual) ? best : 1e300;
 }
 
 // Whether a launch takes that kernel: where its estimate is well below what the others take.  others_us: the estimate of the launch that it would
 // be, cut along K or not.  Those estimates are of launches in a chain; in the measure of taps_us, launches by themselves, cut ones take 1.3 times
 // theirs and whole ones 1.12, in Darknet's layout 1.55 and 1.3 (stores in the short rows of a tile), with a residual 1.25 and 0.95 (1.05 alone, but 64 x 64 x 152 x 152 -> 128
-// is 516 -> 485 us alone and 548 -> 568 inside YOLOv3-608).  On 300 random 3x3
-// launches the rule takes 80 here, 4 of them to their loss (of 5 to 8 %), and all of the launches take 0.947 of what they did: 16 x 256 x 52 x 52
+// is 516 -> 485 us alone and 548 -> 568 inside YOLOv3-608).  On 200 random 3x3
+// launches the rule takes 68 here, 7 of them to their loss (of 4 to 13 %), 18 in less than 0.8 of the time, and all of the launches take 0.946 of what they did: 16 x 256 x 52 x 52
 // -> 512 in Darknet's layout 153 -> 126 us, 2 x 120 x 76 x 76 -> 128 26.8 -> 14.2, 256 x 128 x 28 x 28 -> 128 128 -> 106, 34 x 232 x 38 x 38 -> 255 in bf16 85 -> 42.
 // Launches of many rounds of pairs over 256 filters run into the power cap in either kernel (64 x 256 x 38 x 38 -> 512 265 -> 261 alone, 300 -> 307
 // inside YOLOv3-608) and stay where less padding is multiplied.
 // The kernel adds the products of a 3x3 layer in another order, so g is that of the whole batch where the plan is for a part of it, and of one image where
 // there are two: an image's sums then hang neither on the parts nor on the other image.
 // 1x1 layers add in the same order and are never cut here: what they gain is that their filters are loaded once (wide tiles, which are at least even alone, take a
-// tenth less power: 64 x 512 x 52 x 52 -> 256 in bf16 53.2 -> 51.9 us alone, 62.9 -> 59.5 back to back) and the stores in
-// Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138, with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch that does not fill the
-// pairs of SMs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
+// tenth less power: 64 x 512 x 52 x 52 -> 256 in bf16 53.2 -> 51.9 us alone, 62.9 -> 59.5 back to back; 256 -> 128 at
+// 64 x 76 x 76 inside YOLOv3-608 110 -> 99) and the stores in
+// Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138, with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two
+// rounds of pairs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
 static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
@@ -912,7 +919,7 @@ static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double other
     const double slack = yolo ? 1.0 : nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 0.95) : cut ? 1.3 : 1.12;
     const double us = best_taps(p, g, channels_last, nchw_out, residual, yolo);
     if (us >= 1e300 || knob == 2) return us < 1e300;
-    if (g.size == 1) return !cut && p->tp.total_tiles >= sm_count() / 2 && us < (yolo ? 0.9 : p->tp.resident && p->tp.bn >= 192 ? 1.05 : 0.8) * slack * others_us;
+    if (g.size == 1) return !cut && p->tp.total_tiles >= sm_count() && us < (yolo ? 0.9 : p->tp.resident && (p->tp.bn >= 192 || (p->tp.bn >= 128 && p->tp.c_blocks >= 8)) ? 1.05 : 0.8) * slack * others_us;
     return us < 0.9 * slack * others_us;
 }
 
@@ -928,7 +935,10 @@ static int build_taps_args(dnb_conv_plan *p, const dnb_tensor *x, const void *y_
     DNB_TRY(ensure_status(p));
     const uint64_t pix = (uint64_t)x->cpitch * es;
     const uint64_t dims[4] = {(uint64_t)p->c_pad, (uint64_t)g.w, (uint64_t)g.h, (uint64_t)g.batch}, strides[3] = {pix, pix * g.w, pix * g.w * g.h};
-    if (a.taps == 9) {
+    if (a.boxes) {
+        const uint32_t box[4] = {(uint32_t)a.bk, 10u, 18u, 1u};
+        DNB_TRY(encode_tensor_map(&a.tmx, a.bf16, 4, x->data, dims, strides, box, 128));
+    } else if (a.taps == 9) {
         DNB_TRY(encode_im2col_map(&a.tmx, a.bf16, x->data, dims, strides, (uint32_t)a.bk, (uint32_t)a.rows));
     } else {
         const uint64_t flat_dims[3] = {(uint64_t)p->c_pad, (uint64_t)a.pixels, 1}, flat_strides[2] = {pix, pix * a.pixels};
@@ -1147,7 +1157,8 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             if (may_cut) dcut = cut_at(dg);
             pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
         }
-        const double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, a.taps * a.c_blocks, residual != nullptr, res && res->yolo_entries);
+        double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, a.taps * a.c_blocks, residual != nullptr, res && res->yolo_entries);
+        if (!dcut.splits && !da.pair && da.bn > 128 && da.bn <= 192) others *= 0.85;   // (that estimate is of 256 filters)
         p->tc_taps = taps_pay(p, dg, dcut.splits != 0, others, res, y_nhwc != nullptr, nchw_out) &&
                      best_taps(p, g, y_nhwc != nullptr, nchw_out, residual != nullptr, res && res->yolo_entries) < 1e300;
     }

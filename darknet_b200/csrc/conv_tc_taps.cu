@@ -13,6 +13,8 @@
 // Roles (352 threads, CTA pairs with cta_group::2 MMAs): warp 0 loads filters, warp 10 pixels, warp 1 of the even CTA issues the MMAs, warps 2..9 drain the
 // accumulator: each a chunk of 128 bytes of every pixel of its 32, staged in rows of its own, stored eight lanes a pixel.  No two epilogue warps meet.
 // Where the layer's filters fit shared memory beside two boxes they are loaded once (64 -> 64 in TF32).
+// Wide maps are cut into boxes of 8 x 16 pixels instead (boxes): a load is one of 10 x 18, eight-row groups of the A operand are ten rows apart, and what a row
+// of such a load costs is a third of what one of an im2col load does (1.1 ns, 3.7), of which a map of 304 columns would want 740 a tile.
 // 1x1 layers run here too (ONE): a position is a pixel of the batch, a plain load of 128 of them serves a block of channels; what is gained there is that the
 // filters stay in shared memory (512 -> 256 in bf16: 128 KB of each CTA of a pair) and the stores in Darknet's layout.
 // K runs over blocks of channels, then taps (conv_tc.cu and conv_tc_split.cu: taps, then blocks).
@@ -33,6 +35,7 @@
 namespace dnb {
 
 constexpr int TAPS_THREADS = 352;
+constexpr int TAPS_RES_ROWS = 3;   // sets of staged rows of a warp where a residual lands in them
 
 struct TapsShared {
     uint64_t x_full[TAPS_MAX_X], x_empty[TAPS_MAX_X];
@@ -102,6 +105,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
     const uint32_t tmem_base = sh->tmem_base;
 
     const int c_blocks = a.c_blocks, n_tiles = a.n_tiles, total_tiles = a.total_tiles, bn = a.bn, pitch = a.pitch;
+    const bool boxes = !ONE && a.boxes != 0;
     const int tile_step = (int)(gridDim.x >> 1), first_tile = (int)(blockIdx.x >> 1);
     const long long wait_limit = a.wait_limit;
     int *const status = a.status;
@@ -148,8 +152,15 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         grid_dependency_wait();
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int pt = min(pixel_tile(tile), last);   // the second CTA of the last of an odd number of pixel tiles does the first's again, and stores nothing
-            const int at = pt * 128, row = ONE ? 0 : at / pitch, img = ONE ? 0 : row / h1;
-            const int x0 = at - row * pitch - 1, y0 = row - img * h1 - 1;
+            int at = pt * 128, x0 = 0, y0 = 0, img = 0;
+            if (!ONE && boxes) {
+                const int tw = pt % a.tiles_w, t = pt / a.tiles_w, th = t % a.tiles_h;
+                x0 = 8 * tw - 1; y0 = 16 * th - 1; img = t / a.tiles_h;
+            } else if (!ONE) {
+                const int row = at / pitch;
+                img = row / h1;
+                x0 = at - row * pitch - 1; y0 = row - img * h1 - 1;
+            }
             for (int cb = 0; cb < c_blocks; ++cb) {
                 ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, TAPS_WAIT_EMPTY, wait_limit);
                 if (!ok) break;
@@ -157,6 +168,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                     const uint32_t bar = full0 + 8 * stage;
                     if (leader) mbar_expect_tx(bar, 2u * bytes);
                     if (ONE) tma_load_3d_pair(ring + stage * slot_bytes, map, bar, cb * bk, at, 0);
+                    else if (boxes) tma_load_4d_pair(ring + stage * slot_bytes, map, bar, cb * bk, x0, y0, img);
                     else tma_load_im2col_4d_pair(ring + stage * slot_bytes, map, bar, cb * bk, x0, y0, img);
                 }
                 __syncwarp();
@@ -169,7 +181,9 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         if (leader) {
             const uint32_t idesc = mma_idesc<KIND>(256u, (uint32_t)bn);
             const int w_stages = a.w_stages, x_stages = a.x_stages;
-            const uint64_t dx0 = make_smem_desc(ring, 128), dw0 = make_smem_desc(w_ring, 128);
+            uint64_t dx0 = make_smem_desc(ring, 128);
+            if (boxes) dx0 = (dx0 & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(pitch * 8) << 32);   // groups of eight rows: a box's rows apart
+            const uint64_t dw0 = make_smem_desc(w_ring, 128);
             const uint64_t x_step = a.x_slot >> 4, w_step = a.w_bytes >> 4, row_step = (uint64_t)(pitch - 2) * 8;   // from tap (kh, 2) to (kh + 1, 0)
             const uint32_t xf = smem_u32(&sh->x_full[0]), xe = smem_u32(&sh->x_empty[0]), wf = smem_u32(&sh->w_full[0]), we = smem_u32(&sh->w_empty[0]);
             const bool resident = a.resident != 0, no_mma = (a.debug & 16) != 0;
@@ -228,7 +242,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         const uint8_t *const res_base = reinterpret_cast<const uint8_t *>(a.ep.residual);
         const float alpha = a.ep.alpha, beta = a.ep.beta;
         const int dbg = a.debug, yolo_entries = ACT == TAPS_YOLO ? a.ep.yolo_entries : 1;
-        uint8_t *const staged0 = stage_out + (size_t)(warp - 2) * (RES ? 8192 : 4096);
+        uint8_t *const staged0 = stage_out + (size_t)(warp - 2) * (RES ? TAPS_RES_ROWS * 4096 : 4096);
         // the pixel of this lane's position of a tile, -1 for one of the extra column or row, or past the batch
         auto pixel_of = [&](int tile, int &b, int &y, int &x) {
             const int pt = pixel_tile(tile);
@@ -239,6 +253,12 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 if (y_nchw) { b = f / plane; x = f - b * plane; }
                 return pt < ptiles && f < a.pixels ? f : -1;
             }
+            if (boxes) {
+                const int m = quarter * 32 + lane, tw = pt % a.tiles_w, t = pt / a.tiles_w, th = t % a.tiles_h;
+                b = t / a.tiles_h;
+                x = 8 * tw + (m & 7); y = 16 * th + (m >> 3);
+                return pt < ptiles && x < g.w && y < g.h ? (b * g.h + y) * g.w + x : -1;
+            }
             const int f = pt * 128 + pitch + 1 + quarter * 32 + lane, row = f / pitch;
             x = f - row * pitch - 1;
             b = row / h1;
@@ -247,9 +267,9 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         };
         const int piece = lane & 7, sub = lane >> 3, q_xor = lane & 7;
 
-        // Residual: 128 bytes of each of the warp's 32 pixels, eight lanes a pixel, into the staged rows, one chunk ahead and across tiles.
+        // Residual: 128 bytes of each of the warp's 32 pixels, eight lanes a pixel, into the staged rows, two chunks ahead and across tiles.
         int pf_tile = first_tile, pf_c = group, pf_pixel = -1, pf_at = -1;
-        uint32_t pf_count = 0;
+        uint32_t pf_rows = 0, rows_now = 0;   // which of the staged rows the next request, this chunk has
         auto request_residual = [&]() {
             while (pf_c >= chunks) { pf_c -= chunks; pf_tile += tile_step; }
             if (pf_tile < total_tiles && !(dbg & 1)) {
@@ -259,7 +279,7 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                     pf_at = pf_tile;
                 }
                 const int ch = (pf_tile % n_tiles) * bn + pf_c * CPC + piece * (16 / OES);
-                const uint32_t dst = smem_u32(staged0 + (pf_count & 1) * 4096);
+                const uint32_t dst = smem_u32(staged0 + pf_rows * 4096);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int r = 4 * i + sub, px = __shfl_sync(0xffffffffu, pf_pixel, r);
@@ -268,22 +288,17 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                 }
             }
             pf_c += 2;
-            ++pf_count;
+            if (++pf_rows == TAPS_RES_ROWS) pf_rows = 0;
             cp_async_commit();
         };
-        if (RES) request_residual();
+        if (RES)
+            for (int i = 1; i < TAPS_RES_ROWS; ++i) request_residual();
 
-        uint32_t chunk_count = 0;
         int it = 0, c = group;
         for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
             const int acc = it & 1, nt = tile % n_tiles;
             int b, y, x;
             const int pixel = pixel_of(tile, b, y, x);
-            if (RES && group == 0 && !(dbg & 1) && tile + tile_step < total_tiles) {   // the next tile's residual into L2
-                int b2, y2, x2;
-                const int px = pixel_of(tile + tile_step, b2, y2, x2), n0 = (tile + tile_step) % n_tiles * bn, bytes = (min(bn, y_chan - n0)) * OES;
-                if (px >= 0 && bytes > 0) prefetch_l2(res_base + (size_t)px * res_pix + (size_t)n0 * OES, (uint32_t)bytes);
-            }
             if (!mbar_wait(smem_u32(&sh->acc_full[acc]), (it >> 1) & 1, abort_flag, status, TAPS_WAIT_ACC_FULL, 0, wait_limit)) break;
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * acc_stride;
@@ -291,10 +306,11 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
             for (; c < chunks; c += 2) {
                 const int c0 = c * CPC;
                 if (dbg & 8) continue;
-                uint8_t *const staged = staged0 + (RES ? (chunk_count & 1) * 4096 : 0), *const row = staged + lane * 128;
+                uint8_t *const staged = staged0 + rows_now * 4096, *const row = staged + lane * 128;
+                if (RES && ++rows_now == TAPS_RES_ROWS) rows_now = 0;
                 if (RES) {
-                    cp_async_wait<0>();
-                    __syncwarp();            // ... of all lanes; and their stores have read the other rows
+                    cp_async_wait<TAPS_RES_ROWS - 2>();
+                    __syncwarp();            // ... of all lanes; and their stores have read the last chunk's rows
                     request_residual();
                 }
                 uint32_t r[CPC];
@@ -375,7 +391,6 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
                             dst[(size_t)j * plane] = v;
                         }
                 }
-                ++chunk_count;
             }
             c -= chunks;
             tc_fence_before();

@@ -718,9 +718,10 @@ TAPS = {   # one load of pixels for the nine taps: tiles across rows and images,
 }
 
 
+@pytest.mark.parametrize("boxes", ["0", "1"])
 @pytest.mark.parametrize("name", list(TAPS))
 @pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
-def test_one_load_for_nine_taps(name, mode, tol, monkeypatch):
+def test_one_load_for_nine_taps(name, mode, tol, boxes, monkeypatch):
     """Whole numbers, whose sums are exact in any order: equal to the kernel that loads tap by tap to the bit, in either layout.  Others: within the mode's
     tolerance of the checker; with a residual to the kernel's output plus it, rounded once more."""
     import ctypes as C
@@ -728,12 +729,14 @@ def test_one_load_for_nine_taps(name, mode, tol, monkeypatch):
     import torch
     from gpu_util import dev_nhwc, empty_nhwc, host_from_nhwc, padding_is_zero
     case = conv_case(760, **TAPS[name])
+    monkeypatch.setenv("DNB_TC_TAPS_BOX", boxes)
     whole = dict(case, x=np.rint(2 * case["x"]), w=np.rint(case["w"] / np.abs(case["w"]).max() * 6), biases=np.rint(9 * case["biases"]), scales=None, mean=None, var=None)
     out = {}
     for knob in ("0", "2"):
         monkeypatch.setenv("DNB_TC_TAPS", knob)
         plan, a, b = run_conv(whole, mode, "nhwc", "nchw", both=True)
         assert ("one_load_for_nine_taps" in plan.describe()) == (knob == "2"), plan.describe()
+        assert (" boxes" in plan.describe()) == (knob == "2" and boxes == "1")
         plan, c, _ = run_conv(whole, mode, "nhwc", "nhwc")
         assert np.array_equal(a, b) and np.array_equal(a, c)
         out[knob] = a
