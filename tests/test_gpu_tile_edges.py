@@ -840,3 +840,28 @@ def test_calls_go_to_the_current_stream():
             assert _stream().value == b.cuda_stream and _stream(a.cuda_stream).value == a.cuda_stream
         assert _stream().value == a.cuda_stream
     assert (_stream().value or 0) == torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("channels,height,width", [(32, 1, 1), (33, 1, 7), (127, 3, 3), (128, 8, 1), (129, 7, 7), (260, 8, 8), (1000, 13, 5), (100, 23, 27), (6000, 5, 2)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_global_average_keeps_its_order(channels, height, width, dtype):
+    """Row j adds pixels j, j + 8, ...; the eight rows are added in order and divided by the pixels: equal to the bit to that, and channels
+    of a wider map that are not the tensor's stay out of it."""
+    import numpy as np
+    import torch
+    dt, batch = getattr(torch, dtype), 5 if channels > 2000 else 3
+    pitch = (channels + 7) // 8 * 8 + 8
+    full = torch.randn((batch, height, width, pitch), generator=torch.Generator().manual_seed(channels)).to(dt)
+    rows = full[..., :channels].float().numpy().reshape(batch, height * width, channels)
+    want = np.zeros((batch, channels), np.float32)
+    for j in range(8):
+        row = np.zeros((batch, channels), np.float32)
+        for p in range(j, height * width, 8):
+            row += rows[:, p]
+        want += row
+    want = torch.from_numpy(want / np.float32(height * width)).to(dt).float().numpy()
+    x, y = full.cuda(), torch.full((batch, 1, 1, pitch), -7.0, dtype=dt, device="cuda")
+    dn.avgpool(dn.as_tensor(x, dn.NHWC, channels), dn.as_tensor(y, dn.NHWC, channels))
+    torch.cuda.synchronize()
+    got = y.float().cpu().numpy()[:, 0, 0]
+    assert np.array_equal(got[:, :channels], want) and (got[:, channels:] == -7.0).all()
