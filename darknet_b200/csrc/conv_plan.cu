@@ -904,9 +904,9 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
 // there are two: an image's sums then hang neither on the parts nor on the other image.
 // 1x1 layers add in the same order and are never cut here: what they gain is that their filters are loaded once (wide tiles, which are at least even alone, take a
 // tenth less power: 64 x 512 x 52 x 52 -> 256 in bf16 53.2 -> 51.9 us alone, 62.9 -> 59.5 back to back; 256 -> 128 at
-// 64 x 76 x 76 inside YOLOv3-608 110 -> 99) and the stores in
-// Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138, with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two
-// rounds of pairs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
+// 64 x 76 x 76 inside YOLOv3-608 110 -> 99, 512 -> 256 at 64 x 32 x 32 in bf16 35 -> 29; 128 filters only over six rounds of pairs and more: 512 -> 128
+// at 256 x 28 x 28 102.7 -> 100.8, at 64 x 32 x 32 in bf16 23 -> 25) and the stores in Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138,
+// with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two rounds of pairs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
 static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
@@ -919,7 +919,13 @@ static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double other
     const double slack = yolo ? 1.0 : nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 0.95) : cut ? 1.3 : 1.12;
     const double us = best_taps(p, g, channels_last, nchw_out, residual, yolo);
     if (us >= 1e300 || knob == 2) return us < 1e300;
-    if (g.size == 1) return !cut && p->tp.total_tiles >= sm_count() && us < (yolo ? 0.9 : p->tp.resident && (p->tp.bn >= 192 || (p->tp.bn >= 128 && p->tp.c_blocks >= 8)) ? 1.05 : 0.8) * slack * others_us;
+    if (g.size == 1) {
+        const TapsArgs &t = p->tp;
+        const double bytes = (double)t.pixels * (t.c_blocks * 128.0 + g.n * (nchw_out || !t.bf16 ? 4.0 : 2.0)) / 6.1e6 + 7.2;   // no kernel is faster
+        const double others = slack * others_us > bytes ? slack * others_us : bytes;
+        const bool even = t.resident && (t.bn >= 192 || (t.bn >= 128 && t.c_blocks >= 8 && t.total_tiles >= 3 * sm_count()));
+        return !cut && t.total_tiles >= sm_count() && us < (yolo ? 0.9 : even ? 1.05 : 0.8) * others;
+    }
     return us < 0.9 * slack * others_us;
 }
 
