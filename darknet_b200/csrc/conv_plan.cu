@@ -904,9 +904,11 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
 // there are two: an image's sums then hang neither on the parts nor on the other image.
 // 1x1 layers add in the same order and are never cut here: what they gain is that their filters are loaded once (wide tiles, which are at least even alone, take a
 // tenth less power: 64 x 512 x 52 x 52 -> 256 in bf16 53.2 -> 51.9 us alone, 62.9 -> 59.5 back to back; 256 -> 128 at
-// 64 x 76 x 76 inside YOLOv3-608 110 -> 99, 512 -> 256 at 64 x 32 x 32 in bf16 35 -> 29; 128 filters only over six rounds of pairs and more: 512 -> 128
-// at 256 x 28 x 28 102.7 -> 100.8, at 64 x 32 x 32 in bf16 23 -> 25) and the stores in Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138,
-// with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two rounds of pairs is not worth their set-up (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
+// 64 x 76 x 76 inside YOLOv3-608 110 -> 99, 512 -> 256 at 64 x 32 x 32 in bf16 35 -> 29; 128 filters over four rounds of pairs and
+// more where six blocks of pixels fit beside them: 256 -> 128 at 32 x 52 x 52 30.5 -> 26.5, 512 -> 128 at 32 x 52 x 52 in bf16 26.8 -> 24.0; over ten where fewer do: 512 ->
+// 128 at 256 x 28 x 28 102.7 -> 100.8, but at 40 x 46 x 46 42.3 -> 46.2) and the stores in Darknet's layout (255 filters at 64 x 76 x 76 180 -> 138,
+// with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two rounds of pairs is not worth their set-up
+// (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
 static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
@@ -923,7 +925,7 @@ static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double other
         const TapsArgs &t = p->tp;
         const double bytes = (double)t.pixels * (t.c_blocks * 128.0 + g.n * (nchw_out || !t.bf16 ? 4.0 : 2.0)) / 6.1e6 + 7.2;   // no kernel is faster
         const double others = slack * others_us > bytes ? slack * others_us : bytes;
-        const bool even = t.resident && (t.bn >= 192 || (t.bn >= 128 && t.c_blocks >= 8 && t.total_tiles >= 3 * sm_count()));
+        const bool even = t.resident && (t.bn >= 192 || (t.bn >= 128 && t.c_blocks >= 8 && t.total_tiles >= (t.x_stages == TAPS_MAX_X ? 2 : 5) * sm_count()));
         return !cut && t.total_tiles >= sm_count() && us < (yolo ? 0.9 : even ? 1.05 : 0.8) * others;
     }
     return us < 0.9 * slack * others_us;
