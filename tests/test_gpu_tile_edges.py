@@ -723,7 +723,7 @@ TAPS = {   # one load of pixels for the nine taps: tiles across rows and images,
 @pytest.mark.parametrize("mode,tol", [(dn.MODE_TF32, 1e-2), (dn.MODE_BF16, 3e-2)])
 def test_one_load_for_nine_taps(name, mode, tol, boxes, monkeypatch):
     """Whole numbers, whose sums are exact in any order: equal to the kernel that loads tap by tap to the bit, in either layout.  Others: within the mode's
-    tolerance of the checker; with a residual to the kernel's output plus it, rounded once more."""
+    tolerance against the oracle; with a residual to the kernel's output plus it, rounded once more."""
     import ctypes as C
     import numpy as np
     import torch
