@@ -912,13 +912,21 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
 static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
-    const char *e = getenv("DNB_TC_TAPS"), *split = getenv("DNB_TC_SPLITK");
+    const char *e = getenv("DNB_TC_TAPS");
     const int knob = e ? atoi(e) : 1;
     if (knob == 0) return false;
-    if (!e && (getenv("DNB_TC_PAIR") || getenv("DNB_TC_EPI") || getenv("DNB_TC_HALO") || getenv("DNB_TC_WARP_STORES") || (split && atoi(split) > 1))) return false;
     const bool residual = res && res->residual;
     const bool yolo = res && res->yolo_entries > 0;
     const double slack = yolo ? 1.0 : nchw_out ? (cut ? 1.55 : 1.3) : residual ? (cut ? 1.25 : 0.95) : cut ? 1.3 : 1.12;
+    if (knob != 2) {   // what no choice of tiles would change: small launches, whose plans are most of their first call
+        const int c_blocks = (p->c_pad * (p->kernel == K_TC_BF16 ? 2 : 4) + 127) / 128;
+        if (g.size == 1 && (cut || (((long long)g.batch * g.h * g.w + 127) / 128 + 1) / 2 * ((p->n_pad + 63) / 64) < sm_count())) return false;
+        if (g.size == 3 && 5.3 + 9.0 * c_blocks * 0.174 + 0.65 >= 0.9 * slack * others_us) return false;
+    }
+    if (!e) {
+        const char *const split = getenv("DNB_TC_SPLITK");
+        if (getenv("DNB_TC_PAIR") || getenv("DNB_TC_EPI") || getenv("DNB_TC_HALO") || getenv("DNB_TC_WARP_STORES") || (split && atoi(split) > 1)) return false;
+    }
     const double us = best_taps(p, g, channels_last, nchw_out, residual, yolo);
     if (us >= 1e300 || knob == 2) return us < 1e300;
     if (g.size == 1) {

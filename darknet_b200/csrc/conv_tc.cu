@@ -40,6 +40,7 @@
 // (forward_shortcut_layer_gpu, src/shortcut_layer.c:75-80; src/blas_kernels.cu:711-745) when the caller asks for the fusion.
 #include <cuda.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1015,9 +1016,12 @@ size_t tmem_smem(size_t bytes, int cols)
 
 int conv_tc_max_smem()
 {
+    static std::atomic<int> cached[64];   // asked for by every plan and launch
     int dev = 0, v = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && (v = cached[dev].load(std::memory_order_relaxed)) > 0) return v;
     if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    if (dev < 64) cached[dev].store(v, std::memory_order_relaxed);
     return v;
 }
 
