@@ -465,6 +465,9 @@ conv_stem_rows_pool_kernel(const __grid_constant__ StemTcArgs a)
         if (more) fetch(tile + gridDim.x);
         if (lane == 0) tma_store_wait_read0();   // the last tile's store has read this warp's rows
         __syncwarp();
+#pragma unroll
+        for (int q = PIECES; q < 8; ++q)         // ... whose values, where an im2col row has none, an infinity among them would multiply the filters' zeros
+            *reinterpret_cast<uint4 *>(row + ((q ^ sw) << 4)) = make_uint4(0u, 0u, 0u, 0u);
         build(from + (it & 1) * (C * PLANE));
         __syncthreads();
         if (tid == 0) multiply(0);

@@ -865,3 +865,32 @@ def test_global_average_keeps_its_order(channels, height, width, dtype):
     torch.cuda.synchronize()
     got = y.float().cpu().numpy()[:, 0, 0]
     assert np.array_equal(got[:, :channels], want) and (got[:, channels:] == -7.0).all()
+
+
+@pytest.mark.parametrize("odd", ["bias", "pixel"])
+@pytest.mark.parametrize("channels", [1, 3])
+def test_a_first_layers_tiles_keep_to_themselves(odd, channels, tmp_path, monkeypatch):
+    """More tiles than CTAs at once: an infinite value of one tile changes nothing in the tiles that the same CTA does after it.  As in two launches, to the bit."""
+    import numpy as np
+    from darknet_b200 import synth
+    batch, size = 8, 224                                     # 784 tiles; four CTAs an SM are 592
+    cfg = (synth._net(batch, size, size, channels) + synth._conv(32, 3) + "\n[maxpool]\nsize=2\nstride=2\n" + synth._conv(32, 3, xnor=True) + "\n[avgpool]\n")
+    params = synth.seeded_params(cfg, 23)
+    x = synth.seeded_input(cfg, 24, "normal")
+    if odd == "bias":
+        params[0].biases[31] = np.inf
+    else:
+        params[0].weights[28:] = np.abs(params[0].weights[28:])
+        x[:4, 0, 10::64, 10::32] = np.inf
+    path = str(tmp_path / "i.weights")
+    synth.write_weights(path, params)
+    out = []
+    for fuse in ("0", "1"):
+        monkeypatch.setenv("DNB_FUSE_POOL", fuse)
+        net = dn.Network(cfg, path, dn.MODE_TF32, text=True)
+        net.predict(x)
+        out.append([net.layer_output(i) for i in (1, 2)] + [net.launches])
+        net.close()
+    assert out[1][-1] < out[0][-1] and np.isinf(out[0][0]).any()
+    for a, b in zip(out[0][:-1], out[1][:-1]):
+        assert np.array_equal(a, b, equal_nan=True)
