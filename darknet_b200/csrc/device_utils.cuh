@@ -108,12 +108,12 @@ __device__ __forceinline__ uint32_t four_signs(uint4 v)
            (__uint_as_float(v.w) > 0.f ? 0x01u : 0xFFu) << 24;
 }
 
-// The same of four that are no NaN: as integers, one less than those that are not > 0 is negative.
+// The same of four that are no NaN: of what is not > 0 the value itself or, of +0, one less is negative as an integer (-0 needs the former).
 __device__ __forceinline__ uint32_t four_signs_no_nan(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
 {
     uint32_t ab, cd;
-    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(ab) : "r"(a - 1u), "r"(b - 1u));   // their signs, as bytes
-    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(cd) : "r"(c - 1u), "r"(d - 1u));
+    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(ab) : "r"(a | (a - 1u)), "r"(b | (b - 1u)));   // their signs, as bytes
+    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(cd) : "r"(c | (c - 1u)), "r"(d | (d - 1u)));
     return __byte_perm(ab, cd, 0x5410u) | 0x01010101u;
 }
 

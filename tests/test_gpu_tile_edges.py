@@ -894,3 +894,40 @@ def test_a_first_layers_tiles_keep_to_themselves(odd, channels, tmp_path, monkey
     assert out[1][-1] < out[0][-1] and np.isinf(out[0][0]).any()
     for a, b in zip(out[0][:-1], out[1][:-1]):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("odd", ["zeros", "nan_bias", "scales", "pixels"])
+@pytest.mark.parametrize("batch,size", [(2, 88), (3, 36)])     # maps that end inside a tile of 16 x 8 windows, both ways
+def test_signs_of_a_first_layer_with_its_maxpool(odd, batch, size, tmp_path, monkeypatch):
+    """What the next xnor layer makes of values that are -0, infinite or NaN before they are rounded: as in two launches, to the bit.  A zero
+    sum of a filter with a negative scale and a bias of -0 is -0, and so is a NaN or a tiny negative value once it is rounded to TF32."""
+    import numpy as np
+    from darknet_b200 import synth
+    cfg = (synth._net(batch, size, size) + synth._conv(32, 3) + "\n[maxpool]\nsize=2\nstride=2\n" + synth._conv(48, 3, xnor=True) + "\n[avgpool]\n")
+    params = synth.seeded_params(cfg, 21)
+    x = synth.seeded_input(cfg, 22, "normal")
+    first = params[0]
+    first.rolling_mean[:] = 0
+    first.biases[:8] = -0.0
+    first.scales[:32:2] *= -1
+    first.biases[8:12] = -1e-42
+    x[:, :, size // 3:] = 0
+    if odd == "nan_bias":
+        first.biases[[0, 5, 31]] = np.nan
+        first.biases[[1, 30]] = np.inf, -np.inf
+    if odd == "scales":
+        first.scales[[2, 9, 28]] = 0.0, -0.0, np.nan
+    if odd == "pixels":
+        x[0, 0, 8, 6], x[0, 1, size - 2, 2], x[-1, 2, 4, size - 2] = np.nan, np.inf, -np.inf
+    path = str(tmp_path / "s.weights")
+    synth.write_weights(path, params)
+    out = []
+    for fuse in ("0", "1"):
+        monkeypatch.setenv("DNB_FUSE_POOL", fuse)
+        net = dn.Network(cfg, path, dn.MODE_TF32, text=True)
+        net.predict(x)
+        out.append([net.layer_output(i) for i in (1, 2)] + [net.launches])
+        net.close()
+    assert out[1][-1] < out[0][-1]
+    for a, b in zip(out[0][:-1], out[1][:-1]):
+        assert np.array_equal(a, b, equal_nan=True)
