@@ -274,7 +274,8 @@ struct dnb_conv_plan {
     int tc_x_cpitch;
     const void *tc_y_ptr;    // NHWC output the store map was built for
     const void *tc_res_ptr;  // fused residual the load map was built for (NULL: none)
-    int tc_res_cpitch, tc_res_c, tc_res_stride;
+    int tc_res_cpitch, tc_res_c, tc_res_stride, tc_res_act;
+    int tc_yolo;             // the cached launch block was built for a launch with a [yolo] layer's logistic
     int tc_y_cpitch, tc_y_dtype;
     // xnor layers in a row (tensor-core kind): the producer's epilogue writes the consumer's int8 operand
     dnb_conv_plan *sign_consumer;   // this plan also fills that plan's x_i8 (set by the network object), or null

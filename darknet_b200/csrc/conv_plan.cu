@@ -970,6 +970,9 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     const void *residual = res ? res->residual : nullptr;   // fused residual, if any
     const int res_cpitch = res ? res->res_cpitch : 0, res_stride = residual ? res->res_stride : 1, res_c = residual ? res->res_c : 0;
     TcArgs &a = p->tc;
+    p->tc_x_ptr = nullptr;   // until all of the block is there
+    p->tc_res_act = residual ? res->activation2 : DNB_LINEAR;
+    p->tc_yolo = res && res->yolo_entries > 0 ? 1 : 0;
     // A 1x1 convolution (stride 1, no padding) does not care which pixels are neighbours: with Darknet's layout among
     // the outputs, the h x w plane is treated as one row of h*w pixels, so that a tile is a run of up to 128 contiguous
     // pixels of every filter plane (and of the channels-last input) instead of a wt x ht patch.  DNB_TC_FLAT=0: never.
@@ -1456,7 +1459,7 @@ static int conv_forward_impl(dnb_conv_plan *p, const dnb_tensor *x, const dnb_te
         DNB_FAIL(DNB_EINVAL, "conv: a %s plan writes channels-last output as %s", kKernelNames[p->kernel], want == DNB_BF16 ? "bf16" : "f32");
     if (p->tc_x_ptr != xin.data || p->tc_x_cpitch != xin.cpitch || p->tc_y_ptr != y_nhwc || p->tc_y_cpitch != y_cpitch ||
         p->tc_y_dtype != y_dtype || !p->status || p->tc_res_ptr != ep.residual || p->tc_res_cpitch != ep.res_cpitch ||
-        (ep.residual && (p->tc_res_c != ep.res_c || p->tc_res_stride != ep.res_stride)) ||
+        (ep.residual && (p->tc_res_c != ep.res_c || p->tc_res_stride != ep.res_stride || p->tc_res_act != ep.activation2)) || p->tc_yolo != (ep.yolo_entries > 0 ? 1 : 0) ||
         p->tc_nchw_out != (y_nchw ? 1 : 0) || p->tc_pool != (pool ? 1 : 0))
         DNB_TRY(build_tc_args(p, &xin, y_nhwc, y_dtype, y_cpitch, &ep, y_nchw != nullptr, nullptr, 0, pool));
     if (p->tc_split) {

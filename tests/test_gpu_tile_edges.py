@@ -931,3 +931,42 @@ def test_signs_of_a_first_layer_with_its_maxpool(odd, batch, size, tmp_path, mon
     assert out[1][-1] < out[0][-1]
     for a, b in zip(out[0][:-1], out[1][:-1]):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
+def test_one_plan_several_epilogues(mode, monkeypatch):
+    """One plan and its tensors, called with one epilogue after another, each of which another kernel may have to do: as a new plan does each, to the bit."""
+    import ctypes as C
+    import numpy as np
+    import torch
+    from gpu_util import dev_nhwc, empty_nchw, empty_nhwc
+    monkeypatch.setenv("DNB_TC_TAPS", "2")
+    store = torch.bfloat16 if mode == dn.MODE_BF16 else torch.float32
+    case = conv_case(780, b=3, c=64, h=15, w=14, n=96, size=3)
+    xt, xd = dev_nhwc(case["x"], store)
+    at, ad = dev_nhwc(np.random.Generator(np.random.Philox(key=[8, 9])).standard_normal((3, 96, 15, 14), dtype=np.float32), store)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def plan_of(act):
+        p = dn.ConvPlan(3, 64, 15, 14, 96, 3, 1, 1, 1, True, act, False, mode)
+        p.set_params(case["w"], case["biases"], case["scales"], case["mean"], case["var"])
+        return p
+
+    def call(plan, what, yt, yd):
+        if what == "forward":
+            plan.forward(xd, yd)
+        elif what == "yolo":
+            dn.check(dn.lib().dnb_conv_yolo_forward(plan.handle, C.byref(xd), C.byref(yd), 3, 27, stream))
+        else:
+            dn.check(dn.lib().dnb_conv_shortcut_forward(plan.handle, C.byref(xd), C.byref(ad), C.byref(yd), 1.0, 1.0, dn.ACTIVATIONS[what], stream))
+        torch.cuda.synchronize()
+        plan.check_status()
+        return yt.float().cpu().numpy()
+
+    for act, empty, calls in (("leaky", lambda: empty_nhwc(3, 96, 15, 14, store), ["linear", "leaky", "relu", "linear", "forward", "leaky"]),
+                              ("linear", lambda: empty_nchw(3, 96, 15, 14), ["forward", "yolo", "forward", "yolo"])):
+        yt, yd = empty()
+        plan = plan_of(act)
+        for what in calls:
+            got = call(plan, what, yt, yd)
+            assert np.array_equal(got, call(plan_of(act), what, *empty())), (act, what)
