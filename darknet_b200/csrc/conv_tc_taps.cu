@@ -121,15 +121,17 @@ conv_tc_taps_kernel(const __grid_constant__ TapsArgs a)
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        // resident: every filter tile once, in the order of the ring's slots
-        const int begin = resident ? 0 : first_tile, end = resident ? n_tiles : total_tiles, step = resident ? 1 : tile_step;
-        for (int tile = begin; tile < end && ok; tile += step) {
-            const int n0 = (tile % n_tiles) * bn + (int)cta_rank * half;
+        // resident: once each of the filter tiles that this pair's tiles have (they come round in a cycle), in the slot that is its own.  No other: nobody
+        // would wait for its load, which could still be on its way when the CTA's shared memory is given back.
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+            const int nt = tile % n_tiles, n0 = nt * bn + (int)cta_rank * half;
+            if (resident && tile != first_tile && nt == first_tile % n_tiles) break;
+            if (resident) { stage = nt * c_blocks * TAPS; phase = 0; }
             for (int cb = 0; cb < c_blocks && ok; ++cb)
                 for (int tap = 0; tap < TAPS; ++tap) {
                     ok = mbar_wait_warp(empty0 + 8 * stage, phase ^ 1, abort_flag, status, TAPS_WAIT_EMPTY, wait_limit);
                     if (!ok) break;
-                    if (withhold && tile == begin && cb == c_blocks - 1 && tap == TAPS - 1) { ok = false; break; }   // wait-expiry test
+                    if (withhold && tile == first_tile && cb == c_blocks - 1 && tap == TAPS - 1) { ok = false; break; }   // wait-expiry test
                     if (elect_one()) {
                         const uint32_t bar = full0 + 8 * stage;
                         if (leader) mbar_expect_tx(bar, 2u * bytes);

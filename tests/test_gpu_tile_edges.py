@@ -829,6 +829,26 @@ def test_1x1_layers_with_their_filters_in_place(name, mode, tol, monkeypatch):
     parity(out["2"][0], oracle_conv(case), tol)
 
 
+@pytest.mark.parametrize("filters", [128, 192, 250])     # tiles of 64: with 74 pairs of CTAs a pair meets one of two, all of three, two of four
+@pytest.mark.parametrize("batch,height,width", [(1, 13, 13), (9, 52, 51)])     # one tile a pair; four rounds and more
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
+def test_a_pair_loads_the_filters_that_it_multiplies(filters, batch, height, width, mode, monkeypatch):
+    """1x1 layers with several filter tiles in place: equal to the kernel with a ring to the bit, in either layout."""
+    import numpy as np
+    case = conv_case(775, b=batch, c=72, h=height, w=width, n=filters, size=1)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    monkeypatch.setenv("DNB_TC_TAPS_BN", "64")
+    out = {}
+    for knob in ("0", "2"):
+        monkeypatch.setenv("DNB_TC_TAPS", knob)
+        plan, a, b = run_conv(case, mode, "nhwc", "nchw", both=True)
+        assert ("one_load_for_a_block resident" in plan.describe()) == (knob == "2"), plan.describe()
+        assert knob == "0" or "bn=64" in plan.describe(), plan.describe()
+        out[knob] = a
+        assert np.array_equal(a, b)
+    assert np.array_equal(out["0"], out["2"])
+
+
 def test_calls_go_to_the_current_stream():
     """Inside torch's stream contexts, nested and left again, and to the stream that the caller names."""
     import torch
