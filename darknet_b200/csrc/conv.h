@@ -155,7 +155,7 @@ struct alignas(64) TapsArgs {
     int bf16;             // operands and channels-last output bf16, else f32 (TF32 products)
     int taps, pixels;     // 9, or 1 (1x1 layers); of those the pixels of the whole batch
     int bk, c_blocks;     // channels of a block (128 bytes), blocks
-    int bn, n_tiles;      // filters per tile, a multiple of 16
+    int bn, n_tiles;      // filters per tile, a multiple of 32
     int boxes;            // 1: tiles are boxes of 8 x 16 pixels, a load one of 10 x 18, by tiles_w and tiles_h of an image; 0: 128 positions in a row
     int tiles_w, tiles_h;
     int pitch, rows;      // positions of a row (w + 1, of a box 10); of a tile's load (128 + 2 * pitch + 2, of a box 180)

@@ -884,7 +884,7 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
     for (int bn = 64; bn <= 256; bn *= 2)
         for (int boxes = 0; boxes < 2; ++boxes) {
             if (be && atoi(be) != boxes) continue;
-            const int width = bn < p->n_pad ? bn : p->n_pad;
+            const int width = bn < p->n_pad ? bn : round_up(p->n_pad, 32);   // (MMAs of 256 rows have columns in steps of 32)
             if ((only && bn != only) || (bn > 64 && bn / 2 >= p->n_pad) || !taps_tiles(p, g, width, boxes, channels_last, residual)) continue;
             const double us = taps_us(p->tp, nchw_out, residual, yolo);
             if (us < best) { best = us; best_bn = width; best_boxes = boxes; }

@@ -466,7 +466,7 @@ int launch_conv_tc_taps(const TapsArgs &a, cudaStream_t s)
     if ((a.ep.activation != DNB_LEAKY && a.ep.activation != DNB_LINEAR) || (a.ep.residual && (a.ep.activation2 != act2 || !a.y_nhwc || a.taps == 1)) ||
         (yolo && (a.ep.activation != DNB_LINEAR || a.ep.residual || a.y_nhwc || a.taps != 1)))
         DNB_FAIL(DNB_EINVAL, "conv_tc_taps: no variant of this epilogue");
-    if (a.bn < 16 || a.bn > 256 || a.bn % 16 || a.x_stages < 2 || a.x_stages > TAPS_MAX_X || a.w_stages < 1 || a.w_stages > TAPS_MAX_W || a.rows > 1024)
+    if (a.bn < 32 || a.bn > 256 || a.bn % 32 || a.x_stages < 2 || a.x_stages > TAPS_MAX_X || a.w_stages < 1 || a.w_stages > TAPS_MAX_W || a.rows > 1024)
         DNB_FAIL(DNB_EINVAL, "conv_tc_taps: plan out of range (bn %d, stages %d and %d, rows %d)", a.bn, a.x_stages, a.w_stages, a.rows);
     const TapsKernel kern = yolo ? (a.bf16 ? conv_tc_taps_kernel<TAPS_YOLO, true, false, true> : conv_tc_taps_kernel<TAPS_YOLO, false, false, true>)
                                  : a.ep.activation == DNB_LEAKY ? taps_kernel_of<DNB_LEAKY>(a.bf16 != 0, a.ep.residual != nullptr, a.taps == 1)

@@ -849,6 +849,26 @@ def test_a_pair_loads_the_filters_that_it_multiplies(filters, batch, height, wid
     assert np.array_equal(out["0"], out["2"])
 
 
+@pytest.mark.parametrize("filters", [16, 40, 80, 200, 232])
+@pytest.mark.parametrize("size", [1, 3])
+def test_pairs_multiply_columns_in_steps_of_32(filters, size, monkeypatch):
+    """Layers whose filters are an odd number of sixteens: whole numbers, equal to single CTAs to the bit, in either layout."""
+    import re
+    import numpy as np
+    case = conv_case(776, b=2, c=64, h=19, w=18, n=filters, size=size)
+    case = dict(case, x=np.rint(2 * case["x"]), w=np.rint(case["w"] / np.abs(case["w"]).max() * 6), biases=np.rint(9 * case["biases"]), scales=None, mean=None, var=None)
+    monkeypatch.setenv("DNB_TC_SPLITK", "0")
+    out = {}
+    for knob in ("0", "2"):
+        monkeypatch.setenv("DNB_TC_TAPS", knob)
+        plan, a, b = run_conv(case, dn.MODE_TF32, "nhwc", "nchw", both=True)
+        assert ("one_load_for" in plan.describe()) == (knob == "2"), plan.describe()
+        assert knob == "0" or int(re.search(r"bn=(\d+)", plan.describe()).group(1)) % 32 == 0, plan.describe()
+        assert np.array_equal(a, b)
+        out[knob] = a
+    assert np.array_equal(out["0"], out["2"])
+
+
 def test_calls_go_to_the_current_stream():
     """Inside torch's stream contexts, nested and left again, and to the stream that the caller names."""
     import torch
