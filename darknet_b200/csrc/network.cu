@@ -487,11 +487,10 @@ static int build_network(const char *text, int mode, int batch_override, dnb_net
     // on the tensor cores adds in the reference's order of the products.
     for (Layer &L : net->layers) if (L.plan) L.plan->keep_k_order = any_xnor;
     // Sums stay in one order where their last bits grow: a classifier's [softmax] makes 0.015 of a probability of one TF32 bit (ResNet-50, 256 images), and
-    // bf16 roundings add up over a deep network (YOLOv3's outputs move by 1 to 2 % with the order, those of YOLOv3-tiny, 13 convolutions, by 0.25).
+    // bf16 roundings add up over a network's layers (YOLOv3's outputs move by 1 to 2 % with the order, those of YOLOv3-tiny by 0.25).
     bool any_softmax = false;
-    int convolutions = 0;
-    for (const Layer &L : net->layers) { any_softmax |= L.kind == L_SOFTMAX; convolutions += L.kind == L_CONV; }
-    if (any_softmax || (net->mode == DNB_MODE_BF16 && convolutions > 24))
+    for (const Layer &L : net->layers) any_softmax |= L.kind == L_SOFTMAX;
+    if (any_softmax || net->mode == DNB_MODE_BF16)
         for (Layer &L : net->layers) if (L.plan) L.plan->tap_order = true;
     const Layer &last = net->layers.back();
     net->outputs = last.out_c * last.out_h * last.out_w;

@@ -869,6 +869,41 @@ def test_pairs_multiply_columns_in_steps_of_32(filters, size, monkeypatch):
     assert np.array_equal(out["0"], out["2"])
 
 
+@pytest.mark.parametrize("mode,tail", [(dn.MODE_TF32, "yolo"), (dn.MODE_BF16, "yolo"), (dn.MODE_TF32, "softmax"), (dn.MODE_TF32, "xnor")])
+def test_networks_that_keep_the_order_of_their_sums(mode, tail, tmp_path, monkeypatch):
+    """3x3 layers over several blocks of channels, of a size that takes the kernel with one load for nine taps by itself, whose sums run in another order: a TF32
+    detector's do; those of networks whose sums keep theirs (bf16, a [softmax], xnor layers), however few their layers, do not, and the outputs are what they are without that kernel, to the bit."""
+    import numpy as np
+    from darknet_b200 import synth
+    layers = synth._conv(64, 3) + synth._conv(120, 3) + synth._conv(128, 3)
+    if tail == "yolo":
+        layers += synth._conv(90, 1, bn=False, act="linear") + synth._yolo("0,1", "10,14, 23,27", 2, 40)
+    elif tail == "softmax":
+        layers += synth._conv(90, 1, bn=False, act="linear") + "\n[avgpool]\n\n[softmax]\ngroups=1\n"
+    else:
+        layers += synth._conv(64, 3, xnor=True) + "\n[avgpool]\n"
+    cfg = synth._net(12, 128, 128) + layers
+    path = str(tmp_path / "o.weights")
+    synth.write_weights(path, synth.seeded_params(cfg, 25))
+    x = synth.seeded_input(cfg, 26)
+    out = []
+    for knob in (None, "0"):
+        monkeypatch.delenv("DNB_TC_TAPS", raising=False)
+        if knob:
+            monkeypatch.setenv("DNB_TC_TAPS", knob)
+        net = dn.Network(cfg, path, mode, text=True)
+        result = net.predict(x).copy()
+        out.append((net.layer_output(2), result))
+        moved = "one_load_for_nine_taps" in net.layer_describe(2)
+        assert moved == (knob is None and mode == dn.MODE_TF32 and tail == "yolo"), net.layer_describe(2)
+        net.close()
+    for a, b in zip(*out):
+        if mode == dn.MODE_TF32 and tail == "yolo":
+            parity(a, b, 1e-2)
+        else:
+            assert np.array_equal(a, b)
+
+
 def test_calls_go_to_the_current_stream():
     """Inside torch's stream contexts, nested and left again, and to the stream that the caller names."""
     import torch
