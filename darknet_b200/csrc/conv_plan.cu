@@ -4,6 +4,7 @@
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
 #include <vector>
 
@@ -423,6 +424,26 @@ extern "C" int dnb_conv_plan_set_diagnostics(dnb_conv_plan *p, long long wait_li
 }
 
 // ------------------------------------------------------------------ tensor-core launch block
+// The tuning knobs of a launch block (DNB_TC_..., null where unset), from one pass over the environment.  A block asks for some of them several times, some 25
+// lookups of the whole environment: without them a block of a 1x1 layer takes 4.9 us, 5.5 before (90 variables).
+struct Knobs {
+    const char *bn = nullptr, *pair = nullptr, *epi = nullptr, *halo = nullptr, *warp_stores = nullptr, *splitk = nullptr, *flat = nullptr, *debug = nullptr, *srb = nullptr,
+               *min_stages = nullptr, *ctas = nullptr, *max2 = nullptr, *shortk = nullptr, *stages = nullptr, *taps = nullptr, *taps_bn = nullptr, *taps_box = nullptr;
+    Knobs()
+    {
+        const struct { const char *name, **value; } all[] = {
+            {"BN", &bn}, {"PAIR", &pair}, {"EPI", &epi}, {"HALO", &halo}, {"WARP_STORES", &warp_stores}, {"SPLITK", &splitk}, {"FLAT", &flat}, {"DEBUG", &debug}, {"SRB", &srb},
+            {"MIN_STAGES", &min_stages}, {"CTAS", &ctas}, {"MAX2", &max2}, {"SHORTK", &shortk}, {"STAGES", &stages}, {"TAPS", &taps}, {"TAPS_BN", &taps_bn}, {"TAPS_BOX", &taps_box}};
+        for (char **e = environ; e && *e; ++e) {
+            if (strncmp(*e, "DNB_TC_", 7) != 0) continue;
+            const char *const name = *e + 7, *const eq = strchr(name, '=');
+            if (!eq) continue;
+            for (const auto &k : all)
+                if (strlen(k.name) == (size_t)(eq - name) && strncmp(k.name, name, (size_t)(eq - name)) == 0) *k.value = eq + 1;
+        }
+    }
+};
+
 // Relative cost of writing NCHW output in runs of `run` contiguous pixels (tuning knob DNB_TC_NCHW_PENALTY scales it;
 // 0 = the tile that suits channels-last output).
 static double nchw_run_penalty(int run)
@@ -693,7 +714,7 @@ static double uncut_us(const TcArgs &a, int k_iters, bool residual)
 
 // Tiles of the persistent kernel for a launch of geometry g: pixel box, filters per tile, pairs.  a.row_bytes, a.c_blocks are set.
 // plain: by the number of tiles alone (see uncut_us).
-static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual, bool pool = false, bool plain = false)
+static void pick_persistent_tiles(const dnb_conv_plan *p, const Knobs &knobs, const ConvGeom &g, TcArgs &a, bool nchw_out, bool channels_last, int y_cpitch, bool residual, bool pool = false, bool plain = false)
 {
     const bool bf16 = p->kernel == K_TC_BF16, i8 = p->kernel == K_XNOR;
     pick_pixel_tile(g, nchw_out, &a.wt, &a.ht, &a.bt, pool);
@@ -715,7 +736,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
         }
     }
     // Tuning knobs for experiments: DNB_TC_BN (filters per tile, a multiple of 64) and DNB_TC_STAGES.
-    if (const char *e = getenv("DNB_TC_BN")) {
+    if (const char *e = knobs.bn) {
         const int v = atoi(e);
         if (v >= 64 && v <= 256 && v % 64 == 0 && p->n_pad > v) a.bn = v;
     }
@@ -755,7 +776,7 @@ static void pick_persistent_tiles(const dnb_conv_plan *p, const ConvGeom &g, TcA
     // 20 in single CTAs).  DNB_TC_PAIR: 0 never, 1 3x3 layers of fewer iterations too, 2 every layer the geometry allows.
     a.pair = 0;
     {
-        const char *e = getenv("DNB_TC_PAIR");
+        const char *e = knobs.pair;
         const int knob = e ? atoi(e) : -1;
         // (the pair kernel is built for 128-byte staged rows only: it needs a channels-last output at least that wide)
         // Enough pair tiles to occupy every pair of SMs; or, for long K loops (small batches of the 19x19 and 38x38
@@ -874,11 +895,11 @@ static double taps_us(const TapsArgs &a, bool nchw_out, bool residual, bool yolo
 }
 
 // The best tile of a launch of geometry g, in p->tp; its estimated time, or 1e300.
-static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last, bool nchw_out, bool residual, bool yolo)
+static double best_taps(dnb_conv_plan *p, const Knobs &knobs, const ConvGeom &g, bool channels_last, bool nchw_out, bool residual, bool yolo)
 {
-    const char *e = getenv("DNB_TC_TAPS_BN");
+    const char *e = knobs.taps_bn;
     const int only = e ? atoi(e) : 0;
-    const char *be = getenv("DNB_TC_TAPS_BOX");
+    const char *be = knobs.taps_box;
     int best_bn = 0, best_boxes = 0;
     double best = 1e300;
     for (int bn = 64; bn <= 256; bn *= 2)
@@ -910,9 +931,9 @@ static double best_taps(dnb_conv_plan *p, const ConvGeom &g, bool channels_last,
 // with a [yolo] layer's logistic 271 -> 174, 345 -> 226 inside YOLOv3-608); a launch of less than two rounds of pairs is not worth their set-up
 // (255 filters and the logistic at 26 x 26, one image: 7.2 us, 8.9 here).
 // DNB_TC_TAPS: 0 never, 2 wherever the kernel has the variant; the other kernels' knobs ask for those kernels.
-static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
+static bool taps_pay(dnb_conv_plan *p, const Knobs &knobs, const ConvGeom &g, bool cut, double others_us, const ConvEpilogue *res, bool channels_last, bool nchw_out)
 {
-    const char *e = getenv("DNB_TC_TAPS");
+    const char *e = knobs.taps;
     const int knob = e ? atoi(e) : 1;
     if (knob == 0) return false;
     const bool residual = res && res->residual;
@@ -924,10 +945,10 @@ static bool taps_pay(dnb_conv_plan *p, const ConvGeom &g, bool cut, double other
         if (g.size == 3 && 5.3 + 9.0 * c_blocks * 0.174 + 0.65 >= 0.9 * slack * others_us) return false;
     }
     if (!e) {
-        const char *const split = getenv("DNB_TC_SPLITK");
-        if (getenv("DNB_TC_PAIR") || getenv("DNB_TC_EPI") || getenv("DNB_TC_HALO") || getenv("DNB_TC_WARP_STORES") || (split && atoi(split) > 1)) return false;
+        const char *const split = knobs.splitk;
+        if (knobs.pair || knobs.epi || knobs.halo || knobs.warp_stores || (split && atoi(split) > 1)) return false;
     }
-    const double us = best_taps(p, g, channels_last, nchw_out, residual, yolo);
+    const double us = best_taps(p, knobs, g, channels_last, nchw_out, residual, yolo);
     if (us >= 1e300 || knob == 2) return us < 1e300;
     if (g.size == 1) {
         const TapsArgs &t = p->tp;
@@ -969,6 +990,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
 {
     const void *residual = res ? res->residual : nullptr;   // fused residual, if any
     const int res_cpitch = res ? res->res_cpitch : 0, res_stride = residual ? res->res_stride : 1, res_c = residual ? res->res_c : 0;
+    const Knobs knobs;
     TcArgs &a = p->tc;
     p->tc_x_ptr = nullptr;   // until all of the block is there
     p->tc_res_act = residual ? res->activation2 : DNB_LINEAR;
@@ -978,7 +1000,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // pixels of every filter plane (and of the channels-last input) instead of a wt x ht patch.  DNB_TC_FLAT=0: never.
     ConvGeom g = p->g;
     {
-        const char *e = getenv("DNB_TC_FLAT");
+        const char *e = knobs.flat;
         if (nchw_out && g.size == 1 && g.stride == 1 && g.pad == 0 && !(e && atoi(e) == 0)) {
             g.w = g.out_w = g.w * g.h;
             g.h = g.out_h = 1;
@@ -994,10 +1016,10 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.bk = a.row_bytes / es;
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
     a.taps = g.size * g.size;
-    a.debug = (getenv("DNB_TC_DEBUG") ? atoi(getenv("DNB_TC_DEBUG")) : 0) | p->debug_bits;
+    a.debug = (knobs.debug ? atoi(knobs.debug) : 0) | p->debug_bits;
     a.wait_limit = p->wait_limit > 0 ? p->wait_limit : DEFAULT_WAIT_CYCLES;
     p->tc_taps = p->tc_split = false;
-    pick_persistent_tiles(p, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, pool);
+    pick_persistent_tiles(p, knobs, g, a, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, pool);
     a.pool = pool ? 1 : 0;
     a.n_pad = p->n_pad;
     a.n_tot = a.n_tiles * a.bn;
@@ -1013,11 +1035,11 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     int srb = pitch_bytes >= 128 ? 128 : (pitch_bytes >= 64 ? 64 : 32);
     if (srb < min_srb) srb = min_srb;  // the box may be wider than a narrow tensor: the TMA unit clips it
     if (sign_out && (pitch_bytes < 128 || !i8)) DNB_FAIL(DNB_EINVAL, "conv: the sign output needs an int8-kind plan with at least 32 output channels");
-    if (const char *e = getenv("DNB_TC_SRB")) {   // tuning knob: widest staged row to try (128, 64 or 32)
+    if (const char *e = knobs.srb) {   // tuning knob: widest staged row to try (128, 64 or 32)
         const int v = atoi(e);
         if ((v == 128 || v == 64 || v == 32) && v >= min_srb && v < srb && !a.pair) srb = v;
     }
-    const int min_stages = getenv("DNB_TC_MIN_STAGES") ? atoi(getenv("DNB_TC_MIN_STAGES")) : 4;
+    const int min_stages = knobs.min_stages ? atoi(knobs.min_stages) : 4;
     // two accumulators of bn columns; TMEM is allocated in powers of two >= 32 columns
     a.tmem_cols = 32;
     while (a.tmem_cols < 2 * a.bn) a.tmem_cols *= 2;
@@ -1030,7 +1052,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     a.sign_out = sign_out;
     a.sign_cpitch = sign_cpitch;
     int stages = 0;
-    const bool allow2 = getenv("DNB_TC_CTAS") ? atoi(getenv("DNB_TC_CTAS")) >= 2 : true;
+    const bool allow2 = knobs.ctas ? atoi(knobs.ctas) >= 2 : true;
     a.a_slot = a.a_box_slot = a.a_box_bytes = a.a_pitch = 0;
     a.epi_groups = 1;
     a.halo = 0;
@@ -1043,7 +1065,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     // Pooled launches stage nothing and their epilogue is the longer part: as many CTAs as TMEM takes (xnor 32 -> 64 at 128 x 112 x 112 103 us with two, 93 with
     // three, 90 with four; 16 -> 32 in TF32 at 16 x 208 x 208 49, 42, 37)
     const int most_ctas = pool && a.tmem_cols <= 128 ? 4 : 2;
-    const int halo_knob = getenv("DNB_TC_HALO") ? atoi(getenv("DNB_TC_HALO")) : 1;
+    const int halo_knob = knobs.halo ? atoi(knobs.halo) : 1;
     if (halo_knob != 0 && g.size == 3 && g.pad == 1 && a.n_tiles == 1 && !a.pair && g.out_w >= 8 && g.out_h >= 16) {
         const int lattices = g.stride * g.stride, htiles = ((g.out_w + 7) / 8) * ((g.out_h + 15) / 16) * g.batch;
         a.a_pitch = g.stride == 1 ? 10 : 9;
@@ -1078,7 +1100,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     if (!a.halo) {
         // (not when every tile has an SM of its own: one deep ring then)
         if (allow2 && a.tmem_cols <= 256 && !a.pair && a.total_tiles > sm_count()) {
-            const int max2 = getenv("DNB_TC_MAX2") ? atoi(getenv("DNB_TC_MAX2")) : 4;   // ring slots per CTA when two share the SM
+            const int max2 = knobs.max2 ? atoi(knobs.max2) : 4;   // ring slots per CTA when two share the SM
             const long budget = (228L * 1024) / 2 - 2048;   // per CTA when two share the SM (1 KB each is reserved by the system)
             for (int srb2 = srb; srb2 >= min_srb; srb2 /= 2) {   // narrower staged rows if that is what makes two CTAs fit
                 const int s2 = (int)((budget - (long)conv_tc_fixed_smem(srb2, a.bn, a.stage_bufs)) / (a.a_bytes + a.b_bytes));
@@ -1094,9 +1116,9 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         //  * xnor layers: 256 -> 128 at 128 x 28 x 28 28.1 -> 26.6, 512 -> 256 at 14 x 14 21.0 -> 19.0
         // Other single CTAs are bound by memory (512 -> 256 at 64 x 52 x 52 in bf16 52 and 52), with a residual they want its tiles by TMA, three
         // chunks ahead (64 -> 256 at 256 x 56 x 56 342 us, 416 through this path).  DNB_TC_EPI=1: one group (pairs with a residual: two).
-        const int loop = g.size * g.size * a.c_blocks, epi_knob = getenv("DNB_TC_EPI") ? atoi(getenv("DNB_TC_EPI")) : 2;
+        const int loop = g.size * g.size * a.c_blocks, epi_knob = knobs.epi ? atoi(knobs.epi) : 2;
         const bool two = pool ? false : residual ? a.pair != 0 : epi_knob != 1 && (a.pair ? loop < 32 : nchw_out || i8);
-        if (a.ctas_per_sm == 1 && two && (a.pair || !getenv("DNB_TC_SRB")) && (!y_nhwc || srb == 128)) {
+        if (a.ctas_per_sm == 1 && two && (a.pair || !knobs.srb) && (!y_nhwc || srb == 128)) {
             const int bufs = y_nhwc ? a.stage_bufs : 0;
             const int fit = (int)((max_smem - (long)conv_tc_fixed_smem(128, a.bn, bufs)) / (a.a_bytes + a.b_bytes));
             if (fit >= 3) { a.epi_groups = 2; a.stage_bufs = bufs; stages = fit; srb = 128; }
@@ -1106,7 +1128,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
             // The exception is a fused residual behind a short K loop, where the epilogue (one round of barrier,
             // residual wait and store per staged chunk) would outlast the tile's MMAs: fewer, wider chunks then.
             const int k_iters = g.size * g.size * a.c_blocks;
-            const bool short_k_rule = getenv("DNB_TC_SHORTK") ? atoi(getenv("DNB_TC_SHORTK")) != 0 : true;
+            const bool short_k_rule = knobs.shortk ? atoi(knobs.shortk) != 0 : true;
             const int short_k = bf16 ? 32 : 64;   // measured: 76x76x128 -> 256 layers want the wide rows in both modes, 38x38x256 -> 512 only in TF32
             const int want = (residual && k_iters < short_k && min_stages > 3 && short_k_rule) ? 3 : min_stages;
             for (;; srb /= 2) {
@@ -1116,7 +1138,7 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         }
     }
     if (stages > 8) stages = 8;
-    if (const char *e = getenv("DNB_TC_STAGES")) {
+    if (const char *e = knobs.stages) {
         const int v = atoi(e);
         if (v >= 2 && v <= stages) stages = v;
     }
@@ -1126,17 +1148,14 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
     {   // DNB_TC_WARP_STORES=1 (experiment, off): every epilogue warp stores its own 32 rows and the four warps meet once
         // per tile instead of twice per chunk.  Measured on YOLOv3-608 b64: the layers' event times drop by 0.5 %, the
         // step replayed as one CUDA graph takes 2 % longer (18.5 -> 18.9 ms), batch 8 and ResNet-50 do not move.
-        const char *e = getenv("DNB_TC_WARP_STORES");
+        const char *e = knobs.warp_stores;
         a.warp_stores = e ? (atoi(e) != 0) : 0;
     }
     // A launch that leaves SMs idle, or whose few tiles have a long K loop: one tile per cluster, K cut across it
     // (conv_tc_split.cu).  Chosen where its estimate is below the persistent kernel's, which overlaps a tile's epilogue with the
     // next one's MMAs and therefore wins once every SM has a few tiles.  DNB_TC_SPLITK: 0 never, N forces N ranges (tests).
-    const bool may_cut = [&] {
-        const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
-        const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1;
-        return knob != 0 && !a.halo && !pool && (i8 || !p->keep_k_order) && (knob > 1 || pair_knob != 2);
-    }();
+    const int split_knob = knobs.splitk ? atoi(knobs.splitk) : -1, pair_knob = knobs.pair ? atoi(knobs.pair) : 1;
+    const bool may_cut = split_knob != 0 && !pool && (i8 || !p->keep_k_order) && (split_knob > 1 || pair_knob != 2);
     // pixels of a 1x1 layer in one row: of the whole batch where nothing is stored per image
     auto flat = [&](ConvGeom sg) {
         if (sg.size == 1 && sg.stride == 1 && sg.pad == 0) {
@@ -1147,39 +1166,39 @@ static int build_tc_args(dnb_conv_plan *p, const dnb_tensor *x, void *y_nhwc, in
         return sg;
     };
     auto cut_at = [&](const ConvGeom &at) {   // the cut launch of that geometry, no ranges where it is not cut
-        const char *e = getenv("DNB_TC_SPLITK"), *pe = getenv("DNB_TC_PAIR");
-        const int knob = e ? atoi(e) : -1, pair_knob = pe ? atoi(pe) : 1, k_iters = at.size * at.size * a.c_blocks;
+        const int k_iters = at.size * at.size * a.c_blocks;
         SplitQuery q;
         q.row_bytes = a.row_bytes; q.k_iters = k_iters; q.n_pad = p->n_pad; q.max_smem = max_smem;
         q.pair_ok = pair_knob > 0 && a.row_bytes == 128 && at.n % 256 == 0 && k_iters >= 16;
         q.residual = residual != nullptr;
         q.long_sum = at.c * at.size * at.size >= 8192;
-        if (knob > 1) return choose_split(q, flat(at), knob < 8 ? knob : 8, true, at.batch);
+        if (split_knob > 1) return choose_split(q, flat(at), split_knob < 8 ? split_knob : 8, true, at.batch);
         // decided at one image for two images also (see choose_split)
         ConvGeom dg = at;
         if (at.batch == 2) dg.batch = 1;
         TcArgs da = a;
-        pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, false, true);
+        pick_persistent_tiles(p, knobs, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr, false, true);
         SplitPlan sp = choose_split(q, flat(dg), 0, false, dg.batch);
         if (!(sp.cost < uncut_us(da, k_iters, q.residual))) sp = SplitPlan();
         else if (at.batch == 2) sp = choose_split(q, flat(at), sp.splits, false, 2);
         return sp;
     };
-    const SplitPlan cut = may_cut ? cut_at(g) : SplitPlan();
+    const SplitPlan cut = may_cut && !a.halo ? cut_at(g) : SplitPlan();
     if (!pool && !i8 && taps_covers(p, res, nchw_out)) {
         const int whole = p->whole_batch > g.batch ? p->whole_batch : g.batch;
         ConvGeom dg = g;
         dg.batch = whole <= 2 ? 1 : whole;
         SplitPlan dcut = cut;
         TcArgs da = a;
-        if (dg.batch != g.batch) {
-            if (may_cut) dcut = cut_at(dg);
-            pick_persistent_tiles(p, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
+        if (dg.batch != g.batch || a.halo) {   // (nor does the choice hang on whether this part has its weights in place)
+            dcut = may_cut ? cut_at(dg) : SplitPlan();
+            pick_persistent_tiles(p, knobs, dg, da, nchw_out, y_nhwc != nullptr, y_cpitch, residual != nullptr);
         }
         double others = dcut.splits ? dcut.cost : persistent_us(da.pair, da.bn, da.total_tiles, a.taps * a.c_blocks, residual != nullptr, res && res->yolo_entries);
         if (!dcut.splits && !da.pair && da.bn > 128 && da.bn <= 192) others *= 0.85;   // (that estimate is of 256 filters)
-        p->tc_taps = taps_pay(p, dg, dcut.splits != 0, others, res, y_nhwc != nullptr, nchw_out) &&
-                     best_taps(p, g, y_nhwc != nullptr, nchw_out, residual != nullptr, res && res->yolo_entries) < 1e300;
+        // (the tile that it was decided with is there already, unless it is that of another batch)
+        p->tc_taps = taps_pay(p, knobs, dg, dcut.splits != 0, others, res, y_nhwc != nullptr, nchw_out) &&
+                     (dg.batch == g.batch || best_taps(p, knobs, g, y_nhwc != nullptr, nchw_out, residual != nullptr, res && res->yolo_entries) < 1e300);
     }
     if (p->tc_taps) DNB_TRY(build_taps_args(p, x, y_nhwc, y_cpitch));
     else if (cut.splits) DNB_TRY(build_split_args(p, x, flat(g), cut, kind, es, y_nhwc, y_cpitch, sign_out, sign_cpitch));
@@ -1564,12 +1583,13 @@ bool conv_pool_fusable(dnb_conv_plan *p, bool in_order)
     }
     if (p->kernel != K_TC_TF32 && !bf16 && !i8) return false;
     if (p->d.activation != DNB_LEAKY || g.out_h % 2 || g.out_w % 2 || g.n * (bf16 ? 2 : 4) < 128 || g.n % 8) return false;
+    const Knobs knobs;
     TcArgs a;
     const int es = i8 ? 1 : bf16 ? 2 : 4, c_pad = i8 ? p->c_pad_i8 : p->c_pad;
     a.row_bytes = c_pad * es >= 128 ? 128 : c_pad * es >= 64 ? 64 : 32;
     a.bk = a.row_bytes / es;
     a.c_blocks = (c_pad + a.bk - 1) / a.bk;
-    pick_persistent_tiles(p, g, a, false, true, g.n, false);
+    pick_persistent_tiles(p, knobs, g, a, false, true, g.n, false);
     const int k_iters = g.size * g.size * a.c_blocks;
     if (a.pair || a.total_tiles < (k_iters <= 12 ? sm_count() / 2 : sm_count())) return false;
     p->pool_fits = 1;

@@ -904,6 +904,55 @@ def test_networks_that_keep_the_order_of_their_sums(mode, tail, tmp_path, monkey
             assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("mode", [dn.MODE_TF32, dn.MODE_BF16])
+def test_parts_of_a_batch_keep_its_kernels(mode, tmp_path, monkeypatch):
+    """A step that runs in parts, first layers and last ones with plans of their own over fewer images: those plans choose between the kernels whose sums run in
+    different orders as the whole batch's does, and the results are its, to the bit."""
+    import numpy as np
+    import torch
+    from darknet_b200 import synth
+    monkeypatch.delenv("DNB_TC_TAPS", raising=False)
+    cfg = (synth._net(16, 256, 256) + synth._conv(32, 3) + synth._conv(64, 3, stride=2) + synth._conv(128, 3) + synth._conv(64, 1) + synth._conv(128, 3) + synth._conv(128, 3) +
+           synth._conv(90, 1, bn=False, act="linear") + synth._yolo("0,1", "10,14, 23,27", 2, 40))
+    path = str(tmp_path / "b.weights")
+    synth.write_weights(path, synth.seeded_params(cfg, 27))
+    x = synth.seeded_input(cfg, 28)
+    whole, parts = (dn.Network(cfg, path, mode, text=True) for _ in range(2))
+    whole.forward(torch.from_numpy(x).cuda())
+    torch.cuda.synchronize()
+    got = parts.predict(x)
+    tiles = lambda net, i: net.layer_describe(i).split("tiles=")[1].split()[0]  # noqa: E731
+    for i in (2, 4):
+        assert "one_load_for_nine_taps" in whole.layer_describe(i) and "one_load_for_nine_taps" in parts.layer_describe(i), i
+    assert int(tiles(parts, 2)) < int(tiles(whole, 2))
+    assert np.array_equal(got.reshape(-1), whole.layer_output(7).reshape(-1))
+    whole.close(), parts.close()
+
+
+@pytest.mark.parametrize("mode,batch,c,n,height,width,layout,taken", [
+    (dn.MODE_TF32, 2, 96, 96, 239, 210, "nhwc", True), (dn.MODE_TF32, 2, 40, 96, 260, 104, "nhwc", True), (dn.MODE_BF16, 2, 96, 96, 112, 229, "nhwc", True),
+    (dn.MODE_BF16, 2, 128, 96, 126, 224, "nhwc", True), (dn.MODE_TF32, 4, 512, 1024, 19, 19, "nhwc", True), (dn.MODE_TF32, 8, 256, 512, 52, 52, "nchw", True),
+    (dn.MODE_TF32, 2, 96, 128, 76, 75, "nhwc", False), (dn.MODE_TF32, 2, 64, 64, 152, 152, "nhwc", False), (dn.MODE_BF16, 2, 128, 256, 38, 38, "nhwc", False),
+    (dn.MODE_TF32, 2, 256, 96, 100, 90, "nhwc", False)])
+def test_layers_that_take_one_load_for_nine_taps_by_themselves(mode, batch, c, n, height, width, layout, taken, monkeypatch):
+    """The choice as it is without a knob.  Two images take what one takes, and an image's result is the same, to the bit; whole numbers are what they are without the kernel."""
+    import numpy as np
+    for knob in ("DNB_TC_TAPS", "DNB_TC_SPLITK", "DNB_TC_PAIR"):
+        monkeypatch.delenv(knob, raising=False)
+    case = conv_case(785, b=batch, c=c, h=height, w=width, n=n, size=3, bn=False)
+    plan, whole, _ = run_conv(case, mode, "nhwc", layout)
+    assert ("one_load_for_nine_taps" in plan.describe()) == taken, plan.describe()
+    if batch == 2:
+        for k in range(2):
+            alone, one, _ = run_conv(dict(case, x=case["x"][k:k + 1]), mode, "nhwc", layout)
+            assert ("one_load" in alone.describe()) == taken and np.array_equal(one[0], whole[k]), alone.describe()
+    case = dict(case, x=np.rint(2 * case["x"]), w=np.rint(case["w"] / np.abs(case["w"]).max() * 6), biases=np.rint(9 * case["biases"]))
+    out = [run_conv(case, mode, "nhwc", layout)[1]]
+    monkeypatch.setenv("DNB_TC_TAPS", "0")
+    out.append(run_conv(case, mode, "nhwc", layout)[1])
+    assert np.array_equal(*out)
+
+
 def test_calls_go_to_the_current_stream():
     """Inside torch's stream contexts, nested and left again, and to the stream that the caller names."""
     import torch
