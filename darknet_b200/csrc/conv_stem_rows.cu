@@ -277,7 +277,7 @@ conv_stem_rows_kernel(const __grid_constant__ StemTcArgs a)
 //  * the pixels of the same place in their windows are one MMA's 128 rows: a thread finds the four sums of its window in four accumulators, and what it
 //    scales, activates and rounds is the largest, none of which changes which one that is.  Sums of filters with a negative scale change sign first.  A
 //    warp that meets an infinity or NaN finishes all four, as the layer alone would, and then compares.
-// 128 x 224 x 224: 250 -> 142 us.  Bytes: 51; the sixteen MMAs a tile, 77 clocks each: 55; shared memory (rows written and read by the MMAs, patch): some 80.
+// 128 x 224 x 224: 250 -> 144 us.  Bytes: 51; the sixteen MMAs a tile, 77 clocks each: 55; shared memory (rows written and read by the MMAs, patch): some 80.
 // (The upper pixels' sums compared while the lower ones are multiplied: the same time.)
 constexpr int SRP_TW = 16, SRP_TH = 8, SRP_PITCH = 2 * SRP_TW + 2, SRP_ROWS = 2 * SRP_TH + 2;
 

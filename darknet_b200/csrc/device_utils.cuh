@@ -108,12 +108,14 @@ __device__ __forceinline__ uint32_t four_signs(uint4 v)
            (__uint_as_float(v.w) > 0.f ? 0x01u : 0xFFu) << 24;
 }
 
-// The same of four that are no NaN: of what is not > 0 the value itself or, of +0, one less is negative as an integer (-0 needs the former).
+// The same of four that are no NaN.  As integers the value itself, or one less, which for +0 wraps, has its top bit set where it is not > 0 (-0 among them):
+// so has the larger of the two.
 __device__ __forceinline__ uint32_t four_signs_no_nan(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
 {
+    auto not_positive = [](uint32_t v) { return __viaddmax_u32(v, 0xffffffffu, v); };
     uint32_t ab, cd;
-    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(ab) : "r"(a | (a - 1u)), "r"(b | (b - 1u)));   // their signs, as bytes
-    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(cd) : "r"(c | (c - 1u)), "r"(d | (d - 1u)));
+    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(ab) : "r"(not_positive(a)), "r"(not_positive(b)));   // their signs, as bytes
+    asm("prmt.b32 %0, %1, %2, 0xfb;" : "=r"(cd) : "r"(not_positive(c)), "r"(not_positive(d)));
     return __byte_perm(ab, cd, 0x5410u) | 0x01010101u;
 }
 
