@@ -45,11 +45,12 @@ import numpy as np  # noqa: E402
 
 UNIT = "images/s"
 
-# DRAM traffic of the tensor-core convolution kernel as ncu measured it (dram__bytes_read.sum + dram__bytes_write.sum
-# summed over the kernel's launches of one forward), as (bytes per image, bytes per forward independent of the batch:
-# the weights, read once per launch).  Scaled by the images one step processes.
+# DRAM traffic of the tensor-core convolution kernels as ncu measured it (dram__bytes_read.sum + dram__bytes_write.sum
+# summed over their launches of one forward), as (bytes per image, bytes per forward independent of the batch:
+# the weights, read once per launch).  Scaled by the images one step processes.  YOLOv3's is of a forward of 8 images, 73
+# launches of conv_tc_kernel and one of conv_tc_taps_kernel; larger batches run more of its layers on the latter.
 NCU_DRAM_TRAFFIC = {
-    ("yolov3", "tf32", 608): (545_665_920.0, 247_579_648.0),
+    ("yolov3", "tf32", 608): (547_698_784.0, 247_579_648.0),
     ("conv3x3", "tf32", 224): (488.0e6 / 64, 0.0),
     ("conv1x1", "tf32", 224): (491.0e6 / 64, 0.0),
 }
@@ -352,7 +353,7 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
     peak = bf16_peak / (2.0 if mode == "tf32" else 1.0)
     big3 = np.array([bool(tc[i]) and sections[i][1].get("size") == "3" and shapes[i].c >= 64 for i in range(net.n)])
     big3_tflops = float(flops[big3].sum() / (mean_ms[big3].sum() / 1000.0) / 1e12) if big3.any() else None
-    # the other launches of the same kernel (1x1 layers, 3x3 layers with fewer than 64 input channels) are bound by
+    # the other launches of the same kernels (1x1 layers, 3x3 layers with fewer than 64 input channels) are bound by
     # HBM: algorithmic bytes = input + output of the layer in its storage type, the weights once, and the residual
     # a fused [shortcut] reads, over the same event durations
     es = 2.0 if mode == "bf16" else 4.0
@@ -372,11 +373,17 @@ def roofline_of(net, cfg: str, per_gpu: int, mean_ms, mode: str, workload: str, 
     if small.any() and small_ms > 0:
         gbs = mem_bytes / (small_ms / 1000.0) / 1e9
         hbm_part = {"launches_per_step": int(small.sum()), "ms_per_step": small_ms, "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                    "frac": gbs / peaks["hbm_gbs"], "what": "1x1 layers and 3x3 layers with fewer than 64 input channels: HBM-bound launches of the same kernel"}
-    roofline = {"kernel": "conv_tc_kernel", "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                    "frac": gbs / peaks["hbm_gbs"], "what": "1x1 layers and 3x3 layers with fewer than 64 input channels: HBM-bound launches of the same kernels"}
+    # which kernel each of them runs on (conv_plan.cu chooses by size)
+    launches: dict[str, int] = {}
+    for i in np.nonzero(tc)[0]:
+        d = net.layer_describe(int(i))
+        name = "conv_tc_taps_kernel" if "one_load_for" in d else "conv_tc_split_kernel" if "one_tile_per_cluster" in d else "conv_tc_kernel"
+        launches[name] = launches.get(name, 0) + 1
+    roofline = {"kernel": " + ".join(sorted(launches)), "kernel_launches": launches, "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak,
                 "traffic": (lambda t: None if t is None else t[0] * per_gpu + t[1])(NCU_DRAM_TRAFFIC.get((workload, mode, size))),
-                "traffic_unit": "bytes per step per GPU (ncu dram read+write of all launches of this kernel)",
+                "traffic_unit": "bytes per step per GPU (ncu dram read+write of all launches of these kernels)",
                 "launches_per_step": int(tc.sum()), "avg_launch_ms": tc_ms / max(int(tc.sum()), 1),
                 "share_of_step": tc_ms / float(mean_ms.sum()),
                 "peak_source": f"{peaks['source']}: cuBLAS bf16 {'burst' if alone else 'sustained'} {bf16_peak} TFLOP/s"
