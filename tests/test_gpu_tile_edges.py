@@ -849,6 +849,19 @@ def test_a_pair_loads_the_filters_that_it_multiplies(filters, batch, height, wid
     assert np.array_equal(out["0"], out["2"])
 
 
+def test_filters_in_place_by_themselves(monkeypatch):
+    """A layer that takes two filter tiles in place without a knob, of which a pair meets one: equal to the kernel with a ring to the bit."""
+    import numpy as np
+    for knob in ("DNB_TC_TAPS", "DNB_TC_SPLITK", "DNB_TC_PAIR"):
+        monkeypatch.delenv(knob, raising=False)
+    case = conv_case(777, b=32, c=256, h=38, w=38, n=512, size=1)
+    plan, got, _ = run_conv(case, dn.MODE_BF16, "nhwc", "nhwc")
+    assert "bn=256" in plan.describe() and "one_load_for_a_block resident" in plan.describe(), plan.describe()
+    monkeypatch.setenv("DNB_TC_TAPS", "0")
+    plan, want, _ = run_conv(case, dn.MODE_BF16, "nhwc", "nhwc")
+    assert "one_load" not in plan.describe() and np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("filters", [16, 40, 80, 200, 232])
 @pytest.mark.parametrize("size", [1, 3])
 def test_pairs_multiply_columns_in_steps_of_32(filters, size, monkeypatch):
